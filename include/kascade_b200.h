@@ -67,9 +67,9 @@ typedef enum kascade_algorithm {
 
 /* Tunables.  Zero means "choose automatically" (the autotuned table).  The
  * reference's ruler-selection strategies (ruler_selection.hpp:18-79) size the
- * ruler set by the MPI rank count; on one GPU the mean ruler spacing is the
- * tunable instead (sparse_ruling_set.cpp:120-136 picks; here a counter hash
- * picks). */
+ * ruler set by the MPI rank count; on one GPU the ruler spacing is the tunable
+ * instead (sparse_ruling_set.cpp:120-136 picks; here one element of every
+ * block of that many indices is a ruler, at a hashed offset). */
 typedef struct kascade_opts {
   uint32_t struct_size;       /* sizeof(kascade_opts)                               */
   uint32_t algorithm;         /* kascade_algorithm for list ranking                 */
@@ -349,14 +349,14 @@ KASCADE_API kascade_status kascade_ctx_set_sm_budget(kascade_ctx* ctx, int sms);
  * lanes free up and both lanes' work overlaps on the device.
  * ------------------------------------------------------------------------- */
 typedef struct kascade_server kascade_server;
-/* Batch plans: one batch captured once as a CUDA graph (the whole
- * device-driven pipeline: record build, forest tours, every ruling-set level,
- * propagation) and replayed by one graph launch per call.  The segment table
+/* Batch plans: one batch captured once as a CUDA graph (the whole pipeline:
+ * record build, forest tours, every ruling-set level, propagation) and
+ * replayed by one graph launch per call.  The segment table
  * and the input / weight / output pointers are fixed at creation; their
  * contents may change between launches.  Creation runs the batch once and
- * returns KASCADE_ERR_UNSUPPORTED if it needs the host-driven recursion (a
- * level outgrowing its capacity, e.g. very many roots); a launch that meets
- * that case (new contents with far more roots) returns KASCADE_ERR_TIMEOUT,
+ * returns KASCADE_ERR_UNSUPPORTED for a batch made mostly of list ends (very
+ * many roots); a launch whose new contents run a chain past the write-free
+ * chase's hop cap returns KASCADE_ERR_TIMEOUT,
  * and kascade_rank_batch handles such a batch.  A plan owns its scratch;
  * launches of one plan are ordered on the device.  No counterpart in the
  * reference (its rounds are MPI exchanges per call). */

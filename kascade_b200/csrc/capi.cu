@@ -8,7 +8,7 @@
 
 namespace ks {
 kascade_status root_forest_impl(kascade_ctx& ctx, const uint64_t* parent, uint32_t n, uint64_t* root_out,
-                                uint64_t* depth_out, int keep_roots, const Params& p, cudaStream_t s, bool device_levels = false);
+                                uint64_t* depth_out, int keep_roots, const Params& p, cudaStream_t s, bool host_check);
 kascade_status compute_euler_tour_impl(kascade_ctx& ctx, const uint64_t* parent, uint32_t n, uint64_t* tour,
                                        uint64_t* m_out, cudaStream_t s);
 kascade_status gen_list(uint64_t n, uint64_t seed, uint32_t layout, uint64_t* succ, cudaStream_t s);
@@ -25,7 +25,7 @@ kascade_status unpack_impl(kascade_ctx& ctx, const uint64_t* succ_packed, const 
                            cudaStream_t s);
 kascade_status rank_batch_impl(kascade_ctx& ctx, const kascade_segment* segs, uint32_t nseg, const uint64_t* in,
                                const uint32_t* weights, uint64_t total, uint64_t* root_out, uint64_t* rank_out,
-                               const kascade_opts* opts, cudaStream_t s, bool device_levels);
+                               const kascade_opts* opts, cudaStream_t s, bool host_check);
 }  // namespace ks
 
 using namespace ks;
@@ -49,7 +49,6 @@ kascade_status begin_call(kascade_ctx* ctx, cudaStream_t s, const kascade_opts* 
   ctx->profile = o && o->profile;
   ctx->async_pending = false;
   ctx->host_rerun.set = false;
-  ctx->pending_levels = 0;
   return KASCADE_OK;
 }
 
@@ -70,40 +69,25 @@ kascade_status end_call(kascade_ctx* ctx, cudaStream_t s, kascade_status st, con
   return status_finish(*ctx, s);
 }
 
-// device_levels: the ruling-set recursion keeps its level sizes on the device
-// (no host wait inside the call); a list it cannot hold reports
-// KASCADE_ERR_TIMEOUT and the caller reruns without it.  Only for calls whose
-// outputs are not their inputs (the rerun needs the inputs intact).
+// host_check: see rank_records.  Calls whose status is read later, or whose
+// outputs are their inputs, cannot be rerun on KASCADE_ERR_TIMEOUT and set it.
 kascade_status rank_list_generic(kascade_ctx& ctx, const uint64_t* succ, WKind wk, const void* w, uint64_t n,
                                  uint64_t* root_out, uint64_t* rank_out, int keep_roots, const Params& p,
-                                 cudaStream_t s, bool device_levels = false) {
+                                 cudaStream_t s, bool host_check) {
   if (n == 0) return KASCADE_OK;
   if (n > MAX_LIST) return KASCADE_ERR_TOO_LARGE;
+  const SinkPlain sink{root_out, rank_out, keep_roots};
+  const bool ruling_set = p.algorithm == KASCADE_ALGO_SPARSE_RULING_SET;
+  if (ruling_set && n <= p.base_max) return rank_arrays_one_cta(ctx, succ, wk, w, (uint32_t)n, sink, s);
   Rec* rec = alloc<Rec>(ctx, n);
-  uint32_t* ruler_elem = alloc<uint32_t>(ctx, n);
-  if (!rec || !ruler_elem) return KASCADE_ERR_OOM;
-  if (device_levels && p.algorithm == KASCADE_ALGO_SPARSE_RULING_SET && n > p.base_max && p.max_levels > 0) {
-    uint32_t* r_dev = nullptr;
-    SinkPlain sink{root_out, rank_out, keep_roots};
-    if (n < p.level0_log_min) {
-      KS_TRY(prepare_arrays(ctx, succ, wk, w, (uint32_t)n, rec, ruler_elem, nullptr, p, s, &r_dev));
-      return rank_records_dev(ctx, rec, (uint32_t)n, r_dev, dev_cap_next((uint32_t)n, p.spacing0), ruler_elem,
-                              sink, p, s);
-    }
-    if (!keep_roots) {
-      // the write-free level 0 with the ruler count and the deeper levels on the device
-      KS_TRY(prepare_arrays(ctx, succ, wk, w, (uint32_t)n, rec, ruler_elem, nullptr, p, s, &r_dev));
-      return rank_level0_log(ctx, rec, (uint32_t)n, dev_cap_next((uint32_t)n, p.spacing0), ruler_elem,
-                             sink.log_target((uint32_t)n), p, s, r_dev);
-    }
+  if (!rec) return KASCADE_ERR_OOM;
+  KS_TRY(prepare_arrays(ctx, succ, wk, w, (uint32_t)n, rec, p, s));
+  if (ruling_set) {
+    Extent ext;
+    ext.cap = (uint32_t)n;
+    return rank_records(ctx, rec, (uint32_t)n, ext, Heads{}, sink, p, s, host_check);
   }
-  uint32_t r0 = 0;
-  KS_TRY(prepare_arrays(ctx, succ, wk, w, (uint32_t)n, rec, ruler_elem, &r0, p, s));
-  SinkPlain sink{root_out, rank_out, keep_roots};
-  if (p.algorithm == KASCADE_ALGO_SPARSE_RULING_SET)
-    return rank_records(ctx, rec, (uint32_t)n, r0, ruler_elem, sink, p, s);
-  ctx.last_levels.clear();
-  ctx.last_levels.push_back(n);
+  ctx.last_levels.assign(1, n);
   return pointer_double_records(ctx, rec, (uint32_t)n, nullptr, sink, s);
 }
 
@@ -239,9 +223,9 @@ KASCADE_API uint64_t kascade_scratch_bytes_root_forest(uint64_t n) {
 
 kascade_status rank_list_host_call(kascade_ctx* c, const uint64_t* succ, const uint32_t* weights, uint64_t n,
                                    uint64_t* root_out, uint64_t* rank_out, const kascade_opts* opts,
-                                   cudaStream_t s, bool dev);
+                                   cudaStream_t s, bool host_check);
 kascade_status root_forest_host_call(kascade_ctx* c, const uint64_t* parent, uint64_t n, uint64_t* root_out,
-                                     uint64_t* depth_out, const kascade_opts* opts, cudaStream_t s, bool dev);
+                                     uint64_t* depth_out, const kascade_opts* opts, cudaStream_t s, bool host_check);
 
 KASCADE_API kascade_status kascade_ctx_sync(kascade_ctx* c, void* stream) {
   if (!c) return KASCADE_ERR_INVALID_ARG;
@@ -249,13 +233,13 @@ KASCADE_API kascade_status kascade_ctx_sync(kascade_ctx* c, void* stream) {
   c->async_pending = false;
   kascade_status st = status_finish(*c, as_stream(stream));
   if (st == KASCADE_ERR_TIMEOUT && c->host_rerun.set) {
-    // an async host-buffer call whose level outgrew the device-driven
-    // recursion: rank it again, on the host-driven path, before returning
+    // an async host-buffer call with a chain past the write-free chase's hop
+    // cap: rank it again, checked on the host, before returning
     const kascade_ctx::HostRerun r = c->host_rerun;
     kascade_opts o = r.opts;
     o.async = 0;
-    st = r.kind == 0 ? rank_list_host_call(c, r.succ, r.weights, r.n, r.root_out, r.rank_out, &o, r.stream, false)
-                     : root_forest_host_call(c, r.succ, r.n, r.root_out, r.rank_out, &o, r.stream, false);
+    st = r.kind == 0 ? rank_list_host_call(c, r.succ, r.weights, r.n, r.root_out, r.rank_out, &o, r.stream, true)
+                     : root_forest_host_call(c, r.succ, r.n, r.root_out, r.rank_out, &o, r.stream, true);
   }
   c->host_rerun.set = false;
   return st;
@@ -294,26 +278,26 @@ KASCADE_API kascade_status kascade_rank_list(kascade_ctx* c, const uint64_t* suc
                                              void* stream) {
   cudaStream_t s = as_stream(stream);
   if (n && (!succ || !root_out || !rank_out)) return KASCADE_ERR_INVALID_ARG;
-  const bool dev = !(opts && opts->async);  // an async call's status is read later: no rerun
+  const bool async = opts && opts->async;  // its status is read later: no rerun
   KS_TRY(begin_call(c, s, opts));
   Params p = make_params(*c, opts, n);
   kascade_status st = validate_list(*c, succ, n, opts, p, s);
   if (st == KASCADE_OK)
     st = rank_list_generic(*c, succ, weights ? WKind::U32 : WKind::Unit, weights, n, root_out, rank_out, 0, p, s,
-                           dev);
+                           async);
   st = end_call(c, s, st, opts);
-  if (st != KASCADE_ERR_TIMEOUT || !dev) return st;
-  // a level outgrew the device-driven recursion: rank again on the host-driven path
+  if (st != KASCADE_ERR_TIMEOUT || async) return st;
+  // a chain past the write-free chase's hop cap: rank again, checked on the host
   KS_TRY(begin_call(c, s, opts));
-  st = rank_list_generic(*c, succ, weights ? WKind::U32 : WKind::Unit, weights, n, root_out, rank_out, 0, p, s);
+  st = rank_list_generic(*c, succ, weights ? WKind::U32 : WKind::Unit, weights, n, root_out, rank_out, 0, p, s, true);
   return end_call(c, s, st, opts);
 }
 
-// The host-buffer list call: copies in, ranks (dev: with the device-driven
-// recursion, no host wait inside the call), copies out.
+// The host-buffer list call: copies in, ranks (no host wait inside the call
+// unless host_check), copies out.
 kascade_status rank_list_host_call(kascade_ctx* c, const uint64_t* succ, const uint32_t* weights, uint64_t n,
                                    uint64_t* root_out, uint64_t* rank_out, const kascade_opts* opts,
-                                   cudaStream_t s, bool dev) {
+                                   cudaStream_t s, bool host_check) {
   KS_TRY(begin_call(c, s, opts));
   Params p = make_params(*c, opts, n);
   kascade_status st = KASCADE_OK;
@@ -329,7 +313,8 @@ kascade_status rank_list_host_call(kascade_ctx* c, const uint64_t* succ, const u
     }
     if (st == KASCADE_OK) st = validate_list(*c, d_succ, n, opts, p, s);
     if (st == KASCADE_OK)
-      st = rank_list_generic(*c, d_succ, d_w ? WKind::U32 : WKind::Unit, d_w, n, d_root, d_rank, 0, p, s, dev);
+      st = rank_list_generic(*c, d_succ, d_w ? WKind::U32 : WKind::Unit, d_w, n, d_root, d_rank, 0, p, s,
+                             host_check);
     if (st == KASCADE_OK) {
       cudaError_t e = cudaMemcpyAsync(root_out, d_root, n * 8, cudaMemcpyDeviceToHost, s);
       if (e == cudaSuccess) e = cudaMemcpyAsync(rank_out, d_rank, n * 8, cudaMemcpyDeviceToHost, s);
@@ -348,7 +333,7 @@ KASCADE_API kascade_status kascade_rank_list_host(kascade_ctx* c, const uint64_t
   if (!c) return KASCADE_ERR_INVALID_ARG;
   if (n && (!succ || !root_out || !rank_out)) return KASCADE_ERR_INVALID_ARG;
   if (n > MAX_LIST) return KASCADE_ERR_TOO_LARGE;
-  kascade_status st = rank_list_host_call(c, succ, weights, n, root_out, rank_out, opts, s, true);
+  kascade_status st = rank_list_host_call(c, succ, weights, n, root_out, rank_out, opts, s, false);
   if (opts && opts->async) {
     if (st == KASCADE_OK) {
       c->host_rerun = kascade_ctx::HostRerun{true, 0, succ, weights, n, root_out, rank_out, *opts, s};
@@ -356,9 +341,9 @@ KASCADE_API kascade_status kascade_rank_list_host(kascade_ctx* c, const uint64_t
     return st;
   }
   if (st != KASCADE_ERR_TIMEOUT) return st;
-  // a level outgrew the device-driven recursion: copy in and rank again on
-  // the host-driven path
-  return rank_list_host_call(c, succ, weights, n, root_out, rank_out, opts, s, false);
+  // a chain past the write-free chase's hop cap: copy in and rank again,
+  // checked on the host
+  return rank_list_host_call(c, succ, weights, n, root_out, rank_out, opts, s, true);
 }
 
 KASCADE_API kascade_status kascade_sparse_ruling_set(kascade_ctx* c, const kascade_opts* opts, uint64_t* succ_array,
@@ -375,7 +360,8 @@ KASCADE_API kascade_status kascade_sparse_ruling_set(kascade_ctx* c, const kasca
     if (st == KASCADE_OK && !ok) st = KASCADE_ERR_NOT_A_LIST;
   }
   if (st == KASCADE_OK)
-    st = rank_list_generic(*c, succ_array, WKind::I64, rank_array, n, succ_array, (uint64_t*)rank_array, 1, p, s);
+    st = rank_list_generic(*c, succ_array, WKind::I64, rank_array, n, succ_array, (uint64_t*)rank_array, 1, p, s,
+                           true);
   return end_call(c, s, st, opts);
 }
 
@@ -387,7 +373,7 @@ KASCADE_API kascade_status kascade_pointer_doubling(kascade_ctx* c, const kascad
   Params p = make_params(*c, opts, n);
   p.algorithm = KASCADE_ALGO_POINTER_DOUBLING;
   kascade_status st =
-      rank_list_generic(*c, succ_array, WKind::I64, rank_array, n, succ_array, (uint64_t*)rank_array, 1, p, s);
+      rank_list_generic(*c, succ_array, WKind::I64, rank_array, n, succ_array, (uint64_t*)rank_array, 1, p, s, true);
   return end_call(c, s, st, opts);
 }
 
@@ -438,23 +424,24 @@ KASCADE_API kascade_status kascade_root_forest(kascade_ctx* c, const uint64_t* p
   cudaStream_t s = as_stream(stream);
   if (n && (!parent || !root_out || !depth_out)) return KASCADE_ERR_INVALID_ARG;
   if (n > MAX_FOREST) return KASCADE_ERR_TOO_LARGE;
-  const bool dev = !(opts && opts->async);
+  const bool async = opts && opts->async;
   KS_TRY(begin_call(c, s, opts));
   Params p = make_params(*c, opts, 2 * n);
   p.algorithm = KASCADE_ALGO_SPARSE_RULING_SET;
-  kascade_status st = root_forest_impl(*c, parent, (uint32_t)n, root_out, depth_out, 0, p, s, dev);
+  kascade_status st = root_forest_impl(*c, parent, (uint32_t)n, root_out, depth_out, 0, p, s, async);
   st = end_call(c, s, st, opts);
-  if (st != KASCADE_ERR_TIMEOUT || !dev) return st;
-  // a tour level outgrew the device-driven recursion: again on the host-driven path
+  if (st != KASCADE_ERR_TIMEOUT || async) return st;
+  // a chain past the write-free chase's hop cap: again, checked on the host
   KS_TRY(begin_call(c, s, opts));
-  st = root_forest_impl(*c, parent, (uint32_t)n, root_out, depth_out, 0, p, s);
+  st = root_forest_impl(*c, parent, (uint32_t)n, root_out, depth_out, 0, p, s, true);
   return end_call(c, s, st, opts);
 }
 
-// The host-buffer forest call: copies in, roots (dev: with the device-driven
-// recursion, no host wait inside the call), copies out.
+// The host-buffer forest call: copies in, roots (no host wait inside the call
+// unless host_check), copies out.
 kascade_status root_forest_host_call(kascade_ctx* c, const uint64_t* parent, uint64_t n, uint64_t* root_out,
-                                     uint64_t* depth_out, const kascade_opts* opts, cudaStream_t s, bool dev) {
+                                     uint64_t* depth_out, const kascade_opts* opts, cudaStream_t s,
+                                     bool host_check) {
   KS_TRY(begin_call(c, s, opts));
   Params p = make_params(*c, opts, 2 * n);
   p.algorithm = KASCADE_ALGO_SPARSE_RULING_SET;
@@ -467,7 +454,7 @@ kascade_status root_forest_host_call(kascade_ctx* c, const uint64_t* parent, uin
       d_depth = alloc<uint64_t>(*c, n);
       if (!d_root || !d_depth) st = KASCADE_ERR_OOM;
     }
-    if (st == KASCADE_OK) st = root_forest_impl(*c, d_par, (uint32_t)n, d_root, d_depth, 0, p, s, dev);
+    if (st == KASCADE_OK) st = root_forest_impl(*c, d_par, (uint32_t)n, d_root, d_depth, 0, p, s, host_check);
     if (st == KASCADE_OK) {
       cudaError_t e = cudaMemcpyAsync(root_out, d_root, n * 8, cudaMemcpyDeviceToHost, s);
       if (e == cudaSuccess) e = cudaMemcpyAsync(depth_out, d_depth, n * 8, cudaMemcpyDeviceToHost, s);
@@ -486,16 +473,16 @@ KASCADE_API kascade_status kascade_root_forest_host(kascade_ctx* c, const uint64
   if (!c) return KASCADE_ERR_INVALID_ARG;
   if (n && (!parent || !root_out || !depth_out)) return KASCADE_ERR_INVALID_ARG;
   if (n > MAX_FOREST) return KASCADE_ERR_TOO_LARGE;
-  kascade_status st = root_forest_host_call(c, parent, n, root_out, depth_out, opts, s, true);
+  kascade_status st = root_forest_host_call(c, parent, n, root_out, depth_out, opts, s, false);
   if (opts && opts->async) {
     if (st == KASCADE_OK)
       c->host_rerun = kascade_ctx::HostRerun{true, 1, parent, nullptr, n, root_out, depth_out, *opts, s};
     return st;
   }
   if (st != KASCADE_ERR_TIMEOUT) return st;
-  // a tour level outgrew the device-driven recursion: copy in and root again
-  // on the host-driven path
-  return root_forest_host_call(c, parent, n, root_out, depth_out, opts, s, false);
+  // a chain past the write-free chase's hop cap: copy in and root again,
+  // checked on the host
+  return root_forest_host_call(c, parent, n, root_out, depth_out, opts, s, true);
 }
 
 KASCADE_API kascade_status kascade_rank_via_euler_tour(kascade_ctx* c, const kascade_opts* opts, uint64_t* succ_array,
@@ -515,7 +502,7 @@ KASCADE_API kascade_status kascade_rank_via_euler_tour(kascade_ctx* c, const kas
     if (st == KASCADE_OK)
       st = cuda_status(cudaMemcpyAsync(parent_copy, succ_array, n * 8, cudaMemcpyDeviceToDevice, s));
     if (st == KASCADE_OK)
-      st = root_forest_impl(*c, parent_copy, (uint32_t)n, succ_array, (uint64_t*)rank_array, 1, p, s);
+      st = root_forest_impl(*c, parent_copy, (uint32_t)n, succ_array, (uint64_t*)rank_array, 1, p, s, true);
   }
   return end_call(c, s, st, opts);
 }
@@ -557,17 +544,15 @@ KASCADE_API kascade_status kascade_rank_batch(kascade_ctx* c, const kascade_segm
                                               void* stream) {
   cudaStream_t s = as_stream(stream);
   if (total_n && (!segs || !num_segs || !input || !root_out || !rank_out)) return KASCADE_ERR_INVALID_ARG;
-  // The device-driven recursion (no host waits) first; a batch it cannot hold
-  // (a level outgrowing its capacity, e.g. very many roots) reports
-  // KASCADE_ERR_TIMEOUT and is ranked again on the host-driven path.  Async
-  // calls take the host-driven path directly (their status is read later).
+  // Async calls have their status read later and cannot be rerun.
   const bool async = opts && opts->async;
   KS_TRY(begin_call(c, s, opts));
-  kascade_status st = rank_batch_impl(*c, segs, num_segs, input, weights, total_n, root_out, rank_out, opts, s, !async);
+  kascade_status st = rank_batch_impl(*c, segs, num_segs, input, weights, total_n, root_out, rank_out, opts, s, async);
   st = end_call(c, s, st, opts);
   if (st != KASCADE_ERR_TIMEOUT || async) return st;
+  // a chain past the write-free chase's hop cap: again, checked on the host
   KS_TRY(begin_call(c, s, opts));
-  st = rank_batch_impl(*c, segs, num_segs, input, weights, total_n, root_out, rank_out, opts, s, false);
+  st = rank_batch_impl(*c, segs, num_segs, input, weights, total_n, root_out, rank_out, opts, s, true);
   return end_call(c, s, st, opts);
 }
 
@@ -577,7 +562,7 @@ kascade_status rank_batch_device_call(kascade_ctx* c, const kascade_segment* seg
                                       const uint32_t* weights, uint64_t total, uint64_t* root_out,
                                       uint64_t* rank_out, const kascade_opts* opts, cudaStream_t s) {
   KS_TRY(begin_call(c, s, opts));
-  const kascade_status st = rank_batch_impl(*c, segs, nseg, in, weights, total, root_out, rank_out, opts, s, true);
+  const kascade_status st = rank_batch_impl(*c, segs, nseg, in, weights, total, root_out, rank_out, opts, s, false);
   return end_call(c, s, st, opts);
 }
 kascade_status batch_plan_create(int device, const kascade_segment* segs, uint32_t nseg, const uint64_t* in,

@@ -23,9 +23,8 @@
 //   heads     elements ahead of their list's first ruler were never visited:
 //             the place step finds them (no entry in their slot), presets
 //             their root output to a NOT_REACHED sentinel and lists them;
-//             each walks forward to the first element with outputs (tours
-//             make their heads rulers and report an unreached element as a
-//             ruler-free cycle)
+//             each walks forward to the first element with outputs; a list
+//             end that is no ruler itself is one of them
 //
 // Calls that must leave roots' outputs untouched (the in-place contract) use
 // the stamping level 0 instead: the sentinel presets would overwrite them.
@@ -102,26 +101,25 @@ __device__ __forceinline__ void log_append(bool emit, uint32_t x, uint32_t id, u
   }
 }
 
+// The read-only chase: rulers and their order as in k_chase.  Every ruler and
+// every element a chain passes is logged; a list's end is not (any number of
+// chains may end there).
 template <int C>
-__global__ void __launch_bounds__(512) k_chase_log(const Rec* __restrict__ rec, uint32_t n,
-                                                   const uint32_t* __restrict__ ruler_elem, uint32_t r,
-                                                   const uint32_t* __restrict__ r_dev,
-                                                   Rec* __restrict__ rec_next, uint32_t* __restrict__ work,
-                                                   LogEnt* __restrict__ log, uint32_t* __restrict__ chunk_fill,
+__global__ void __launch_bounds__(512) k_chase_log(const Rec* __restrict__ rec, Extent ext, Rulers rl,
+                                                   uint32_t rulers, Heads heads, Rec* __restrict__ rec_next, uint32_t* __restrict__ rootel_next,
+                                                   uint32_t* __restrict__ work, LogEnt* __restrict__ log,
+                                                   uint32_t* __restrict__ chunk_fill,
                                                    uint32_t* __restrict__ chunk_cursor, uint32_t nchunks,
-                                                   uint32_t max_hops, uint32_t* __restrict__ has_pred,
-                                                   DevStatus* st) {
+                                                   uint32_t max_hops, DevStatus* st) {
   constexpr uint32_t BATCH = 32u * C;
-  // has_pred holds one bit per ruler of the capacity; a count past the
-  // capacity (reported by the caller's count check, and the level redone)
-  // leaves tags beyond it, whose bits are not recorded
-  const uint32_t pred_cap = r;
-  if (r_dev) r = min(r, *r_dev);  // the ruler count on the device, r its capacity
+  const uint32_t n = ext.get();
+  const uint32_t r = rulers + heads.get();
+  if (ext.add && blockIdx.x == 0 && threadIdx.x == 0) st->counter[1] = n;  // level 0's size, reported by the call
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t lt = lanemask_lt();
   uint32_t cid[C], cx[C], hops[C];
   uint64_t acc[C];
-  uint32_t act = 0;
+  uint32_t act = 0, fresh = 0;  // bit c: chain c runs / has not read its ruler's record yet
   uint32_t q_base = 0, q_left = 0;
   bool drained = false;
   uint32_t lpos = 0, lend = 0;  // warp-uniform log chunk
@@ -130,11 +128,19 @@ __global__ void __launch_bounds__(512) k_chase_log(const Rec* __restrict__ rec, 
     cid[c] = cx[c] = hops[c] = 0;
     acc[c] = 0;
   }
+  auto end_chain = [&](uint32_t id, uint64_t dist, uint32_t next, uint32_t root) {
+    Rec o;
+    o.a = dist;
+    o.b = next;
+    o.c = TAG_UNREACHED;
+    st_rec_cg(rec_next + id, o);
+    rootel_next[id] = root;
+  };
   while (true) {
     if (!drained) {
 #pragma unroll
       for (int c = 0; c < C; ++c) {
-        bool need = !(act & (1u << c));
+        bool need = !((act >> c) & 1u);
         uint32_t m = __ballot_sync(FULL, need);
         while (m != 0u && !drained) {
           if (q_left == 0u) {
@@ -151,29 +157,24 @@ __global__ void __launch_bounds__(512) k_chase_log(const Rec* __restrict__ rec, 
           const uint32_t take = min((uint32_t)__popc(m), q_left);
           const uint32_t my_rank = __popc(m & lt);
           const bool mine = need && my_rank < take;
-          uint32_t x0 = 0, id = 0;
           if (mine) {
-            id = q_base + my_rank;
-            x0 = __ldg(ruler_elem + id);
-            const Rec r0 = ld_rec_cg(rec + x0);
-            if (r0.b == x0) {
-              Rec o;
-              o.a = 0;
-              o.b = id;
-              o.c = TAG_UNREACHED;
-              st_rec_cg(rec_next + id, o);
+            const uint32_t id = q_base + my_rank;
+            const uint64_t x0 = id < rulers ? rl.elem(id) : __ldg(heads.elem + (id - rulers));
+            uint32_t j;
+            if (x0 >= n) {
+              end_chain(id, 0, id, 0);  // the last block's ruler, beyond the elements
+            } else if (id >= rulers && rl.is((uint32_t)x0, &j)) {
+              end_chain(id, 0, j, 0);  // a head that is a ruler itself
             } else {
               cid[c] = id;
-              cx[c] = r0.b;
-              acc[c] = r0.a;
+              cx[c] = (uint32_t)x0;
+              acc[c] = 0;
               hops[c] = 0;
               act |= 1u << c;
+              fresh |= 1u << c;
             }
           }
-          // every ruler (root rulers included) logs itself at distance 0
-          log_append(mine, x0, id, 0ull, lpos, lend, log, chunk_fill, chunk_cursor, nchunks, lane, lt, st);
-          const uint32_t served = __ballot_sync(FULL, mine);
-          m &= ~served;
+          m &= ~__ballot_sync(FULL, mine);
           need = need && !mine;
           q_base += take;
           q_left -= take;
@@ -187,41 +188,37 @@ __global__ void __launch_bounds__(512) k_chase_log(const Rec* __restrict__ rec, 
     Rec rr[C];
 #pragma unroll
     for (int c = 0; c < C; ++c)
-      if (act & (1u << c)) rr[c] = ld_rec_cg(rec + cx[c]);
+      if ((act >> c) & 1u) rr[c] = ld_rec_cg(rec + cx[c]);
 #pragma unroll
     for (int c = 0; c < C; ++c) {
       bool emit = false;
       const uint32_t x = cx[c];
       const uint64_t d = acc[c];
-      if (act & (1u << c)) {
-        if (tag_ruler(rr[c].c)) {
-          // back at its own ruler: a rootless cycle holding one ruler
-          if (tag_id(rr[c].c) == cid[c])
-            set_error(st, KASCADE_ERR_CYCLE, cid[c]);
-          else if (has_pred && tag_id(rr[c].c) < pred_cap)  // that ruler has a predecessor in the ruler sub-list
-            atomicOr(has_pred + (tag_id(rr[c].c) >> 5), 1u << (tag_id(rr[c].c) & 31));
-          Rec o;
-          o.a = acc[c];
-          o.b = tag_id(rr[c].c);
-          o.c = TAG_UNREACHED;
-          st_rec_cg(rec_next + cid[c], o);
+      if ((act >> c) & 1u) {
+        const uint32_t y = rr[c].b;
+        const bool first = (fresh >> c) & 1u;
+        fresh &= ~(1u << c);
+        emit = first || y != x;
+        if (y == x) {  // the list's end
+          end_chain(cid[c], d + rr[c].a, cid[c], x);
           act &= ~(1u << c);
         } else {
-          emit = true;
-          acc[c] += rr[c].a;
-          cx[c] = rr[c].b;
-          // Ruler gaps are geometric: a chain longer than max_hops (64x the
-          // mean spacing, probability ~e^-64) is treated as a sign of an
-          // invalid input (a ruler-free cycle behind a ruler); the chain
-          // stops and the host reruns level 0 on the stamping path, which
-          // tells the two cases apart exactly.
-          if (++hops[c] > max_hops) {
+          acc[c] = d + rr[c].a;
+          cx[c] = y;
+          uint32_t j;
+          if (rl.is(y, &j)) {
+            // back at its own ruler: a rootless cycle holding one ruler
+            if (j == cid[c]) set_error(st, KASCADE_ERR_CYCLE, j);
+            end_chain(cid[c], acc[c], j, 0);
+            act &= ~(1u << c);
+          } else if (++hops[c] > max_hops) {
+            // Ruler gaps are geometric: a chain longer than max_hops (64x the
+            // mean spacing, probability ~e^-64) is treated as a sign of an
+            // invalid input (a ruler-free cycle behind a ruler); the chain
+            // stops and the host reruns level 0 on the stamping path, which
+            // tells the two cases apart exactly.
             atomicOr(&st->counter[0], 1ull);
-            Rec o;  // keep the next level's records in range (the level is redone anyway)
-            o.a = 0;
-            o.b = cid[c];
-            o.c = TAG_UNREACHED;
-            st_rec_cg(rec_next + cid[c], o);
+            end_chain(cid[c], 0, cid[c], 0);  // keeps the next level's records in range
             act &= ~(1u << c);
           }
         }
@@ -276,7 +273,7 @@ __device__ uint32_t block_exclusive_scan(uint32_t* v, uint32_t m) {
 //     root(ruler), from the rulers' results of the recursion.  A log chunk
 //     holds the entries of a few hundred chains, so most of these lookups
 //     hit L1.  Entries of elements at or above `limit` (tour down edges: no
-//     output) are only counted, in `beyond`
+//     output) are dropped
 //   otherwise (second pass): tiles inside one window's region, buckets are
 //     its SUBS sub-windows
 // More entries than a bucket holds means some element was logged twice.
@@ -288,7 +285,6 @@ __global__ void __launch_bounds__(PT_THREADS, BLOCKS) k_partition(const LogEnt* 
                                                              const Out* __restrict__ out1, uint32_t limit,
                                                              uint32_t nb, LogEnt* __restrict__ dst,
                                                              uint32_t* __restrict__ dcursor,
-                                                             uint32_t* __restrict__ beyond,
                                                              const uint32_t* __restrict__ used, DevStatus* st) {
   constexpr uint32_t PT_TILE = PT_THREADS * ITEMS;
   constexpr uint32_t PT_TILE_CHUNKS = PT_TILE / LOG_CHUNK;
@@ -299,7 +295,6 @@ __global__ void __launch_bounds__(PT_THREADS, BLOCKS) k_partition(const LogEnt* 
   uint32_t* cnt = reinterpret_cast<uint32_t*>(stage + PT_TILE);  // counts, then the tile's offsets
   uint32_t* gbase = cnt + nbk;                                   // the tile's start in each bucket
   __shared__ uint32_t fills[PT_TILE_CHUNKS];
-  __shared__ uint32_t nbeyond;
   if (FROM_LOG && used) nchunks = min(nchunks, __ldcg(used));
   const uint32_t ntiles =
       FROM_LOG ? (nchunks + PT_TILE_CHUNKS - 1) / PT_TILE_CHUNKS : nb * (WIN / PT_TILE);
@@ -322,11 +317,9 @@ __global__ void __launch_bounds__(PT_THREADS, BLOCKS) k_partition(const LogEnt* 
       const uint32_t c = t * PT_TILE_CHUNKS + threadIdx.x;
       fills[threadIdx.x] = c >= nchunks ? 0u : src_info ? __ldcg(src_info + c) : min(LOG_CHUNK, limit - c * LOG_CHUNK);
     }
-    if (threadIdx.x == 0) nbeyond = 0;
     __syncthreads();
     uint4 v[ITEMS];
     uint32_t pos[ITEMS];
-    uint32_t mine_beyond = 0;
 #pragma unroll
     for (uint32_t k = 0; k < ITEMS; ++k) {
       const uint32_t e = k * PT_THREADS + threadIdx.x;
@@ -350,11 +343,8 @@ __global__ void __launch_bounds__(PT_THREADS, BLOCKS) k_partition(const LogEnt* 
       if (x < limit) {
         const uint32_t b = FROM_LOG ? x >> WIN_SHIFT : (x >> SUB_SHIFT) & (SUBS - 1);
         pos[k] = atomicAdd(&cnt[b], 1u);
-      } else if (FROM_LOG && x != NO_ROOT) {
-        ++mine_beyond;
       }
     }
-    if (FROM_LOG && mine_beyond) atomicAdd(&nbeyond, mine_beyond);
     __syncthreads();
     // one cursor step per bucket the tile touches.  In the second pass (one
     // bucket per thread) the step's result stays in a register until the
@@ -371,7 +361,6 @@ __global__ void __launch_bounds__(PT_THREADS, BLOCKS) k_partition(const LogEnt* 
       else
         gbase[b] = g;
     }
-    if (FROM_LOG && threadIdx.x == 0 && nbeyond) atomicAdd(beyond, nbeyond);
     const uint32_t total = block_exclusive_scan(cnt, nbk);  // cnt now holds the tile's offsets
 #pragma unroll
     for (uint32_t k = 0; k < ITEMS; ++k) {
@@ -402,31 +391,22 @@ __global__ void __launch_bounds__(PT_THREADS, BLOCKS) k_partition(const LogEnt* 
 // (element, root, rank) are read in order and placed in shared memory by
 // element, then the sub-window's outputs are written densely.  Elements
 // without an entry were reached by no chain: their root output becomes
-// NOT_REACHED and they join the unreached list (or, when every list head is
-// a ruler, they lie on a ruler-free cycle).  A batch's roots are written
+// NOT_REACHED and they join the unreached list.  A batch's roots are written
 // relative to their instance.
 __global__ void __launch_bounds__(FIN_THREADS, 2) k_place(const LogEnt* __restrict__ part2,
                                                             const uint32_t* __restrict__ cursor2, uint32_t nb,
-                                                            uint32_t limit, uint32_t n,
-                                                            const uint32_t* __restrict__ beyond, int heads_are_rulers,
-                                                            uint64_t* __restrict__ root_out,
+                                                            uint32_t limit, uint64_t* __restrict__ root_out,
                                                             uint64_t* __restrict__ rank_out,
                                                             uint32_t* __restrict__ ulist,
                                                             uint32_t* __restrict__ ucount, uint32_t ucap,
                                                             const uint64_t* __restrict__ seg_off,
                                                             const uint32_t* __restrict__ hint, uint32_t nseg,
-                                                            const uint32_t* __restrict__ plus_one,
-                                                            const uint32_t* __restrict__ beyond_want, DevStatus* st) {
+                                                            const uint32_t* __restrict__ plus_one, DevStatus* st) {
   extern __shared__ __align__(16) unsigned char smraw[];
   unsigned long long* rank_s = reinterpret_cast<unsigned long long*>(smraw);  // SUB entries
   uint32_t* root_s = reinterpret_cast<uint32_t*>(rank_s + SUB);               // SUB entries
   __shared__ uint32_t plus_s[SUB / 32];                                       // the sub-window's plus_one words
   const uint32_t lane = threadIdx.x & 31u;
-  if (blockIdx.x == 0 && threadIdx.x == 0 && heads_are_rulers) {
-    const uint32_t want = beyond_want ? *beyond_want : n - limit;
-    if (*beyond > want) set_error(st, KASCADE_ERR_NOT_A_LIST, *beyond);
-    if (*beyond < want) set_error(st, KASCADE_ERR_CYCLE, *beyond);
-  }
   const uint32_t items = nb * SUBS;
   for (uint32_t it = blockIdx.x; it < items; it += gridDim.x) {
     const uint32_t lo = it * SUB;  // == window * WIN + sub-window * SUB
@@ -491,10 +471,6 @@ __global__ void __launch_bounds__(FIN_THREADS, 2) k_place(const LogEnt* __restri
       }
       const uint32_t m = __ballot_sync(FULL, un);
       if (m == 0u) continue;
-      if (heads_are_rulers) {
-        if (un) set_error(st, KASCADE_ERR_CYCLE, lo + i);
-        continue;
-      }
       uint32_t base = 0;
       if (lane == 0) base = atomicAdd(ucount, (uint32_t)__popc(m));
       base = __shfl_sync(FULL, base, 0);
@@ -510,18 +486,23 @@ __global__ void __launch_bounds__(FIN_THREADS, 2) k_place(const LogEnt* __restri
   }
 }
 
-// Each unreached element walks forward to the first element with outputs:
-// one the place step wrote (root output not NOT_REACHED) or one another
-// walker finished.  Walkers write the rank, fence, then the root, and readers
-// load the root, fence, then the rank, so a root seen set comes with its
-// rank.  Elements at or above `limit` (a batch's tour down edges) have no
-// outputs and are walked through.  Roots already relative to their instance
-// stay so: a walker and the element it stops at share an instance.
+// Each unreached element walks forward to its list's end or to the first
+// element with outputs: one the place step wrote (root output not
+// NOT_REACHED) or one another walker finished.  Walkers write the rank,
+// fence, then the root, and readers load the root, fence, then the rank, so a
+// root seen set comes with its rank.  Elements at or above `limit` (tour down
+// edges) have no outputs and are walked through.  Roots already relative to
+// their instance stay so (a walker and the element it stops at share an
+// instance); a list end's root is made relative here.  plus_one: outputs that
+// are one more than their rank.
 __global__ void __launch_bounds__(256) k_walk_unreached(const Rec* __restrict__ rec, const uint32_t* __restrict__ ulist,
                                                         const uint32_t* __restrict__ ucount, uint32_t ucap, uint32_t n,
                                                         uint32_t limit, uint64_t* root_out, uint64_t* rank_out,
-                                                        DevStatus* st) {
+                                                        const uint64_t* __restrict__ seg_off,
+                                                        const uint32_t* __restrict__ hint, uint32_t nseg,
+                                                        const uint32_t* __restrict__ plus_one, DevStatus* st) {
   const uint32_t cnt = min(*ucount, ucap);
+  auto extra = [&](uint32_t x) -> uint64_t { return plus_one ? (__ldg(plus_one + (x >> 5)) >> (x & 31)) & 1u : 0u; };
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
     const uint32_t u = ulist[i];
     uint64_t acc = 0;
@@ -531,6 +512,16 @@ __global__ void __launch_bounds__(256) k_walk_unreached(const Rec* __restrict__ 
     while (true) {
       const Rec r = ld_rec_cg(rec + y);
       acc += r.a;
+      if (r.b == y) {  // the list's end
+        uint64_t off = 0;
+        if (seg_off) {
+          uint32_t j = __ldg(hint + (y >> 12));
+          while (j + 1 < nseg && __ldg(seg_off + j + 1) <= y) ++j;
+          off = __ldg(seg_off + j);
+        }
+        base_root = y - off;
+        break;
+      }
       y = r.b;
       if (y >= n) {  // not reachable for a validated input; keeps every load in range
         set_error(st, KASCADE_ERR_OUT_OF_RANGE, u);
@@ -539,7 +530,11 @@ __global__ void __launch_bounds__(256) k_walk_unreached(const Rec* __restrict__ 
       }
       if (y < limit) {
         base_root = __ldcg(reinterpret_cast<const unsigned long long*>(root_out) + y);
-        if (base_root != NOT_REACHED) break;
+        if (base_root != NOT_REACHED) {
+          __threadfence();
+          acc += __ldcg(reinterpret_cast<const unsigned long long*>(rank_out) + y) - extra(y);
+          break;
+        }
       }
       if (y == mark || ++hops > n) {
         set_error(st, KASCADE_ERR_CYCLE, u);
@@ -553,9 +548,7 @@ __global__ void __launch_bounds__(256) k_walk_unreached(const Rec* __restrict__ 
       }
     }
     if (!ok) continue;
-    __threadfence();
-    const unsigned long long base_rank = __ldcg(reinterpret_cast<const unsigned long long*>(rank_out) + y);
-    rank_out[u] = acc + base_rank;
+    rank_out[u] = acc + extra(u);
     __threadfence();
     root_out[u] = base_root;
   }
@@ -592,18 +585,6 @@ kascade_status raise_smem_limits() {
 int g_chase_occ[5][3] = {{-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1}};
 
 template <int C>
-kascade_status launch_chase_log_c(kascade_ctx& ctx, const Rec* rec, uint32_t n, const uint32_t* ruler_elem, uint32_t r,
-                                  const uint32_t* r_dev, Rec* rec_next, uint32_t* work, LogEnt* log,
-                                  uint32_t* chunk_fill, uint32_t* chunk_cursor, uint32_t nchunks, uint32_t max_hops,
-                                  uint32_t* has_pred, unsigned grid, uint32_t block, cudaStream_t s) {
-  ProfScope ps(ctx, "chase", s);
-  k_chase_log<C><<<grid, block, 0, s>>>(rec, n, ruler_elem, r, r_dev, rec_next, work, log, chunk_fill, chunk_cursor,
-                                      nchunks, max_hops, has_pred, ctx.d_status);
-  KS_CHECK_LAUNCH();
-  return KASCADE_OK;
-}
-
-template <int C>
 unsigned chase_grid(const kascade_ctx& ctx, uint32_t r, uint32_t block) {
   const int bi = block == 128 ? 0 : block == 512 ? 2 : 1;
   if (g_chase_occ[C][bi] < 0) {
@@ -624,99 +605,86 @@ unsigned chase_grid(const kascade_ctx& ctx, uint32_t r, uint32_t block) {
 
 }  // namespace
 
-kascade_status rank_level0_log(kascade_ctx& ctx, const Rec* rec, uint32_t n, uint32_t r0, const uint32_t* ruler_elem0,
-                               const LogTarget& t, const Params& p, cudaStream_t s, const uint32_t* r0_dev) {
-  if (r0_dev) ctx.last_levels.assign(1, n);  // the deeper sizes come back with the status
+kascade_status rank_level0_log(kascade_ctx& ctx, const Rec* rec, uint32_t n, const Extent& ext, const Heads& heads,
+                               const LogTarget& t, const Params& p, cudaStream_t s, bool host_check) {
+  Levels lv;
+  KS_TRY(plan_levels(ctx, n, heads, p, &lv));
+  const uint32_t r = lv.n[1];
   const int C = (p.chains == 1 || p.chains == 4) ? (int)p.chains : 2;
   const uint32_t block = p.block;
-  const unsigned grid = C == 1   ? chase_grid<1>(ctx, r0, block)
-                        : C == 4 ? chase_grid<4>(ctx, r0, block)
-                                 : chase_grid<2>(ctx, r0, block);
+  const unsigned grid = C == 1   ? chase_grid<1>(ctx, r, block)
+                        : C == 4 ? chase_grid<4>(ctx, r, block)
+                                 : chase_grid<2>(ctx, r, block);
   const uint64_t warps = (uint64_t)grid * (block / 32);
   const uint32_t nchunks = (uint32_t)(((uint64_t)n + LOG_CHUNK - 1) / LOG_CHUNK + warps + 1);
+  const uint32_t limit = t.limit < n ? t.limit : n;
+  const uint32_t nb = (uint32_t)(((uint64_t)limit + WIN - 1) / WIN);
+  const uint32_t nb1 = nb ? nb : 1;
+  const uint64_t cursor_words = (uint64_t)nb1 * (SUBS + 1) * CURSOR_STRIDE;
   LogEnt* log = alloc<LogEnt>(ctx, (uint64_t)nchunks * LOG_CHUNK);
-  uint32_t* chunk_fill = alloc<uint32_t>(ctx, nchunks);
-  uint32_t* counters = alloc<uint32_t>(ctx, 8);  // chunk cursor, chase work, unreached count, beyond
-  Rec* rec1 = alloc<Rec>(ctx, r0);
-  Out* out1 = alloc<Out>(ctx, r0);
-  uint32_t* lv = r0_dev ? alloc<uint32_t>(ctx, MAX_DEV_LEVELS + 2) : nullptr;  // level sizes (device)
-  // device-driven levels: the rulers a chain ended at (level-1 list heads are the others)
-  const uint64_t pwords = ((uint64_t)r0 + 31) / 32;
-  uint32_t* pred1 = r0_dev ? alloc<uint32_t>(ctx, pwords) : nullptr;
-  if (!log || !chunk_fill || !counters || !rec1 || !out1 || (r0_dev && (!lv || !pred1))) return KASCADE_ERR_OOM;
-  KS_CUDA(cudaMemsetAsync(chunk_fill, 0, sizeof(uint32_t) * nchunks, s));
-  KS_CUDA(cudaMemsetAsync(counters, 0, sizeof(uint32_t) * 8, s));
-  if (r0_dev) {
-    KS_CUDA(cudaMemsetAsync(lv, 0, sizeof(uint32_t) * (MAX_DEV_LEVELS + 2), s));
-    KS_CUDA(cudaMemsetAsync(pred1, 0, sizeof(uint32_t) * pwords, s));
-    // a tour sized for a bound: its length is the output slots plus the down edges
-    if (t.beyond_want) KS_TRY(launch_set_level0(ctx, lv, t.limit, t.beyond_want, s));
-    KS_TRY(launch_check_count(ctx, r0_dev, r0, lv + 1, s));
-  }
-  const uint32_t* r_dev = r0_dev ? lv + 1 : nullptr;
-  uint32_t* chunk_cursor = counters + 0;
-  uint32_t* chase_work = counters + 1;
-  uint32_t* ucount = counters + 2;
-  uint32_t* beyond = counters + 3;
+  // zeroed by one memset: chunk cursor, unreached count; the partition
+  // cursors; the chunks' fill counts
+  const uint64_t zero_words = 8 + cursor_words + nchunks;
+  uint32_t* zero = alloc<uint32_t>(ctx, zero_words);
+  if (!log || !zero) return KASCADE_ERR_OOM;
+  KS_CUDA(cudaMemsetAsync(zero, 0, sizeof(uint32_t) * zero_words, s));
+  uint32_t* chunk_cursor = zero + 0;
+  uint32_t* ucount = zero + 1;
+  uint32_t* cursor1 = zero + 8;
+  uint32_t* cursor2 = cursor1 + (uint64_t)nb1 * CURSOR_STRIDE;
+  uint32_t* chunk_fill = cursor1 + cursor_words;
   const uint64_t cap = p.max_chain ? p.max_chain : 64ull * p.spacing0 + 1024;
   const uint32_t max_hops = cap < n ? (uint32_t)cap : n;
-  switch (C) {
-    case 1:
-      KS_TRY(launch_chase_log_c<1>(ctx, rec, n, ruler_elem0, r0, r_dev, rec1, chase_work, log, chunk_fill,
-                                   chunk_cursor, nchunks, max_hops, pred1, grid, block, s));
-      break;
-    case 4:
-      KS_TRY(launch_chase_log_c<4>(ctx, rec, n, ruler_elem0, r0, r_dev, rec1, chase_work, log, chunk_fill,
-                                   chunk_cursor, nchunks, max_hops, pred1, grid, block, s));
-      break;
-    default:
-      KS_TRY(launch_chase_log_c<2>(ctx, rec, n, ruler_elem0, r0, r_dev, rec1, chase_work, log, chunk_fill,
-                                   chunk_cursor, nchunks, max_hops, pred1, grid, block, s));
-  }
-  // level-1 elements are level-0 rulers: their level-0 index is ruler_elem0
-  int levels = 0;
-  if (r0_dev) {
-    k_hop_cap_status<<<1, 1, 0, s>>>(ctx.d_status);
+  {
+    ProfScope ps(ctx, "chase", s);
+    uint32_t* work = &ctx.d_status->work[0];
+    switch (C) {
+      case 1:
+        k_chase_log<1><<<grid, block, 0, s>>>(rec, ext, lv.rulers[0], lv.r[0], lv.heads, lv.rec[1], lv.rootel[1], work,
+                                              log, chunk_fill, chunk_cursor, nchunks, max_hops, ctx.d_status);
+        break;
+      case 4:
+        k_chase_log<4><<<grid, block, 0, s>>>(rec, ext, lv.rulers[0], lv.r[0], lv.heads, lv.rec[1], lv.rootel[1], work,
+                                              log, chunk_fill, chunk_cursor, nchunks, max_hops, ctx.d_status);
+        break;
+      default:
+        k_chase_log<2><<<grid, block, 0, s>>>(rec, ext, lv.rulers[0], lv.r[0], lv.heads, lv.rec[1], lv.rootel[1], work,
+                                              log, chunk_fill, chunk_cursor, nchunks, max_hops, ctx.d_status);
+    }
     KS_CHECK_LAUNCH();
-    KS_TRY(rank_deep_dev(ctx, rec1, out1, r0, lv, ruler_elem0, pred1, p, s, &levels));
-  } else {
+  }
+  if (host_check) {
     // a chain hit the hop cap: let the caller rerun level 0 on the stamping path
     uint32_t over = 0;
     KS_TRY(read_u32(ctx, reinterpret_cast<const uint32_t*>(&ctx.d_status->counter[0]), &over, s));
     if (over) return KASCADE_ERR_TIMEOUT;
-    KS_TRY(rank_sublist(ctx, rec1, r0, ruler_elem0, out1, 1, p, s));
+  } else {
+    k_hop_cap_status<<<1, 1, 0, s>>>(ctx.d_status);
+    KS_CHECK_LAUNCH();
   }
+  KS_TRY(rank_deep(ctx, lv, p, s));
 
-  const uint32_t limit = t.limit < n ? t.limit : n;
-  const uint32_t nb = (uint32_t)(((uint64_t)limit + WIN - 1) / WIN);
-  const uint32_t nb1 = nb ? nb : 1;
   // first pass: log -> windows (part); second pass: windows -> sub-windows,
   // into the log's memory when it is large enough (the log is dead by then)
   const uint64_t part2_need = (((uint64_t)limit + SUB - 1) / SUB) * SUB;
   LogEnt* part = alloc<LogEnt>(ctx, (uint64_t)nb1 * WIN);
   LogEnt* part2 = (uint64_t)nchunks * LOG_CHUNK >= part2_need ? log : alloc<LogEnt>(ctx, part2_need ? part2_need : 1);
-  uint32_t* cursor = alloc<uint32_t>(ctx, (uint64_t)nb1 * (SUBS + 1) * CURSOR_STRIDE);
-  if (!part || !part2 || !cursor) return KASCADE_ERR_OOM;
-  uint32_t* cursor1 = cursor;
-  uint32_t* cursor2 = cursor + (uint64_t)nb1 * CURSOR_STRIDE;
-  KS_CUDA(cudaMemsetAsync(cursor, 0, sizeof(uint32_t) * nb1 * (SUBS + 1) * CURSOR_STRIDE, s));
+  if (!part || !part2) return KASCADE_ERR_OOM;
   const size_t smem1 = TILE1 * sizeof(LogEnt) + 2 * sizeof(uint32_t) * nb1;
   const size_t smem2 = TILE2 * sizeof(LogEnt) + 2 * sizeof(uint32_t) * SUBS;
-  auto k1 = k_part1;
-  auto k2 = k_part2;
   KS_TRY(raise_smem_limits());
   {
     ProfScope ps(ctx, "resolve", s);
     const uint32_t tiles1 = (nchunks + TILE1 / LOG_CHUNK - 1) / (TILE1 / LOG_CHUNK);
-    k1<<<(unsigned)std::min<uint64_t>(tiles1, (uint64_t)ctx.usable_sms() * P1_BLOCKS), PT_THREADS, smem1, s>>>(
-        log, chunk_fill, nchunks, out1, limit, nb, part, cursor1, beyond, chunk_cursor, ctx.d_status);
+    k_part1<<<(unsigned)std::min<uint64_t>(tiles1, (uint64_t)ctx.usable_sms() * P1_BLOCKS), PT_THREADS, smem1, s>>>(
+        log, chunk_fill, nchunks, lv.out[1], limit, nb, part, cursor1, chunk_cursor, ctx.d_status);
     KS_CHECK_LAUNCH();
   }
   const uint32_t tiles2 = nb * (WIN / TILE2);
   if (tiles2) {
     ProfScope ps(ctx, "partition", s);
-    k2<<<(unsigned)std::min<uint64_t>(tiles2, (uint64_t)ctx.usable_sms() * P2_BLOCKS), PT_THREADS, smem2, s>>>(
-        part, cursor1, 0, nullptr, limit, nb, part2, cursor2, beyond, nullptr, ctx.d_status);
+    k_part2<<<(unsigned)std::min<uint64_t>(tiles2, (uint64_t)ctx.usable_sms() * P2_BLOCKS), PT_THREADS, smem2, s>>>(
+        part, cursor1, 0, nullptr, limit, nb, part2, cursor2, nullptr, ctx.d_status);
     KS_CHECK_LAUNCH();
   }
   // the first pass's output is dead after the second: it holds the unreached list
@@ -727,18 +695,16 @@ kascade_status rank_level0_log(kascade_ctx& ctx, const Rec* rec, uint32_t n, uin
     const uint32_t items = nb * SUBS;
     const size_t smem = SUB * (sizeof(unsigned long long) + sizeof(uint32_t));
     k_place<<<(unsigned)std::max<uint64_t>(1, std::min<uint64_t>(items, (uint64_t)ctx.usable_sms() * 2)),
-                FIN_THREADS, smem, s>>>(part2, cursor2, nb, limit, n, beyond, t.heads_are_rulers, t.root, t.rank,
-                                        ulist, ucount, ucap, t.seg_off, t.hint, t.nseg, t.plus_one, t.beyond_want,
-                                        ctx.d_status);
+                FIN_THREADS, smem, s>>>(part2, cursor2, nb, limit, t.root, t.rank, ulist, ucount, ucap, t.seg_off,
+                                        t.hint, t.nseg, t.plus_one, ctx.d_status);
     KS_CHECK_LAUNCH();
   }
-  if (!t.heads_are_rulers) {
+  {
     ProfScope ps(ctx, "heads", s);
     k_walk_unreached<<<ctx.usable_sms() * 4, 256, 0, s>>>(rec, ulist, ucount, ucap, n, limit, t.root, t.rank,
-                                                      ctx.d_status);
+                                                      t.seg_off, t.hint, t.nseg, t.plus_one, ctx.d_status);
     KS_CHECK_LAUNCH();
   }
-  if (r0_dev) return report_dev_levels(ctx, lv, levels, n, s);
   return KASCADE_OK;
 }
 

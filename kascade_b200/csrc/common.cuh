@@ -60,7 +60,9 @@ struct DevStatus {
   unsigned int code;
   unsigned int pad;
   unsigned long long info;
-  unsigned long long counter[6];
+  unsigned long long counter[6];  // [0]: write-free chains past their hop cap; [1]: level 0's size, when only the device knows it
+  unsigned int work[31];          // per level: rulers handed out beyond the warps' first shares
+  unsigned int heads;             // tour heads found
 };
 
 __device__ __forceinline__ void set_error(DevStatus* st, unsigned int code, unsigned long long info) {

@@ -1,6 +1,8 @@
 // Context plumbing: arena, status word, read-backs, kernel timing.
 #include "ctx.cuh"
 
+#include <cstddef>
+
 namespace ks {
 
 kascade_status cuda_status(cudaError_t e) {
@@ -98,22 +100,17 @@ static void collect_times(kascade_ctx& ctx) {
 }
 
 kascade_status status_finish(kascade_ctx& ctx, cudaStream_t s) {
-  cudaError_t e = cudaMemcpyAsync(ctx.h_pinned, ctx.d_status, sizeof(DevStatus), cudaMemcpyDeviceToHost, s);
+  cudaError_t e =
+      cudaMemcpyAsync(ctx.h_pinned, ctx.d_status, offsetof(DevStatus, work), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) {
     ctx.last_status = cuda_status(e);
     return ctx.last_status;
   }
   collect_times(ctx);
-  if (ctx.pending_levels) {
-    const uint32_t* lv = reinterpret_cast<const uint32_t*>(ctx.h_pinned + KS_PINNED_LEVELS);
-    // level 0's size: the call's n, or the device's count when only that
-    // knows it (a tour sized for a bound)
-    ctx.last_levels.assign(1, lv[0] ? (unsigned long long)lv[0] : ctx.pending_n);
-    for (int k = 1; k <= ctx.pending_levels; ++k) ctx.last_levels.push_back(lv[k]);
-    ctx.pending_levels = 0;
-  }
   const DevStatus* st = reinterpret_cast<const DevStatus*>(ctx.h_pinned);
+  // level 0's size when only the device knew it (a tour sized for a bound)
+  if (st->counter[1] && !ctx.last_levels.empty()) ctx.last_levels[0] = st->counter[1];
   ctx.error_info = st->info;
   ctx.last_status = (kascade_status)st->code;
   return ctx.last_status;

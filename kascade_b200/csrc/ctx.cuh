@@ -40,10 +40,6 @@ struct kascade_ctx {
   std::map<std::string, std::pair<double, unsigned long long>> times;
   std::vector<std::string> time_names;  // stable storage for returned names
   std::vector<unsigned long long> last_levels;
-  // level sizes of a device-driven recursion, copied to the pinned buffer by
-  // the call and read into last_levels when its status is read
-  int pending_levels = 0;
-  unsigned long long pending_n = 0;
   unsigned long long error_info = 0;
   kascade_status last_status = KASCADE_OK;
   // ordering between calls issued on different streams: the next call's
@@ -52,9 +48,9 @@ struct kascade_ctx {
   cudaEvent_t done_event = nullptr;
   cudaStream_t last_stream = nullptr;
   bool async_pending = false;
-  // an async host-buffer call ranked by the device-driven recursion: what
-  // kascade_ctx_sync needs to rank it again on the host-driven path when a
-  // level outgrew that recursion (the host buffers are the call's until then)
+  // an async host-buffer call: what kascade_ctx_sync needs to rank it again
+  // when a chain ran past the write-free chase's hop cap (the host buffers are
+  // the call's until then)
   struct HostRerun {
     bool set = false;
     int kind = 0;                     // 0: kascade_rank_list_host, 1: kascade_root_forest_host
@@ -96,7 +92,6 @@ struct kascade_ctx {
 namespace ks {
 
 constexpr int KS_PINNED_WORDS = 64;
-constexpr int KS_PINNED_LEVELS = 40;  // first word of the device-driven level sizes
 
 // Arena -------------------------------------------------------------------
 kascade_status arena_begin_call(kascade_ctx& ctx, cudaStream_t s);

@@ -60,13 +60,11 @@ constexpr uint32_t NO_CHILD = 0xFFFFFFFFu;
 // compacted into one vertex space with per-forest bases fd[j]:
 // the up edge of compact vertex c of forest j at that vertex's position in
 // the caller's concatenated arrays (foff[j] + c - fd[j]), the down edge into
-// c after all input elements (down_base + c).  Ruler sampling thresholds can
-// differ per forest (size classes).
+// c after all input elements (down_base + c).
 struct SlotsBatch {
-  const uint32_t* fd;       // nf + 1 compact starts
-  const uint32_t* foff;     // nf concatenated offsets
-  const uint32_t* fthresh;  // nf sampling thresholds
-  const uint32_t* fhint;    // per 4096 compact vertices: the forest holding the first
+  const uint32_t* fd;     // nf + 1 compact starts
+  const uint32_t* foff;   // nf concatenated offsets
+  const uint32_t* fhint;  // per 4096 compact vertices: the forest holding the first
   uint32_t nf;
   uint32_t down_base;
   __device__ __forceinline__ uint32_t seg_of(uint32_t c) const {
@@ -84,7 +82,6 @@ struct SlotsBatch {
   }
   __device__ __forceinline__ uint32_t up(uint32_t c, uint32_t j) const { return c - __ldg(fd + j) + __ldg(foff + j); }
   __device__ __forceinline__ uint32_t down(uint32_t c) const { return down_base + c; }
-  __device__ __forceinline__ uint32_t thresh(uint32_t j) const { return __ldg(fthresh + j); }
 };
 
 // Exchange on a child-list head with an L2 evict-last hint: the head array is
@@ -186,37 +183,34 @@ __device__ __forceinline__ void warp_set_bits(uint32_t* __restrict__ bits, bool 
 // loop of weight 0 that no element points to: the slots keep one place per
 // vertex, so the batch's record count stays fixed (a plan's shapes do not
 // depend on its forests' shapes) while the chase visits ~1.5 elements per
-// vertex instead of 2.  A tree's tour starts at the element entering its
-// root's list head (head_bits), which is always a ruler; ibits (vertices with
-// a down edge) tells which element a sibling or first child is entered by.
-// A tile's loads are issued in two independent rounds; rulers are sampled
-// among the slots and numbered with one atomic per tile.
+// vertex instead of 2.  ibits (vertices with a down edge) tells which element
+// a sibling or first child is entered by.  A tile's loads are issued in two
+// independent rounds.  heads: the tours' first vertices become their elements.
 template <class Slots>
 __global__ void __launch_bounds__(256) k_tour_links(const uint32_t* __restrict__ p32, uint32_t n,
                                                     const uint32_t* __restrict__ fc,
                                                     const uint32_t* __restrict__ nsib,
-                                                    const uint32_t* __restrict__ ibits,
-                                                    const uint32_t* __restrict__ head_bits, Rec* __restrict__ rec,
-                                                    uint32_t* __restrict__ ruler_elem, uint32_t* __restrict__ counter,
-                                                    uint32_t* __restrict__ leaf_out, uint32_t salt, Slots slots,
-                                                    DevStatus* st) {
-  __shared__ uint32_t sm[33];
-  __shared__ uint32_t sbase;
+                                                    const uint32_t* __restrict__ ibits, Rec* __restrict__ rec,
+                                                    uint32_t* __restrict__ leaf_out, uint32_t* __restrict__ heads,
+                                                    const uint32_t* __restrict__ nheads, Slots slots) {
   const uint32_t lane = threadIdx.x & 31u;
+  for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < min(*nheads, HEAD_CAP); e += gridDim.x * blockDim.x) {
+    const uint32_t c = heads[e];
+    heads[e] = ((ibits[c >> 5] >> (c & 31)) & 1u) ? slots.down(c) : slots.up(c, slots.seg_of(c));
+  }
   const uint64_t tile_sz = (uint64_t)blockDim.x * TB_BATCH_ITEMS;
   for (uint64_t tile = (uint64_t)blockIdx.x * tile_sz; tile < n; tile += (uint64_t)gridDim.x * tile_sz) {
-    uint32_t pv[TB_BATCH_ITEMS], sib[TB_BATCH_ITEMS], first[TB_BATCH_ITEMS], hw[TB_BATCH_ITEMS], jv[TB_BATCH_ITEMS];
+    uint32_t pv[TB_BATCH_ITEMS], sib[TB_BATCH_ITEMS], first[TB_BATCH_ITEMS], jv[TB_BATCH_ITEMS];
 #pragma unroll
     for (int i = 0; i < TB_BATCH_ITEMS; ++i) {
       const uint64_t v = tile + (uint64_t)i * blockDim.x + threadIdx.x;
       pv[i] = (uint32_t)v;
       sib[i] = first[i] = NO_CHILD;
-      hw[i] = jv[i] = 0;
+      jv[i] = 0;
       if (v < n) {
         pv[i] = __ldcs(p32 + v);  // in range: k_link_children made bad parents roots
         sib[i] = __ldcs(nsib + v);
         first[i] = __ldcs(fc + v);
-        hw[i] = __ldg(head_bits + (v >> 5));
         jv[i] = slots.seg_of((uint32_t)v);  // v, its parent and its children belong to the same forest
       }
     }
@@ -231,91 +225,38 @@ __global__ void __launch_bounds__(256) k_tour_links(const uint32_t* __restrict__
         if (first[i] != NO_CHILD) wfirst[i] = __ldg(ibits + (first[i] >> 5));
       }
     }
-    Rec ru[TB_BATCH_ITEMS], rd[TB_BATCH_ITEMS];
-    uint32_t su[TB_BATCH_ITEMS], sd[TB_BATCH_ITEMS];
-    uint32_t rl = 0, cnt = 0;
 #pragma unroll
     for (int i = 0; i < TB_BATCH_ITEMS; ++i) {
       const uint32_t v = (uint32_t)(tile + (uint64_t)i * blockDim.x + threadIdx.x);
-      su[i] = sd[i] = 0;
       bool leaf = false;
+      uint32_t up = 0;
       if (v < n) {
         const uint32_t j = jv[i], p = pv[i];
-        const uint32_t th = slots.thresh(j);
-        const uint32_t up = slots.up(v, j), down = slots.down(v);
-        su[i] = up;
-        sd[i] = down;
-        rd[i].a = 0;  // a dead self loop unless v keeps a down edge
-        rd[i].b = down;
-        if (p == v) {  // a root: the tour's terminal element (or an isolated vertex)
-          ru[i].a = 0;
-          ru[i].b = up;
-          rl |= 1u << (2 * i);
-          cnt++;
-        } else {
+        const uint32_t down = slots.down(v);
+        up = slots.up(v, j);
+        Rec ru, rd;
+        ru.a = rd.a = 0;
+        ru.b = up;  // a root: the tour's terminal element (or an isolated vertex)
+        rd.b = down;  // a dead self loop unless v keeps a down edge
+        ru.c = rd.c = TAG_UNREACHED;
+        if (p != v) {
           // the element a walk enters child c by: its down edge, or its merged slot
-          const uint32_t up_next = (sib[i] != NO_CHILD)
-                                       ? (((wsib[i] >> (sib[i] & 31)) & 1u) ? slots.down(sib[i]) : slots.up(sib[i], j))
-                                       : slots.up(p, j);
-          const bool head = (hw[i] >> (v & 31)) & 1u;
-          ru[i].b = up_next;
+          ru.b = (sib[i] != NO_CHILD)
+                     ? (((wsib[i] >> (sib[i] & 31)) & 1u) ? slots.down(sib[i]) : slots.up(sib[i], j))
+                     : slots.up(p, j);
           if (first[i] != NO_CHILD) {
-            ru[i].a = 1ull;
-            rd[i].a = ~0ull;  // -1
-            rd[i].b = ((wfirst[i] >> (first[i] & 31)) & 1u) ? slots.down(first[i]) : slots.up(first[i], j);
-            if (sampled(up, salt, th)) {
-              rl |= 1u << (2 * i);
-              cnt++;
-            }
-            if (head || sampled(down, salt, th)) {
-              rl |= 2u << (2 * i);
-              cnt++;
-            }
+            ru.a = 1ull;
+            rd.a = ~0ull;  // -1
+            rd.b = ((wfirst[i] >> (first[i] & 31)) & 1u) ? slots.down(first[i]) : slots.up(first[i], j);
           } else {
-            leaf = true;
-            ru[i].a = 0;  // down (-1) and up (+1) in one element
-            if (head || sampled(up, salt, th)) {
-              rl |= 1u << (2 * i);
-              cnt++;
-            }
+            leaf = true;  // down (-1) and up (+1) in one element of weight 0
           }
         }
+        st_rec_cs(rec + up, ru);
+        st_rec_cs(rec + down, rd);  // every down slot, dead or not: the stores stay coalesced
       }
-      warp_set_bits(leaf_out, leaf, su[i], lane);
+      warp_set_bits(leaf_out, leaf, up, lane);
     }
-    uint32_t total;
-    uint32_t pre = block_exclusive_scan(cnt, sm, &total);
-    if (threadIdx.x == 0) {
-      uint32_t b = total ? atomicAdd(counter, total) : 0u;
-      if ((uint64_t)b + total > MAX_RULERS) set_error(st, KASCADE_ERR_TOO_LARGE, b);
-      sbase = b;
-    }
-    __syncthreads();
-    uint32_t id = sbase + pre;
-#pragma unroll
-    for (int i = 0; i < TB_BATCH_ITEMS; ++i) {
-      const uint64_t v = tile + (uint64_t)i * blockDim.x + threadIdx.x;
-      if (v >= n) continue;
-      ru[i].c = TAG_UNREACHED;
-      rd[i].c = TAG_UNREACHED;
-      if ((rl >> (2 * i)) & 1u) {
-        if (id < MAX_RULERS) {
-          ru[i].c = TAG_RULER | id;
-          ruler_elem[id] = su[i];
-        }
-        id++;
-      }
-      if ((rl >> (2 * i)) & 2u) {
-        if (id < MAX_RULERS) {
-          rd[i].c = TAG_RULER | id;
-          ruler_elem[id] = sd[i];
-        }
-        id++;
-      }
-      st_rec_cs(rec + su[i], ru[i]);
-      st_rec_cs(rec + sd[i], rd[i]);  // every down slot, dead or not: the stores stay coalesced
-    }
-    __syncthreads();
   }
 }
 
@@ -408,13 +349,13 @@ kascade_status sort_children(kascade_ctx& ctx, const uint64_t* parent, uint32_t 
 // the compacted slot n + (their number among those vertices): ibits marks
 // them (one word per 32 vertices) and ipre counts them before each word, so
 // the element a parent or a sibling continues into is found with one read of
-// these L2-resident tables.  head_bits marks the first child of every root
-// (the vertex the tree's tour enters first), so the tour build reads its own
-// word instead of its parent's root bit and list head.
+// these L2-resident tables.  heads lists up to HEAD_CAP tour heads: the
+// vertices (list heads of their roots) whose element a tree's tour starts with.
 __global__ void __launch_bounds__(256) k_internal_words(const uint32_t* __restrict__ p32,
                                                         const uint32_t* __restrict__ fc, uint32_t n,
-                                                        uint32_t* __restrict__ ibits, uint32_t* __restrict__ icount,
-                                                        uint32_t* __restrict__ head_bits) {
+                                                        uint32_t* __restrict__ ibits,
+                                                        uint32_t* __restrict__ icount, uint32_t* __restrict__ heads,
+                                                        uint32_t* __restrict__ nheads) {
   const uint32_t lane = threadIdx.x & 31u;
   const uint64_t tile_sz = (uint64_t)blockDim.x * TB_ITEMS;
   for (uint64_t tile = (uint64_t)blockIdx.x * tile_sz; tile < n; tile += (uint64_t)gridDim.x * tile_sz) {
@@ -430,11 +371,18 @@ __global__ void __launch_bounds__(256) k_internal_words(const uint32_t* __restri
     for (int i = 0; i < TB_ITEMS; ++i) {
       const uint64_t v = tile + (uint64_t)i * blockDim.x + threadIdx.x;
       const uint32_t bits = __ballot_sync(0xffffffffu, v < n && pv[i] != (uint32_t)v && fv[i] != NO_CHILD);
-      // a root's list head enters its tree first: the head of that tree's tour
-      if (v < n && pv[i] == (uint32_t)v && fv[i] != NO_CHILD) atomicOr(head_bits + (fv[i] >> 5), 1u << (fv[i] & 31));
       if (lane == 0 && v < n) {
         ibits[v >> 5] = bits;
         icount[v >> 5] = (uint32_t)__popc(bits);
+      }
+      // a root's list head enters its tree first: the head of that tree's tour
+      const bool head = v < n && pv[i] == (uint32_t)v && fv[i] != NO_CHILD;
+      const uint32_t hm = __ballot_sync(0xffffffffu, head);
+      if (hm) {
+        uint32_t e = 0;
+        if (lane == 0) e = atomicAdd(nheads, (uint32_t)__popc(hm));
+        e = __shfl_sync(0xffffffffu, e, 0) + __popc(hm & lanemask_lt());
+        if (head && e < HEAD_CAP) heads[e] = fv[i];
       }
     }
   }
@@ -469,28 +417,28 @@ struct Entries {
 // of them per vertex.
 __global__ void __launch_bounds__(256) k_tour_leaves(const uint32_t* __restrict__ p32, uint32_t n,
                                                      const uint32_t* __restrict__ fc,
-                                                     const uint32_t* __restrict__ nsib,
-                                                     const uint32_t* __restrict__ head_bits, Entries ent,
-                                                     Rec* __restrict__ rec, uint32_t* __restrict__ ruler_elem,
-                                                     uint32_t* __restrict__ counter, uint32_t salt, uint32_t th,
-                                                     uint32_t* __restrict__ leaf_bits, DevStatus* st) {
-  __shared__ uint32_t sm[33];
-  __shared__ uint32_t sbase;
+                                                     const uint32_t* __restrict__ nsib, Entries ent,
+                                                     Rec* __restrict__ rec, uint32_t* __restrict__ leaf_bits,
+                                                     uint32_t* __restrict__ heads,
+                                                     const uint32_t* __restrict__ nheads) {
   const uint32_t lane = threadIdx.x & 31u;
+  // the tours' first vertices become the elements they are entered by
+  for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < min(*nheads, HEAD_CAP); e += gridDim.x * blockDim.x) {
+    const uint32_t c = heads[e];
+    heads[e] = ent.of(c, ent.word(c));
+  }
   const uint64_t tile_sz = (uint64_t)blockDim.x * TB_ITEMS;
   for (uint64_t tile = (uint64_t)blockIdx.x * tile_sz; tile < n; tile += (uint64_t)gridDim.x * tile_sz) {
-    uint32_t pv[TB_ITEMS], sib[TB_ITEMS], first[TB_ITEMS], hw[TB_ITEMS];
+    uint32_t pv[TB_ITEMS], sib[TB_ITEMS], first[TB_ITEMS];
 #pragma unroll
     for (int i = 0; i < TB_ITEMS; ++i) {
       const uint64_t v = tile + (uint64_t)i * blockDim.x + threadIdx.x;
       pv[i] = (uint32_t)v;
       sib[i] = first[i] = NO_CHILD;
-      hw[i] = 0;
       if (v < n) {
         pv[i] = __ldcs(p32 + v);
         sib[i] = __ldcs(nsib + v);
         first[i] = __ldcs(fc + v);
-        hw[i] = __ldg(head_bits + (v >> 5));
       }
     }
     uint2 wsib[TB_ITEMS], wfirst[TB_ITEMS], wown[TB_ITEMS];
@@ -508,87 +456,33 @@ __global__ void __launch_bounds__(256) k_tour_leaves(const uint32_t* __restrict_
         }
       }
     }
-    Rec ru[TB_ITEMS], rd[TB_ITEMS];
-    uint32_t sd[TB_ITEMS];
-    uint32_t rl = 0, cnt = 0, has_down = 0;
 #pragma unroll
     for (int i = 0; i < TB_ITEMS; ++i) {
       const uint32_t v = (uint32_t)(tile + (uint64_t)i * blockDim.x + threadIdx.x);
-      sd[i] = 0;
       bool leaf = false;
       if (v < n) {
         const uint32_t p = pv[i];
-        if (p == v) {  // a root: the tour's terminal element (or an isolated vertex)
-          ru[i].a = 0;
-          ru[i].b = v;
-          rl |= 1u << (2 * i);
-          cnt++;
-        } else {
-          const uint32_t up_next = (sib[i] != NO_CHILD) ? ent.of(sib[i], wsib[i]) : p;
-          const bool head = (hw[i] >> (v & 31)) & 1u;  // the down edge (or merged element) heading a tour
+        Rec ru, rd;
+        ru.a = 0;
+        ru.b = v;  // a root: the tour's terminal element (or an isolated vertex)
+        ru.c = rd.c = TAG_UNREACHED;
+        if (p != v) {
+          ru.b = (sib[i] != NO_CHILD) ? ent.of(sib[i], wsib[i]) : p;
           if (first[i] != NO_CHILD) {
-            sd[i] = ent.down_slot(v, wown[i]);
-            ru[i].a = 1ull;
-            ru[i].b = up_next;
-            rd[i].a = ~0ull;  // -1
-            rd[i].b = ent.of(first[i], wfirst[i]);
-            has_down |= 1u << i;
-            if (sampled(v, salt, th)) {
-              rl |= 1u << (2 * i);
-              cnt++;
-            }
-            if (head || sampled(sd[i], salt, th)) {
-              rl |= 2u << (2 * i);
-              cnt++;
-            }
+            ru.a = 1ull;
+            rd.a = ~0ull;  // -1
+            rd.b = ent.of(first[i], wfirst[i]);
+            st_rec_cs(rec + ent.down_slot(v, wown[i]), rd);
           } else {
-            leaf = true;
-            ru[i].a = 0;  // down (-1) and up (+1) in one element
-            ru[i].b = up_next;
-            if (head || sampled(v, salt, th)) {
-              rl |= 1u << (2 * i);
-              cnt++;
-            }
+            leaf = true;  // down (-1) and up (+1) in one element of weight 0
           }
         }
+        st_rec_cs(rec + v, ru);
       }
       // a warp's 32 consecutive vertices make one word of leaf bits
       const uint32_t lb = __ballot_sync(0xffffffffu, leaf);
       if (lane == 0 && v < n) leaf_bits[v >> 5] = lb;
     }
-    uint32_t total;
-    uint32_t pre = block_exclusive_scan(cnt, sm, &total);
-    if (threadIdx.x == 0) {
-      uint32_t b = total ? atomicAdd(counter, total) : 0u;
-      if ((uint64_t)b + total > MAX_RULERS) set_error(st, KASCADE_ERR_TOO_LARGE, b);
-      sbase = b;
-    }
-    __syncthreads();
-    uint32_t id = sbase + pre;
-#pragma unroll
-    for (int i = 0; i < TB_ITEMS; ++i) {
-      const uint64_t v = tile + (uint64_t)i * blockDim.x + threadIdx.x;
-      if (v >= n) continue;
-      ru[i].c = TAG_UNREACHED;
-      rd[i].c = TAG_UNREACHED;
-      if ((rl >> (2 * i)) & 1u) {
-        if (id < MAX_RULERS) {
-          ru[i].c = TAG_RULER | id;
-          ruler_elem[id] = (uint32_t)v;
-        }
-        id++;
-      }
-      if ((rl >> (2 * i)) & 2u) {
-        if (id < MAX_RULERS) {
-          rd[i].c = TAG_RULER | id;
-          ruler_elem[id] = sd[i];
-        }
-        id++;
-      }
-      st_rec_cs(rec + v, ru[i]);
-      if ((has_down >> i) & 1u) st_rec_cs(rec + sd[i], rd[i]);
-    }
-    __syncthreads();
   }
 }
 
@@ -604,11 +498,11 @@ kascade_status link_children(kascade_ctx& ctx, const uint64_t* parent, uint32_t 
 }
 
 // Child lists and the leaf-contracted tour records of every vertex at the
-// slots `slots` gives (a batch's forests); ruler ids continue `counter`,
-// leaves are marked in leaf_out (by output position, zeroed by the caller).
+// slots `slots` gives (a batch's forests); leaves are marked in leaf_out (by
+// output position, zeroed by the caller).
 template <class Slots>
 kascade_status build_tour(kascade_ctx& ctx, const uint64_t* parent, uint32_t n, const Slots& slots, Rec* rec,
-                          uint32_t* ruler_elem, uint32_t* counter, uint32_t* leaf_out, uint32_t salt, cudaStream_t s) {
+                          uint32_t* leaf_out, Heads* heads, cudaStream_t s) {
   const uint64_t words = ((uint64_t)n + 31) / 32;
   uint32_t* fc = alloc<uint32_t>(ctx, n);
   uint32_t* nsib = alloc<uint32_t>(ctx, n);
@@ -616,17 +510,17 @@ kascade_status build_tour(kascade_ctx& ctx, const uint64_t* parent, uint32_t n, 
   uint32_t* root_bits = alloc<uint32_t>(ctx, words);
   uint32_t* ibits = alloc<uint32_t>(ctx, words);
   uint32_t* icount = alloc<uint32_t>(ctx, words);
-  uint32_t* head_bits = alloc<uint32_t>(ctx, words);
-  if (!fc || !nsib || !p32 || !root_bits || !ibits || !icount || !head_bits) return KASCADE_ERR_OOM;
-  KS_CUDA(cudaMemsetAsync(head_bits, 0, sizeof(uint32_t) * words, s));
+  uint32_t* head = alloc<uint32_t>(ctx, HEAD_CAP);
+  if (!fc || !nsib || !p32 || !root_bits || !ibits || !icount || !head) return KASCADE_ERR_OOM;
+  *heads = Heads{head, &ctx.d_status->heads, HEAD_CAP};
   KS_TRY(link_children(ctx, parent, n, fc, nsib, p32, root_bits, s));
   ProfScope ps(ctx, "tour_build", s);
-  k_internal_words<<<grid_for(ctx, n, 256, 8), 256, 0, s>>>(p32, fc, n, ibits, icount, head_bits);
+  k_internal_words<<<grid_for(ctx, n, 256, 8), 256, 0, s>>>(p32, fc, n, ibits, icount, head,
+                                                              &ctx.d_status->heads);
   KS_CHECK_LAUNCH();
   const unsigned grid =
       grid_for(ctx, ((uint64_t)n + 256 * TB_BATCH_ITEMS - 1) / (256 * TB_BATCH_ITEMS) * 256, 256, 8);
-  k_tour_links<Slots><<<grid, 256, 0, s>>>(p32, n, fc, nsib, ibits, head_bits, rec, ruler_elem, counter, leaf_out,
-                                           salt, slots, ctx.d_status);
+  k_tour_links<Slots><<<grid, 256, 0, s>>>(p32, n, fc, nsib, ibits, rec, leaf_out, head, &ctx.d_status->heads, slots);
   KS_CHECK_LAUNCH();
   return KASCADE_OK;
 }
@@ -635,12 +529,11 @@ kascade_status build_tour(kascade_ctx& ctx, const uint64_t* parent, uint32_t n, 
 
 kascade_status root_forest_impl(kascade_ctx& ctx, const uint64_t* parent, uint32_t n, uint64_t* root_out,
                                 uint64_t* depth_out, int keep_roots, const Params& p, cudaStream_t s,
-                                bool device_levels) {
+                                bool host_check) {
   if (n == 0) return KASCADE_OK;
   const uint32_t words = (uint32_t)(((uint64_t)n + 31) / 32);
   Rec* rec = alloc<Rec>(ctx, 2ull * n);
-  uint32_t* ruler_elem = alloc<uint32_t>(ctx, 2ull * n);
-  uint32_t* ctr = alloc<uint32_t>(ctx, 2);  // ruler count, down-edge count
+  uint32_t* downs = alloc<uint32_t>(ctx, 1);  // down-edge count
   uint32_t* fc = alloc<uint32_t>(ctx, n);
   uint32_t* nsib = alloc<uint32_t>(ctx, n);
   uint32_t* p32 = alloc<uint32_t>(ctx, n);
@@ -649,63 +542,45 @@ kascade_status root_forest_impl(kascade_ctx& ctx, const uint64_t* parent, uint32
   uint32_t* icount = alloc<uint32_t>(ctx, words);
   uint32_t* ipre = alloc<uint32_t>(ctx, words);
   uint32_t* leaf_bits = alloc<uint32_t>(ctx, words);
-  uint32_t* head_bits = alloc<uint32_t>(ctx, words);
   uint2* iw = alloc<uint2>(ctx, words);
-  if (!rec || !ruler_elem || !ctr || !fc || !nsib || !p32 || !root_bits || !ibits || !icount || !ipre || !leaf_bits ||
-      !head_bits || !iw)
+  uint32_t* head = alloc<uint32_t>(ctx, HEAD_CAP);
+  if (!rec || !downs || !fc || !nsib || !p32 || !root_bits || !ibits || !icount || !ipre || !leaf_bits || !iw || !head)
     return KASCADE_ERR_OOM;
-  KS_CUDA(cudaMemsetAsync(ctr, 0, 2 * sizeof(uint32_t), s));
-  KS_CUDA(cudaMemsetAsync(head_bits, 0, sizeof(uint32_t) * (size_t)words, s));
   KS_TRY(link_children(ctx, parent, n, fc, nsib, p32, root_bits, s));
   {
     ProfScope ps(ctx, "tour_build", s);
-    k_internal_words<<<grid_for(ctx, n, 256, 8), 256, 0, s>>>(p32, fc, n, ibits, icount, head_bits);
+    k_internal_words<<<grid_for(ctx, n, 256, 8), 256, 0, s>>>(p32, fc, n, ibits, icount, head,
+                                                              &ctx.d_status->heads);
     KS_CHECK_LAUNCH();
-    KS_TRY(exclusive_scan_u32(ctx, icount, ipre, words, ctr + 1, s));
+    KS_TRY(exclusive_scan_u32(ctx, icount, ipre, words, downs, s));
     k_internal_pack<<<grid_for(ctx, words, 256, 8), 256, 0, s>>>(ibits, ipre, words, iw);
     KS_CHECK_LAUNCH();
-  }
-  {
-    ProfScope ps(ctx, "tour_build", s);
     const unsigned grid = grid_for(ctx, ((uint64_t)n + 256 * TB_ITEMS - 1) / (256 * TB_ITEMS) * 256, 256, 8);
-    const uint32_t th = (uint32_t)(4294967296.0 / (double)(p.spacing0 < 2 ? 2 : p.spacing0));
-    k_tour_leaves<<<grid, 256, 0, s>>>(p32, n, fc, nsib, head_bits, Entries{iw, n}, rec, ruler_elem, ctr,
-                                       mix32(p.seed ^ 0x70757254u), th, leaf_bits, ctx.d_status);
+    k_tour_leaves<<<grid, 256, 0, s>>>(p32, n, fc, nsib, Entries{iw, n}, rec, leaf_bits, head,
+                                       &ctx.d_status->heads);
     KS_CHECK_LAUNCH();
   }
-  SinkTour sink{root_out, depth_out, n, keep_roots, leaf_bits};
-  // The tour's length m = n + (down edges) is on the device (ctr[1]).  The
-  // device-driven recursion sizes for the bound 2n instead of reading it: no
-  // element points into the unused slots [m, 2n), no chase visits them, and
-  // outputs come only from slots below n; the write-free level 0 takes its
-  // count of down-edge entries from ctr[1].  (Every element below m exists
-  // and m >= n > base_max, so no path that reads every record is taken.)
-  const uint32_t m_cap = 2 * n;  // n <= 2^31 - 1
-  if (device_levels && n > p.base_max && p.max_levels > 0) {
-    sink.downs_dev = ctr + 1;
-    if (m_cap < p.level0_log_min)
-      return rank_records_dev(ctx, rec, m_cap, ctr, dev_cap_next(m_cap, p.spacing0), ruler_elem, sink, p, s);
-    if (!keep_roots)  // the write-free level 0 with the ruler count and the deeper levels on the device
-      return rank_level0_log(ctx, rec, m_cap, dev_cap_next(m_cap, p.spacing0), ruler_elem,
-                             sink.log_target(m_cap), p, s, ctr);
-  }
-  // the host-driven path: the tour's length and the ruler count (host reads)
-  uint32_t downs = 0, r = 0;
-  KS_TRY(read_u32(ctx, ctr + 1, &downs, s));
-  KS_TRY(read_u32(ctx, ctr, &r, s));
-  return rank_records(ctx, rec, n + downs, r, ruler_elem, sink, p, s);
+  // The tour's length n + (down edges) stays on the device: the ranking is
+  // sized for the bound 2n, rulers beyond the length are dead, and outputs
+  // come only from slots below n.
+  Extent ext;
+  ext.cap = 2 * n;  // n <= 2^31 - 1
+  ext.base = n;
+  ext.add = downs;
+  return rank_records(ctx, rec, ext.cap, ext, Heads{head, &ctx.d_status->heads, HEAD_CAP},
+                      SinkTour{root_out, depth_out, n, keep_roots, leaf_bits}, p, s, host_check);
 }
 
 // Tours of a batch of forests whose parents are given in one compact vertex
 // space (fpar[c] = compact parent of compact vertex c); records go to the
-// slots described by SlotsBatch, ruler ids continue `counter`.
+// slots described by SlotsBatch, *heads gets the tours' heads.
 kascade_status batch_tours(kascade_ctx& ctx, const uint64_t* fpar, uint32_t F, const uint32_t* fd, const uint32_t* foff,
-                           const uint32_t* fthresh, const uint32_t* fhint, uint32_t nf, uint32_t down_base, Rec* rec,
-                           uint32_t* ruler_elem, uint32_t* counter, uint32_t* leaf_out, uint32_t salt,
-                           cudaStream_t s) {
+                           const uint32_t* fhint, uint32_t nf, uint32_t down_base, Rec* rec, uint32_t* leaf_out,
+                           Heads* heads, cudaStream_t s) {
+  *heads = Heads{};
   if (F == 0) return KASCADE_OK;
-  const SlotsBatch slots{fd, foff, fthresh, fhint, nf, down_base};
-  return build_tour(ctx, fpar, F, slots, rec, ruler_elem, counter, leaf_out, salt, s);
+  const SlotsBatch slots{fd, foff, fhint, nf, down_base};
+  return build_tour(ctx, fpar, F, slots, rec, leaf_out, heads, s);
 }
 
 kascade_status compute_euler_tour_impl(kascade_ctx& ctx, const uint64_t* parent, uint32_t n, uint64_t* tour,

@@ -2,8 +2,8 @@
 //
 // Reference counterparts (niklas-uhl/kascade):
 //   ruler sampling      lib/kascade/sparse_ruling_set_detail/ruler_selection.hpp:18-115,
-//                       sparse_ruling_set.cpp:106-136 (shuffled candidates) -> here a
-//                       counter hash of the index, plus every root
+//                       sparse_ruling_set.cpp:106-136 (shuffled candidates) -> here one
+//                       element of every block of s indices, at a hashed offset
 //   ruler chasing       sparse_ruling_set.cpp:147-273 (init / work_on_item) and
 //                       ruler_chasing_engine.hpp:57-101 (sync rounds) -> one
 //                       persistent kernel, every hop a dependent 16 B load
@@ -15,8 +15,10 @@
 //   propagation (pull)  ruler_propagation.hpp:148-256 -> one coalesced pass
 //   pointer doubling    pointer_doubling_generic.hpp:43-60, 171-212, 418-438,
 //                       609-700 -> double-buffered jump kernel
+#include <algorithm>
+#include <atomic>
+#include <cmath>
 #include <cstddef>
-#include <cstdio>
 
 #include "ranker.cuh"
 #include "tma.cuh"
@@ -27,9 +29,6 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int PREP_ITEMS = 8;
-constexpr int PROP_ITEMS = 8;
-constexpr int BASE_THREADS = 1024;
-constexpr int BASE_PER_THREAD = 8;  // base_max <= BASE_THREADS * BASE_PER_THREAD
 
 // Weight sources; T is the narrowest type that holds one weight (fewer live
 // registers in the prepare kernel).
@@ -50,86 +49,55 @@ struct WI64 {
   }
 };
 
-inline uint32_t thresh_for(uint32_t spacing) {
-  if (spacing <= 1) return 0xFFFFFFFFu;
-  double t = 4294967296.0 / (double)spacing;
-  return t >= 4294967295.0 ? 0xFFFFFFFFu : (uint32_t)t;
-}
 inline uint32_t salt_for(uint32_t seed, int level) { return mix32(seed + 0x9E3779B9u * (uint32_t)(level + 1)); }
 
 // ---------------------------------------------------------------------------
-// prepare: build records, sample rulers (every root is a ruler), number them.
-// One atomicAdd per 2048-element tile hands out dense ruler ids.
+// prepare: build records.  A root's weight is no part of any rank: its record
+// carries 0, so that a chain ending at it adds the record's word like any.
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ Rec make_rec(uint64_t w, uint64_t succ, uint64_t x) {
+  Rec r;
+  r.a = succ == x ? 0ull : w;
+  r.b = (uint32_t)succ;
+  r.c = TAG_UNREACHED;
+  return r;
+}
+
 template <class W>
 __global__ void __launch_bounds__(256, 4) k_prepare_arrays(const uint64_t* __restrict__ succ, W w, uint32_t n,
-                                                        uint64_t start, Rec* __restrict__ rec,
-                                                        uint32_t* __restrict__ ruler_elem,
-                                                        uint32_t* __restrict__ counter, uint32_t salt,
-                                                        uint32_t thresh, DevStatus* st) {
-  __shared__ uint32_t sm[33];
-  __shared__ uint32_t sbase;
+                                                        uint64_t start, Rec* __restrict__ rec, DevStatus* st) {
   const uint64_t tile_sz = (uint64_t)blockDim.x * PREP_ITEMS;
   for (uint64_t tile = start + (uint64_t)blockIdx.x * tile_sz; tile < n; tile += (uint64_t)gridDim.x * tile_sz) {
-    uint32_t sv[PREP_ITEMS];
+    unsigned long long sv[PREP_ITEMS];
     typename W::T wv[PREP_ITEMS];
-    uint32_t rl = 0, cnt = 0;
 #pragma unroll
     for (int i = 0; i < PREP_ITEMS; ++i) {
-      uint64_t x = tile + (uint64_t)i * blockDim.x + threadIdx.x;
+      const uint64_t x = tile + (uint64_t)i * blockDim.x + threadIdx.x;
       sv[i] = 0;
       wv[i] = 0;
       if (x < n) {
-        unsigned long long s = __ldcs(reinterpret_cast<const unsigned long long*>(succ) + x);
-        if (s >= n) {
-          set_error(st, KASCADE_ERR_OUT_OF_RANGE, x);
-          s = x;
-        }
-        sv[i] = (uint32_t)s;
+        sv[i] = __ldcs(reinterpret_cast<const unsigned long long*>(succ) + x);
         wv[i] = w(x);
-        if (s == x || sampled((uint32_t)x, salt, thresh)) {
-          rl |= 1u << i;
-          cnt++;
-        }
       }
     }
-    uint32_t total;
-    uint32_t pre = block_exclusive_scan(cnt, sm, &total);
-    if (threadIdx.x == 0) {
-      uint32_t b = total ? atomicAdd(counter, total) : 0u;
-      if ((uint64_t)b + total > MAX_RULERS) set_error(st, KASCADE_ERR_TOO_LARGE, b);
-      sbase = b;
-    }
-    __syncthreads();
-    uint32_t id = sbase + pre;
 #pragma unroll
     for (int i = 0; i < PREP_ITEMS; ++i) {
-      uint64_t x = tile + (uint64_t)i * blockDim.x + threadIdx.x;
-      if (x < n) {
-        Rec r;
-        r.a = wv[i];
-        r.b = sv[i];
-        r.c = TAG_UNREACHED;
-        if (rl & (1u << i)) {
-          if (id < MAX_RULERS) {
-            r.c = TAG_RULER | id;
-            ruler_elem[id] = (uint32_t)x;
-          }
-          id++;
-        }
-        rec[x] = r;
+      const uint64_t x = tile + (uint64_t)i * blockDim.x + threadIdx.x;
+      if (x >= n) continue;
+      if (sv[i] >= n) {
+        set_error(st, KASCADE_ERR_OUT_OF_RANGE, x);
+        sv[i] = x;
       }
+      rec[x] = make_rec(wv[i], sv[i], x);
     }
-    __syncthreads();
   }
 }
 
 // The same work for 16 B-aligned inputs, with the input tiles moved by bulk
 // (TMA) copies: a persistent block keeps PT_STAGES tiles of succ (and
-// weights) in flight into shared memory while it numbers the rulers of an
-// earlier tile and writes its records, so the loads no longer wait behind the
-// block scan and the ruler-id atomic.  Full tiles only; the caller hands the
-// tail to k_prepare_arrays.
+// weights) in flight into shared memory while it writes the records of an
+// earlier tile.  Full tiles only; the caller hands the tail to
+// k_prepare_arrays.
 constexpr int PT_TILE = 2048;
 constexpr int PT_STAGES = 4;
 constexpr int PT_ITEMS = PT_TILE / 256;
@@ -137,14 +105,10 @@ constexpr int PT_ITEMS = PT_TILE / 256;
 template <bool W32>
 __global__ void __launch_bounds__(256) k_prepare_tma(const uint64_t* __restrict__ succ, const uint32_t* __restrict__ w,
                                                      uint32_t n, uint32_t ntiles, Rec* __restrict__ rec,
-                                                     uint32_t* __restrict__ ruler_elem,
-                                                     uint32_t* __restrict__ counter, uint32_t salt, uint32_t thresh,
                                                      DevStatus* st) {
   constexpr uint32_t SB = PT_TILE * 8, WB = W32 ? PT_TILE * 4 : 0, STAGE = SB + WB;
   extern __shared__ __align__(128) unsigned char dyn[];
   __shared__ __align__(8) uint64_t bar[PT_STAGES];
-  __shared__ uint32_t sm[33];
-  __shared__ uint32_t sbase;
   const uint32_t tid = threadIdx.x;
   if (tid == 0) {
     for (int i = 0; i < PT_STAGES; ++i) mbar_init(&bar[i], 1);
@@ -183,7 +147,6 @@ __global__ void __launch_bounds__(256) k_prepare_tma(const uint64_t* __restrict_
     const uint32_t* ws = reinterpret_cast<const uint32_t*>(dyn + sg * STAGE + SB);
     const uint64_t base = (uint64_t)t * PT_TILE;
     uint32_t sv[PT_ITEMS], wv[PT_ITEMS];
-    uint32_t rl = 0, cnt = 0;
 #pragma unroll
     for (int i = 0; i < PT_ITEMS; ++i) {
       const uint32_t j = i * 256 + tid;
@@ -195,152 +158,66 @@ __global__ void __launch_bounds__(256) k_prepare_tma(const uint64_t* __restrict_
       }
       sv[i] = (uint32_t)sx;
       wv[i] = W32 ? ws[j] : 1u;
-      if (sx == x || sampled(x, salt, thresh)) {
-        rl |= 1u << i;
-        cnt++;
-      }
     }
     __syncthreads();  // the stage is read: refill it with this block's tile k + PT_STAGES
     if (tid == 0) {
       fence_proxy_async();
       issue(k + PT_STAGES);
     }
-    uint32_t total;
-    const uint32_t pre = block_exclusive_scan(cnt, sm, &total);
-    if (tid == 0) {
-      const uint32_t b = total ? atomicAdd(counter, total) : 0u;
-      if ((uint64_t)b + total > MAX_RULERS) set_error(st, KASCADE_ERR_TOO_LARGE, b);
-      sbase = b;
-    }
-    __syncthreads();
-    uint32_t id = sbase + pre;
 #pragma unroll
     for (int i = 0; i < PT_ITEMS; ++i) {
       const uint32_t x = (uint32_t)(base + i * 256 + tid);
-      Rec r;
-      r.a = wv[i];
-      r.b = sv[i];
-      r.c = TAG_UNREACHED;
-      if (rl & (1u << i)) {
-        if (id < MAX_RULERS) {
-          r.c = TAG_RULER | id;
-          ruler_elem[id] = x;
-        }
-        id++;
-      }
-      st_rec_cs(rec + x, r);
+      st_rec_cs(rec + x, make_rec(wv[i], sv[i], x));
     }
-    __syncthreads();
   }
 }
 
-// Deeper levels: the chase of the level above wrote the records (tag
-// unreached); sample rulers in place and record each ruler's level-0 index.
-// n_dev (device-driven recursion): the level's size is read from device
-// memory, n is then its capacity; rulers beyond cap_next are reported as an
-// overflow (KASCADE_ERR_TIMEOUT, the caller reruns on the host-driven path).
-// has_pred (optional): bit x set when a chain of the level above ended at x;
-// an element without it heads its list at this level and becomes a ruler, so
-// no element of this level is left for propagation to walk to its first
-// ruler (a batch's level holds one list per instance, and the longest of
-// those walks would set the propagation's duration).
-__global__ void __launch_bounds__(256) k_prepare_level(Rec* __restrict__ rec, uint32_t n,
-                                                       const uint32_t* __restrict__ n_dev, uint32_t cap_next,
-                                                       const uint32_t* __restrict__ elem0,
-                                                       uint32_t* __restrict__ ruler_elem,
-                                                       uint32_t* __restrict__ elem0_next,
-                                                       uint32_t* __restrict__ counter, uint32_t salt,
-                                                       uint32_t thresh, const uint32_t* __restrict__ has_pred,
-                                                       DevStatus* st) {
-  __shared__ uint32_t sm[33];
-  __shared__ uint32_t sbase;
-  if (n_dev) n = min(*n_dev, n);
-  const uint64_t tile_sz = (uint64_t)blockDim.x * PREP_ITEMS;
-  for (uint64_t tile = (uint64_t)blockIdx.x * tile_sz; tile < n; tile += (uint64_t)gridDim.x * tile_sz) {
-    Rec rv[PREP_ITEMS];
-    uint32_t rl = 0, cnt = 0;
-#pragma unroll
-    for (int i = 0; i < PREP_ITEMS; ++i) {
-      uint64_t x = tile + (uint64_t)i * blockDim.x + threadIdx.x;
-      if (x < n) {
-        rv[i] = rec[x];
-        if (rv[i].b >= n) {  // never for records the level above wrote; kept as a guard
-          set_error(st, KASCADE_ERR_OUT_OF_RANGE, x);
-          rv[i].b = (uint32_t)x;
-        }
-        const bool head = has_pred && !((__ldg(has_pred + (x >> 5)) >> (x & 31)) & 1u);
-        if (rv[i].b == (uint32_t)x || head || sampled((uint32_t)x, salt, thresh)) {
-          rl |= 1u << i;
-          cnt++;
-        }
-      }
-    }
-    uint32_t total;
-    uint32_t pre = block_exclusive_scan(cnt, sm, &total);
-    if (threadIdx.x == 0) sbase = total ? atomicAdd(counter, total) : 0u;
-    __syncthreads();
-    uint32_t id = sbase + pre;
-#pragma unroll
-    for (int i = 0; i < PREP_ITEMS; ++i) {
-      uint64_t x = tile + (uint64_t)i * blockDim.x + threadIdx.x;
-      if (x < n) {
-        Rec r = rv[i];
-        r.c = TAG_UNREACHED;
-        if (rl & (1u << i)) {
-          if (id < cap_next) {
-            r.c = TAG_RULER | id;
-            ruler_elem[id] = (uint32_t)x;
-            elem0_next[id] = elem0 ? elem0[x] : (uint32_t)x;
-          } else {
-            set_error(st, KASCADE_ERR_TIMEOUT, id);  // more rulers than the next level holds
-          }
-          id++;
-        }
-        rec[x] = r;
-      }
-    }
-    __syncthreads();
-  }
-}
-
-// A chain that ends on an error still leaves its ruler a valid next-level
-// record (a self loop), so that later levels only ever see in-range indices.
-__device__ __forceinline__ void end_chain_on_error(Rec* rec_next, uint32_t id) {
+// The record of ruler `id` at the next level: its chain ended at ruler `next`,
+// or (next == id) at the list's end, whose level-0 root goes to *rootel.
+__device__ __forceinline__ void end_chain(Rec* rec_next, uint32_t id, uint64_t dist, uint32_t next) {
   Rec o;
-  o.a = 0;
-  o.b = id;
+  o.a = dist;
+  o.b = next;
   o.c = TAG_UNREACHED;
   st_rec_cg(rec_next + id, o);
 }
 
 // ---------------------------------------------------------------------------
-// chase: persistent, C chains in flight per thread, rulers handed out to each
-// warp in batches of 32*C from one global counter.  A hop reads the 16 B
-// record of the next element; an unreached element is stamped with
-// (distance from ruler, ruler id) in the same record.  A chain ends at the
-// next ruler (or root) and writes its ruler's sub-list record:
-// (weight = distance to that ruler, successor = that ruler's id).
+// chase: C chains in flight per thread, one per ruler.  A hop reads the 16 B
+// record of the next element and stamps (distance from ruler, ruler id) into
+// it.  A chain ends in front of the next ruler, known from the index alone,
+// or at the list's end.  A warp's first rulers are its own share, later ones
+// come from one counter; only the first `lanes` lanes of a warp work, so that
+// few rulers spread over all SMs and a warp's hop waits for few loads (a
+// dependent L2 hop costs 0.23 us alone and 0.43 us for 32 lanes together).
+// A new chain's first load shares an iteration with the other lanes' hops.
 // ---------------------------------------------------------------------------
+// head_base: where level k >= 1 keeps its heads (level 0: heads.elem lists
+// them).  A head's own record is stamped at distance 0.
 template <int C>
-__global__ void __launch_bounds__(512) k_chase(Rec* __restrict__ rec, uint32_t n, const uint32_t* __restrict__ n_dev,
-                                               const uint32_t* __restrict__ ruler_elem, uint32_t r,
-                                               const uint32_t* __restrict__ r_dev, Rec* __restrict__ rec_next,
-                                               uint32_t* __restrict__ work, uint32_t* __restrict__ has_pred,
-                                               DevStatus* st) {
-  // device-driven recursion: sizes from device memory, n and r capacities
-  // (has_pred holds one bit per ruler of the capacity; a count past it is
-  // reported by the caller's count check and the level redone)
-  const uint32_t pred_cap = r;
-  if (n_dev) n = min(*n_dev, n);
-  if (r_dev) r = min(*r_dev, r);
-  constexpr uint32_t BATCH = 32u * C;
+__global__ void __launch_bounds__(512) k_chase(Rec* __restrict__ rec, Extent ext, Rulers rl, uint32_t rulers,
+                                               Heads heads, uint32_t head_base,
+                                               const uint32_t* __restrict__ rootel, Rec* __restrict__ rec_next,
+                                               uint32_t* __restrict__ rootel_next, uint32_t* __restrict__ work,
+                                               uint32_t lanes, DevStatus* st) {
+  const uint32_t n = ext.get();
+  const uint32_t r = rulers + heads.get();
+  // level 0's size, reported by the call
+  if (!rootel && ext.add && blockIdx.x == 0 && threadIdx.x == 0) st->counter[1] = n;
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t lt = lanemask_lt();
+  const uint32_t batch = lanes * C;
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+  const uint32_t warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   uint32_t cid[C], cx[C], hops[C];
   uint64_t acc[C];
-  uint32_t act = 0;
-  uint32_t q_base = 0, q_left = 0;  // warp-uniform local batch of ruler ids
-  bool drained = false;             // warp-uniform
+  uint32_t act = 0, fresh = 0;  // bit c: chain c runs / has not read its ruler's record yet
+  // warp-uniform: this warp's ruler ids at hand, and whether more may follow
+  uint32_t q_base = warp * batch;
+  uint32_t q_left = q_base < r ? r - q_base : 0u;
+  if (q_left > batch) q_left = batch;
+  const uint32_t first = warps * batch;  // ids from here on are handed out by the counter
+  bool drained = false;
 #pragma unroll
   for (int c = 0; c < C; ++c) {
     cid[c] = cx[c] = hops[c] = 0;
@@ -350,43 +227,50 @@ __global__ void __launch_bounds__(512) k_chase(Rec* __restrict__ rec, uint32_t n
     if (!drained) {
 #pragma unroll
       for (int c = 0; c < C; ++c) {
-        bool need = !(act & (1u << c));
+        bool need = lane < lanes && !((act >> c) & 1u);
         uint32_t m = __ballot_sync(FULL, need);
         while (m != 0u && !drained) {
           if (q_left == 0u) {
-            uint32_t b = 0;
-            if (lane == 0) b = atomicAdd(work, BATCH);
-            b = __shfl_sync(FULL, b, 0);
+            uint32_t b = r;
+            if (first < r) {
+              uint32_t t = 0;
+              if (lane == 0) t = atomicAdd(work, batch);
+              b = first + __shfl_sync(FULL, t, 0);
+            }
             if (b >= r) {
               drained = true;
               break;
             }
             q_base = b;
-            q_left = min(BATCH, r - b);
+            q_left = r - b;
+            if (q_left > batch) q_left = batch;
           }
           const uint32_t take = min((uint32_t)__popc(m), q_left);
           const uint32_t my_rank = __popc(m & lt);
           const bool mine = need && my_rank < take;
           if (mine) {
             const uint32_t id = q_base + my_rank;
-            const uint32_t x0 = __ldg(ruler_elem + id);
-            const Rec r0 = ld_rec_cg(rec + x0);
-            if (r0.b == x0) {
-              Rec o;
-              o.a = 0;
-              o.b = id;
-              o.c = TAG_UNREACHED;
-              st_rec_cg(rec_next + id, o);
+            uint64_t x0;
+            if (id < rulers)
+              x0 = rl.elem(id);
+            else
+              x0 = rootel ? head_base + (id - rulers) : __ldg(heads.elem + (id - rulers));
+            uint32_t j;
+            if (x0 >= n) {
+              end_chain(rec_next, id, 0, id);  // the last block's ruler, beyond the elements
+            } else if (id >= rulers && rl.is((uint32_t)x0, &j) && j < rulers) {
+              end_chain(rec_next, id, 0, j);  // a head that is a ruler itself
+              rootel_next[id] = 0;
             } else {
               cid[c] = id;
-              cx[c] = r0.b;
-              acc[c] = r0.a;
+              cx[c] = (uint32_t)x0;
+              acc[c] = 0;
               hops[c] = 0;
               act |= 1u << c;
+              fresh |= 1u << c;
             }
           }
-          const uint32_t served = __ballot_sync(FULL, mine);
-          m &= ~served;
+          m &= ~__ballot_sync(FULL, mine);
           need = need && !mine;
           q_base += take;
           q_left -= take;
@@ -400,41 +284,48 @@ __global__ void __launch_bounds__(512) k_chase(Rec* __restrict__ rec, uint32_t n
     Rec rr[C];
 #pragma unroll
     for (int c = 0; c < C; ++c)
-      if (act & (1u << c)) rr[c] = ld_rec_cg(rec + cx[c]);
+      if ((act >> c) & 1u) rr[c] = ld_rec_cg(rec + cx[c]);
 #pragma unroll
     for (int c = 0; c < C; ++c) {
-      if (!(act & (1u << c))) continue;
-      const uint32_t tg = rr[c].c;
-      if (tag_unreached(tg)) {
-        Rec wv;
-        wv.a = acc[c];
-        wv.b = rr[c].b;
-        wv.c = cid[c];
-        st_rec_cg(rec + cx[c], wv);
-        acc[c] += rr[c].a;
-        cx[c] = rr[c].b;
-        if (++hops[c] > n) {
-          set_error(st, KASCADE_ERR_CYCLE, cid[c]);
-          end_chain_on_error(rec_next, cid[c]);
-          act &= ~(1u << c);
-        }
-      } else if (tag_ruler(tg)) {
-        // back at its own ruler: a cycle without a root that holds one ruler
-        // (a valid chain only ends at another ruler)
-        if (tag_id(tg) == cid[c])
-          set_error(st, KASCADE_ERR_CYCLE, cid[c]);
-        else if (has_pred && tag_id(tg) < pred_cap)
-          atomicOr(has_pred + (tag_id(tg) >> 5), 1u << (tag_id(tg) & 31));  // that ruler has a predecessor
-        Rec o;
-        o.a = acc[c];
-        o.b = tag_id(tg);
-        o.c = TAG_UNREACHED;
-        st_rec_cg(rec_next + cid[c], o);
+      if (!((act >> c) & 1u)) continue;
+      const uint32_t x = cx[c], y = rr[c].b;
+      const uint64_t d = acc[c];
+      if (y == x) {  // the list's end (never stamped: any number of chains may end here)
+        end_chain(rec_next, cid[c], d + rr[c].a, cid[c]);
+        rootel_next[cid[c]] = rootel ? __ldg(rootel + x) : x;
         act &= ~(1u << c);
-      } else {
-        // already stamped by another chase: two predecessors
-        set_error(st, KASCADE_ERR_NOT_A_LIST, cx[c]);
-        end_chain_on_error(rec_next, cid[c]);
+        fresh &= ~(1u << c);
+        continue;
+      }
+      const bool start = (fresh >> c) & 1u;
+      fresh &= ~(1u << c);
+      if (!start || cid[c] >= rulers) {
+        if (!tag_unreached(rr[c].c)) {  // stamped by another chain: two predecessors
+          set_error(st, KASCADE_ERR_NOT_A_LIST, x);
+          end_chain(rec_next, cid[c], 0, cid[c]);
+          rootel_next[cid[c]] = 0;
+          act &= ~(1u << c);
+          continue;
+        }
+        Rec wv;
+        wv.a = d;
+        wv.b = y;
+        wv.c = cid[c];
+        st_rec_cg(rec + x, wv);
+      }
+      acc[c] = d + rr[c].a;
+      cx[c] = y;
+      uint32_t j;
+      if (rl.is(y, &j)) {
+        // back at its own ruler: a cycle without a root that holds one ruler
+        if (j == cid[c]) set_error(st, KASCADE_ERR_CYCLE, j);
+        end_chain(rec_next, cid[c], acc[c], j);
+        rootel_next[cid[c]] = 0;
+        act &= ~(1u << c);
+      } else if (++hops[c] > n) {
+        set_error(st, KASCADE_ERR_CYCLE, cid[c]);
+        end_chain(rec_next, cid[c], 0, cid[c]);
+        rootel_next[cid[c]] = 0;
         act &= ~(1u << c);
       }
     }
@@ -444,159 +335,452 @@ __global__ void __launch_bounds__(512) k_chase(Rec* __restrict__ rec, uint32_t n
 // ---------------------------------------------------------------------------
 // propagate: rank(x) = rank(ruler) - distance(ruler, x); elements no chase
 // reached (ahead of their list's first ruler) walk forward to the first
-// stamped element and add the weights they pass.
+// ruler, stamped element or list end and add the weights they pass.  A block
+// collects those and walks them together after its streaming work, one per
+// thread: walked where they are met, each stalled its warp for its whole walk
+// (512 lists in 2.6e7 elements: 2.0 -> 1.7 ms for the whole call).
 // ---------------------------------------------------------------------------
+constexpr uint32_t PROP_WALKS = 512;  // elements a block collects
+
 template <class Sink>
-__global__ void __launch_bounds__(256) k_propagate(const Rec* __restrict__ rec, uint32_t n_out, uint32_t n_all,
-                                                   const uint32_t* __restrict__ n_dev, uint64_t start,
-                                                   const Out* __restrict__ out_next, uint32_t out_cap, Sink sink,
-                                                   DevStatus* st) {
-  // out_cap: entries of out_next.  Only the device-driven recursion can meet
-  // a larger id (a level that outgrew its capacity, already reported as
-  // KASCADE_ERR_TIMEOUT); such elements are skipped.
-  if (n_dev) n_all = n_out = min(*n_dev, n_out);
-  const uint32_t stride = gridDim.x * blockDim.x;
-  const uint64_t pol = l2_keep_policy();
-  for (uint64_t base = start + (uint64_t)blockIdx.x * blockDim.x * PROP_ITEMS + threadIdx.x; base < n_out;
-       base += (uint64_t)stride * PROP_ITEMS) {
-    Rec rv[PROP_ITEMS];
-#pragma unroll
-    for (int i = 0; i < PROP_ITEMS; ++i) {
-      uint64_t x = base + (uint64_t)i * blockDim.x;
-      if (x < n_out) rv[i] = ld_rec_cs(rec + x);
+__device__ __forceinline__ void walk_to_result(const Rec* __restrict__ rec, uint32_t x, uint32_t n_all,
+                                               const Rulers& rl, const uint32_t* __restrict__ rootel,
+                                               const Out* __restrict__ out_next, const Sink& sink, DevStatus* st) {
+  Rec r = ld_rec_cg(rec + x);
+  // Brent's cycle detection keeps an invalid (rootless, ruler-free) cycle to
+  // O(cycle length) steps instead of n per element
+  uint64_t acc = r.a;
+  uint32_t y = r.b, hops = 0, lam = 0, power = 1, mark = x;
+  while (true) {
+    uint32_t id;
+    if (rl.is(y, &id)) {
+      const Out o = ld_out(out_next + id);
+      sink.put(x, acc + o.rank, o.root, false);
+      return;
     }
-    // every stamped element's ruler result, all loads in flight together
-    // (they would otherwise wait behind the previous element's stores)
-    Out ov[PROP_ITEMS];
-#pragma unroll
-    for (int i = 0; i < PROP_ITEMS; ++i) {
-      uint64_t x = base + (uint64_t)i * blockDim.x;
-      ov[i] = Out{0, 0, 0};
-      if (x < n_out && !tag_unreached(rv[i].c)) {
-        const uint32_t id = tag_ruler(rv[i].c) ? tag_id(rv[i].c) : rv[i].c;
-        if (id < out_cap) ov[i] = ld_out_keep(out_next + id, pol);
-      }
+    r = ld_rec_cg(rec + y);
+    if (!tag_unreached(r.c)) {
+      const Out o = ld_out(out_next + r.c);
+      sink.put(x, acc + o.rank - r.a, o.root, false);
+      return;
     }
-#pragma unroll
-    for (int i = 0; i < PROP_ITEMS; ++i) {
-      uint64_t x = base + (uint64_t)i * blockDim.x;
-      if (x >= n_out) continue;
-      Rec r = rv[i];
-      Out o = ov[i];
-      bool is_root = false;
-      uint64_t acc = 0;
-      if (tag_unreached(r.c)) {
-        // Brent's cycle detection keeps an invalid (rootless, ruler-free)
-        // cycle to O(cycle length) steps instead of n per element.
-        uint32_t hops = 0, lam = 0, power = 1, mark = (uint32_t)x;
-        bool cyc = false;
-        while (tag_unreached(r.c)) {
-          acc += r.a;
-          const uint32_t y = r.b;
-          if (y == mark || ++hops > n_all) {
-            cyc = true;
-            break;
-          }
-          if (++lam == power) {
-            mark = y;
-            power <<= 1;
-            lam = 0;
-          }
-          r = ld_rec_cg(rec + y);
-        }
-        if (cyc) {
-          set_error(st, KASCADE_ERR_CYCLE, x);
-          continue;
-        }
-        const uint32_t id = tag_ruler(r.c) ? tag_id(r.c) : r.c;
-        if (id >= out_cap) {
-          set_error(st, KASCADE_ERR_TIMEOUT, id);
-          continue;
-        }
-        o = ld_out(out_next + id);
-      } else {
-        if ((tag_ruler(r.c) ? tag_id(r.c) : r.c) >= out_cap) {
-          set_error(st, KASCADE_ERR_TIMEOUT, x);
-          continue;
-        }
-        if (tag_ruler(r.c)) is_root = (r.b == (uint32_t)x);
-      }
-      uint64_t rank;
-      uint32_t root;
-      if (tag_ruler(r.c)) {
-        rank = o.rank + acc;
-        root = o.root;
-      } else {
-        rank = o.rank - r.a + acc;
-        root = o.root;
-      }
-      sink.put((uint32_t)x, rank, root, is_root);
+    acc += r.a;
+    if (r.b == y) {
+      sink.put(x, acc, rootel ? __ldg(rootel + y) : y, false);
+      return;
     }
+    if (y == mark || ++hops > n_all) {
+      set_error(st, KASCADE_ERR_CYCLE, x);
+      return;
+    }
+    if (++lam == power) {
+      mark = y;
+      power <<= 1;
+      lam = 0;
+    }
+    y = r.b;
   }
 }
 
-// ---------------------------------------------------------------------------
-// base case: one CTA, Wyllie pointer jumping in shared memory.
-// ---------------------------------------------------------------------------
-template <class Sink>
-__global__ void __launch_bounds__(BASE_THREADS) k_base(const Rec* __restrict__ rec, uint32_t n,
-                                                       const uint32_t* __restrict__ elem0, Sink sink,
-                                                       DevStatus* st) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  uint64_t* rk = reinterpret_cast<uint64_t*>(smem);
-  uint32_t* sc = reinterpret_cast<uint32_t*>(smem + 8ull * n);
-  uint8_t* isroot = smem + 12ull * n;
-  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-    Rec r = rec[i];
-    if (r.b >= n) {  // guard: treat as a root and report
-      set_error(st, KASCADE_ERR_OUT_OF_RANGE, i);
-      r.b = i;
+template <class Sink, int ITEMS>
+__global__ void __launch_bounds__(256) k_propagate(const Rec* __restrict__ rec, uint32_t n_out, Extent ext,
+                                                   Rulers rl, uint32_t rulers, const uint32_t* __restrict__ rootel,
+                                                   const Out* __restrict__ out_next, Sink sink, DevStatus* st) {
+  __shared__ uint32_t walks[PROP_WALKS];
+  __shared__ uint32_t nwalks;
+  if (threadIdx.x == 0) nwalks = 0;
+  __syncthreads();
+  const uint32_t n_all = ext.get();  // records exist up to here
+  n_out = min(n_out, n_all);
+  const uint32_t stride = gridDim.x * blockDim.x;
+  const uint64_t pol = l2_keep_policy();
+  for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x * ITEMS + threadIdx.x; base < n_out;
+       base += (uint64_t)stride * ITEMS) {
+    Rec rv[ITEMS];
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+      const uint64_t x = base + (uint64_t)i * blockDim.x;
+      if (x < n_out) rv[i] = ld_rec_cs(rec + x);
     }
-    bool root = (r.b == i);
-    sc[i] = r.b;
-    rk[i] = root ? 0ull : r.a;
-    isroot[i] = root ? 1 : 0;
+    // every ruler's or stamped element's result, all loads in flight together
+    // (they would otherwise wait behind the previous element's stores)
+    Out ov[ITEMS];
+    uint32_t found = 0;  // bit i: ov[i] holds the result of item i's ruler
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+      const uint64_t x = base + (uint64_t)i * blockDim.x;
+      ov[i] = Out{0, 0, 0};
+      if (x >= n_out) continue;
+      uint32_t id;
+      if (rl.is((uint32_t)x, &id) && id < rulers) {  // (a head's index may lie past the last block)
+        rv[i].c = TAG_RULER;
+        found |= 1u << i;
+      } else if (!tag_unreached(rv[i].c)) {
+        id = rv[i].c;
+        found |= 1u << i;
+      }
+      if ((found >> i) & 1u) ov[i] = ld_out_keep(out_next + id, pol);
+    }
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+      const uint64_t x = base + (uint64_t)i * blockDim.x;
+      if (x >= n_out) continue;
+      const Rec r = rv[i];
+      const bool is_root = r.b == (uint32_t)x && (r.c == TAG_RULER || tag_unreached(r.c));
+      if ((found >> i) & 1u) {
+        sink.put((uint32_t)x, ov[i].rank - (r.c == TAG_RULER ? 0ull : r.a), ov[i].root, is_root);
+      } else if (is_root) {
+        sink.put((uint32_t)x, r.a, rootel ? __ldg(rootel + x) : (uint32_t)x, true);
+      } else {
+        const uint32_t w = atomicAdd(&nwalks, 1u);
+        if (w < PROP_WALKS)
+          walks[w] = (uint32_t)x;
+        else
+          walk_to_result(rec, (uint32_t)x, n_all, rl, rootel, out_next, sink, st);
+      }
+    }
   }
   __syncthreads();
-  int round = 0;
+  for (uint32_t w = threadIdx.x; w < min(nwalks, PROP_WALKS); w += blockDim.x)
+    walk_to_result(rec, walks[w], n_all, rl, rootel, out_next, sink, st);
+}
+
+// ---------------------------------------------------------------------------
+// One CTA ranks up to ONE_CTA_MAX elements in shared memory: the last level
+// of the recursion, or a whole small input straight from the caller's arrays.
+// The elements are loaded once; at most CTA_RULERS rulers (placed as on every
+// level) walk and stamp as in k_chase, pointer jumping ranks the rulers
+// (<= 10 rounds), and every element reads its ruler's result.  Against
+// pointer jumping over all elements (13 rounds of 16 elements per thread at
+// 8192: 51 us) each element is touched once.  Each element's word also says
+// whether its successor is a ruler or a list's end, so a hop is one exchange.
+// With several lists, their heads (no predecessor) start chains as well, so
+// that no run of elements ahead of a first ruler is walked element by element.
+// Two chains that meet (a tree, not a list) are found by the exchange; an
+// input of at most `tree_max` elements is then done again without stamps,
+// every element walking to its first ruler, which ranks any forest.
+// ---------------------------------------------------------------------------
+constexpr uint32_t CTA_THREADS = 1024;
+constexpr uint32_t CTA_RULERS = 1024;
+constexpr uint32_t CTA_HEADS = 1024;
+constexpr uint32_t CTA_CHAINS = CTA_RULERS / CTA_THREADS;
+constexpr uint32_t CTA_LOADS = 8;           // elements a thread has in flight while loading
+constexpr uint32_t CTA_ILP = 4;             // elements a thread has in flight in shared memory
+constexpr uint32_t CTA_FLAG = 0x80000000u;  // next: stamped, low bits the chain; rnext: the list's end
+constexpr uint32_t CTA_END = 0x40000000u;   // next: the successor ends the list
+constexpr uint32_t CTA_RUL = 0x20000000u;   // next: the successor is a ruler
+constexpr uint32_t CTA_IDX = 0x1FFFFFFFu;
+constexpr size_t cta_smem(uint64_t n) {
+  return (size_t)((n + CTA_RULERS + CTA_HEADS) * 12 + CTA_HEADS * 2 + (n + 31) / 32 * 4);
+}
+
+// Element sources: the records of a level (a list end's carries its rank), or
+// the caller's arrays (a root's weight is no part of any rank).
+struct CtaRecords {
+  static constexpr bool kEndWeight = true;
+  const Rec* rec;
+  const uint32_t* rootel;
+  __device__ __forceinline__ void load(uint32_t x, uint64_t* a, uint32_t* b) const {
+    const Rec r = ld_rec_cg(rec + x);
+    *a = r.a;
+    *b = r.b;
+  }
+  __device__ __forceinline__ uint32_t root_of(uint32_t x) const { return rootel ? __ldg(rootel + x) : x; }
+};
+template <class W>
+struct CtaArrays {
+  static constexpr bool kEndWeight = false;
+  const uint64_t* succ;
+  W w;
+  __device__ __forceinline__ void load(uint32_t x, uint64_t* a, uint32_t* b) const {
+    const unsigned long long s = __ldcg(reinterpret_cast<const unsigned long long*>(succ) + x);
+    *a = w(x);
+    *b = s > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)s;  // beyond any element: found out of range
+  }
+  __device__ __forceinline__ uint32_t root_of(uint32_t x) const { return x; }
+};
+
+template <class Src, class Sink>
+__global__ void __launch_bounds__(CTA_THREADS, 1) k_rank_cta(Src src, Extent ext, Sink sink, uint32_t tree_max,
+                                                             int level0, DevStatus* st) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ uint32_t nends, nheads;
+  const uint32_t n = ext.get();
+  unsigned long long* dist = reinterpret_cast<unsigned long long*>(smem);  // weight, once stamped the distance
+  unsigned long long* rdist = dist + ext.cap;                              // per chain: distance, then rank
+  uint32_t* next = reinterpret_cast<uint32_t*>(rdist + CTA_RULERS + CTA_HEADS);
+  uint32_t* rnext = next + ext.cap;  // per chain: next ruler or CTA_FLAG | list end, then the root
+  uint32_t* pred = rnext + CTA_RULERS + CTA_HEADS;
+  uint16_t* hlist = reinterpret_cast<uint16_t*>(pred + (ext.cap + 31) / 32);
+  const uint32_t tid = threadIdx.x;
+  const uint32_t words = (n + 31) / 32;
+  if (level0 && ext.add && tid == 0) st->counter[1] = n;
+  const bool all = n <= CTA_RULERS;  // every element is a ruler
+  const Rulers rl = make_rulers((n + CTA_RULERS - 1) / CTA_RULERS, 0x63746121u);
+  const uint32_t rulers = all ? n : (n + rl.s - 1) / rl.s;
+  auto ruler = [&](uint32_t x, uint32_t* j) {
+    if (all) {
+      *j = x;
+      return true;
+    }
+    return rl.is(x, j);
+  };
+  bool stamp = true;
+  uint32_t heads = 0;
   while (true) {
-    uint32_t ns[BASE_PER_THREAD];
-    uint64_t nr[BASE_PER_THREAD];
-    int changed = 0;
+    if (tid == 0) nends = nheads = 0;
+    for (uint32_t w = tid; w < words; w += CTA_THREADS) pred[w] = 0;
+    __syncthreads();
+    uint32_t ends = 0;
+    for (uint32_t x0 = tid; x0 < n; x0 += CTA_THREADS * CTA_LOADS) {
+      uint64_t a[CTA_LOADS];
+      uint32_t b[CTA_LOADS];
 #pragma unroll
-    for (int j = 0; j < BASE_PER_THREAD; ++j) {
-      uint32_t i = threadIdx.x + j * blockDim.x;
-      if (i < n) {
-        uint32_t s = sc[i];
-        if (!isroot[s]) {
-          ns[j] = sc[s];
-          nr[j] = rk[i] + rk[s];
-          changed = 1;
-        } else {
-          ns[j] = s;
-          nr[j] = rk[i];
+      for (uint32_t i = 0; i < CTA_LOADS; ++i) {
+        const uint32_t x = x0 + i * CTA_THREADS;
+        if (x < n) src.load(x, &a[i], &b[i]);
+      }
+#pragma unroll
+      for (uint32_t i = 0; i < CTA_LOADS; ++i) {
+        const uint32_t x = x0 + i * CTA_THREADS;
+        if (x >= n) continue;
+        if (b[i] >= n) {
+          set_error(st, KASCADE_ERR_OUT_OF_RANGE, x);
+          b[i] = x;
         }
+        dist[x] = (Src::kEndWeight || b[i] != x) ? a[i] : 0ull;
+        next[x] = b[i];
+        ends += b[i] == x ? 1u : 0u;
+      }
+    }
+    ends = __reduce_add_sync(FULL, ends);
+    if ((tid & 31u) == 0 && ends) atomicAdd(&nends, ends);
+    __syncthreads();
+    // what each successor is; with several lists, who has a predecessor
+    const bool many = stamp && !all && nends > 2;
+    for (uint32_t x0 = tid; x0 < n; x0 += CTA_THREADS * CTA_ILP) {
+      uint32_t y[CTA_ILP], z[CTA_ILP];
+#pragma unroll
+      for (uint32_t i = 0; i < CTA_ILP; ++i) {
+        const uint32_t x = x0 + i * CTA_THREADS;
+        y[i] = x < n ? next[x] : x;
+      }
+#pragma unroll
+      for (uint32_t i = 0; i < CTA_ILP; ++i) z[i] = x0 + i * CTA_THREADS < n ? next[y[i]] & CTA_IDX : 0u;
+#pragma unroll
+      for (uint32_t i = 0; i < CTA_ILP; ++i) {
+        const uint32_t x = x0 + i * CTA_THREADS;
+        uint32_t j;
+        if (x >= n || y[i] == x) continue;
+        next[x] = y[i] | (z[i] == y[i] ? CTA_END : 0u) | (ruler(y[i], &j) ? CTA_RUL : 0u);
+        if (many) atomicOr(&pred[y[i] >> 5], 1u << (y[i] & 31));
       }
     }
     __syncthreads();
+    if (many) {
+      for (uint32_t w = tid; w < words; w += CTA_THREADS) {
+        uint32_t m = ~pred[w];
+        while (m) {
+          const uint32_t x = w * 32 + (uint32_t)__ffs(m) - 1;
+          m &= m - 1;
+          uint32_t j;
+          if (x >= n || next[x] == x || rl.is(x, &j)) continue;
+          const uint32_t e = atomicAdd(&nheads, 1u);
+          if (e < CTA_HEADS) hlist[e] = (uint16_t)x;
+        }
+      }
+      __syncthreads();
+      heads = min(nheads, CTA_HEADS);
+    }
+    // chains: ids of rulers, then (from CTA_RULERS on) of heads; a thread's
+    // chains go hop by hop together
+    uint32_t id[CTA_CHAINS], cur[CTA_CHAINS], hops = 0, act = 0;
+    unsigned long long acc[CTA_CHAINS];
+    int clash = 0;
+    // the chain has passed acc and its next word is f: at its end, or at cur
+    auto arrive = [&](uint32_t c, uint32_t f) {
+      const uint32_t y = f & CTA_IDX;
+      if (f & CTA_RUL) {
+        rdist[id[c]] = acc[c];
+        rnext[id[c]] = all ? y : rl.block_of(y);
+        return false;
+      }
+      if (f & CTA_END) {
+        rdist[id[c]] = acc[c] + dist[y];
+        rnext[id[c]] = CTA_FLAG | y;
+        return false;
+      }
+      cur[c] = y;
+      return true;
+    };
+    auto begin = [&](uint32_t c) {
+      uint32_t x0 = n;
+      if (id[c] < rulers)
+        x0 = all ? id[c] : (uint32_t)rl.elem(id[c]);
+      else if (id[c] >= CTA_RULERS && id[c] - CTA_RULERS < heads)
+        x0 = hlist[id[c] - CTA_RULERS];
+      if (x0 >= n) return false;
+      const uint32_t f = next[x0];
+      acc[c] = dist[x0];
+      if (f == x0) {
+        rdist[id[c]] = acc[c];
+        rnext[id[c]] = CTA_FLAG | x0;
+        return false;
+      }
+      if (id[c] >= CTA_RULERS) {  // a head is stamped by its own chain
+        next[x0] = CTA_FLAG | id[c];
+        dist[x0] = 0;
+      }
+      return arrive(c, f);
+    };
 #pragma unroll
-    for (int j = 0; j < BASE_PER_THREAD; ++j) {
-      uint32_t i = threadIdx.x + j * blockDim.x;
-      if (i < n) {
-        sc[i] = ns[j];
-        rk[i] = nr[j];
+    for (uint32_t c = 0; c < CTA_CHAINS; ++c) {
+      id[c] = tid + c * CTA_THREADS;
+      cur[c] = 0;
+      acc[c] = 0;
+      bool on = begin(c);
+      if (!on && heads) {
+        id[c] += CTA_RULERS;
+        on = begin(c);
+      }
+      if (on) act |= 1u << c;
+    }
+    while (act) {
+      ++hops;
+#pragma unroll
+      for (uint32_t c = 0; c < CTA_CHAINS; ++c) {
+        if (!((act >> c) & 1u)) continue;
+        const uint32_t x = cur[c];
+        const uint32_t f = stamp ? atomicExch(&next[x], CTA_FLAG | id[c]) : next[x];
+        bool on = false;
+        if ((f & CTA_FLAG) || hops > 2 * n) {
+          // two chains met, or a cycle without a ruler
+          if (f & CTA_FLAG) clash = 1;
+          rdist[id[c]] = 0;
+          rnext[id[c]] = id[c];  // never ends: the rounds below report the cycle
+        } else {
+          const unsigned long long w = dist[x];
+          if (stamp) dist[x] = acc[c];
+          acc[c] += w;
+          on = arrive(c, f);
+        }
+        if (!on && id[c] < CTA_RULERS && heads) {
+          id[c] += CTA_RULERS;
+          on = begin(c);
+        }
+        if (!on) act &= ~(1u << c);
       }
     }
-    if (!__syncthreads_or(changed)) break;
-    if (++round > 40) {
-      if (threadIdx.x == 0) set_error(st, KASCADE_ERR_CYCLE, 0);
-      break;
+    clash = __syncthreads_or(clash);
+    if (!clash) break;
+    if (n > tree_max) {
+      if (tid == 0) set_error(st, KASCADE_ERR_NOT_A_LIST, n);
+      return;
+    }
+    stamp = false;  // again from the source, without stamps
+    heads = 0;
+  }
+  // pointer jumping over the rulers
+  for (int round = 0;; ++round) {
+    unsigned long long d[CTA_CHAINS];
+    uint32_t nx[CTA_CHAINS];
+    int busy = 0;
+#pragma unroll
+    for (uint32_t c = 0; c < CTA_CHAINS; ++c) {
+      const uint32_t j = tid + c * CTA_THREADS;
+      nx[c] = CTA_FLAG;
+      d[c] = 0;
+      if (j >= rulers || (!all && rl.elem(j) >= n)) continue;
+      nx[c] = rnext[j];
+      d[c] = rdist[j];
+      if (!(nx[c] & CTA_FLAG)) {
+        d[c] += rdist[nx[c]];
+        nx[c] = rnext[nx[c]];
+        busy = 1;
+      }
+    }
+    if (!__syncthreads_or(busy)) break;
+    if (round > 11) {  // 2^11 > CTA_RULERS: what has not ended by now never does
+      if (tid == 0) set_error(st, KASCADE_ERR_CYCLE, n);
+      return;
+    }
+#pragma unroll
+    for (uint32_t c = 0; c < CTA_CHAINS; ++c) {
+      const uint32_t j = tid + c * CTA_THREADS;
+      if (j >= rulers || (!all && rl.elem(j) >= n)) continue;
+      rdist[j] = d[c];
+      rnext[j] = nx[c];
+    }
+    __syncthreads();
+  }
+  // the heads' chains end at a ruler or a list end; then every chain's root
+  for (uint32_t h = tid; h < heads; h += CTA_THREADS) {
+    const uint32_t j = CTA_RULERS + h, nx = rnext[j];
+    if (!(nx & CTA_FLAG)) {
+      rdist[j] += rdist[nx];
+      rnext[j] = rnext[nx];
     }
   }
-  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-    uint32_t rt = sc[i];
-    if (elem0) rt = elem0[rt];
-    sink.put(i, rk[i], rt, isroot[i] != 0);
+  __syncthreads();
+  for (uint32_t j = tid; j < CTA_RULERS + heads; j += CTA_THREADS)
+    if (j < rulers ? (all || rl.elem(j) < n) : j >= CTA_RULERS) rnext[j] = src.root_of(rnext[j] & ~CTA_FLAG);
+  __syncthreads();
+  for (uint32_t x0 = tid; x0 < n; x0 += CTA_THREADS * CTA_ILP) {
+    uint32_t f[CTA_ILP], j[CTA_ILP];
+    unsigned long long d[CTA_ILP];
+#pragma unroll
+    for (uint32_t i = 0; i < CTA_ILP; ++i) {
+      const uint32_t x = x0 + i * CTA_THREADS;
+      f[i] = x < n ? next[x] : 0u;
+      d[i] = x < n ? dist[x] : 0ull;
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < CTA_ILP; ++i) {
+      const uint32_t x = x0 + i * CTA_THREADS;
+      if (x >= n) continue;
+      const bool end = f[i] == x;
+      uint32_t root = 0;
+      if (ruler(x, &j[i])) {
+        d[i] = rdist[j[i]];
+        root = rnext[j[i]];
+      } else if (f[i] & CTA_FLAG) {
+        d[i] = rdist[f[i] & CTA_IDX] - d[i];
+        root = rnext[f[i] & CTA_IDX];
+      } else if (end) {
+        root = src.root_of(x);
+      } else {  // ahead of its list's first ruler: walk
+        uint32_t hops = 0, w = f[i];
+        bool ok = true;
+        while (true) {
+          const uint32_t y = w & CTA_IDX;
+          if (w & CTA_RUL) {
+            const uint32_t k = all ? y : rl.block_of(y);
+            d[i] += rdist[k];
+            root = rnext[k];
+            break;
+          }
+          if (w & CTA_END) {
+            d[i] += dist[y];
+            root = src.root_of(y);
+            break;
+          }
+          w = next[y];
+          if (w & CTA_FLAG) {
+            d[i] += rdist[w & CTA_IDX] - dist[y];
+            root = rnext[w & CTA_IDX];
+            break;
+          }
+          d[i] += dist[y];
+          if (++hops > n) {
+            set_error(st, KASCADE_ERR_CYCLE, x);
+            ok = false;
+            break;
+          }
+        }
+        if (!ok) continue;
+      }
+      sink.put(x, d[i], root, end);
+    }
   }
 }
 
@@ -604,10 +788,9 @@ __global__ void __launch_bounds__(BASE_THREADS) k_base(const Rec* __restrict__ r
 // pointer doubling: double-buffered jump rounds over 16 B records.
 // done bit 0: successor is a root; bit 1: the element is a root.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_pd_init(const Rec* __restrict__ rec, uint32_t n,
-                                                 const uint32_t* __restrict__ n_dev, PdRec* __restrict__ a,
-                                                 DevStatus* st) {
-  if (n_dev) n = min(*n_dev, n);
+__global__ void __launch_bounds__(256) k_pd_init(const Rec* __restrict__ rec, Extent ext,
+                                                 PdRec* __restrict__ a, DevStatus* st) {
+  const uint32_t n = ext.get();
   for (uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (uint64_t)gridDim.x * blockDim.x) {
     Rec r = rec[x];
     if (r.b >= n) {  // guard: treat as a root and report
@@ -616,7 +799,7 @@ __global__ void __launch_bounds__(256) k_pd_init(const Rec* __restrict__ rec, ui
     }
     bool root = (r.b == (uint32_t)x);
     PdRec p;
-    p.rank = root ? 0ull : r.a;
+    p.rank = r.a;  // a list end's record holds its own rank: 0 on level 0
     p.succ = r.b;
     p.done = root ? 3u : 0u;
     a[x] = p;
@@ -630,9 +813,9 @@ __global__ void __launch_bounds__(256) k_pd_init(const Rec* __restrict__ rec, ui
 // of the device-driven recursion (at most 2^17 elements, L2-resident, a fixed
 // number of launches) takes JUMPS = 3: half the launches for three reads each.
 template <int JUMPS>
-__global__ void __launch_bounds__(256) k_pd_round(const PdRec* __restrict__ a, PdRec* __restrict__ b, uint32_t n,
-                                                  const uint32_t* __restrict__ n_dev, uint32_t* __restrict__ active) {
-  if (n_dev) n = min(*n_dev, n);
+__global__ void __launch_bounds__(256) k_pd_round(const PdRec* __restrict__ a, PdRec* __restrict__ b, Extent ext,
+                                                  uint32_t* __restrict__ active) {
+  const uint32_t n = ext.get();
   uint32_t cnt = 0;
   for (uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (uint64_t)gridDim.x * blockDim.x) {
     PdRec e = a[x];
@@ -653,10 +836,9 @@ __global__ void __launch_bounds__(256) k_pd_round(const PdRec* __restrict__ a, P
 }
 
 template <class Sink>
-__global__ void __launch_bounds__(256) k_pd_final(const PdRec* __restrict__ a, uint32_t n,
-                                                  const uint32_t* __restrict__ n_dev,
+__global__ void __launch_bounds__(256) k_pd_final(const PdRec* __restrict__ a, Extent ext,
                                                   const uint32_t* __restrict__ elem0, Sink sink) {
-  if (n_dev) n = min(*n_dev, n);
+  const uint32_t n = ext.get();
   for (uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (uint64_t)gridDim.x * blockDim.x) {
     PdRec e = a[x];
     uint32_t rt = e.succ;
@@ -667,20 +849,10 @@ __global__ void __launch_bounds__(256) k_pd_final(const PdRec* __restrict__ a, u
 
 // After a fixed number of rounds every element must point at a root; one that
 // does not sits on a rootless cycle.
-__global__ void __launch_bounds__(256) k_pd_check(const PdRec* __restrict__ a, uint32_t n,
-                                                  const uint32_t* __restrict__ n_dev, DevStatus* st) {
-  if (n_dev) n = min(*n_dev, n);
+__global__ void __launch_bounds__(256) k_pd_check(const PdRec* __restrict__ a, Extent ext, DevStatus* st) {
+  const uint32_t n = ext.get();
   for (uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (uint64_t)gridDim.x * blockDim.x)
     if (!(a[x].done & 1u)) set_error(st, KASCADE_ERR_CYCLE, x);
-}
-
-// A level's size (device) against its capacity: more means the device-driven
-// recursion cannot hold it; the caller reruns on the host-driven path.
-__global__ void k_check_count(const uint32_t* __restrict__ cnt, uint32_t cap, uint32_t* __restrict__ copy,
-                              DevStatus* st) {
-  const uint32_t c = *cnt;
-  if (copy) *copy = c;
-  if (c > cap) set_error(st, KASCADE_ERR_TIMEOUT, c);
 }
 
 // ---------------------------------------------------------------------------
@@ -712,99 +884,108 @@ int occupancy(K kernel, int block, size_t smem) {
   return nb < 1 ? 1 : nb;
 }
 
+// Resident blocks per SM of the chase, by chains per thread and block size.
 template <int C>
-kascade_status launch_chase_c(kascade_ctx& ctx, Rec* rec, uint32_t n, const uint32_t* ruler_elem, uint32_t r,
-                              Rec* rec_next, uint32_t* work, uint32_t block, cudaStream_t s) {
-  static int occ[3] = {-1, -1, -1};  // blocks of 128, 256, 512 threads
+int chase_occupancy(uint32_t block) {
+  static std::atomic<int> occ[3] = {{-1}, {-1}, {-1}};  // blocks of 128, 256, 512 threads
   const int bi = block == 128 ? 0 : block == 512 ? 2 : 1;
-  if (occ[bi] < 0) occ[bi] = occupancy(k_chase<C>, (int)block, 0);
-  unsigned grid = (unsigned)(ctx.usable_sms() * occ[bi]);
-  const uint64_t warps_per_block = block / 32;
-  uint64_t need = ((uint64_t)r + 32ull * C - 1) / (32ull * C);  // warps worth of work
-  uint64_t need_blocks = (need + warps_per_block - 1) / warps_per_block;
-  if (need_blocks < grid) grid = (unsigned)(need_blocks ? need_blocks : 1);
+  int v = occ[bi].load();
+  if (v < 0) occ[bi].store(v = occupancy(k_chase<C>, (int)block, 0));
+  return v;
+}
+
+// Warps that share a level's rulers before a warp works with more lanes: the
+// L2 serves dependent hops of this many resident warps at full speed.
+constexpr uint64_t CHASE_SPREAD_WARPS_PER_SM = 32;
+
+template <int C>
+kascade_status launch_chase_c(kascade_ctx& ctx, const Levels& lv, int k, const Extent& ext, uint32_t block,
+                              cudaStream_t s) {
+  const uint32_t r = lv.n[k + 1];
+  const uint64_t wpb = block / 32;
+  const uint64_t max_grid = (uint64_t)ctx.usable_sms() * chase_occupancy<C>(block);
+  const uint64_t spread = std::min<uint64_t>(max_grid * wpb, (uint64_t)ctx.usable_sms() * CHASE_SPREAD_WARPS_PER_SM);
+  const uint32_t lanes = (uint32_t)std::min<uint64_t>(32, std::max<uint64_t>(1, (r + spread * C - 1) / (spread * C)));
+  const uint64_t need = ((uint64_t)r + lanes * C - 1) / (lanes * C);  // warps worth of work
+  const unsigned grid = (unsigned)std::min<uint64_t>(max_grid, (need + wpb - 1) / wpb);
   ProfScope ps(ctx, "chase", s);
-  k_chase<C><<<grid, block, 0, s>>>(rec, n, nullptr, ruler_elem, r, nullptr, rec_next, work, nullptr, ctx.d_status);
+  k_chase<C><<<grid, block, 0, s>>>(lv.rec[k], ext, lv.rulers[k], lv.r[k], lv.heads, k ? lv.r[k - 1] : 0u,
+                                    lv.rootel[k], lv.rec[k + 1], lv.rootel[k + 1], &ctx.d_status->work[k], lanes,
+                                    ctx.d_status);
   KS_CHECK_LAUNCH();
   return KASCADE_OK;
 }
 
-kascade_status launch_chase(kascade_ctx& ctx, Rec* rec, uint32_t n, const uint32_t* ruler_elem, uint32_t r,
-                            Rec* rec_next, const Params& p, cudaStream_t s) {
-  uint32_t* work = alloc<uint32_t>(ctx, 1);
-  if (!work) return KASCADE_ERR_OOM;
-  KS_CUDA(cudaMemsetAsync(work, 0, sizeof(uint32_t), s));
-  switch (p.chains) {
+// Level k's chase (k = 0: the caller's records).
+kascade_status launch_chase(kascade_ctx& ctx, const Levels& lv, int k, const Extent& ext, uint32_t chains,
+                            uint32_t block, cudaStream_t s) {
+  switch (chains) {
     case 1:
-      return launch_chase_c<1>(ctx, rec, n, ruler_elem, r, rec_next, work, p.block, s);
+      return launch_chase_c<1>(ctx, lv, k, ext, block, s);
     case 4:
-      return launch_chase_c<4>(ctx, rec, n, ruler_elem, r, rec_next, work, p.block, s);
+      return launch_chase_c<4>(ctx, lv, k, ext, block, s);
     default:
-      return launch_chase_c<2>(ctx, rec, n, ruler_elem, r, rec_next, work, p.block, s);
+      return launch_chase_c<2>(ctx, lv, k, ext, block, s);
   }
 }
 
-// Chase with sizes in device memory: n and r are the capacities.
-template <int C>
-kascade_status launch_chase_dev_c(kascade_ctx& ctx, Rec* rec, uint32_t n, const uint32_t* n_dev,
-                                  const uint32_t* ruler_elem, uint32_t r, const uint32_t* r_dev, Rec* rec_next,
-                                  uint32_t* work, uint32_t* has_pred, uint32_t block, cudaStream_t s) {
-  static int occ[3] = {-1, -1, -1};
-  const int bi = block == 128 ? 0 : block == 512 ? 2 : 1;
-  if (occ[bi] < 0) occ[bi] = occupancy(k_chase<C>, (int)block, 0);
-  unsigned grid = (unsigned)(ctx.usable_sms() * occ[bi]);
-  const uint64_t warps_per_block = block / 32;
-  const uint64_t need = ((uint64_t)r + 32ull * C - 1) / (32ull * C);
-  const uint64_t need_blocks = (need + warps_per_block - 1) / warps_per_block;
-  if (need_blocks < grid) grid = (unsigned)(need_blocks ? need_blocks : 1);
-  ProfScope ps(ctx, "chase", s);
-  k_chase<C><<<grid, block, 0, s>>>(rec, n, n_dev, ruler_elem, r, r_dev, rec_next, work, has_pred, ctx.d_status);
-  KS_CHECK_LAUNCH();
-  return KASCADE_OK;
-}
-
-kascade_status launch_chase_dev(kascade_ctx& ctx, Rec* rec, uint32_t n, const uint32_t* n_dev,
-                                const uint32_t* ruler_elem, uint32_t r, const uint32_t* r_dev, Rec* rec_next,
-                                uint32_t* work, uint32_t* has_pred, const Params& p, cudaStream_t s) {
-  switch (p.chains) {
-    case 1:
-      return launch_chase_dev_c<1>(ctx, rec, n, n_dev, ruler_elem, r, r_dev, rec_next, work, has_pred, p.block, s);
-    case 4:
-      return launch_chase_dev_c<4>(ctx, rec, n, n_dev, ruler_elem, r, r_dev, rec_next, work, has_pred, p.block, s);
-    default:
-      return launch_chase_dev_c<2>(ctx, rec, n, n_dev, ruler_elem, r, r_dev, rec_next, work, has_pred, p.block, s);
-  }
-}
-
+// Level k's results from level k + 1's.  Small levels take two elements per
+// thread instead of eight, so that they fill the chip.
 template <class Sink>
-kascade_status launch_propagate(kascade_ctx& ctx, const Rec* rec, uint32_t n_out, uint32_t n_all, const Out* out_next,
-                                uint32_t out_cap, const Sink& sink, cudaStream_t s) {
+kascade_status launch_propagate(kascade_ctx& ctx, const Levels& lv, int k, uint32_t n_out, const Extent& ext,
+                                const Sink& sink, cudaStream_t s) {
   ProfScope ps(ctx, "propagate", s);
-  const unsigned grid = grid_for(ctx, ((uint64_t)n_out + PROP_ITEMS - 1) / PROP_ITEMS, 256, 8);
-  k_propagate<Sink><<<grid, 256, 0, s>>>(rec, n_out, n_all, nullptr, 0, out_next, out_cap, sink, ctx.d_status);
+  if (n_out <= (uint64_t)ctx.usable_sms() * 256 * 8 * 4) {
+    const unsigned grid = grid_for(ctx, ((uint64_t)n_out + 1) / 2, 256, 8);
+    k_propagate<Sink, 2><<<grid, 256, 0, s>>>(lv.rec[k], n_out, ext, lv.rulers[k], lv.r[k], lv.rootel[k],
+                                              lv.out[k + 1], sink, ctx.d_status);
+  } else {
+    const unsigned grid = grid_for(ctx, ((uint64_t)n_out + 7) / 8, 256, 8);
+    k_propagate<Sink, 8><<<grid, 256, 0, s>>>(lv.rec[k], n_out, ext, lv.rulers[k], lv.r[k], lv.rootel[k],
+                                              lv.out[k + 1], sink, ctx.d_status);
+  }
   KS_CHECK_LAUNCH();
   return KASCADE_OK;
 }
 
-template <class Sink>
-kascade_status launch_base(kascade_ctx& ctx, const Rec* rec, uint32_t n, const uint32_t* elem0, const Sink& sink,
-                           cudaStream_t s) {
-  if (n == 0) return KASCADE_OK;
-  size_t smem = 13ull * n + 16;
-  static bool configured = false;
-  if (!configured) {
-    KS_CUDA(cudaFuncSetAttribute(k_base<Sink>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(13 * BASE_THREADS * BASE_PER_THREAD + 16)));
-    configured = true;
+template <class Src, class Sink>
+kascade_status launch_rank_cta(kascade_ctx& ctx, const Src& src, const Extent& ext, const Sink& sink,
+                               uint32_t tree_max, int level0, cudaStream_t s) {
+  static std::atomic<uint64_t> raised{0};  // kernel attributes are per device
+  const uint64_t bit = 1ull << (ctx.device & 63);
+  if (!(raised.load() & bit)) {
+    KS_CUDA(cudaFuncSetAttribute(k_rank_cta<Src, Sink>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)cta_smem(ONE_CTA_MAX)));
+    raised.fetch_or(bit);
   }
   ProfScope ps(ctx, "base_case", s);
-  k_base<Sink><<<1, BASE_THREADS, smem, s>>>(rec, n, elem0, sink, ctx.d_status);
+  k_rank_cta<Src, Sink><<<1, CTA_THREADS, cta_smem(ext.cap), s>>>(src, ext, sink, tree_max, level0, ctx.d_status);
   KS_CHECK_LAUNCH();
   return KASCADE_OK;
 }
 
-kascade_status rank_deep(kascade_ctx& ctx, Rec* rec, uint32_t n, const uint32_t* elem0, const SinkOut& sink,
-                         int level, const Params& p, cudaStream_t s);
+// Ruler spacing of a deeper level of n elements: levels of equal spacing down
+// to the one-CTA size, as many as cost least.  A level costs its longest
+// chain, spacing x ln(rulers) dependent hops, and launches worth ~36 hops
+// (measured on L2-resident levels: 0.25 us a hop, ~9 us for a level's chase
+// and propagation launches).
+uint32_t deep_spacing(uint32_t n, uint32_t target) {
+  uint32_t best = 4;
+  double best_cost = 1e300;
+  for (int levels = 1; levels <= 8; ++levels) {
+    const double sp = std::max(4.0, std::ceil(std::pow((double)n / target, 1.0 / levels)));
+    double cost = 36.0 * levels, m = n;
+    for (int i = 0; i < levels; ++i) {
+      m = std::max(2.0, m / sp);
+      cost += sp * std::log(m);
+    }
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = (uint32_t)sp;
+    }
+  }
+  return best;
+}
 
 }  // namespace
 
@@ -837,74 +1018,76 @@ Params make_params(const kascade_ctx& ctx, const kascade_opts* o, uint64_t n) {
       p.max_chain = o->max_chain;
     }
   }
-  if (p.base_max > (uint32_t)(BASE_THREADS * BASE_PER_THREAD)) p.base_max = BASE_THREADS * BASE_PER_THREAD;
+  if (p.base_max > ONE_CTA_MAX) p.base_max = ONE_CTA_MAX;
   if (p.block != 128 && p.block != 512) p.block = 256;
   if (p.spacing0 < 2) p.spacing0 = 2;
-  if (p.spacing_deep < 2) p.spacing_deep = 2;
+  if (p.spacing_deep == 1) p.spacing_deep = 2;
   return p;
 }
 
 kascade_status prepare_arrays(kascade_ctx& ctx, const uint64_t* succ, WKind wk, const void* w, uint32_t n, Rec* rec,
-                              uint32_t* ruler_elem, uint32_t* r_out, const Params& p, cudaStream_t s,
-                              uint32_t** r_dev) {
-  uint32_t* ctr = alloc<uint32_t>(ctx, 1);
-  if (!ctr) return KASCADE_ERR_OOM;
-  if (r_dev) *r_dev = ctr;
-  KS_CUDA(cudaMemsetAsync(ctr, 0, sizeof(uint32_t), s));
-  uint32_t salt = salt_for(p.seed, 0), th = thresh_for(p.spacing0);
-  {
-    ProfScope ps(ctx, "prepare", s);
-    // full tiles of 16 B-aligned inputs go through the bulk-copy kernel
-    uint64_t start = 0;
-    const bool aligned = (reinterpret_cast<uintptr_t>(succ) % 16 == 0) &&
-                         (wk == WKind::Unit || (wk == WKind::U32 && reinterpret_cast<uintptr_t>(w) % 16 == 0));
-    const uint32_t ntiles = n / PT_TILE;
-    if (aligned && ntiles >= (uint32_t)ctx.usable_sms()) {
-      const unsigned g = (unsigned)std::min<uint64_t>(ntiles, (uint64_t)ctx.usable_sms() * 2);
-      if (wk == WKind::U32) {
-        constexpr int smem = PT_STAGES * PT_TILE * 12;
-        static bool raised = false;
-        if (!raised) {
-          KS_CUDA(cudaFuncSetAttribute(k_prepare_tma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-          raised = true;
-        }
-        k_prepare_tma<true><<<g, 256, smem, s>>>(succ, (const uint32_t*)w, n, ntiles, rec, ruler_elem, ctr, salt, th,
-                                                 ctx.d_status);
-      } else {
-        constexpr int smem = PT_STAGES * PT_TILE * 8;
-        static bool raised = false;
-        if (!raised) {
-          KS_CUDA(cudaFuncSetAttribute(k_prepare_tma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-          raised = true;
-        }
-        k_prepare_tma<false><<<g, 256, smem, s>>>(succ, nullptr, n, ntiles, rec, ruler_elem, ctr, salt, th,
-                                                  ctx.d_status);
+                              const Params& p, cudaStream_t s) {
+  (void)p;
+  ProfScope ps(ctx, "prepare", s);
+  // full tiles of 16 B-aligned inputs go through the bulk-copy kernel
+  uint64_t start = 0;
+  const bool aligned = (reinterpret_cast<uintptr_t>(succ) % 16 == 0) &&
+                       (wk == WKind::Unit || (wk == WKind::U32 && reinterpret_cast<uintptr_t>(w) % 16 == 0));
+  const uint32_t ntiles = n / PT_TILE;
+  if (aligned && ntiles >= (uint32_t)ctx.usable_sms()) {
+    const unsigned g = (unsigned)std::min<uint64_t>(ntiles, (uint64_t)ctx.usable_sms() * 2);
+    if (wk == WKind::U32) {
+      constexpr int smem = PT_STAGES * PT_TILE * 12;
+      static bool raised = false;
+      if (!raised) {
+        KS_CUDA(cudaFuncSetAttribute(k_prepare_tma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        raised = true;
       }
-      KS_CHECK_LAUNCH();
-      start = (uint64_t)ntiles * PT_TILE;
-    }
-    if (start < n) {
-      const uint64_t rest = n - start;
-      const unsigned grid = grid_for(ctx, (rest + 256 * PREP_ITEMS - 1) / (256 * PREP_ITEMS) * 256, 256, 8);
-      switch (wk) {
-        case WKind::Unit:
-          k_prepare_arrays<WUnit><<<grid, 256, 0, s>>>(succ, WUnit{}, n, start, rec, ruler_elem, ctr, salt, th,
-                                                       ctx.d_status);
-          break;
-        case WKind::U32:
-          k_prepare_arrays<WU32><<<grid, 256, 0, s>>>(succ, WU32{(const uint32_t*)w}, n, start, rec, ruler_elem, ctr,
-                                                      salt, th, ctx.d_status);
-          break;
-        case WKind::I64:
-          k_prepare_arrays<WI64><<<grid, 256, 0, s>>>(succ, WI64{(const int64_t*)w}, n, start, rec, ruler_elem, ctr,
-                                                      salt, th, ctx.d_status);
-          break;
+      k_prepare_tma<true><<<g, 256, smem, s>>>(succ, (const uint32_t*)w, n, ntiles, rec, ctx.d_status);
+    } else {
+      constexpr int smem = PT_STAGES * PT_TILE * 8;
+      static bool raised = false;
+      if (!raised) {
+        KS_CUDA(cudaFuncSetAttribute(k_prepare_tma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        raised = true;
       }
-      KS_CHECK_LAUNCH();
+      k_prepare_tma<false><<<g, 256, smem, s>>>(succ, nullptr, n, ntiles, rec, ctx.d_status);
     }
+    KS_CHECK_LAUNCH();
+    start = (uint64_t)ntiles * PT_TILE;
   }
-  // r_out == nullptr: the count stays on the device (*r_dev)
-  return r_out ? read_u32(ctx, ctr, r_out, s) : KASCADE_OK;
+  if (start < n) {
+    const uint64_t rest = n - start;
+    const unsigned grid = grid_for(ctx, (rest + 256 * PREP_ITEMS - 1) / (256 * PREP_ITEMS) * 256, 256, 8);
+    switch (wk) {
+      case WKind::Unit:
+        k_prepare_arrays<WUnit><<<grid, 256, 0, s>>>(succ, WUnit{}, n, start, rec, ctx.d_status);
+        break;
+      case WKind::U32:
+        k_prepare_arrays<WU32><<<grid, 256, 0, s>>>(succ, WU32{(const uint32_t*)w}, n, start, rec, ctx.d_status);
+        break;
+      case WKind::I64:
+        k_prepare_arrays<WI64><<<grid, 256, 0, s>>>(succ, WI64{(const int64_t*)w}, n, start, rec, ctx.d_status);
+        break;
+    }
+    KS_CHECK_LAUNCH();
+  }
+  return KASCADE_OK;
+}
+
+kascade_status rank_arrays_one_cta(kascade_ctx& ctx, const uint64_t* succ, WKind wk, const void* w, uint32_t n,
+                                   const SinkPlain& sink, cudaStream_t s) {
+  ctx.last_levels.assign(1, n);
+  Extent ext;
+  ext.cap = n;
+  switch (wk) {
+    case WKind::Unit:
+      return launch_rank_cta(ctx, CtaArrays<WUnit>{succ, WUnit{}}, ext, sink, ONE_CTA_TREES, 1, s);
+    case WKind::U32:
+      return launch_rank_cta(ctx, CtaArrays<WU32>{succ, WU32{(const uint32_t*)w}}, ext, sink, ONE_CTA_TREES, 1, s);
+    default:
+      return launch_rank_cta(ctx, CtaArrays<WI64>{succ, WI64{(const int64_t*)w}}, ext, sink, ONE_CTA_TREES, 1, s);
+  }
 }
 
 template <class Sink>
@@ -916,9 +1099,11 @@ kascade_status pointer_double_records(kascade_ctx& ctx, const Rec* rec, uint32_t
   uint32_t* active = alloc<uint32_t>(ctx, 1);
   if (!a || !b || !active) return KASCADE_ERR_OOM;
   unsigned grid = grid_for(ctx, n, 256, 8);
+  Extent ext;
+  ext.cap = n;
   {
     ProfScope ps(ctx, "pd_init", s);
-    k_pd_init<<<grid, 256, 0, s>>>(rec, n, nullptr, a, ctx.d_status);
+    k_pd_init<<<grid, 256, 0, s>>>(rec, ext, a, ctx.d_status);
     KS_CHECK_LAUNCH();
   }
   int rounds = 0;
@@ -926,7 +1111,7 @@ kascade_status pointer_double_records(kascade_ctx& ctx, const Rec* rec, uint32_t
     KS_CUDA(cudaMemsetAsync(active, 0, sizeof(uint32_t), s));
     {
       ProfScope ps(ctx, "pd_round", s);
-      k_pd_round<1><<<grid, 256, 0, s>>>(a, b, n, nullptr, active);
+      k_pd_round<1><<<grid, 256, 0, s>>>(a, b, ext, active);
       KS_CHECK_LAUNCH();
     }
     PdRec* t = a;
@@ -942,269 +1127,109 @@ kascade_status pointer_double_records(kascade_ctx& ctx, const Rec* rec, uint32_t
   }
   {
     ProfScope ps(ctx, "pd_final", s);
-    k_pd_final<Sink><<<grid, 256, 0, s>>>(a, n, nullptr, elem0, sink);
+    k_pd_final<Sink><<<grid, 256, 0, s>>>(a, ext, elem0, sink);
     KS_CHECK_LAUNCH();
   }
   return KASCADE_OK;
 }
 
-namespace {
-
-kascade_status rank_deep(kascade_ctx& ctx, Rec* rec, uint32_t n, const uint32_t* elem0, const SinkOut& sink,
-                         int level, const Params& p, cudaStream_t s) {
-  ctx.last_levels.push_back(n);
-  if (n <= p.base_max) return launch_base(ctx, rec, n, elem0, sink, s);
-  uint32_t* ruler_elem = alloc<uint32_t>(ctx, n);
-  uint32_t* elem0_next = alloc<uint32_t>(ctx, n);
-  uint32_t* ctr = alloc<uint32_t>(ctx, 1);
-  if (!ruler_elem || !elem0_next || !ctr) return KASCADE_ERR_OOM;
-  KS_CUDA(cudaMemsetAsync(ctr, 0, sizeof(uint32_t), s));
-  unsigned grid = grid_for(ctx, ((uint64_t)n + 256 * PREP_ITEMS - 1) / (256 * PREP_ITEMS) * 256, 256, 8);
-  {
-    ProfScope ps(ctx, "prepare_level", s);
-    k_prepare_level<<<grid, 256, 0, s>>>(rec, n, nullptr, n, elem0, ruler_elem, elem0_next, ctr,
-                                         salt_for(p.seed, level), thresh_for(p.spacing_deep), nullptr,
-                                         ctx.d_status);
+// Doubling for a fixed number of rounds, enough for any list the level can
+// hold: no host wait.  Only a recursion depth limited by the caller ends on a
+// level larger than one CTA ranks.
+static kascade_status pointer_double_level(kascade_ctx& ctx, const Rec* rec, const Extent& ext,
+                                           const uint32_t* rootel, Out* out, cudaStream_t s) {
+  const uint32_t m = ext.cap;
+  PdRec* a = alloc<PdRec>(ctx, m);
+  PdRec* b = alloc<PdRec>(ctx, m);
+  uint32_t* active = alloc<uint32_t>(ctx, 1);
+  if (!a || !b || !active) return KASCADE_ERR_OOM;
+  const unsigned grid = grid_for(ctx, m, 256, 8);
+  ProfScope ps(ctx, "pd_final_level", s);
+  k_pd_init<<<grid, 256, 0, s>>>(rec, ext, a, ctx.d_status);
+  KS_CHECK_LAUNCH();
+  // rounds of reach x4 until 4^rounds >= 4m: any list of at most m elements
+  int lg = 0;
+  while ((1ull << lg) < m) ++lg;
+  const int rounds = (lg + 1) / 2 + 1;
+  for (int i = 0; i < rounds; ++i) {
+    k_pd_round<3><<<grid, 256, 0, s>>>(a, b, ext, active);
     KS_CHECK_LAUNCH();
+    std::swap(a, b);
   }
-  uint32_t r = 0;
-  KS_TRY(read_u32(ctx, ctr, &r, s));
-  if ((uint32_t)level >= p.max_levels || (uint64_t)r * 10 > (uint64_t)n * 7)
-    return pointer_double_records(ctx, rec, n, elem0, sink, s);
-  Rec* rec_next = alloc<Rec>(ctx, r);
-  Out* out_next = alloc<Out>(ctx, r);
-  if (!rec_next || !out_next) return KASCADE_ERR_OOM;
-  KS_TRY(launch_chase(ctx, rec, n, ruler_elem, r, rec_next, p, s));
-  KS_TRY(rank_deep(ctx, rec_next, r, elem0_next, SinkOut{out_next}, level + 1, p, s));
-  return launch_propagate(ctx, rec, n, n, out_next, r, sink, s);
+  k_pd_check<<<grid, 256, 0, s>>>(a, ext, ctx.d_status);
+  KS_CHECK_LAUNCH();
+  k_pd_final<SinkOut><<<grid, 256, 0, s>>>(a, ext, rootel, SinkOut{out});
+  KS_CHECK_LAUNCH();
+  return KASCADE_OK;
 }
 
-}  // namespace
+kascade_status plan_levels(kascade_ctx& ctx, uint32_t n, const Heads& heads, const Params& p, Levels* lv) {
+  *lv = Levels{};
+  const int max_levels = (int)std::min<uint32_t>(p.max_levels, MAX_LEVELS);
+  lv->heads = heads;
+  // the last level holds the heads too: a caller's base case below them takes none
+  if (p.base_max < 2 * heads.cap) lv->heads = Heads{};
+  const uint32_t extra = lv->heads.cap;
+  const uint32_t base = std::max(1u, p.base_max - extra);
+  int k = 0;
+  uint32_t m = n;  // the elements of level k that rulers are placed among
+  lv->n[0] = n;
+  while (m > base && k < max_levels) {
+    const uint32_t sp = k == 0           ? p.spacing0
+                        : p.spacing_deep ? p.spacing_deep
+                                         : deep_spacing(m, ONE_CTA_MAX - extra);
+    lv->rulers[k] = make_rulers(sp, salt_for(p.seed, k));
+    lv->r[k] = m = ruler_count(m, lv->rulers[k]);
+    lv->n[k + 1] = m + extra;
+    ++k;
+  }
+  lv->last = k;
+  ctx.last_levels.assign(1, n);
+  for (int i = 1; i <= k; ++i) {
+    ctx.last_levels.push_back(lv->r[i - 1]);
+    lv->rec[i] = alloc<Rec>(ctx, lv->n[i]);
+    lv->rootel[i] = alloc<uint32_t>(ctx, lv->n[i]);
+    lv->out[i] = alloc<Out>(ctx, lv->n[i]);
+    if (!lv->rec[i] || !lv->rootel[i] || !lv->out[i]) return KASCADE_ERR_OOM;
+  }
+  return KASCADE_OK;
+}
+
+kascade_status rank_deep(kascade_ctx& ctx, const Levels& lv, const Params& p, cudaStream_t s) {
+  // deeper levels are L2-resident: one chain per thread saturates the L2
+  (void)p;
+  for (int k = 1; k < lv.last; ++k) KS_TRY(launch_chase(ctx, lv, k, lv.extent(k), 1, 256, s));
+  const int L = lv.last;
+  if (lv.n[L] <= ONE_CTA_MAX) {
+    KS_TRY(launch_rank_cta(ctx, CtaRecords{lv.rec[L], lv.rootel[L]}, lv.extent(L), SinkOut{lv.out[L]}, 0, 0, s));
+  } else {
+    KS_TRY(pointer_double_level(ctx, lv.rec[L], lv.extent(L), lv.rootel[L], lv.out[L], s));
+  }
+  for (int k = L - 1; k >= 1; --k) KS_TRY(launch_propagate(ctx, lv, k, lv.n[k], lv.extent(k), SinkOut{lv.out[k]}, s));
+  return KASCADE_OK;
+}
 
 template <class Sink>
-kascade_status rank_records(kascade_ctx& ctx, Rec* rec, uint32_t n, uint32_t r0, uint32_t* ruler_elem0,
-                            const Sink& sink, const Params& p, cudaStream_t s) {
-  ctx.last_levels.clear();
-  ctx.last_levels.push_back(n);
+kascade_status rank_records(kascade_ctx& ctx, Rec* rec, uint32_t n, const Extent& ext, const Heads& heads,
+                            const Sink& sink, const Params& p, cudaStream_t s, bool host_check) {
   if (n == 0) return KASCADE_OK;
-  if (n <= p.base_max) return launch_base(ctx, rec, n, nullptr, sink, s);
-  if (p.algorithm != KASCADE_ALGO_SPARSE_RULING_SET || p.max_levels == 0 || (uint64_t)r0 * 10 > (uint64_t)n * 7)
-    return pointer_double_records(ctx, rec, n, nullptr, sink, s);
+  if (n <= p.base_max) {
+    ctx.last_levels.assign(1, n);
+    return launch_rank_cta(ctx, CtaRecords{rec, nullptr}, ext, sink, ONE_CTA_TREES, 1, s);
+  }
   if (Sink::kWriteFree && n >= p.level0_log_min && !sink.log_target(n).keep_roots) {
-    const kascade_status st = rank_level0_log(ctx, rec, n, r0, ruler_elem0, sink.log_target(n), p, s);
-    if (st != KASCADE_ERR_TIMEOUT) return st;
+    const kascade_status st = rank_level0_log(ctx, rec, n, ext, heads, sink.log_target(n), p, s, host_check);
+    if (!host_check || st != KASCADE_ERR_TIMEOUT) return st;
     // a chain exceeded the write-free path's hop cap (invalid input, or an
     // astronomically unlikely ruler gap): redo level 0 on the stamping path
-    KS_CUDA(cudaMemsetAsync(&ctx.d_status->counter[0], 0, sizeof(unsigned long long), s));
+    KS_TRY(status_reset(ctx, s));
   }
-  Rec* rec1 = alloc<Rec>(ctx, r0);
-  Out* out1 = alloc<Out>(ctx, r0);
-  if (!rec1 || !out1) return KASCADE_ERR_OOM;
-  KS_TRY(launch_chase(ctx, rec, n, ruler_elem0, r0, rec1, p, s));
-  // level-1 elements are level-0 rulers: their level-0 index is ruler_elem0
-  KS_TRY(rank_deep(ctx, rec1, r0, ruler_elem0, SinkOut{out1}, 1, p, s));
-  return launch_propagate(ctx, rec, sink.limit(n), n, out1, r0, sink, s);
-}
-
-// ---------------------------------------------------------------------------
-// Recursion without host waits.  Level sizes stay in device memory; every
-// kernel is sized for its level's capacity and reads the size at run time.
-// Capacities shrink by the deep-level ruler density (1.5x margin plus room for
-// roots); the last level (at most DEV_FINAL elements, or the first that stops
-// shrinking) runs pointer doubling for a fixed number of rounds.  A level that
-// outgrows its capacity reports KASCADE_ERR_TIMEOUT and the caller reruns on
-// the host-driven path.  The sequence of launches depends only on n and the
-// capacities, so it can be captured in a CUDA graph.
-// ---------------------------------------------------------------------------
-constexpr uint32_t DEV_FINAL = 1u << 17;
-constexpr uint32_t DEV_ROOT_MARGIN = 1u << 16;
-
-uint32_t dev_cap_next(uint32_t cap, uint32_t spacing) {
-  const uint64_t nx = (uint64_t)cap * 3 / (2ull * (spacing < 2 ? 2 : spacing)) + DEV_ROOT_MARGIN;
-  return nx < cap ? (uint32_t)nx : cap;
-}
-
-// Levels 1.. of the device-driven recursion.  rec1 / out1 hold caps1
-// elements; cnt[1] (device) holds level 1's size once the level-0 chase that
-// writes rec1 has run, already checked against caps1; elem0_1 gives each
-// level-1 element's level-0 index.  Fills out1 and cnt[2..L]; *levels = L.
-kascade_status rank_deep_dev(kascade_ctx& ctx, Rec* rec1, Out* out1, uint32_t cap1, uint32_t* cnt,
-                             const uint32_t* elem0_1, const uint32_t* pred1, const Params& p, cudaStream_t s,
-                             int* levels) {
-  uint32_t caps[MAX_DEV_LEVELS + 1];
-  caps[1] = cap1;
-  int L = 1;
-  while (caps[L] > DEV_FINAL && L < MAX_DEV_LEVELS) {
-    const uint32_t nx = dev_cap_next(caps[L], p.spacing_deep);
-    if ((uint64_t)nx * 10 >= (uint64_t)caps[L] * 9) break;  // no longer shrinking: final level here
-    caps[L + 1] = nx;
-    ++L;
-  }
-  Rec* recs[MAX_DEV_LEVELS + 1];
-  Out* outs[MAX_DEV_LEVELS + 1];
-  uint32_t* rulers[MAX_DEV_LEVELS + 1];
-  const uint32_t* elem0s[MAX_DEV_LEVELS + 1];
-  const uint32_t* sizes[MAX_DEV_LEVELS + 1];
-  uint32_t* preds[MAX_DEV_LEVELS + 1] = {};  // level k: which elements a chain of level k-1 ended at
-  recs[1] = rec1;
-  outs[1] = out1;
-  elem0s[1] = elem0_1;
-  sizes[1] = cnt + 1;
-  preds[1] = const_cast<uint32_t*>(pred1);
-  for (int k = 1; k <= L; ++k) {
-    if (k > 1) {
-      recs[k] = alloc<Rec>(ctx, caps[k]);
-      outs[k] = alloc<Out>(ctx, caps[k]);
-      if (!recs[k] || !outs[k]) return KASCADE_ERR_OOM;
-    }
-    if (k < L) {
-      rulers[k] = alloc<uint32_t>(ctx, caps[k + 1]);
-      uint32_t* e0 = alloc<uint32_t>(ctx, caps[k + 1]);
-      if (!rulers[k] || !e0) return KASCADE_ERR_OOM;
-      elem0s[k + 1] = e0;
-      sizes[k + 1] = cnt + k + 1;
-    }
-    if (k > 1 && k < L) {  // the last level is ranked by doubling and samples no rulers
-      const uint64_t words = ((uint64_t)caps[k] + 31) / 32;
-      preds[k] = alloc<uint32_t>(ctx, words);
-      if (!preds[k]) return KASCADE_ERR_OOM;
-      KS_CUDA(cudaMemsetAsync(preds[k], 0, sizeof(uint32_t) * words, s));
-    }
-  }
-  for (int k = 1; k < L; ++k) {
-    {
-      ProfScope ps(ctx, "prepare_level", s);
-      const unsigned grid =
-          grid_for(ctx, ((uint64_t)caps[k] + 256 * PREP_ITEMS - 1) / (256 * PREP_ITEMS) * 256, 256, 8);
-      k_prepare_level<<<grid, 256, 0, s>>>(recs[k], caps[k], sizes[k], caps[k + 1], elem0s[k], rulers[k],
-                                           const_cast<uint32_t*>(elem0s[k + 1]), cnt + k + 1,
-                                           salt_for(p.seed, k), thresh_for(p.spacing_deep), preds[k],
-                                           ctx.d_status);
-      KS_CHECK_LAUNCH();
-    }
-    uint32_t* work = alloc<uint32_t>(ctx, 1);
-    if (!work) return KASCADE_ERR_OOM;
-    KS_CUDA(cudaMemsetAsync(work, 0, sizeof(uint32_t), s));
-    KS_TRY(launch_chase_dev(ctx, recs[k], caps[k], sizes[k], rulers[k], caps[k + 1], sizes[k + 1], recs[k + 1], work,
-                            k + 1 < L ? preds[k + 1] : nullptr, p, s));
-  }
-  // final level: pointer doubling, enough rounds for any list it can hold
-  {
-    const uint32_t m = caps[L];
-    PdRec* a = alloc<PdRec>(ctx, m);
-    PdRec* b = alloc<PdRec>(ctx, m);
-    uint32_t* active = alloc<uint32_t>(ctx, 1);
-    if (!a || !b || !active) return KASCADE_ERR_OOM;
-    const unsigned grid = grid_for(ctx, m, 256, 8);
-    ProfScope ps(ctx, "pd_final_level", s);
-    k_pd_init<<<grid, 256, 0, s>>>(recs[L], m, sizes[L], a, ctx.d_status);
-    KS_CHECK_LAUNCH();
-    // rounds of reach x4 until 4^rounds >= 4m: any list of at most m elements
-    int lg = 0;
-    while ((1ull << lg) < m) ++lg;
-    const int rounds = (lg + 1) / 2 + 1;
-    for (int i = 0; i < rounds; ++i) {
-      k_pd_round<3><<<grid, 256, 0, s>>>(a, b, m, sizes[L], active);
-      KS_CHECK_LAUNCH();
-      PdRec* t = a;
-      a = b;
-      b = t;
-    }
-    k_pd_check<<<grid, 256, 0, s>>>(a, m, sizes[L], ctx.d_status);
-    KS_CHECK_LAUNCH();
-    k_pd_final<SinkOut><<<grid, 256, 0, s>>>(a, m, sizes[L], elem0s[L], SinkOut{outs[L]});
-    KS_CHECK_LAUNCH();
-  }
-  // propagate back up to level 1
-  for (int k = L - 1; k >= 1; --k) {
-    ProfScope ps(ctx, "propagate", s);
-    const unsigned grid = grid_for(ctx, ((uint64_t)caps[k] + PROP_ITEMS - 1) / PROP_ITEMS, 256, 8);
-    k_propagate<SinkOut><<<grid, 256, 0, s>>>(recs[k], caps[k], caps[k], sizes[k], 0, outs[k + 1], caps[k + 1],
-                                              SinkOut{outs[k]}, ctx.d_status);
-    KS_CHECK_LAUNCH();
-  }
-  *levels = L;
-  return KASCADE_OK;
-}
-
-__global__ void k_set_level0(uint32_t* lv, uint32_t base, const uint32_t* add) { lv[0] = base + *add; }
-
-kascade_status launch_set_level0(kascade_ctx& ctx, uint32_t* lv, uint32_t base, const uint32_t* add,
-                                 cudaStream_t s) {
-  (void)ctx;
-  k_set_level0<<<1, 1, 0, s>>>(lv, base, add);
-  KS_CHECK_LAUNCH();
-  return KASCADE_OK;
-}
-
-kascade_status launch_check_count(kascade_ctx& ctx, const uint32_t* cnt, uint32_t cap, uint32_t* copy,
-                                  cudaStream_t s) {
-  k_check_count<<<1, 1, 0, s>>>(cnt, cap, copy, ctx.d_status);
-  KS_CHECK_LAUNCH();
-  return KASCADE_OK;
-}
-
-kascade_status report_dev_levels(kascade_ctx& ctx, const uint32_t* cnt, int L, uint32_t n, cudaStream_t s) {
-  KS_CUDA(cudaMemcpyAsync(reinterpret_cast<uint32_t*>(ctx.h_pinned + KS_PINNED_LEVELS), cnt,
-                          sizeof(uint32_t) * (L + 1), cudaMemcpyDeviceToHost, s));
-  ctx.pending_levels = L;
-  ctx.pending_n = n;
-  return KASCADE_OK;
-}
-
-// the device count to add to a sink's element count for level 0's size
-// (tours sized for a bound), or null
-template <class Sink>
-const uint32_t* level0_add(const Sink&) {
-  return nullptr;
-}
-template <>
-const uint32_t* level0_add<SinkTour>(const SinkTour& t) {
-  return t.downs_dev;
-}
-
-template <class Sink>
-kascade_status rank_records_dev(kascade_ctx& ctx, Rec* rec, uint32_t n, const uint32_t* r0_dev, uint32_t cap1,
-                                uint32_t* ruler_elem0, const Sink& sink, const Params& p, cudaStream_t s) {
-  ctx.last_levels.clear();
-  ctx.last_levels.push_back(n);
-  if (n == 0) return KASCADE_OK;
-  if (cap1 > n) cap1 = n;
-  uint32_t* cnt = alloc<uint32_t>(ctx, MAX_DEV_LEVELS + 2);
-  Rec* rec1 = alloc<Rec>(ctx, cap1);
-  Out* out1 = alloc<Out>(ctx, cap1);
-  const uint64_t pwords = ((uint64_t)cap1 + 31) / 32;
-  uint32_t* pred1 = alloc<uint32_t>(ctx, pwords);
-  if (!cnt || !rec1 || !out1 || !pred1) return KASCADE_ERR_OOM;
-  KS_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * (MAX_DEV_LEVELS + 2), s));
-  KS_CUDA(cudaMemsetAsync(pred1, 0, sizeof(uint32_t) * pwords, s));
-  if (const uint32_t* d = level0_add(sink)) KS_TRY(launch_set_level0(ctx, cnt, sink.limit(n), d, s));
-  KS_TRY(launch_check_count(ctx, r0_dev, cap1, cnt + 1, s));
-  // level 0 chase: capacities as bounds, the ruler count from device memory
-  {
-    uint32_t* work = alloc<uint32_t>(ctx, 1);
-    if (!work) return KASCADE_ERR_OOM;
-    KS_CUDA(cudaMemsetAsync(work, 0, sizeof(uint32_t), s));
-    KS_TRY(launch_chase_dev(ctx, rec, n, nullptr, ruler_elem0, cap1, r0_dev, rec1, work, pred1, p, s));
-  }
-  // level-1 elements are level-0 rulers: their level-0 index is ruler_elem0
-  int L = 1;
-  KS_TRY(rank_deep_dev(ctx, rec1, out1, cap1, cnt, ruler_elem0, pred1, p, s, &L));
-  KS_TRY(launch_propagate(ctx, rec, sink.limit(n), n, out1, cap1, sink, s));
-  // the level sizes travel back with the call's status
-  return report_dev_levels(ctx, cnt, L, n, s);
-}
-
-template kascade_status rank_records_dev<SinkBatch>(kascade_ctx&, Rec*, uint32_t, const uint32_t*, uint32_t,
-                                                    uint32_t*, const SinkBatch&, const Params&, cudaStream_t);
-template kascade_status rank_records_dev<SinkTour>(kascade_ctx&, Rec*, uint32_t, const uint32_t*, uint32_t,
-                                                   uint32_t*, const SinkTour&, const Params&, cudaStream_t);
-template kascade_status rank_records_dev<SinkPlain>(kascade_ctx&, Rec*, uint32_t, const uint32_t*, uint32_t,
-                                                    uint32_t*, const SinkPlain&, const Params&, cudaStream_t);
-
-kascade_status rank_sublist(kascade_ctx& ctx, Rec* rec, uint32_t n, const uint32_t* elem0, Out* out, int level,
-                            const Params& p, cudaStream_t s) {
-  return rank_deep(ctx, rec, n, elem0, SinkOut{out}, level, p, s);
+  Levels lv;
+  KS_TRY(plan_levels(ctx, n, heads, p, &lv));
+  lv.rec[0] = rec;
+  KS_TRY(launch_chase(ctx, lv, 0, ext, p.chains, p.block, s));
+  KS_TRY(rank_deep(ctx, lv, p, s));
+  return launch_propagate(ctx, lv, 0, sink.limit(n), ext, sink, s);
 }
 
 kascade_status check_is_list(kascade_ctx& ctx, const uint64_t* succ, uint64_t n, int* ok, cudaStream_t s) {
@@ -1227,17 +1252,13 @@ kascade_status check_is_list(kascade_ctx& ctx, const uint64_t* succ, uint64_t n,
 }
 
 // explicit instantiations for the level-0 sinks
-template kascade_status rank_records<SinkPlain>(kascade_ctx&, Rec*, uint32_t, uint32_t, uint32_t*, const SinkPlain&,
-                                                const Params&, cudaStream_t);
-template kascade_status rank_records<SinkTour>(kascade_ctx&, Rec*, uint32_t, uint32_t, uint32_t*, const SinkTour&,
-                                               const Params&, cudaStream_t);
-template kascade_status rank_records<SinkBatch>(kascade_ctx&, Rec*, uint32_t, uint32_t, uint32_t*, const SinkBatch&,
-                                                const Params&, cudaStream_t);
-template kascade_status pointer_double_records<SinkBatch>(kascade_ctx&, const Rec*, uint32_t, const uint32_t*,
-                                                          const SinkBatch&, cudaStream_t);
+template kascade_status rank_records<SinkPlain>(kascade_ctx&, Rec*, uint32_t, const Extent&, const Heads&,
+                                                const SinkPlain&, const Params&, cudaStream_t, bool);
+template kascade_status rank_records<SinkTour>(kascade_ctx&, Rec*, uint32_t, const Extent&, const Heads&,
+                                               const SinkTour&, const Params&, cudaStream_t, bool);
+template kascade_status rank_records<SinkBatch>(kascade_ctx&, Rec*, uint32_t, const Extent&, const Heads&,
+                                                const SinkBatch&, const Params&, cudaStream_t, bool);
 template kascade_status pointer_double_records<SinkPlain>(kascade_ctx&, const Rec*, uint32_t, const uint32_t*,
                                                           const SinkPlain&, cudaStream_t);
-template kascade_status pointer_double_records<SinkTour>(kascade_ctx&, const Rec*, uint32_t, const uint32_t*,
-                                                         const SinkTour&, cudaStream_t);
 
 }  // namespace ks

@@ -1,17 +1,25 @@
 // Internal interface of the ruling-set list ranker.
 //
 // Pipeline for a list of n elements held as 16 B records (Rec):
-//   prepare   : counter-hash ruler sampling + ruler ids       (level 0 from the
-//               caller's arrays, deeper levels in place)
-//   chase     : every ruler walks its successors until the next ruler,
-//               stamping (ruler id, distance) into each record it passes and
-//               writing the ruler's sub-list record for the next level
-//   recurse   : the sub-list of rulers is ranked the same way, down to a
-//               one-CTA shared-memory base case (or pointer doubling when a
-//               level does not shrink)
+//   prepare   : records from the caller's arrays
+//   chase     : every ruler walks its successors until the next ruler or the
+//               list's end, stamping (ruler id, distance) into each record it
+//               passes and writing the ruler's record of the next level
+//   recurse   : the list of rulers is ranked the same way, down to a one-CTA
+//               shared-memory ranker
 //   propagate : one coalesced pass: rank = rank(ruler) - distance, root =
 //               root(ruler); elements ahead of their list's first ruler walk
-//               forward to the first stamped element
+//               forward to the first element with a result
+//
+// Rulers are placed by position (struct Rulers): one in every block of s
+// consecutive indices, at an offset hashed from the block's number.  A
+// ruler's id is its block's number, so ids need no numbering pass, no list of
+// ruler elements and no tag in the records: a chain knows from the index
+// alone that the next element is a ruler and ends without reading it, and
+// every level's size is ceil(n / s), known on the host before the first
+// launch.  A gap between rulers along a list is at most as long as with
+// independent samples of rate 1 / s (blocks that a gap meets more than once
+// only help).
 #pragma once
 
 #include "common.cuh"
@@ -20,11 +28,11 @@
 namespace ks {
 
 struct Params {
-  uint32_t spacing0 = 48;      // mean elements per ruler, level 0
-  uint32_t spacing_deep = 24;  // mean elements per ruler, deeper levels
+  uint32_t spacing0 = 48;     // mean elements per ruler, level 0
+  uint32_t spacing_deep = 0;  // mean elements per ruler, deeper levels (0: by level size)
   uint32_t max_levels = 6;
-  uint32_t base_max = 8192;    // one-CTA base case bound
-  uint32_t chains = 2;         // chains in flight per thread (1, 2 or 4)
+  uint32_t base_max = 16384;  // one-CTA ranker bound
+  uint32_t chains = 2;        // chains in flight per thread (1, 2 or 4)
   uint32_t block = 256;
   uint32_t seed = 0x6b617363u;
   uint32_t algorithm = KASCADE_ALGO_SPARSE_RULING_SET;
@@ -34,8 +42,60 @@ struct Params {
 
 Params make_params(const kascade_ctx& ctx, const kascade_opts* opts, uint64_t n);
 
-// Mean ruler spacing for an instance of n elements (the size-class table).
-uint32_t spacing_for(const kascade_ctx& ctx, uint64_t n);
+// Ruler placement of one level: element x lies in block x / s, whose ruler is
+// at offset hash(block) in [0, s).  The last block's ruler may fall beyond
+// the level's elements; its id is then dead (a record no element points to).
+// Division by s: the round-up multiply-and-shift for any 32-bit x.
+struct Rulers {
+  uint32_t s = 2, mul = 0, sh = 0, salt = 0;
+  __device__ __forceinline__ uint32_t offset(uint32_t j) const { return __umulhi(mix32(j ^ salt), s); }
+  __device__ __forceinline__ uint64_t elem(uint32_t j) const { return (uint64_t)j * s + offset(j); }
+  __device__ __forceinline__ uint32_t block_of(uint32_t x) const {
+    const uint32_t t = __umulhi(x, mul);
+    return (t + ((x - t) >> 1)) >> sh;
+  }
+  // whether x is a ruler; *j: its block (its id when it is one)
+  __device__ __forceinline__ bool is(uint32_t x, uint32_t* j) const {
+    const uint32_t b = block_of(x);
+    *j = b;
+    return x - b * s == offset(b);
+  }
+};
+__host__ __device__ inline Rulers make_rulers(uint32_t s, uint32_t salt) {
+  Rulers r;
+  if (s < 2) s = 2;
+  if (s > 0x80000000u) s = 0x80000000u;
+  uint32_t l = 1;
+  while (l < 31 && (1ull << l) < s) ++l;
+  r.s = s;
+  r.mul = (uint32_t)(((1ull << 32) * ((1ull << l) - s)) / s + 1);
+  r.sh = l - 1;
+  r.salt = salt;
+  return r;
+}
+inline uint32_t ruler_count(uint32_t n, const Rulers& r) { return (uint32_t)(((uint64_t)n + r.s - 1) / r.s); }
+
+// A level's element count when only the device knows it: base + *add, at most
+// the capacity the launch was sized for (add == nullptr: the capacity).
+struct Extent {
+  uint32_t cap = 0;
+  uint32_t base = 0;
+  const uint32_t* add = nullptr;
+  __device__ __forceinline__ uint32_t get() const { return add ? (uint32_t)min((uint64_t)cap, (uint64_t)base + __ldg(add)) : cap; }
+};
+
+// Known list heads of level 0 (a tour's heads are known when it is built):
+// they start chains of their own, so that no element ahead of its list's
+// first ruler is left to walk.  Head e's chain has the id after the rulers',
+// r + e; level k + 1 keeps it as the element after its rulers' ones, where it
+// is a head again.  Heads beyond the capacity stay unreached and walk.
+struct Heads {
+  const uint32_t* elem = nullptr;   // level-0 elements (device)
+  const uint32_t* count = nullptr;  // how many (device); more than cap: the first cap
+  uint32_t cap = 0;
+  __device__ __forceinline__ uint32_t get() const { return cap ? min(cap, __ldg(count)) : 0u; }
+};
+constexpr uint32_t HEAD_CAP = 2048;
 
 // Where results of level 0 go ------------------------------------------------
 // A sink receives, for element x, its rank, its root (level-0 index) and
@@ -47,7 +107,6 @@ struct LogTarget {
   uint64_t* rank;
   uint32_t limit;        // elements [0, limit) produce output
   int keep_roots;        // leave roots' entries untouched
-  int heads_are_rulers;  // every list head is a ruler: no element is left unreached
   // a batch of instances in one index space: roots are reported relative to
   // their instance (seg_off: nseg instance offsets, hint[k]: the instance
   // holding element k * 4096); null for a single instance
@@ -57,9 +116,6 @@ struct LogTarget {
   // bit x set: element x's rank output is one more than its rank in the list
   // (a tree rooting's leaves, whose down and up edge share one element)
   const uint32_t* plus_one = nullptr;
-  // heads_are_rulers: how many elements at or above limit a valid input logs
-  // (device memory; null: every element from limit to n)
-  const uint32_t* beyond_want = nullptr;
 };
 
 // Plain arrays. keep_roots: leave root entries untouched (the reference's
@@ -71,7 +127,7 @@ struct SinkPlain {
   int keep_roots;
   // elements [0, limit(n)) produce output
   uint32_t limit(uint32_t n) const { return n; }
-  LogTarget log_target(uint32_t n) const { return LogTarget{root, rank, n, keep_roots, 0}; }
+  LogTarget log_target(uint32_t n) const { return LogTarget{root, rank, n, keep_roots}; }
   __device__ __forceinline__ void put(uint32_t x, uint64_t rk, uint32_t rt, bool is_root) const {
     if (is_root) {
       if (!keep_roots) {
@@ -96,15 +152,10 @@ struct SinkTour {
   uint32_t nv;
   int keep_roots;
   const uint32_t* leaf_bits = nullptr;
-  // the tour's down-edge count in device memory when the records are sized
-  // for a bound (2 nv) rather than the tour's length
-  const uint32_t* downs_dev = nullptr;
   uint32_t limit(uint32_t n) const { return n < nv ? n : nv; }
-  // the tour build makes every tour head a ruler
   LogTarget log_target(uint32_t n) const {
-    LogTarget t{root, depth, limit(n), keep_roots, 1};
+    LogTarget t{root, depth, limit(n), keep_roots};
     t.plus_one = leaf_bits;
-    t.beyond_want = downs_dev;
     return t;
   }
   __device__ __forceinline__ void put(uint32_t x, uint64_t rk, uint32_t rt, bool is_root) const {
@@ -139,7 +190,7 @@ struct SinkBatch {
   const uint32_t* plus_one = nullptr;
   uint32_t limit(uint32_t n) const { return n < total ? n : total; }
   LogTarget log_target(uint32_t n) const {
-    LogTarget t{root, rank, limit(n), 0, 0, seg_off, hint, nseg};
+    LogTarget t{root, rank, limit(n), 0, seg_off, hint, nseg};
     t.plus_one = plus_one;
     return t;
   }
@@ -168,75 +219,73 @@ struct SinkOut {
   Out* out;
   uint32_t limit(uint32_t n) const { return n; }
   __device__ __forceinline__ void put(uint32_t x, uint64_t rk, uint32_t rt, bool is_root) const {
-    st_out(out + x, is_root ? 0ull : rk, rt);
+    (void)is_root;  // a deeper level's list end carries its rank like every element
+    st_out(out + x, rk, rt);
   }
 };
 
 // Weight readers for building level-0 records.
 enum class WKind { Unit, U32, I64 };
 
-// Build level-0 records from (succ, weights), sample rulers and number them.
-// ruler_elem must hold n entries; *r_out receives the ruler count.
-kascade_status prepare_arrays(kascade_ctx& ctx, const uint64_t* succ, WKind wk, const void* w,
-                              uint32_t n, Rec* rec, uint32_t* ruler_elem, uint32_t* r_out,
-                              const Params& p, cudaStream_t s, uint32_t** r_dev = nullptr);
+// Build level-0 records from (succ, weights); a root's record carries weight 0.
+kascade_status prepare_arrays(kascade_ctx& ctx, const uint64_t* succ, WKind wk, const void* w, uint32_t n, Rec* rec,
+                              const Params& p, cudaStream_t s);
 
-// Rank level-0 records that carry ruler tags (r0 rulers, listed in
-// ruler_elem0) and deliver the results to the sink.
+// Rank n <= ONE_CTA_MAX elements straight from the caller's arrays in one
+// launch.  Any forest is accepted up to ONE_CTA_TREES elements; above, lists.
+constexpr uint32_t ONE_CTA_MAX = 16384;
+constexpr uint32_t ONE_CTA_TREES = 8192;
+kascade_status rank_arrays_one_cta(kascade_ctx& ctx, const uint64_t* succ, WKind wk, const void* w, uint32_t n,
+                                   const SinkPlain& sink, cudaStream_t s);
+
+// Rank level-0 records and deliver the results to the sink.  Every level's
+// size is known on the host: no host wait between the launches.  `ext`: the
+// record count when only the device knows it (ext.cap == n).
+// The write-free level 0 can report KASCADE_ERR_TIMEOUT (a chain past its hop
+// cap): in the status word, or as the return value with host_check (the call
+// then waits for the chase before anything is written to the outputs, and
+// falls back to the stamping level 0 by itself).
 template <class Sink>
-kascade_status rank_records(kascade_ctx& ctx, Rec* rec, uint32_t n, uint32_t r0,
-                            uint32_t* ruler_elem0, const Sink& sink, const Params& p,
-                            cudaStream_t s);
+kascade_status rank_records(kascade_ctx& ctx, Rec* rec, uint32_t n, const Extent& ext, const Heads& heads,
+                            const Sink& sink, const Params& p, cudaStream_t s, bool host_check);
 
-// Rank a deeper level (records written by the chase of the level above, tags
-// unassigned); results go to out[0..n).  elem0 maps this level's elements to
-// level-0 indices.
-kascade_status rank_sublist(kascade_ctx& ctx, Rec* rec, uint32_t n, const uint32_t* elem0, Out* out,
-                            int level, const Params& p, cudaStream_t s);
-
-// The recursion without host waits (see ranker.cu): r0_dev holds the level-0
-// ruler count, cap1 bounds it.  Errors, including a level that outgrows its
-// capacity (KASCADE_ERR_TIMEOUT: rerun on the host-driven path), land in the
-// device status word.
-template <class Sink>
-kascade_status rank_records_dev(kascade_ctx& ctx, Rec* rec, uint32_t n, const uint32_t* r0_dev, uint32_t cap1,
-                                uint32_t* ruler_elem0, const Sink& sink, const Params& p, cudaStream_t s);
-uint32_t dev_cap_next(uint32_t cap, uint32_t spacing);
-constexpr int MAX_DEV_LEVELS = 8;
-// Levels 1.. of that recursion: rec1 / out1 hold cap1 elements, cnt (device,
-// MAX_DEV_LEVELS + 2 words) holds level 1's size in cnt[1] once the level-0
-// chase has run; pred1 (optional, cap1 bits): level-1 elements a level-0
-// chain ended at (the others head their lists and become rulers); fills out1
-// and cnt[2..L], *levels = L.
-kascade_status rank_deep_dev(kascade_ctx& ctx, Rec* rec1, Out* out1, uint32_t cap1, uint32_t* cnt,
-                             const uint32_t* elem0_1, const uint32_t* pred1, const Params& p, cudaStream_t s,
-                             int* levels);
-// *copy = *cnt, and KASCADE_ERR_TIMEOUT in the status word when it exceeds cap.
-// lv[0] = base + *add: level 0's size in the device-driven level array when
-// only the device knows it (a tour's length), reported in place of the call's n.
-kascade_status launch_set_level0(kascade_ctx& ctx, uint32_t* lv, uint32_t base, const uint32_t* add,
-                                 cudaStream_t s);
-kascade_status launch_check_count(kascade_ctx& ctx, const uint32_t* cnt, uint32_t cap, uint32_t* copy,
-                                  cudaStream_t s);
-// Level sizes cnt[1..L] travel back with the call's status read.
-kascade_status report_dev_levels(kascade_ctx& ctx, const uint32_t* cnt, int L, uint32_t n, cudaStream_t s);
+// The levels of one call.  Level k >= 1 holds level k - 1's rulers, then its
+// heads: records {distance, next ruler}, the root of a list end and results.
+constexpr int MAX_LEVELS = 24;
+struct Levels {
+  int last = 0;                  // the level ranked by one CTA (or by doubling)
+  uint32_t n[MAX_LEVELS + 1];    // elements per level, heads (their capacity) included
+  uint32_t r[MAX_LEVELS];        // rulers of level k; level k + 1 has r[k] + heads.cap elements
+  Rulers rulers[MAX_LEVELS];     // their placement
+  Heads heads;
+  Rec* rec[MAX_LEVELS + 1];
+  uint32_t* rootel[MAX_LEVELS + 1];  // level k >= 1: a list end's root as a level-0 element
+  Out* out[MAX_LEVELS + 1];
+  Extent extent(int k) const {
+    Extent e;
+    e.cap = n[k];
+    if (k && heads.cap) {
+      e.base = r[k - 1];
+      e.add = heads.count;
+    }
+    return e;
+  }
+};
+kascade_status plan_levels(kascade_ctx& ctx, uint32_t n, const Heads& heads, const Params& p, Levels* lv);
+// Levels 1..last once the level-0 chase has written level 1: fills lv.out[1].
+kascade_status rank_deep(kascade_ctx& ctx, const Levels& lv, const Params& p, cudaStream_t s);
 
 kascade_status compute_stats(kascade_ctx& ctx, const uint64_t* root, const int64_t* rank, uint64_t n, int level,
                              kascade_stats* out, kascade_tree_stats* per_tree, uint64_t per_tree_cap,
                              uint64_t* per_tree_count, cudaStream_t s);
 
 // Write-free level 0: read-only chase that logs (element, ruler, distance),
-// recursion on the ruler sub-list, then two radix passes over the log by
-// element and a dense placement into the outputs.  With r0_dev the ruler
-// count stays on the device (r0 is then its capacity) and so does the
-// recursion: no host wait; a chain past the hop cap or a level past its
-// capacity reports KASCADE_ERR_TIMEOUT in the status word (rerun on the
-// host-driven path).  Without it, a chain past the hop cap returns
-// KASCADE_ERR_TIMEOUT directly (level 0 again on the stamping path).
-kascade_status rank_level0_log(kascade_ctx& ctx, const Rec* rec, uint32_t n, uint32_t r0,
-                               const uint32_t* ruler_elem0, const LogTarget& t, const Params& p,
-                               cudaStream_t s, const uint32_t* r0_dev = nullptr);
-
+// recursion on the ruler list, then two radix passes over the log by element
+// and a dense placement into the outputs.  A chain past the hop cap becomes
+// KASCADE_ERR_TIMEOUT: in the status word, or (host_check) the return value,
+// with no output written yet.
+kascade_status rank_level0_log(kascade_ctx& ctx, const Rec* rec, uint32_t n, const Extent& ext, const Heads& heads,
+                               const LogTarget& t, const Params& p, cudaStream_t s, bool host_check);
 
 // Pointer doubling on level-0 records (tags ignored).
 template <class Sink>
