@@ -79,19 +79,18 @@ typedef struct kascade_opts {
                                  (sparse_ruling_set_rounds, configuration.hpp:70)  */
   uint32_t base_case_size;    /* at most this many elements go to the one-CTA
                                  base case (0 = auto)                              */
-  uint32_t chains_per_thread; /* independent chains in flight per thread (0=auto) */
+  uint32_t chains_per_thread; /* accepted, no effect (one chain per thread is the
+                                 fastest form at every size)                       */
   uint32_t block_size;        /* threads per CTA of the chase kernel (0 = auto)     */
   uint32_t validate;          /* 1: check is_list before a list-only algorithm      */
   uint32_t async;             /* 1: return after enqueueing; see kascade_ctx_sync   */
   uint32_t profile;           /* 1: time each kernel with CUDA events               */
   uint32_t seed;              /* ruler-sampling seed                                */
-  uint32_t level0_mode;       /* first level: 0 auto (write-free from 2^25
-                                 elements on, where it is faster), 1 stamping
-                                 chase, 2 write-free chase (read-only chase, log,
-                                 radix partition by element, dense placement);
-                                 in-place calls always stamp                      */
-  uint32_t max_chain;         /* hop cap of the write-free chase before it hands
-                                 level 0 to the stamping chase (0 = 64 x spacing)  */
+  uint32_t level0_mode;       /* first level: 0 by size, 1 stamping chase, 2
+                                 write-free chase (read-only chase, log, radix
+                                 partition by element, dense placement; what 0
+                                 takes from 8 to 12 million elements on)           */
+  uint32_t max_chain;         /* accepted, no effect (chains have no hop cap)      */
 } kascade_opts;
 
 typedef struct kascade_ctx kascade_ctx;
@@ -355,9 +354,7 @@ typedef struct kascade_server kascade_server;
  * and the input / weight / output pointers are fixed at creation; their
  * contents may change between launches.  Creation runs the batch once and
  * returns KASCADE_ERR_UNSUPPORTED for a batch made mostly of list ends (very
- * many roots); a launch whose new contents run a chain past the write-free
- * chase's hop cap returns KASCADE_ERR_TIMEOUT,
- * and kascade_rank_batch handles such a batch.  A plan owns its scratch;
+ * many roots), which kascade_rank_batch handles.  A plan owns its scratch;
  * launches of one plan are ordered on the device.  No counterpart in the
  * reference (its rounds are MPI exchanges per call). */
 typedef struct kascade_batch_plan kascade_batch_plan;

@@ -553,7 +553,7 @@ def get_size_classes(ctx: Context):
 
 
 def set_class_launch(ctx: Context, chains, blocks, single_spacing=None) -> None:
-    """Per size class: chains per chase thread (1, 2, 4), chase block size
+    """Per size class: chains per chase thread (1, 2, 4; no effect), chase block size
     (128, 256, 512) and, optionally, the ruler spacing of calls that rank one
     instance on their own; one entry per class of the current table."""
     k = len(chains)

@@ -10,8 +10,8 @@
 //                                              a leaf's down and up edge in one)
 //   down edges of all forests (F of them)   -> records total_n .. total_n+F-1
 //                                              (a leaf's or a root's: a dead self loop)
-// The ruler spacing is one per batch, from the size class (the context's
-// size-class table, filled by the autotuner) that holds most of its records.
+// The ruler spacing is one per batch, from the size class of its record count
+// (the context's size-class table, filled by the autotuner).
 // Roots are reported relative to their own instance.
 #include <algorithm>
 #include <cstring>
@@ -23,8 +23,8 @@
 namespace ks {
 
 kascade_status batch_tours(kascade_ctx& ctx, const uint64_t* fpar, uint32_t F, const uint32_t* fd, const uint32_t* foff,
-                           const uint32_t* fhint, uint32_t nf, uint32_t down_base, Rec* rec, uint32_t* leaf_out,
-                           Heads* heads, cudaStream_t s);
+                           const uint32_t* fhint, uint32_t nf, uint32_t down_base, const Level0& l0,
+                           const Rulers& rl, uint32_t* leaf_out, Heads* heads, cudaStream_t s);
 
 namespace {
 
@@ -48,24 +48,25 @@ struct __align__(16) Item {
 };
 
 struct BWUnit {
-  __device__ __forceinline__ uint64_t operator()(uint64_t) const { return 1ull; }
+  __device__ __forceinline__ uint32_t operator()(uint64_t) const { return 1u; }
 };
 struct BWU32 {
   const uint32_t* p;
-  __device__ __forceinline__ uint64_t operator()(uint64_t g) const { return (uint64_t)__ldcs(p + g); }
+  __device__ __forceinline__ uint32_t operator()(uint64_t g) const { return __ldcs(p + g); }
 };
 
-template <class W>
+template <class F, class W>
 __global__ void __launch_bounds__(BP_THREADS) k_batch_prepare(const Item* __restrict__ items, uint32_t nitems,
                                                               const DSeg* __restrict__ segs,
-                                                              const uint64_t* __restrict__ in, W w,
-                                                              Rec* __restrict__ rec, uint64_t* __restrict__ fpar,
-                                                              DevStatus* st) {
+                                                              const uint64_t* __restrict__ in, W w, Rulers rl,
+                                                              typename F::R* __restrict__ rec,
+                                                              typename F::S* __restrict__ stamp,
+                                                              uint64_t* __restrict__ fpar, DevStatus* st) {
   for (uint32_t it = blockIdx.x; it < nitems; it += gridDim.x) {
     const Item item = items[it];
     const DSeg sg = segs[item.seg];
     if (sg.kind == KASCADE_SEG_LIST) {
-      uint64_t wv[BP_PER];
+      uint32_t wv[BP_PER];
       unsigned long long lv[BP_PER];
       // every load of the item first (independent, all in flight together),
       // then the checks
@@ -91,11 +92,10 @@ __global__ void __launch_bounds__(BP_THREADS) k_batch_prepare(const Item* __rest
           if (bad == ~0ull) bad = g;
           loc = k;
         }
-        Rec r;
-        r.a = loc == k ? 0ull : wv[i];  // a root's weight is no part of any rank
-        r.b = (uint32_t)(sg.off + loc);
-        r.c = TAG_UNREACHED;
-        rec[g] = r;
+        const uint32_t b = (uint32_t)(sg.off + loc);
+        uint32_t j;
+        F::put(rec + g, loc == k ? 0u : wv[i], b, rl.is(b, &j));  // a root's weight is no part of any rank
+        if (stamp) F::clear(stamp + g);
       }
       if (bad != ~0ull) set_error(st, KASCADE_ERR_OUT_OF_RANGE, bad);
     } else {
@@ -140,34 +140,30 @@ __global__ void __launch_bounds__(BP_THREADS) k_count_ends(const Item* __restric
 
 }  // namespace
 
-constexpr uint32_t WRITE_FREE_MIN_SPACING = 48;
-
 // Host tables of one batch: built from the segment list, uploaded into the
 // context's arena.  Kept apart from the launches so that a plan can upload
 // them once and capture only the device work.
 struct BatchTables {
   std::vector<DSeg> dsegs;
   std::vector<Item> items;
-  std::vector<uint32_t> fd, foff, hint, fhint;
+  std::vector<uint32_t> fd, foff, hint, fhint, tour;  // tour: bit j set when instance j is a forest
   std::vector<unsigned long long> seg_off;
   uint64_t total = 0, F = 0;
   uint32_t nseg = 0, nf = 0, M = 0;
-  size_t dom_class = 0;  // the size class holding most of the batch's records
   // device copies
   DSeg* d_segs = nullptr;
   Item* d_items = nullptr;
-  uint32_t *d_fd = nullptr, *d_foff = nullptr, *d_hint = nullptr, *d_fhint = nullptr;
+  uint32_t *d_fd = nullptr, *d_foff = nullptr, *d_hint = nullptr, *d_fhint = nullptr, *d_tour = nullptr;
   unsigned long long* d_off = nullptr;
 };
 
-kascade_status batch_build_tables(const kascade_ctx& ctx, const kascade_segment* segs, uint32_t nseg, uint64_t total,
-                                  BatchTables& t) {
+kascade_status batch_build_tables(const kascade_segment* segs, uint32_t nseg, uint64_t total, BatchTables& t) {
   t = BatchTables{};
   t.nseg = nseg;
   t.total = total;
   t.dsegs.resize(nseg);
   t.seg_off.resize(nseg);
-  std::vector<uint64_t> class_elems(ctx.class_max.size(), 0);
+  t.tour.assign((nseg + 31) / 32, 0u);
   t.items.reserve(total / ITEM + nseg);
   uint64_t expect = 0;
   for (uint32_t i = 0; i < nseg; ++i) {
@@ -176,13 +172,12 @@ kascade_status batch_build_tables(const kascade_ctx& ctx, const kascade_segment*
       return KASCADE_ERR_INVALID_ARG;
     expect += g.size;
     const bool forest = g.kind == KASCADE_SEG_FOREST;
-    const uint64_t records = forest ? 2 * g.size : g.size;
-    class_elems[ctx.class_of(records)] += records;
     t.dsegs[i] = DSeg{g.offset, (uint32_t)g.size, g.kind, (uint32_t)t.F, 0};
     t.seg_off[i] = g.offset;
     if (forest) {
       t.fd.push_back((uint32_t)t.F);
       t.foff.push_back((uint32_t)g.offset);
+      t.tour[i >> 5] |= 1u << (i & 31);
       t.F += g.size;
     }
     for (uint64_t st = 0; st < g.size; st += ITEM)
@@ -213,7 +208,6 @@ kascade_status batch_build_tables(const kascade_ctx& ctx, const kascade_segment*
     }
   }
   t.M = (uint32_t)(total + t.F);
-  t.dom_class = std::max_element(class_elems.begin(), class_elems.end()) - class_elems.begin();
   return KASCADE_OK;
 }
 
@@ -225,13 +219,15 @@ kascade_status batch_upload_tables(kascade_ctx& ctx, BatchTables& t, cudaStream_
   t.d_off = alloc<unsigned long long>(ctx, t.nseg);
   t.d_hint = alloc<uint32_t>(ctx, t.hint.size());
   t.d_fhint = alloc<uint32_t>(ctx, t.fhint.size());
-  if (!t.d_segs || !t.d_items || !t.d_fd || !t.d_foff || !t.d_off || !t.d_hint || !t.d_fhint)
+  t.d_tour = alloc<uint32_t>(ctx, t.tour.size());
+  if (!t.d_segs || !t.d_items || !t.d_fd || !t.d_foff || !t.d_off || !t.d_hint || !t.d_fhint || !t.d_tour)
     return KASCADE_ERR_OOM;
   KS_CUDA(cudaMemcpyAsync(t.d_segs, t.dsegs.data(), sizeof(DSeg) * t.nseg, cudaMemcpyHostToDevice, s));
   KS_CUDA(cudaMemcpyAsync(t.d_items, t.items.data(), sizeof(Item) * t.items.size(), cudaMemcpyHostToDevice, s));
   KS_CUDA(cudaMemcpyAsync(t.d_fd, t.fd.data(), sizeof(uint32_t) * t.fd.size(), cudaMemcpyHostToDevice, s));
   if (t.nf) {
     KS_CUDA(cudaMemcpyAsync(t.d_foff, t.foff.data(), sizeof(uint32_t) * t.nf, cudaMemcpyHostToDevice, s));
+    KS_CUDA(cudaMemcpyAsync(t.d_tour, t.tour.data(), sizeof(uint32_t) * t.tour.size(), cudaMemcpyHostToDevice, s));
   }
   KS_CUDA(cudaMemcpyAsync(t.d_off, t.seg_off.data(), sizeof(unsigned long long) * t.nseg, cudaMemcpyHostToDevice, s));
   KS_CUDA(cudaMemcpyAsync(t.d_hint, t.hint.data(), sizeof(uint32_t) * t.hint.size(), cudaMemcpyHostToDevice, s));
@@ -239,69 +235,72 @@ kascade_status batch_upload_tables(kascade_ctx& ctx, BatchTables& t, cudaStream_
   return KASCADE_OK;
 }
 
-// The batch's parameters: ruler spacing, chains and block size come from the
-// class that holds most of its records (one chase launch serves every
-// instance).  A batch large enough for the write-free level 0 spaces its
-// rulers more widely: its chase is read-only and cheap per hop, so fewer
-// rulers (a smaller recursion) pay off.
+// The batch's parameters: ruler spacing and block size from the class of its
+// record count (one chase launch serves every instance).
 Params batch_params(const kascade_ctx& ctx, const BatchTables& t, const kascade_opts* opts) {
   Params p = make_params(ctx, opts, t.M);
-  const size_t k = t.dom_class;
-  if (!(opts && opts->ruler_spacing)) {
-    p.spacing0 = std::max(2u, ctx.class_spacing[k]);
-    if (t.M >= p.level0_log_min) p.spacing0 = std::max(p.spacing0, WRITE_FREE_MIN_SPACING);
-  }
-  if (!(opts && opts->chains_per_thread)) p.chains = ctx.class_chains[k];
-  if (!(opts && opts->block_size))
-    p.block = (ctx.class_block[k] == 128 || ctx.class_block[k] == 512) ? ctx.class_block[k] : 256u;
+  if (!(opts && opts->ruler_spacing)) p.spacing0 = std::max(2u, ctx.class_spacing[ctx.class_of(t.M)]);
   p.algorithm = KASCADE_ALGO_SPARSE_RULING_SET;
   return p;
 }
 
 // The device work of one batch over uploaded tables: no host tables are read
-// and, without host_check, no host waits -- a stream capture of this call is
-// a replayable CUDA graph.
+// and there are no host waits -- a stream capture of this call is a replayable
+// CUDA graph.
 kascade_status batch_enqueue(kascade_ctx& ctx, const BatchTables& t, const uint64_t* in, const uint32_t* weights,
-                             uint64_t* root_out, uint64_t* rank_out, const kascade_opts* opts, cudaStream_t s,
-                             bool host_check) {
+                             uint64_t* root_out, uint64_t* rank_out, const kascade_opts* opts, cudaStream_t s) {
   const uint32_t M = t.M;
-  Rec* rec = alloc<Rec>(ctx, M);
+  const Params p = batch_params(ctx, t, opts);
+  Level0 l0;
+  KS_TRY(alloc_level0(ctx, plan_level0(p, M, weights ? WKind::U32 : WKind::Unit), M, &l0));
+  const Rulers rl = level0_rulers(p);
   uint64_t* fpar = alloc<uint64_t>(ctx, t.F + 1);
   // forest leaves by output position: their rank is one less than their depth
   const uint64_t leaf_words = t.F ? (t.total + 31) / 32 : 0;
   uint32_t* leaf_out = leaf_words ? alloc<uint32_t>(ctx, leaf_words) : nullptr;
-  if (!rec || !fpar || (leaf_words && !leaf_out)) return KASCADE_ERR_OOM;
+  if (!fpar || (leaf_words && !leaf_out)) return KASCADE_ERR_OOM;
   if (leaf_out) KS_CUDA(cudaMemsetAsync(leaf_out, 0, sizeof(uint32_t) * leaf_words, s));
-  const Params p = batch_params(ctx, t, opts);
   {
     ProfScope ps(ctx, "batch_prepare", s);
-    const unsigned grid = (unsigned)std::min<uint64_t>(t.items.size(), (uint64_t)ctx.usable_sms() * 8);
-    if (weights)
-      k_batch_prepare<BWU32><<<grid, BP_THREADS, 0, s>>>(t.d_items, (uint32_t)t.items.size(), t.d_segs, in,
-                                                         BWU32{weights}, rec, fpar, ctx.d_status);
+    const uint32_t items = (uint32_t)t.items.size();
+    const unsigned grid = (unsigned)std::min<uint64_t>(items, (uint64_t)ctx.usable_sms() * 8);
+    auto prepare = [&](auto f, auto w) {
+      using F = decltype(f);
+      k_batch_prepare<F><<<grid, BP_THREADS, 0, s>>>(t.d_items, items, t.d_segs, in, w, rl, l0.records<F>(),
+                                                     l0.stamps<F>(), fpar, ctx.d_status);
+    };
+    if (l0.fmt == Format::F8x16)
+      prepare(F8x16{}, BWU32{weights});
+    else if (l0.fmt == Format::F8x8)
+      prepare(F8x8{}, BWUnit{});
+    else if (l0.fmt == Format::F16i && weights)
+      prepare(F16i{}, BWU32{weights});
+    else if (l0.fmt == Format::F16i)
+      prepare(F16i{}, BWUnit{});
+    else if (weights)
+      prepare(F16x16{}, BWU32{weights});
     else
-      k_batch_prepare<BWUnit><<<grid, BP_THREADS, 0, s>>>(t.d_items, (uint32_t)t.items.size(), t.d_segs, in,
-                                                          BWUnit{}, rec, fpar, ctx.d_status);
+      prepare(F16x16{}, BWUnit{});
     KS_CHECK_LAUNCH();
   }
   Heads heads;
-  KS_TRY(batch_tours(ctx, fpar, (uint32_t)t.F, t.d_fd, t.d_foff, t.d_fhint, t.nf, (uint32_t)t.total, rec, leaf_out,
-                     &heads, s));
+  KS_TRY(batch_tours(ctx, fpar, (uint32_t)t.F, t.d_fd, t.d_foff, t.d_fhint, t.nf, (uint32_t)t.total, l0, rl,
+                     leaf_out, &heads, s));
   SinkBatch sink{root_out, rank_out, (uint32_t)t.total, reinterpret_cast<const uint64_t*>(t.d_off), t.d_hint, t.nseg,
-                 leaf_out};
+                 leaf_out, t.F ? t.d_tour : nullptr};
   Extent ext;
   ext.cap = M;
-  return rank_records(ctx, rec, M, ext, heads, sink, p, s, host_check);
+  return rank_records(ctx, l0, M, ext, heads, sink, p, s);
 }
 
 kascade_status rank_batch_impl(kascade_ctx& ctx, const kascade_segment* segs, uint32_t nseg, const uint64_t* in,
                                const uint32_t* weights, uint64_t total, uint64_t* root_out, uint64_t* rank_out,
-                               const kascade_opts* opts, cudaStream_t s, bool host_check) {
+                               const kascade_opts* opts, cudaStream_t s) {
   if (total == 0) return KASCADE_OK;
   BatchTables t;
-  KS_TRY(batch_build_tables(ctx, segs, nseg, total, t));
+  KS_TRY(batch_build_tables(segs, nseg, total, t));
   KS_TRY(batch_upload_tables(ctx, t, s));
-  return batch_enqueue(ctx, t, in, weights, root_out, rank_out, opts, s, host_check);
+  return batch_enqueue(ctx, t, in, weights, root_out, rank_out, opts, s);
 }
 
 // Whether a batch may be planned: one made mostly of list ends may not (as
@@ -324,7 +323,7 @@ static kascade_status plan_admits(kascade_ctx& ctx, const BatchTables& t, const 
 // ---------------------------------------------------------------------------
 // Plans: one batch captured as a CUDA graph and replayed.
 // ---------------------------------------------------------------------------
-// A complete call on the device-driven path (status read back), in capi.cu.
+// A complete call (status read back), in capi.cu.
 kascade_status rank_batch_device_call(kascade_ctx* c, const kascade_segment* segs, uint32_t nseg, const uint64_t* in,
                                       const uint32_t* weights, uint64_t total, uint64_t* root_out,
                                       uint64_t* rank_out, const kascade_opts* opts, cudaStream_t s);
@@ -366,12 +365,11 @@ kascade_status batch_plan_create(int device, const kascade_segment* segs, uint32
   cudaStream_t s = plan->stream;
   // 1. one eager run, which grows the plan's arena to what the batch needs
   kascade_status st = rank_batch_device_call(plan->ctx, segs, nseg, in, weights, total, root_out, rank_out, &opts, s);
-  if (st == KASCADE_ERR_TIMEOUT) return fail(KASCADE_ERR_UNSUPPORTED);
   if (st != KASCADE_OK) return fail(st);
   // 2. tables uploaded outside the capture, the device work captured
   st = arena_begin_call(ctx, s);
   BatchTables t;
-  if (st == KASCADE_OK) st = batch_build_tables(ctx, segs, nseg, total, t);
+  if (st == KASCADE_OK) st = batch_build_tables(segs, nseg, total, t);
   if (st == KASCADE_OK) st = batch_upload_tables(ctx, t, s);
   if (st == KASCADE_OK) st = plan_admits(ctx, t, in, &opts, s);
   if (st == KASCADE_OK && cudaStreamSynchronize(s) != cudaSuccess) st = KASCADE_ERR_CUDA;
@@ -382,7 +380,7 @@ kascade_status batch_plan_create(int device, const kascade_segment* segs, uint32
     return fail(KASCADE_ERR_CUDA);
   }
   st = status_reset(ctx, s);
-  if (st == KASCADE_OK) st = batch_enqueue(ctx, t, in, weights, root_out, rank_out, &opts, s, false);
+  if (st == KASCADE_OK) st = batch_enqueue(ctx, t, in, weights, root_out, rank_out, &opts, s);
   cudaGraph_t g = nullptr;
   const cudaError_t ce = cudaStreamEndCapture(s, &g);
   plan->graph = g;

@@ -8,7 +8,7 @@
 
 namespace ks {
 kascade_status root_forest_impl(kascade_ctx& ctx, const uint64_t* parent, uint32_t n, uint64_t* root_out,
-                                uint64_t* depth_out, int keep_roots, const Params& p, cudaStream_t s, bool host_check);
+                                uint64_t* depth_out, int keep_roots, const Params& p, cudaStream_t s);
 kascade_status compute_euler_tour_impl(kascade_ctx& ctx, const uint64_t* parent, uint32_t n, uint64_t* tour,
                                        uint64_t* m_out, cudaStream_t s);
 kascade_status gen_list(uint64_t n, uint64_t seed, uint32_t layout, uint64_t* succ, cudaStream_t s);
@@ -25,7 +25,7 @@ kascade_status unpack_impl(kascade_ctx& ctx, const uint64_t* succ_packed, const 
                            cudaStream_t s);
 kascade_status rank_batch_impl(kascade_ctx& ctx, const kascade_segment* segs, uint32_t nseg, const uint64_t* in,
                                const uint32_t* weights, uint64_t total, uint64_t* root_out, uint64_t* rank_out,
-                               const kascade_opts* opts, cudaStream_t s, bool host_check);
+                               const kascade_opts* opts, cudaStream_t s);
 }  // namespace ks
 
 using namespace ks;
@@ -48,7 +48,6 @@ kascade_status begin_call(kascade_ctx* ctx, cudaStream_t s, const kascade_opts* 
   KS_TRY(status_reset(*ctx, s));
   ctx->profile = o && o->profile;
   ctx->async_pending = false;
-  ctx->host_rerun.set = false;
   return KASCADE_OK;
 }
 
@@ -69,24 +68,25 @@ kascade_status end_call(kascade_ctx* ctx, cudaStream_t s, kascade_status st, con
   return status_finish(*ctx, s);
 }
 
-// host_check: see rank_records.  Calls whose status is read later, or whose
-// outputs are their inputs, cannot be rerun on KASCADE_ERR_TIMEOUT and set it.
 kascade_status rank_list_generic(kascade_ctx& ctx, const uint64_t* succ, WKind wk, const void* w, uint64_t n,
                                  uint64_t* root_out, uint64_t* rank_out, int keep_roots, const Params& p,
-                                 cudaStream_t s, bool host_check) {
+                                 cudaStream_t s) {
   if (n == 0) return KASCADE_OK;
   if (n > MAX_LIST) return KASCADE_ERR_TOO_LARGE;
   const SinkPlain sink{root_out, rank_out, keep_roots};
-  const bool ruling_set = p.algorithm == KASCADE_ALGO_SPARSE_RULING_SET;
-  if (ruling_set && n <= p.base_max) return rank_arrays_one_cta(ctx, succ, wk, w, (uint32_t)n, sink, s);
-  Rec* rec = alloc<Rec>(ctx, n);
-  if (!rec) return KASCADE_ERR_OOM;
-  KS_TRY(prepare_arrays(ctx, succ, wk, w, (uint32_t)n, rec, p, s));
-  if (ruling_set) {
+  Level0 l0;
+  if (p.algorithm == KASCADE_ALGO_SPARSE_RULING_SET) {
+    if (n <= p.base_max) return rank_arrays_one_cta(ctx, succ, wk, w, (uint32_t)n, sink, s);
+    KS_TRY(alloc_level0(ctx, plan_level0(p, n, wk), n, &l0));
+    KS_TRY(prepare_arrays(ctx, succ, wk, w, (uint32_t)n, l0, level0_rulers(p), s));
     Extent ext;
     ext.cap = (uint32_t)n;
-    return rank_records(ctx, rec, (uint32_t)n, ext, Heads{}, sink, p, s, host_check);
+    return rank_records(ctx, l0, (uint32_t)n, ext, Heads{}, sink, p, s);
   }
+  Rec* rec = alloc<Rec>(ctx, n);
+  if (!rec) return KASCADE_ERR_OOM;
+  l0.rec = rec;
+  KS_TRY(prepare_arrays(ctx, succ, wk, w, (uint32_t)n, l0, level0_rulers(p), s));
   ctx.last_levels.assign(1, n);
   return pointer_double_records(ctx, rec, (uint32_t)n, nullptr, sink, s);
 }
@@ -221,28 +221,11 @@ KASCADE_API uint64_t kascade_scratch_bytes_root_forest(uint64_t n) {
   return 16 * n + 8 * n + 32 * n + 8 * n + 32 * n + 16 * n + (80 * n) / 16 + (192ull << 20);
 }
 
-kascade_status rank_list_host_call(kascade_ctx* c, const uint64_t* succ, const uint32_t* weights, uint64_t n,
-                                   uint64_t* root_out, uint64_t* rank_out, const kascade_opts* opts,
-                                   cudaStream_t s, bool host_check);
-kascade_status root_forest_host_call(kascade_ctx* c, const uint64_t* parent, uint64_t n, uint64_t* root_out,
-                                     uint64_t* depth_out, const kascade_opts* opts, cudaStream_t s, bool host_check);
-
 KASCADE_API kascade_status kascade_ctx_sync(kascade_ctx* c, void* stream) {
   if (!c) return KASCADE_ERR_INVALID_ARG;
   if (!c->async_pending) return c->last_status;
   c->async_pending = false;
-  kascade_status st = status_finish(*c, as_stream(stream));
-  if (st == KASCADE_ERR_TIMEOUT && c->host_rerun.set) {
-    // an async host-buffer call with a chain past the write-free chase's hop
-    // cap: rank it again, checked on the host, before returning
-    const kascade_ctx::HostRerun r = c->host_rerun;
-    kascade_opts o = r.opts;
-    o.async = 0;
-    st = r.kind == 0 ? rank_list_host_call(c, r.succ, r.weights, r.n, r.root_out, r.rank_out, &o, r.stream, true)
-                     : root_forest_host_call(c, r.succ, r.n, r.root_out, r.rank_out, &o, r.stream, true);
-  }
-  c->host_rerun.set = false;
-  return st;
+  return status_finish(*c, as_stream(stream));
 }
 
 KASCADE_API uint64_t kascade_ctx_error_info(kascade_ctx* c) { return c ? c->error_info : 0; }
@@ -278,26 +261,24 @@ KASCADE_API kascade_status kascade_rank_list(kascade_ctx* c, const uint64_t* suc
                                              void* stream) {
   cudaStream_t s = as_stream(stream);
   if (n && (!succ || !root_out || !rank_out)) return KASCADE_ERR_INVALID_ARG;
-  const bool async = opts && opts->async;  // its status is read later: no rerun
   KS_TRY(begin_call(c, s, opts));
   Params p = make_params(*c, opts, n);
   kascade_status st = validate_list(*c, succ, n, opts, p, s);
   if (st == KASCADE_OK)
-    st = rank_list_generic(*c, succ, weights ? WKind::U32 : WKind::Unit, weights, n, root_out, rank_out, 0, p, s,
-                           async);
-  st = end_call(c, s, st, opts);
-  if (st != KASCADE_ERR_TIMEOUT || async) return st;
-  // a chain past the write-free chase's hop cap: rank again, checked on the host
-  KS_TRY(begin_call(c, s, opts));
-  st = rank_list_generic(*c, succ, weights ? WKind::U32 : WKind::Unit, weights, n, root_out, rank_out, 0, p, s, true);
+    st = rank_list_generic(*c, succ, weights ? WKind::U32 : WKind::Unit, weights, n, root_out, rank_out, 0, p, s);
   return end_call(c, s, st, opts);
 }
 
-// The host-buffer list call: copies in, ranks (no host wait inside the call
-// unless host_check), copies out.
-kascade_status rank_list_host_call(kascade_ctx* c, const uint64_t* succ, const uint32_t* weights, uint64_t n,
-                                   uint64_t* root_out, uint64_t* rank_out, const kascade_opts* opts,
-                                   cudaStream_t s, bool host_check) {
+// The host-buffer list call: copies in, ranks (no host wait inside the call),
+// copies out.  With opts->async the host buffers belong to the call until
+// kascade_ctx_sync.
+KASCADE_API kascade_status kascade_rank_list_host(kascade_ctx* c, const uint64_t* succ, const uint32_t* weights,
+                                                  uint64_t n, uint64_t* root_out, uint64_t* rank_out,
+                                                  const kascade_opts* opts, void* stream) {
+  cudaStream_t s = as_stream(stream);
+  if (!c) return KASCADE_ERR_INVALID_ARG;
+  if (n && (!succ || !root_out || !rank_out)) return KASCADE_ERR_INVALID_ARG;
+  if (n > MAX_LIST) return KASCADE_ERR_TOO_LARGE;
   KS_TRY(begin_call(c, s, opts));
   Params p = make_params(*c, opts, n);
   kascade_status st = KASCADE_OK;
@@ -313,37 +294,14 @@ kascade_status rank_list_host_call(kascade_ctx* c, const uint64_t* succ, const u
     }
     if (st == KASCADE_OK) st = validate_list(*c, d_succ, n, opts, p, s);
     if (st == KASCADE_OK)
-      st = rank_list_generic(*c, d_succ, d_w ? WKind::U32 : WKind::Unit, d_w, n, d_root, d_rank, 0, p, s,
-                             host_check);
+      st = rank_list_generic(*c, d_succ, d_w ? WKind::U32 : WKind::Unit, d_w, n, d_root, d_rank, 0, p, s);
     if (st == KASCADE_OK) {
       cudaError_t e = cudaMemcpyAsync(root_out, d_root, n * 8, cudaMemcpyDeviceToHost, s);
       if (e == cudaSuccess) e = cudaMemcpyAsync(rank_out, d_rank, n * 8, cudaMemcpyDeviceToHost, s);
       st = cuda_status(e);
     }
   }
-  // opts->async: return once enqueued; the host buffers belong to the call
-  // until kascade_ctx_sync
   return end_call(c, s, st, opts);
-}
-
-KASCADE_API kascade_status kascade_rank_list_host(kascade_ctx* c, const uint64_t* succ, const uint32_t* weights,
-                                                  uint64_t n, uint64_t* root_out, uint64_t* rank_out,
-                                                  const kascade_opts* opts, void* stream) {
-  cudaStream_t s = as_stream(stream);
-  if (!c) return KASCADE_ERR_INVALID_ARG;
-  if (n && (!succ || !root_out || !rank_out)) return KASCADE_ERR_INVALID_ARG;
-  if (n > MAX_LIST) return KASCADE_ERR_TOO_LARGE;
-  kascade_status st = rank_list_host_call(c, succ, weights, n, root_out, rank_out, opts, s, false);
-  if (opts && opts->async) {
-    if (st == KASCADE_OK) {
-      c->host_rerun = kascade_ctx::HostRerun{true, 0, succ, weights, n, root_out, rank_out, *opts, s};
-    }
-    return st;
-  }
-  if (st != KASCADE_ERR_TIMEOUT) return st;
-  // a chain past the write-free chase's hop cap: copy in and rank again,
-  // checked on the host
-  return rank_list_host_call(c, succ, weights, n, root_out, rank_out, opts, s, true);
 }
 
 KASCADE_API kascade_status kascade_sparse_ruling_set(kascade_ctx* c, const kascade_opts* opts, uint64_t* succ_array,
@@ -360,8 +318,7 @@ KASCADE_API kascade_status kascade_sparse_ruling_set(kascade_ctx* c, const kasca
     if (st == KASCADE_OK && !ok) st = KASCADE_ERR_NOT_A_LIST;
   }
   if (st == KASCADE_OK)
-    st = rank_list_generic(*c, succ_array, WKind::I64, rank_array, n, succ_array, (uint64_t*)rank_array, 1, p, s,
-                           true);
+    st = rank_list_generic(*c, succ_array, WKind::I64, rank_array, n, succ_array, (uint64_t*)rank_array, 1, p, s);
   return end_call(c, s, st, opts);
 }
 
@@ -373,7 +330,7 @@ KASCADE_API kascade_status kascade_pointer_doubling(kascade_ctx* c, const kascad
   Params p = make_params(*c, opts, n);
   p.algorithm = KASCADE_ALGO_POINTER_DOUBLING;
   kascade_status st =
-      rank_list_generic(*c, succ_array, WKind::I64, rank_array, n, succ_array, (uint64_t*)rank_array, 1, p, s, true);
+      rank_list_generic(*c, succ_array, WKind::I64, rank_array, n, succ_array, (uint64_t*)rank_array, 1, p, s);
   return end_call(c, s, st, opts);
 }
 
@@ -424,24 +381,21 @@ KASCADE_API kascade_status kascade_root_forest(kascade_ctx* c, const uint64_t* p
   cudaStream_t s = as_stream(stream);
   if (n && (!parent || !root_out || !depth_out)) return KASCADE_ERR_INVALID_ARG;
   if (n > MAX_FOREST) return KASCADE_ERR_TOO_LARGE;
-  const bool async = opts && opts->async;
   KS_TRY(begin_call(c, s, opts));
   Params p = make_params(*c, opts, 2 * n);
   p.algorithm = KASCADE_ALGO_SPARSE_RULING_SET;
-  kascade_status st = root_forest_impl(*c, parent, (uint32_t)n, root_out, depth_out, 0, p, s, async);
-  st = end_call(c, s, st, opts);
-  if (st != KASCADE_ERR_TIMEOUT || async) return st;
-  // a chain past the write-free chase's hop cap: again, checked on the host
-  KS_TRY(begin_call(c, s, opts));
-  st = root_forest_impl(*c, parent, (uint32_t)n, root_out, depth_out, 0, p, s, true);
+  const kascade_status st = root_forest_impl(*c, parent, (uint32_t)n, root_out, depth_out, 0, p, s);
   return end_call(c, s, st, opts);
 }
 
-// The host-buffer forest call: copies in, roots (no host wait inside the call
-// unless host_check), copies out.
-kascade_status root_forest_host_call(kascade_ctx* c, const uint64_t* parent, uint64_t n, uint64_t* root_out,
-                                     uint64_t* depth_out, const kascade_opts* opts, cudaStream_t s,
-                                     bool host_check) {
+// The host-buffer forest call, as kascade_rank_list_host.
+KASCADE_API kascade_status kascade_root_forest_host(kascade_ctx* c, const uint64_t* parent, uint64_t n,
+                                                    uint64_t* root_out, uint64_t* depth_out, const kascade_opts* opts,
+                                                    void* stream) {
+  cudaStream_t s = as_stream(stream);
+  if (!c) return KASCADE_ERR_INVALID_ARG;
+  if (n && (!parent || !root_out || !depth_out)) return KASCADE_ERR_INVALID_ARG;
+  if (n > MAX_FOREST) return KASCADE_ERR_TOO_LARGE;
   KS_TRY(begin_call(c, s, opts));
   Params p = make_params(*c, opts, 2 * n);
   p.algorithm = KASCADE_ALGO_SPARSE_RULING_SET;
@@ -454,35 +408,14 @@ kascade_status root_forest_host_call(kascade_ctx* c, const uint64_t* parent, uin
       d_depth = alloc<uint64_t>(*c, n);
       if (!d_root || !d_depth) st = KASCADE_ERR_OOM;
     }
-    if (st == KASCADE_OK) st = root_forest_impl(*c, d_par, (uint32_t)n, d_root, d_depth, 0, p, s, host_check);
+    if (st == KASCADE_OK) st = root_forest_impl(*c, d_par, (uint32_t)n, d_root, d_depth, 0, p, s);
     if (st == KASCADE_OK) {
       cudaError_t e = cudaMemcpyAsync(root_out, d_root, n * 8, cudaMemcpyDeviceToHost, s);
       if (e == cudaSuccess) e = cudaMemcpyAsync(depth_out, d_depth, n * 8, cudaMemcpyDeviceToHost, s);
       st = cuda_status(e);
     }
   }
-  // opts->async: return once enqueued; the host buffers belong to the call
-  // until kascade_ctx_sync
   return end_call(c, s, st, opts);
-}
-
-KASCADE_API kascade_status kascade_root_forest_host(kascade_ctx* c, const uint64_t* parent, uint64_t n,
-                                                    uint64_t* root_out, uint64_t* depth_out, const kascade_opts* opts,
-                                                    void* stream) {
-  cudaStream_t s = as_stream(stream);
-  if (!c) return KASCADE_ERR_INVALID_ARG;
-  if (n && (!parent || !root_out || !depth_out)) return KASCADE_ERR_INVALID_ARG;
-  if (n > MAX_FOREST) return KASCADE_ERR_TOO_LARGE;
-  kascade_status st = root_forest_host_call(c, parent, n, root_out, depth_out, opts, s, false);
-  if (opts && opts->async) {
-    if (st == KASCADE_OK)
-      c->host_rerun = kascade_ctx::HostRerun{true, 1, parent, nullptr, n, root_out, depth_out, *opts, s};
-    return st;
-  }
-  if (st != KASCADE_ERR_TIMEOUT) return st;
-  // a chain past the write-free chase's hop cap: copy in and root again,
-  // checked on the host
-  return root_forest_host_call(c, parent, n, root_out, depth_out, opts, s, true);
 }
 
 KASCADE_API kascade_status kascade_rank_via_euler_tour(kascade_ctx* c, const kascade_opts* opts, uint64_t* succ_array,
@@ -502,7 +435,7 @@ KASCADE_API kascade_status kascade_rank_via_euler_tour(kascade_ctx* c, const kas
     if (st == KASCADE_OK)
       st = cuda_status(cudaMemcpyAsync(parent_copy, succ_array, n * 8, cudaMemcpyDeviceToDevice, s));
     if (st == KASCADE_OK)
-      st = root_forest_impl(*c, parent_copy, (uint32_t)n, succ_array, (uint64_t*)rank_array, 1, p, s, true);
+      st = root_forest_impl(*c, parent_copy, (uint32_t)n, succ_array, (uint64_t*)rank_array, 1, p, s);
   }
   return end_call(c, s, st, opts);
 }
@@ -544,15 +477,8 @@ KASCADE_API kascade_status kascade_rank_batch(kascade_ctx* c, const kascade_segm
                                               void* stream) {
   cudaStream_t s = as_stream(stream);
   if (total_n && (!segs || !num_segs || !input || !root_out || !rank_out)) return KASCADE_ERR_INVALID_ARG;
-  // Async calls have their status read later and cannot be rerun.
-  const bool async = opts && opts->async;
   KS_TRY(begin_call(c, s, opts));
-  kascade_status st = rank_batch_impl(*c, segs, num_segs, input, weights, total_n, root_out, rank_out, opts, s, async);
-  st = end_call(c, s, st, opts);
-  if (st != KASCADE_ERR_TIMEOUT || async) return st;
-  // a chain past the write-free chase's hop cap: again, checked on the host
-  KS_TRY(begin_call(c, s, opts));
-  st = rank_batch_impl(*c, segs, num_segs, input, weights, total_n, root_out, rank_out, opts, s, true);
+  const kascade_status st = rank_batch_impl(*c, segs, num_segs, input, weights, total_n, root_out, rank_out, opts, s);
   return end_call(c, s, st, opts);
 }
 
@@ -562,7 +488,7 @@ kascade_status rank_batch_device_call(kascade_ctx* c, const kascade_segment* seg
                                       const uint32_t* weights, uint64_t total, uint64_t* root_out,
                                       uint64_t* rank_out, const kascade_opts* opts, cudaStream_t s) {
   KS_TRY(begin_call(c, s, opts));
-  const kascade_status st = rank_batch_impl(*c, segs, nseg, in, weights, total, root_out, rank_out, opts, s, false);
+  const kascade_status st = rank_batch_impl(*c, segs, nseg, in, weights, total, root_out, rank_out, opts, s);
   return end_call(c, s, st, opts);
 }
 kascade_status batch_plan_create(int device, const kascade_segment* segs, uint32_t nseg, const uint64_t* in,

@@ -26,9 +26,6 @@
 //             each walks forward to the first element with outputs; a list
 //             end that is no ruler itself is one of them
 //
-// Calls that must leave roots' outputs untouched (the in-place contract) use
-// the stamping level 0 instead: the sentinel presets would overwrite them.
-//
 // Reference counterparts: the chase of sparse_ruling_set.cpp:147-273 (whose
 // per-element writes are the reference's messages), ruler_propagation.hpp:
 // 148-256 (pull) and post_invert.hpp:195-264 (unreached fix-up).
@@ -42,12 +39,16 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 constexpr uint32_t LOG_CHUNK = 1024;  // entries per warp-owned log chunk
+constexpr int LOG_REFILL = 6;         // idle lanes worth a refill
+constexpr uint32_t LOG_CHAINS_PER_SM = 1024;
 constexpr uint32_t WIN_SHIFT = 20;    // 2^20 elements per window (first partition pass)
 constexpr uint32_t WIN = 1u << WIN_SHIFT;
 constexpr uint32_t SUB_SHIFT = 13;  // 2^13 elements per sub-window (second pass; resolved in shared memory)
 constexpr uint32_t SUB = 1u << SUB_SHIFT;
 constexpr uint32_t SUBS = WIN / SUB;    // sub-windows per window
 constexpr uint32_t MAX_BUCKETS = 4096;  // windows for 2^32 elements
+constexpr uint32_t DIRECT_MAX = 1u << 22;  // one partition pass up to this size (512 sub-windows)
+static_assert(DIRECT_MAX / SUB <= MAX_BUCKETS, "sub-windows per pass");
 constexpr uint32_t CURSOR_STRIDE = 8;   // one 32 B sector per cursor (spreads the atomics)
 constexpr uint32_t PT_THREADS = 256;    // partition: threads per block
 // entries per thread (a tile is PT_THREADS x ITEMS entries) and resident
@@ -69,15 +70,25 @@ __device__ __forceinline__ void st_log(LogEnt* p, uint32_t x, uint32_t id, uint6
   __stcs(reinterpret_cast<uint4*>(p), make_uint4(x, id, (uint32_t)off, (uint32_t)(off >> 32)));
 }
 
-// Warp-cooperative append of one entry per emitting lane.  pos/end describe
-// the warp's current log chunk and are warp-uniform.
-__device__ __forceinline__ void log_append(bool emit, uint32_t x, uint32_t id, uint64_t off, uint32_t& pos,
-                                           uint32_t& end, LogEnt* __restrict__ log, uint32_t* __restrict__ chunk_fill,
+// A warp's place in the log: the chunk it owns (all values warp-uniform).
+struct LogCursor {
+  uint32_t pos = 0, end = 0;
+};
+
+// Warp-cooperative append of one entry per emitting lane.
+__device__ __forceinline__ void log_append(bool emit, uint32_t x, uint32_t id, uint64_t off, LogCursor& cur,
+                                           LogEnt* __restrict__ log, uint32_t* __restrict__ chunk_fill,
                                            uint32_t* __restrict__ chunk_cursor, uint32_t nchunks, uint32_t lane,
                                            uint32_t lt, DevStatus* st) {
   uint32_t m = __ballot_sync(FULL, emit);
+  const uint32_t cnt = (uint32_t)__popc(m);
+  if (cur.pos + cnt < cur.end) {  // all of them fit, and the chunk is not full after
+    if (emit) st_log(log + cur.pos + __popc(m & lt), x, id, off);
+    cur.pos += cnt;
+    return;
+  }
   while (m != 0u) {
-    if (pos == end) {
+    if (cur.pos == cur.end) {
       uint32_t ch = 0;
       if (lane == 0) ch = atomicAdd(chunk_cursor, 1u);
       ch = __shfl_sync(FULL, ch, 0);
@@ -86,147 +97,119 @@ __device__ __forceinline__ void log_append(bool emit, uint32_t x, uint32_t id, u
         if (lane == 0) set_error(st, KASCADE_ERR_NOT_A_LIST, ch);
         return;
       }
-      pos = ch * LOG_CHUNK;
-      end = pos + LOG_CHUNK;
+      cur.pos = ch * LOG_CHUNK;
+      cur.end = cur.pos + LOG_CHUNK;
     }
-    const uint32_t take = min((uint32_t)__popc(m), end - pos);
+    const uint32_t take = min((uint32_t)__popc(m), cur.end - cur.pos);
     const uint32_t my = __popc(m & lt);
     const bool mine = emit && my < take;
-    if (mine) st_log(log + pos + my, x, id, off);
-    const uint32_t served = __ballot_sync(FULL, mine);
-    m &= ~served;
+    if (mine) st_log(log + cur.pos + my, x, id, off);
+    m &= ~__ballot_sync(FULL, mine);
     emit = emit && !mine;
-    pos += take;
-    if (pos == end && lane == 0) chunk_fill[(pos - 1) / LOG_CHUNK] = LOG_CHUNK;
+    cur.pos += take;
+    if (cur.pos == cur.end && lane == 0) chunk_fill[(cur.pos - 1) / LOG_CHUNK] = LOG_CHUNK;
   }
 }
 
-// The read-only chase: rulers and their order as in k_chase.  Every ruler and
-// every element a chain passes is logged; a list's end is not (any number of
-// chains may end there).
-template <int C>
-__global__ void __launch_bounds__(512) k_chase_log(const Rec* __restrict__ rec, Extent ext, Rulers rl,
-                                                   uint32_t rulers, Heads heads, Rec* __restrict__ rec_next, uint32_t* __restrict__ rootel_next,
-                                                   uint32_t* __restrict__ work, LogEnt* __restrict__ log,
-                                                   uint32_t* __restrict__ chunk_fill,
+// The read-only chase: one chain per thread, rulers and chain ends as in
+// k_chase.  Every ruler and every element a chain passes is logged; a list's
+// end is not (any number of chains may end there).  Bound by the random reads'
+// DRAM fetches at large sizes and by instructions at L2-resident ones; 1024
+// chains per SM are enough for either (2^28 elements: 768 / 1024 / 1536 / 2048
+// chains 7.27 / 7.30 / 7.41 / 7.48 ms; two or four chains per thread are
+// slower).
+template <class F>
+__global__ void __launch_bounds__(512) k_chase_log(const typename F::R* __restrict__ rec, Extent ext, Rulers rl,
+                                                   uint32_t rulers, Heads heads, Rulers rl_next,
+                                                   Rec* __restrict__ rec_next, uint4* __restrict__ stamp_next,
+                                                   uint32_t* __restrict__ rootel_next, uint32_t* __restrict__ work,
+                                                   LogEnt* __restrict__ log, uint32_t* __restrict__ chunk_fill,
                                                    uint32_t* __restrict__ chunk_cursor, uint32_t nchunks,
-                                                   uint32_t max_hops, DevStatus* st) {
-  constexpr uint32_t BATCH = 32u * C;
+                                                   uint32_t hop_cap, DevStatus* st) {
   const uint32_t n = ext.get();
   const uint32_t r = rulers + heads.get();
   if (ext.add && blockIdx.x == 0 && threadIdx.x == 0) st->counter[1] = n;  // level 0's size, reported by the call
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t lt = lanemask_lt();
-  uint32_t cid[C], cx[C], hops[C];
-  uint64_t acc[C];
-  uint32_t act = 0, fresh = 0;  // bit c: chain c runs / has not read its ruler's record yet
-  uint32_t q_base = 0, q_left = 0;
-  bool drained = false;
-  uint32_t lpos = 0, lend = 0;  // warp-uniform log chunk
-#pragma unroll
-  for (int c = 0; c < C; ++c) {
-    cid[c] = cx[c] = hops[c] = 0;
-    acc[c] = 0;
-  }
-  auto end_chain = [&](uint32_t id, uint64_t dist, uint32_t next, uint32_t root) {
-    Rec o;
-    o.a = dist;
-    o.b = next;
-    o.c = TAG_UNREACHED;
-    st_rec_cg(rec_next + id, o);
-    rootel_next[id] = root;
-  };
-  while (true) {
-    if (!drained) {
-#pragma unroll
-      for (int c = 0; c < C; ++c) {
-        bool need = !((act >> c) & 1u);
-        uint32_t m = __ballot_sync(FULL, need);
-        while (m != 0u && !drained) {
-          if (q_left == 0u) {
-            uint32_t b = 0;
-            if (lane == 0) b = atomicAdd(work, BATCH);
-            b = __shfl_sync(FULL, b, 0);
-            if (b >= r) {
-              drained = true;
-              break;
-            }
-            q_base = b;
-            q_left = min(BATCH, r - b);
-          }
-          const uint32_t take = min((uint32_t)__popc(m), q_left);
-          const uint32_t my_rank = __popc(m & lt);
-          const bool mine = need && my_rank < take;
-          if (mine) {
-            const uint32_t id = q_base + my_rank;
-            const uint64_t x0 = id < rulers ? rl.elem(id) : __ldg(heads.elem + (id - rulers));
-            uint32_t j;
-            if (x0 >= n) {
-              end_chain(id, 0, id, 0);  // the last block's ruler, beyond the elements
-            } else if (id >= rulers && rl.is((uint32_t)x0, &j)) {
-              end_chain(id, 0, j, 0);  // a head that is a ruler itself
-            } else {
-              cid[c] = id;
-              cx[c] = (uint32_t)x0;
-              acc[c] = 0;
-              hops[c] = 0;
-              act |= 1u << c;
-              fresh |= 1u << c;
-            }
-          }
-          m &= ~__ballot_sync(FULL, mine);
-          need = need && !mine;
-          q_base += take;
-          q_left -= take;
-        }
-      }
+  const uint32_t first = gridDim.x * blockDim.x;  // ids from here on are handed out by the counter
+  uint32_t id = 0, x = 0, hops = 0;
+  uint64_t acc = 0;
+  Hop h{0, 0, false};  // the record of x, asked for
+  bool act = false, own = false;  // own: x is the chain's first element
+  auto begin = [&](uint32_t i) {
+    id = i;
+    const uint64_t x0 = i < rulers ? rl.elem(i) : __ldg(heads.elem + (i - rulers));
+    uint32_t j;
+    if (x0 >= n) {
+      end_chain(rec_next, stamp_next, rl_next, i, 0, i);  // the last block's ruler, beyond the elements
+    } else if (i >= rulers && rl.is((uint32_t)x0, &j)) {
+      end_chain(rec_next, stamp_next, rl_next, i, 0, j);  // a head that is a ruler itself
+    } else {
+      x = (uint32_t)x0;
+      h = F::hop(rec + x);
+      acc = 0;
+      hops = 0;
+      act = own = true;
     }
-    if (!__any_sync(FULL, act != 0u)) {
-      if (drained) break;
+  };
+  const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i0 < r) begin(i0);
+  bool more = first < r;  // warp-uniform
+  LogCursor cur;
+  while (true) {
+    const uint32_t running = __ballot_sync(FULL, act);
+    if (more && (running == 0u || __popc(running) <= 32 - LOG_REFILL)) {
+      const uint32_t idle = ~running;
+      uint32_t b = 0;
+      if (lane == 0) b = first + atomicAdd(work, (uint32_t)__popc(idle));
+      b = __shfl_sync(FULL, b, 0);
+      if (b >= r) more = false;
+      const uint32_t i = b + __popc(idle & lt);
+      if (!act && i < r) begin(i);
       continue;
     }
-    Rec rr[C];
-#pragma unroll
-    for (int c = 0; c < C; ++c)
-      if ((act >> c) & 1u) rr[c] = ld_rec_cg(rec + cx[c]);
-#pragma unroll
-    for (int c = 0; c < C; ++c) {
-      bool emit = false;
-      const uint32_t x = cx[c];
-      const uint64_t d = acc[c];
-      if ((act >> c) & 1u) {
-        const uint32_t y = rr[c].b;
-        const bool first = (fresh >> c) & 1u;
-        fresh &= ~(1u << c);
-        emit = first || y != x;
-        if (y == x) {  // the list's end
-          end_chain(cid[c], d + rr[c].a, cid[c], x);
-          act &= ~(1u << c);
-        } else {
-          acc[c] = d + rr[c].a;
-          cx[c] = y;
-          uint32_t j;
-          if (rl.is(y, &j)) {
-            // back at its own ruler: a rootless cycle holding one ruler
-            if (j == cid[c]) set_error(st, KASCADE_ERR_CYCLE, j);
-            end_chain(cid[c], acc[c], j, 0);
-            act &= ~(1u << c);
-          } else if (++hops[c] > max_hops) {
-            // Ruler gaps are geometric: a chain longer than max_hops (64x the
-            // mean spacing, probability ~e^-64) is treated as a sign of an
-            // invalid input (a ruler-free cycle behind a ruler); the chain
-            // stops and the host reruns level 0 on the stamping path, which
-            // tells the two cases apart exactly.
-            atomicOr(&st->counter[0], 1ull);
-            end_chain(cid[c], 0, cid[c], 0);  // keeps the next level's records in range
-            act &= ~(1u << c);
+    if (running == 0u) {
+      if (!more) break;
+      continue;
+    }
+    bool emit = false;
+    const uint32_t lx = x, lid = id;
+    const uint64_t ld = acc;
+    if (act) {
+      const uint32_t y = h.b;
+      const uint64_t d = acc + h.w;
+      const bool end = y == x, stop = end || h.ruler;
+      emit = own || !end;
+      own = false;
+      if (!stop) {
+        h = F::hop(rec + y);
+        acc = d;
+        x = y;
+        if (++hops == hop_cap) {
+          hops = 0;
+          if (endless<F>(rec, y)) {
+            set_error(st, KASCADE_ERR_CYCLE, id);
+            end_chain(rec_next, stamp_next, rl_next, id, 0, id);
+            act = false;
           }
         }
+      } else {
+        uint32_t next = id;
+        if (end) {
+          rootel_next[id] = x;
+        } else {
+          next = rl.block_of(y);
+          // back at its own ruler: a rootless cycle holding one ruler
+          if (next == id) set_error(st, KASCADE_ERR_CYCLE, id);
+        }
+        end_chain(rec_next, stamp_next, rl_next, id, d, next);
+        act = false;
       }
-      log_append(emit, x, cid[c], d, lpos, lend, log, chunk_fill, chunk_cursor, nchunks, lane, lt, st);
     }
+    log_append(emit, lx, lid, ld, cur, log, chunk_fill, chunk_cursor, nchunks, lane, lt, st);
   }
-  if (lane == 0 && lend != 0 && lpos != lend) chunk_fill[(lend - 1) / LOG_CHUNK] = LOG_CHUNK - (lend - lpos);
+  if (lane == 0 && cur.end != 0 && cur.pos != cur.end)
+    chunk_fill[(cur.end - 1) / LOG_CHUNK] = LOG_CHUNK - (cur.end - cur.pos);
 }
 
 // Exclusive prefix sum of v[0, m) in place (shared memory, m <= MAX_BUCKETS);
@@ -268,7 +251,9 @@ __device__ uint32_t block_exclusive_scan(uint32_t* v, uint32_t m) {
 // consecutive threads: every global store is part of a contiguous run, so
 // L2 sees whole lines instead of one 16 B piece per store.
 //   FROM_LOG (first pass): tiles of PT_TILE_CHUNKS log chunks, buckets are
-//     windows of WIN elements.  Each log entry (element, ruler id, distance)
+//     windows of 2^shift elements -- the sub-windows themselves where there
+//     are few enough, and there is no second pass then.  Each log entry
+//     (element, ruler id, distance)
 //     is resolved on the way: rank = rank(ruler) - distance, root =
 //     root(ruler), from the rulers' results of the recursion.  A log chunk
 //     holds the entries of a few hundred chains, so most of these lookups
@@ -283,7 +268,7 @@ template <bool FROM_LOG, uint32_t ITEMS, uint32_t BLOCKS>
 __global__ void __launch_bounds__(PT_THREADS, BLOCKS) k_partition(const LogEnt* __restrict__ src,
                                                              const uint32_t* __restrict__ src_info, uint32_t nchunks,
                                                              const Out* __restrict__ out1, uint32_t limit,
-                                                             uint32_t nb, LogEnt* __restrict__ dst,
+                                                             uint32_t shift, uint32_t nb, LogEnt* __restrict__ dst,
                                                              uint32_t* __restrict__ dcursor,
                                                              const uint32_t* __restrict__ used, DevStatus* st) {
   constexpr uint32_t PT_TILE = PT_THREADS * ITEMS;
@@ -341,7 +326,7 @@ __global__ void __launch_bounds__(PT_THREADS, BLOCKS) k_partition(const LogEnt* 
       pos[k] = NO_ROOT;
       const uint32_t x = v[k].x;
       if (x < limit) {
-        const uint32_t b = FROM_LOG ? x >> WIN_SHIFT : (x >> SUB_SHIFT) & (SUBS - 1);
+        const uint32_t b = FROM_LOG ? x >> shift : (x >> SUB_SHIFT) & (SUBS - 1);
         pos[k] = atomicAdd(&cnt[b], 1u);
       }
     }
@@ -366,21 +351,21 @@ __global__ void __launch_bounds__(PT_THREADS, BLOCKS) k_partition(const LogEnt* 
     for (uint32_t k = 0; k < ITEMS; ++k) {
       if (pos[k] == NO_ROOT) continue;
       const uint32_t x = v[k].x;
-      const uint32_t b = FROM_LOG ? x >> WIN_SHIFT : (x >> SUB_SHIFT) & (SUBS - 1);
+      const uint32_t b = FROM_LOG ? x >> shift : (x >> SUB_SHIFT) & (SUBS - 1);
       stage[cnt[b] + pos[k]] = v[k];
     }
     if (one_per_thread && threadIdx.x < nbk) gbase[threadIdx.x] = g_mine;
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < total; i += PT_THREADS) {
       const uint4 e = stage[i];
-      const uint32_t b = FROM_LOG ? e.x >> WIN_SHIFT : (e.x >> SUB_SHIFT) & (SUBS - 1);
+      const uint32_t b = FROM_LOG ? e.x >> shift : (e.x >> SUB_SHIFT) & (SUBS - 1);
       const uint32_t p = gbase[b] + (i - cnt[b]);
-      const uint32_t cap = FROM_LOG ? WIN : SUB;
+      const uint32_t cap = FROM_LOG ? 1u << shift : SUB;
       if (p >= cap) {
         set_error(st, KASCADE_ERR_NOT_A_LIST, e.x);  // an element logged twice
         continue;
       }
-      const uint64_t d = FROM_LOG ? (uint64_t)b * WIN + p : (uint64_t)w * WIN + (uint64_t)b * SUB + p;
+      const uint64_t d = FROM_LOG ? ((uint64_t)b << shift) + p : (uint64_t)w * WIN + (uint64_t)b * SUB + p;
       __stcg(reinterpret_cast<uint4*>(dst + d), e);
     }
     __syncthreads();
@@ -392,7 +377,8 @@ __global__ void __launch_bounds__(PT_THREADS, BLOCKS) k_partition(const LogEnt* 
 // element, then the sub-window's outputs are written densely.  Elements
 // without an entry were reached by no chain: their root output becomes
 // NOT_REACHED and they join the unreached list.  A batch's roots are written
-// relative to their instance.
+// relative to their instance, depths modulo 2^32.  keep_roots: a root's rank
+// output stays as it is (its root output already names it).
 __global__ void __launch_bounds__(FIN_THREADS, 2) k_place(const LogEnt* __restrict__ part2,
                                                             const uint32_t* __restrict__ cursor2, uint32_t nb,
                                                             uint32_t limit, uint64_t* __restrict__ root_out,
@@ -401,7 +387,9 @@ __global__ void __launch_bounds__(FIN_THREADS, 2) k_place(const LogEnt* __restri
                                                             uint32_t* __restrict__ ucount, uint32_t ucap,
                                                             const uint64_t* __restrict__ seg_off,
                                                             const uint32_t* __restrict__ hint, uint32_t nseg,
-                                                            const uint32_t* __restrict__ plus_one, DevStatus* st) {
+                                                            const uint32_t* __restrict__ plus_one, int tour,
+                                                            const uint32_t* __restrict__ seg_tour, int keep_roots,
+                                                            DevStatus* st) {
   extern __shared__ __align__(16) unsigned char smraw[];
   unsigned long long* rank_s = reinterpret_cast<unsigned long long*>(smraw);  // SUB entries
   uint32_t* root_s = reinterpret_cast<uint32_t*>(rank_s + SUB);               // SUB entries
@@ -443,12 +431,14 @@ __global__ void __launch_bounds__(FIN_THREADS, 2) k_place(const LogEnt* __restri
     // and the next instance's; a thread's elements only move forward
     uint32_t jseg = 0;
     unsigned long long cur_off = 0, next_off = ~0ull;
+    bool depths = tour != 0;
     if (seg_off) {
       const uint32_t x0 = lo + threadIdx.x;
       jseg = __ldg(hint + (x0 >> 12));
       while (jseg + 1 < nseg && __ldg(seg_off + jseg + 1) <= x0) ++jseg;
       cur_off = __ldg(seg_off + jseg);
       next_off = jseg + 1 < nseg ? __ldg(seg_off + jseg + 1) : ~0ull;
+      if (seg_tour) depths = (__ldg(seg_tour + (jseg >> 5)) >> (jseg & 31)) & 1u;
     }
     for (uint32_t i0 = 0; i0 < len; i0 += FIN_THREADS) {
       const uint32_t i = i0 + threadIdx.x;
@@ -461,13 +451,15 @@ __global__ void __launch_bounds__(FIN_THREADS, 2) k_place(const LogEnt* __restri
             ++jseg;
             cur_off = next_off;
             next_off = jseg + 1 < nseg ? __ldg(seg_off + jseg + 1) : ~0ull;
+            if (seg_tour) depths = (__ldg(seg_tour + (jseg >> 5)) >> (jseg & 31)) & 1u;
           }
         }
         const unsigned long long ibase = un ? 0ull : cur_off;
         __stcs(reinterpret_cast<unsigned long long*>(root_out) + lo + i,
                un ? NOT_REACHED : (unsigned long long)r - ibase);
-        const unsigned long long add = plus_one ? (plus_s[i >> 5] >> (i & 31)) & 1u : 0u;
-        __stcs(reinterpret_cast<unsigned long long*>(rank_out) + lo + i, un ? 0ull : rank_s[i] + add);
+        unsigned long long k = un ? 0ull : rank_s[i];
+        if (depths) k = (uint32_t)k + ((plus_s[i >> 5] >> (i & 31)) & 1u);
+        if (!(keep_roots && (un || r == lo + i))) __stcs(reinterpret_cast<unsigned long long*>(rank_out) + lo + i, k);
       }
       const uint32_t m = __ballot_sync(FULL, un);
       if (m == 0u) continue;
@@ -493,36 +485,42 @@ __global__ void __launch_bounds__(FIN_THREADS, 2) k_place(const LogEnt* __restri
 // root seen set comes with its rank.  Elements at or above `limit` (tour down
 // edges) have no outputs and are walked through.  Roots already relative to
 // their instance stay so (a walker and the element it stops at share an
-// instance); a list end's root is made relative here.  plus_one: outputs that
-// are one more than their rank.
-__global__ void __launch_bounds__(256) k_walk_unreached(const Rec* __restrict__ rec, const uint32_t* __restrict__ ulist,
+// instance); a list end's root is made relative here.  keep_roots: a root's
+// rank output is the caller's, its rank 0.
+template <class F>
+__global__ void __launch_bounds__(256) k_walk_unreached(const typename F::R* __restrict__ rec,
+                                                        const uint32_t* __restrict__ ulist,
                                                         const uint32_t* __restrict__ ucount, uint32_t ucap, uint32_t n,
                                                         uint32_t limit, uint64_t* root_out, uint64_t* rank_out,
                                                         const uint64_t* __restrict__ seg_off,
                                                         const uint32_t* __restrict__ hint, uint32_t nseg,
-                                                        const uint32_t* __restrict__ plus_one, DevStatus* st) {
+                                                        const uint32_t* __restrict__ plus_one, int tour,
+                                                        const uint32_t* __restrict__ seg_tour, int keep_roots,
+                                                        DevStatus* st) {
   const uint32_t cnt = min(*ucount, ucap);
-  auto extra = [&](uint32_t x) -> uint64_t { return plus_one ? (__ldg(plus_one + (x >> 5)) >> (x & 31)) & 1u : 0u; };
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
     const uint32_t u = ulist[i];
+    uint64_t off = 0;
+    bool depths = tour != 0;
+    if (seg_off) {
+      uint32_t j = __ldg(hint + (u >> 12));
+      while (j + 1 < nseg && __ldg(seg_off + j + 1) <= u) ++j;
+      off = __ldg(seg_off + j);
+      if (seg_tour) depths = (__ldg(seg_tour + (j >> 5)) >> (j & 31)) & 1u;
+    }
+    auto extra = [&](uint32_t x) -> uint64_t { return depths ? (__ldg(plus_one + (x >> 5)) >> (x & 31)) & 1u : 0u; };
     uint64_t acc = 0;
-    uint32_t y = u, mark = u, power = 1, lam = 0, hops = 0;
+    uint32_t y = u, mark = u, hops = 0;
     unsigned long long base_root = NOT_REACHED;
     bool ok = true;
     while (true) {
-      const Rec r = ld_rec_cg(rec + y);
-      acc += r.a;
-      if (r.b == y) {  // the list's end
-        uint64_t off = 0;
-        if (seg_off) {
-          uint32_t j = __ldg(hint + (y >> 12));
-          while (j + 1 < nseg && __ldg(seg_off + j + 1) <= y) ++j;
-          off = __ldg(seg_off + j);
-        }
+      const Hop h = F::hop(rec + y);
+      acc += h.w;
+      if (h.b == y) {  // the list's end
         base_root = y - off;
         break;
       }
-      y = r.b;
+      y = h.b;
       if (y >= n) {  // not reachable for a validated input; keeps every load in range
         set_error(st, KASCADE_ERR_OUT_OF_RANGE, u);
         ok = false;
@@ -532,32 +530,24 @@ __global__ void __launch_bounds__(256) k_walk_unreached(const Rec* __restrict__ 
         base_root = __ldcg(reinterpret_cast<const unsigned long long*>(root_out) + y);
         if (base_root != NOT_REACHED) {
           __threadfence();
-          acc += __ldcg(reinterpret_cast<const unsigned long long*>(rank_out) + y) - extra(y);
+          if (base_root + off != y || !keep_roots)
+            acc += __ldcg(reinterpret_cast<const unsigned long long*>(rank_out) + y) - extra(y);
           break;
         }
       }
-      if (y == mark || ++hops > n) {
+      if (y == mark) {
         set_error(st, KASCADE_ERR_CYCLE, u);
         ok = false;
         break;
       }
-      if (++lam == power) {
-        mark = y;
-        power <<= 1;
-        lam = 0;
-      }
+      ++hops;
+      if ((hops & (hops - 1)) == 0) mark = y;
     }
     if (!ok) continue;
-    rank_out[u] = acc + extra(u);
+    if (!(keep_roots && base_root + off == u)) rank_out[u] = (depths ? (uint32_t)acc : acc) + extra(u);
     __threadfence();
     root_out[u] = base_root;
   }
-}
-
-// A chain that hit the hop cap, as a status: the device-driven call then
-// reruns on the host-driven path, whose level 0 tells the cases apart.
-__global__ void k_hop_cap_status(DevStatus* st) {
-  if (st->counter[0]) set_error(st, KASCADE_ERR_TIMEOUT, st->counter[0]);
 }
 
 constexpr uint32_t TILE1 = PT_THREADS * P1_ITEMS, TILE2 = PT_THREADS * P2_ITEMS;
@@ -582,113 +572,95 @@ kascade_status raise_smem_limits() {
   return KASCADE_OK;
 }
 
-int g_chase_occ[5][3] = {{-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1}};
-
-template <int C>
+template <class F>
 unsigned chase_grid(const kascade_ctx& ctx, uint32_t r, uint32_t block) {
-  const int bi = block == 128 ? 0 : block == 512 ? 2 : 1;
-  if (g_chase_occ[C][bi] < 0) {
-    int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_chase_log<C>, (int)block, 0) != cudaSuccess) {
-      cudaGetLastError();
-      nb = 1;
-    }
-    g_chase_occ[C][bi] = nb < 1 ? 1 : nb;
-  }
-  unsigned grid = (unsigned)(ctx.usable_sms() * g_chase_occ[C][bi]);
-  const uint64_t warps_per_block = block / 32;
-  const uint64_t need = ((uint64_t)r + 32ull * C - 1) / (32ull * C);
-  const uint64_t need_blocks = (need + warps_per_block - 1) / warps_per_block;
-  if (need_blocks < grid) grid = (unsigned)(need_blocks ? need_blocks : 1);
-  return grid;
+  const uint64_t grid = (uint64_t)ctx.usable_sms() * std::max(1u, LOG_CHAINS_PER_SM / block);
+  return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(grid, ((uint64_t)r + block - 1) / block));
 }
 
-}  // namespace
+// The chase's log and its size.
+struct Log {
+  LogEnt* ent = nullptr;
+  uint32_t* fill = nullptr;  // per chunk
+  uint32_t* cursor = nullptr;
+  uint32_t nchunks = 0;
+};
 
-kascade_status rank_level0_log(kascade_ctx& ctx, const Rec* rec, uint32_t n, const Extent& ext, const Heads& heads,
-                               const LogTarget& t, const Params& p, cudaStream_t s, bool host_check) {
+template <class F>
+kascade_status rank_level0_log_as(kascade_ctx& ctx, const Level0& l0, uint32_t n, const Extent& ext,
+                                  const Heads& heads, const LogTarget& t, const Params& p, cudaStream_t s) {
   Levels lv;
   KS_TRY(plan_levels(ctx, n, heads, p, &lv));
   const uint32_t r = lv.n[1];
-  const int C = (p.chains == 1 || p.chains == 4) ? (int)p.chains : 2;
   const uint32_t block = p.block;
-  const unsigned grid = C == 1   ? chase_grid<1>(ctx, r, block)
-                        : C == 4 ? chase_grid<4>(ctx, r, block)
-                                 : chase_grid<2>(ctx, r, block);
+  const unsigned grid = chase_grid<F>(ctx, r, block);
   const uint64_t warps = (uint64_t)grid * (block / 32);
-  const uint32_t nchunks = (uint32_t)(((uint64_t)n + LOG_CHUNK - 1) / LOG_CHUNK + warps + 1);
+  Log log;
+  log.nchunks = (uint32_t)(((uint64_t)n + LOG_CHUNK - 1) / LOG_CHUNK + warps + 1);
   const uint32_t limit = t.limit < n ? t.limit : n;
   const uint32_t nb = (uint32_t)(((uint64_t)limit + WIN - 1) / WIN);
   const uint32_t nb1 = nb ? nb : 1;
   const uint64_t cursor_words = (uint64_t)nb1 * (SUBS + 1) * CURSOR_STRIDE;
-  LogEnt* log = alloc<LogEnt>(ctx, (uint64_t)nchunks * LOG_CHUNK);
+  log.ent = alloc<LogEnt>(ctx, (uint64_t)log.nchunks * LOG_CHUNK);
   // zeroed by one memset: chunk cursor, unreached count; the partition
   // cursors; the chunks' fill counts
-  const uint64_t zero_words = 8 + cursor_words + nchunks;
+  const uint64_t zero_words = 8 + cursor_words + log.nchunks;
   uint32_t* zero = alloc<uint32_t>(ctx, zero_words);
-  if (!log || !zero) return KASCADE_ERR_OOM;
+  if (!log.ent || !zero) return KASCADE_ERR_OOM;
   KS_CUDA(cudaMemsetAsync(zero, 0, sizeof(uint32_t) * zero_words, s));
-  uint32_t* chunk_cursor = zero + 0;
+  log.cursor = zero + 0;
   uint32_t* ucount = zero + 1;
   uint32_t* cursor1 = zero + 8;
   uint32_t* cursor2 = cursor1 + (uint64_t)nb1 * CURSOR_STRIDE;
-  uint32_t* chunk_fill = cursor1 + cursor_words;
-  const uint64_t cap = p.max_chain ? p.max_chain : 64ull * p.spacing0 + 1024;
-  const uint32_t max_hops = cap < n ? (uint32_t)cap : n;
+  log.fill = cursor1 + cursor_words;
   {
     ProfScope ps(ctx, "chase", s);
-    uint32_t* work = &ctx.d_status->work[0];
-    switch (C) {
-      case 1:
-        k_chase_log<1><<<grid, block, 0, s>>>(rec, ext, lv.rulers[0], lv.r[0], lv.heads, lv.rec[1], lv.rootel[1], work,
-                                              log, chunk_fill, chunk_cursor, nchunks, max_hops, ctx.d_status);
-        break;
-      case 4:
-        k_chase_log<4><<<grid, block, 0, s>>>(rec, ext, lv.rulers[0], lv.r[0], lv.heads, lv.rec[1], lv.rootel[1], work,
-                                              log, chunk_fill, chunk_cursor, nchunks, max_hops, ctx.d_status);
-        break;
-      default:
-        k_chase_log<2><<<grid, block, 0, s>>>(rec, ext, lv.rulers[0], lv.r[0], lv.heads, lv.rec[1], lv.rootel[1], work,
-                                              log, chunk_fill, chunk_cursor, nchunks, max_hops, ctx.d_status);
-    }
+    k_chase_log<F><<<grid, block, 0, s>>>(l0.records<F>(), ext, lv.rulers[0], lv.r[0], lv.heads, lv.rulers[1],
+                                          lv.rec[1], lv.stamp[1], lv.rootel[1], &ctx.d_status->work[0], log.ent,
+                                          log.fill, log.cursor, log.nchunks, hop_cap(lv.rulers[0]), ctx.d_status);
     KS_CHECK_LAUNCH();
   }
-  if (host_check) {
-    // a chain hit the hop cap: let the caller rerun level 0 on the stamping path
-    uint32_t over = 0;
-    KS_TRY(read_u32(ctx, reinterpret_cast<const uint32_t*>(&ctx.d_status->counter[0]), &over, s));
-    if (over) return KASCADE_ERR_TIMEOUT;
-  } else {
-    k_hop_cap_status<<<1, 1, 0, s>>>(ctx.d_status);
-    KS_CHECK_LAUNCH();
-  }
-  KS_TRY(rank_deep(ctx, lv, p, s));
+  KS_TRY(rank_deep(ctx, lv, s));
 
-  // first pass: log -> windows (part); second pass: windows -> sub-windows,
-  // into the log's memory when it is large enough (the log is dead by then)
-  const uint64_t part2_need = (((uint64_t)limit + SUB - 1) / SUB) * SUB;
-  LogEnt* part = alloc<LogEnt>(ctx, (uint64_t)nb1 * WIN);
-  LogEnt* part2 = (uint64_t)nchunks * LOG_CHUNK >= part2_need ? log : alloc<LogEnt>(ctx, part2_need ? part2_need : 1);
+  // Up to DIRECT_MAX elements the log goes straight to the sub-windows;
+  // larger ones in two passes, windows (part), then sub-windows into the log's
+  // memory when it is large enough (the log is dead by then).
+  const bool direct = limit <= DIRECT_MAX;
+  const uint32_t nsub = (uint32_t)(((uint64_t)limit + SUB - 1) / SUB);
+  const uint64_t part2_need = (uint64_t)nsub * SUB;
+  LogEnt* part = alloc<LogEnt>(ctx, direct ? std::max<uint64_t>(part2_need, 1) : (uint64_t)nb1 * WIN);
+  LogEnt* part2 = direct                                                ? part
+                  : (uint64_t)log.nchunks * LOG_CHUNK >= part2_need ? log.ent
+                                                                    : alloc<LogEnt>(ctx, part2_need ? part2_need : 1);
   if (!part || !part2) return KASCADE_ERR_OOM;
-  const size_t smem1 = TILE1 * sizeof(LogEnt) + 2 * sizeof(uint32_t) * nb1;
-  const size_t smem2 = TILE2 * sizeof(LogEnt) + 2 * sizeof(uint32_t) * SUBS;
   KS_TRY(raise_smem_limits());
-  {
+  if (direct) {
     ProfScope ps(ctx, "resolve", s);
-    const uint32_t tiles1 = (nchunks + TILE1 / LOG_CHUNK - 1) / (TILE1 / LOG_CHUNK);
-    k_part1<<<(unsigned)std::min<uint64_t>(tiles1, (uint64_t)ctx.usable_sms() * P1_BLOCKS), PT_THREADS, smem1, s>>>(
-        log, chunk_fill, nchunks, lv.out[1], limit, nb, part, cursor1, chunk_cursor, ctx.d_status);
+    const uint32_t tiles = (log.nchunks + TILE1 / LOG_CHUNK - 1) / (TILE1 / LOG_CHUNK);
+    const size_t smem = TILE1 * sizeof(LogEnt) + 2 * sizeof(uint32_t) * std::max(nsub, 1u);
+    k_part1<<<(unsigned)std::min<uint64_t>(tiles, (uint64_t)ctx.usable_sms() * P1_BLOCKS), PT_THREADS, smem, s>>>(
+        log.ent, log.fill, log.nchunks, lv.out[1], limit, SUB_SHIFT, nsub, part, cursor2, log.cursor, ctx.d_status);
     KS_CHECK_LAUNCH();
+  } else {
+    const size_t smem1 = TILE1 * sizeof(LogEnt) + 2 * sizeof(uint32_t) * nb1;
+    const size_t smem2 = TILE2 * sizeof(LogEnt) + 2 * sizeof(uint32_t) * SUBS;
+    {
+      ProfScope ps(ctx, "resolve", s);
+      const uint32_t tiles1 = (log.nchunks + TILE1 / LOG_CHUNK - 1) / (TILE1 / LOG_CHUNK);
+      k_part1<<<(unsigned)std::min<uint64_t>(tiles1, (uint64_t)ctx.usable_sms() * P1_BLOCKS), PT_THREADS, smem1, s>>>(
+          log.ent, log.fill, log.nchunks, lv.out[1], limit, WIN_SHIFT, nb, part, cursor1, log.cursor, ctx.d_status);
+      KS_CHECK_LAUNCH();
+    }
+    const uint32_t tiles2 = nb * (WIN / TILE2);
+    if (tiles2) {
+      ProfScope ps(ctx, "partition", s);
+      k_part2<<<(unsigned)std::min<uint64_t>(tiles2, (uint64_t)ctx.usable_sms() * P2_BLOCKS), PT_THREADS, smem2, s>>>(
+          part, cursor1, 0, nullptr, limit, 0, nb, part2, cursor2, nullptr, ctx.d_status);
+      KS_CHECK_LAUNCH();
+    }
   }
-  const uint32_t tiles2 = nb * (WIN / TILE2);
-  if (tiles2) {
-    ProfScope ps(ctx, "partition", s);
-    k_part2<<<(unsigned)std::min<uint64_t>(tiles2, (uint64_t)ctx.usable_sms() * P2_BLOCKS), PT_THREADS, smem2, s>>>(
-        part, cursor1, 0, nullptr, limit, nb, part2, cursor2, nullptr, ctx.d_status);
-    KS_CHECK_LAUNCH();
-  }
-  // the first pass's output is dead after the second: it holds the unreached list
-  uint32_t* ulist = reinterpret_cast<uint32_t*>(part);
+  // the first pass's source or output is dead by now: it holds the unreached list
+  uint32_t* ulist = reinterpret_cast<uint32_t*>(direct ? log.ent : part);
   const uint32_t ucap = limit;
   {
     ProfScope ps(ctx, "place", s);
@@ -696,16 +668,26 @@ kascade_status rank_level0_log(kascade_ctx& ctx, const Rec* rec, uint32_t n, con
     const size_t smem = SUB * (sizeof(unsigned long long) + sizeof(uint32_t));
     k_place<<<(unsigned)std::max<uint64_t>(1, std::min<uint64_t>(items, (uint64_t)ctx.usable_sms() * 2)),
                 FIN_THREADS, smem, s>>>(part2, cursor2, nb, limit, t.root, t.rank, ulist, ucount, ucap, t.seg_off,
-                                        t.hint, t.nseg, t.plus_one, ctx.d_status);
+                                        t.hint, t.nseg, t.plus_one, t.tour, t.seg_tour, t.keep_roots, ctx.d_status);
     KS_CHECK_LAUNCH();
   }
   {
     ProfScope ps(ctx, "heads", s);
-    k_walk_unreached<<<ctx.usable_sms() * 4, 256, 0, s>>>(rec, ulist, ucount, ucap, n, limit, t.root, t.rank,
-                                                      t.seg_off, t.hint, t.nseg, t.plus_one, ctx.d_status);
+    k_walk_unreached<F><<<ctx.usable_sms() * 4, 256, 0, s>>>(l0.records<F>(), ulist, ucount, ucap, n, limit, t.root,
+                                                             t.rank, t.seg_off, t.hint, t.nseg, t.plus_one, t.tour,
+                                                             t.seg_tour, t.keep_roots, ctx.d_status);
     KS_CHECK_LAUNCH();
   }
   return KASCADE_OK;
+}
+
+}  // namespace
+
+kascade_status rank_level0_log(kascade_ctx& ctx, const Level0& l0, uint32_t n, const Extent& ext, const Heads& heads,
+                               const LogTarget& t, const Params& p, cudaStream_t s) {
+  // records of 32-bit weights are alike with and without 64-bit stamps
+  if (l0.fmt == Format::F16x16) return rank_level0_log_as<F16x16>(ctx, l0, n, ext, heads, t, p, s);
+  return rank_level0_log_as<F8x16>(ctx, l0, n, ext, heads, t, p, s);
 }
 
 }  // namespace ks

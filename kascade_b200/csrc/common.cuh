@@ -60,7 +60,9 @@ struct DevStatus {
   unsigned int code;
   unsigned int pad;
   unsigned long long info;
-  unsigned long long counter[6];  // [0]: write-free chains past their hop cap; [1]: level 0's size, when only the device knows it
+  // [1]: level 0's size, when only the device knows it; [2], [3]: elements
+  // stamped by chains / found stamped (more of the former: two chains met)
+  unsigned long long counter[6];
   unsigned int work[31];          // per level: rulers handed out beyond the warps' first shares
   unsigned int heads;             // tour heads found
 };
@@ -114,6 +116,138 @@ __device__ __forceinline__ void st_rec_cs(Rec* p, Rec r) {
   uint4 v = make_uint4((uint32_t)r.a, (uint32_t)(r.a >> 32), r.b, r.c);
   __stcs(reinterpret_cast<uint4*>(p), v);
 }
+// ---------------------------------------------------------------------------
+// Record formats of a level.  A record holds an element's weight and
+// successor and is only ever read while chains run: both halves of the L2
+// keep copies, and a dependent hop costs 0.15-0.22 us; with the stamp stored
+// into the record it had just been read from, every hop paid the cross-die
+// coherence (0.26-0.44 us).  Stamps (ruler id, distance) have an array of
+// their own.
+// A record also says whether its successor is a ruler, so that a hop needs no
+// index arithmetic (it was a third of the chase's instructions) and a chain
+// knows that it ends before it asks for another record.  8 B records keep that
+// bit in the successor word: at most 2^31 elements.
+//   F8x8   32-bit weights whose distances are wanted modulo 2^32 only (unit
+//          weights: a chain is shorter; tours: depths), 8 B stamps
+//   F8x16  32-bit weights, 64-bit distances
+//   F16x16 64-bit weights (in-place calls, every deeper level)
+//   F16i   any weights, the stamp stored into the record: half the memory of
+//          F16x16, for sizes at which that decides what stays in L2
+// ---------------------------------------------------------------------------
+struct __align__(8) Rec8 {
+  uint32_t b;  // successor | REC8_RULER when that is a ruler
+  uint32_t w;  // weight
+};
+constexpr uint32_t REC8_RULER = 0x80000000u;
+constexpr uint64_t REC8_MAX = 0x80000000ull;  // elements
+struct Hop {
+  uint64_t w;
+  uint32_t b;
+  bool ruler;  // whether b is one
+};
+struct Stamp {
+  uint32_t id;  // TAG_UNREACHED: none
+  uint64_t dist;
+};
+struct Stamp8 {
+  using S = uint2;
+  static __device__ __forceinline__ void put(S* p, uint32_t id, uint64_t dist) {
+    __stcg(p, make_uint2(id, (uint32_t)dist));
+  }
+  static __device__ __forceinline__ void clear(S* p) { __stcg(p, make_uint2(TAG_UNREACHED, 0u)); }
+  static __device__ __forceinline__ Stamp get_stream(const S* p) {
+    const uint2 v = __ldcs(p);
+    return Stamp{v.x, v.y};
+  }
+  static __device__ __forceinline__ Stamp get(const S* p) {
+    const uint2 v = __ldcg(p);
+    return Stamp{v.x, v.y};
+  }
+};
+struct Stamp16 {
+  using S = uint4;
+  static __device__ __forceinline__ void put(S* p, uint32_t id, uint64_t dist) {
+    __stcg(p, make_uint4((uint32_t)dist, (uint32_t)(dist >> 32), id, 0u));
+  }
+  static __device__ __forceinline__ void clear(S* p) { __stcg(p, make_uint4(0u, 0u, TAG_UNREACHED, 0u)); }
+  static __device__ __forceinline__ Stamp get_stream(const S* p) {
+    const uint4 v = __ldcs(p);
+    return Stamp{v.z, (uint64_t)v.x | ((uint64_t)v.y << 32)};
+  }
+  static __device__ __forceinline__ Stamp get(const S* p) {
+    const uint4 v = __ldcg(p);
+    return Stamp{v.z, (uint64_t)v.x | ((uint64_t)v.y << 32)};
+  }
+};
+struct Record8 {
+  using R = Rec8;
+  static constexpr uint64_t kMaxElems = REC8_MAX;
+  static __device__ __forceinline__ Hop unpack(uint2 v) {
+    return Hop{v.y, v.x & ~REC8_RULER, (v.x & REC8_RULER) != 0u};
+  }
+  static __device__ __forceinline__ Hop hop(const R* p) { return unpack(__ldcg(reinterpret_cast<const uint2*>(p))); }
+  static __device__ __forceinline__ void put(R* p, uint64_t w, uint32_t b, bool ruler) {
+    __stcg(reinterpret_cast<uint2*>(p), make_uint2(b | (ruler ? REC8_RULER : 0u), (uint32_t)w));
+  }
+};
+struct Record16 {
+  using R = Rec;
+  static __device__ __forceinline__ Hop hop(const R* p) {
+    const Rec r = ld_rec_cg(p);
+    return Hop{r.a, r.b, r.c != 0u};
+  }
+  static __device__ __forceinline__ void put(R* p, uint64_t w, uint32_t b, bool ruler) {
+    Rec r;
+    r.a = w;
+    r.b = b;
+    r.c = ruler ? 1u : 0u;
+    st_rec_cg(p, r);
+  }
+};
+template <class Record, class StampT>
+struct Split : Record, StampT {
+  static constexpr bool kInPlace = false;
+  using Record::put;
+  static __device__ __forceinline__ void stamp(typename StampT::S* p, uint32_t id, uint64_t d, const Hop&) {
+    StampT::put(p, id, d);
+  }
+};
+using F8x8 = Split<Record8, Stamp8>;
+using F8x16 = Split<Record8, Stamp16>;
+using F16x16 = Split<Record16, Stamp16>;
+struct F16i {
+  static constexpr bool kInPlace = true;
+  using R = Rec;
+  using S = Rec;  // the records themselves
+  static constexpr uint32_t NONE = 0x7FFFFFFFu, RULER = 0x80000000u;  // word c: ruler id or NONE, successor's bit
+  static __device__ __forceinline__ Hop hop(const R* p) {
+    const Rec r = ld_rec_cg(p);
+    return Hop{r.a, r.b, (r.c & RULER) != 0u};
+  }
+  static __device__ __forceinline__ void put(R* p, uint64_t w, uint32_t b, bool ruler) {
+    Rec r;
+    r.a = w;
+    r.b = b;
+    r.c = NONE | (ruler ? RULER : 0u);
+    st_rec_cg(p, r);
+  }
+  static __device__ __forceinline__ void stamp(S* p, uint32_t id, uint64_t d, const Hop& h) {
+    Rec r;
+    r.a = d;
+    r.b = h.b;
+    r.c = id | (h.ruler ? RULER : 0u);
+    st_rec_cg(p, r);
+  }
+  static __device__ __forceinline__ void clear(S*) {}  // part of put
+  static __device__ __forceinline__ Stamp unpack(const Rec& r) {
+    const uint32_t id = r.c & ~RULER;
+    return Stamp{id == NONE ? TAG_UNREACHED : id, r.a};
+  }
+  static __device__ __forceinline__ Stamp get_stream(const S* p) { return unpack(ld_rec_cs(p)); }
+  static __device__ __forceinline__ Stamp get(const S* p) { return unpack(ld_rec_cg(p)); }
+};
+enum class Format { F8x8, F8x16, F16x16, F16i };
+
 __device__ __forceinline__ Out ld_out(const Out* p) {
   uint4 v = __ldcg(reinterpret_cast<const uint4*>(p));
   Out o;

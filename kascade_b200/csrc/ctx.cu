@@ -113,6 +113,8 @@ kascade_status status_finish(kascade_ctx& ctx, cudaStream_t s) {
   if (st->counter[1] && !ctx.last_levels.empty()) ctx.last_levels[0] = st->counter[1];
   ctx.error_info = st->info;
   ctx.last_status = (kascade_status)st->code;
+  // two chains stamped one element: it has two predecessors
+  if (ctx.last_status == KASCADE_OK && st->counter[2] != st->counter[3]) ctx.last_status = KASCADE_ERR_NOT_A_LIST;
   return ctx.last_status;
 }
 

@@ -48,30 +48,14 @@ struct kascade_ctx {
   cudaEvent_t done_event = nullptr;
   cudaStream_t last_stream = nullptr;
   bool async_pending = false;
-  // an async host-buffer call: what kascade_ctx_sync needs to rank it again
-  // when a chain ran past the write-free chase's hop cap (the host buffers are
-  // the call's until then)
-  struct HostRerun {
-    bool set = false;
-    int kind = 0;                     // 0: kascade_rank_list_host, 1: kascade_root_forest_host
-    const uint64_t* succ = nullptr;  // successors, or parents
-    const uint32_t* weights = nullptr;
-    unsigned long long n = 0;
-    uint64_t* root_out = nullptr;
-    uint64_t* rank_out = nullptr;  // ranks, or depths
-    kascade_opts opts{};
-    cudaStream_t stream = nullptr;
-  } host_rerun;
-  // size classes: instances of at most class_max[i] elements use a mean ruler
-  // spacing of class_spacing[i] inside a batch; a call (or a batch, by the class holding
-  // most of its elements) chases with class_chains[i] chains per thread in
-  // blocks of class_block[i] threads.  Defaults: the autotuner's table.
+  // size classes: a batch of at most class_max[i] records uses a ruler spacing
+  // of class_spacing[i], a call that ranks one list or tour of that size
+  // class_spacing_single[i]; both chase in blocks of class_block[i] threads.
+  // (class_chains: kept for its callers, no effect.)  Defaults: the tuned table.
   std::vector<unsigned long long> class_max = KS_TUNED_MAX;
   std::vector<uint32_t> class_spacing = KS_TUNED_SPACING;
   std::vector<uint32_t> class_chains = KS_TUNED_CHAINS;
   std::vector<uint32_t> class_block = KS_TUNED_BLOCK;
-  // spacing for a call that ranks one instance on its own: fewer, larger
-  // levels pay off there, since each level costs launches and a host wait
   std::vector<uint32_t> class_spacing_single = KS_TUNED_SPACING_SINGLE;
   int class_of(unsigned long long n) const {
     for (size_t i = 0; i < class_max.size(); ++i)

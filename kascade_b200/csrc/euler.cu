@@ -55,6 +55,7 @@ __global__ void __launch_bounds__(256) k_seg_bounds(const uint32_t* __restrict__
 }
 
 constexpr uint32_t NO_CHILD = 0xFFFFFFFFu;
+constexpr uint32_t TOUR_DOWN = 0xFFFFFFFFu;  // a down edge's weight: -1 modulo 2^32 (an up edge's is 1)
 
 // Where a batch's forest tour records live, by vertex.  The forests are
 // compacted into one vertex space with per-forest bases fd[j]:
@@ -186,11 +187,13 @@ __device__ __forceinline__ void warp_set_bits(uint32_t* __restrict__ bits, bool 
 // vertex instead of 2.  ibits (vertices with a down edge) tells which element
 // a sibling or first child is entered by.  A tile's loads are issued in two
 // independent rounds.  heads: the tours' first vertices become their elements.
-template <class Slots>
+template <class F, class Slots>
 __global__ void __launch_bounds__(256) k_tour_links(const uint32_t* __restrict__ p32, uint32_t n,
                                                     const uint32_t* __restrict__ fc,
                                                     const uint32_t* __restrict__ nsib,
-                                                    const uint32_t* __restrict__ ibits, Rec* __restrict__ rec,
+                                                    const uint32_t* __restrict__ ibits,
+                                                    Rulers rl, typename F::R* __restrict__ rec,
+                                                    typename F::S* __restrict__ stamp,
                                                     uint32_t* __restrict__ leaf_out, uint32_t* __restrict__ heads,
                                                     const uint32_t* __restrict__ nheads, Slots slots) {
   const uint32_t lane = threadIdx.x & 31u;
@@ -234,26 +237,29 @@ __global__ void __launch_bounds__(256) k_tour_links(const uint32_t* __restrict__
         const uint32_t j = jv[i], p = pv[i];
         const uint32_t down = slots.down(v);
         up = slots.up(v, j);
-        Rec ru, rd;
-        ru.a = rd.a = 0;
-        ru.b = up;  // a root: the tour's terminal element (or an isolated vertex)
-        rd.b = down;  // a dead self loop unless v keeps a down edge
-        ru.c = rd.c = TAG_UNREACHED;
+        uint32_t uw = 0, dw = 0;
+        uint32_t ub = up;  // a root: the tour's terminal element (or an isolated vertex)
+        uint32_t db = down;  // a dead self loop unless v keeps a down edge
         if (p != v) {
           // the element a walk enters child c by: its down edge, or its merged slot
-          ru.b = (sib[i] != NO_CHILD)
+          ub = (sib[i] != NO_CHILD)
                      ? (((wsib[i] >> (sib[i] & 31)) & 1u) ? slots.down(sib[i]) : slots.up(sib[i], j))
                      : slots.up(p, j);
           if (first[i] != NO_CHILD) {
-            ru.a = 1ull;
-            rd.a = ~0ull;  // -1
-            rd.b = ((wfirst[i] >> (first[i] & 31)) & 1u) ? slots.down(first[i]) : slots.up(first[i], j);
+            uw = 1u;
+            dw = TOUR_DOWN;
+            db = ((wfirst[i] >> (first[i] & 31)) & 1u) ? slots.down(first[i]) : slots.up(first[i], j);
           } else {
             leaf = true;  // down (-1) and up (+1) in one element of weight 0
           }
         }
-        st_rec_cs(rec + up, ru);
-        st_rec_cs(rec + down, rd);  // every down slot, dead or not: the stores stay coalesced
+        uint32_t k;
+        F::put(rec + up, uw, ub, rl.is(ub, &k));
+        F::put(rec + down, dw, db, rl.is(db, &k));  // every down slot, dead or not: the stores stay coalesced
+        if (stamp) {
+          F::clear(stamp + up);
+          F::clear(stamp + down);
+        }
       }
       warp_set_bits(leaf_out, leaf, up, lane);
     }
@@ -415,10 +421,13 @@ struct Entries {
 // (the vertex's own words; the table words of its sibling, its first child
 // and itself), so a tile waits for two memory latencies rather than a chain
 // of them per vertex.
+template <class F>
 __global__ void __launch_bounds__(256) k_tour_leaves(const uint32_t* __restrict__ p32, uint32_t n,
                                                      const uint32_t* __restrict__ fc,
                                                      const uint32_t* __restrict__ nsib, Entries ent,
-                                                     Rec* __restrict__ rec, uint32_t* __restrict__ leaf_bits,
+                                                     Rulers rl, typename F::R* __restrict__ rec,
+                                                     typename F::S* __restrict__ stamp,
+                                                     uint32_t* __restrict__ leaf_bits,
                                                      uint32_t* __restrict__ heads,
                                                      const uint32_t* __restrict__ nheads) {
   const uint32_t lane = threadIdx.x & 31u;
@@ -462,22 +471,23 @@ __global__ void __launch_bounds__(256) k_tour_leaves(const uint32_t* __restrict_
       bool leaf = false;
       if (v < n) {
         const uint32_t p = pv[i];
-        Rec ru, rd;
-        ru.a = 0;
-        ru.b = v;  // a root: the tour's terminal element (or an isolated vertex)
-        ru.c = rd.c = TAG_UNREACHED;
+        uint32_t uw = 0, ub = v;  // a root: the tour's terminal element (or an isolated vertex)
         if (p != v) {
-          ru.b = (sib[i] != NO_CHILD) ? ent.of(sib[i], wsib[i]) : p;
+          ub = (sib[i] != NO_CHILD) ? ent.of(sib[i], wsib[i]) : p;
           if (first[i] != NO_CHILD) {
-            ru.a = 1ull;
-            rd.a = ~0ull;  // -1
-            rd.b = ent.of(first[i], wfirst[i]);
-            st_rec_cs(rec + ent.down_slot(v, wown[i]), rd);
+            uw = 1u;
+            const uint32_t down = ent.down_slot(v, wown[i]);
+            const uint32_t db = ent.of(first[i], wfirst[i]);
+            uint32_t k;
+            F::put(rec + down, TOUR_DOWN, db, rl.is(db, &k));
+            if (stamp) F::clear(stamp + down);
           } else {
             leaf = true;  // down (-1) and up (+1) in one element of weight 0
           }
         }
-        st_rec_cs(rec + v, ru);
+        uint32_t k;
+        F::put(rec + v, uw, ub, rl.is(ub, &k));
+        if (stamp) F::clear(stamp + v);
       }
       // a warp's 32 consecutive vertices make one word of leaf bits
       const uint32_t lb = __ballot_sync(0xffffffffu, leaf);
@@ -501,8 +511,8 @@ kascade_status link_children(kascade_ctx& ctx, const uint64_t* parent, uint32_t 
 // slots `slots` gives (a batch's forests); leaves are marked in leaf_out (by
 // output position, zeroed by the caller).
 template <class Slots>
-kascade_status build_tour(kascade_ctx& ctx, const uint64_t* parent, uint32_t n, const Slots& slots, Rec* rec,
-                          uint32_t* leaf_out, Heads* heads, cudaStream_t s) {
+kascade_status build_tour(kascade_ctx& ctx, const uint64_t* parent, uint32_t n, const Slots& slots, const Level0& l0,
+                          const Rulers& rl, uint32_t* leaf_out, Heads* heads, cudaStream_t s) {
   const uint64_t words = ((uint64_t)n + 31) / 32;
   uint32_t* fc = alloc<uint32_t>(ctx, n);
   uint32_t* nsib = alloc<uint32_t>(ctx, n);
@@ -520,7 +530,19 @@ kascade_status build_tour(kascade_ctx& ctx, const uint64_t* parent, uint32_t n, 
   KS_CHECK_LAUNCH();
   const unsigned grid =
       grid_for(ctx, ((uint64_t)n + 256 * TB_BATCH_ITEMS - 1) / (256 * TB_BATCH_ITEMS) * 256, 256, 8);
-  k_tour_links<Slots><<<grid, 256, 0, s>>>(p32, n, fc, nsib, ibits, rec, leaf_out, head, &ctx.d_status->heads, slots);
+  auto links = [&](auto f) {
+    using F = decltype(f);
+    k_tour_links<F, Slots><<<grid, 256, 0, s>>>(p32, n, fc, nsib, ibits, rl, l0.records<F>(), l0.stamps<F>(), leaf_out,
+                                                head, &ctx.d_status->heads, slots);
+  };
+  if (l0.fmt == Format::F8x8)
+    links(F8x8{});
+  else if (l0.fmt == Format::F8x16)
+    links(F8x16{});
+  else if (l0.fmt == Format::F16i)
+    links(F16i{});
+  else
+    links(F16x16{});
   KS_CHECK_LAUNCH();
   return KASCADE_OK;
 }
@@ -528,11 +550,14 @@ kascade_status build_tour(kascade_ctx& ctx, const uint64_t* parent, uint32_t n, 
 }  // namespace
 
 kascade_status root_forest_impl(kascade_ctx& ctx, const uint64_t* parent, uint32_t n, uint64_t* root_out,
-                                uint64_t* depth_out, int keep_roots, const Params& p, cudaStream_t s,
-                                bool host_check) {
+                                uint64_t* depth_out, int keep_roots, const Params& p, cudaStream_t s) {
   if (n == 0) return KASCADE_OK;
   const uint32_t words = (uint32_t)(((uint64_t)n + 31) / 32);
-  Rec* rec = alloc<Rec>(ctx, 2ull * n);
+  Level0 l0;
+  // the tour has at most 2n elements, about 1.5n with its leaves contracted
+  Level0Plan plan = plan_level0(p, (3ull * n + 1) / 2, WKind::Unit);
+  if (2ull * n > REC8_MAX && plan.fmt == Format::F8x8) plan.fmt = Format::F16x16;
+  KS_TRY(alloc_level0(ctx, plan, 2ull * n, &l0));
   uint32_t* downs = alloc<uint32_t>(ctx, 1);  // down-edge count
   uint32_t* fc = alloc<uint32_t>(ctx, n);
   uint32_t* nsib = alloc<uint32_t>(ctx, n);
@@ -544,7 +569,7 @@ kascade_status root_forest_impl(kascade_ctx& ctx, const uint64_t* parent, uint32
   uint32_t* leaf_bits = alloc<uint32_t>(ctx, words);
   uint2* iw = alloc<uint2>(ctx, words);
   uint32_t* head = alloc<uint32_t>(ctx, HEAD_CAP);
-  if (!rec || !downs || !fc || !nsib || !p32 || !root_bits || !ibits || !icount || !ipre || !leaf_bits || !iw || !head)
+  if (!downs || !fc || !nsib || !p32 || !root_bits || !ibits || !icount || !ipre || !leaf_bits || !iw || !head)
     return KASCADE_ERR_OOM;
   KS_TRY(link_children(ctx, parent, n, fc, nsib, p32, root_bits, s));
   {
@@ -556,31 +581,40 @@ kascade_status root_forest_impl(kascade_ctx& ctx, const uint64_t* parent, uint32
     k_internal_pack<<<grid_for(ctx, words, 256, 8), 256, 0, s>>>(ibits, ipre, words, iw);
     KS_CHECK_LAUNCH();
     const unsigned grid = grid_for(ctx, ((uint64_t)n + 256 * TB_ITEMS - 1) / (256 * TB_ITEMS) * 256, 256, 8);
-    k_tour_leaves<<<grid, 256, 0, s>>>(p32, n, fc, nsib, Entries{iw, n}, rec, leaf_bits, head,
-                                       &ctx.d_status->heads);
+    auto leaves = [&](auto f) {
+      using F = decltype(f);
+      k_tour_leaves<F><<<grid, 256, 0, s>>>(p32, n, fc, nsib, Entries{iw, n}, level0_rulers(p), l0.records<F>(),
+                                            l0.stamps<F>(), leaf_bits, head, &ctx.d_status->heads);
+    };
+    if (l0.fmt == Format::F8x8)
+      leaves(F8x8{});
+    else if (l0.fmt == Format::F16i)
+      leaves(F16i{});
+    else
+      leaves(F16x16{});
     KS_CHECK_LAUNCH();
   }
   // The tour's length n + (down edges) stays on the device: the ranking is
   // sized for the bound 2n, rulers beyond the length are dead, and outputs
   // come only from slots below n.
   Extent ext;
-  ext.cap = 2 * n;  // n <= 2^31 - 1
+  ext.cap = 2 * n;
   ext.base = n;
   ext.add = downs;
-  return rank_records(ctx, rec, ext.cap, ext, Heads{head, &ctx.d_status->heads, HEAD_CAP},
-                      SinkTour{root_out, depth_out, n, keep_roots, leaf_bits}, p, s, host_check);
+  return rank_records(ctx, l0, ext.cap, ext, Heads{head, &ctx.d_status->heads, HEAD_CAP},
+                      SinkTour{root_out, depth_out, n, keep_roots, leaf_bits}, p, s);
 }
 
 // Tours of a batch of forests whose parents are given in one compact vertex
 // space (fpar[c] = compact parent of compact vertex c); records go to the
 // slots described by SlotsBatch, *heads gets the tours' heads.
 kascade_status batch_tours(kascade_ctx& ctx, const uint64_t* fpar, uint32_t F, const uint32_t* fd, const uint32_t* foff,
-                           const uint32_t* fhint, uint32_t nf, uint32_t down_base, Rec* rec, uint32_t* leaf_out,
-                           Heads* heads, cudaStream_t s) {
+                           const uint32_t* fhint, uint32_t nf, uint32_t down_base, const Level0& l0,
+                           const Rulers& rl, uint32_t* leaf_out, Heads* heads, cudaStream_t s) {
   *heads = Heads{};
   if (F == 0) return KASCADE_OK;
   const SlotsBatch slots{fd, foff, fhint, nf, down_base};
-  return build_tour(ctx, fpar, F, slots, rec, leaf_out, heads, s);
+  return build_tour(ctx, fpar, F, slots, l0, rl, leaf_out, heads, s);
 }
 
 kascade_status compute_euler_tour_impl(kascade_ctx& ctx, const uint64_t* parent, uint32_t n, uint64_t* tour,

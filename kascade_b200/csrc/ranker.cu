@@ -52,20 +52,14 @@ struct WI64 {
 inline uint32_t salt_for(uint32_t seed, int level) { return mix32(seed + 0x9E3779B9u * (uint32_t)(level + 1)); }
 
 // ---------------------------------------------------------------------------
-// prepare: build records.  A root's weight is no part of any rank: its record
-// carries 0, so that a chain ending at it adds the record's word like any.
+// prepare: build records, clear the stamps (stamp == nullptr: the write-free
+// path has none).  A root's weight is no part of any rank: its record carries
+// 0, so that a chain ending at it adds the record's word like any.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ Rec make_rec(uint64_t w, uint64_t succ, uint64_t x) {
-  Rec r;
-  r.a = succ == x ? 0ull : w;
-  r.b = (uint32_t)succ;
-  r.c = TAG_UNREACHED;
-  return r;
-}
-
-template <class W>
+template <class F, class W>
 __global__ void __launch_bounds__(256, 4) k_prepare_arrays(const uint64_t* __restrict__ succ, W w, uint32_t n,
-                                                        uint64_t start, Rec* __restrict__ rec, DevStatus* st) {
+                                                        uint64_t start, Rulers rl, typename F::R* __restrict__ rec,
+                                                        typename F::S* __restrict__ stamp, DevStatus* st) {
   const uint64_t tile_sz = (uint64_t)blockDim.x * PREP_ITEMS;
   for (uint64_t tile = start + (uint64_t)blockIdx.x * tile_sz; tile < n; tile += (uint64_t)gridDim.x * tile_sz) {
     unsigned long long sv[PREP_ITEMS];
@@ -88,24 +82,27 @@ __global__ void __launch_bounds__(256, 4) k_prepare_arrays(const uint64_t* __res
         set_error(st, KASCADE_ERR_OUT_OF_RANGE, x);
         sv[i] = x;
       }
-      rec[x] = make_rec(wv[i], sv[i], x);
+      uint32_t j;
+      F::put(rec + x, sv[i] == x ? 0 : wv[i], (uint32_t)sv[i], rl.is((uint32_t)sv[i], &j));
+      if (stamp) F::clear(stamp + x);
     }
   }
 }
 
-// The same work for 16 B-aligned inputs, with the input tiles moved by bulk
-// (TMA) copies: a persistent block keeps PT_STAGES tiles of succ (and
-// weights) in flight into shared memory while it writes the records of an
-// earlier tile.  Full tiles only; the caller hands the tail to
+// The same work for 16 B-aligned inputs with 32-bit weights, with the input
+// tiles moved by bulk (TMA) copies: a persistent block keeps PT_STAGES tiles
+// of succ (and weights) in flight into shared memory while it writes the
+// records of an earlier tile.  Full tiles only; the caller hands the tail to
 // k_prepare_arrays.
 constexpr int PT_TILE = 2048;
 constexpr int PT_STAGES = 4;
 constexpr int PT_ITEMS = PT_TILE / 256;
 
-template <bool W32>
+template <class F, bool W32>
 __global__ void __launch_bounds__(256) k_prepare_tma(const uint64_t* __restrict__ succ, const uint32_t* __restrict__ w,
-                                                     uint32_t n, uint32_t ntiles, Rec* __restrict__ rec,
-                                                     DevStatus* st) {
+                                                     uint32_t n, uint32_t ntiles, Rulers rl,
+                                                     typename F::R* __restrict__ rec,
+                                                     typename F::S* __restrict__ stamp, DevStatus* st) {
   constexpr uint32_t SB = PT_TILE * 8, WB = W32 ? PT_TILE * 4 : 0, STAGE = SB + WB;
   extern __shared__ __align__(128) unsigned char dyn[];
   __shared__ __align__(8) uint64_t bar[PT_STAGES];
@@ -167,169 +164,132 @@ __global__ void __launch_bounds__(256) k_prepare_tma(const uint64_t* __restrict_
 #pragma unroll
     for (int i = 0; i < PT_ITEMS; ++i) {
       const uint32_t x = (uint32_t)(base + i * 256 + tid);
-      st_rec_cs(rec + x, make_rec(wv[i], sv[i], x));
+      uint32_t j;
+      F::put(rec + x, sv[i] == x ? 0u : wv[i], sv[i], rl.is(sv[i], &j));
+      if (stamp) F::clear(stamp + x);
     }
   }
 }
 
-// The record of ruler `id` at the next level: its chain ended at ruler `next`,
-// or (next == id) at the list's end, whose level-0 root goes to *rootel.
-__device__ __forceinline__ void end_chain(Rec* rec_next, uint32_t id, uint64_t dist, uint32_t next) {
-  Rec o;
-  o.a = dist;
-  o.b = next;
-  o.c = TAG_UNREACHED;
-  st_rec_cg(rec_next + id, o);
-}
-
 // ---------------------------------------------------------------------------
-// chase: C chains in flight per thread, one per ruler.  A hop reads the 16 B
-// record of the next element and stamps (distance from ruler, ruler id) into
-// it.  A chain ends in front of the next ruler, known from the index alone,
-// or at the list's end.  A warp's first rulers are its own share, later ones
-// come from one counter; only the first `lanes` lanes of a warp work, so that
-// few rulers spread over all SMs and a warp's hop waits for few loads (a
-// dependent L2 hop costs 0.23 us alone and 0.43 us for 32 lanes together).
-// A new chain's first load shares an iteration with the other lanes' hops.
-// ---------------------------------------------------------------------------
+// chase: one chain per thread, one per ruler.  A hop reads the record of the
+// next element and stamps (distance from ruler, ruler id) for it.  A chain
+// ends in front of the next ruler or at the list's end.  A warp's first rulers
+// are its own share, later ones come from one counter, for several idle lanes
+// at a time; only the first `lanes` lanes of a warp work, so that few rulers
+// spread over all SMs and a warp's hop waits for few loads.
+//
+// Bound by the longest chains' dependent hops, and by instructions while most
+// chains run (a warp issues them for its last running lane too).  The next
+// record is asked for as soon as its index is known, before the element at
+// hand is stamped.
+//
 // head_base: where level k >= 1 keeps its heads (level 0: heads.elem lists
-// them).  A head's own record is stamped at distance 0.
-template <int C>
-__global__ void __launch_bounds__(512) k_chase(Rec* __restrict__ rec, Extent ext, Rulers rl, uint32_t rulers,
-                                               Heads heads, uint32_t head_base,
-                                               const uint32_t* __restrict__ rootel, Rec* __restrict__ rec_next,
+// them).  A head's own element is stamped at distance 0.  limit: stamps of
+// elements below it are counted; propagation counts the elements it finds
+// stamped, and fewer than stamps made mean that two chains met.  hop_cap: a
+// chain this long looks for a cycle ahead.
+// ---------------------------------------------------------------------------
+constexpr int CHASE_REFILL = 8;  // idle lanes worth a refill
+
+template <class F>
+__global__ void __launch_bounds__(512) k_chase(const typename F::R* rec, typename F::S* stamp, Extent ext, Rulers rl,
+                                               uint32_t rulers, Heads heads, uint32_t head_base,
+                                               const uint32_t* __restrict__ rootel, Rulers rl_next,
+                                               Rec* __restrict__ rec_next, uint4* __restrict__ stamp_next,
                                                uint32_t* __restrict__ rootel_next, uint32_t* __restrict__ work,
-                                               uint32_t lanes, DevStatus* st) {
+                                               uint32_t lanes, uint32_t limit, uint32_t hop_cap, DevStatus* st) {
   const uint32_t n = ext.get();
   const uint32_t r = rulers + heads.get();
   // level 0's size, reported by the call
   if (!rootel && ext.add && blockIdx.x == 0 && threadIdx.x == 0) st->counter[1] = n;
   const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t lt = lanemask_lt();
-  const uint32_t batch = lanes * C;
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
   const uint32_t warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  uint32_t cid[C], cx[C], hops[C];
-  uint64_t acc[C];
-  uint32_t act = 0, fresh = 0;  // bit c: chain c runs / has not read its ruler's record yet
-  // warp-uniform: this warp's ruler ids at hand, and whether more may follow
-  uint32_t q_base = warp * batch;
-  uint32_t q_left = q_base < r ? r - q_base : 0u;
-  if (q_left > batch) q_left = batch;
-  const uint32_t first = warps * batch;  // ids from here on are handed out by the counter
-  bool drained = false;
-#pragma unroll
-  for (int c = 0; c < C; ++c) {
-    cid[c] = cx[c] = hops[c] = 0;
-    acc[c] = 0;
-  }
-  while (true) {
-    if (!drained) {
-#pragma unroll
-      for (int c = 0; c < C; ++c) {
-        bool need = lane < lanes && !((act >> c) & 1u);
-        uint32_t m = __ballot_sync(FULL, need);
-        while (m != 0u && !drained) {
-          if (q_left == 0u) {
-            uint32_t b = r;
-            if (first < r) {
-              uint32_t t = 0;
-              if (lane == 0) t = atomicAdd(work, batch);
-              b = first + __shfl_sync(FULL, t, 0);
-            }
-            if (b >= r) {
-              drained = true;
-              break;
-            }
-            q_base = b;
-            q_left = r - b;
-            if (q_left > batch) q_left = batch;
-          }
-          const uint32_t take = min((uint32_t)__popc(m), q_left);
-          const uint32_t my_rank = __popc(m & lt);
-          const bool mine = need && my_rank < take;
-          if (mine) {
-            const uint32_t id = q_base + my_rank;
-            uint64_t x0;
-            if (id < rulers)
-              x0 = rl.elem(id);
-            else
-              x0 = rootel ? head_base + (id - rulers) : __ldg(heads.elem + (id - rulers));
-            uint32_t j;
-            if (x0 >= n) {
-              end_chain(rec_next, id, 0, id);  // the last block's ruler, beyond the elements
-            } else if (id >= rulers && rl.is((uint32_t)x0, &j) && j < rulers) {
-              end_chain(rec_next, id, 0, j);  // a head that is a ruler itself
-              rootel_next[id] = 0;
-            } else {
-              cid[c] = id;
-              cx[c] = (uint32_t)x0;
-              acc[c] = 0;
-              hops[c] = 0;
-              act |= 1u << c;
-              fresh |= 1u << c;
-            }
-          }
-          m &= ~__ballot_sync(FULL, mine);
-          need = need && !mine;
-          q_base += take;
-          q_left -= take;
-        }
-      }
+  const uint32_t first = warps * lanes;  // ids from here on are handed out by the counter
+  uint32_t id = 0, x = 0, hops = 0, stamps = 0;
+  uint64_t acc = 0;
+  Hop h{0, 0, false};             // the record of x, asked for
+  bool act = false, own = false;  // own: x is the chain's first element and a ruler (not stamped)
+  auto begin = [&](uint32_t i) {
+    id = i;
+    uint64_t x0;
+    if (i < rulers)
+      x0 = rl.elem(i);
+    else
+      x0 = rootel ? head_base + (i - rulers) : __ldg(heads.elem + (i - rulers));
+    uint32_t j;
+    if (x0 >= n) {
+      end_chain(rec_next, stamp_next, rl_next, i, 0, i);  // the last block's ruler, beyond the elements
+    } else if (i >= rulers && rl.is((uint32_t)x0, &j) && j < rulers) {
+      end_chain(rec_next, stamp_next, rl_next, i, 0, j);  // a head that is a ruler itself
+    } else {
+      x = (uint32_t)x0;
+      h = F::hop(rec + x);
+      acc = 0;
+      hops = 0;
+      own = i < rulers;
+      act = true;
     }
-    if (!__any_sync(FULL, act != 0u)) {
-      if (drained) break;
+  };
+  if (lane < lanes && warp * lanes + lane < r) begin(warp * lanes + lane);
+  bool more = first < r;  // warp-uniform
+  while (true) {
+    const uint32_t running = __ballot_sync(FULL, act);
+    if (more && (running == 0u || __popc(running) + CHASE_REFILL <= (int)lanes)) {
+      const uint32_t idle = ~running & (lanes == 32 ? FULL : (1u << lanes) - 1u);
+      uint32_t b = 0;
+      if (lane == 0) b = first + atomicAdd(work, (uint32_t)__popc(idle));
+      b = __shfl_sync(FULL, b, 0);
+      if (b >= r) more = false;
+      const uint32_t i = b + __popc(idle & lanemask_lt());
+      if (((idle >> lane) & 1u) && i < r) begin(i);
       continue;
     }
-    Rec rr[C];
-#pragma unroll
-    for (int c = 0; c < C; ++c)
-      if ((act >> c) & 1u) rr[c] = ld_rec_cg(rec + cx[c]);
-#pragma unroll
-    for (int c = 0; c < C; ++c) {
-      if (!((act >> c) & 1u)) continue;
-      const uint32_t x = cx[c], y = rr[c].b;
-      const uint64_t d = acc[c];
-      if (y == x) {  // the list's end (never stamped: any number of chains may end here)
-        end_chain(rec_next, cid[c], d + rr[c].a, cid[c]);
-        rootel_next[cid[c]] = rootel ? __ldg(rootel + x) : x;
-        act &= ~(1u << c);
-        fresh &= ~(1u << c);
-        continue;
-      }
-      const bool start = (fresh >> c) & 1u;
-      fresh &= ~(1u << c);
-      if (!start || cid[c] >= rulers) {
-        if (!tag_unreached(rr[c].c)) {  // stamped by another chain: two predecessors
-          set_error(st, KASCADE_ERR_NOT_A_LIST, x);
-          end_chain(rec_next, cid[c], 0, cid[c]);
-          rootel_next[cid[c]] = 0;
-          act &= ~(1u << c);
-          continue;
-        }
-        Rec wv;
-        wv.a = d;
-        wv.b = y;
-        wv.c = cid[c];
-        st_rec_cg(rec + x, wv);
-      }
-      acc[c] = d + rr[c].a;
-      cx[c] = y;
-      uint32_t j;
-      if (rl.is(y, &j)) {
+    if (running == 0u) {
+      if (!more) break;
+      continue;
+    }
+    if (!act) continue;
+    const uint32_t y = h.b;
+    const uint64_t d = acc + h.w;
+    const bool end = y == x, stop = end || h.ruler;
+    // the next record's request goes out ahead of a stamp of its own array (a
+    // stamp in the record goes first: the next record may share its sector)
+    const Hop at = h;
+    if (!F::kInPlace && !stop) h = F::hop(rec + y);
+    if (!end && !own) {
+      F::stamp(stamp + x, id, acc, at);
+      stamps += x < limit ? 1u : 0u;
+    }
+    if (F::kInPlace && !stop) h = F::hop(rec + y);
+    if (stop) {  // (a list's end is not stamped: any number of chains may end there)
+      uint32_t next = id;
+      if (end) {
+        rootel_next[id] = rootel ? __ldg(rootel + x) : x;
+      } else {
+        next = rl.block_of(y);
         // back at its own ruler: a cycle without a root that holds one ruler
-        if (j == cid[c]) set_error(st, KASCADE_ERR_CYCLE, j);
-        end_chain(rec_next, cid[c], acc[c], j);
-        rootel_next[cid[c]] = 0;
-        act &= ~(1u << c);
-      } else if (++hops[c] > n) {
-        set_error(st, KASCADE_ERR_CYCLE, cid[c]);
-        end_chain(rec_next, cid[c], 0, cid[c]);
-        rootel_next[cid[c]] = 0;
-        act &= ~(1u << c);
+        if (next == id) set_error(st, KASCADE_ERR_CYCLE, id);
+      }
+      end_chain(rec_next, stamp_next, rl_next, id, d, next);
+      act = false;
+      continue;
+    }
+    own = false;
+    acc = d;
+    x = y;
+    if (++hops == hop_cap) {
+      hops = 0;
+      if (endless<F>(rec, y)) {
+        set_error(st, KASCADE_ERR_CYCLE, id);
+        end_chain(rec_next, stamp_next, rl_next, id, 0, id);
+        act = false;
       }
     }
   }
+  stamps = __reduce_add_sync(FULL, stamps);
+  if (lane == 0 && stamps) atomicAdd(&st->counter[2], (unsigned long long)stamps);
 }
 
 // ---------------------------------------------------------------------------
@@ -342,65 +302,65 @@ __global__ void __launch_bounds__(512) k_chase(Rec* __restrict__ rec, Extent ext
 // ---------------------------------------------------------------------------
 constexpr uint32_t PROP_WALKS = 512;  // elements a block collects
 
-template <class Sink>
-__device__ __forceinline__ void walk_to_result(const Rec* __restrict__ rec, uint32_t x, uint32_t n_all,
-                                               const Rulers& rl, const uint32_t* __restrict__ rootel,
-                                               const Out* __restrict__ out_next, const Sink& sink, DevStatus* st) {
-  Rec r = ld_rec_cg(rec + x);
-  // Brent's cycle detection keeps an invalid (rootless, ruler-free) cycle to
-  // O(cycle length) steps instead of n per element
-  uint64_t acc = r.a;
-  uint32_t y = r.b, hops = 0, lam = 0, power = 1, mark = x;
+template <class F, class Sink>
+__device__ __forceinline__ void walk_to_result(const typename F::R* __restrict__ rec,
+                                               const typename F::S* __restrict__ stamp, uint32_t x, const Rulers& rl,
+                                               const uint32_t* __restrict__ rootel, const Out* __restrict__ out_next,
+                                               const Sink& sink, DevStatus* st) {
+  Hop h = F::hop(rec + x);
+  uint64_t acc = h.w;
+  uint32_t y = h.b, hops = 0, mark = x;
   while (true) {
-    uint32_t id;
-    if (rl.is(y, &id)) {
-      const Out o = ld_out(out_next + id);
+    if (h.ruler) {
+      const Out o = ld_out(out_next + rl.block_of(y));
       sink.put(x, acc + o.rank, o.root, false);
       return;
     }
-    r = ld_rec_cg(rec + y);
-    if (!tag_unreached(r.c)) {
-      const Out o = ld_out(out_next + r.c);
-      sink.put(x, acc + o.rank - r.a, o.root, false);
+    h = F::hop(rec + y);
+    const Stamp t = F::get(stamp + y);
+    if (t.id != TAG_UNREACHED) {
+      const Out o = ld_out(out_next + t.id);
+      sink.put(x, acc + o.rank - t.dist, o.root, false);
       return;
     }
-    acc += r.a;
-    if (r.b == y) {
+    acc += h.w;
+    if (h.b == y) {
       sink.put(x, acc, rootel ? __ldg(rootel + y) : y, false);
       return;
     }
-    if (y == mark || ++hops > n_all) {
+    // an invalid (rootless, ruler-free) cycle comes back to a marked element
+    // in a number of steps proportional to its length
+    if (y == mark) {
       set_error(st, KASCADE_ERR_CYCLE, x);
       return;
     }
-    if (++lam == power) {
-      mark = y;
-      power <<= 1;
-      lam = 0;
-    }
-    y = r.b;
+    ++hops;
+    if ((hops & (hops - 1)) == 0) mark = y;
+    y = h.b;
   }
 }
 
-template <class Sink, int ITEMS>
-__global__ void __launch_bounds__(256) k_propagate(const Rec* __restrict__ rec, uint32_t n_out, Extent ext,
-                                                   Rulers rl, uint32_t rulers, const uint32_t* __restrict__ rootel,
+template <class F, class Sink, int ITEMS>
+__global__ void __launch_bounds__(256) k_propagate(const typename F::R* __restrict__ rec,
+                                                   const typename F::S* __restrict__ stamp, uint32_t n_out,
+                                                   Extent ext, Rulers rl, uint32_t rulers,
+                                                   const uint32_t* __restrict__ rootel,
                                                    const Out* __restrict__ out_next, Sink sink, DevStatus* st) {
   __shared__ uint32_t walks[PROP_WALKS];
-  __shared__ uint32_t nwalks;
-  if (threadIdx.x == 0) nwalks = 0;
+  __shared__ uint32_t nwalks, nfound;
+  if (threadIdx.x == 0) nwalks = nfound = 0;
   __syncthreads();
-  const uint32_t n_all = ext.get();  // records exist up to here
-  n_out = min(n_out, n_all);
+  n_out = min(n_out, ext.get());  // records exist up to here
   const uint32_t stride = gridDim.x * blockDim.x;
   const uint64_t pol = l2_keep_policy();
+  uint32_t stamped = 0;
   for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x * ITEMS + threadIdx.x; base < n_out;
        base += (uint64_t)stride * ITEMS) {
-    Rec rv[ITEMS];
+    Stamp sv[ITEMS];
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
       const uint64_t x = base + (uint64_t)i * blockDim.x;
-      if (x < n_out) rv[i] = ld_rec_cs(rec + x);
+      if (x < n_out) sv[i] = F::get_stream(stamp + x);
     }
     // every ruler's or stamped element's result, all loads in flight together
     // (they would otherwise wait behind the previous element's stores)
@@ -413,11 +373,12 @@ __global__ void __launch_bounds__(256) k_propagate(const Rec* __restrict__ rec, 
       if (x >= n_out) continue;
       uint32_t id;
       if (rl.is((uint32_t)x, &id) && id < rulers) {  // (a head's index may lie past the last block)
-        rv[i].c = TAG_RULER;
+        sv[i].dist = 0;
         found |= 1u << i;
-      } else if (!tag_unreached(rv[i].c)) {
-        id = rv[i].c;
+      } else if (sv[i].id != TAG_UNREACHED) {
+        id = sv[i].id;
         found |= 1u << i;
+        ++stamped;
       }
       if ((found >> i) & 1u) ov[i] = ld_out_keep(out_next + id, pol);
     }
@@ -425,24 +386,29 @@ __global__ void __launch_bounds__(256) k_propagate(const Rec* __restrict__ rec, 
     for (int i = 0; i < ITEMS; ++i) {
       const uint64_t x = base + (uint64_t)i * blockDim.x;
       if (x >= n_out) continue;
-      const Rec r = rv[i];
-      const bool is_root = r.b == (uint32_t)x && (r.c == TAG_RULER || tag_unreached(r.c));
       if ((found >> i) & 1u) {
-        sink.put((uint32_t)x, ov[i].rank - (r.c == TAG_RULER ? 0ull : r.a), ov[i].root, is_root);
-      } else if (is_root) {
-        sink.put((uint32_t)x, r.a, rootel ? __ldg(rootel + x) : (uint32_t)x, true);
+        // a result whose root is the element itself: it is a ruler and a root
+        sink.put((uint32_t)x, ov[i].rank - sv[i].dist, ov[i].root, !rootel && ov[i].root == (uint32_t)x);
+        continue;
+      }
+      const Hop h = F::hop(rec + x);
+      if (h.b == (uint32_t)x) {
+        sink.put((uint32_t)x, h.w, rootel ? __ldg(rootel + x) : (uint32_t)x, true);
       } else {
         const uint32_t w = atomicAdd(&nwalks, 1u);
         if (w < PROP_WALKS)
           walks[w] = (uint32_t)x;
         else
-          walk_to_result(rec, (uint32_t)x, n_all, rl, rootel, out_next, sink, st);
+          walk_to_result<F>(rec, stamp, (uint32_t)x, rl, rootel, out_next, sink, st);
       }
     }
   }
+  stamped = __reduce_add_sync(FULL, stamped);
+  if ((threadIdx.x & 31u) == 0 && stamped) atomicAdd(&nfound, stamped);
   __syncthreads();
+  if (threadIdx.x == 0 && nfound) atomicAdd(&st->counter[3], (unsigned long long)nfound);
   for (uint32_t w = threadIdx.x; w < min(nwalks, PROP_WALKS); w += blockDim.x)
-    walk_to_result(rec, walks[w], n_all, rl, rootel, out_next, sink, st);
+    walk_to_result<F>(rec, stamp, walks[w], rl, rootel, out_next, sink, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -453,17 +419,17 @@ __global__ void __launch_bounds__(256) k_propagate(const Rec* __restrict__ rec, 
 // (<= 10 rounds), and every element reads its ruler's result.  Against
 // pointer jumping over all elements (13 rounds of 16 elements per thread at
 // 8192: 51 us) each element is touched once.  Each element's word also says
-// whether its successor is a ruler or a list's end, so a hop is one exchange.
+// whether its successor is a ruler or a list's end, so a hop is one read and
+// one write of the word and of the distance.
 // With several lists, their heads (no predecessor) start chains as well, so
 // that no run of elements ahead of a first ruler is walked element by element.
-// Two chains that meet (a tree, not a list) are found by the exchange; an
-// input of at most `tree_max` elements is then done again without stamps,
-// every element walking to its first ruler, which ranks any forest.
+// Two chains that meet (a tree, not a list) leave fewer stamped elements than
+// stamps; an input of at most `tree_max` elements is then done again without
+// stamps, every element walking to its first ruler, which ranks any forest.
 // ---------------------------------------------------------------------------
 constexpr uint32_t CTA_THREADS = 1024;
 constexpr uint32_t CTA_RULERS = 1024;
 constexpr uint32_t CTA_HEADS = 1024;
-constexpr uint32_t CTA_CHAINS = CTA_RULERS / CTA_THREADS;
 constexpr uint32_t CTA_LOADS = 8;           // elements a thread has in flight while loading
 constexpr uint32_t CTA_ILP = 4;             // elements a thread has in flight in shared memory
 constexpr uint32_t CTA_FLAG = 0x80000000u;  // next: stamped, low bits the chain; rnext: the list's end
@@ -471,19 +437,20 @@ constexpr uint32_t CTA_END = 0x40000000u;   // next: the successor ends the list
 constexpr uint32_t CTA_RUL = 0x20000000u;   // next: the successor is a ruler
 constexpr uint32_t CTA_IDX = 0x1FFFFFFFu;
 constexpr size_t cta_smem(uint64_t n) {
-  return (size_t)((n + CTA_RULERS + CTA_HEADS) * 12 + CTA_HEADS * 2 + (n + 31) / 32 * 4);
+  return (size_t)((n + CTA_RULERS + CTA_HEADS) * 12 + CTA_HEADS * 2 + (n + 3) / 4 * 4);
 }
 
 // Element sources: the records of a level (a list end's carries its rank), or
 // the caller's arrays (a root's weight is no part of any rank).
+template <class F>
 struct CtaRecords {
   static constexpr bool kEndWeight = true;
-  const Rec* rec;
+  const typename F::R* rec;
   const uint32_t* rootel;
   __device__ __forceinline__ void load(uint32_t x, uint64_t* a, uint32_t* b) const {
-    const Rec r = ld_rec_cg(rec + x);
-    *a = r.a;
-    *b = r.b;
+    const Hop h = F::hop(rec + x);
+    *a = h.w;
+    *b = h.b;
   }
   __device__ __forceinline__ uint32_t root_of(uint32_t x) const { return rootel ? __ldg(rootel + x) : x; }
 };
@@ -504,45 +471,43 @@ template <class Src, class Sink>
 __global__ void __launch_bounds__(CTA_THREADS, 1) k_rank_cta(Src src, Extent ext, Sink sink, uint32_t tree_max,
                                                              int level0, DevStatus* st) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ uint32_t nends, nheads;
+  __shared__ uint32_t nends, nheads, nstamps;
   const uint32_t n = ext.get();
   unsigned long long* dist = reinterpret_cast<unsigned long long*>(smem);  // weight, once stamped the distance
   unsigned long long* rdist = dist + ext.cap;                              // per chain: distance, then rank
   uint32_t* next = reinterpret_cast<uint32_t*>(rdist + CTA_RULERS + CTA_HEADS);
   uint32_t* rnext = next + ext.cap;  // per chain: next ruler or CTA_FLAG | list end, then the root
-  uint32_t* pred = rnext + CTA_RULERS + CTA_HEADS;
-  uint16_t* hlist = reinterpret_cast<uint16_t*>(pred + (ext.cap + 31) / 32);
-  const uint32_t tid = threadIdx.x;
-  const uint32_t words = (n + 31) / 32;
+  uint32_t* predw = rnext + CTA_RULERS + CTA_HEADS;
+  unsigned char* pred = reinterpret_cast<unsigned char*>(predw);  // 1: has a predecessor
+  uint16_t* hlist = reinterpret_cast<uint16_t*>(predw + (ext.cap + 3) / 4);
+  const uint32_t tid = threadIdx.x, nthreads = blockDim.x;
   if (level0 && ext.add && tid == 0) st->counter[1] = n;
   const bool all = n <= CTA_RULERS;  // every element is a ruler
   const Rulers rl = make_rulers((n + CTA_RULERS - 1) / CTA_RULERS, 0x63746121u);
   const uint32_t rulers = all ? n : (n + rl.s - 1) / rl.s;
-  auto ruler = [&](uint32_t x, uint32_t* j) {
-    if (all) {
-      *j = x;
-      return true;
-    }
-    return rl.is(x, j);
+  auto ruler = [&](uint32_t x) {
+    uint32_t j;
+    return all || rl.is(x, &j);
   };
+  auto elem = [&](uint32_t j) { return all ? j : (uint32_t)rl.elem(j); };
   bool stamp = true;
   uint32_t heads = 0;
   while (true) {
-    if (tid == 0) nends = nheads = 0;
-    for (uint32_t w = tid; w < words; w += CTA_THREADS) pred[w] = 0;
+    if (tid == 0) nends = nheads = nstamps = 0;
+    for (uint32_t w = tid; w < (n + 3) / 4; w += nthreads) predw[w] = 0;
     __syncthreads();
     uint32_t ends = 0;
-    for (uint32_t x0 = tid; x0 < n; x0 += CTA_THREADS * CTA_LOADS) {
+    for (uint32_t x0 = tid; x0 < n; x0 += nthreads * CTA_LOADS) {
       uint64_t a[CTA_LOADS];
       uint32_t b[CTA_LOADS];
 #pragma unroll
       for (uint32_t i = 0; i < CTA_LOADS; ++i) {
-        const uint32_t x = x0 + i * CTA_THREADS;
+        const uint32_t x = x0 + i * nthreads;
         if (x < n) src.load(x, &a[i], &b[i]);
       }
 #pragma unroll
       for (uint32_t i = 0; i < CTA_LOADS; ++i) {
-        const uint32_t x = x0 + i * CTA_THREADS;
+        const uint32_t x = x0 + i * nthreads;
         if (x >= n) continue;
         if (b[i] >= n) {
           set_error(st, KASCADE_ERR_OUT_OF_RANGE, x);
@@ -558,33 +523,31 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) k_rank_cta(Src src, Extent ext
     __syncthreads();
     // what each successor is; with several lists, who has a predecessor
     const bool many = stamp && !all && nends > 2;
-    for (uint32_t x0 = tid; x0 < n; x0 += CTA_THREADS * CTA_ILP) {
+    for (uint32_t x0 = tid; x0 < n; x0 += nthreads * CTA_ILP) {
       uint32_t y[CTA_ILP], z[CTA_ILP];
 #pragma unroll
       for (uint32_t i = 0; i < CTA_ILP; ++i) {
-        const uint32_t x = x0 + i * CTA_THREADS;
+        const uint32_t x = x0 + i * nthreads;
         y[i] = x < n ? next[x] : x;
       }
 #pragma unroll
-      for (uint32_t i = 0; i < CTA_ILP; ++i) z[i] = x0 + i * CTA_THREADS < n ? next[y[i]] & CTA_IDX : 0u;
+      for (uint32_t i = 0; i < CTA_ILP; ++i) z[i] = x0 + i * nthreads < n ? next[y[i]] & CTA_IDX : 0u;
 #pragma unroll
       for (uint32_t i = 0; i < CTA_ILP; ++i) {
-        const uint32_t x = x0 + i * CTA_THREADS;
-        uint32_t j;
+        const uint32_t x = x0 + i * nthreads;
         if (x >= n || y[i] == x) continue;
-        next[x] = y[i] | (z[i] == y[i] ? CTA_END : 0u) | (ruler(y[i], &j) ? CTA_RUL : 0u);
-        if (many) atomicOr(&pred[y[i] >> 5], 1u << (y[i] & 31));
+        next[x] = y[i] | (z[i] == y[i] ? CTA_END : 0u) | (ruler(y[i]) ? CTA_RUL : 0u);
+        if (many) pred[y[i]] = 1;
       }
     }
     __syncthreads();
     if (many) {
-      for (uint32_t w = tid; w < words; w += CTA_THREADS) {
-        uint32_t m = ~pred[w];
-        while (m) {
-          const uint32_t x = w * 32 + (uint32_t)__ffs(m) - 1;
-          m &= m - 1;
-          uint32_t j;
-          if (x >= n || next[x] == x || rl.is(x, &j)) continue;
+      for (uint32_t w = tid; w < (n + 3) / 4; w += nthreads) {
+        const uint32_t pw = predw[w];
+        if (pw == 0x01010101u) continue;
+        for (uint32_t i = 0; i < 4; ++i) {
+          const uint32_t x = w * 4 + i;
+          if (((pw >> (8 * i)) & 1u) || x >= n || next[x] == x || ruler(x)) continue;
           const uint32_t e = atomicAdd(&nheads, 1u);
           if (e < CTA_HEADS) hlist[e] = (uint16_t)x;
         }
@@ -592,105 +555,84 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) k_rank_cta(Src src, Extent ext
       __syncthreads();
       heads = min(nheads, CTA_HEADS);
     }
-    // chains: ids of rulers, then (from CTA_RULERS on) of heads; a thread's
-    // chains go hop by hop together
-    uint32_t id[CTA_CHAINS], cur[CTA_CHAINS], hops = 0, act = 0;
-    unsigned long long acc[CTA_CHAINS];
-    int clash = 0;
-    // the chain has passed acc and its next word is f: at its end, or at cur
-    auto arrive = [&](uint32_t c, uint32_t f) {
-      const uint32_t y = f & CTA_IDX;
-      if (f & CTA_RUL) {
-        rdist[id[c]] = acc[c];
-        rnext[id[c]] = all ? y : rl.block_of(y);
-        return false;
+    // chains of the rulers, then (ids from CTA_RULERS on) of the heads
+    uint32_t stamps = 0, loops = 0;
+    for (uint32_t k = tid; k < rulers + heads; k += nthreads) {
+      const uint32_t id = k < rulers ? k : CTA_RULERS + (k - rulers);
+      const uint32_t x0 = k < rulers ? elem(k) : hlist[k - rulers];
+      if (x0 >= n) continue;
+      uint32_t f = next[x0];
+      unsigned long long acc = dist[x0];
+      if (f == x0) {  // a list's end
+        rdist[id] = acc;
+        rnext[id] = CTA_FLAG | x0;
+        continue;
       }
-      if (f & CTA_END) {
-        rdist[id[c]] = acc[c] + dist[y];
-        rnext[id[c]] = CTA_FLAG | y;
-        return false;
-      }
-      cur[c] = y;
-      return true;
-    };
-    auto begin = [&](uint32_t c) {
-      uint32_t x0 = n;
-      if (id[c] < rulers)
-        x0 = all ? id[c] : (uint32_t)rl.elem(id[c]);
-      else if (id[c] >= CTA_RULERS && id[c] - CTA_RULERS < heads)
-        x0 = hlist[id[c] - CTA_RULERS];
-      if (x0 >= n) return false;
-      const uint32_t f = next[x0];
-      acc[c] = dist[x0];
-      if (f == x0) {
-        rdist[id[c]] = acc[c];
-        rnext[id[c]] = CTA_FLAG | x0;
-        return false;
-      }
-      if (id[c] >= CTA_RULERS) {  // a head is stamped by its own chain
-        next[x0] = CTA_FLAG | id[c];
+      if (stamp) {  // no other chain passes a ruler or a head
+        next[x0] = CTA_FLAG | id;
         dist[x0] = 0;
       }
-      return arrive(c, f);
-    };
-#pragma unroll
-    for (uint32_t c = 0; c < CTA_CHAINS; ++c) {
-      id[c] = tid + c * CTA_THREADS;
-      cur[c] = 0;
-      acc[c] = 0;
-      bool on = begin(c);
-      if (!on && heads) {
-        id[c] += CTA_RULERS;
-        on = begin(c);
+      uint32_t hops = 0;
+      while (!(f & (CTA_FLAG | CTA_END | CTA_RUL))) {
+        const uint32_t x = f;
+        f = next[x];
+        const unsigned long long w = dist[x];
+        if (stamp) {
+          next[x] = CTA_FLAG | id;
+          dist[x] = acc;
+          ++stamps;
+        } else if (++hops > n) {  // a cycle without a ruler
+          f = CTA_FLAG;
+        }
+        acc += w;
       }
-      if (on) act |= 1u << c;
-    }
-    while (act) {
-      ++hops;
-#pragma unroll
-      for (uint32_t c = 0; c < CTA_CHAINS; ++c) {
-        if (!((act >> c) & 1u)) continue;
-        const uint32_t x = cur[c];
-        const uint32_t f = stamp ? atomicExch(&next[x], CTA_FLAG | id[c]) : next[x];
-        bool on = false;
-        if ((f & CTA_FLAG) || hops > 2 * n) {
-          // two chains met, or a cycle without a ruler
-          if (f & CTA_FLAG) clash = 1;
-          rdist[id[c]] = 0;
-          rnext[id[c]] = id[c];  // never ends: the rounds below report the cycle
-        } else {
-          const unsigned long long w = dist[x];
-          if (stamp) dist[x] = acc[c];
-          acc[c] += w;
-          on = arrive(c, f);
-        }
-        if (!on && id[c] < CTA_RULERS && heads) {
-          id[c] += CTA_RULERS;
-          on = begin(c);
-        }
-        if (!on) act &= ~(1u << c);
+      const uint32_t y = f & CTA_IDX;
+      if (f & CTA_FLAG) {  // another chain's element: counted below
+        loops = 1;
+        rdist[id] = 0;
+        rnext[id] = id < CTA_RULERS ? id : 0u;
+      } else if (f & CTA_RUL) {
+        rdist[id] = acc;
+        rnext[id] = all ? y : rl.block_of(y);
+      } else {
+        rdist[id] = acc + (y == x0 ? 0ull : dist[y]);
+        rnext[id] = CTA_FLAG | y;
       }
     }
-    clash = __syncthreads_or(clash);
-    if (!clash) break;
+    if (!stamp) break;
+    stamps = __reduce_add_sync(FULL, stamps);
+    if ((tid & 31u) == 0 && stamps) atomicAdd(&nstamps, stamps);
+    uint32_t marks = 0;  // stamped elements that are no chain's first
+    const int clash = __syncthreads_or((int)loops);
+    for (uint32_t x = tid; x < n; x += nthreads) marks += next[x] >> 31;
+    for (uint32_t k = tid; k < rulers + heads; k += nthreads) {
+      const uint32_t x0 = k < rulers ? elem(k) : hlist[k - rulers];
+      if (x0 < n && (next[x0] & CTA_FLAG)) --marks;
+    }
+    marks = __reduce_add_sync(FULL, marks);
+    if ((tid & 31u) == 0 && marks) atomicSub(&nstamps, marks);
+    __syncthreads();
+    if (!clash && nstamps == 0) break;
     if (n > tree_max) {
       if (tid == 0) set_error(st, KASCADE_ERR_NOT_A_LIST, n);
       return;
     }
+    __syncthreads();
     stamp = false;  // again from the source, without stamps
     heads = 0;
   }
+  __syncthreads();
   // pointer jumping over the rulers
   for (int round = 0;; ++round) {
-    unsigned long long d[CTA_CHAINS];
-    uint32_t nx[CTA_CHAINS];
+    unsigned long long d[CTA_RULERS / 256];
+    uint32_t nx[CTA_RULERS / 256];
     int busy = 0;
 #pragma unroll
-    for (uint32_t c = 0; c < CTA_CHAINS; ++c) {
-      const uint32_t j = tid + c * CTA_THREADS;
+    for (uint32_t c = 0; c < CTA_RULERS / 256; ++c) {
+      const uint32_t j = tid + c * nthreads;
       nx[c] = CTA_FLAG;
       d[c] = 0;
-      if (j >= rulers || (!all && rl.elem(j) >= n)) continue;
+      if (j >= rulers || elem(j) >= n) continue;
       nx[c] = rnext[j];
       d[c] = rdist[j];
       if (!(nx[c] & CTA_FLAG)) {
@@ -705,16 +647,16 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) k_rank_cta(Src src, Extent ext
       return;
     }
 #pragma unroll
-    for (uint32_t c = 0; c < CTA_CHAINS; ++c) {
-      const uint32_t j = tid + c * CTA_THREADS;
-      if (j >= rulers || (!all && rl.elem(j) >= n)) continue;
+    for (uint32_t c = 0; c < CTA_RULERS / 256; ++c) {
+      const uint32_t j = tid + c * nthreads;
+      if (j >= rulers || elem(j) >= n) continue;
       rdist[j] = d[c];
       rnext[j] = nx[c];
     }
     __syncthreads();
   }
   // the heads' chains end at a ruler or a list end; then every chain's root
-  for (uint32_t h = tid; h < heads; h += CTA_THREADS) {
+  for (uint32_t h = tid; h < heads; h += nthreads) {
     const uint32_t j = CTA_RULERS + h, nx = rnext[j];
     if (!(nx & CTA_FLAG)) {
       rdist[j] += rdist[nx];
@@ -722,33 +664,35 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) k_rank_cta(Src src, Extent ext
     }
   }
   __syncthreads();
-  for (uint32_t j = tid; j < CTA_RULERS + heads; j += CTA_THREADS)
-    if (j < rulers ? (all || rl.elem(j) < n) : j >= CTA_RULERS) rnext[j] = src.root_of(rnext[j] & ~CTA_FLAG);
+  for (uint32_t k = tid; k < rulers + heads; k += nthreads) {
+    const uint32_t j = k < rulers ? k : CTA_RULERS + (k - rulers);
+    if (k >= rulers || elem(k) < n) rnext[j] = src.root_of(rnext[j] & ~CTA_FLAG);
+  }
   __syncthreads();
-  for (uint32_t x0 = tid; x0 < n; x0 += CTA_THREADS * CTA_ILP) {
-    uint32_t f[CTA_ILP], j[CTA_ILP];
+  for (uint32_t x0 = tid; x0 < n; x0 += nthreads * CTA_ILP) {
+    uint32_t f[CTA_ILP];
     unsigned long long d[CTA_ILP];
 #pragma unroll
     for (uint32_t i = 0; i < CTA_ILP; ++i) {
-      const uint32_t x = x0 + i * CTA_THREADS;
+      const uint32_t x = x0 + i * nthreads;
       f[i] = x < n ? next[x] : 0u;
       d[i] = x < n ? dist[x] : 0ull;
     }
 #pragma unroll
     for (uint32_t i = 0; i < CTA_ILP; ++i) {
-      const uint32_t x = x0 + i * CTA_THREADS;
+      const uint32_t x = x0 + i * nthreads;
       if (x >= n) continue;
-      const bool end = f[i] == x;
-      uint32_t root = 0;
-      if (ruler(x, &j[i])) {
-        d[i] = rdist[j[i]];
-        root = rnext[j[i]];
-      } else if (f[i] & CTA_FLAG) {
+      uint32_t root = 0, j;
+      if (f[i] & CTA_FLAG) {
         d[i] = rdist[f[i] & CTA_IDX] - d[i];
         root = rnext[f[i] & CTA_IDX];
-      } else if (end) {
+      } else if (f[i] == x) {
         root = src.root_of(x);
-      } else {  // ahead of its list's first ruler: walk
+      } else if (!stamp && (all || rl.is(x, &j))) {
+        j = all ? x : rl.block_of(x);
+        d[i] = rdist[j];
+        root = rnext[j];
+      } else {  // ahead of its list's first ruler (or nothing is stamped): walk
         uint32_t hops = 0, w = f[i];
         bool ok = true;
         while (true) {
@@ -779,7 +723,7 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) k_rank_cta(Src src, Extent ext
         }
         if (!ok) continue;
       }
-      sink.put(x, d[i], root, end);
+      sink.put(x, d[i], root, f[i] == x);
     }
   }
 }
@@ -884,13 +828,13 @@ int occupancy(K kernel, int block, size_t smem) {
   return nb < 1 ? 1 : nb;
 }
 
-// Resident blocks per SM of the chase, by chains per thread and block size.
-template <int C>
+// Resident blocks per SM of the chase.
+template <class F>
 int chase_occupancy(uint32_t block) {
   static std::atomic<int> occ[3] = {{-1}, {-1}, {-1}};  // blocks of 128, 256, 512 threads
   const int bi = block == 128 ? 0 : block == 512 ? 2 : 1;
   int v = occ[bi].load();
-  if (v < 0) occ[bi].store(v = occupancy(k_chase<C>, (int)block, 0));
+  if (v < 0) occ[bi].store(v = occupancy(k_chase<F>, (int)block, 0));
   return v;
 }
 
@@ -898,51 +842,41 @@ int chase_occupancy(uint32_t block) {
 // L2 serves dependent hops of this many resident warps at full speed.
 constexpr uint64_t CHASE_SPREAD_WARPS_PER_SM = 32;
 
-template <int C>
-kascade_status launch_chase_c(kascade_ctx& ctx, const Levels& lv, int k, const Extent& ext, uint32_t block,
-                              cudaStream_t s) {
+// Level k's chase.  limit: the elements whose results are wanted.
+template <class F>
+kascade_status launch_chase(kascade_ctx& ctx, const Levels& lv, int k, const typename F::R* rec, typename F::S* stamp,
+                            const Extent& ext, uint32_t limit, uint32_t block, cudaStream_t s) {
   const uint32_t r = lv.n[k + 1];
   const uint64_t wpb = block / 32;
-  const uint64_t max_grid = (uint64_t)ctx.usable_sms() * chase_occupancy<C>(block);
+  const uint64_t max_grid = (uint64_t)ctx.usable_sms() * chase_occupancy<F>(block);
   const uint64_t spread = std::min<uint64_t>(max_grid * wpb, (uint64_t)ctx.usable_sms() * CHASE_SPREAD_WARPS_PER_SM);
-  const uint32_t lanes = (uint32_t)std::min<uint64_t>(32, std::max<uint64_t>(1, (r + spread * C - 1) / (spread * C)));
-  const uint64_t need = ((uint64_t)r + lanes * C - 1) / (lanes * C);  // warps worth of work
+  const uint32_t lanes = (uint32_t)std::min<uint64_t>(32, std::max<uint64_t>(1, (r + spread - 1) / spread));
+  const uint64_t need = ((uint64_t)r + lanes - 1) / lanes;  // warps worth of work
   const unsigned grid = (unsigned)std::min<uint64_t>(max_grid, (need + wpb - 1) / wpb);
   ProfScope ps(ctx, "chase", s);
-  k_chase<C><<<grid, block, 0, s>>>(lv.rec[k], ext, lv.rulers[k], lv.r[k], lv.heads, k ? lv.r[k - 1] : 0u,
-                                    lv.rootel[k], lv.rec[k + 1], lv.rootel[k + 1], &ctx.d_status->work[k], lanes,
+  k_chase<F><<<grid, block, 0, s>>>(rec, stamp, ext, lv.rulers[k], lv.r[k], lv.heads, k ? lv.r[k - 1] : 0u,
+                                    lv.rootel[k], lv.rulers[k + 1], lv.rec[k + 1], lv.stamp[k + 1],
+                                    lv.rootel[k + 1], &ctx.d_status->work[k], lanes, limit, hop_cap(lv.rulers[k]),
                                     ctx.d_status);
   KS_CHECK_LAUNCH();
   return KASCADE_OK;
 }
 
-// Level k's chase (k = 0: the caller's records).
-kascade_status launch_chase(kascade_ctx& ctx, const Levels& lv, int k, const Extent& ext, uint32_t chains,
-                            uint32_t block, cudaStream_t s) {
-  switch (chains) {
-    case 1:
-      return launch_chase_c<1>(ctx, lv, k, ext, block, s);
-    case 4:
-      return launch_chase_c<4>(ctx, lv, k, ext, block, s);
-    default:
-      return launch_chase_c<2>(ctx, lv, k, ext, block, s);
-  }
-}
-
 // Level k's results from level k + 1's.  Small levels take two elements per
 // thread instead of eight, so that they fill the chip.
-template <class Sink>
-kascade_status launch_propagate(kascade_ctx& ctx, const Levels& lv, int k, uint32_t n_out, const Extent& ext,
-                                const Sink& sink, cudaStream_t s) {
+template <class F, class Sink>
+kascade_status launch_propagate(kascade_ctx& ctx, const Levels& lv, int k, const typename F::R* rec,
+                                const typename F::S* stamp, uint32_t n_out, const Extent& ext, const Sink& sink,
+                                cudaStream_t s) {
   ProfScope ps(ctx, "propagate", s);
   if (n_out <= (uint64_t)ctx.usable_sms() * 256 * 8 * 4) {
     const unsigned grid = grid_for(ctx, ((uint64_t)n_out + 1) / 2, 256, 8);
-    k_propagate<Sink, 2><<<grid, 256, 0, s>>>(lv.rec[k], n_out, ext, lv.rulers[k], lv.r[k], lv.rootel[k],
-                                              lv.out[k + 1], sink, ctx.d_status);
+    k_propagate<F, Sink, 2><<<grid, 256, 0, s>>>(rec, stamp, n_out, ext, lv.rulers[k], lv.r[k], lv.rootel[k],
+                                                 lv.out[k + 1], sink, ctx.d_status);
   } else {
     const unsigned grid = grid_for(ctx, ((uint64_t)n_out + 7) / 8, 256, 8);
-    k_propagate<Sink, 8><<<grid, 256, 0, s>>>(lv.rec[k], n_out, ext, lv.rulers[k], lv.r[k], lv.rootel[k],
-                                              lv.out[k + 1], sink, ctx.d_status);
+    k_propagate<F, Sink, 8><<<grid, 256, 0, s>>>(rec, stamp, n_out, ext, lv.rulers[k], lv.r[k], lv.rootel[k],
+                                                 lv.out[k + 1], sink, ctx.d_status);
   }
   KS_CHECK_LAUNCH();
   return KASCADE_OK;
@@ -959,7 +893,9 @@ kascade_status launch_rank_cta(kascade_ctx& ctx, const Src& src, const Extent& e
     raised.fetch_or(bit);
   }
   ProfScope ps(ctx, "base_case", s);
-  k_rank_cta<Src, Sink><<<1, CTA_THREADS, cta_smem(ext.cap), s>>>(src, ext, sink, tree_max, level0, ctx.d_status);
+  // one ruler per thread; a small input's few barriers are cheaper with fewer warps
+  const unsigned threads = ext.cap <= 1024 ? 256 : CTA_THREADS;
+  k_rank_cta<Src, Sink><<<1, threads, cta_smem(ext.cap), s>>>(src, ext, sink, tree_max, level0, ctx.d_status);
   KS_CHECK_LAUNCH();
   return KASCADE_OK;
 }
@@ -1012,11 +948,7 @@ Params make_params(const kascade_ctx& ctx, const kascade_opts* o, uint64_t n) {
     if (o->block_size) p.block = o->block_size;
     if (o->seed) p.seed = o->seed;
     p.algorithm = o->algorithm;
-    if (o->struct_size >= offsetof(kascade_opts, max_chain) + sizeof(uint32_t)) {
-      if (o->level0_mode == 1) p.level0_log_min = 0xFFFFFFFFu;
-      if (o->level0_mode == 2) p.level0_log_min = 0;
-      p.max_chain = o->max_chain;
-    }
+    if (o->struct_size >= offsetof(kascade_opts, max_chain) + sizeof(uint32_t)) p.level0_mode = o->level0_mode;
   }
   if (p.base_max > ONE_CTA_MAX) p.base_max = ONE_CTA_MAX;
   if (p.block != 128 && p.block != 512) p.block = 256;
@@ -1025,54 +957,103 @@ Params make_params(const kascade_ctx& ctx, const kascade_opts* o, uint64_t n) {
   return p;
 }
 
-kascade_status prepare_arrays(kascade_ctx& ctx, const uint64_t* succ, WKind wk, const void* w, uint32_t n, Rec* rec,
-                              const Params& p, cudaStream_t s) {
-  (void)p;
-  ProfScope ps(ctx, "prepare", s);
-  // full tiles of 16 B-aligned inputs go through the bulk-copy kernel
+// The three ways to run level 0, by what stays in L2 (lists of random order,
+// unit / 32-bit / 64-bit weights, us):
+//   split records and stamps while both fit: 4e6 elements 247 / 310 / 417
+//     against 279 / 287 / 331 with the stamp in the record, 3e6 213 / 224
+//     against 242 / 249, 6e6 396 / 500 / 617 against 384 / 389 / 444
+//   stamps in 16 B records while those fit, 8e6: 531 / 536 / 605
+//   write-free above: 8e6 522 / 528 / 653, 1.2e7 711 / 719 against 815 / 823
+Level0Plan plan_level0(const Params& p, uint64_t n, WKind wk) {
+  constexpr uint64_t SPLIT_BYTES = 88ull << 20;
+  const uint64_t split = n * (wk == WKind::Unit ? 16 : wk == WKind::U32 ? 24 : 32);
+  const uint64_t log_min = wk == WKind::I64 ? 12000000 : 8000000;
+  Level0Plan plan;
+  plan.write_free = p.level0_mode == 2 || (p.level0_mode != 1 && n >= log_min);
+  if (!plan.write_free && split > SPLIT_BYTES && n < F16i::NONE)
+    plan.fmt = Format::F16i;
+  else if (n > REC8_MAX || wk == WKind::I64)
+    plan.fmt = Format::F16x16;
+  else
+    plan.fmt = wk == WKind::Unit ? Format::F8x8 : Format::F8x16;
+  return plan;
+}
+
+Rulers level0_rulers(const Params& p) { return make_rulers(p.spacing0, salt_for(p.seed, 0)); }
+
+kascade_status alloc_level0(kascade_ctx& ctx, const Level0Plan& plan, uint64_t cap, Level0* l0) {
+  const bool wide = plan.fmt == Format::F16x16 || plan.fmt == Format::F16i;
+  l0->fmt = plan.fmt;
+  l0->rec = alloc<char>(ctx, cap * (wide ? 16 : 8));
+  if (!l0->rec) return KASCADE_ERR_OOM;
+  if (plan.write_free) return KASCADE_OK;
+  l0->stamp = plan.fmt == Format::F16i ? l0->rec : alloc<char>(ctx, cap * (plan.fmt == Format::F8x8 ? 8 : 16));
+  return l0->stamp ? KASCADE_OK : KASCADE_ERR_OOM;
+}
+
+namespace {
+
+template <class F, class W>
+kascade_status prepare_plain(kascade_ctx& ctx, const uint64_t* succ, const W& w, uint32_t n, uint64_t start,
+                             const Level0& l0, const Rulers& rl, cudaStream_t s) {
+  if (start >= n) return KASCADE_OK;
+  const uint64_t rest = n - start;
+  const unsigned grid = grid_for(ctx, (rest + 256 * PREP_ITEMS - 1) / (256 * PREP_ITEMS) * 256, 256, 8);
+  k_prepare_arrays<F, W><<<grid, 256, 0, s>>>(succ, w, n, start, rl, l0.records<F>(), l0.stamps<F>(), ctx.d_status);
+  KS_CHECK_LAUNCH();
+  return KASCADE_OK;
+}
+
+// Full tiles of 16 B-aligned inputs go through the bulk-copy kernel, the rest
+// through the plain one.
+template <class F, bool W32, class W>
+kascade_status prepare_tiles(kascade_ctx& ctx, const uint64_t* succ, const uint32_t* w32, const W& w, uint32_t n,
+                             const Level0& l0, const Rulers& rl, cudaStream_t s) {
   uint64_t start = 0;
-  const bool aligned = (reinterpret_cast<uintptr_t>(succ) % 16 == 0) &&
-                       (wk == WKind::Unit || (wk == WKind::U32 && reinterpret_cast<uintptr_t>(w) % 16 == 0));
+  const bool aligned = reinterpret_cast<uintptr_t>(succ) % 16 == 0 &&
+                       (!W32 || reinterpret_cast<uintptr_t>(w32) % 16 == 0);
   const uint32_t ntiles = n / PT_TILE;
   if (aligned && ntiles >= (uint32_t)ctx.usable_sms()) {
     const unsigned g = (unsigned)std::min<uint64_t>(ntiles, (uint64_t)ctx.usable_sms() * 2);
-    if (wk == WKind::U32) {
-      constexpr int smem = PT_STAGES * PT_TILE * 12;
-      static bool raised = false;
-      if (!raised) {
-        KS_CUDA(cudaFuncSetAttribute(k_prepare_tma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        raised = true;
-      }
-      k_prepare_tma<true><<<g, 256, smem, s>>>(succ, (const uint32_t*)w, n, ntiles, rec, ctx.d_status);
-    } else {
-      constexpr int smem = PT_STAGES * PT_TILE * 8;
-      static bool raised = false;
-      if (!raised) {
-        KS_CUDA(cudaFuncSetAttribute(k_prepare_tma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        raised = true;
-      }
-      k_prepare_tma<false><<<g, 256, smem, s>>>(succ, nullptr, n, ntiles, rec, ctx.d_status);
+    constexpr int smem = PT_STAGES * PT_TILE * (W32 ? 12 : 8);
+    static std::atomic<uint64_t> raised{0};
+    const uint64_t bit = 1ull << (ctx.device & 63);
+    if (!(raised.load() & bit)) {
+      KS_CUDA(cudaFuncSetAttribute(k_prepare_tma<F, W32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      raised.fetch_or(bit);
     }
+    k_prepare_tma<F, W32><<<g, 256, smem, s>>>(succ, w32, n, ntiles, rl, l0.records<F>(), l0.stamps<F>(),
+                                                ctx.d_status);
     KS_CHECK_LAUNCH();
     start = (uint64_t)ntiles * PT_TILE;
   }
-  if (start < n) {
-    const uint64_t rest = n - start;
-    const unsigned grid = grid_for(ctx, (rest + 256 * PREP_ITEMS - 1) / (256 * PREP_ITEMS) * 256, 256, 8);
-    switch (wk) {
-      case WKind::Unit:
-        k_prepare_arrays<WUnit><<<grid, 256, 0, s>>>(succ, WUnit{}, n, start, rec, ctx.d_status);
-        break;
-      case WKind::U32:
-        k_prepare_arrays<WU32><<<grid, 256, 0, s>>>(succ, WU32{(const uint32_t*)w}, n, start, rec, ctx.d_status);
-        break;
-      case WKind::I64:
-        k_prepare_arrays<WI64><<<grid, 256, 0, s>>>(succ, WI64{(const int64_t*)w}, n, start, rec, ctx.d_status);
-        break;
-    }
-    KS_CHECK_LAUNCH();
+  return prepare_plain<F>(ctx, succ, w, n, start, l0, rl, s);
+}
+
+}  // namespace
+
+kascade_status prepare_arrays(kascade_ctx& ctx, const uint64_t* succ, WKind wk, const void* w, uint32_t n,
+                              const Level0& l0, const Rulers& rl, cudaStream_t s) {
+  ProfScope ps(ctx, "prepare", s);
+  const uint32_t* w32 = static_cast<const uint32_t*>(w);
+  if (wk == WKind::Unit && l0.fmt == Format::F8x8)
+    return prepare_tiles<F8x8, false>(ctx, succ, nullptr, WUnit{}, n, l0, rl, s);
+  if (wk == WKind::U32 && l0.fmt == Format::F8x16)
+    return prepare_tiles<F8x16, true>(ctx, succ, w32, WU32{w32}, n, l0, rl, s);
+  if (l0.fmt == Format::F16i) {
+    if (wk == WKind::Unit) return prepare_tiles<F16i, false>(ctx, succ, nullptr, WUnit{}, n, l0, rl, s);
+    if (wk == WKind::U32) return prepare_tiles<F16i, true>(ctx, succ, w32, WU32{w32}, n, l0, rl, s);
+    return prepare_plain<F16i>(ctx, succ, WI64{static_cast<const int64_t*>(w)}, n, 0, l0, rl, s);
   }
-  return KASCADE_OK;
+  // 64-bit records (pointer doubling takes these for every weight kind)
+  switch (wk) {
+    case WKind::Unit:
+      return prepare_plain<F16x16>(ctx, succ, WUnit{}, n, 0, l0, rl, s);
+    case WKind::U32:
+      return prepare_plain<F16x16>(ctx, succ, WU32{w32}, n, 0, l0, rl, s);
+    default:
+      return prepare_plain<F16x16>(ctx, succ, WI64{static_cast<const int64_t*>(w)}, n, 0, l0, rl, s);
+  }
 }
 
 kascade_status rank_arrays_one_cta(kascade_ctx& ctx, const uint64_t* succ, WKind wk, const void* w, uint32_t n,
@@ -1163,6 +1144,9 @@ static kascade_status pointer_double_level(kascade_ctx& ctx, const Rec* rec, con
   return KASCADE_OK;
 }
 
+// Ruler gaps are geometric: longer than this has probability ~e^-64.
+uint32_t hop_cap(const Rulers& rl) { return (uint32_t)std::min<uint64_t>(64ull * rl.s + 1024, 0xFFFFFFFFull); }
+
 kascade_status plan_levels(kascade_ctx& ctx, uint32_t n, const Heads& heads, const Params& p, Levels* lv) {
   *lv = Levels{};
   const int max_levels = (int)std::min<uint32_t>(p.max_levels, MAX_LEVELS);
@@ -1178,7 +1162,7 @@ kascade_status plan_levels(kascade_ctx& ctx, uint32_t n, const Heads& heads, con
     const uint32_t sp = k == 0           ? p.spacing0
                         : p.spacing_deep ? p.spacing_deep
                                          : deep_spacing(m, ONE_CTA_MAX - extra);
-    lv->rulers[k] = make_rulers(sp, salt_for(p.seed, k));
+    lv->rulers[k] = k == 0 ? level0_rulers(p) : make_rulers(sp, salt_for(p.seed, k));
     lv->r[k] = m = ruler_count(m, lv->rulers[k]);
     lv->n[k + 1] = m + extra;
     ++k;
@@ -1188,48 +1172,64 @@ kascade_status plan_levels(kascade_ctx& ctx, uint32_t n, const Heads& heads, con
   for (int i = 1; i <= k; ++i) {
     ctx.last_levels.push_back(lv->r[i - 1]);
     lv->rec[i] = alloc<Rec>(ctx, lv->n[i]);
+    lv->stamp[i] = i < k ? alloc<uint4>(ctx, lv->n[i]) : nullptr;
     lv->rootel[i] = alloc<uint32_t>(ctx, lv->n[i]);
     lv->out[i] = alloc<Out>(ctx, lv->n[i]);
-    if (!lv->rec[i] || !lv->rootel[i] || !lv->out[i]) return KASCADE_ERR_OOM;
+    if (!lv->rec[i] || (i < k && !lv->stamp[i]) || !lv->rootel[i] || !lv->out[i]) return KASCADE_ERR_OOM;
   }
   return KASCADE_OK;
 }
 
-kascade_status rank_deep(kascade_ctx& ctx, const Levels& lv, const Params& p, cudaStream_t s) {
-  // deeper levels are L2-resident: one chain per thread saturates the L2
-  (void)p;
-  for (int k = 1; k < lv.last; ++k) KS_TRY(launch_chase(ctx, lv, k, lv.extent(k), 1, 256, s));
+kascade_status rank_deep(kascade_ctx& ctx, const Levels& lv, cudaStream_t s) {
+  for (int k = 1; k < lv.last; ++k)
+    KS_TRY(launch_chase<F16x16>(ctx, lv, k, lv.rec[k], lv.stamp[k], lv.extent(k), lv.n[k], 256, s));
   const int L = lv.last;
   if (lv.n[L] <= ONE_CTA_MAX) {
-    KS_TRY(launch_rank_cta(ctx, CtaRecords{lv.rec[L], lv.rootel[L]}, lv.extent(L), SinkOut{lv.out[L]}, 0, 0, s));
+    KS_TRY(launch_rank_cta(ctx, CtaRecords<F16x16>{lv.rec[L], lv.rootel[L]}, lv.extent(L), SinkOut{lv.out[L]}, 0, 0,
+                           s));
   } else {
     KS_TRY(pointer_double_level(ctx, lv.rec[L], lv.extent(L), lv.rootel[L], lv.out[L], s));
   }
-  for (int k = L - 1; k >= 1; --k) KS_TRY(launch_propagate(ctx, lv, k, lv.n[k], lv.extent(k), SinkOut{lv.out[k]}, s));
+  for (int k = L - 1; k >= 1; --k)
+    KS_TRY(launch_propagate<F16x16>(ctx, lv, k, lv.rec[k], lv.stamp[k], lv.n[k], lv.extent(k), SinkOut{lv.out[k]},
+                                    s));
   return KASCADE_OK;
 }
 
-template <class Sink>
-kascade_status rank_records(kascade_ctx& ctx, Rec* rec, uint32_t n, const Extent& ext, const Heads& heads,
-                            const Sink& sink, const Params& p, cudaStream_t s, bool host_check) {
-  if (n == 0) return KASCADE_OK;
+namespace {
+
+template <class F, class Sink>
+kascade_status rank_records_as(kascade_ctx& ctx, const Level0& l0, uint32_t n, const Extent& ext, const Heads& heads,
+                               const Sink& sink, const Params& p, cudaStream_t s) {
+  const typename F::R* rec = l0.records<F>();
   if (n <= p.base_max) {
     ctx.last_levels.assign(1, n);
-    return launch_rank_cta(ctx, CtaRecords{rec, nullptr}, ext, sink, ONE_CTA_TREES, 1, s);
-  }
-  if (Sink::kWriteFree && n >= p.level0_log_min && !sink.log_target(n).keep_roots) {
-    const kascade_status st = rank_level0_log(ctx, rec, n, ext, heads, sink.log_target(n), p, s, host_check);
-    if (!host_check || st != KASCADE_ERR_TIMEOUT) return st;
-    // a chain exceeded the write-free path's hop cap (invalid input, or an
-    // astronomically unlikely ruler gap): redo level 0 on the stamping path
-    KS_TRY(status_reset(ctx, s));
+    return launch_rank_cta(ctx, CtaRecords<F>{rec, nullptr}, ext, sink, ONE_CTA_TREES, 1, s);
   }
   Levels lv;
   KS_TRY(plan_levels(ctx, n, heads, p, &lv));
-  lv.rec[0] = rec;
-  KS_TRY(launch_chase(ctx, lv, 0, ext, p.chains, p.block, s));
-  KS_TRY(rank_deep(ctx, lv, p, s));
-  return launch_propagate(ctx, lv, 0, sink.limit(n), ext, sink, s);
+  KS_TRY(launch_chase<F>(ctx, lv, 0, rec, l0.stamps<F>(), ext, sink.limit(n), p.block, s));
+  KS_TRY(rank_deep(ctx, lv, s));
+  return launch_propagate<F>(ctx, lv, 0, rec, l0.stamps<F>(), sink.limit(n), ext, sink, s);
+}
+
+}  // namespace
+
+template <class Sink>
+kascade_status rank_records(kascade_ctx& ctx, const Level0& l0, uint32_t n, const Extent& ext, const Heads& heads,
+                            const Sink& sink, const Params& p, cudaStream_t s) {
+  if (n == 0) return KASCADE_OK;
+  if (n > p.base_max && !l0.stamp) return rank_level0_log(ctx, l0, n, ext, heads, sink.log_target(n), p, s);
+  switch (l0.fmt) {
+    case Format::F8x8:
+      return rank_records_as<F8x8>(ctx, l0, n, ext, heads, sink, p, s);
+    case Format::F8x16:
+      return rank_records_as<F8x16>(ctx, l0, n, ext, heads, sink, p, s);
+    case Format::F16i:
+      return rank_records_as<F16i>(ctx, l0, n, ext, heads, sink, p, s);
+    default:
+      return rank_records_as<F16x16>(ctx, l0, n, ext, heads, sink, p, s);
+  }
 }
 
 kascade_status check_is_list(kascade_ctx& ctx, const uint64_t* succ, uint64_t n, int* ok, cudaStream_t s) {
@@ -1252,12 +1252,12 @@ kascade_status check_is_list(kascade_ctx& ctx, const uint64_t* succ, uint64_t n,
 }
 
 // explicit instantiations for the level-0 sinks
-template kascade_status rank_records<SinkPlain>(kascade_ctx&, Rec*, uint32_t, const Extent&, const Heads&,
-                                                const SinkPlain&, const Params&, cudaStream_t, bool);
-template kascade_status rank_records<SinkTour>(kascade_ctx&, Rec*, uint32_t, const Extent&, const Heads&,
-                                               const SinkTour&, const Params&, cudaStream_t, bool);
-template kascade_status rank_records<SinkBatch>(kascade_ctx&, Rec*, uint32_t, const Extent&, const Heads&,
-                                                const SinkBatch&, const Params&, cudaStream_t, bool);
+template kascade_status rank_records<SinkPlain>(kascade_ctx&, const Level0&, uint32_t, const Extent&, const Heads&,
+                                                const SinkPlain&, const Params&, cudaStream_t);
+template kascade_status rank_records<SinkTour>(kascade_ctx&, const Level0&, uint32_t, const Extent&, const Heads&,
+                                               const SinkTour&, const Params&, cudaStream_t);
+template kascade_status rank_records<SinkBatch>(kascade_ctx&, const Level0&, uint32_t, const Extent&, const Heads&,
+                                                const SinkBatch&, const Params&, cudaStream_t);
 template kascade_status pointer_double_records<SinkPlain>(kascade_ctx&, const Rec*, uint32_t, const uint32_t*,
                                                           const SinkPlain&, cudaStream_t);
 

@@ -1,9 +1,9 @@
 // Internal interface of the ruling-set list ranker.
 //
-// Pipeline for a list of n elements held as 16 B records (Rec):
-//   prepare   : records from the caller's arrays
+// Pipeline for a list of n elements:
+//   prepare   : records {weight, successor} from the caller's arrays
 //   chase     : every ruler walks its successors until the next ruler or the
-//               list's end, stamping (ruler id, distance) into each record it
+//               list's end, stamping (ruler id, distance) for each element it
 //               passes and writing the ruler's record of the next level
 //   recurse   : the list of rulers is ranked the same way, down to a one-CTA
 //               shared-memory ranker
@@ -36,8 +36,7 @@ struct Params {
   uint32_t block = 256;
   uint32_t seed = 0x6b617363u;
   uint32_t algorithm = KASCADE_ALGO_SPARSE_RULING_SET;
-  uint32_t level0_log_min = 1u << 25;  // level 0 uses the write-free path from this size on
-  uint32_t max_chain = 0;              // write-free chase hop cap (0: 64 x spacing0 + 1024)
+  uint32_t level0_mode = 0;  // 0: by size, 1: stamps, 2: write-free
 };
 
 Params make_params(const kascade_ctx& ctx, const kascade_opts* opts, uint64_t n);
@@ -116,12 +115,15 @@ struct LogTarget {
   // bit x set: element x's rank output is one more than its rank in the list
   // (a tree rooting's leaves, whose down and up edge share one element)
   const uint32_t* plus_one = nullptr;
+  // depths: ranks modulo 2^32 -- of every element (tour), or of the instances
+  // with their bit set (a batch's forests)
+  int tour = 0;
+  const uint32_t* seg_tour = nullptr;
 };
 
 // Plain arrays. keep_roots: leave root entries untouched (the reference's
 // in-place contract); otherwise roots get (x, 0).
 struct SinkPlain {
-  static constexpr bool kWriteFree = true;
   uint64_t* root;
   uint64_t* rank;
   int keep_roots;
@@ -143,10 +145,10 @@ struct SinkPlain {
 
 // Euler tour: elements 0..nv-1 are the vertices' up edges (roots: the tour's
 // terminal element), so only those produce output.
-// leaf_bits (optional): bit v set for a leaf whose down and up edge are one
-// element of weight 0, whose rank is then one less than the leaf's depth.
+// A down edge's weight is -1 modulo 2^32, so a depth is its rank modulo 2^32.
+// leaf_bits: bit v set for a leaf whose down and up edge are one element of
+// weight 0, whose rank is then one less than the leaf's depth.
 struct SinkTour {
-  static constexpr bool kWriteFree = true;
   uint64_t* root;
   uint64_t* depth;
   uint32_t nv;
@@ -156,6 +158,7 @@ struct SinkTour {
   LogTarget log_target(uint32_t n) const {
     LogTarget t{root, depth, limit(n), keep_roots};
     t.plus_one = leaf_bits;
+    t.tour = 1;
     return t;
   }
   __device__ __forceinline__ void put(uint32_t x, uint64_t rk, uint32_t rt, bool is_root) const {
@@ -167,9 +170,9 @@ struct SinkTour {
       }
       return;
     }
-    if (leaf_bits) rk += (__ldg(leaf_bits + (x >> 5)) >> (x & 31)) & 1u;
+    const uint32_t d = (uint32_t)rk + ((__ldg(leaf_bits + (x >> 5)) >> (x & 31)) & 1u);
     __stcs(root + x, (unsigned long long)rt);
-    __stcs(depth + x, (unsigned long long)rk);
+    __stcs(depth + x, (unsigned long long)d);
   }
 };
 
@@ -177,10 +180,10 @@ struct SinkTour {
 // roots are reported relative to their instance.  seg_off holds the nseg
 // instance offsets (non-decreasing), hint[k] the instance containing element
 // k * 4096.  Elements at or beyond `total` (tour down edges) give no output.
-// plus_one (optional): bit x set for a forest leaf whose down and up edge are
-// one element, whose rank is then one less than the leaf's depth.
+// seg_tour: bit j set for a forest, whose depths are ranks modulo 2^32 (null:
+// lists only); plus_one: bit x set for a forest leaf whose down and up edge
+// are one element, whose rank is then one less than the leaf's depth.
 struct SinkBatch {
-  static constexpr bool kWriteFree = true;
   uint64_t* root;
   uint64_t* rank;
   uint32_t total;
@@ -188,26 +191,26 @@ struct SinkBatch {
   const uint32_t* hint;
   uint32_t nseg;
   const uint32_t* plus_one = nullptr;
+  const uint32_t* seg_tour = nullptr;
   uint32_t limit(uint32_t n) const { return n < total ? n : total; }
   LogTarget log_target(uint32_t n) const {
     LogTarget t{root, rank, limit(n), 0, seg_off, hint, nseg};
     t.plus_one = plus_one;
+    t.seg_tour = seg_tour;
     return t;
-  }
-  __device__ __forceinline__ uint64_t base_of(uint32_t x) const {
-    uint32_t j = __ldg(hint + (x >> 12));
-    while (j + 1 < nseg && __ldg(seg_off + j + 1) <= x) ++j;
-    return __ldg(seg_off + j);
   }
   __device__ __forceinline__ void put(uint32_t x, uint64_t rk, uint32_t rt, bool is_root) const {
     if (x >= total) return;
-    const uint64_t b = base_of(x);
+    uint32_t j = __ldg(hint + (x >> 12));
+    while (j + 1 < nseg && __ldg(seg_off + j + 1) <= x) ++j;
+    const uint64_t b = __ldg(seg_off + j);
     if (is_root) {
       __stcs(root + x, (unsigned long long)(x - b));
       __stcs(rank + x, 0ull);
       return;
     }
-    if (plus_one) rk += (__ldg(plus_one + (x >> 5)) >> (x & 31)) & 1u;
+    if (seg_tour && ((__ldg(seg_tour + (j >> 5)) >> (j & 31)) & 1u))
+      rk = (uint32_t)rk + ((__ldg(plus_one + (x >> 5)) >> (x & 31)) & 1u);
     __stcs(root + x, (unsigned long long)(rt - b));
     __stcs(rank + x, (unsigned long long)rk);
   }
@@ -215,9 +218,7 @@ struct SinkBatch {
 
 // Deeper levels write Out records.
 struct SinkOut {
-  static constexpr bool kWriteFree = false;
   Out* out;
-  uint32_t limit(uint32_t n) const { return n; }
   __device__ __forceinline__ void put(uint32_t x, uint64_t rk, uint32_t rt, bool is_root) const {
     (void)is_root;  // a deeper level's list end carries its rank like every element
     st_out(out + x, rk, rt);
@@ -227,13 +228,37 @@ struct SinkOut {
 // Weight readers for building level-0 records.
 enum class WKind { Unit, U32, I64 };
 
-// Build level-0 records from (succ, weights); a root's record carries weight 0.
-kascade_status prepare_arrays(kascade_ctx& ctx, const uint64_t* succ, WKind wk, const void* w, uint32_t n, Rec* rec,
-                              const Params& p, cudaStream_t s);
+// Level 0 of a call: its records, and their stamps on the stamping path (null
+// on the write-free one).
+struct Level0 {
+  Format fmt = Format::F16x16;
+  void* rec = nullptr;
+  void* stamp = nullptr;
+  template <class F>
+  typename F::R* records() const { return static_cast<typename F::R*>(rec); }
+  template <class F>
+  typename F::S* stamps() const { return static_cast<typename F::S*>(stamp); }
+};
+// How level 0 of n elements of that weight kind (tours: Unit) runs: the
+// records' format, and whether it takes the write-free path.
+struct Level0Plan {
+  Format fmt;
+  bool write_free;
+};
+Level0Plan plan_level0(const Params& p, uint64_t n, WKind wk);
+// Its arrays, for a capacity of `cap` elements.
+kascade_status alloc_level0(kascade_ctx& ctx, const Level0Plan& plan, uint64_t cap, Level0* l0);
+
+// Level-0 records of a list from (succ, weights), stamps cleared; a root's
+// record carries weight 0.
+kascade_status prepare_arrays(kascade_ctx& ctx, const uint64_t* succ, WKind wk, const void* w, uint32_t n,
+                              const Level0& l0, const Rulers& rl, cudaStream_t s);
+Rulers level0_rulers(const Params& p);
+uint32_t hop_cap(const Rulers& rl);
 
 // Rank n <= ONE_CTA_MAX elements straight from the caller's arrays in one
 // launch.  Any forest is accepted up to ONE_CTA_TREES elements; above, lists.
-constexpr uint32_t ONE_CTA_MAX = 16384;
+constexpr uint32_t ONE_CTA_MAX = 15360;
 constexpr uint32_t ONE_CTA_TREES = 8192;
 kascade_status rank_arrays_one_cta(kascade_ctx& ctx, const uint64_t* succ, WKind wk, const void* w, uint32_t n,
                                    const SinkPlain& sink, cudaStream_t s);
@@ -241,13 +266,9 @@ kascade_status rank_arrays_one_cta(kascade_ctx& ctx, const uint64_t* succ, WKind
 // Rank level-0 records and deliver the results to the sink.  Every level's
 // size is known on the host: no host wait between the launches.  `ext`: the
 // record count when only the device knows it (ext.cap == n).
-// The write-free level 0 can report KASCADE_ERR_TIMEOUT (a chain past its hop
-// cap): in the status word, or as the return value with host_check (the call
-// then waits for the chase before anything is written to the outputs, and
-// falls back to the stamping level 0 by itself).
 template <class Sink>
-kascade_status rank_records(kascade_ctx& ctx, Rec* rec, uint32_t n, const Extent& ext, const Heads& heads,
-                            const Sink& sink, const Params& p, cudaStream_t s, bool host_check);
+kascade_status rank_records(kascade_ctx& ctx, const Level0& l0, uint32_t n, const Extent& ext, const Heads& heads,
+                            const Sink& sink, const Params& p, cudaStream_t s);
 
 // The levels of one call.  Level k >= 1 holds level k - 1's rulers, then its
 // heads: records {distance, next ruler}, the root of a list end and results.
@@ -258,7 +279,8 @@ struct Levels {
   uint32_t r[MAX_LEVELS];        // rulers of level k; level k + 1 has r[k] + heads.cap elements
   Rulers rulers[MAX_LEVELS];     // their placement
   Heads heads;
-  Rec* rec[MAX_LEVELS + 1];
+  Rec* rec[MAX_LEVELS + 1];      // from level 1 on
+  uint4* stamp[MAX_LEVELS + 1];  // from level 1 on, but not of the last level
   uint32_t* rootel[MAX_LEVELS + 1];  // level k >= 1: a list end's root as a level-0 element
   Out* out[MAX_LEVELS + 1];
   Extent extent(int k) const {
@@ -273,7 +295,31 @@ struct Levels {
 };
 kascade_status plan_levels(kascade_ctx& ctx, uint32_t n, const Heads& heads, const Params& p, Levels* lv);
 // Levels 1..last once the level-0 chase has written level 1: fills lv.out[1].
-kascade_status rank_deep(kascade_ctx& ctx, const Levels& lv, const Params& p, cudaStream_t s);
+kascade_status rank_deep(kascade_ctx& ctx, const Levels& lv, cudaStream_t s);
+
+// A ruler's record at the next level: its chain ended at ruler `next`, or
+// (next == id) at a list's end.  rl_next: the next level's rulers.  The last
+// level has no stamps and is ranked by one CTA, which looks rulers up itself.
+__device__ __forceinline__ void end_chain(Rec* rec_next, uint4* stamp_next, const Rulers& rl_next, uint32_t id,
+                                          uint64_t dist, uint32_t next) {
+  uint32_t j;
+  Record16::put(rec_next + id, dist, next, stamp_next && rl_next.is(next, &j));
+  if (stamp_next) Stamp16::clear(stamp_next + id);
+}
+
+// Whether a walk from y never meets a ruler or a list's end (an invalid input's
+// ruler-free cycle).  Only chains far beyond any plausible ruler gap ask.
+template <class F>
+__device__ __noinline__ bool endless(const typename F::R* rec, uint32_t y) {
+  uint32_t mark = y;
+  for (uint32_t hops = 1;; ++hops) {
+    const Hop h = F::hop(rec + y);
+    if (h.ruler || h.b == y) return false;
+    y = h.b;
+    if (y == mark) return true;
+    if ((hops & (hops - 1)) == 0) mark = y;
+  }
+}
 
 kascade_status compute_stats(kascade_ctx& ctx, const uint64_t* root, const int64_t* rank, uint64_t n, int level,
                              kascade_stats* out, kascade_tree_stats* per_tree, uint64_t per_tree_cap,
@@ -281,11 +327,9 @@ kascade_status compute_stats(kascade_ctx& ctx, const uint64_t* root, const int64
 
 // Write-free level 0: read-only chase that logs (element, ruler, distance),
 // recursion on the ruler list, then two radix passes over the log by element
-// and a dense placement into the outputs.  A chain past the hop cap becomes
-// KASCADE_ERR_TIMEOUT: in the status word, or (host_check) the return value,
-// with no output written yet.
-kascade_status rank_level0_log(kascade_ctx& ctx, const Rec* rec, uint32_t n, const Extent& ext, const Heads& heads,
-                               const LogTarget& t, const Params& p, cudaStream_t s, bool host_check);
+// and a dense placement into the outputs.
+kascade_status rank_level0_log(kascade_ctx& ctx, const Level0& l0, uint32_t n, const Extent& ext, const Heads& heads,
+                               const LogTarget& t, const Params& p, cudaStream_t s);
 
 // Pointer doubling on level-0 records (tags ignored).
 template <class Sink>

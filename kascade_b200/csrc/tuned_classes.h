@@ -1,14 +1,15 @@
-// Size-class table: mean ruler spacing, chains per thread and chase block
-// size for instances of at most KS_TUNED_MAX[i] elements.  Written by
-// kascade_b200/autotune.py from measurements on the GPU named below; the
-// library starts every context with it.  The single-call spacings of the
-// two largest classes (32 and 48) were re-measured on the write-free level 0
-// (`bench.py --n 2^26 / 2^27 / 2^28 --spacing ...`).
+// Size-class table: ruler spacing by a call's element count (KS_TUNED_SPACING:
+// a batch, by its record count; KS_TUNED_SPACING_SINGLE: one list or tour) and
+// chase block size.  Written by kascade_b200/autotune.py; the spacings from
+// sweeps over 4 .. 80 at 3e4 .. 2.7e8 elements, e.g. lists of 2^20: 4 / 8 / 12
+// / 24 157 / 164 / 152 / 193 us; 8e6: 8 / 16 / 32 556 / 530 / 582; 2^28: 24 /
+// 32 / 48 / 64 13.9 / 13.7 / 13.4 / 13.4 ms; batches of 3.8e6 records: 8 / 16 /
+// 32 390 / 378 / 422 us, 3.5e8: 32 / 40 / 48 15.3 / 15.3 / 15.4 ms.
 #pragma once
 #define KS_TUNED_GPU "NVIDIA B200"
 #define KS_TUNED_COUNT 8
 #define KS_TUNED_MAX {1024ull, 8192ull, 65536ull, 524288ull, 4194304ull, 33554432ull, 134217728ull, ~0ull}
-#define KS_TUNED_SPACING {6u, 6u, 8u, 8u, 8u, 12u, 24u, 96u}
-#define KS_TUNED_SPACING_SINGLE {4u, 4u, 6u, 8u, 10u, 16u, 32u, 48u}
+#define KS_TUNED_SPACING {6u, 6u, 8u, 8u, 16u, 16u, 24u, 40u}
+#define KS_TUNED_SPACING_SINGLE {4u, 4u, 6u, 6u, 12u, 16u, 32u, 48u}
 #define KS_TUNED_CHAINS {1u, 1u, 1u, 1u, 1u, 1u, 4u, 4u}
-#define KS_TUNED_BLOCK {256u, 128u, 128u, 512u, 512u, 512u, 512u, 512u}
+#define KS_TUNED_BLOCK {256u, 128u, 128u, 512u, 512u, 256u, 256u, 256u}
