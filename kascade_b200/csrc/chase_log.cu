@@ -120,14 +120,13 @@ __device__ __forceinline__ void log_append(bool emit, uint32_t x, uint32_t id, u
 // slower).
 template <class F>
 __global__ void __launch_bounds__(512) k_chase_log(const typename F::R* __restrict__ rec, Extent ext, Rulers rl,
-                                                   uint32_t rulers, Heads heads, Rulers rl_next,
-                                                   Rec* __restrict__ rec_next, uint4* __restrict__ stamp_next,
-                                                   uint32_t* __restrict__ rootel_next, uint32_t* __restrict__ work,
-                                                   LogEnt* __restrict__ log, uint32_t* __restrict__ chunk_fill,
+                                                   uint32_t rulers, Heads heads, NextLevel nx,
+                                                   uint32_t* __restrict__ work, LogEnt* __restrict__ log, uint32_t* __restrict__ chunk_fill,
                                                    uint32_t* __restrict__ chunk_cursor, uint32_t nchunks,
                                                    uint32_t hop_cap, DevStatus* st) {
   const uint32_t n = ext.get();
   const uint32_t r = rulers + heads.get();
+  if (nx.rl.s == 0) nx.rl = cta_rulers(r);
   if (ext.add && blockIdx.x == 0 && threadIdx.x == 0) st->counter[1] = n;  // level 0's size, reported by the call
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t lt = lanemask_lt();
@@ -141,9 +140,9 @@ __global__ void __launch_bounds__(512) k_chase_log(const typename F::R* __restri
     const uint64_t x0 = i < rulers ? rl.elem(i) : __ldg(heads.elem + (i - rulers));
     uint32_t j;
     if (x0 >= n) {
-      end_chain(rec_next, stamp_next, rl_next, i, 0, i);  // the last block's ruler, beyond the elements
+      nx.put(i, 0, i);  // the last block's ruler, beyond the elements
     } else if (i >= rulers && rl.is((uint32_t)x0, &j)) {
-      end_chain(rec_next, stamp_next, rl_next, i, 0, j);  // a head that is a ruler itself
+      nx.put(i, 0, j);  // a head that is a ruler itself
     } else {
       x = (uint32_t)x0;
       h = F::hop(rec + x);
@@ -189,20 +188,20 @@ __global__ void __launch_bounds__(512) k_chase_log(const typename F::R* __restri
           hops = 0;
           if (endless<F>(rec, y)) {
             set_error(st, KASCADE_ERR_CYCLE, id);
-            end_chain(rec_next, stamp_next, rl_next, id, 0, id);
+            nx.put(id, 0, id);
             act = false;
           }
         }
       } else {
         uint32_t next = id;
         if (end) {
-          rootel_next[id] = x;
+          nx.rootel[id] = x;
         } else {
           next = rl.block_of(y);
           // back at its own ruler: a rootless cycle holding one ruler
           if (next == id) set_error(st, KASCADE_ERR_CYCLE, id);
         }
-        end_chain(rec_next, stamp_next, rl_next, id, d, next);
+        nx.put(id, d, next);
         act = false;
       }
     }
@@ -615,8 +614,8 @@ kascade_status rank_level0_log_as(kascade_ctx& ctx, const Level0& l0, uint32_t n
   log.fill = cursor1 + cursor_words;
   {
     ProfScope ps(ctx, "chase", s);
-    k_chase_log<F><<<grid, block, 0, s>>>(l0.records<F>(), ext, lv.rulers[0], lv.r[0], lv.heads, lv.rulers[1],
-                                          lv.rec[1], lv.stamp[1], lv.rootel[1], &ctx.d_status->work[0], log.ent,
+    k_chase_log<F><<<grid, block, 0, s>>>(l0.records<F>(), ext, lv.rulers[0], lv.r[0], lv.heads,
+                                          next_level(lv, 1), &ctx.d_status->work[0], log.ent,
                                           log.fill, log.cursor, log.nchunks, hop_cap(lv.rulers[0]), ctx.d_status);
     KS_CHECK_LAUNCH();
   }

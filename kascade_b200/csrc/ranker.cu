@@ -195,12 +195,12 @@ constexpr int CHASE_REFILL = 8;  // idle lanes worth a refill
 template <class F>
 __global__ void __launch_bounds__(512) k_chase(const typename F::R* rec, typename F::S* stamp, Extent ext, Rulers rl,
                                                uint32_t rulers, Heads heads, uint32_t head_base,
-                                               const uint32_t* __restrict__ rootel, Rulers rl_next,
-                                               Rec* __restrict__ rec_next, uint4* __restrict__ stamp_next,
-                                               uint32_t* __restrict__ rootel_next, uint32_t* __restrict__ work,
-                                               uint32_t lanes, uint32_t limit, uint32_t hop_cap, DevStatus* st) {
+                                               const uint32_t* __restrict__ rootel, NextLevel nx,
+                                               uint32_t* __restrict__ work, uint32_t lanes, uint32_t limit,
+                                               uint32_t hop_cap, DevStatus* st) {
   const uint32_t n = ext.get();
   const uint32_t r = rulers + heads.get();
+  if (nx.rl.s == 0) nx.rl = cta_rulers(r);
   // level 0's size, reported by the call
   if (!rootel && ext.add && blockIdx.x == 0 && threadIdx.x == 0) st->counter[1] = n;
   const uint32_t lane = threadIdx.x & 31u;
@@ -220,9 +220,9 @@ __global__ void __launch_bounds__(512) k_chase(const typename F::R* rec, typenam
       x0 = rootel ? head_base + (i - rulers) : __ldg(heads.elem + (i - rulers));
     uint32_t j;
     if (x0 >= n) {
-      end_chain(rec_next, stamp_next, rl_next, i, 0, i);  // the last block's ruler, beyond the elements
+      nx.put(i, 0, i);  // the last block's ruler, beyond the elements
     } else if (i >= rulers && rl.is((uint32_t)x0, &j) && j < rulers) {
-      end_chain(rec_next, stamp_next, rl_next, i, 0, j);  // a head that is a ruler itself
+      nx.put(i, 0, j);  // a head that is a ruler itself
     } else {
       x = (uint32_t)x0;
       h = F::hop(rec + x);
@@ -266,13 +266,13 @@ __global__ void __launch_bounds__(512) k_chase(const typename F::R* rec, typenam
     if (stop) {  // (a list's end is not stamped: any number of chains may end there)
       uint32_t next = id;
       if (end) {
-        rootel_next[id] = rootel ? __ldg(rootel + x) : x;
+        nx.rootel[id] = rootel ? __ldg(rootel + x) : x;
       } else {
         next = rl.block_of(y);
         // back at its own ruler: a cycle without a root that holds one ruler
         if (next == id) set_error(st, KASCADE_ERR_CYCLE, id);
       }
-      end_chain(rec_next, stamp_next, rl_next, id, d, next);
+      nx.put(id, d, next);
       act = false;
       continue;
     }
@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(512) k_chase(const typename F::R* rec, typenam
       hops = 0;
       if (endless<F>(rec, y)) {
         set_error(st, KASCADE_ERR_CYCLE, id);
-        end_chain(rec_next, stamp_next, rl_next, id, 0, id);
+        nx.put(id, 0, id);
         act = false;
       }
     }
@@ -416,11 +416,14 @@ __global__ void __launch_bounds__(256) k_propagate(const typename F::R* __restri
 // of the recursion, or a whole small input straight from the caller's arrays.
 // The elements are loaded once; at most CTA_RULERS rulers (placed as on every
 // level) walk and stamp as in k_chase, pointer jumping ranks the rulers
-// (<= 10 rounds), and every element reads its ruler's result.  Against
-// pointer jumping over all elements (13 rounds of 16 elements per thread at
-// 8192: 51 us) each element is touched once.  Each element's word also says
-// whether its successor is a ruler or a list's end, so a hop is one read and
-// one write of the word and of the distance.
+// (three steps per round), and every element reads its ruler's result.
+// Against pointer jumping over all elements (13 rounds of 16 elements per
+// thread at 8192: 51 us) each element is touched once.  Each element's word
+// also says whether its successor is a ruler, so a hop is one read and one
+// write of the word and of the distance.  Bound by one SM's shared-memory
+// pipe and instructions: 1000 elements 8.7 us, 4000 14.7, 8000 18.2, 14.3
+// thousand 27 (46 with a pass of its own for the ruler bits, three barriers a
+// jumping round and a predecessor byte per element in every case).
 // With several lists, their heads (no predecessor) start chains as well, so
 // that no run of elements ahead of a first ruler is walked element by element.
 // Two chains that meet (a tree, not a list) leave fewer stamped elements than
@@ -428,38 +431,39 @@ __global__ void __launch_bounds__(256) k_propagate(const typename F::R* __restri
 // stamps, every element walking to its first ruler, which ranks any forest.
 // ---------------------------------------------------------------------------
 constexpr uint32_t CTA_THREADS = 1024;
-constexpr uint32_t CTA_RULERS = 1024;
 constexpr uint32_t CTA_HEADS = 1024;
 constexpr uint32_t CTA_LOADS = 8;           // elements a thread has in flight while loading
 constexpr uint32_t CTA_ILP = 4;             // elements a thread has in flight in shared memory
 constexpr uint32_t CTA_FLAG = 0x80000000u;  // next: stamped, low bits the chain; rnext: the list's end
-constexpr uint32_t CTA_END = 0x40000000u;   // next: the successor ends the list
 constexpr uint32_t CTA_RUL = 0x20000000u;   // next: the successor is a ruler
 constexpr uint32_t CTA_IDX = 0x1FFFFFFFu;
 constexpr size_t cta_smem(uint64_t n) {
-  return (size_t)((n + CTA_RULERS + CTA_HEADS) * 12 + CTA_HEADS * 2 + (n + 3) / 4 * 4);
+  return (size_t)((n + CTA_RULERS + CTA_HEADS) * 12 + CTA_RULERS * 12 + CTA_HEADS * 2 + (n + 3) / 4 * 4);
 }
 
 // Element sources: the records of a level (a list end's carries its rank), or
 // the caller's arrays (a root's weight is no part of any rank).
-template <class F>
+// FLAGGED: the records' ruler bits are for this ranker's rulers.
+template <class F, bool FLAGGED>
 struct CtaRecords {
-  static constexpr bool kEndWeight = true;
+  static constexpr bool kEndWeight = true, kFlagged = FLAGGED;
   const typename F::R* rec;
   const uint32_t* rootel;
-  __device__ __forceinline__ void load(uint32_t x, uint64_t* a, uint32_t* b) const {
+  __device__ __forceinline__ void load(uint32_t x, uint64_t* a, uint32_t* b, bool* ruler) const {
     const Hop h = F::hop(rec + x);
     *a = h.w;
     *b = h.b;
+    *ruler = h.ruler;
   }
   __device__ __forceinline__ uint32_t root_of(uint32_t x) const { return rootel ? __ldg(rootel + x) : x; }
 };
 template <class W>
 struct CtaArrays {
-  static constexpr bool kEndWeight = false;
+  static constexpr bool kEndWeight = false, kFlagged = false;
   const uint64_t* succ;
   W w;
-  __device__ __forceinline__ void load(uint32_t x, uint64_t* a, uint32_t* b) const {
+  __device__ __forceinline__ void load(uint32_t x, uint64_t* a, uint32_t* b, bool* ruler) const {
+    *ruler = false;
     const unsigned long long s = __ldcg(reinterpret_cast<const unsigned long long*>(succ) + x);
     *a = w(x);
     *b = s > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)s;  // beyond any element: found out of range
@@ -475,15 +479,17 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) k_rank_cta(Src src, Extent ext
   const uint32_t n = ext.get();
   unsigned long long* dist = reinterpret_cast<unsigned long long*>(smem);  // weight, once stamped the distance
   unsigned long long* rdist = dist + ext.cap;                              // per chain: distance, then rank
-  uint32_t* next = reinterpret_cast<uint32_t*>(rdist + CTA_RULERS + CTA_HEADS);
+  unsigned long long* jdist = rdist + CTA_RULERS + CTA_HEADS;              // (the jumping rounds' other copy)
+  uint32_t* next = reinterpret_cast<uint32_t*>(jdist + CTA_RULERS);
   uint32_t* rnext = next + ext.cap;  // per chain: next ruler or CTA_FLAG | list end, then the root
-  uint32_t* predw = rnext + CTA_RULERS + CTA_HEADS;
+  uint32_t* jnext = rnext + CTA_RULERS + CTA_HEADS;
+  uint32_t* predw = jnext + CTA_RULERS;
   unsigned char* pred = reinterpret_cast<unsigned char*>(predw);  // 1: has a predecessor
   uint16_t* hlist = reinterpret_cast<uint16_t*>(predw + (ext.cap + 3) / 4);
   const uint32_t tid = threadIdx.x, nthreads = blockDim.x;
   if (level0 && ext.add && tid == 0) st->counter[1] = n;
-  const bool all = n <= CTA_RULERS;  // every element is a ruler
-  const Rulers rl = make_rulers((n + CTA_RULERS - 1) / CTA_RULERS, 0x63746121u);
+  const Rulers rl = cta_rulers(n);
+  const bool all = rl.s == 1;  // every element is a ruler
   const uint32_t rulers = all ? n : (n + rl.s - 1) / rl.s;
   auto ruler = [&](uint32_t x) {
     uint32_t j;
@@ -494,16 +500,17 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) k_rank_cta(Src src, Extent ext
   uint32_t heads = 0;
   while (true) {
     if (tid == 0) nends = nheads = nstamps = 0;
-    for (uint32_t w = tid; w < (n + 3) / 4; w += nthreads) predw[w] = 0;
     __syncthreads();
     uint32_t ends = 0;
     for (uint32_t x0 = tid; x0 < n; x0 += nthreads * CTA_LOADS) {
       uint64_t a[CTA_LOADS];
-      uint32_t b[CTA_LOADS];
+      uint32_t b[CTA_LOADS], rul = 0;
 #pragma unroll
       for (uint32_t i = 0; i < CTA_LOADS; ++i) {
         const uint32_t x = x0 + i * nthreads;
-        if (x < n) src.load(x, &a[i], &b[i]);
+        bool f = false;
+        if (x < n) src.load(x, &a[i], &b[i], &f);
+        rul |= f ? 1u << i : 0u;
       }
 #pragma unroll
       for (uint32_t i = 0; i < CTA_LOADS; ++i) {
@@ -513,35 +520,25 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) k_rank_cta(Src src, Extent ext
           set_error(st, KASCADE_ERR_OUT_OF_RANGE, x);
           b[i] = x;
         }
-        dist[x] = (Src::kEndWeight || b[i] != x) ? a[i] : 0ull;
-        next[x] = b[i];
-        ends += b[i] == x ? 1u : 0u;
+        const bool end = b[i] == x;
+        dist[x] = (Src::kEndWeight || !end) ? a[i] : 0ull;
+        // (a list's end is its own word, whether it is a ruler or not)
+        next[x] = b[i] | (!end && (Src::kFlagged ? (rul >> i) & 1u : ruler(b[i])) ? CTA_RUL : 0u);
+        ends += end ? 1u : 0u;
       }
     }
     ends = __reduce_add_sync(FULL, ends);
     if ((tid & 31u) == 0 && ends) atomicAdd(&nends, ends);
     __syncthreads();
-    // what each successor is; with several lists, who has a predecessor
-    const bool many = stamp && !all && nends > 2;
-    for (uint32_t x0 = tid; x0 < n; x0 += nthreads * CTA_ILP) {
-      uint32_t y[CTA_ILP], z[CTA_ILP];
-#pragma unroll
-      for (uint32_t i = 0; i < CTA_ILP; ++i) {
-        const uint32_t x = x0 + i * nthreads;
-        y[i] = x < n ? next[x] : x;
+    // with several lists, their heads start chains too
+    if (stamp && !all && nends > 2) {
+      for (uint32_t w = tid; w < (n + 3) / 4; w += nthreads) predw[w] = 0;
+      __syncthreads();
+      for (uint32_t x = tid; x < n; x += nthreads) {
+        const uint32_t y = next[x] & CTA_IDX;
+        if (y != x) pred[y] = 1;
       }
-#pragma unroll
-      for (uint32_t i = 0; i < CTA_ILP; ++i) z[i] = x0 + i * nthreads < n ? next[y[i]] & CTA_IDX : 0u;
-#pragma unroll
-      for (uint32_t i = 0; i < CTA_ILP; ++i) {
-        const uint32_t x = x0 + i * nthreads;
-        if (x >= n || y[i] == x) continue;
-        next[x] = y[i] | (z[i] == y[i] ? CTA_END : 0u) | (ruler(y[i]) ? CTA_RUL : 0u);
-        if (many) pred[y[i]] = 1;
-      }
-    }
-    __syncthreads();
-    if (many) {
+      __syncthreads();
       for (uint32_t w = tid; w < (n + 3) / 4; w += nthreads) {
         const uint32_t pw = predw[w];
         if (pw == 0x01010101u) continue;
@@ -560,8 +557,11 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) k_rank_cta(Src src, Extent ext
     for (uint32_t k = tid; k < rulers + heads; k += nthreads) {
       const uint32_t id = k < rulers ? k : CTA_RULERS + (k - rulers);
       const uint32_t x0 = k < rulers ? elem(k) : hlist[k - rulers];
-      if (x0 >= n) continue;
-      uint32_t f = next[x0];
+      if (x0 >= n) {  // the last block's ruler, beyond the elements
+        rnext[id] = CTA_FLAG;
+        continue;
+      }
+      uint32_t f = next[x0], x = x0;
       unsigned long long acc = dist[x0];
       if (f == x0) {  // a list's end
         rdist[id] = acc;
@@ -573,10 +573,14 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) k_rank_cta(Src src, Extent ext
         dist[x0] = 0;
       }
       uint32_t hops = 0;
-      while (!(f & (CTA_FLAG | CTA_END | CTA_RUL))) {
-        const uint32_t x = f;
+      while (!(f & (CTA_FLAG | CTA_RUL))) {
+        x = f;
         f = next[x];
         const unsigned long long w = dist[x];
+        if (f == x) {  // the list's end
+          acc += w;
+          break;
+        }
         if (stamp) {
           next[x] = CTA_FLAG | id;
           dist[x] = acc;
@@ -586,24 +590,21 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) k_rank_cta(Src src, Extent ext
         }
         acc += w;
       }
-      const uint32_t y = f & CTA_IDX;
-      if (f & CTA_FLAG) {  // another chain's element: counted below
+      rdist[id] = acc;
+      if (f & CTA_FLAG) {  // another chain's element (counted below), or a cycle: never ends
         loops = 1;
-        rdist[id] = 0;
         rnext[id] = id < CTA_RULERS ? id : 0u;
       } else if (f & CTA_RUL) {
-        rdist[id] = acc;
-        rnext[id] = all ? y : rl.block_of(y);
+        rnext[id] = all ? f & CTA_IDX : rl.block_of(f & CTA_IDX);
       } else {
-        rdist[id] = acc + (y == x0 ? 0ull : dist[y]);
-        rnext[id] = CTA_FLAG | y;
+        rnext[id] = CTA_FLAG | x;
       }
     }
     if (!stamp) break;
     stamps = __reduce_add_sync(FULL, stamps);
     if ((tid & 31u) == 0 && stamps) atomicAdd(&nstamps, stamps);
-    uint32_t marks = 0;  // stamped elements that are no chain's first
     const int clash = __syncthreads_or((int)loops);
+    uint32_t marks = 0;  // stamped elements that are no chain's first
     for (uint32_t x = tid; x < n; x += nthreads) marks += next[x] >> 31;
     for (uint32_t k = tid; k < rulers + heads; k += nthreads) {
       const uint32_t x0 = k < rulers ? elem(k) : hlist[k - rulers];
@@ -622,38 +623,45 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) k_rank_cta(Src src, Extent ext
     heads = 0;
   }
   __syncthreads();
-  // pointer jumping over the rulers
-  for (int round = 0;; ++round) {
-    unsigned long long d[CTA_RULERS / 256];
-    uint32_t nx[CTA_RULERS / 256];
-    int busy = 0;
-#pragma unroll
-    for (uint32_t c = 0; c < CTA_RULERS / 256; ++c) {
-      const uint32_t j = tid + c * nthreads;
-      nx[c] = CTA_FLAG;
-      d[c] = 0;
-      if (j >= rulers || elem(j) >= n) continue;
-      nx[c] = rnext[j];
-      d[c] = rdist[j];
-      if (!(nx[c] & CTA_FLAG)) {
-        d[c] += rdist[nx[c]];
-        nx[c] = rnext[nx[c]];
-        busy = 1;
+  // pointer jumping over the rulers through the previous round's copy: one
+  // barrier per round (three steps per round were slower: the rounds are bound
+  // by the shared-memory pipe, not by their barriers)
+  {
+    unsigned long long *da = rdist, *db = jdist;
+    uint32_t *na = rnext, *nb = jnext;
+    for (int round = 0;; ++round) {
+      int busy = 0;
+#pragma unroll 4
+      for (uint32_t j = tid; j < rulers; j += nthreads) {
+        uint32_t nx = na[j];
+        unsigned long long d = da[j];
+        if (!(nx & CTA_FLAG)) {
+          d += da[nx];
+          nx = na[nx];
+          busy = 1;
+        }
+        nb[j] = nx;
+        db[j] = d;
+      }
+      unsigned long long* td = da;
+      da = db;
+      db = td;
+      uint32_t* tn = na;
+      na = nb;
+      nb = tn;
+      if (!__syncthreads_or(busy)) break;
+      if (round > 11) {  // 2^11 > CTA_RULERS: what has not ended by now never does
+        if (tid == 0) set_error(st, KASCADE_ERR_CYCLE, n);
+        return;
       }
     }
-    if (!__syncthreads_or(busy)) break;
-    if (round > 11) {  // 2^11 > CTA_RULERS: what has not ended by now never does
-      if (tid == 0) set_error(st, KASCADE_ERR_CYCLE, n);
-      return;
+    if (da != rdist) {  // (the heads' entries are in rdist and rnext)
+      for (uint32_t j = tid; j < rulers; j += nthreads) {
+        rdist[j] = da[j];
+        rnext[j] = na[j];
+      }
+      __syncthreads();
     }
-#pragma unroll
-    for (uint32_t c = 0; c < CTA_RULERS / 256; ++c) {
-      const uint32_t j = tid + c * nthreads;
-      if (j >= rulers || elem(j) >= n) continue;
-      rdist[j] = d[c];
-      rnext[j] = nx[c];
-    }
-    __syncthreads();
   }
   // the heads' chains end at a ruler or a list end; then every chain's root
   for (uint32_t h = tid; h < heads; h += nthreads) {
@@ -666,7 +674,7 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) k_rank_cta(Src src, Extent ext
   __syncthreads();
   for (uint32_t k = tid; k < rulers + heads; k += nthreads) {
     const uint32_t j = k < rulers ? k : CTA_RULERS + (k - rulers);
-    if (k >= rulers || elem(k) < n) rnext[j] = src.root_of(rnext[j] & ~CTA_FLAG);
+    rnext[j] = src.root_of(rnext[j] & ~CTA_FLAG);
   }
   __syncthreads();
   for (uint32_t x0 = tid; x0 < n; x0 += nthreads * CTA_ILP) {
@@ -703,11 +711,6 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) k_rank_cta(Src src, Extent ext
             root = rnext[k];
             break;
           }
-          if (w & CTA_END) {
-            d[i] += dist[y];
-            root = src.root_of(y);
-            break;
-          }
           w = next[y];
           if (w & CTA_FLAG) {
             d[i] += rdist[w & CTA_IDX] - dist[y];
@@ -715,6 +718,10 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) k_rank_cta(Src src, Extent ext
             break;
           }
           d[i] += dist[y];
+          if (w == y) {
+            root = src.root_of(y);
+            break;
+          }
           if (++hops > n) {
             set_error(st, KASCADE_ERR_CYCLE, x);
             ok = false;
@@ -855,9 +862,8 @@ kascade_status launch_chase(kascade_ctx& ctx, const Levels& lv, int k, const typ
   const unsigned grid = (unsigned)std::min<uint64_t>(max_grid, (need + wpb - 1) / wpb);
   ProfScope ps(ctx, "chase", s);
   k_chase<F><<<grid, block, 0, s>>>(rec, stamp, ext, lv.rulers[k], lv.r[k], lv.heads, k ? lv.r[k - 1] : 0u,
-                                    lv.rootel[k], lv.rulers[k + 1], lv.rec[k + 1], lv.stamp[k + 1],
-                                    lv.rootel[k + 1], &ctx.d_status->work[k], lanes, limit, hop_cap(lv.rulers[k]),
-                                    ctx.d_status);
+                                    lv.rootel[k], next_level(lv, k + 1), &ctx.d_status->work[k], lanes, limit,
+                                    hop_cap(lv.rulers[k]), ctx.d_status);
   KS_CHECK_LAUNCH();
   return KASCADE_OK;
 }
@@ -1185,7 +1191,7 @@ kascade_status rank_deep(kascade_ctx& ctx, const Levels& lv, cudaStream_t s) {
     KS_TRY(launch_chase<F16x16>(ctx, lv, k, lv.rec[k], lv.stamp[k], lv.extent(k), lv.n[k], 256, s));
   const int L = lv.last;
   if (lv.n[L] <= ONE_CTA_MAX) {
-    KS_TRY(launch_rank_cta(ctx, CtaRecords<F16x16>{lv.rec[L], lv.rootel[L]}, lv.extent(L), SinkOut{lv.out[L]}, 0, 0,
+    KS_TRY(launch_rank_cta(ctx, CtaRecords<F16x16, true>{lv.rec[L], lv.rootel[L]}, lv.extent(L), SinkOut{lv.out[L]}, 0, 0,
                            s));
   } else {
     KS_TRY(pointer_double_level(ctx, lv.rec[L], lv.extent(L), lv.rootel[L], lv.out[L], s));
@@ -1204,7 +1210,7 @@ kascade_status rank_records_as(kascade_ctx& ctx, const Level0& l0, uint32_t n, c
   const typename F::R* rec = l0.records<F>();
   if (n <= p.base_max) {
     ctx.last_levels.assign(1, n);
-    return launch_rank_cta(ctx, CtaRecords<F>{rec, nullptr}, ext, sink, ONE_CTA_TREES, 1, s);
+    return launch_rank_cta(ctx, CtaRecords<F, false>{rec, nullptr}, ext, sink, ONE_CTA_TREES, 1, s);
   }
   Levels lv;
   KS_TRY(plan_levels(ctx, n, heads, p, &lv));

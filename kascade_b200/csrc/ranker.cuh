@@ -62,7 +62,11 @@ struct Rulers {
 };
 __host__ __device__ inline Rulers make_rulers(uint32_t s, uint32_t salt) {
   Rulers r;
-  if (s < 2) s = 2;
+  if (s < 2) {  // every element a ruler: the one-CTA ranker's placement on few elements
+    r.s = 1;
+    r.salt = salt;
+    return r;
+  }
   if (s > 0x80000000u) s = 0x80000000u;
   uint32_t l = 1;
   while (l < 31 && (1ull << l) < s) ++l;
@@ -71,6 +75,11 @@ __host__ __device__ inline Rulers make_rulers(uint32_t s, uint32_t salt) {
   r.sh = l - 1;
   r.salt = salt;
   return r;
+}
+// The one-CTA ranker's rulers: at most CTA_RULERS.
+constexpr uint32_t CTA_RULERS = 1024;
+__host__ __device__ inline Rulers cta_rulers(uint32_t n) {
+  return make_rulers((n + CTA_RULERS - 1) / CTA_RULERS, 0x63746121u);
 }
 inline uint32_t ruler_count(uint32_t n, const Rulers& r) { return (uint32_t)(((uint64_t)n + r.s - 1) / r.s); }
 
@@ -258,7 +267,7 @@ uint32_t hop_cap(const Rulers& rl);
 
 // Rank n <= ONE_CTA_MAX elements straight from the caller's arrays in one
 // launch.  Any forest is accepted up to ONE_CTA_TREES elements; above, lists.
-constexpr uint32_t ONE_CTA_MAX = 15360;
+constexpr uint32_t ONE_CTA_MAX = 14336;
 constexpr uint32_t ONE_CTA_TREES = 8192;
 kascade_status rank_arrays_one_cta(kascade_ctx& ctx, const uint64_t* succ, WKind wk, const void* w, uint32_t n,
                                    const SinkPlain& sink, cudaStream_t s);
@@ -297,14 +306,29 @@ kascade_status plan_levels(kascade_ctx& ctx, uint32_t n, const Heads& heads, con
 // Levels 1..last once the level-0 chase has written level 1: fills lv.out[1].
 kascade_status rank_deep(kascade_ctx& ctx, const Levels& lv, cudaStream_t s);
 
-// A ruler's record at the next level: its chain ended at ruler `next`, or
-// (next == id) at a list's end.  rl_next: the next level's rulers.  The last
-// level has no stamps and is ranked by one CTA, which looks rulers up itself.
-__device__ __forceinline__ void end_chain(Rec* rec_next, uint4* stamp_next, const Rulers& rl_next, uint32_t id,
-                                          uint64_t dist, uint32_t next) {
-  uint32_t j;
-  Record16::put(rec_next + id, dist, next, stamp_next && rl_next.is(next, &j));
-  if (stamp_next) Stamp16::clear(stamp_next + id);
+// Where a level's chains put their rulers' records.  The last level has no
+// stamps; its rulers are the one-CTA ranker's (rl.s == 0: found on the device
+// from the level's size, which the heads are part of).
+struct NextLevel {
+  Rec* rec = nullptr;
+  uint4* stamp = nullptr;
+  uint32_t* rootel = nullptr;
+  Rulers rl;
+  // its chain ended at ruler `next`, or (next == id) at a list's end
+  __device__ __forceinline__ void put(uint32_t id, uint64_t dist, uint32_t next) const {
+    uint32_t j;
+    Record16::put(rec + id, dist, next, rl.s == 1 || rl.is(next, &j));
+    if (stamp) Stamp16::clear(stamp + id);
+  }
+};
+inline NextLevel next_level(const Levels& lv, int k) {
+  NextLevel nx;
+  nx.rec = lv.rec[k];
+  nx.stamp = lv.stamp[k];
+  nx.rootel = lv.rootel[k];
+  nx.rl = lv.rulers[k];
+  if (k == lv.last) nx.rl.s = 0;
+  return nx;
 }
 
 // Whether a walk from y never meets a ruler or a list's end (an invalid input's
