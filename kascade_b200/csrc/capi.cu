@@ -76,19 +76,14 @@ kascade_status rank_list_generic(kascade_ctx& ctx, const uint64_t* succ, WKind w
   const SinkPlain sink{root_out, rank_out, keep_roots};
   Level0 l0;
   if (p.algorithm == KASCADE_ALGO_SPARSE_RULING_SET) {
-    if (n <= p.base_max) return rank_arrays_one_cta(ctx, succ, wk, w, (uint32_t)n, sink, s);
+    if (n <= p.base_max) return rank_arrays_one_cta(ctx, succ, wk, w, (uint32_t)n, sink, CTA_SMALL_TREES, s);
     KS_TRY(alloc_level0(ctx, plan_level0(p, n, wk), n, &l0));
     KS_TRY(prepare_arrays(ctx, succ, wk, w, (uint32_t)n, l0, level0_rulers(p), s));
     Extent ext;
     ext.cap = (uint32_t)n;
     return rank_records(ctx, l0, (uint32_t)n, ext, Heads{}, sink, p, s);
   }
-  Rec* rec = alloc<Rec>(ctx, n);
-  if (!rec) return KASCADE_ERR_OOM;
-  l0.rec = rec;
-  KS_TRY(prepare_arrays(ctx, succ, wk, w, (uint32_t)n, l0, level0_rulers(p), s));
-  ctx.last_levels.assign(1, n);
-  return pointer_double_records(ctx, rec, (uint32_t)n, nullptr, sink, s);
+  return rank_forest_weighted(ctx, succ, wk, w, (uint32_t)n, sink, p, s);
 }
 
 kascade_status validate_list(kascade_ctx& ctx, const uint64_t* succ, uint64_t n, const kascade_opts* o,
@@ -427,16 +422,9 @@ KASCADE_API kascade_status kascade_rank_via_euler_tour(kascade_ctx* c, const kas
   Params p = make_params(*c, opts, 2 * n);
   p.algorithm = KASCADE_ALGO_SPARSE_RULING_SET;
   kascade_status st = KASCADE_OK;
-  if (n) {
-    // the parent array is read by the sort before any output is written, but
-    // the tour build reads it no more; results go straight to the arrays
-    uint64_t* parent_copy = alloc<uint64_t>(*c, n);
-    if (!parent_copy) st = KASCADE_ERR_OOM;
-    if (st == KASCADE_OK)
-      st = cuda_status(cudaMemcpyAsync(parent_copy, succ_array, n * 8, cudaMemcpyDeviceToDevice, s));
-    if (st == KASCADE_OK)
-      st = root_forest_impl(*c, parent_copy, (uint32_t)n, succ_array, (uint64_t*)rank_array, 1, p, s);
-  }
+  // the outputs are written after the last read of the parents (they are read
+  // once, when the records are built)
+  if (n) st = root_forest_impl(*c, succ_array, (uint32_t)n, succ_array, (uint64_t*)rank_array, 1, p, s);
   return end_call(c, s, st, opts);
 }
 

@@ -127,7 +127,6 @@ __global__ void __launch_bounds__(512) k_chase_log(const typename F::R* __restri
   const uint32_t n = ext.get();
   const uint32_t r = rulers + heads.get();
   if (nx.rl.s == 0) nx.rl = cta_rulers(r);
-  if (ext.add && blockIdx.x == 0 && threadIdx.x == 0) st->counter[1] = n;  // level 0's size, reported by the call
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t lt = lanemask_lt();
   const uint32_t first = gridDim.x * blockDim.x;  // ids from here on are handed out by the counter
@@ -386,7 +385,7 @@ __global__ void __launch_bounds__(FIN_THREADS, 2) k_place(const LogEnt* __restri
                                                             uint32_t* __restrict__ ucount, uint32_t ucap,
                                                             const uint64_t* __restrict__ seg_off,
                                                             const uint32_t* __restrict__ hint, uint32_t nseg,
-                                                            const uint32_t* __restrict__ plus_one, int tour,
+                                                            const uint32_t* __restrict__ plus_one,
                                                             const uint32_t* __restrict__ seg_tour, int keep_roots,
                                                             DevStatus* st) {
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -430,7 +429,7 @@ __global__ void __launch_bounds__(FIN_THREADS, 2) k_place(const LogEnt* __restri
     // and the next instance's; a thread's elements only move forward
     uint32_t jseg = 0;
     unsigned long long cur_off = 0, next_off = ~0ull;
-    bool depths = tour != 0;
+    bool depths = false;
     if (seg_off) {
       const uint32_t x0 = lo + threadIdx.x;
       jseg = __ldg(hint + (x0 >> 12));
@@ -493,14 +492,14 @@ __global__ void __launch_bounds__(256) k_walk_unreached(const typename F::R* __r
                                                         uint32_t limit, uint64_t* root_out, uint64_t* rank_out,
                                                         const uint64_t* __restrict__ seg_off,
                                                         const uint32_t* __restrict__ hint, uint32_t nseg,
-                                                        const uint32_t* __restrict__ plus_one, int tour,
+                                                        const uint32_t* __restrict__ plus_one,
                                                         const uint32_t* __restrict__ seg_tour, int keep_roots,
                                                         DevStatus* st) {
   const uint32_t cnt = min(*ucount, ucap);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
     const uint32_t u = ulist[i];
     uint64_t off = 0;
-    bool depths = tour != 0;
+    bool depths = false;
     if (seg_off) {
       uint32_t j = __ldg(hint + (u >> 12));
       while (j + 1 < nseg && __ldg(seg_off + j + 1) <= u) ++j;
@@ -667,13 +666,13 @@ kascade_status rank_level0_log_as(kascade_ctx& ctx, const Level0& l0, uint32_t n
     const size_t smem = SUB * (sizeof(unsigned long long) + sizeof(uint32_t));
     k_place<<<(unsigned)std::max<uint64_t>(1, std::min<uint64_t>(items, (uint64_t)ctx.usable_sms() * 2)),
                 FIN_THREADS, smem, s>>>(part2, cursor2, nb, limit, t.root, t.rank, ulist, ucount, ucap, t.seg_off,
-                                        t.hint, t.nseg, t.plus_one, t.tour, t.seg_tour, t.keep_roots, ctx.d_status);
+                                        t.hint, t.nseg, t.plus_one, t.seg_tour, t.keep_roots, ctx.d_status);
     KS_CHECK_LAUNCH();
   }
   {
     ProfScope ps(ctx, "heads", s);
     k_walk_unreached<F><<<ctx.usable_sms() * 4, 256, 0, s>>>(l0.records<F>(), ulist, ucount, ucap, n, limit, t.root,
-                                                             t.rank, t.seg_off, t.hint, t.nseg, t.plus_one, t.tour,
+                                                             t.rank, t.seg_off, t.hint, t.nseg, t.plus_one,
                                                              t.seg_tour, t.keep_roots, ctx.d_status);
     KS_CHECK_LAUNCH();
   }

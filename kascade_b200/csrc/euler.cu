@@ -347,20 +347,12 @@ kascade_status sort_children(kascade_ctx& ctx, const uint64_t* parent, uint32_t 
   return KASCADE_OK;
 }
 
-// Leaf contraction of a single forest's tour.  A leaf's down edge is
-// followed by its own up edge (weights -1 and +1), so the two become one
-// element of weight 0 at the leaf's slot v: every other rank is unchanged
-// and the leaf's depth is that element's rank + 1 (leaf_bits tells the
-// output step).  Only non-root vertices with children keep a down edge, at
-// the compacted slot n + (their number among those vertices): ibits marks
-// them (one word per 32 vertices) and ipre counts them before each word, so
-// the element a parent or a sibling continues into is found with one read of
-// these L2-resident tables.  heads lists up to HEAD_CAP tour heads: the
-// vertices (list heads of their roots) whose element a tree's tour starts with.
+// The vertices with a down edge (ibits: not a root, not a leaf), and up to
+// HEAD_CAP tour heads: the vertices (list heads of their roots) whose element
+// a tree's tour starts with.
 __global__ void __launch_bounds__(256) k_internal_words(const uint32_t* __restrict__ p32,
                                                         const uint32_t* __restrict__ fc, uint32_t n,
-                                                        uint32_t* __restrict__ ibits,
-                                                        uint32_t* __restrict__ icount, uint32_t* __restrict__ heads,
+                                                        uint32_t* __restrict__ ibits, uint32_t* __restrict__ heads,
                                                         uint32_t* __restrict__ nheads) {
   const uint32_t lane = threadIdx.x & 31u;
   const uint64_t tile_sz = (uint64_t)blockDim.x * TB_ITEMS;
@@ -377,10 +369,7 @@ __global__ void __launch_bounds__(256) k_internal_words(const uint32_t* __restri
     for (int i = 0; i < TB_ITEMS; ++i) {
       const uint64_t v = tile + (uint64_t)i * blockDim.x + threadIdx.x;
       const uint32_t bits = __ballot_sync(0xffffffffu, v < n && pv[i] != (uint32_t)v && fv[i] != NO_CHILD);
-      if (lane == 0 && v < n) {
-        ibits[v >> 5] = bits;
-        icount[v >> 5] = (uint32_t)__popc(bits);
-      }
+      if (lane == 0 && v < n) ibits[v >> 5] = bits;
       // a root's list head enters its tree first: the head of that tree's tour
       const bool head = v < n && pv[i] == (uint32_t)v && fv[i] != NO_CHILD;
       const uint32_t hm = __ballot_sync(0xffffffffu, head);
@@ -390,108 +379,6 @@ __global__ void __launch_bounds__(256) k_internal_words(const uint32_t* __restri
         e = __shfl_sync(0xffffffffu, e, 0) + __popc(hm & lanemask_lt());
         if (head && e < HEAD_CAP) heads[e] = fv[i];
       }
-    }
-  }
-}
-
-// (bits, down edges before the word) of every word of 32 vertices
-__global__ void __launch_bounds__(256) k_internal_pack(const uint32_t* __restrict__ ibits,
-                                                       const uint32_t* __restrict__ ipre, uint32_t words,
-                                                       uint2* __restrict__ iw) {
-  for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < words; w += gridDim.x * blockDim.x)
-    iw[w] = make_uint2(ibits[w], ipre[w]);
-}
-
-struct Entries {
-  const uint2* iw;  // per word of 32 vertices: (down-edge bits, down edges before it)
-  uint32_t n;
-  __device__ __forceinline__ uint2 word(uint32_t c) const { return __ldg(iw + (c >> 5)); }
-  // the element a walk enters vertex c by, from c's word: its down edge, or
-  // its merged slot
-  __device__ __forceinline__ uint32_t of(uint32_t c, uint2 w) const {
-    const uint32_t below = w.x & ((1u << (c & 31)) - 1u);
-    return ((w.x >> (c & 31)) & 1u) ? n + w.y + (uint32_t)__popc(below) : c;
-  }
-  __device__ __forceinline__ uint32_t down_slot(uint32_t v, uint2 w) const {  // v has a down edge
-    return n + w.y + (uint32_t)__popc(w.x & ((1u << (v & 31)) - 1u));
-  }
-};
-
-// One tile of TB_ITEMS vertices per thread in two rounds of independent loads
-// (the vertex's own words; the table words of its sibling, its first child
-// and itself), so a tile waits for two memory latencies rather than a chain
-// of them per vertex.
-template <class F>
-__global__ void __launch_bounds__(256) k_tour_leaves(const uint32_t* __restrict__ p32, uint32_t n,
-                                                     const uint32_t* __restrict__ fc,
-                                                     const uint32_t* __restrict__ nsib, Entries ent,
-                                                     Rulers rl, typename F::R* __restrict__ rec,
-                                                     typename F::S* __restrict__ stamp,
-                                                     uint32_t* __restrict__ leaf_bits,
-                                                     uint32_t* __restrict__ heads,
-                                                     const uint32_t* __restrict__ nheads) {
-  const uint32_t lane = threadIdx.x & 31u;
-  // the tours' first vertices become the elements they are entered by
-  for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < min(*nheads, HEAD_CAP); e += gridDim.x * blockDim.x) {
-    const uint32_t c = heads[e];
-    heads[e] = ent.of(c, ent.word(c));
-  }
-  const uint64_t tile_sz = (uint64_t)blockDim.x * TB_ITEMS;
-  for (uint64_t tile = (uint64_t)blockIdx.x * tile_sz; tile < n; tile += (uint64_t)gridDim.x * tile_sz) {
-    uint32_t pv[TB_ITEMS], sib[TB_ITEMS], first[TB_ITEMS];
-#pragma unroll
-    for (int i = 0; i < TB_ITEMS; ++i) {
-      const uint64_t v = tile + (uint64_t)i * blockDim.x + threadIdx.x;
-      pv[i] = (uint32_t)v;
-      sib[i] = first[i] = NO_CHILD;
-      if (v < n) {
-        pv[i] = __ldcs(p32 + v);
-        sib[i] = __ldcs(nsib + v);
-        first[i] = __ldcs(fc + v);
-      }
-    }
-    uint2 wsib[TB_ITEMS], wfirst[TB_ITEMS], wown[TB_ITEMS];
-#pragma unroll
-    for (int i = 0; i < TB_ITEMS; ++i) {
-      const uint32_t v = (uint32_t)(tile + (uint64_t)i * blockDim.x + threadIdx.x);
-      if (pv[i] >= n) pv[i] = v;  // k_link_children made bad parents roots; keeps every read in range
-      const bool child = v < n && pv[i] != v;
-      wsib[i] = wfirst[i] = wown[i] = make_uint2(0, 0);
-      if (child) {
-        if (sib[i] != NO_CHILD) wsib[i] = ent.word(sib[i]);
-        if (first[i] != NO_CHILD) {
-          wfirst[i] = ent.word(first[i]);
-          wown[i] = ent.word(v);
-        }
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < TB_ITEMS; ++i) {
-      const uint32_t v = (uint32_t)(tile + (uint64_t)i * blockDim.x + threadIdx.x);
-      bool leaf = false;
-      if (v < n) {
-        const uint32_t p = pv[i];
-        uint32_t uw = 0, ub = v;  // a root: the tour's terminal element (or an isolated vertex)
-        if (p != v) {
-          ub = (sib[i] != NO_CHILD) ? ent.of(sib[i], wsib[i]) : p;
-          if (first[i] != NO_CHILD) {
-            uw = 1u;
-            const uint32_t down = ent.down_slot(v, wown[i]);
-            const uint32_t db = ent.of(first[i], wfirst[i]);
-            uint32_t k;
-            F::put(rec + down, TOUR_DOWN, db, rl.is(db, &k));
-            if (stamp) F::clear(stamp + down);
-          } else {
-            leaf = true;  // down (-1) and up (+1) in one element of weight 0
-          }
-        }
-        uint32_t k;
-        F::put(rec + v, uw, ub, rl.is(ub, &k));
-        if (stamp) F::clear(stamp + v);
-      }
-      // a warp's 32 consecutive vertices make one word of leaf bits
-      const uint32_t lb = __ballot_sync(0xffffffffu, leaf);
-      if (lane == 0 && v < n) leaf_bits[v >> 5] = lb;
     }
   }
 }
@@ -519,13 +406,12 @@ kascade_status build_tour(kascade_ctx& ctx, const uint64_t* parent, uint32_t n, 
   uint32_t* p32 = alloc<uint32_t>(ctx, n);
   uint32_t* root_bits = alloc<uint32_t>(ctx, words);
   uint32_t* ibits = alloc<uint32_t>(ctx, words);
-  uint32_t* icount = alloc<uint32_t>(ctx, words);
   uint32_t* head = alloc<uint32_t>(ctx, HEAD_CAP);
-  if (!fc || !nsib || !p32 || !root_bits || !ibits || !icount || !head) return KASCADE_ERR_OOM;
+  if (!fc || !nsib || !p32 || !root_bits || !ibits || !head) return KASCADE_ERR_OOM;
   *heads = Heads{head, &ctx.d_status->heads, HEAD_CAP};
   KS_TRY(link_children(ctx, parent, n, fc, nsib, p32, root_bits, s));
   ProfScope ps(ctx, "tour_build", s);
-  k_internal_words<<<grid_for(ctx, n, 256, 8), 256, 0, s>>>(p32, fc, n, ibits, icount, head,
+  k_internal_words<<<grid_for(ctx, n, 256, 8), 256, 0, s>>>(p32, fc, n, ibits, head,
                                                               &ctx.d_status->heads);
   KS_CHECK_LAUNCH();
   const unsigned grid =
@@ -548,62 +434,6 @@ kascade_status build_tour(kascade_ctx& ctx, const uint64_t* parent, uint32_t n, 
 }
 
 }  // namespace
-
-kascade_status root_forest_impl(kascade_ctx& ctx, const uint64_t* parent, uint32_t n, uint64_t* root_out,
-                                uint64_t* depth_out, int keep_roots, const Params& p, cudaStream_t s) {
-  if (n == 0) return KASCADE_OK;
-  const uint32_t words = (uint32_t)(((uint64_t)n + 31) / 32);
-  Level0 l0;
-  // the tour has at most 2n elements, about 1.5n with its leaves contracted
-  Level0Plan plan = plan_level0(p, (3ull * n + 1) / 2, WKind::Unit);
-  if (2ull * n > REC8_MAX && plan.fmt == Format::F8x8) plan.fmt = Format::F16x16;
-  KS_TRY(alloc_level0(ctx, plan, 2ull * n, &l0));
-  uint32_t* downs = alloc<uint32_t>(ctx, 1);  // down-edge count
-  uint32_t* fc = alloc<uint32_t>(ctx, n);
-  uint32_t* nsib = alloc<uint32_t>(ctx, n);
-  uint32_t* p32 = alloc<uint32_t>(ctx, n);
-  uint32_t* root_bits = alloc<uint32_t>(ctx, words);
-  uint32_t* ibits = alloc<uint32_t>(ctx, words);
-  uint32_t* icount = alloc<uint32_t>(ctx, words);
-  uint32_t* ipre = alloc<uint32_t>(ctx, words);
-  uint32_t* leaf_bits = alloc<uint32_t>(ctx, words);
-  uint2* iw = alloc<uint2>(ctx, words);
-  uint32_t* head = alloc<uint32_t>(ctx, HEAD_CAP);
-  if (!downs || !fc || !nsib || !p32 || !root_bits || !ibits || !icount || !ipre || !leaf_bits || !iw || !head)
-    return KASCADE_ERR_OOM;
-  KS_TRY(link_children(ctx, parent, n, fc, nsib, p32, root_bits, s));
-  {
-    ProfScope ps(ctx, "tour_build", s);
-    k_internal_words<<<grid_for(ctx, n, 256, 8), 256, 0, s>>>(p32, fc, n, ibits, icount, head,
-                                                              &ctx.d_status->heads);
-    KS_CHECK_LAUNCH();
-    KS_TRY(exclusive_scan_u32(ctx, icount, ipre, words, downs, s));
-    k_internal_pack<<<grid_for(ctx, words, 256, 8), 256, 0, s>>>(ibits, ipre, words, iw);
-    KS_CHECK_LAUNCH();
-    const unsigned grid = grid_for(ctx, ((uint64_t)n + 256 * TB_ITEMS - 1) / (256 * TB_ITEMS) * 256, 256, 8);
-    auto leaves = [&](auto f) {
-      using F = decltype(f);
-      k_tour_leaves<F><<<grid, 256, 0, s>>>(p32, n, fc, nsib, Entries{iw, n}, level0_rulers(p), l0.records<F>(),
-                                            l0.stamps<F>(), leaf_bits, head, &ctx.d_status->heads);
-    };
-    if (l0.fmt == Format::F8x8)
-      leaves(F8x8{});
-    else if (l0.fmt == Format::F16i)
-      leaves(F16i{});
-    else
-      leaves(F16x16{});
-    KS_CHECK_LAUNCH();
-  }
-  // The tour's length n + (down edges) stays on the device: the ranking is
-  // sized for the bound 2n, rulers beyond the length are dead, and outputs
-  // come only from slots below n.
-  Extent ext;
-  ext.cap = 2 * n;
-  ext.base = n;
-  ext.add = downs;
-  return rank_records(ctx, l0, ext.cap, ext, Heads{head, &ctx.d_status->heads, HEAD_CAP},
-                      SinkTour{root_out, depth_out, n, keep_roots, leaf_bits}, p, s);
-}
 
 // Tours of a batch of forests whose parents are given in one compact vertex
 // space (fpar[c] = compact parent of compact vertex c); records go to the

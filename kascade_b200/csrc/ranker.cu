@@ -49,8 +49,6 @@ struct WI64 {
   }
 };
 
-inline uint32_t salt_for(uint32_t seed, int level) { return mix32(seed + 0x9E3779B9u * (uint32_t)(level + 1)); }
-
 // ---------------------------------------------------------------------------
 // prepare: build records, clear the stamps (stamp == nullptr: the write-free
 // path has none).  A root's weight is no part of any rank: its record carries
@@ -201,8 +199,6 @@ __global__ void __launch_bounds__(512) k_chase(const typename F::R* rec, typenam
   const uint32_t n = ext.get();
   const uint32_t r = rulers + heads.get();
   if (nx.rl.s == 0) nx.rl = cta_rulers(r);
-  // level 0's size, reported by the call
-  if (!rootel && ext.add && blockIdx.x == 0 && threadIdx.x == 0) st->counter[1] = n;
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
   const uint32_t warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -427,8 +423,9 @@ __global__ void __launch_bounds__(256) k_propagate(const typename F::R* __restri
 // With several lists, their heads (no predecessor) start chains as well, so
 // that no run of elements ahead of a first ruler is walked element by element.
 // Two chains that meet (a tree, not a list) leave fewer stamped elements than
-// stamps; an input of at most `tree_max` elements is then done again without
-// stamps, every element walking to its first ruler, which ranks any forest.
+// stamps; CTA_SMALL_TREES does an input of at most ONE_CTA_TREES elements again
+// without stamps, every element walking to its first ruler, which ranks any
+// forest; CTA_TREES and CTA_ROOTING do so from the start.
 // ---------------------------------------------------------------------------
 constexpr uint32_t CTA_THREADS = 1024;
 constexpr uint32_t CTA_HEADS = 1024;
@@ -472,8 +469,8 @@ struct CtaArrays {
 };
 
 template <class Src, class Sink>
-__global__ void __launch_bounds__(CTA_THREADS, 1) k_rank_cta(Src src, Extent ext, Sink sink, uint32_t tree_max,
-                                                             int level0, DevStatus* st) {
+__global__ void __launch_bounds__(CTA_THREADS, 1) k_rank_cta(Src src, Extent ext, Sink sink, CtaMode mode,
+                                                             DevStatus* st) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ uint32_t nends, nheads, nstamps;
   const uint32_t n = ext.get();
@@ -487,7 +484,6 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) k_rank_cta(Src src, Extent ext
   unsigned char* pred = reinterpret_cast<unsigned char*>(predw);  // 1: has a predecessor
   uint16_t* hlist = reinterpret_cast<uint16_t*>(predw + (ext.cap + 3) / 4);
   const uint32_t tid = threadIdx.x, nthreads = blockDim.x;
-  if (level0 && ext.add && tid == 0) st->counter[1] = n;
   const Rulers rl = cta_rulers(n);
   const bool all = rl.s == 1;  // every element is a ruler
   const uint32_t rulers = all ? n : (n + rl.s - 1) / rl.s;
@@ -496,7 +492,7 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) k_rank_cta(Src src, Extent ext
     return all || rl.is(x, &j);
   };
   auto elem = [&](uint32_t j) { return all ? j : (uint32_t)rl.elem(j); };
-  bool stamp = true;
+  bool stamp = mode <= CTA_SMALL_TREES;
   uint32_t heads = 0;
   while (true) {
     if (tid == 0) nends = nheads = nstamps = 0;
@@ -530,6 +526,19 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) k_rank_cta(Src src, Extent ext
     ends = __reduce_add_sync(FULL, ends);
     if ((tid & 31u) == 0 && ends) atomicAdd(&nends, ends);
     __syncthreads();
+    if (mode == CTA_ROOTING) {  // report the tour's length: the vertices, and those between a root and a leaf again
+      for (uint32_t w = tid; w < (n + 3) / 4; w += nthreads) predw[w] = 0;
+      __syncthreads();
+      for (uint32_t x = tid; x < n; x += nthreads) {
+        const uint32_t y = next[x] & CTA_IDX;
+        if (y != x) pred[y] = 1;
+      }
+      __syncthreads();
+      uint32_t downs = 0;
+      for (uint32_t x = tid; x < n; x += nthreads) downs += pred[x] && next[x] != x ? 1u : 0u;
+      downs = __reduce_add_sync(FULL, downs);
+      if ((tid & 31u) == 0) atomicAdd(&st->counter[1], (unsigned long long)(downs + (tid == 0 ? n : 0u)));
+    }
     // with several lists, their heads start chains too
     if (stamp && !all && nends > 2) {
       for (uint32_t w = tid; w < (n + 3) / 4; w += nthreads) predw[w] = 0;
@@ -614,7 +623,7 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) k_rank_cta(Src src, Extent ext
     if ((tid & 31u) == 0 && marks) atomicSub(&nstamps, marks);
     __syncthreads();
     if (!clash && nstamps == 0) break;
-    if (n > tree_max) {
+    if (mode == CTA_LISTS || n > ONE_CTA_TREES) {
       if (tid == 0) set_error(st, KASCADE_ERR_NOT_A_LIST, n);
       return;
     }
@@ -890,7 +899,7 @@ kascade_status launch_propagate(kascade_ctx& ctx, const Levels& lv, int k, const
 
 template <class Src, class Sink>
 kascade_status launch_rank_cta(kascade_ctx& ctx, const Src& src, const Extent& ext, const Sink& sink,
-                               uint32_t tree_max, int level0, cudaStream_t s) {
+                               CtaMode mode, cudaStream_t s) {
   static std::atomic<uint64_t> raised{0};  // kernel attributes are per device
   const uint64_t bit = 1ull << (ctx.device & 63);
   if (!(raised.load() & bit)) {
@@ -901,7 +910,7 @@ kascade_status launch_rank_cta(kascade_ctx& ctx, const Src& src, const Extent& e
   ProfScope ps(ctx, "base_case", s);
   // one ruler per thread; a small input's few barriers are cheaper with fewer warps
   const unsigned threads = ext.cap <= 1024 ? 256 : CTA_THREADS;
-  k_rank_cta<Src, Sink><<<1, threads, cta_smem(ext.cap), s>>>(src, ext, sink, tree_max, level0, ctx.d_status);
+  k_rank_cta<Src, Sink><<<1, threads, cta_smem(ext.cap), s>>>(src, ext, sink, mode, ctx.d_status);
   KS_CHECK_LAUNCH();
   return KASCADE_OK;
 }
@@ -946,7 +955,7 @@ Params make_params(const kascade_ctx& ctx, const kascade_opts* o, uint64_t n) {
     p.block = ctx.class_block[k];
   }
   if (o) {
-    if (o->ruler_spacing) p.spacing0 = o->ruler_spacing;
+    if (o->ruler_spacing) p.spacing0 = p.spacing_given = o->ruler_spacing;
     if (o->ruler_spacing_deep) p.spacing_deep = o->ruler_spacing_deep;
     if (o->max_levels) p.max_levels = o->max_levels;
     if (o->base_case_size) p.base_max = o->base_case_size;
@@ -1063,61 +1072,31 @@ kascade_status prepare_arrays(kascade_ctx& ctx, const uint64_t* succ, WKind wk, 
 }
 
 kascade_status rank_arrays_one_cta(kascade_ctx& ctx, const uint64_t* succ, WKind wk, const void* w, uint32_t n,
-                                   const SinkPlain& sink, cudaStream_t s) {
+                                   const SinkPlain& sink, CtaMode mode, cudaStream_t s) {
   ctx.last_levels.assign(1, n);
   Extent ext;
   ext.cap = n;
   switch (wk) {
     case WKind::Unit:
-      return launch_rank_cta(ctx, CtaArrays<WUnit>{succ, WUnit{}}, ext, sink, ONE_CTA_TREES, 1, s);
+      return launch_rank_cta(ctx, CtaArrays<WUnit>{succ, WUnit{}}, ext, sink, mode, s);
     case WKind::U32:
-      return launch_rank_cta(ctx, CtaArrays<WU32>{succ, WU32{(const uint32_t*)w}}, ext, sink, ONE_CTA_TREES, 1, s);
+      return launch_rank_cta(ctx, CtaArrays<WU32>{succ, WU32{(const uint32_t*)w}}, ext, sink, mode, s);
     default:
-      return launch_rank_cta(ctx, CtaArrays<WI64>{succ, WI64{(const int64_t*)w}}, ext, sink, ONE_CTA_TREES, 1, s);
+      return launch_rank_cta(ctx, CtaArrays<WI64>{succ, WI64{(const int64_t*)w}}, ext, sink, mode, s);
   }
 }
 
-template <class Sink>
-kascade_status pointer_double_records(kascade_ctx& ctx, const Rec* rec, uint32_t n, const uint32_t* elem0,
-                                      const Sink& sink, cudaStream_t s) {
-  if (n == 0) return KASCADE_OK;
-  PdRec* a = alloc<PdRec>(ctx, n);
-  PdRec* b = alloc<PdRec>(ctx, n);
-  uint32_t* active = alloc<uint32_t>(ctx, 1);
-  if (!a || !b || !active) return KASCADE_ERR_OOM;
-  unsigned grid = grid_for(ctx, n, 256, 8);
+kascade_status rank_trees_one_cta(kascade_ctx& ctx, const Rec8* rec, const uint32_t* rootel, uint32_t n, uint2* out,
+                                  cudaStream_t s) {
   Extent ext;
   ext.cap = n;
-  {
-    ProfScope ps(ctx, "pd_init", s);
-    k_pd_init<<<grid, 256, 0, s>>>(rec, ext, a, ctx.d_status);
-    KS_CHECK_LAUNCH();
-  }
-  int rounds = 0;
-  while (true) {
-    KS_CUDA(cudaMemsetAsync(active, 0, sizeof(uint32_t), s));
-    {
-      ProfScope ps(ctx, "pd_round", s);
-      k_pd_round<1><<<grid, 256, 0, s>>>(a, b, ext, active);
-      KS_CHECK_LAUNCH();
-    }
-    PdRec* t = a;
-    a = b;
-    b = t;
-    uint32_t left = 0;
-    KS_TRY(read_u32(ctx, active, &left, s));
-    if (left == 0) break;
-    if (++rounds > 64) {
-      ctx.error_info = left;
-      return KASCADE_ERR_CYCLE;
-    }
-  }
-  {
-    ProfScope ps(ctx, "pd_final", s);
-    k_pd_final<Sink><<<grid, 256, 0, s>>>(a, ext, elem0, sink);
-    KS_CHECK_LAUNCH();
-  }
-  return KASCADE_OK;
+  return launch_rank_cta(ctx, CtaRecords<F8x8, true>{rec, rootel}, ext, SinkOut8{out}, CTA_TREES, s);
+}
+kascade_status rank_trees_one_cta(kascade_ctx& ctx, const Rec* rec, const uint32_t* rootel, uint32_t n, Out* out,
+                                  cudaStream_t s) {
+  Extent ext;
+  ext.cap = n;
+  return launch_rank_cta(ctx, CtaRecords<F16x16, true>{rec, rootel}, ext, SinkOut{out}, CTA_TREES, s);
 }
 
 // Doubling for a fixed number of rounds, enough for any list the level can
@@ -1191,8 +1170,8 @@ kascade_status rank_deep(kascade_ctx& ctx, const Levels& lv, cudaStream_t s) {
     KS_TRY(launch_chase<F16x16>(ctx, lv, k, lv.rec[k], lv.stamp[k], lv.extent(k), lv.n[k], 256, s));
   const int L = lv.last;
   if (lv.n[L] <= ONE_CTA_MAX) {
-    KS_TRY(launch_rank_cta(ctx, CtaRecords<F16x16, true>{lv.rec[L], lv.rootel[L]}, lv.extent(L), SinkOut{lv.out[L]}, 0, 0,
-                           s));
+    KS_TRY(launch_rank_cta(ctx, CtaRecords<F16x16, true>{lv.rec[L], lv.rootel[L]}, lv.extent(L), SinkOut{lv.out[L]},
+                           CTA_LISTS, s));
   } else {
     KS_TRY(pointer_double_level(ctx, lv.rec[L], lv.extent(L), lv.rootel[L], lv.out[L], s));
   }
@@ -1210,7 +1189,7 @@ kascade_status rank_records_as(kascade_ctx& ctx, const Level0& l0, uint32_t n, c
   const typename F::R* rec = l0.records<F>();
   if (n <= p.base_max) {
     ctx.last_levels.assign(1, n);
-    return launch_rank_cta(ctx, CtaRecords<F, false>{rec, nullptr}, ext, sink, ONE_CTA_TREES, 1, s);
+    return launch_rank_cta(ctx, CtaRecords<F, false>{rec, nullptr}, ext, sink, CTA_SMALL_TREES, s);
   }
   Levels lv;
   KS_TRY(plan_levels(ctx, n, heads, p, &lv));
@@ -1260,11 +1239,7 @@ kascade_status check_is_list(kascade_ctx& ctx, const uint64_t* succ, uint64_t n,
 // explicit instantiations for the level-0 sinks
 template kascade_status rank_records<SinkPlain>(kascade_ctx&, const Level0&, uint32_t, const Extent&, const Heads&,
                                                 const SinkPlain&, const Params&, cudaStream_t);
-template kascade_status rank_records<SinkTour>(kascade_ctx&, const Level0&, uint32_t, const Extent&, const Heads&,
-                                               const SinkTour&, const Params&, cudaStream_t);
 template kascade_status rank_records<SinkBatch>(kascade_ctx&, const Level0&, uint32_t, const Extent&, const Heads&,
                                                 const SinkBatch&, const Params&, cudaStream_t);
-template kascade_status pointer_double_records<SinkPlain>(kascade_ctx&, const Rec*, uint32_t, const uint32_t*,
-                                                          const SinkPlain&, cudaStream_t);
 
 }  // namespace ks

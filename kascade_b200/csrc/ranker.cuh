@@ -29,6 +29,7 @@ namespace ks {
 
 struct Params {
   uint32_t spacing0 = 48;     // mean elements per ruler, level 0
+  uint32_t spacing_given = 0;  // the caller's, if any
   uint32_t spacing_deep = 0;  // mean elements per ruler, deeper levels (0: by level size)
   uint32_t max_levels = 6;
   uint32_t base_max = 16384;  // one-CTA ranker bound
@@ -81,6 +82,7 @@ constexpr uint32_t CTA_RULERS = 1024;
 __host__ __device__ inline Rulers cta_rulers(uint32_t n) {
   return make_rulers((n + CTA_RULERS - 1) / CTA_RULERS, 0x63746121u);
 }
+inline uint32_t salt_for(uint32_t seed, int level) { return mix32(seed + 0x9E3779B9u * (uint32_t)(level + 1)); }
 inline uint32_t ruler_count(uint32_t n, const Rulers& r) { return (uint32_t)(((uint64_t)n + r.s - 1) / r.s); }
 
 // A level's element count when only the device knows it: base + *add, at most
@@ -124,9 +126,7 @@ struct LogTarget {
   // bit x set: element x's rank output is one more than its rank in the list
   // (a tree rooting's leaves, whose down and up edge share one element)
   const uint32_t* plus_one = nullptr;
-  // depths: ranks modulo 2^32 -- of every element (tour), or of the instances
-  // with their bit set (a batch's forests)
-  int tour = 0;
+  // depths: ranks modulo 2^32, of the instances with their bit set (a batch's forests)
   const uint32_t* seg_tour = nullptr;
 };
 
@@ -149,39 +149,6 @@ struct SinkPlain {
     }
     __stcs(root + x, (unsigned long long)rt);
     __stcs(rank + x, (unsigned long long)rk);
-  }
-};
-
-// Euler tour: elements 0..nv-1 are the vertices' up edges (roots: the tour's
-// terminal element), so only those produce output.
-// A down edge's weight is -1 modulo 2^32, so a depth is its rank modulo 2^32.
-// leaf_bits: bit v set for a leaf whose down and up edge are one element of
-// weight 0, whose rank is then one less than the leaf's depth.
-struct SinkTour {
-  uint64_t* root;
-  uint64_t* depth;
-  uint32_t nv;
-  int keep_roots;
-  const uint32_t* leaf_bits = nullptr;
-  uint32_t limit(uint32_t n) const { return n < nv ? n : nv; }
-  LogTarget log_target(uint32_t n) const {
-    LogTarget t{root, depth, limit(n), keep_roots};
-    t.plus_one = leaf_bits;
-    t.tour = 1;
-    return t;
-  }
-  __device__ __forceinline__ void put(uint32_t x, uint64_t rk, uint32_t rt, bool is_root) const {
-    if (x >= nv) return;
-    if (is_root) {
-      if (!keep_roots) {
-        __stcs(root + x, (unsigned long long)x);
-        __stcs(depth + x, 0ull);
-      }
-      return;
-    }
-    const uint32_t d = (uint32_t)rk + ((__ldg(leaf_bits + (x >> 5)) >> (x & 31)) & 1u);
-    __stcs(root + x, (unsigned long long)rt);
-    __stcs(depth + x, (unsigned long long)d);
   }
 };
 
@@ -234,6 +201,15 @@ struct SinkOut {
   }
 };
 
+// Results of a tree rooting's deeper levels: depths fit 32 bits.
+struct SinkOut8 {
+  uint2* out;  // (depth, root)
+  __device__ __forceinline__ void put(uint32_t x, uint64_t rk, uint32_t rt, bool is_root) const {
+    (void)is_root;
+    __stcg(out + x, make_uint2((uint32_t)rk, rt));
+  }
+};
+
 // Weight readers for building level-0 records.
 enum class WKind { Unit, U32, I64 };
 
@@ -269,8 +245,19 @@ uint32_t hop_cap(const Rulers& rl);
 // launch.  Any forest is accepted up to ONE_CTA_TREES elements; above, lists.
 constexpr uint32_t ONE_CTA_MAX = 14336;
 constexpr uint32_t ONE_CTA_TREES = 8192;
+// What the one-CTA ranker takes: lists only; lists, and trees up to
+// ONE_CTA_TREES elements; trees; trees whose tour's length is to be reported.
+enum CtaMode : uint32_t { CTA_LISTS, CTA_SMALL_TREES, CTA_TREES, CTA_ROOTING };
 kascade_status rank_arrays_one_cta(kascade_ctx& ctx, const uint64_t* succ, WKind wk, const void* w, uint32_t n,
-                                   const SinkPlain& sink, cudaStream_t s);
+                                   const SinkPlain& sink, CtaMode mode, cudaStream_t s);
+// A forest's last level (its records' ruler bits are for cta_rulers(n)).
+kascade_status rank_trees_one_cta(kascade_ctx& ctx, const Rec8* rec, const uint32_t* rootel, uint32_t n, uint2* out,
+                                  cudaStream_t s);
+kascade_status rank_trees_one_cta(kascade_ctx& ctx, const Rec* rec, const uint32_t* rootel, uint32_t n, Out* out,
+                                  cudaStream_t s);
+// Any forest: results of every element (tree.cu).
+kascade_status rank_forest_weighted(kascade_ctx& ctx, const uint64_t* succ, WKind wk, const void* w, uint32_t n,
+                                    const SinkPlain& sink, const Params& p, cudaStream_t s);
 
 // Rank level-0 records and deliver the results to the sink.  Every level's
 // size is known on the host: no host wait between the launches.  `ext`: the
@@ -354,12 +341,6 @@ kascade_status compute_stats(kascade_ctx& ctx, const uint64_t* root, const int64
 // and a dense placement into the outputs.
 kascade_status rank_level0_log(kascade_ctx& ctx, const Level0& l0, uint32_t n, const Extent& ext, const Heads& heads,
                                const LogTarget& t, const Params& p, cudaStream_t s);
-
-// Pointer doubling on level-0 records (tags ignored).
-template <class Sink>
-kascade_status pointer_double_records(kascade_ctx& ctx, const Rec* rec, uint32_t n,
-                                      const uint32_t* elem0, const Sink& sink,
-                                      cudaStream_t s);
 
 // Validation: *ok = 1 if no element has two predecessors.
 kascade_status check_is_list(kascade_ctx& ctx, const uint64_t* succ, uint64_t n, int* ok,
