@@ -1086,16 +1086,12 @@ kascade_status rank_arrays_one_cta(kascade_ctx& ctx, const uint64_t* succ, WKind
   }
 }
 
-kascade_status rank_trees_one_cta(kascade_ctx& ctx, const Rec8* rec, const uint32_t* rootel, uint32_t n, uint2* out,
-                                  cudaStream_t s) {
-  Extent ext;
-  ext.cap = n;
+kascade_status rank_trees_one_cta(kascade_ctx& ctx, const Rec8* rec, const uint32_t* rootel, const Extent& ext,
+                                  uint2* out, cudaStream_t s) {
   return launch_rank_cta(ctx, CtaRecords<F8x8, true>{rec, rootel}, ext, SinkOut8{out}, CTA_TREES, s);
 }
-kascade_status rank_trees_one_cta(kascade_ctx& ctx, const Rec* rec, const uint32_t* rootel, uint32_t n, Out* out,
-                                  cudaStream_t s) {
-  Extent ext;
-  ext.cap = n;
+kascade_status rank_trees_one_cta(kascade_ctx& ctx, const Rec* rec, const uint32_t* rootel, const Extent& ext,
+                                  Out* out, cudaStream_t s) {
   return launch_rank_cta(ctx, CtaRecords<F16x16, true>{rec, rootel}, ext, SinkOut{out}, CTA_TREES, s);
 }
 

@@ -85,13 +85,20 @@ __host__ __device__ inline Rulers cta_rulers(uint32_t n) {
 inline uint32_t salt_for(uint32_t seed, int level) { return mix32(seed + 0x9E3779B9u * (uint32_t)(level + 1)); }
 inline uint32_t ruler_count(uint32_t n, const Rulers& r) { return (uint32_t)(((uint64_t)n + r.s - 1) / r.s); }
 
-// A level's element count when only the device knows it: base + *add, at most
-// the capacity the launch was sized for (add == nullptr: the capacity).
+// A level's element count when only the device knows it: (base + *add) / div,
+// rounded up, at most the capacity the launch was sized for (add == nullptr:
+// the capacity).
 struct Extent {
   uint32_t cap = 0;
   uint32_t base = 0;
   const uint32_t* add = nullptr;
-  __device__ __forceinline__ uint32_t get() const { return add ? (uint32_t)min((uint64_t)cap, (uint64_t)base + __ldg(add)) : cap; }
+  uint32_t div = 1;
+  __device__ __forceinline__ uint32_t get() const {
+    if (!add) return cap;
+    uint32_t v = (uint32_t)min((uint64_t)0xFFFFFFFFu, (uint64_t)base + __ldg(add));
+    if (div != 1) v = v / div + (v % div != 0u ? 1u : 0u);
+    return min(cap, v);
+  }
 };
 
 // Known list heads of level 0 (a tour's heads are known when it is built):
@@ -251,10 +258,10 @@ enum CtaMode : uint32_t { CTA_LISTS, CTA_SMALL_TREES, CTA_TREES, CTA_ROOTING };
 kascade_status rank_arrays_one_cta(kascade_ctx& ctx, const uint64_t* succ, WKind wk, const void* w, uint32_t n,
                                    const SinkPlain& sink, CtaMode mode, cudaStream_t s);
 // A forest's last level (its records' ruler bits are for cta_rulers(n)).
-kascade_status rank_trees_one_cta(kascade_ctx& ctx, const Rec8* rec, const uint32_t* rootel, uint32_t n, uint2* out,
-                                  cudaStream_t s);
-kascade_status rank_trees_one_cta(kascade_ctx& ctx, const Rec* rec, const uint32_t* rootel, uint32_t n, Out* out,
-                                  cudaStream_t s);
+kascade_status rank_trees_one_cta(kascade_ctx& ctx, const Rec8* rec, const uint32_t* rootel, const Extent& ext,
+                                  uint2* out, cudaStream_t s);
+kascade_status rank_trees_one_cta(kascade_ctx& ctx, const Rec* rec, const uint32_t* rootel, const Extent& ext,
+                                  Out* out, cudaStream_t s);
 // Any forest: results of every element (tree.cu).
 kascade_status rank_forest_weighted(kascade_ctx& ctx, const uint64_t* succ, WKind wk, const void* w, uint32_t n,
                                     const SinkPlain& sink, const Params& p, cudaStream_t s);

@@ -28,7 +28,12 @@ namespace {
 
 constexpr int TREE_THREADS = 256;
 constexpr int TREE_PREP_ITEMS = 8;
-constexpr uint32_t TREE_SPACING = 3;
+constexpr int TREE_OUT_ITEMS = 4;  // (2: 1.07 ms, 4 and 8: 0.95 for 2^26 vertices)
+// Mean elements per ruler.  Large levels are bound by what they read at
+// random, (s + 1) s / (s - 1) reads an element over all levels; small ones by
+// their longest walks and by launches.  2^26 caterpillars, s = 2 / 3 / 4:
+// 4.0 / 4.2 / 4.4 ms; 4.2M random recursive trees 314 / 275 / 250 us.
+constexpr uint32_t TREE_SPACING = 4, TREE_SPACING_LARGE = 2, TREE_LARGE = 1u << 23;
 // Largest last level: without stamps the one-CTA ranker's walks grow with its
 // spacing (3100 elements 15 us, 6200 24, 8300 44, 12500 75; a level above it
 // costs ~13 us).
@@ -73,63 +78,225 @@ struct Tree16 {
   }
 };
 
-__device__ __forceinline__ bool bit_of(const uint32_t* bits, uint32_t x) {
-  return (__ldg(bits + (x >> 5)) >> (x & 31)) & 1u;
+// ---------------------------------------------------------------------------
+// Tree rooting works on the vertices that have children, renumbered densely:
+// a leaf is on nobody's path, and its result is its parent's with one more
+// step.  Half the vertices of random recursive trees and of caterpillars are
+// leaves; what the walks read at random is then half as large (2^26
+// caterpillars: 134 MB instead of 268, about the L2).
+// ---------------------------------------------------------------------------
+constexpr int WORDS_PER = 8;  // words of 32 vertices a thread counts
+constexpr uint32_t WORDS_TILE = TREE_THREADS * WORDS_PER;
+
+__device__ __forceinline__ uint64_t parent_of(const uint64_t* parent, uint64_t v, uint32_t n) {
+  return v < n ? __ldcs(reinterpret_cast<const unsigned long long*>(parent) + v) : v;
 }
 
-// Level-0 records of a tree rooting, and a bit for every vertex with a child
-// (zeroed by the caller): a ruler without one is on nobody's path.
-__global__ void __launch_bounds__(TREE_THREADS) k_tree_prepare(const uint64_t* __restrict__ parent, uint32_t n,
-                                                               Rulers rl, uint32_t* __restrict__ rec,
-                                                               uint32_t* __restrict__ inner, DevStatus* st) {
+// A byte set for every vertex with a child (zeroed by the caller).  A parent
+// out of range is reported; its vertex counts as a root everywhere.
+// Bytes and not bits, although bound by the L2 either way: 2^26 caterpillars
+// 0.56 ms against 0.40 with an atomic OR per vertex, but a hundred hubs with all
+// the leaves 0.3 ms against 15 (atomics on a few words come one at a time), and
+// asking for the word before the atomic costs 0.63.
+__global__ void __launch_bounds__(TREE_THREADS) k_tree_inner(const uint64_t* __restrict__ parent, uint32_t n,
+                                                             unsigned char* __restrict__ inner, DevStatus* st) {
   const uint64_t tile_sz = (uint64_t)blockDim.x * TREE_PREP_ITEMS;
   for (uint64_t tile = (uint64_t)blockIdx.x * tile_sz; tile < n; tile += (uint64_t)gridDim.x * tile_sz) {
     uint64_t p[TREE_PREP_ITEMS];
-    uint32_t w[TREE_PREP_ITEMS];
+#pragma unroll
+    for (int i = 0; i < TREE_PREP_ITEMS; ++i) p[i] = parent_of(parent, tile + (uint64_t)i * blockDim.x + threadIdx.x, n);
 #pragma unroll
     for (int i = 0; i < TREE_PREP_ITEMS; ++i) {
       const uint64_t v = tile + (uint64_t)i * blockDim.x + threadIdx.x;
-      p[i] = v < n ? __ldcs(reinterpret_cast<const unsigned long long*>(parent) + v) : v;
-    }
-#pragma unroll
-    for (int i = 0; i < TREE_PREP_ITEMS; ++i) {
-      const uint64_t v = tile + (uint64_t)i * blockDim.x + threadIdx.x;
-      w[i] = 0xFFFFFFFFu;
-      if (v >= n) continue;
       if (p[i] >= n) {
-        set_error(st, KASCADE_ERR_OUT_OF_RANGE, v);
+        if (v < n) set_error(st, KASCADE_ERR_OUT_OF_RANGE, v);
         p[i] = v;
       }
-      if (p[i] != v) w[i] = __ldcg(inner + (p[i] >> 5));  // a set bit is not set again: a star's root stays cheap
-    }
-#pragma unroll
-    for (int i = 0; i < TREE_PREP_ITEMS; ++i) {
-      const uint64_t v = tile + (uint64_t)i * blockDim.x + threadIdx.x;
-      if (v >= n) continue;
-      const uint32_t b = (uint32_t)p[i];
-      if (!((w[i] >> (b & 31)) & 1u)) atomicOr(inner + (b >> 5), 1u << (b & 31));
-      uint32_t j;
-      rec[v] = b | (b != (uint32_t)v && rl.is(b, &j) ? REC8_RULER : 0u);
+      if (p[i] != v) __stcg(inner + p[i], (unsigned char)1);
     }
   }
 }
 
-// Every ruler's walk to the next ruler or its root.  inner: level 0's vertices
-// with a child (null: not known).
+// The bits of 32 vertices' bytes (each 0 or 1).
+__device__ __forceinline__ uint32_t inner_word(const unsigned char* inner, uint32_t w) {
+  const uint4 a = __ldcg(reinterpret_cast<const uint4*>(inner) + 2ull * w);
+  const uint4 b = __ldcg(reinterpret_cast<const uint4*>(inner) + 2ull * w + 1);
+  auto four = [](uint32_t v) { return (v * 0x01020408u) >> 24; };  // byte i's bit to bit i
+  return four(a.x) | four(a.y) << 4 | four(a.z) << 8 | four(a.w) << 12 | four(b.x) << 16 | four(b.y) << 20 |
+         four(b.z) << 24 | four(b.w) << 28;
+}
+
+__device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t* sm) {  // all threads get it
+  v = __reduce_add_sync(0xffffffffu, v);
+  if ((threadIdx.x & 31u) == 0) sm[threadIdx.x >> 5] = v;
+  __syncthreads();
+  uint32_t t = 0;
+#pragma unroll
+  for (int i = 0; i < TREE_THREADS / 32; ++i) t += sm[i];
+  __syncthreads();
+  return t;
+}
+
+// Vertices with children per tile of words.
+__global__ void __launch_bounds__(TREE_THREADS) k_tree_count(const unsigned char* __restrict__ inner, uint32_t words,
+                                                             uint32_t* __restrict__ sums) {
+  __shared__ uint32_t sm[TREE_THREADS / 32];
+  const uint32_t base = blockIdx.x * WORDS_TILE;
+  uint32_t c = 0;
+#pragma unroll
+  for (int i = 0; i < WORDS_PER; ++i) {
+    const uint32_t w = base + i * TREE_THREADS + threadIdx.x;
+    if (w < words) c += __popc(inner_word(inner, w));
+  }
+  c = block_sum(c, sm);
+  if (threadIdx.x == 0) sums[blockIdx.x] = c;
+}
+
+// iw[w] = (bits, bits set before word w), and their number.  A block adds up
+// the tiles before its own.
+__global__ void __launch_bounds__(TREE_THREADS) k_tree_number(const unsigned char* __restrict__ inner, uint32_t words,
+                                                              const uint32_t* __restrict__ sums,
+                                                              uint2* __restrict__ iw, uint32_t* __restrict__ count) {
+  __shared__ uint32_t sm[TREE_THREADS / 32];
+  __shared__ uint32_t tile[WORDS_TILE];
+  uint32_t before = 0;
+  for (uint32_t b = threadIdx.x; b < blockIdx.x; b += TREE_THREADS) before += sums[b];
+  before = block_sum(before, sm);
+  const uint32_t base = blockIdx.x * WORDS_TILE;
+#pragma unroll
+  for (int i = 0; i < WORDS_PER; ++i) {
+    const uint32_t w = base + i * TREE_THREADS + threadIdx.x;
+    tile[i * TREE_THREADS + threadIdx.x] = w < words ? inner_word(inner, w) : 0u;
+  }
+  __syncthreads();
+  uint32_t mine = 0;
+#pragma unroll
+  for (int i = 0; i < WORDS_PER; ++i) mine += __popc(tile[threadIdx.x * WORDS_PER + i]);
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= (uint32_t)o) incl += t;
+  }
+  if (lane == 31u) sm[threadIdx.x >> 5] = incl;
+  __syncthreads();
+  uint32_t pre = before + incl - mine;
+  for (uint32_t i = 0; i < (threadIdx.x >> 5); ++i) pre += sm[i];
+#pragma unroll
+  for (int i = 0; i < WORDS_PER; ++i) {
+    const uint32_t at = threadIdx.x * WORDS_PER + i;
+    const uint32_t bits = tile[at];
+    if (base + at < words) iw[base + at] = make_uint2(bits, pre);
+    pre += __popc(bits);
+  }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == TREE_THREADS - 1) *count = pre;
+}
+
+// A vertex with children: its number.
+__device__ __forceinline__ uint32_t number_of(uint2 w, uint32_t v) {
+  return w.y + (uint32_t)__popc(w.x & ((1u << (v & 31)) - 1u));
+}
+
+// The records of the numbered vertices; vert: their vertices (the roots').
+// Reports the tour's length: the vertices, and once more those with children
+// that are not roots.
+__global__ void __launch_bounds__(TREE_THREADS) k_tree_records(const uint64_t* __restrict__ parent, uint32_t n,
+                                                               const uint2* __restrict__ iw, Rulers rl,
+                                                               uint32_t* __restrict__ rec,
+                                                               uint32_t* __restrict__ vert, DevStatus* st) {
+  const uint64_t tile_sz = (uint64_t)blockDim.x * TREE_PREP_ITEMS;
+  uint32_t downs = 0;
+  for (uint64_t tile = (uint64_t)blockIdx.x * tile_sz; tile < n; tile += (uint64_t)gridDim.x * tile_sz) {
+    uint64_t p[TREE_PREP_ITEMS];
+    uint2 own[TREE_PREP_ITEMS], up[TREE_PREP_ITEMS];
+#pragma unroll
+    for (int i = 0; i < TREE_PREP_ITEMS; ++i) {
+      const uint64_t v = tile + (uint64_t)i * blockDim.x + threadIdx.x;
+      p[i] = parent_of(parent, v, n);
+      own[i] = v < n ? __ldg(iw + (v >> 5)) : make_uint2(0, 0);
+    }
+#pragma unroll
+    for (int i = 0; i < TREE_PREP_ITEMS; ++i) {
+      const uint64_t v = tile + (uint64_t)i * blockDim.x + threadIdx.x;
+      if (p[i] >= n) p[i] = v;
+      if (!((own[i].x >> (v & 31)) & 1u)) p[i] = ~0ull;  // a leaf
+      up[i] = p[i] < n ? __ldg(iw + (p[i] >> 5)) : make_uint2(0, 0);
+    }
+#pragma unroll
+    for (int i = 0; i < TREE_PREP_ITEMS; ++i) {
+      const uint64_t v = tile + (uint64_t)i * blockDim.x + threadIdx.x;
+      if (p[i] >= n) continue;
+      const uint32_t c = number_of(own[i], (uint32_t)v);
+      uint32_t b = number_of(up[i], (uint32_t)p[i]), j;
+      if (p[i] == v)
+        vert[c] = (uint32_t)v;
+      else
+        ++downs, b |= rl.is(b, &j) ? REC8_RULER : 0u;
+      rec[c] = b;
+    }
+  }
+  downs = __reduce_add_sync(0xffffffffu, downs);
+  if ((threadIdx.x & 31u) == 0 && downs) atomicAdd(&st->counter[1], (unsigned long long)downs);
+  if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&st->counter[1], (unsigned long long)n);
+}
+
+// Every vertex's result from the numbered ones' (depth, root).
+__global__ void __launch_bounds__(TREE_THREADS) k_tree_leaves(const uint64_t* parent, uint32_t n,
+                                                              const uint2* __restrict__ iw,
+                                                              const uint2* __restrict__ out, SinkPlain sink) {
+  const uint64_t tile_sz = (uint64_t)blockDim.x * TREE_OUT_ITEMS;
+  for (uint64_t tile = (uint64_t)blockIdx.x * tile_sz; tile < n; tile += (uint64_t)gridDim.x * tile_sz) {
+    uint64_t p[TREE_OUT_ITEMS];
+    uint2 w[TREE_OUT_ITEMS], o[TREE_OUT_ITEMS];
+    bool leaf[TREE_OUT_ITEMS];
+#pragma unroll
+    for (int i = 0; i < TREE_OUT_ITEMS; ++i) {
+      const uint64_t v = tile + (uint64_t)i * blockDim.x + threadIdx.x;
+      p[i] = parent_of(parent, v, n);
+      w[i] = v < n ? __ldg(iw + (v >> 5)) : make_uint2(0, 0);
+    }
+#pragma unroll
+    for (int i = 0; i < TREE_OUT_ITEMS; ++i) {
+      const uint64_t v = tile + (uint64_t)i * blockDim.x + threadIdx.x;
+      if (p[i] >= n) p[i] = v;
+      leaf[i] = !((w[i].x >> (v & 31)) & 1u);
+      if (leaf[i] && p[i] != v) w[i] = __ldg(iw + (p[i] >> 5));
+    }
+#pragma unroll
+    for (int i = 0; i < TREE_OUT_ITEMS; ++i) {
+      const uint64_t v = tile + (uint64_t)i * blockDim.x + threadIdx.x;
+      o[i] = make_uint2(0, 0);
+      if (p[i] != v) o[i] = __ldg(out + number_of(w[i], leaf[i] ? (uint32_t)p[i] : (uint32_t)v));
+    }
+#pragma unroll
+    for (int i = 0; i < TREE_OUT_ITEMS; ++i) {
+      const uint64_t v = tile + (uint64_t)i * blockDim.x + threadIdx.x;
+      if (v < n) sink.put((uint32_t)v, o[i].x + (leaf[i] ? 1u : 0u), o[i].y, p[i] == v);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Levels.
+// ---------------------------------------------------------------------------
+// Every ruler's walk to the next ruler or its root.  next.s == 0: the last
+// level's rulers are the one-CTA ranker's.
 template <class L, class N>
-__global__ void __launch_bounds__(TREE_THREADS) k_tree_chase(const typename L::R* __restrict__ rec, uint32_t n,
-                                                             Rulers rl, uint32_t rulers,
-                                                             const uint32_t* __restrict__ inner,
+__global__ void __launch_bounds__(TREE_THREADS) k_tree_chase(const typename L::R* __restrict__ rec, Extent ext,
+                                                             Rulers rl, Extent next_ext,
                                                              const uint32_t* __restrict__ rootel,
                                                              typename N::R* __restrict__ nrec,
                                                              uint32_t* __restrict__ nroot, Rulers nrl,
                                                              uint32_t hop_cap, DevStatus* st) {
+  const uint32_t n = ext.get(), rulers = next_ext.get();
+  if (nrl.s == 0) nrl = cta_rulers(rulers);
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rulers; i += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t id = (uint32_t)i;
     const uint64_t x0 = rl.elem(id);
     uint64_t acc = 0;
     uint32_t next = id, k;
-    if (x0 < n && (!inner || bit_of(inner, (uint32_t)x0))) {
+    if (x0 < n) {  // (the last block's ruler may lie beyond the elements)
       uint32_t x = (uint32_t)x0, hops = 0;
       while (true) {
         const Hop h = L::hop(rec + x);
@@ -159,26 +326,21 @@ __global__ void __launch_bounds__(TREE_THREADS) k_tree_chase(const typename L::R
 }
 
 // Every element's result: its ruler's, or the first ruler's on its path.
-// inner (level 0): the vertices with children are counted for the call's
-// report of its tour's length.
 template <class L, class N, class Sink>
-__global__ void __launch_bounds__(TREE_THREADS) k_tree_propagate(const typename L::R* __restrict__ rec, uint32_t n,
-                                                                 Rulers rl, const uint32_t* __restrict__ inner,
-                                                                 const uint32_t* __restrict__ rootel,
+__global__ void __launch_bounds__(TREE_THREADS) k_tree_propagate(const typename L::R* __restrict__ rec, Extent ext,
+                                                                 Rulers rl, const uint32_t* __restrict__ rootel,
                                                                  const typename N::O* __restrict__ out, Sink sink,
                                                                  DevStatus* st) {
-  uint32_t downs = 0;
+  const uint32_t n = ext.get();
   for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t x = (uint32_t)v;
     Hop h = L::hop(rec + x);
-    const bool in = !inner || bit_of(inner, x);
     if (h.b == x) {
       sink.put(x, L::kEndWeight ? h.w : 0ull, rootel ? __ldg(rootel + x) : x, true);
       continue;
     }
-    if (inner && in) ++downs;
     uint32_t j;
-    if (in && rl.is(x, &j)) {
+    if (rl.is(x, &j)) {
       const Out o = N::out(out + j);
       sink.put(x, o.rank, o.root, false);
       continue;
@@ -203,44 +365,41 @@ __global__ void __launch_bounds__(TREE_THREADS) k_tree_propagate(const typename 
       set_error(st, KASCADE_ERR_CYCLE, x);
     }
   }
-  if (inner) {
-    downs = __reduce_add_sync(0xffffffffu, downs);
-    if ((threadIdx.x & 31u) == 0 && downs) atomicAdd(&st->counter[1], (unsigned long long)downs);
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&st->counter[1], (unsigned long long)n);
-  }
 }
 
 struct TreeLevels {
   int last = 0;
-  uint32_t n[MAX_LEVELS + 1];
+  Extent ext[MAX_LEVELS + 1];
   Rulers rulers[MAX_LEVELS + 1];
 };
 
-TreeLevels plan_tree(uint32_t n, const Params& p) {
+// Levels of n elements, or of as many of them as *count says.
+TreeLevels plan_tree(uint32_t n, const uint32_t* count, const Params& p) {
   TreeLevels lv;
   const uint32_t base = std::max(1u, std::min(p.base_max, TREE_BASE));
-  uint32_t m = n;
   int k = 0;
-  lv.n[0] = n;
-  while (m > base && k < MAX_LEVELS) {
-    const uint32_t s = k == 0 ? (p.spacing_given ? p.spacing_given : TREE_SPACING)
-                              : (p.spacing_deep ? p.spacing_deep : TREE_SPACING);
+  lv.ext[0].cap = n;
+  lv.ext[0].add = count;
+  while (lv.ext[k].cap > base && k < MAX_LEVELS) {
+    const uint32_t given = k == 0 ? p.spacing_given : p.spacing_deep;
+    const uint32_t s = given ? std::max(2u, given) : lv.ext[k].cap > TREE_LARGE ? TREE_SPACING_LARGE : TREE_SPACING;
     lv.rulers[k] = make_rulers(s, salt_for(p.seed, k));
-    m = ruler_count(m, lv.rulers[k]);
-    lv.n[++k] = m;
+    lv.ext[k + 1].cap = ruler_count(lv.ext[k].cap, lv.rulers[k]);
+    lv.ext[k + 1].add = count;
+    lv.ext[k + 1].div = (uint32_t)std::min<uint64_t>((uint64_t)lv.ext[k].div * lv.rulers[k].s, 0xFFFFFFFFu);
+    ++k;
   }
   lv.last = k;
-  lv.rulers[k] = cta_rulers(m);
+  lv.rulers[k].s = 0;
   return lv;
 }
 
 template <class L, class N>
 kascade_status tree_chase(kascade_ctx& ctx, const TreeLevels& lv, int k, const typename L::R* rec,
-                          const uint32_t* inner, const uint32_t* rootel, typename N::R* nrec, uint32_t* nroot,
-                          cudaStream_t s) {
+                          const uint32_t* rootel, typename N::R* nrec, uint32_t* nroot, cudaStream_t s) {
   ProfScope ps(ctx, "chase", s);
-  k_tree_chase<L, N><<<grid_for(ctx, lv.n[k + 1], TREE_THREADS, 8), TREE_THREADS, 0, s>>>(
-      rec, lv.n[k], lv.rulers[k], lv.n[k + 1], inner, rootel, nrec, nroot, lv.rulers[k + 1], hop_cap(lv.rulers[k]),
+  k_tree_chase<L, N><<<grid_for(ctx, lv.ext[k + 1].cap, TREE_THREADS, 8), TREE_THREADS, 0, s>>>(
+      rec, lv.ext[k], lv.rulers[k], lv.ext[k + 1], rootel, nrec, nroot, lv.rulers[k + 1], hop_cap(lv.rulers[k]),
       ctx.d_status);
   KS_CHECK_LAUNCH();
   return KASCADE_OK;
@@ -248,35 +407,35 @@ kascade_status tree_chase(kascade_ctx& ctx, const TreeLevels& lv, int k, const t
 
 template <class L, class N, class Sink>
 kascade_status tree_propagate(kascade_ctx& ctx, const TreeLevels& lv, int k, const typename L::R* rec,
-                              const uint32_t* inner, const uint32_t* rootel, const typename N::O* out,
-                              const Sink& sink, cudaStream_t s) {
+                              const uint32_t* rootel, const typename N::O* out, const Sink& sink, cudaStream_t s) {
   ProfScope ps(ctx, "propagate", s);
-  k_tree_propagate<L, N, Sink><<<grid_for(ctx, lv.n[k], TREE_THREADS, 8), TREE_THREADS, 0, s>>>(
-      rec, lv.n[k], lv.rulers[k], inner, rootel, out, sink, ctx.d_status);
+  k_tree_propagate<L, N, Sink><<<grid_for(ctx, lv.ext[k].cap, TREE_THREADS, 8), TREE_THREADS, 0, s>>>(
+      rec, lv.ext[k], lv.rulers[k], rootel, out, sink, ctx.d_status);
   KS_CHECK_LAUNCH();
   return KASCADE_OK;
 }
 
 // Levels 0..last from level 0's records; there is at least one ruler level.
 template <class L, class N, class SinkN, class Sink>
-kascade_status rank_tree(kascade_ctx& ctx, const TreeLevels& lv, const typename L::R* rec, const uint32_t* inner,
+kascade_status rank_tree(kascade_ctx& ctx, const TreeLevels& lv, const typename L::R* rec, const uint32_t* rootel,
                          const Sink& sink, cudaStream_t s) {
   typename N::R* nrec[MAX_LEVELS + 1] = {};
   uint32_t* nroot[MAX_LEVELS + 1] = {};
   typename N::O* nout[MAX_LEVELS + 1] = {};
   for (int k = 1; k <= lv.last; ++k) {
-    nrec[k] = alloc<typename N::R>(ctx, lv.n[k]);
-    nroot[k] = alloc<uint32_t>(ctx, lv.n[k]);
-    nout[k] = alloc<typename N::O>(ctx, lv.n[k]);
+    const uint64_t cap = lv.ext[k].cap;
+    nrec[k] = alloc<typename N::R>(ctx, cap);
+    nroot[k] = alloc<uint32_t>(ctx, cap);
+    nout[k] = alloc<typename N::O>(ctx, cap);
     if (!nrec[k] || !nroot[k] || !nout[k]) return KASCADE_ERR_OOM;
   }
-  KS_TRY((tree_chase<L, N>(ctx, lv, 0, rec, inner, nullptr, nrec[1], nroot[1], s)));
+  KS_TRY((tree_chase<L, N>(ctx, lv, 0, rec, rootel, nrec[1], nroot[1], s)));
   for (int k = 1; k < lv.last; ++k)
-    KS_TRY((tree_chase<N, N>(ctx, lv, k, nrec[k], nullptr, nroot[k], nrec[k + 1], nroot[k + 1], s)));
-  KS_TRY(rank_trees_one_cta(ctx, nrec[lv.last], nroot[lv.last], lv.n[lv.last], nout[lv.last], s));
+    KS_TRY((tree_chase<N, N>(ctx, lv, k, nrec[k], nroot[k], nrec[k + 1], nroot[k + 1], s)));
+  KS_TRY(rank_trees_one_cta(ctx, nrec[lv.last], nroot[lv.last], lv.ext[lv.last], nout[lv.last], s));
   for (int k = lv.last - 1; k >= 1; --k)
-    KS_TRY((tree_propagate<N, N>(ctx, lv, k, nrec[k], nullptr, nroot[k], nout[k + 1], SinkN{nout[k]}, s)));
-  return tree_propagate<L, N>(ctx, lv, 0, rec, inner, nullptr, nout[1], sink, s);
+    KS_TRY((tree_propagate<N, N>(ctx, lv, k, nrec[k], nroot[k], nout[k + 1], SinkN{nout[k]}, s)));
+  return tree_propagate<L, N>(ctx, lv, 0, rec, rootel, nout[1], sink, s);
 }
 
 }  // namespace
@@ -285,27 +444,47 @@ kascade_status root_forest_impl(kascade_ctx& ctx, const uint64_t* parent, uint32
                                 uint64_t* depth_out, int keep_roots, const Params& p, cudaStream_t s) {
   if (n == 0) return KASCADE_OK;
   const SinkPlain sink{root_out, depth_out, keep_roots};
-  const TreeLevels lv = plan_tree(n, p);
+  uint32_t* count = alloc<uint32_t>(ctx, 1);
+  if (!count) return KASCADE_ERR_OOM;
+  const TreeLevels lv = plan_tree(n, count, p);
   if (lv.last == 0) return rank_arrays_one_cta(ctx, parent, WKind::Unit, nullptr, n, sink, CTA_ROOTING, s);
-  ctx.last_levels.assign(lv.n, lv.n + lv.last + 1);
+  ctx.last_levels.assign(1, n);
+  for (int k = 1; k <= lv.last; ++k) ctx.last_levels.push_back(lv.ext[k].cap);
   const uint32_t words = (uint32_t)(((uint64_t)n + 31) / 32);
+  const uint32_t tiles = (words + WORDS_TILE - 1) / WORDS_TILE;
+  unsigned char* inner = alloc<unsigned char>(ctx, 32ull * words);
+  uint32_t* sums = alloc<uint32_t>(ctx, tiles);
+  uint2* iw = alloc<uint2>(ctx, words);
   uint32_t* rec = alloc<uint32_t>(ctx, n);
-  uint32_t* inner = alloc<uint32_t>(ctx, words);
-  if (!rec || !inner) return KASCADE_ERR_OOM;
+  uint32_t* vert = alloc<uint32_t>(ctx, n);
+  uint2* out = alloc<uint2>(ctx, n);
+  if (!inner || !sums || !iw || !rec || !vert || !out) return KASCADE_ERR_OOM;
   {
     ProfScope ps(ctx, "prepare", s);
-    KS_CUDA(cudaMemsetAsync(inner, 0, sizeof(uint32_t) * (size_t)words, s));
-    const unsigned grid =
-        grid_for(ctx, ((uint64_t)n + TREE_PREP_ITEMS - 1) / TREE_PREP_ITEMS, TREE_THREADS, 8);
-    k_tree_prepare<<<grid, TREE_THREADS, 0, s>>>(parent, n, lv.rulers[0], rec, inner, ctx.d_status);
+    KS_CUDA(cudaMemsetAsync(inner, 0, 32ull * words, s));
+    const unsigned grid = grid_for(ctx, ((uint64_t)n + TREE_PREP_ITEMS - 1) / TREE_PREP_ITEMS, TREE_THREADS, 8);
+    k_tree_inner<<<grid, TREE_THREADS, 0, s>>>(parent, n, inner, ctx.d_status);
+    KS_CHECK_LAUNCH();
+    if (tiles > 1) {
+      k_tree_count<<<tiles, TREE_THREADS, 0, s>>>(inner, words, sums);
+      KS_CHECK_LAUNCH();
+    }
+    k_tree_number<<<tiles, TREE_THREADS, 0, s>>>(inner, words, sums, iw, count);
+    KS_CHECK_LAUNCH();
+    k_tree_records<<<grid, TREE_THREADS, 0, s>>>(parent, n, iw, lv.rulers[0], rec, vert, ctx.d_status);
     KS_CHECK_LAUNCH();
   }
-  return rank_tree<TreeUnit, Tree8, SinkOut8>(ctx, lv, rec, inner, sink, s);
+  KS_TRY((rank_tree<TreeUnit, Tree8, SinkOut8>(ctx, lv, rec, vert, SinkOut8{out}, s)));
+  ProfScope ps(ctx, "leaves", s);
+  const unsigned grid = grid_for(ctx, ((uint64_t)n + TREE_OUT_ITEMS - 1) / TREE_OUT_ITEMS, TREE_THREADS, 8);
+  k_tree_leaves<<<grid, TREE_THREADS, 0, s>>>(parent, n, iw, out, sink);
+  KS_CHECK_LAUNCH();
+  return KASCADE_OK;
 }
 
 kascade_status rank_forest_weighted(kascade_ctx& ctx, const uint64_t* succ, WKind wk, const void* w, uint32_t n,
                                     const SinkPlain& sink, const Params& p, cudaStream_t s) {
-  const TreeLevels lv = plan_tree(n, p);
+  const TreeLevels lv = plan_tree(n, nullptr, p);
   if (lv.last == 0) return rank_arrays_one_cta(ctx, succ, wk, w, n, sink, CTA_TREES, s);
   ctx.last_levels.assign(1, n);
   Level0 l0;  // F16x16, no stamps
