@@ -381,6 +381,7 @@ kascade_status batch_plan_create(int device, const kascade_segment* segs, uint32
   }
   st = status_reset(ctx, s);
   if (st == KASCADE_OK) st = batch_enqueue(ctx, t, in, weights, root_out, rank_out, &opts, s);
+  if (st == KASCADE_OK) st = status_publish(ctx, s);
   cudaGraph_t g = nullptr;
   const cudaError_t ce = cudaStreamEndCapture(s, &g);
   plan->graph = g;
@@ -400,6 +401,7 @@ kascade_status batch_plan_launch(kascade_batch_plan* plan, cudaStream_t s) {
   // the plan's scratch is reused by every launch: order after the previous one
   if (ctx.done_event && ctx.last_stream != s) KS_CUDA(cudaStreamWaitEvent(s, ctx.done_event, 0));
   KS_CUDA(cudaGraphLaunch(plan->exec, s));
+  ctx.published = true;  // by a captured kernel
   cudaEventRecord(ctx.done_event, s);
   ctx.last_stream = s;
   return status_finish(ctx, s);

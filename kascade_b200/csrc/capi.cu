@@ -58,12 +58,13 @@ kascade_status end_call(kascade_ctx* ctx, cudaStream_t s, kascade_status st, con
     // a host-side error: let the enqueued work drain before reporting
     cudaStreamSynchronize(s);
     cudaGetLastError();
+    ctx->status_dirty = true;
     ctx->last_status = st;
     return st;
   }
   if (o && o->async) {
     ctx->async_pending = true;
-    return KASCADE_OK;
+    return status_publish(*ctx, s);
   }
   return status_finish(*ctx, s);
 }

@@ -494,7 +494,7 @@ __global__ void __launch_bounds__(256) k_walk_unreached(const typename F::R* __r
                                                         const uint32_t* __restrict__ hint, uint32_t nseg,
                                                         const uint32_t* __restrict__ plus_one,
                                                         const uint32_t* __restrict__ seg_tour, int keep_roots,
-                                                        DevStatus* st) {
+                                                        DevStatus* st, unsigned long long* status) {
   const uint32_t cnt = min(*ucount, ucap);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
     const uint32_t u = ulist[i];
@@ -546,6 +546,7 @@ __global__ void __launch_bounds__(256) k_walk_unreached(const typename F::R* __r
     __threadfence();
     root_out[u] = base_root;
   }
+  publish_status(st, status);
 }
 
 constexpr uint32_t TILE1 = PT_THREADS * P1_ITEMS, TILE2 = PT_THREADS * P2_ITEMS;
@@ -673,7 +674,7 @@ kascade_status rank_level0_log_as(kascade_ctx& ctx, const Level0& l0, uint32_t n
     ProfScope ps(ctx, "heads", s);
     k_walk_unreached<F><<<ctx.usable_sms() * 4, 256, 0, s>>>(l0.records<F>(), ulist, ucount, ucap, n, limit, t.root,
                                                              t.rank, t.seg_off, t.hint, t.nseg, t.plus_one,
-                                                             t.seg_tour, t.keep_roots, ctx.d_status);
+                                                             t.seg_tour, t.keep_roots, ctx.d_status, status_host(ctx));
     KS_CHECK_LAUNCH();
   }
   return KASCADE_OK;

@@ -5,6 +5,7 @@
 // chase's own write lands in the same 32 B sector it just read.
 #pragma once
 
+#include <cstddef>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -58,7 +59,7 @@ struct __align__(16) PdRec {
 // ---------------------------------------------------------------------------
 struct DevStatus {
   unsigned int code;
-  unsigned int pad;
+  unsigned int blocks;  // of a call's last kernel: done so far
   unsigned long long info;
   // [1]: level 0's size, when only the device knows it; [2], [3]: elements
   // stamped by chains / found stamped (more of the former: two chains met)
@@ -69,6 +70,31 @@ struct DevStatus {
 
 __device__ __forceinline__ void set_error(DevStatus* st, unsigned int code, unsigned long long info) {
   if (atomicCAS(&st->code, 0u, code) == 0u) st->info = info;
+}
+
+// The words of a status that the host reads.
+constexpr uint32_t STATUS_WORDS = 8;
+static_assert(offsetof(DevStatus, work) == STATUS_WORDS * 8 && sizeof(DevStatus) % 8 == 0, "status words");
+
+// The end of a call's last kernel: its last block to finish copies the status
+// to the host's pinned words (host == nullptr: not here) and clears it for the
+// next call.  A call of one launch is then that launch: with a memset ahead of
+// it and a copy behind it 1000 elements took 38.7 us instead of 30.
+// Called by all threads of every block.
+__device__ __forceinline__ void publish_status(DevStatus* st, unsigned long long* host) {
+  if (!host) return;
+  __syncthreads();
+  if (threadIdx.x >= 32u) return;
+  uint32_t last = 1;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (gridDim.x > 1) last = atomicAdd(&st->blocks, 1u) == gridDim.x - 1 ? 1u : 0u;
+    __threadfence();
+  }
+  if (!__shfl_sync(0xffffffffu, last, 0)) return;
+  unsigned long long* w = reinterpret_cast<unsigned long long*>(st);
+  if (threadIdx.x < STATUS_WORDS) *(volatile unsigned long long*)(host + threadIdx.x) = __ldcg(w + threadIdx.x);
+  if (threadIdx.x < sizeof(DevStatus) / 8) __stcg(w + threadIdx.x, 0ull);
 }
 
 // ---------------------------------------------------------------------------

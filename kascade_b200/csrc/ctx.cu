@@ -79,7 +79,24 @@ cudaError_t ensure_device(int device) {
 }
 
 kascade_status status_reset(kascade_ctx& ctx, cudaStream_t s) {
-  KS_CUDA(cudaMemsetAsync(ctx.d_status, 0, sizeof(DevStatus), s));
+  if (ctx.status_dirty) KS_CUDA(cudaMemsetAsync(ctx.d_status, 0, sizeof(DevStatus), s));
+  ctx.status_dirty = true;
+  ctx.published = false;
+  return KASCADE_OK;
+}
+
+unsigned long long* status_host(kascade_ctx& ctx) {
+  ctx.published = true;
+  ctx.status_dirty = false;
+  return ctx.h_pinned;
+}
+
+static __global__ void k_publish_status(DevStatus* st, unsigned long long* host) { publish_status(st, host); }
+
+kascade_status status_publish(kascade_ctx& ctx, cudaStream_t s) {
+  if (ctx.published) return KASCADE_OK;
+  k_publish_status<<<1, 32, 0, s>>>(ctx.d_status, status_host(ctx));
+  KS_CHECK_LAUNCH();
   return KASCADE_OK;
 }
 
@@ -100,12 +117,13 @@ static void collect_times(kascade_ctx& ctx) {
 }
 
 kascade_status status_finish(kascade_ctx& ctx, cudaStream_t s) {
-  cudaError_t e =
-      cudaMemcpyAsync(ctx.h_pinned, ctx.d_status, offsetof(DevStatus, work), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) {
-    ctx.last_status = cuda_status(e);
-    return ctx.last_status;
+  kascade_status ps = status_publish(ctx, s);
+  if (ps == KASCADE_OK) ps = cuda_status(cudaStreamSynchronize(s));
+  ctx.published = false;  // (a call's later kernels are read by another status_finish)
+  if (ps != KASCADE_OK) {
+    ctx.status_dirty = true;
+    ctx.last_status = ps;
+    return ps;
   }
   collect_times(ctx);
   const DevStatus* st = reinterpret_cast<const DevStatus*>(ctx.h_pinned);

@@ -19,6 +19,9 @@ struct kascade_ctx {
   size_t smem_optin = 0;
   ks::DevStatus* d_status = nullptr;
   unsigned long long* h_pinned = nullptr;  // KS_PINNED_WORDS words
+  // the device status: whether a call since its last clearing may have left it
+  // non-zero, and whether the call's last kernel copies it to h_pinned
+  bool status_dirty = false, published = false;
   // scratch arena: blocks are never freed inside a call, so pointers handed
   // out by alloc() stay valid until the next begin_call()
   struct Block {
@@ -93,9 +96,14 @@ T* alloc(kascade_ctx& ctx, size_t count) {
 
 // Status --------------------------------------------------------------------
 kascade_status cuda_status(cudaError_t e);
-// Clear the device status word (stream-ordered).
+// Start a call: the device status is zero (stream-ordered).
 kascade_status status_reset(kascade_ctx& ctx, cudaStream_t s);
-// Synchronise `s`, read the device status word, collect kernel timings.
+// For the launch that ends a call's device work: where its publish_status puts
+// the status.
+unsigned long long* status_host(kascade_ctx& ctx);
+// Copy the status to the host by a launch of its own unless a kernel does.
+kascade_status status_publish(kascade_ctx& ctx, cudaStream_t s);
+// Synchronise `s`, read the status, collect kernel timings.
 kascade_status status_finish(kascade_ctx& ctx, cudaStream_t s);
 // Read one device word into the pinned buffer and wait for it.
 kascade_status read_u32(kascade_ctx& ctx, const uint32_t* dptr, uint32_t* out, cudaStream_t s);

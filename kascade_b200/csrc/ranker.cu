@@ -341,7 +341,8 @@ __global__ void __launch_bounds__(256) k_propagate(const typename F::R* __restri
                                                    const typename F::S* __restrict__ stamp, uint32_t n_out,
                                                    Extent ext, Rulers rl, uint32_t rulers,
                                                    const uint32_t* __restrict__ rootel,
-                                                   const Out* __restrict__ out_next, Sink sink, DevStatus* st) {
+                                                   const Out* __restrict__ out_next, Sink sink, DevStatus* st,
+                                                   unsigned long long* status) {
   __shared__ uint32_t walks[PROP_WALKS];
   __shared__ uint32_t nwalks, nfound;
   if (threadIdx.x == 0) nwalks = nfound = 0;
@@ -405,6 +406,7 @@ __global__ void __launch_bounds__(256) k_propagate(const typename F::R* __restri
   if (threadIdx.x == 0 && nfound) atomicAdd(&st->counter[3], (unsigned long long)nfound);
   for (uint32_t w = threadIdx.x; w < min(nwalks, PROP_WALKS); w += blockDim.x)
     walk_to_result<F>(rec, stamp, walks[w], rl, rootel, out_next, sink, st);
+  publish_status(st, status);
 }
 
 // ---------------------------------------------------------------------------
@@ -469,8 +471,8 @@ struct CtaArrays {
 };
 
 template <class Src, class Sink>
-__global__ void __launch_bounds__(CTA_THREADS, 1) k_rank_cta(Src src, Extent ext, Sink sink, CtaMode mode,
-                                                             DevStatus* st) {
+__device__ __forceinline__ void rank_cta(const Src& src, const Extent& ext, const Sink& sink, CtaMode mode,
+                                         DevStatus* st) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ uint32_t nends, nheads, nstamps;
   const uint32_t n = ext.get();
@@ -744,6 +746,14 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) k_rank_cta(Src src, Extent ext
   }
 }
 
+// status: see publish_status.
+template <class Src, class Sink>
+__global__ void __launch_bounds__(CTA_THREADS, 1) k_rank_cta(Src src, Extent ext, Sink sink, CtaMode mode,
+                                                             DevStatus* st, unsigned long long* status) {
+  rank_cta(src, ext, sink, mode, st);
+  publish_status(st, status);
+}
+
 // ---------------------------------------------------------------------------
 // pointer doubling: double-buffered jump rounds over 16 B records.
 // done bit 0: successor is a root; bit 1: the element is a root.
@@ -884,14 +894,15 @@ kascade_status launch_propagate(kascade_ctx& ctx, const Levels& lv, int k, const
                                 const typename F::S* stamp, uint32_t n_out, const Extent& ext, const Sink& sink,
                                 cudaStream_t s) {
   ProfScope ps(ctx, "propagate", s);
+  unsigned long long* status = k == 0 ? status_host(ctx) : nullptr;
   if (n_out <= (uint64_t)ctx.usable_sms() * 256 * 8 * 4) {
     const unsigned grid = grid_for(ctx, ((uint64_t)n_out + 1) / 2, 256, 8);
     k_propagate<F, Sink, 2><<<grid, 256, 0, s>>>(rec, stamp, n_out, ext, lv.rulers[k], lv.r[k], lv.rootel[k],
-                                                 lv.out[k + 1], sink, ctx.d_status);
+                                                 lv.out[k + 1], sink, ctx.d_status, status);
   } else {
     const unsigned grid = grid_for(ctx, ((uint64_t)n_out + 7) / 8, 256, 8);
     k_propagate<F, Sink, 8><<<grid, 256, 0, s>>>(rec, stamp, n_out, ext, lv.rulers[k], lv.r[k], lv.rootel[k],
-                                                 lv.out[k + 1], sink, ctx.d_status);
+                                                 lv.out[k + 1], sink, ctx.d_status, status);
   }
   KS_CHECK_LAUNCH();
   return KASCADE_OK;
@@ -899,7 +910,7 @@ kascade_status launch_propagate(kascade_ctx& ctx, const Levels& lv, int k, const
 
 template <class Src, class Sink>
 kascade_status launch_rank_cta(kascade_ctx& ctx, const Src& src, const Extent& ext, const Sink& sink,
-                               CtaMode mode, cudaStream_t s) {
+                               CtaMode mode, bool last, cudaStream_t s) {
   static std::atomic<uint64_t> raised{0};  // kernel attributes are per device
   const uint64_t bit = 1ull << (ctx.device & 63);
   if (!(raised.load() & bit)) {
@@ -910,7 +921,8 @@ kascade_status launch_rank_cta(kascade_ctx& ctx, const Src& src, const Extent& e
   ProfScope ps(ctx, "base_case", s);
   // one ruler per thread; a small input's few barriers are cheaper with fewer warps
   const unsigned threads = ext.cap <= 1024 ? 256 : CTA_THREADS;
-  k_rank_cta<Src, Sink><<<1, threads, cta_smem(ext.cap), s>>>(src, ext, sink, mode, ctx.d_status);
+  k_rank_cta<Src, Sink><<<1, threads, cta_smem(ext.cap), s>>>(src, ext, sink, mode, ctx.d_status,
+                                                                last ? status_host(ctx) : nullptr);
   KS_CHECK_LAUNCH();
   return KASCADE_OK;
 }
@@ -1078,21 +1090,21 @@ kascade_status rank_arrays_one_cta(kascade_ctx& ctx, const uint64_t* succ, WKind
   ext.cap = n;
   switch (wk) {
     case WKind::Unit:
-      return launch_rank_cta(ctx, CtaArrays<WUnit>{succ, WUnit{}}, ext, sink, mode, s);
+      return launch_rank_cta(ctx, CtaArrays<WUnit>{succ, WUnit{}}, ext, sink, mode, true, s);
     case WKind::U32:
-      return launch_rank_cta(ctx, CtaArrays<WU32>{succ, WU32{(const uint32_t*)w}}, ext, sink, mode, s);
+      return launch_rank_cta(ctx, CtaArrays<WU32>{succ, WU32{(const uint32_t*)w}}, ext, sink, mode, true, s);
     default:
-      return launch_rank_cta(ctx, CtaArrays<WI64>{succ, WI64{(const int64_t*)w}}, ext, sink, mode, s);
+      return launch_rank_cta(ctx, CtaArrays<WI64>{succ, WI64{(const int64_t*)w}}, ext, sink, mode, true, s);
   }
 }
 
 kascade_status rank_trees_one_cta(kascade_ctx& ctx, const Rec8* rec, const uint32_t* rootel, const Extent& ext,
                                   uint2* out, cudaStream_t s) {
-  return launch_rank_cta(ctx, CtaRecords<F8x8, true>{rec, rootel}, ext, SinkOut8{out}, CTA_TREES, s);
+  return launch_rank_cta(ctx, CtaRecords<F8x8, true>{rec, rootel}, ext, SinkOut8{out}, CTA_TREES, false, s);
 }
 kascade_status rank_trees_one_cta(kascade_ctx& ctx, const Rec* rec, const uint32_t* rootel, const Extent& ext,
                                   Out* out, cudaStream_t s) {
-  return launch_rank_cta(ctx, CtaRecords<F16x16, true>{rec, rootel}, ext, SinkOut{out}, CTA_TREES, s);
+  return launch_rank_cta(ctx, CtaRecords<F16x16, true>{rec, rootel}, ext, SinkOut{out}, CTA_TREES, false, s);
 }
 
 // Doubling for a fixed number of rounds, enough for any list the level can
@@ -1167,7 +1179,7 @@ kascade_status rank_deep(kascade_ctx& ctx, const Levels& lv, cudaStream_t s) {
   const int L = lv.last;
   if (lv.n[L] <= ONE_CTA_MAX) {
     KS_TRY(launch_rank_cta(ctx, CtaRecords<F16x16, true>{lv.rec[L], lv.rootel[L]}, lv.extent(L), SinkOut{lv.out[L]},
-                           CTA_LISTS, s));
+                           CTA_LISTS, false, s));
   } else {
     KS_TRY(pointer_double_level(ctx, lv.rec[L], lv.extent(L), lv.rootel[L], lv.out[L], s));
   }
@@ -1185,7 +1197,7 @@ kascade_status rank_records_as(kascade_ctx& ctx, const Level0& l0, uint32_t n, c
   const typename F::R* rec = l0.records<F>();
   if (n <= p.base_max) {
     ctx.last_levels.assign(1, n);
-    return launch_rank_cta(ctx, CtaRecords<F, false>{rec, nullptr}, ext, sink, CTA_SMALL_TREES, s);
+    return launch_rank_cta(ctx, CtaRecords<F, false>{rec, nullptr}, ext, sink, CTA_SMALL_TREES, true, s);
   }
   Levels lv;
   KS_TRY(plan_levels(ctx, n, heads, p, &lv));

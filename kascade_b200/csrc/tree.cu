@@ -244,7 +244,8 @@ __global__ void __launch_bounds__(TREE_THREADS) k_tree_records(const uint64_t* _
 // Every vertex's result from the numbered ones' (depth, root).
 __global__ void __launch_bounds__(TREE_THREADS) k_tree_leaves(const uint64_t* parent, uint32_t n,
                                                               const uint2* __restrict__ iw,
-                                                              const uint2* __restrict__ out, SinkPlain sink) {
+                                                              const uint2* __restrict__ out, SinkPlain sink,
+                                                              DevStatus* st, unsigned long long* status) {
   const uint64_t tile_sz = (uint64_t)blockDim.x * TREE_OUT_ITEMS;
   for (uint64_t tile = (uint64_t)blockIdx.x * tile_sz; tile < n; tile += (uint64_t)gridDim.x * tile_sz) {
     uint64_t p[TREE_OUT_ITEMS];
@@ -275,6 +276,7 @@ __global__ void __launch_bounds__(TREE_THREADS) k_tree_leaves(const uint64_t* pa
       if (v < n) sink.put((uint32_t)v, o[i].x + (leaf[i] ? 1u : 0u), o[i].y, p[i] == v);
     }
   }
+  publish_status(st, status);
 }
 
 // ---------------------------------------------------------------------------
@@ -330,7 +332,7 @@ template <class L, class N, class Sink>
 __global__ void __launch_bounds__(TREE_THREADS) k_tree_propagate(const typename L::R* __restrict__ rec, Extent ext,
                                                                  Rulers rl, const uint32_t* __restrict__ rootel,
                                                                  const typename N::O* __restrict__ out, Sink sink,
-                                                                 DevStatus* st) {
+                                                                 DevStatus* st, unsigned long long* status) {
   const uint32_t n = ext.get();
   for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t x = (uint32_t)v;
@@ -365,6 +367,7 @@ __global__ void __launch_bounds__(TREE_THREADS) k_tree_propagate(const typename 
       set_error(st, KASCADE_ERR_CYCLE, x);
     }
   }
+  publish_status(st, status);
 }
 
 struct TreeLevels {
@@ -407,10 +410,11 @@ kascade_status tree_chase(kascade_ctx& ctx, const TreeLevels& lv, int k, const t
 
 template <class L, class N, class Sink>
 kascade_status tree_propagate(kascade_ctx& ctx, const TreeLevels& lv, int k, const typename L::R* rec,
-                              const uint32_t* rootel, const typename N::O* out, const Sink& sink, cudaStream_t s) {
+                              const uint32_t* rootel, const typename N::O* out, const Sink& sink, bool last,
+                              cudaStream_t s) {
   ProfScope ps(ctx, "propagate", s);
   k_tree_propagate<L, N, Sink><<<grid_for(ctx, lv.ext[k].cap, TREE_THREADS, 8), TREE_THREADS, 0, s>>>(
-      rec, lv.ext[k], lv.rulers[k], rootel, out, sink, ctx.d_status);
+      rec, lv.ext[k], lv.rulers[k], rootel, out, sink, ctx.d_status, last ? status_host(ctx) : nullptr);
   KS_CHECK_LAUNCH();
   return KASCADE_OK;
 }
@@ -418,7 +422,7 @@ kascade_status tree_propagate(kascade_ctx& ctx, const TreeLevels& lv, int k, con
 // Levels 0..last from level 0's records; there is at least one ruler level.
 template <class L, class N, class SinkN, class Sink>
 kascade_status rank_tree(kascade_ctx& ctx, const TreeLevels& lv, const typename L::R* rec, const uint32_t* rootel,
-                         const Sink& sink, cudaStream_t s) {
+                         const Sink& sink, bool last, cudaStream_t s) {
   typename N::R* nrec[MAX_LEVELS + 1] = {};
   uint32_t* nroot[MAX_LEVELS + 1] = {};
   typename N::O* nout[MAX_LEVELS + 1] = {};
@@ -434,8 +438,8 @@ kascade_status rank_tree(kascade_ctx& ctx, const TreeLevels& lv, const typename 
     KS_TRY((tree_chase<N, N>(ctx, lv, k, nrec[k], nroot[k], nrec[k + 1], nroot[k + 1], s)));
   KS_TRY(rank_trees_one_cta(ctx, nrec[lv.last], nroot[lv.last], lv.ext[lv.last], nout[lv.last], s));
   for (int k = lv.last - 1; k >= 1; --k)
-    KS_TRY((tree_propagate<N, N>(ctx, lv, k, nrec[k], nroot[k], nout[k + 1], SinkN{nout[k]}, s)));
-  return tree_propagate<L, N>(ctx, lv, 0, rec, rootel, nout[1], sink, s);
+    KS_TRY((tree_propagate<N, N>(ctx, lv, k, nrec[k], nroot[k], nout[k + 1], SinkN{nout[k]}, false, s)));
+  return tree_propagate<L, N>(ctx, lv, 0, rec, rootel, nout[1], sink, last, s);
 }
 
 }  // namespace
@@ -474,10 +478,10 @@ kascade_status root_forest_impl(kascade_ctx& ctx, const uint64_t* parent, uint32
     k_tree_records<<<grid, TREE_THREADS, 0, s>>>(parent, n, iw, lv.rulers[0], rec, vert, ctx.d_status);
     KS_CHECK_LAUNCH();
   }
-  KS_TRY((rank_tree<TreeUnit, Tree8, SinkOut8>(ctx, lv, rec, vert, SinkOut8{out}, s)));
+  KS_TRY((rank_tree<TreeUnit, Tree8, SinkOut8>(ctx, lv, rec, vert, SinkOut8{out}, false, s)));
   ProfScope ps(ctx, "leaves", s);
   const unsigned grid = grid_for(ctx, ((uint64_t)n + TREE_OUT_ITEMS - 1) / TREE_OUT_ITEMS, TREE_THREADS, 8);
-  k_tree_leaves<<<grid, TREE_THREADS, 0, s>>>(parent, n, iw, out, sink);
+  k_tree_leaves<<<grid, TREE_THREADS, 0, s>>>(parent, n, iw, out, sink, ctx.d_status, status_host(ctx));
   KS_CHECK_LAUNCH();
   return KASCADE_OK;
 }
@@ -492,7 +496,7 @@ kascade_status rank_forest_weighted(kascade_ctx& ctx, const uint64_t* succ, WKin
   if (!rec) return KASCADE_ERR_OOM;
   l0.rec = rec;
   KS_TRY(prepare_arrays(ctx, succ, wk, w, n, l0, lv.rulers[0], s));
-  return rank_tree<Tree16, Tree16, SinkOut>(ctx, lv, rec, nullptr, sink, s);
+  return rank_tree<Tree16, Tree16, SinkOut>(ctx, lv, rec, nullptr, sink, true, s);
 }
 
 }  // namespace ks
