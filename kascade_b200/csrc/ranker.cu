@@ -928,7 +928,9 @@ kascade_status launch_rank_cta(kascade_ctx& ctx, const Src& src, const Extent& e
 }
 
 // Ruler spacing of a deeper level of n elements: levels of equal spacing down
-// to the one-CTA size, as many as cost least.  A level costs its longest
+// to `target`, as many as cost least.  The target is three quarters of what
+// one CTA ranks: its time grows with its elements (2^20: 87382 elements to
+// 12484 153 us, to 9710 138; 2e6: 200 and 193, 4e6: 278 and 285).  A level costs its longest
 // chain, spacing x ln(rulers) dependent hops, and launches worth ~36 hops
 // (measured on L2-resident levels: 0.25 us a hop, ~9 us for a level's chase
 // and propagation launches).
@@ -1154,7 +1156,7 @@ kascade_status plan_levels(kascade_ctx& ctx, uint32_t n, const Heads& heads, con
   while (m > base && k < max_levels) {
     const uint32_t sp = k == 0           ? p.spacing0
                         : p.spacing_deep ? p.spacing_deep
-                                         : deep_spacing(m, ONE_CTA_MAX - extra);
+                                         : deep_spacing(m, ONE_CTA_MAX * 3 / 4 - extra);
     lv->rulers[k] = k == 0 ? level0_rulers(p) : make_rulers(sp, salt_for(p.seed, k));
     lv->r[k] = m = ruler_count(m, lv->rulers[k]);
     lv->n[k + 1] = m + extra;
