@@ -32,12 +32,14 @@ __global__ void __launch_bounds__(256) k_gen_forest(uint64_t n, ks_perm perm, ui
 
 // list_ranking.cpp:60-80
 __global__ void __launch_bounds__(256) k_initial_state(const uint64_t* __restrict__ succ, uint64_t n,
-                                                       uint64_t* __restrict__ root, int64_t* __restrict__ rank) {
+                                                       uint64_t* __restrict__ root, int64_t* __restrict__ rank,
+                                                       DevStatus* st, unsigned long long* status) {
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t s = succ[i];
     root[i] = s;
     rank[i] = (s == i) ? 0 : 1;
   }
+  publish_status(st, status);
 }
 
 __global__ void __launch_bounds__(256) k_fill_u64(uint64_t* __restrict__ a, uint64_t n, uint64_t v) {
@@ -121,7 +123,7 @@ kascade_status gen_forest(uint64_t n, uint64_t seed, uint32_t kind, uint64_t blo
 kascade_status initial_state(kascade_ctx& ctx, const uint64_t* succ, uint64_t n, uint64_t* root, int64_t* rank,
                              cudaStream_t s) {
   if (n == 0) return KASCADE_OK;
-  k_initial_state<<<grid_for(ctx, n, 256, 8), 256, 0, s>>>(succ, n, root, rank);
+  k_initial_state<<<grid_for(ctx, n, 256, 8), 256, 0, s>>>(succ, n, root, rank, ctx.d_status, status_host(ctx));
   KS_CHECK_LAUNCH();
   return KASCADE_OK;
 }
