@@ -47,7 +47,12 @@ constexpr uint32_t SUB_SHIFT = 13;  // 2^13 elements per sub-window (second pass
 constexpr uint32_t SUB = 1u << SUB_SHIFT;
 constexpr uint32_t SUBS = WIN / SUB;    // sub-windows per window
 constexpr uint32_t MAX_BUCKETS = 4096;  // windows for 2^32 elements
-constexpr uint32_t DIRECT_MAX = 1u << 22;  // one partition pass up to this size (512 sub-windows)
+// One partition pass up to this size: 2e7 elements in runs of 64 890 -> 810 us,
+// a batch of 2e7 records 1554 -> 1471, lists of random order 985 -> 1019 at
+// 1.6e7 and equal at 3.3e7 (a tile's entries then fall into as many
+// sub-windows, and neither way of writing them coalesces).  A call that asks
+// for this path takes two passes from 2^22 elements on.
+constexpr uint32_t DIRECT_MAX = 1u << 25, DIRECT_MAX_FORCED = 1u << 22;
 static_assert(DIRECT_MAX / SUB <= MAX_BUCKETS, "sub-windows per pass");
 constexpr uint32_t CURSOR_STRIDE = 8;   // one 32 B sector per cursor (spreads the atomics)
 constexpr uint32_t PT_THREADS = 256;    // partition: threads per block
@@ -624,7 +629,7 @@ kascade_status rank_level0_log_as(kascade_ctx& ctx, const Level0& l0, uint32_t n
   // Up to DIRECT_MAX elements the log goes straight to the sub-windows;
   // larger ones in two passes, windows (part), then sub-windows into the log's
   // memory when it is large enough (the log is dead by then).
-  const bool direct = limit <= DIRECT_MAX;
+  const bool direct = limit <= (p.level0_mode == 2 ? DIRECT_MAX_FORCED : DIRECT_MAX);
   const uint32_t nsub = (uint32_t)(((uint64_t)limit + SUB - 1) / SUB);
   const uint64_t part2_need = (uint64_t)nsub * SUB;
   LogEnt* part = alloc<LogEnt>(ctx, direct ? std::max<uint64_t>(part2_need, 1) : (uint64_t)nb1 * WIN);
