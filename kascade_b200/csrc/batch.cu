@@ -2,17 +2,13 @@
 // ranked together.
 //
 // The instances arrive concatenated (instance-local indices) with a segment
-// table.  They are laid out in one record space so that a single ruler chase
-// -- one persistent launch with one device work queue -- serves every
-// instance:
-//   list element g (concatenated position)  -> record g
-//   forest vertex g                         -> record g (its up edge / tour end;
-//                                              a leaf's down and up edge in one)
-//   down edges of all forests (F of them)   -> records total_n .. total_n+F-1
-//                                              (a leaf's or a root's: a dead self loop)
-// The ruler spacing is one per batch, from the size class of its record count
-// (the context's size-class table, filled by the autotuner).
-// Roots are reported relative to their own instance.
+// table.  One pass over them numbers the lists' elements densely in one space
+// and the forests' vertices in another; all lists are then ranked as one
+// (rank_records) and all forests as one (tree.cu): a single ruler chase, one
+// launch with one work queue, serves every list.  Ruler spacing and block size
+// are one per batch, from the size class of its list elements (the context's
+// size-class table, filled by the autotuner).  Outputs go straight to the
+// instances' places, roots relative to their own instance.
 #include <algorithm>
 #include <cstring>
 #include <new>
@@ -22,30 +18,37 @@
 
 namespace ks {
 
-kascade_status batch_tours(kascade_ctx& ctx, const uint64_t* fpar, uint32_t F, const uint32_t* fd, const uint32_t* foff,
-                           const uint32_t* fhint, uint32_t nf, uint32_t down_base, const Level0& l0,
-                           const Rulers& rl, uint32_t* leaf_out, Heads* heads, cudaStream_t s);
-
 namespace {
 
-constexpr uint32_t ITEM = 4096;  // elements per work item
+constexpr uint32_t TILE = 4096;  // positions per tile, and per entry of a segment hint
 constexpr int BP_THREADS = 256;
-constexpr int BP_PER = ITEM / BP_THREADS;
+constexpr int BP_PER = 8;  // positions a thread has in flight
 
-struct __align__(16) DSeg {
-  unsigned long long off;
-  uint32_t size;
-  uint32_t kind;
-  uint32_t fd;  // forests: base in the compact forest vertex space
-  uint32_t pad;
+// (first element in its kind's dense numbering, kind) of every instance.
+struct BatchIn {
+  const uint64_t* in;
+  SegMap pos;  // the instances in the caller's arrays (no delta)
+  const uint2* kinds;
 };
 
-struct __align__(16) Item {
-  uint32_t seg;
-  uint32_t start;
-  uint32_t count;
-  uint32_t pad;
-};
+// The segment hints of an element range: hint[k] is the segment of element
+// 4096 k, the last entry that of the last element.
+__global__ void __launch_bounds__(BP_THREADS) k_batch_hints(const uint32_t* __restrict__ base, uint32_t n,
+                                                            uint32_t elems, uint32_t entries,
+                                                            uint32_t* __restrict__ hint) {
+  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < entries; k += gridDim.x * blockDim.x) {
+    const uint32_t x = (uint32_t)min((uint64_t)k * TILE, (uint64_t)elems - 1);
+    uint32_t lo = 0, hi = n;  // the last j with base[j] <= x
+    while (hi - lo > 1) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (base[mid] <= x)
+        lo = mid;
+      else
+        hi = mid;
+    }
+    hint[k] = lo;
+  }
+}
 
 struct BWUnit {
   __device__ __forceinline__ uint32_t operator()(uint64_t) const { return 1u; }
@@ -55,191 +58,161 @@ struct BWU32 {
   __device__ __forceinline__ uint32_t operator()(uint64_t g) const { return __ldcs(p + g); }
 };
 
+// List elements' records, and forest vertices' parents, from the caller's
+// arrays.  Streaming; a tile inside one instance (hints alike) looks its
+// segment up once.
 template <class F, class W>
-__global__ void __launch_bounds__(BP_THREADS) k_batch_prepare(const Item* __restrict__ items, uint32_t nitems,
-                                                              const DSeg* __restrict__ segs,
-                                                              const uint64_t* __restrict__ in, W w, Rulers rl,
+__global__ void __launch_bounds__(BP_THREADS) k_batch_prepare(BatchIn b, uint32_t total, W w, Rulers rl,
                                                               typename F::R* __restrict__ rec,
                                                               typename F::S* __restrict__ stamp,
-                                                              uint64_t* __restrict__ fpar, DevStatus* st) {
-  for (uint32_t it = blockIdx.x; it < nitems; it += gridDim.x) {
-    const Item item = items[it];
-    const DSeg sg = segs[item.seg];
-    if (sg.kind == KASCADE_SEG_LIST) {
-      uint32_t wv[BP_PER];
-      unsigned long long lv[BP_PER];
-      // every load of the item first (independent, all in flight together),
-      // then the checks
+                                                              uint32_t* __restrict__ fpar, DevStatus* st) {
+  constexpr uint32_t STEP = BP_THREADS * BP_PER;
+  const uint32_t steps = (uint32_t)(((uint64_t)total + STEP - 1) / STEP);
+  for (uint32_t t = blockIdx.x; t < steps; t += gridDim.x) {
+    const uint64_t g0 = (uint64_t)t * STEP;
+    uint64_t v[BP_PER];
+    uint32_t wv[BP_PER];
 #pragma unroll
-      for (int i = 0; i < BP_PER; ++i) {
-        const uint32_t k = item.start + i * BP_THREADS + threadIdx.x;
-        lv[i] = 0;
-        wv[i] = 0;
-        if (k < item.start + item.count) {
-          const uint64_t g = sg.off + k;
-          lv[i] = __ldcs(reinterpret_cast<const unsigned long long*>(in) + g);
-          wv[i] = w(g);
-        }
-      }
-      uint64_t bad = ~0ull;  // the first element whose successor is out of its instance
+    for (int i = 0; i < BP_PER; ++i) {
+      const uint64_t g = g0 + i * BP_THREADS + threadIdx.x;
+      v[i] = g < total ? __ldcs(b.in + g) : 0;
+      wv[i] = g < total ? w(g) : 0u;
+    }
+    // (a step lies within one tile of the hints)
+    const uint32_t j0 = __ldg(b.pos.hint + (uint32_t)(g0 / TILE)), j1 = __ldg(b.pos.hint + (uint32_t)(g0 / TILE) + 1);
+    uint32_t j = j0, off = 0, size = 0;
+    uint2 kind = make_uint2(0, 0);
+    auto segment = [&]() {
+      off = __ldg(b.pos.base + j);
+      size = __ldg(b.pos.base + j + 1) - off;
+      kind = __ldg(b.kinds + j);
+    };
+    if (j0 == j1) segment();
 #pragma unroll
-      for (int i = 0; i < BP_PER; ++i) {
-        const uint32_t k = item.start + i * BP_THREADS + threadIdx.x;
-        if (k >= item.start + item.count) continue;
-        const uint64_t g = sg.off + k;
-        unsigned long long loc = lv[i];
-        if (loc >= sg.size) {
-          if (bad == ~0ull) bad = g;
-          loc = k;
-        }
-        const uint32_t b = (uint32_t)(sg.off + loc);
-        uint32_t j;
-        F::put(rec + g, loc == k ? 0u : wv[i], b, rl.is(b, &j));  // a root's weight is no part of any rank
-        if (stamp) F::clear(stamp + g);
+    for (int i = 0; i < BP_PER; ++i) {
+      const uint64_t g = g0 + i * BP_THREADS + threadIdx.x;
+      if (g >= total) continue;
+      if (j0 != j1) {
+        j = b.pos.find((uint32_t)g);
+        segment();
       }
-      if (bad != ~0ull) set_error(st, KASCADE_ERR_OUT_OF_RANGE, bad);
-    } else {
-      unsigned long long pv[BP_PER];
-#pragma unroll
-      for (int i = 0; i < BP_PER; ++i) {
-        const uint32_t k = item.start + i * BP_THREADS + threadIdx.x;
-        pv[i] = k < item.start + item.count ? __ldcs(reinterpret_cast<const unsigned long long*>(in) + sg.off + k) : 0;
+      const uint32_t k = (uint32_t)g - off;
+      if (v[i] >= size) {
+        set_error(st, KASCADE_ERR_OUT_OF_RANGE, g);
+        v[i] = k;
       }
-      uint64_t bad = ~0ull;
-#pragma unroll
-      for (int i = 0; i < BP_PER; ++i) {
-        const uint32_t k = item.start + i * BP_THREADS + threadIdx.x;
-        if (k >= item.start + item.count) continue;
-        unsigned long long par = pv[i];
-        if (par >= sg.size) {
-          if (bad == ~0ull) bad = sg.off + k;
-          par = k;
-        }
-        __stcs(reinterpret_cast<unsigned long long*>(fpar) + sg.fd + k, (unsigned long long)(sg.fd + par));
+      const uint32_t x = kind.x + k, y = kind.x + (uint32_t)v[i];
+      if (kind.y == KASCADE_SEG_LIST) {
+        uint32_t q;
+        F::put(rec + x, x == y ? 0u : wv[i], y, rl.is(y, &q));  // a root's weight is no part of any rank
+        if (stamp) F::clear(stamp + x);
+      } else {
+        __stcs(fpar + x, y);
       }
-      if (bad != ~0ull) set_error(st, KASCADE_ERR_OUT_OF_RANGE, bad);
     }
   }
 }
+static_assert(TILE % (BP_THREADS * BP_PER) == 0, "a step lies within a tile");
 
-// The list ends among the inputs (counted when a plan is made).
-__global__ void __launch_bounds__(BP_THREADS) k_count_ends(const Item* __restrict__ items, uint32_t nitems,
-                                                           const DSeg* __restrict__ segs,
-                                                           const uint64_t* __restrict__ in,
-                                                           uint32_t* __restrict__ count) {
+// The list ends and roots among the inputs (counted when a plan is made).
+__global__ void __launch_bounds__(BP_THREADS) k_count_ends(BatchIn b, uint32_t total, uint32_t* __restrict__ count) {
   uint32_t c = 0;
-  for (uint32_t it = blockIdx.x; it < nitems; it += gridDim.x) {
-    const Item item = items[it];
-    const uint64_t off = segs[item.seg].off;
-    for (uint32_t k = item.start + threadIdx.x; k < item.start + item.count; k += BP_THREADS)
-      c += in[off + k] == k ? 1u : 0u;
-  }
+  for (uint64_t g = (uint64_t)blockIdx.x * BP_THREADS + threadIdx.x; g < total; g += (uint64_t)gridDim.x * BP_THREADS)
+    c += b.in[g] == g - __ldg(b.pos.base + b.pos.find((uint32_t)g)) ? 1u : 0u;
   c = __reduce_add_sync(0xffffffffu, c);
   if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, c);
 }
 
 }  // namespace
 
-// Host tables of one batch: built from the segment list, uploaded into the
-// context's arena.  Kept apart from the launches so that a plan can upload
-// them once and capture only the device work.
+// Tables of one batch: what the host knows of the segments in one upload, the
+// hints filled in on the device.  Kept apart from the launches so that a plan
+// can upload them once and capture only the device work.
 struct BatchTables {
-  std::vector<DSeg> dsegs;
-  std::vector<Item> items;
-  std::vector<uint32_t> fd, foff, hint, fhint, tour;  // tour: bit j set when instance j is a forest
-  std::vector<unsigned long long> seg_off;
-  uint64_t total = 0, F = 0;
-  uint32_t nseg = 0, nf = 0, M = 0;
+  std::vector<uint32_t> host;
+  uint64_t total = 0;
+  uint32_t nseg = 0, L = 0, F = 0;  // list elements, forest vertices
+  uint32_t nl = 0, nf = 0;
   // device copies
-  DSeg* d_segs = nullptr;
-  Item* d_items = nullptr;
-  uint32_t *d_fd = nullptr, *d_foff = nullptr, *d_hint = nullptr, *d_fhint = nullptr, *d_tour = nullptr;
-  unsigned long long* d_off = nullptr;
+  SegMap pos, lists, forests;
+  const uint2* kinds = nullptr;
 };
 
 kascade_status batch_build_tables(const kascade_segment* segs, uint32_t nseg, uint64_t total, BatchTables& t) {
   t = BatchTables{};
   t.nseg = nseg;
   t.total = total;
-  t.dsegs.resize(nseg);
-  t.seg_off.resize(nseg);
-  t.tour.assign((nseg + 31) / 32, 0u);
-  t.items.reserve(total / ITEM + nseg);
-  uint64_t expect = 0;
+  uint64_t expect = 0, F = 0;
   for (uint32_t i = 0; i < nseg; ++i) {
     const kascade_segment& g = segs[i];
     if (g.offset != expect || g.size > 0x7FFFFFFFull || (g.kind != KASCADE_SEG_LIST && g.kind != KASCADE_SEG_FOREST))
       return KASCADE_ERR_INVALID_ARG;
     expect += g.size;
-    const bool forest = g.kind == KASCADE_SEG_FOREST;
-    t.dsegs[i] = DSeg{g.offset, (uint32_t)g.size, g.kind, (uint32_t)t.F, 0};
-    t.seg_off[i] = g.offset;
-    if (forest) {
-      t.fd.push_back((uint32_t)t.F);
-      t.foff.push_back((uint32_t)g.offset);
-      t.tour[i >> 5] |= 1u << (i & 31);
-      t.F += g.size;
+    if (g.kind == KASCADE_SEG_FOREST) {
+      F += g.size;
+      ++t.nf;
+    } else {
+      ++t.nl;
     }
-    for (uint64_t st = 0; st < g.size; st += ITEM)
-      t.items.push_back(Item{i, (uint32_t)st, (uint32_t)std::min<uint64_t>(ITEM, g.size - st), 0});
   }
   if (expect != total) return KASCADE_ERR_INVALID_ARG;
-  if (total + t.F > MAX_ELEMS) return KASCADE_ERR_TOO_LARGE;
-  t.nf = (uint32_t)t.fd.size();
-  t.fd.push_back((uint32_t)t.F);
-  t.hint.resize((size_t)((total + 4095) / 4096) + 1);
-  {
-    uint32_t j = 0;
-    for (size_t k = 0; k < t.hint.size(); ++k) {
-      const uint64_t x = (uint64_t)k * 4096;
-      while (j + 1 < nseg && t.seg_off[j + 1] <= x) ++j;
-      t.hint[k] = j;
-    }
+  if (total + F > MAX_ELEMS) return KASCADE_ERR_TOO_LARGE;
+  t.F = (uint32_t)F;
+  t.L = (uint32_t)(total - F);
+  // kinds (pairs), positions, lists (base, delta), forests (base, delta)
+  t.host.resize(2ull * nseg + (nseg + 1) + (2ull * t.nl + 1) + (2ull * t.nf + 1));
+  uint32_t* kinds = t.host.data();
+  uint32_t* pos = kinds + 2ull * nseg;
+  uint32_t* base[2] = {pos + nseg + 1, pos + nseg + 1 + 2ull * t.nl + 1};  // lists, forests
+  uint32_t* delta[2] = {base[0] + t.nl + 1, base[1] + t.nf + 1};
+  uint32_t at[2] = {0, 0}, q[2] = {0, 0};
+  for (uint32_t i = 0; i < nseg; ++i) {
+    const int f = segs[i].kind == KASCADE_SEG_FOREST;
+    kinds[2ull * i] = at[f];
+    kinds[2ull * i + 1] = segs[i].kind;
+    pos[i] = (uint32_t)segs[i].offset;
+    base[f][q[f]] = at[f];
+    delta[f][q[f]] = (uint32_t)segs[i].offset - at[f];
+    ++q[f];
+    at[f] += (uint32_t)segs[i].size;
   }
-  // per 4096 compact forest vertices: the forest holding the first (and one
-  // entry past the last block, so a block's search range is [fhint[k], fhint[k+1]])
-  t.fhint.resize((size_t)((t.F + 4095) / 4096) + 1);
-  {
-    uint32_t j = 0;
-    for (size_t k = 0; k < t.fhint.size(); ++k) {
-      const uint64_t c = (uint64_t)k * 4096;
-      while (j + 1 < t.nf && t.fd[j + 1] <= c) ++j;
-      t.fhint[k] = j;
-    }
-  }
-  t.M = (uint32_t)(total + t.F);
+  pos[nseg] = (uint32_t)total;
+  base[0][t.nl] = t.L;
+  base[1][t.nf] = t.F;
   return KASCADE_OK;
 }
 
 kascade_status batch_upload_tables(kascade_ctx& ctx, BatchTables& t, cudaStream_t s) {
-  t.d_segs = alloc<DSeg>(ctx, t.nseg);
-  t.d_items = alloc<Item>(ctx, t.items.size() + 1);
-  t.d_fd = alloc<uint32_t>(ctx, t.fd.size());
-  t.d_foff = alloc<uint32_t>(ctx, t.foff.size() + 1);
-  t.d_off = alloc<unsigned long long>(ctx, t.nseg);
-  t.d_hint = alloc<uint32_t>(ctx, t.hint.size());
-  t.d_fhint = alloc<uint32_t>(ctx, t.fhint.size());
-  t.d_tour = alloc<uint32_t>(ctx, t.tour.size());
-  if (!t.d_segs || !t.d_items || !t.d_fd || !t.d_foff || !t.d_off || !t.d_hint || !t.d_fhint || !t.d_tour)
-    return KASCADE_ERR_OOM;
-  KS_CUDA(cudaMemcpyAsync(t.d_segs, t.dsegs.data(), sizeof(DSeg) * t.nseg, cudaMemcpyHostToDevice, s));
-  KS_CUDA(cudaMemcpyAsync(t.d_items, t.items.data(), sizeof(Item) * t.items.size(), cudaMemcpyHostToDevice, s));
-  KS_CUDA(cudaMemcpyAsync(t.d_fd, t.fd.data(), sizeof(uint32_t) * t.fd.size(), cudaMemcpyHostToDevice, s));
-  if (t.nf) {
-    KS_CUDA(cudaMemcpyAsync(t.d_foff, t.foff.data(), sizeof(uint32_t) * t.nf, cudaMemcpyHostToDevice, s));
-    KS_CUDA(cudaMemcpyAsync(t.d_tour, t.tour.data(), sizeof(uint32_t) * t.tour.size(), cudaMemcpyHostToDevice, s));
-  }
-  KS_CUDA(cudaMemcpyAsync(t.d_off, t.seg_off.data(), sizeof(unsigned long long) * t.nseg, cudaMemcpyHostToDevice, s));
-  KS_CUDA(cudaMemcpyAsync(t.d_hint, t.hint.data(), sizeof(uint32_t) * t.hint.size(), cudaMemcpyHostToDevice, s));
-  KS_CUDA(cudaMemcpyAsync(t.d_fhint, t.fhint.data(), sizeof(uint32_t) * t.fhint.size(), cudaMemcpyHostToDevice, s));
-  return KASCADE_OK;
+  uint32_t* d = alloc<uint32_t>(ctx, t.host.size());
+  if (!d) return KASCADE_ERR_OOM;
+  KS_CUDA(cudaMemcpyAsync(d, t.host.data(), sizeof(uint32_t) * t.host.size(), cudaMemcpyHostToDevice, s));
+  t.kinds = reinterpret_cast<const uint2*>(d);
+  const uint32_t* pos = d + 2ull * t.nseg;
+  const uint32_t* lists = pos + t.nseg + 1;
+  const uint32_t* forests = lists + 2ull * t.nl + 1;
+  auto map = [&](SegMap* m, const uint32_t* base, uint32_t n, uint64_t elems) {
+    m->base = base;
+    m->delta = base + n + 1;
+    m->n = n;
+    if (elems == 0) return KASCADE_OK;
+    const uint32_t entries = (uint32_t)((elems + TILE - 1) / TILE) + 1;
+    uint32_t* hint = alloc<uint32_t>(ctx, entries);
+    if (!hint) return KASCADE_ERR_OOM;
+    m->hint = hint;
+    k_batch_hints<<<grid_for(ctx, entries, BP_THREADS, 8), BP_THREADS, 0, s>>>(base, n, (uint32_t)elems, entries, hint);
+    KS_CHECK_LAUNCH();
+    return KASCADE_OK;
+  };
+  KS_TRY(map(&t.pos, pos, t.nseg, t.total));
+  KS_TRY(map(&t.lists, lists, t.nl, t.L));
+  return map(&t.forests, forests, t.nf, t.F);
 }
 
-// The batch's parameters: ruler spacing and block size from the class of its
-// record count (one chase launch serves every instance).
-Params batch_params(const kascade_ctx& ctx, const BatchTables& t, const kascade_opts* opts) {
-  Params p = make_params(ctx, opts, t.M);
-  if (!(opts && opts->ruler_spacing)) p.spacing0 = std::max(2u, ctx.class_spacing[ctx.class_of(t.M)]);
+// A batch's parameters: ruler spacing and block size from the class of its
+// record count.
+Params batch_params(const kascade_ctx& ctx, uint64_t records, const kascade_opts* opts) {
+  Params p = make_params(ctx, opts, records);
+  if (!(opts && opts->ruler_spacing)) p.spacing0 = std::max(2u, ctx.class_spacing[ctx.class_of(records)]);
   p.algorithm = KASCADE_ALGO_SPARSE_RULING_SET;
   return p;
 }
@@ -249,25 +222,19 @@ Params batch_params(const kascade_ctx& ctx, const BatchTables& t, const kascade_
 // CUDA graph.
 kascade_status batch_enqueue(kascade_ctx& ctx, const BatchTables& t, const uint64_t* in, const uint32_t* weights,
                              uint64_t* root_out, uint64_t* rank_out, const kascade_opts* opts, cudaStream_t s) {
-  const uint32_t M = t.M;
-  const Params p = batch_params(ctx, t, opts);
+  const Params p = batch_params(ctx, t.L, opts);
   Level0 l0;
-  KS_TRY(alloc_level0(ctx, plan_level0(p, M, weights ? WKind::U32 : WKind::Unit), M, &l0));
+  KS_TRY(alloc_level0(ctx, plan_level0(p, t.L, weights ? WKind::U32 : WKind::Unit), t.L, &l0));
   const Rulers rl = level0_rulers(p);
-  uint64_t* fpar = alloc<uint64_t>(ctx, t.F + 1);
-  // forest leaves by output position: their rank is one less than their depth
-  const uint64_t leaf_words = t.F ? (t.total + 31) / 32 : 0;
-  uint32_t* leaf_out = leaf_words ? alloc<uint32_t>(ctx, leaf_words) : nullptr;
-  if (!fpar || (leaf_words && !leaf_out)) return KASCADE_ERR_OOM;
-  if (leaf_out) KS_CUDA(cudaMemsetAsync(leaf_out, 0, sizeof(uint32_t) * leaf_words, s));
+  uint32_t* fpar = alloc<uint32_t>(ctx, t.F);
+  if (!fpar) return KASCADE_ERR_OOM;
   {
     ProfScope ps(ctx, "batch_prepare", s);
-    const uint32_t items = (uint32_t)t.items.size();
-    const unsigned grid = (unsigned)std::min<uint64_t>(items, (uint64_t)ctx.usable_sms() * 8);
+    const unsigned grid = grid_for(ctx, (t.total + BP_PER - 1) / BP_PER, BP_THREADS, 8);
     auto prepare = [&](auto f, auto w) {
       using F = decltype(f);
-      k_batch_prepare<F><<<grid, BP_THREADS, 0, s>>>(t.d_items, items, t.d_segs, in, w, rl, l0.records<F>(),
-                                                     l0.stamps<F>(), fpar, ctx.d_status);
+      k_batch_prepare<F><<<grid, BP_THREADS, 0, s>>>(BatchIn{in, t.pos, t.kinds}, (uint32_t)t.total, w, rl,
+                                                     l0.records<F>(), l0.stamps<F>(), fpar, ctx.d_status);
     };
     if (l0.fmt == Format::F8x16)
       prepare(F8x16{}, BWU32{weights});
@@ -283,14 +250,13 @@ kascade_status batch_enqueue(kascade_ctx& ctx, const BatchTables& t, const uint6
       prepare(F16x16{}, BWUnit{});
     KS_CHECK_LAUNCH();
   }
-  Heads heads;
-  KS_TRY(batch_tours(ctx, fpar, (uint32_t)t.F, t.d_fd, t.d_foff, t.d_fhint, t.nf, (uint32_t)t.total, l0, rl,
-                     leaf_out, &heads, s));
-  SinkBatch sink{root_out, rank_out, (uint32_t)t.total, reinterpret_cast<const uint64_t*>(t.d_off), t.d_hint, t.nseg,
-                 leaf_out, t.F ? t.d_tour : nullptr};
-  Extent ext;
-  ext.cap = M;
-  return rank_records(ctx, l0, M, ext, heads, sink, p, s);
+  KS_TRY(root_forests(ctx, fpar, t.F, SinkBatch{root_out, rank_out, t.forests}, t.L == 0, p, s));
+  ctx.last_levels.assign(1, 0);
+  // (trees among the lists of a small batch are ranked, as in a small call)
+  const CtaMode mode = t.total + t.F > ONE_CTA_TREES ? CTA_LISTS : CTA_SMALL_TREES;
+  KS_TRY(rank_records(ctx, l0, t.L, SinkBatch{root_out, rank_out, t.lists}, mode, p, s));
+  ctx.last_levels[0] = t.total;
+  return KASCADE_OK;
 }
 
 kascade_status rank_batch_impl(kascade_ctx& ctx, const kascade_segment* segs, uint32_t nseg, const uint64_t* in,
@@ -310,14 +276,15 @@ static kascade_status plan_admits(kascade_ctx& ctx, const BatchTables& t, const 
   uint32_t* count = alloc<uint32_t>(ctx, 1);
   if (!count) return KASCADE_ERR_OOM;
   KS_CUDA(cudaMemsetAsync(count, 0, sizeof(uint32_t), s));
-  const unsigned grid = (unsigned)std::min<uint64_t>(t.items.size(), (uint64_t)ctx.usable_sms() * 8);
-  k_count_ends<<<grid, BP_THREADS, 0, s>>>(t.d_items, (uint32_t)t.items.size(), t.d_segs, in, count);
+  k_count_ends<<<grid_for(ctx, t.total, BP_THREADS, 8), BP_THREADS, 0, s>>>(BatchIn{in, t.pos, t.kinds},
+                                                                            (uint32_t)t.total, count);
   KS_CHECK_LAUNCH();
   uint32_t ends = 0;
   KS_TRY(read_u32(ctx, count, &ends, s));
-  const uint64_t rulers = t.M / batch_params(ctx, t, opts).spacing0;
+  const uint64_t records = t.total + t.F;
+  const uint64_t rulers = records / batch_params(ctx, records, opts).spacing0;
   const uint64_t most = rulers * 3 / 2 + 65536;
-  return ends + rulers > std::min<uint64_t>(most, t.M) ? KASCADE_ERR_UNSUPPORTED : KASCADE_OK;
+  return ends + rulers > std::min<uint64_t>(most, records) ? KASCADE_ERR_UNSUPPORTED : KASCADE_OK;
 }
 
 // ---------------------------------------------------------------------------

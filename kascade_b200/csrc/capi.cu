@@ -80,9 +80,7 @@ kascade_status rank_list_generic(kascade_ctx& ctx, const uint64_t* succ, WKind w
     if (n <= p.base_max) return rank_arrays_one_cta(ctx, succ, wk, w, (uint32_t)n, sink, CTA_SMALL_TREES, s);
     KS_TRY(alloc_level0(ctx, plan_level0(p, n, wk), n, &l0));
     KS_TRY(prepare_arrays(ctx, succ, wk, w, (uint32_t)n, l0, level0_rulers(p), s));
-    Extent ext;
-    ext.cap = (uint32_t)n;
-    return rank_records(ctx, l0, (uint32_t)n, ext, Heads{}, sink, p, s);
+    return rank_records(ctx, l0, (uint32_t)n, sink, CTA_SMALL_TREES, p, s);
   }
   return rank_forest_weighted(ctx, succ, wk, w, (uint32_t)n, sink, p, s);
 }

@@ -124,14 +124,11 @@ __device__ __forceinline__ void log_append(bool emit, uint32_t x, uint32_t id, u
 // chains 7.27 / 7.30 / 7.41 / 7.48 ms; two or four chains per thread are
 // slower).
 template <class F>
-__global__ void __launch_bounds__(512) k_chase_log(const typename F::R* __restrict__ rec, Extent ext, Rulers rl,
-                                                   uint32_t rulers, Heads heads, NextLevel nx,
+__global__ void __launch_bounds__(512) k_chase_log(const typename F::R* __restrict__ rec, uint32_t n, Rulers rl,
+                                                   uint32_t r, NextLevel nx,
                                                    uint32_t* __restrict__ work, LogEnt* __restrict__ log, uint32_t* __restrict__ chunk_fill,
                                                    uint32_t* __restrict__ chunk_cursor, uint32_t nchunks,
                                                    uint32_t hop_cap, DevStatus* st) {
-  const uint32_t n = ext.get();
-  const uint32_t r = rulers + heads.get();
-  if (nx.rl.s == 0) nx.rl = cta_rulers(r);
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t lt = lanemask_lt();
   const uint32_t first = gridDim.x * blockDim.x;  // ids from here on are handed out by the counter
@@ -141,12 +138,9 @@ __global__ void __launch_bounds__(512) k_chase_log(const typename F::R* __restri
   bool act = false, own = false;  // own: x is the chain's first element
   auto begin = [&](uint32_t i) {
     id = i;
-    const uint64_t x0 = i < rulers ? rl.elem(i) : __ldg(heads.elem + (i - rulers));
-    uint32_t j;
+    const uint64_t x0 = rl.elem(i);
     if (x0 >= n) {
       nx.put(i, 0, i);  // the last block's ruler, beyond the elements
-    } else if (i >= rulers && rl.is((uint32_t)x0, &j)) {
-      nx.put(i, 0, j);  // a head that is a ruler itself
     } else {
       x = (uint32_t)x0;
       h = F::hop(rec + x);
@@ -260,8 +254,7 @@ __device__ uint32_t block_exclusive_scan(uint32_t* v, uint32_t m) {
 //     is resolved on the way: rank = rank(ruler) - distance, root =
 //     root(ruler), from the rulers' results of the recursion.  A log chunk
 //     holds the entries of a few hundred chains, so most of these lookups
-//     hit L1.  Entries of elements at or above `limit` (tour down edges: no
-//     output) are dropped
+//     hit L1
 //   otherwise (second pass): tiles inside one window's region, buckets are
 //     its SUBS sub-windows
 // More entries than a bucket holds means some element was logged twice.
@@ -379,24 +372,19 @@ __global__ void __launch_bounds__(PT_THREADS, BLOCKS) k_partition(const LogEnt* 
 // (element, root, rank) are read in order and placed in shared memory by
 // element, then the sub-window's outputs are written densely.  Elements
 // without an entry were reached by no chain: their root output becomes
-// NOT_REACHED and they join the unreached list.  A batch's roots are written
-// relative to their instance, depths modulo 2^32.  keep_roots: a root's rank
-// output stays as it is (its root output already names it).
+// NOT_REACHED and they join the unreached list.  seg: a batch's outputs.
+// keep_roots: a root's rank output stays as it is (its root output already
+// names it).
 __global__ void __launch_bounds__(FIN_THREADS, 2) k_place(const LogEnt* __restrict__ part2,
                                                             const uint32_t* __restrict__ cursor2, uint32_t nb,
                                                             uint32_t limit, uint64_t* __restrict__ root_out,
                                                             uint64_t* __restrict__ rank_out,
                                                             uint32_t* __restrict__ ulist,
                                                             uint32_t* __restrict__ ucount, uint32_t ucap,
-                                                            const uint64_t* __restrict__ seg_off,
-                                                            const uint32_t* __restrict__ hint, uint32_t nseg,
-                                                            const uint32_t* __restrict__ plus_one,
-                                                            const uint32_t* __restrict__ seg_tour, int keep_roots,
-                                                            DevStatus* st) {
+                                                            SegMap seg, int keep_roots, DevStatus* st) {
   extern __shared__ __align__(16) unsigned char smraw[];
   unsigned long long* rank_s = reinterpret_cast<unsigned long long*>(smraw);  // SUB entries
   uint32_t* root_s = reinterpret_cast<uint32_t*>(rank_s + SUB);               // SUB entries
-  __shared__ uint32_t plus_s[SUB / 32];                                       // the sub-window's plus_one words
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t items = nb * SUBS;
   for (uint32_t it = blockIdx.x; it < items; it += gridDim.x) {
@@ -405,9 +393,6 @@ __global__ void __launch_bounds__(FIN_THREADS, 2) k_place(const LogEnt* __restri
     const uint32_t len = min(SUB, limit - lo);
     const uint32_t cnt = min(__ldcg(cursor2 + (uint64_t)it * CURSOR_STRIDE), SUB);
     for (uint32_t i = threadIdx.x; i < SUB; i += FIN_THREADS) root_s[i] = NO_ROOT;
-    // lo is a multiple of SUB: the sub-window's bits are whole words
-    if (plus_one)
-      for (uint32_t i = threadIdx.x; i < (len + 31) / 32; i += FIN_THREADS) plus_s[i] = __ldg(plus_one + (lo >> 5) + i);
     __syncthreads();
     const LogEnt* src = part2 + (uint64_t)it * SUB;
     for (uint32_t g = 0; g < SUB / FIN_THREADS; g += FIN_GROUP) {
@@ -430,18 +415,14 @@ __global__ void __launch_bounds__(FIN_THREADS, 2) k_place(const LogEnt* __restri
       }
     }
     __syncthreads();
-    // a batch: the instance holding this thread's first element, its offset
-    // and the next instance's; a thread's elements only move forward
-    uint32_t jseg = 0;
-    unsigned long long cur_off = 0, next_off = ~0ull;
-    bool depths = false;
-    if (seg_off) {
-      const uint32_t x0 = lo + threadIdx.x;
-      jseg = __ldg(hint + (x0 >> 12));
-      while (jseg + 1 < nseg && __ldg(seg_off + jseg + 1) <= x0) ++jseg;
-      cur_off = __ldg(seg_off + jseg);
-      next_off = jseg + 1 < nseg ? __ldg(seg_off + jseg + 1) : ~0ull;
-      if (seg_tour) depths = (__ldg(seg_tour + (jseg >> 5)) >> (jseg & 31)) & 1u;
+    // a batch: the segment holding this thread's first element, its base and
+    // the next one's; a thread's elements only move forward
+    uint32_t jseg = 0, cur_base = 0, delta = 0, next_base = 0xFFFFFFFFu;
+    if (seg.n && threadIdx.x < len) {
+      jseg = seg.find(lo + threadIdx.x);
+      cur_base = __ldg(seg.base + jseg);
+      delta = __ldg(seg.delta + jseg);
+      next_base = __ldg(seg.base + jseg + 1);
     }
     for (uint32_t i0 = 0; i0 < len; i0 += FIN_THREADS) {
       const uint32_t i = i0 + threadIdx.x;
@@ -449,20 +430,16 @@ __global__ void __launch_bounds__(FIN_THREADS, 2) k_place(const LogEnt* __restri
       if (i < len) {
         const uint32_t r = root_s[i];
         un = r == NO_ROOT;
-        if (seg_off) {
-          while (lo + i >= next_off) {
-            ++jseg;
-            cur_off = next_off;
-            next_off = jseg + 1 < nseg ? __ldg(seg_off + jseg + 1) : ~0ull;
-            if (seg_tour) depths = (__ldg(seg_tour + (jseg >> 5)) >> (jseg & 31)) & 1u;
-          }
+        while (seg.n && lo + i >= next_base) {  // (the last segment ends where the elements do)
+          ++jseg;
+          cur_base = next_base;
+          delta = __ldg(seg.delta + jseg);
+          next_base = __ldg(seg.base + jseg + 1);
         }
-        const unsigned long long ibase = un ? 0ull : cur_off;
-        __stcs(reinterpret_cast<unsigned long long*>(root_out) + lo + i,
-               un ? NOT_REACHED : (unsigned long long)r - ibase);
-        unsigned long long k = un ? 0ull : rank_s[i];
-        if (depths) k = (uint32_t)k + ((plus_s[i >> 5] >> (i & 31)) & 1u);
-        if (!(keep_roots && (un || r == lo + i))) __stcs(reinterpret_cast<unsigned long long*>(rank_out) + lo + i, k);
+        const uint32_t g = lo + i + delta;
+        __stcs(reinterpret_cast<unsigned long long*>(root_out) + g, un ? NOT_REACHED : (unsigned long long)(r - cur_base));
+        const unsigned long long k = un ? 0ull : rank_s[i];
+        if (!(keep_roots && (un || r == lo + i))) __stcs(reinterpret_cast<unsigned long long*>(rank_out) + g, k);
       }
       const uint32_t m = __ballot_sync(FULL, un);
       if (m == 0u) continue;
@@ -485,33 +462,25 @@ __global__ void __launch_bounds__(FIN_THREADS, 2) k_place(const LogEnt* __restri
 // element with outputs: one the place step wrote (root output not
 // NOT_REACHED) or one another walker finished.  Walkers write the rank,
 // fence, then the root, and readers load the root, fence, then the rank, so a
-// root seen set comes with its rank.  Elements at or above `limit` (tour down
-// edges) have no outputs and are walked through.  Roots already relative to
-// their instance stay so (a walker and the element it stops at share an
-// instance); a list end's root is made relative here.  keep_roots: a root's
-// rank output is the caller's, its rank 0.
+// root seen set comes with its rank.  Roots already relative to their instance
+// stay so (a walker and the element it stops at share an instance); a list
+// end's root is made relative here.  keep_roots: a root's rank output is the
+// caller's, its rank 0.
 template <class F>
 __global__ void __launch_bounds__(256) k_walk_unreached(const typename F::R* __restrict__ rec,
                                                         const uint32_t* __restrict__ ulist,
-                                                        const uint32_t* __restrict__ ucount, uint32_t ucap, uint32_t n,
-                                                        uint32_t limit, uint64_t* root_out, uint64_t* rank_out,
-                                                        const uint64_t* __restrict__ seg_off,
-                                                        const uint32_t* __restrict__ hint, uint32_t nseg,
-                                                        const uint32_t* __restrict__ plus_one,
-                                                        const uint32_t* __restrict__ seg_tour, int keep_roots,
-                                                        DevStatus* st, unsigned long long* status) {
-  const uint32_t cnt = min(*ucount, ucap);
+                                                        const uint32_t* __restrict__ ucount, uint32_t n,
+                                                        uint64_t* root_out, uint64_t* rank_out, SegMap seg,
+                                                        int keep_roots, DevStatus* st, unsigned long long* status) {
+  const uint32_t cnt = min(*ucount, n);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
     const uint32_t u = ulist[i];
-    uint64_t off = 0;
-    bool depths = false;
-    if (seg_off) {
-      uint32_t j = __ldg(hint + (u >> 12));
-      while (j + 1 < nseg && __ldg(seg_off + j + 1) <= u) ++j;
-      off = __ldg(seg_off + j);
-      if (seg_tour) depths = (__ldg(seg_tour + (j >> 5)) >> (j & 31)) & 1u;
+    uint32_t base = 0, delta = 0;
+    if (seg.n) {
+      const uint32_t j = seg.find(u);
+      base = __ldg(seg.base + j);
+      delta = __ldg(seg.delta + j);
     }
-    auto extra = [&](uint32_t x) -> uint64_t { return depths ? (__ldg(plus_one + (x >> 5)) >> (x & 31)) & 1u : 0u; };
     uint64_t acc = 0;
     uint32_t y = u, mark = u, hops = 0;
     unsigned long long base_root = NOT_REACHED;
@@ -520,7 +489,7 @@ __global__ void __launch_bounds__(256) k_walk_unreached(const typename F::R* __r
       const Hop h = F::hop(rec + y);
       acc += h.w;
       if (h.b == y) {  // the list's end
-        base_root = y - off;
+        base_root = y - base;
         break;
       }
       y = h.b;
@@ -529,14 +498,12 @@ __global__ void __launch_bounds__(256) k_walk_unreached(const typename F::R* __r
         ok = false;
         break;
       }
-      if (y < limit) {
-        base_root = __ldcg(reinterpret_cast<const unsigned long long*>(root_out) + y);
-        if (base_root != NOT_REACHED) {
-          __threadfence();
-          if (base_root + off != y || !keep_roots)
-            acc += __ldcg(reinterpret_cast<const unsigned long long*>(rank_out) + y) - extra(y);
-          break;
-        }
+      const uint32_t g = y + delta;
+      base_root = __ldcg(reinterpret_cast<const unsigned long long*>(root_out) + g);
+      if (base_root != NOT_REACHED) {
+        __threadfence();
+        if (base_root + base != y || !keep_roots) acc += __ldcg(reinterpret_cast<const unsigned long long*>(rank_out) + g);
+        break;
       }
       if (y == mark) {
         set_error(st, KASCADE_ERR_CYCLE, u);
@@ -547,9 +514,10 @@ __global__ void __launch_bounds__(256) k_walk_unreached(const typename F::R* __r
       if ((hops & (hops - 1)) == 0) mark = y;
     }
     if (!ok) continue;
-    if (!(keep_roots && base_root + off == u)) rank_out[u] = (depths ? (uint32_t)acc : acc) + extra(u);
+    const uint32_t g = u + delta;
+    if (!(keep_roots && base_root + base == u)) rank_out[g] = acc;
     __threadfence();
-    root_out[u] = base_root;
+    root_out[g] = base_root;
   }
   publish_status(st, status);
 }
@@ -591,18 +559,17 @@ struct Log {
 };
 
 template <class F>
-kascade_status rank_level0_log_as(kascade_ctx& ctx, const Level0& l0, uint32_t n, const Extent& ext,
-                                  const Heads& heads, const LogTarget& t, const Params& p, cudaStream_t s) {
+kascade_status rank_level0_log_as(kascade_ctx& ctx, const Level0& l0, uint32_t n, const LogTarget& t, const Params& p,
+                                  cudaStream_t s) {
   Levels lv;
-  KS_TRY(plan_levels(ctx, n, heads, p, &lv));
+  KS_TRY(plan_levels(ctx, n, p, &lv));
   const uint32_t r = lv.n[1];
   const uint32_t block = p.block;
   const unsigned grid = chase_grid<F>(ctx, r, block);
   const uint64_t warps = (uint64_t)grid * (block / 32);
   Log log;
   log.nchunks = (uint32_t)(((uint64_t)n + LOG_CHUNK - 1) / LOG_CHUNK + warps + 1);
-  const uint32_t limit = t.limit < n ? t.limit : n;
-  const uint32_t nb = (uint32_t)(((uint64_t)limit + WIN - 1) / WIN);
+  const uint32_t nb = (uint32_t)(((uint64_t)n + WIN - 1) / WIN);
   const uint32_t nb1 = nb ? nb : 1;
   const uint64_t cursor_words = (uint64_t)nb1 * (SUBS + 1) * CURSOR_STRIDE;
   log.ent = alloc<LogEnt>(ctx, (uint64_t)log.nchunks * LOG_CHUNK);
@@ -619,8 +586,8 @@ kascade_status rank_level0_log_as(kascade_ctx& ctx, const Level0& l0, uint32_t n
   log.fill = cursor1 + cursor_words;
   {
     ProfScope ps(ctx, "chase", s);
-    k_chase_log<F><<<grid, block, 0, s>>>(l0.records<F>(), ext, lv.rulers[0], lv.r[0], lv.heads,
-                                          next_level(lv, 1), &ctx.d_status->work[0], log.ent,
+    k_chase_log<F><<<grid, block, 0, s>>>(l0.records<F>(), n, lv.rulers[0], r, next_level(lv, 1),
+                                          &ctx.d_status->work[0], log.ent,
                                           log.fill, log.cursor, log.nchunks, hop_cap(lv.rulers[0]), ctx.d_status);
     KS_CHECK_LAUNCH();
   }
@@ -629,8 +596,8 @@ kascade_status rank_level0_log_as(kascade_ctx& ctx, const Level0& l0, uint32_t n
   // Up to DIRECT_MAX elements the log goes straight to the sub-windows;
   // larger ones in two passes, windows (part), then sub-windows into the log's
   // memory when it is large enough (the log is dead by then).
-  const bool direct = limit <= (p.level0_mode == 2 ? DIRECT_MAX_FORCED : DIRECT_MAX);
-  const uint32_t nsub = (uint32_t)(((uint64_t)limit + SUB - 1) / SUB);
+  const bool direct = n <= (p.level0_mode == 2 ? DIRECT_MAX_FORCED : DIRECT_MAX);
+  const uint32_t nsub = (uint32_t)(((uint64_t)n + SUB - 1) / SUB);
   const uint64_t part2_need = (uint64_t)nsub * SUB;
   LogEnt* part = alloc<LogEnt>(ctx, direct ? std::max<uint64_t>(part2_need, 1) : (uint64_t)nb1 * WIN);
   LogEnt* part2 = direct                                                ? part
@@ -643,7 +610,7 @@ kascade_status rank_level0_log_as(kascade_ctx& ctx, const Level0& l0, uint32_t n
     const uint32_t tiles = (log.nchunks + TILE1 / LOG_CHUNK - 1) / (TILE1 / LOG_CHUNK);
     const size_t smem = TILE1 * sizeof(LogEnt) + 2 * sizeof(uint32_t) * std::max(nsub, 1u);
     k_part1<<<(unsigned)std::min<uint64_t>(tiles, (uint64_t)ctx.usable_sms() * P1_BLOCKS), PT_THREADS, smem, s>>>(
-        log.ent, log.fill, log.nchunks, lv.out[1], limit, SUB_SHIFT, nsub, part, cursor2, log.cursor, ctx.d_status);
+        log.ent, log.fill, log.nchunks, lv.out[1], n, SUB_SHIFT, nsub, part, cursor2, log.cursor, ctx.d_status);
     KS_CHECK_LAUNCH();
   } else {
     const size_t smem1 = TILE1 * sizeof(LogEnt) + 2 * sizeof(uint32_t) * nb1;
@@ -652,34 +619,32 @@ kascade_status rank_level0_log_as(kascade_ctx& ctx, const Level0& l0, uint32_t n
       ProfScope ps(ctx, "resolve", s);
       const uint32_t tiles1 = (log.nchunks + TILE1 / LOG_CHUNK - 1) / (TILE1 / LOG_CHUNK);
       k_part1<<<(unsigned)std::min<uint64_t>(tiles1, (uint64_t)ctx.usable_sms() * P1_BLOCKS), PT_THREADS, smem1, s>>>(
-          log.ent, log.fill, log.nchunks, lv.out[1], limit, WIN_SHIFT, nb, part, cursor1, log.cursor, ctx.d_status);
+          log.ent, log.fill, log.nchunks, lv.out[1], n, WIN_SHIFT, nb, part, cursor1, log.cursor, ctx.d_status);
       KS_CHECK_LAUNCH();
     }
     const uint32_t tiles2 = nb * (WIN / TILE2);
     if (tiles2) {
       ProfScope ps(ctx, "partition", s);
       k_part2<<<(unsigned)std::min<uint64_t>(tiles2, (uint64_t)ctx.usable_sms() * P2_BLOCKS), PT_THREADS, smem2, s>>>(
-          part, cursor1, 0, nullptr, limit, 0, nb, part2, cursor2, nullptr, ctx.d_status);
+          part, cursor1, 0, nullptr, n, 0, nb, part2, cursor2, nullptr, ctx.d_status);
       KS_CHECK_LAUNCH();
     }
   }
   // the first pass's source or output is dead by now: it holds the unreached list
   uint32_t* ulist = reinterpret_cast<uint32_t*>(direct ? log.ent : part);
-  const uint32_t ucap = limit;
   {
     ProfScope ps(ctx, "place", s);
     const uint32_t items = nb * SUBS;
     const size_t smem = SUB * (sizeof(unsigned long long) + sizeof(uint32_t));
     k_place<<<(unsigned)std::max<uint64_t>(1, std::min<uint64_t>(items, (uint64_t)ctx.usable_sms() * 2)),
-                FIN_THREADS, smem, s>>>(part2, cursor2, nb, limit, t.root, t.rank, ulist, ucount, ucap, t.seg_off,
-                                        t.hint, t.nseg, t.plus_one, t.seg_tour, t.keep_roots, ctx.d_status);
+                FIN_THREADS, smem, s>>>(part2, cursor2, nb, n, t.root, t.rank, ulist, ucount, n, t.seg, t.keep_roots,
+                                        ctx.d_status);
     KS_CHECK_LAUNCH();
   }
   {
     ProfScope ps(ctx, "heads", s);
-    k_walk_unreached<F><<<ctx.usable_sms() * 4, 256, 0, s>>>(l0.records<F>(), ulist, ucount, ucap, n, limit, t.root,
-                                                             t.rank, t.seg_off, t.hint, t.nseg, t.plus_one,
-                                                             t.seg_tour, t.keep_roots, ctx.d_status, status_host(ctx));
+    k_walk_unreached<F><<<ctx.usable_sms() * 4, 256, 0, s>>>(l0.records<F>(), ulist, ucount, n, t.root, t.rank, t.seg,
+                                                             t.keep_roots, ctx.d_status, status_host(ctx));
     KS_CHECK_LAUNCH();
   }
   return KASCADE_OK;
@@ -687,11 +652,11 @@ kascade_status rank_level0_log_as(kascade_ctx& ctx, const Level0& l0, uint32_t n
 
 }  // namespace
 
-kascade_status rank_level0_log(kascade_ctx& ctx, const Level0& l0, uint32_t n, const Extent& ext, const Heads& heads,
-                               const LogTarget& t, const Params& p, cudaStream_t s) {
+kascade_status rank_level0_log(kascade_ctx& ctx, const Level0& l0, uint32_t n, const LogTarget& t, const Params& p,
+                               cudaStream_t s) {
   // records of 32-bit weights are alike with and without 64-bit stamps
-  if (l0.fmt == Format::F16x16) return rank_level0_log_as<F16x16>(ctx, l0, n, ext, heads, t, p, s);
-  return rank_level0_log_as<F8x16>(ctx, l0, n, ext, heads, t, p, s);
+  if (l0.fmt == Format::F16x16) return rank_level0_log_as<F16x16>(ctx, l0, n, t, p, s);
+  return rank_level0_log_as<F8x16>(ctx, l0, n, t, p, s);
 }
 
 }  // namespace ks

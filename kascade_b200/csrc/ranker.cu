@@ -182,23 +182,17 @@ __global__ void __launch_bounds__(256) k_prepare_tma(const uint64_t* __restrict_
 // record is asked for as soon as its index is known, before the element at
 // hand is stamped.
 //
-// head_base: where level k >= 1 keeps its heads (level 0: heads.elem lists
-// them).  A head's own element is stamped at distance 0.  limit: stamps of
-// elements below it are counted; propagation counts the elements it finds
-// stamped, and fewer than stamps made mean that two chains met.  hop_cap: a
-// chain this long looks for a cycle ahead.
+// Stamps are counted; propagation counts the elements it finds stamped, and
+// fewer than stamps made mean that two chains met.  hop_cap: a chain this long
+// looks for a cycle ahead.
 // ---------------------------------------------------------------------------
 constexpr int CHASE_REFILL = 8;  // idle lanes worth a refill
 
 template <class F>
-__global__ void __launch_bounds__(512) k_chase(const typename F::R* rec, typename F::S* stamp, Extent ext, Rulers rl,
-                                               uint32_t rulers, Heads heads, uint32_t head_base,
-                                               const uint32_t* __restrict__ rootel, NextLevel nx,
-                                               uint32_t* __restrict__ work, uint32_t lanes, uint32_t limit,
-                                               uint32_t hop_cap, DevStatus* st) {
-  const uint32_t n = ext.get();
-  const uint32_t r = rulers + heads.get();
-  if (nx.rl.s == 0) nx.rl = cta_rulers(r);
+__global__ void __launch_bounds__(512) k_chase(const typename F::R* rec, typename F::S* stamp, uint32_t n, Rulers rl,
+                                               uint32_t r, const uint32_t* __restrict__ rootel, NextLevel nx,
+                                               uint32_t* __restrict__ work, uint32_t lanes, uint32_t hop_cap,
+                                               DevStatus* st) {
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
   const uint32_t warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -206,26 +200,18 @@ __global__ void __launch_bounds__(512) k_chase(const typename F::R* rec, typenam
   uint32_t id = 0, x = 0, hops = 0, stamps = 0;
   uint64_t acc = 0;
   Hop h{0, 0, false};             // the record of x, asked for
-  bool act = false, own = false;  // own: x is the chain's first element and a ruler (not stamped)
+  bool act = false, own = false;  // own: x is the chain's ruler (not stamped)
   auto begin = [&](uint32_t i) {
     id = i;
-    uint64_t x0;
-    if (i < rulers)
-      x0 = rl.elem(i);
-    else
-      x0 = rootel ? head_base + (i - rulers) : __ldg(heads.elem + (i - rulers));
-    uint32_t j;
+    const uint64_t x0 = rl.elem(i);
     if (x0 >= n) {
       nx.put(i, 0, i);  // the last block's ruler, beyond the elements
-    } else if (i >= rulers && rl.is((uint32_t)x0, &j) && j < rulers) {
-      nx.put(i, 0, j);  // a head that is a ruler itself
     } else {
       x = (uint32_t)x0;
       h = F::hop(rec + x);
       acc = 0;
       hops = 0;
-      own = i < rulers;
-      act = true;
+      act = own = true;
     }
   };
   if (lane < lanes && warp * lanes + lane < r) begin(warp * lanes + lane);
@@ -256,7 +242,7 @@ __global__ void __launch_bounds__(512) k_chase(const typename F::R* rec, typenam
     if (!F::kInPlace && !stop) h = F::hop(rec + y);
     if (!end && !own) {
       F::stamp(stamp + x, id, acc, at);
-      stamps += x < limit ? 1u : 0u;
+      ++stamps;
     }
     if (F::kInPlace && !stop) h = F::hop(rec + y);
     if (stop) {  // (a list's end is not stamped: any number of chains may end there)
@@ -338,8 +324,7 @@ __device__ __forceinline__ void walk_to_result(const typename F::R* __restrict__
 
 template <class F, class Sink, int ITEMS>
 __global__ void __launch_bounds__(256) k_propagate(const typename F::R* __restrict__ rec,
-                                                   const typename F::S* __restrict__ stamp, uint32_t n_out,
-                                                   Extent ext, Rulers rl, uint32_t rulers,
+                                                   const typename F::S* __restrict__ stamp, uint32_t n, Rulers rl,
                                                    const uint32_t* __restrict__ rootel,
                                                    const Out* __restrict__ out_next, Sink sink, DevStatus* st,
                                                    unsigned long long* status) {
@@ -347,17 +332,16 @@ __global__ void __launch_bounds__(256) k_propagate(const typename F::R* __restri
   __shared__ uint32_t nwalks, nfound;
   if (threadIdx.x == 0) nwalks = nfound = 0;
   __syncthreads();
-  n_out = min(n_out, ext.get());  // records exist up to here
   const uint32_t stride = gridDim.x * blockDim.x;
   const uint64_t pol = l2_keep_policy();
   uint32_t stamped = 0;
-  for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x * ITEMS + threadIdx.x; base < n_out;
+  for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x * ITEMS + threadIdx.x; base < n;
        base += (uint64_t)stride * ITEMS) {
     Stamp sv[ITEMS];
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
       const uint64_t x = base + (uint64_t)i * blockDim.x;
-      if (x < n_out) sv[i] = F::get_stream(stamp + x);
+      if (x < n) sv[i] = F::get_stream(stamp + x);
     }
     // every ruler's or stamped element's result, all loads in flight together
     // (they would otherwise wait behind the previous element's stores)
@@ -367,9 +351,9 @@ __global__ void __launch_bounds__(256) k_propagate(const typename F::R* __restri
     for (int i = 0; i < ITEMS; ++i) {
       const uint64_t x = base + (uint64_t)i * blockDim.x;
       ov[i] = Out{0, 0, 0};
-      if (x >= n_out) continue;
+      if (x >= n) continue;
       uint32_t id;
-      if (rl.is((uint32_t)x, &id) && id < rulers) {  // (a head's index may lie past the last block)
+      if (rl.is((uint32_t)x, &id)) {
         sv[i].dist = 0;
         found |= 1u << i;
       } else if (sv[i].id != TAG_UNREACHED) {
@@ -382,7 +366,7 @@ __global__ void __launch_bounds__(256) k_propagate(const typename F::R* __restri
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
       const uint64_t x = base + (uint64_t)i * blockDim.x;
-      if (x >= n_out) continue;
+      if (x >= n) continue;
       if ((found >> i) & 1u) {
         // a result whose root is the element itself: it is a ruler and a root
         sink.put((uint32_t)x, ov[i].rank - sv[i].dist, ov[i].root, !rootel && ov[i].root == (uint32_t)x);
@@ -456,14 +440,14 @@ struct CtaRecords {
   }
   __device__ __forceinline__ uint32_t root_of(uint32_t x) const { return rootel ? __ldg(rootel + x) : x; }
 };
-template <class W>
+template <class W, class I = uint64_t>
 struct CtaArrays {
   static constexpr bool kEndWeight = false, kFlagged = false;
-  const uint64_t* succ;
+  const I* succ;
   W w;
   __device__ __forceinline__ void load(uint32_t x, uint64_t* a, uint32_t* b, bool* ruler) const {
     *ruler = false;
-    const unsigned long long s = __ldcg(reinterpret_cast<const unsigned long long*>(succ) + x);
+    const uint64_t s = __ldcg(succ + x);
     *a = w(x);
     *b = s > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)s;  // beyond any element: found out of range
   }
@@ -868,10 +852,10 @@ int chase_occupancy(uint32_t block) {
 // L2 serves dependent hops of this many resident warps at full speed.
 constexpr uint64_t CHASE_SPREAD_WARPS_PER_SM = 32;
 
-// Level k's chase.  limit: the elements whose results are wanted.
+// Level k's chase.
 template <class F>
 kascade_status launch_chase(kascade_ctx& ctx, const Levels& lv, int k, const typename F::R* rec, typename F::S* stamp,
-                            const Extent& ext, uint32_t limit, uint32_t block, cudaStream_t s) {
+                            uint32_t block, cudaStream_t s) {
   const uint32_t r = lv.n[k + 1];
   const uint64_t wpb = block / 32;
   const uint64_t max_grid = (uint64_t)ctx.usable_sms() * chase_occupancy<F>(block);
@@ -880,9 +864,8 @@ kascade_status launch_chase(kascade_ctx& ctx, const Levels& lv, int k, const typ
   const uint64_t need = ((uint64_t)r + lanes - 1) / lanes;  // warps worth of work
   const unsigned grid = (unsigned)std::min<uint64_t>(max_grid, (need + wpb - 1) / wpb);
   ProfScope ps(ctx, "chase", s);
-  k_chase<F><<<grid, block, 0, s>>>(rec, stamp, ext, lv.rulers[k], lv.r[k], lv.heads, k ? lv.r[k - 1] : 0u,
-                                    lv.rootel[k], next_level(lv, k + 1), &ctx.d_status->work[k], lanes, limit,
-                                    hop_cap(lv.rulers[k]), ctx.d_status);
+  k_chase<F><<<grid, block, 0, s>>>(rec, stamp, lv.n[k], lv.rulers[k], r, lv.rootel[k], next_level(lv, k + 1),
+                                    &ctx.d_status->work[k], lanes, hop_cap(lv.rulers[k]), ctx.d_status);
   KS_CHECK_LAUNCH();
   return KASCADE_OK;
 }
@@ -891,17 +874,17 @@ kascade_status launch_chase(kascade_ctx& ctx, const Levels& lv, int k, const typ
 // thread instead of eight, so that they fill the chip.
 template <class F, class Sink>
 kascade_status launch_propagate(kascade_ctx& ctx, const Levels& lv, int k, const typename F::R* rec,
-                                const typename F::S* stamp, uint32_t n_out, const Extent& ext, const Sink& sink,
-                                cudaStream_t s) {
+                                const typename F::S* stamp, const Sink& sink, cudaStream_t s) {
+  const uint32_t n = lv.n[k];
   ProfScope ps(ctx, "propagate", s);
   unsigned long long* status = k == 0 ? status_host(ctx) : nullptr;
-  if (n_out <= (uint64_t)ctx.usable_sms() * 256 * 8 * 4) {
-    const unsigned grid = grid_for(ctx, ((uint64_t)n_out + 1) / 2, 256, 8);
-    k_propagate<F, Sink, 2><<<grid, 256, 0, s>>>(rec, stamp, n_out, ext, lv.rulers[k], lv.r[k], lv.rootel[k],
+  if (n <= (uint64_t)ctx.usable_sms() * 256 * 8 * 4) {
+    const unsigned grid = grid_for(ctx, ((uint64_t)n + 1) / 2, 256, 8);
+    k_propagate<F, Sink, 2><<<grid, 256, 0, s>>>(rec, stamp, n, lv.rulers[k], lv.rootel[k],
                                                  lv.out[k + 1], sink, ctx.d_status, status);
   } else {
-    const unsigned grid = grid_for(ctx, ((uint64_t)n_out + 7) / 8, 256, 8);
-    k_propagate<F, Sink, 8><<<grid, 256, 0, s>>>(rec, stamp, n_out, ext, lv.rulers[k], lv.r[k], lv.rootel[k],
+    const unsigned grid = grid_for(ctx, ((uint64_t)n + 7) / 8, 256, 8);
+    k_propagate<F, Sink, 8><<<grid, 256, 0, s>>>(rec, stamp, n, lv.rulers[k], lv.rootel[k],
                                                  lv.out[k + 1], sink, ctx.d_status, status);
   }
   KS_CHECK_LAUNCH();
@@ -965,7 +948,6 @@ Params make_params(const kascade_ctx& ctx, const kascade_opts* o, uint64_t n) {
   {
     const int k = ctx.class_of(n);
     p.spacing0 = ctx.class_spacing_single[k];
-    p.chains = ctx.class_chains[k];
     p.block = ctx.class_block[k];
   }
   if (o) {
@@ -973,7 +955,6 @@ Params make_params(const kascade_ctx& ctx, const kascade_opts* o, uint64_t n) {
     if (o->ruler_spacing_deep) p.spacing_deep = o->ruler_spacing_deep;
     if (o->max_levels) p.max_levels = o->max_levels;
     if (o->base_case_size) p.base_max = o->base_case_size;
-    if (o->chains_per_thread) p.chains = o->chains_per_thread;
     if (o->block_size) p.block = o->block_size;
     if (o->seed) p.seed = o->seed;
     p.algorithm = o->algorithm;
@@ -1100,6 +1081,12 @@ kascade_status rank_arrays_one_cta(kascade_ctx& ctx, const uint64_t* succ, WKind
   }
 }
 
+kascade_status rank_parents_one_cta(kascade_ctx& ctx, const uint32_t* parent, uint32_t n, const SinkBatch& sink,
+                                    bool last, cudaStream_t s) {
+  Extent ext;
+  ext.cap = n;
+  return launch_rank_cta(ctx, CtaArrays<WUnit, uint32_t>{parent, WUnit{}}, ext, sink, CTA_TREES, last, s);
+}
 kascade_status rank_trees_one_cta(kascade_ctx& ctx, const Rec8* rec, const uint32_t* rootel, const Extent& ext,
                                   uint2* out, cudaStream_t s) {
   return launch_rank_cta(ctx, CtaRecords<F8x8, true>{rec, rootel}, ext, SinkOut8{out}, CTA_TREES, false, s);
@@ -1142,30 +1129,22 @@ static kascade_status pointer_double_level(kascade_ctx& ctx, const Rec* rec, con
 // Ruler gaps are geometric: longer than this has probability ~e^-64.
 uint32_t hop_cap(const Rulers& rl) { return (uint32_t)std::min<uint64_t>(64ull * rl.s + 1024, 0xFFFFFFFFull); }
 
-kascade_status plan_levels(kascade_ctx& ctx, uint32_t n, const Heads& heads, const Params& p, Levels* lv) {
+kascade_status plan_levels(kascade_ctx& ctx, uint32_t n, const Params& p, Levels* lv) {
   *lv = Levels{};
   const int max_levels = (int)std::min<uint32_t>(p.max_levels, MAX_LEVELS);
-  lv->heads = heads;
-  // the last level holds the heads too: a caller's base case below them takes none
-  if (p.base_max < 2 * heads.cap) lv->heads = Heads{};
-  const uint32_t extra = lv->heads.cap;
-  const uint32_t base = std::max(1u, p.base_max - extra);
+  const uint32_t base = std::max(1u, p.base_max);
   int k = 0;
-  uint32_t m = n;  // the elements of level k that rulers are placed among
   lv->n[0] = n;
-  while (m > base && k < max_levels) {
-    const uint32_t sp = k == 0           ? p.spacing0
-                        : p.spacing_deep ? p.spacing_deep
-                                         : deep_spacing(m, ONE_CTA_MAX * 3 / 4 - extra);
+  while (lv->n[k] > base && k < max_levels) {
+    const uint32_t sp = p.spacing_deep ? p.spacing_deep : deep_spacing(lv->n[k], ONE_CTA_MAX * 3 / 4);
     lv->rulers[k] = k == 0 ? level0_rulers(p) : make_rulers(sp, salt_for(p.seed, k));
-    lv->r[k] = m = ruler_count(m, lv->rulers[k]);
-    lv->n[k + 1] = m + extra;
+    lv->n[k + 1] = ruler_count(lv->n[k], lv->rulers[k]);
     ++k;
   }
   lv->last = k;
-  ctx.last_levels.assign(1, n);
+  lv->rulers[k] = cta_rulers(lv->n[k]);
+  ctx.last_levels.assign(lv->n, lv->n + k + 1);
   for (int i = 1; i <= k; ++i) {
-    ctx.last_levels.push_back(lv->r[i - 1]);
     lv->rec[i] = alloc<Rec>(ctx, lv->n[i]);
     lv->stamp[i] = i < k ? alloc<uint4>(ctx, lv->n[i]) : nullptr;
     lv->rootel[i] = alloc<uint32_t>(ctx, lv->n[i]);
@@ -1177,53 +1156,56 @@ kascade_status plan_levels(kascade_ctx& ctx, uint32_t n, const Heads& heads, con
 
 kascade_status rank_deep(kascade_ctx& ctx, const Levels& lv, cudaStream_t s) {
   for (int k = 1; k < lv.last; ++k)
-    KS_TRY(launch_chase<F16x16>(ctx, lv, k, lv.rec[k], lv.stamp[k], lv.extent(k), lv.n[k], 256, s));
+    KS_TRY(launch_chase<F16x16>(ctx, lv, k, lv.rec[k], lv.stamp[k], 256, s));
   const int L = lv.last;
+  Extent ext;
+  ext.cap = lv.n[L];
   if (lv.n[L] <= ONE_CTA_MAX) {
-    KS_TRY(launch_rank_cta(ctx, CtaRecords<F16x16, true>{lv.rec[L], lv.rootel[L]}, lv.extent(L), SinkOut{lv.out[L]},
-                           CTA_LISTS, false, s));
+    KS_TRY(launch_rank_cta(ctx, CtaRecords<F16x16, true>{lv.rec[L], lv.rootel[L]}, ext, SinkOut{lv.out[L]}, CTA_LISTS,
+                           false, s));
   } else {
-    KS_TRY(pointer_double_level(ctx, lv.rec[L], lv.extent(L), lv.rootel[L], lv.out[L], s));
+    KS_TRY(pointer_double_level(ctx, lv.rec[L], ext, lv.rootel[L], lv.out[L], s));
   }
   for (int k = L - 1; k >= 1; --k)
-    KS_TRY(launch_propagate<F16x16>(ctx, lv, k, lv.rec[k], lv.stamp[k], lv.n[k], lv.extent(k), SinkOut{lv.out[k]},
-                                    s));
+    KS_TRY(launch_propagate<F16x16>(ctx, lv, k, lv.rec[k], lv.stamp[k], SinkOut{lv.out[k]}, s));
   return KASCADE_OK;
 }
 
 namespace {
 
 template <class F, class Sink>
-kascade_status rank_records_as(kascade_ctx& ctx, const Level0& l0, uint32_t n, const Extent& ext, const Heads& heads,
-                               const Sink& sink, const Params& p, cudaStream_t s) {
+kascade_status rank_records_as(kascade_ctx& ctx, const Level0& l0, uint32_t n, const Sink& sink, CtaMode mode,
+                               const Params& p, cudaStream_t s) {
   const typename F::R* rec = l0.records<F>();
   if (n <= p.base_max) {
     ctx.last_levels.assign(1, n);
-    return launch_rank_cta(ctx, CtaRecords<F, false>{rec, nullptr}, ext, sink, CTA_SMALL_TREES, true, s);
+    Extent ext;
+    ext.cap = n;
+    return launch_rank_cta(ctx, CtaRecords<F, false>{rec, nullptr}, ext, sink, mode, true, s);
   }
   Levels lv;
-  KS_TRY(plan_levels(ctx, n, heads, p, &lv));
-  KS_TRY(launch_chase<F>(ctx, lv, 0, rec, l0.stamps<F>(), ext, sink.limit(n), p.block, s));
+  KS_TRY(plan_levels(ctx, n, p, &lv));
+  KS_TRY(launch_chase<F>(ctx, lv, 0, rec, l0.stamps<F>(), p.block, s));
   KS_TRY(rank_deep(ctx, lv, s));
-  return launch_propagate<F>(ctx, lv, 0, rec, l0.stamps<F>(), sink.limit(n), ext, sink, s);
+  return launch_propagate<F>(ctx, lv, 0, rec, l0.stamps<F>(), sink, s);
 }
 
 }  // namespace
 
 template <class Sink>
-kascade_status rank_records(kascade_ctx& ctx, const Level0& l0, uint32_t n, const Extent& ext, const Heads& heads,
-                            const Sink& sink, const Params& p, cudaStream_t s) {
+kascade_status rank_records(kascade_ctx& ctx, const Level0& l0, uint32_t n, const Sink& sink, CtaMode mode,
+                            const Params& p, cudaStream_t s) {
   if (n == 0) return KASCADE_OK;
-  if (n > p.base_max && !l0.stamp) return rank_level0_log(ctx, l0, n, ext, heads, sink.log_target(n), p, s);
+  if (n > p.base_max && !l0.stamp) return rank_level0_log(ctx, l0, n, sink.log_target(), p, s);
   switch (l0.fmt) {
     case Format::F8x8:
-      return rank_records_as<F8x8>(ctx, l0, n, ext, heads, sink, p, s);
+      return rank_records_as<F8x8>(ctx, l0, n, sink, mode, p, s);
     case Format::F8x16:
-      return rank_records_as<F8x16>(ctx, l0, n, ext, heads, sink, p, s);
+      return rank_records_as<F8x16>(ctx, l0, n, sink, mode, p, s);
     case Format::F16i:
-      return rank_records_as<F16i>(ctx, l0, n, ext, heads, sink, p, s);
+      return rank_records_as<F16i>(ctx, l0, n, sink, mode, p, s);
     default:
-      return rank_records_as<F16x16>(ctx, l0, n, ext, heads, sink, p, s);
+      return rank_records_as<F16x16>(ctx, l0, n, sink, mode, p, s);
   }
 }
 
@@ -1247,9 +1229,9 @@ kascade_status check_is_list(kascade_ctx& ctx, const uint64_t* succ, uint64_t n,
 }
 
 // explicit instantiations for the level-0 sinks
-template kascade_status rank_records<SinkPlain>(kascade_ctx&, const Level0&, uint32_t, const Extent&, const Heads&,
-                                                const SinkPlain&, const Params&, cudaStream_t);
-template kascade_status rank_records<SinkBatch>(kascade_ctx&, const Level0&, uint32_t, const Extent&, const Heads&,
-                                                const SinkBatch&, const Params&, cudaStream_t);
+template kascade_status rank_records<SinkPlain>(kascade_ctx&, const Level0&, uint32_t, const SinkPlain&, CtaMode,
+                                                const Params&, cudaStream_t);
+template kascade_status rank_records<SinkBatch>(kascade_ctx&, const Level0&, uint32_t, const SinkBatch&, CtaMode,
+                                                const Params&, cudaStream_t);
 
 }  // namespace ks

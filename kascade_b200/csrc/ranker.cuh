@@ -33,7 +33,6 @@ struct Params {
   uint32_t spacing_deep = 0;  // mean elements per ruler, deeper levels (0: by level size)
   uint32_t max_levels = 6;
   uint32_t base_max = 16384;  // one-CTA ranker bound
-  uint32_t chains = 2;        // chains in flight per thread (1, 2 or 4)
   uint32_t block = 256;
   uint32_t seed = 0x6b617363u;
   uint32_t algorithm = KASCADE_ALGO_SPARSE_RULING_SET;
@@ -101,40 +100,38 @@ struct Extent {
   }
 };
 
-// Known list heads of level 0 (a tour's heads are known when it is built):
-// they start chains of their own, so that no element ahead of its list's
-// first ruler is left to walk.  Head e's chain has the id after the rulers',
-// r + e; level k + 1 keeps it as the element after its rulers' ones, where it
-// is a head again.  Heads beyond the capacity stay unreached and walk.
-struct Heads {
-  const uint32_t* elem = nullptr;   // level-0 elements (device)
-  const uint32_t* count = nullptr;  // how many (device); more than cap: the first cap
-  uint32_t cap = 0;
-  __device__ __forceinline__ uint32_t get() const { return cap ? min(cap, __ldg(count)) : 0u; }
-};
-constexpr uint32_t HEAD_CAP = 2048;
-
 // Where results of level 0 go ------------------------------------------------
 // A sink receives, for element x, its rank, its root (level-0 index) and
 // whether x itself is a root.
+
+// Segments of an element range and where their outputs go: a batch's list or
+// forest elements, instance after instance, are numbered densely; outputs are
+// at the instances' places in the caller's arrays, roots relative to their
+// instance.  At most 2^32 elements: offsets wrap.
+struct SegMap {
+  const uint32_t* base = nullptr;   // n + 1: the segments' first elements, non-decreasing; then the end
+  const uint32_t* delta = nullptr;  // element + delta: its place in the outputs
+  const uint32_t* hint = nullptr;   // [k]: the segment of element 4096 k, and one more for the end
+  uint32_t n = 0;                   // 0: one instance, in place
+  __device__ __forceinline__ uint32_t find(uint32_t x) const {  // the last j with base[j] <= x
+    uint32_t lo = __ldg(hint + (x >> 12)), hi = min(__ldg(hint + (x >> 12) + 1) + 1, n);
+    while (hi - lo > 1) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (__ldg(base + mid) <= x)
+        lo = mid;
+      else
+        hi = mid;
+    }
+    return lo;
+  }
+};
 
 // Level-0 output description for the write-free (log) pipeline.
 struct LogTarget {
   uint64_t* root;
   uint64_t* rank;
-  uint32_t limit;        // elements [0, limit) produce output
-  int keep_roots;        // leave roots' entries untouched
-  // a batch of instances in one index space: roots are reported relative to
-  // their instance (seg_off: nseg instance offsets, hint[k]: the instance
-  // holding element k * 4096); null for a single instance
-  const uint64_t* seg_off = nullptr;
-  const uint32_t* hint = nullptr;
-  uint32_t nseg = 0;
-  // bit x set: element x's rank output is one more than its rank in the list
-  // (a tree rooting's leaves, whose down and up edge share one element)
-  const uint32_t* plus_one = nullptr;
-  // depths: ranks modulo 2^32, of the instances with their bit set (a batch's forests)
-  const uint32_t* seg_tour = nullptr;
+  int keep_roots;  // leave roots' entries untouched
+  SegMap seg;
 };
 
 // Plain arrays. keep_roots: leave root entries untouched (the reference's
@@ -143,9 +140,7 @@ struct SinkPlain {
   uint64_t* root;
   uint64_t* rank;
   int keep_roots;
-  // elements [0, limit(n)) produce output
-  uint32_t limit(uint32_t n) const { return n; }
-  LogTarget log_target(uint32_t n) const { return LogTarget{root, rank, n, keep_roots}; }
+  LogTarget log_target() const { return LogTarget{root, rank, keep_roots, SegMap{}}; }
   __device__ __forceinline__ void put(uint32_t x, uint64_t rk, uint32_t rt, bool is_root) const {
     if (is_root) {
       if (!keep_roots) {
@@ -159,43 +154,17 @@ struct SinkPlain {
   }
 };
 
-// A batch of independent instances concatenated into one index space:
-// roots are reported relative to their instance.  seg_off holds the nseg
-// instance offsets (non-decreasing), hint[k] the instance containing element
-// k * 4096.  Elements at or beyond `total` (tour down edges) give no output.
-// seg_tour: bit j set for a forest, whose depths are ranks modulo 2^32 (null:
-// lists only); plus_one: bit x set for a forest leaf whose down and up edge
-// are one element, whose rank is then one less than the leaf's depth.
+// A batch's lists or forests.
 struct SinkBatch {
   uint64_t* root;
   uint64_t* rank;
-  uint32_t total;
-  const uint64_t* seg_off;
-  const uint32_t* hint;
-  uint32_t nseg;
-  const uint32_t* plus_one = nullptr;
-  const uint32_t* seg_tour = nullptr;
-  uint32_t limit(uint32_t n) const { return n < total ? n : total; }
-  LogTarget log_target(uint32_t n) const {
-    LogTarget t{root, rank, limit(n), 0, seg_off, hint, nseg};
-    t.plus_one = plus_one;
-    t.seg_tour = seg_tour;
-    return t;
-  }
+  SegMap seg;
+  LogTarget log_target() const { return LogTarget{root, rank, 0, seg}; }
   __device__ __forceinline__ void put(uint32_t x, uint64_t rk, uint32_t rt, bool is_root) const {
-    if (x >= total) return;
-    uint32_t j = __ldg(hint + (x >> 12));
-    while (j + 1 < nseg && __ldg(seg_off + j + 1) <= x) ++j;
-    const uint64_t b = __ldg(seg_off + j);
-    if (is_root) {
-      __stcs(root + x, (unsigned long long)(x - b));
-      __stcs(rank + x, 0ull);
-      return;
-    }
-    if (seg_tour && ((__ldg(seg_tour + (j >> 5)) >> (j & 31)) & 1u))
-      rk = (uint32_t)rk + ((__ldg(plus_one + (x >> 5)) >> (x & 31)) & 1u);
-    __stcs(root + x, (unsigned long long)(rt - b));
-    __stcs(rank + x, (unsigned long long)rk);
+    const uint32_t j = seg.find(x);
+    const uint32_t b = __ldg(seg.base + j), g = x + __ldg(seg.delta + j);
+    __stcs(root + g, (unsigned long long)((is_root ? x : rt) - b));
+    __stcs(rank + g, is_root ? 0ull : (unsigned long long)rk);
   }
 };
 
@@ -262,6 +231,12 @@ kascade_status rank_trees_one_cta(kascade_ctx& ctx, const Rec8* rec, const uint3
                                   uint2* out, cudaStream_t s);
 kascade_status rank_trees_one_cta(kascade_ctx& ctx, const Rec* rec, const uint32_t* rootel, const Extent& ext,
                                   Out* out, cudaStream_t s);
+kascade_status rank_parents_one_cta(kascade_ctx& ctx, const uint32_t* parent, uint32_t n, const SinkBatch& sink,
+                                    bool last, cudaStream_t s);
+// A batch's forests, parents in one compact vertex space (tree.cu).  last: the
+// call's last device work.
+kascade_status root_forests(kascade_ctx& ctx, const uint32_t* parent, uint32_t n, const SinkBatch& sink, bool last,
+                            const Params& p, cudaStream_t s);
 // Any forest: results of every element (tree.cu).
 kascade_status rank_forest_weighted(kascade_ctx& ctx, const uint64_t* succ, WKind wk, const void* w, uint32_t n,
                                     const SinkPlain& sink, const Params& p, cudaStream_t s);
@@ -270,39 +245,27 @@ kascade_status rank_forest_weighted(kascade_ctx& ctx, const uint64_t* succ, WKin
 // size is known on the host: no host wait between the launches.  `ext`: the
 // record count when only the device knows it (ext.cap == n).
 template <class Sink>
-kascade_status rank_records(kascade_ctx& ctx, const Level0& l0, uint32_t n, const Extent& ext, const Heads& heads,
-                            const Sink& sink, const Params& p, cudaStream_t s);
+kascade_status rank_records(kascade_ctx& ctx, const Level0& l0, uint32_t n, const Sink& sink, CtaMode mode,
+                            const Params& p, cudaStream_t s);
 
-// The levels of one call.  Level k >= 1 holds level k - 1's rulers, then its
-// heads: records {distance, next ruler}, the root of a list end and results.
+// The levels of one call.  Level k >= 1 holds level k - 1's rulers: records
+// {distance, next ruler}, the root of a list end and results.
 constexpr int MAX_LEVELS = 24;
 struct Levels {
   int last = 0;                  // the level ranked by one CTA (or by doubling)
-  uint32_t n[MAX_LEVELS + 1];    // elements per level, heads (their capacity) included
-  uint32_t r[MAX_LEVELS];        // rulers of level k; level k + 1 has r[k] + heads.cap elements
-  Rulers rulers[MAX_LEVELS];     // their placement
-  Heads heads;
+  uint32_t n[MAX_LEVELS + 1];    // elements per level
+  Rulers rulers[MAX_LEVELS + 1];  // each level's rulers; the last one's: the one-CTA ranker's
   Rec* rec[MAX_LEVELS + 1];      // from level 1 on
   uint4* stamp[MAX_LEVELS + 1];  // from level 1 on, but not of the last level
   uint32_t* rootel[MAX_LEVELS + 1];  // level k >= 1: a list end's root as a level-0 element
   Out* out[MAX_LEVELS + 1];
-  Extent extent(int k) const {
-    Extent e;
-    e.cap = n[k];
-    if (k && heads.cap) {
-      e.base = r[k - 1];
-      e.add = heads.count;
-    }
-    return e;
-  }
 };
-kascade_status plan_levels(kascade_ctx& ctx, uint32_t n, const Heads& heads, const Params& p, Levels* lv);
+kascade_status plan_levels(kascade_ctx& ctx, uint32_t n, const Params& p, Levels* lv);
 // Levels 1..last once the level-0 chase has written level 1: fills lv.out[1].
 kascade_status rank_deep(kascade_ctx& ctx, const Levels& lv, cudaStream_t s);
 
 // Where a level's chains put their rulers' records.  The last level has no
-// stamps; its rulers are the one-CTA ranker's (rl.s == 0: found on the device
-// from the level's size, which the heads are part of).
+// stamps.
 struct NextLevel {
   Rec* rec = nullptr;
   uint4* stamp = nullptr;
@@ -321,7 +284,6 @@ inline NextLevel next_level(const Levels& lv, int k) {
   nx.stamp = lv.stamp[k];
   nx.rootel = lv.rootel[k];
   nx.rl = lv.rulers[k];
-  if (k == lv.last) nx.rl.s = 0;
   return nx;
 }
 
@@ -346,8 +308,8 @@ kascade_status compute_stats(kascade_ctx& ctx, const uint64_t* root, const int64
 // Write-free level 0: read-only chase that logs (element, ruler, distance),
 // recursion on the ruler list, then two radix passes over the log by element
 // and a dense placement into the outputs.
-kascade_status rank_level0_log(kascade_ctx& ctx, const Level0& l0, uint32_t n, const Extent& ext, const Heads& heads,
-                               const LogTarget& t, const Params& p, cudaStream_t s);
+kascade_status rank_level0_log(kascade_ctx& ctx, const Level0& l0, uint32_t n, const LogTarget& t, const Params& p,
+                               cudaStream_t s);
 
 // Validation: *ok = 1 if no element has two predecessors.
 kascade_status check_is_list(kascade_ctx& ctx, const uint64_t* succ, uint64_t n, int* ok,

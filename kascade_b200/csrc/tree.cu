@@ -88,8 +88,10 @@ struct Tree16 {
 constexpr int WORDS_PER = 8;  // words of 32 vertices a thread counts
 constexpr uint32_t WORDS_TILE = TREE_THREADS * WORDS_PER;
 
-__device__ __forceinline__ uint64_t parent_of(const uint64_t* parent, uint64_t v, uint32_t n) {
-  return v < n ? __ldcs(reinterpret_cast<const unsigned long long*>(parent) + v) : v;
+// Parents are the caller's 64-bit indices, or a batch's in one vertex space.
+template <class P>
+__device__ __forceinline__ uint64_t parent_of(const P* parent, uint64_t v, uint32_t n) {
+  return v < n ? __ldcs(parent + v) : v;
 }
 
 // A byte set for every vertex with a child (zeroed by the caller).  A parent
@@ -98,7 +100,8 @@ __device__ __forceinline__ uint64_t parent_of(const uint64_t* parent, uint64_t v
 // 0.56 ms against 0.40 with an atomic OR per vertex, but a hundred hubs with all
 // the leaves 0.3 ms against 15 (atomics on a few words come one at a time), and
 // asking for the word before the atomic costs 0.63.
-__global__ void __launch_bounds__(TREE_THREADS) k_tree_inner(const uint64_t* __restrict__ parent, uint32_t n,
+template <class P>
+__global__ void __launch_bounds__(TREE_THREADS) k_tree_inner(const P* __restrict__ parent, uint32_t n,
                                                              unsigned char* __restrict__ inner, DevStatus* st) {
   const uint64_t tile_sz = (uint64_t)blockDim.x * TREE_PREP_ITEMS;
   for (uint64_t tile = (uint64_t)blockIdx.x * tile_sz; tile < n; tile += (uint64_t)gridDim.x * tile_sz) {
@@ -199,12 +202,14 @@ __device__ __forceinline__ uint32_t number_of(uint2 w, uint32_t v) {
 }
 
 // The records of the numbered vertices; vert: their vertices (the roots').
-// Reports the tour's length: the vertices, and once more those with children
-// that are not roots.
-__global__ void __launch_bounds__(TREE_THREADS) k_tree_records(const uint64_t* __restrict__ parent, uint32_t n,
+// report: the tour's length, the vertices and once more those with children
+// that are not roots, goes to the status.
+template <class P>
+__global__ void __launch_bounds__(TREE_THREADS) k_tree_records(const P* __restrict__ parent, uint32_t n,
                                                                const uint2* __restrict__ iw, Rulers rl,
                                                                uint32_t* __restrict__ rec,
-                                                               uint32_t* __restrict__ vert, DevStatus* st) {
+                                                               uint32_t* __restrict__ vert, bool report,
+                                                               DevStatus* st) {
   const uint64_t tile_sz = (uint64_t)blockDim.x * TREE_PREP_ITEMS;
   uint32_t downs = 0;
   for (uint64_t tile = (uint64_t)blockIdx.x * tile_sz; tile < n; tile += (uint64_t)gridDim.x * tile_sz) {
@@ -236,15 +241,17 @@ __global__ void __launch_bounds__(TREE_THREADS) k_tree_records(const uint64_t* _
       rec[c] = b;
     }
   }
+  if (!report) return;
   downs = __reduce_add_sync(0xffffffffu, downs);
   if ((threadIdx.x & 31u) == 0 && downs) atomicAdd(&st->counter[1], (unsigned long long)downs);
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&st->counter[1], (unsigned long long)n);
 }
 
 // Every vertex's result from the numbered ones' (depth, root).
-__global__ void __launch_bounds__(TREE_THREADS) k_tree_leaves(const uint64_t* parent, uint32_t n,
+template <class P, class Sink>
+__global__ void __launch_bounds__(TREE_THREADS) k_tree_leaves(const P* parent, uint32_t n,
                                                               const uint2* __restrict__ iw,
-                                                              const uint2* __restrict__ out, SinkPlain sink,
+                                                              const uint2* __restrict__ out, Sink sink,
                                                               DevStatus* st, unsigned long long* status) {
   const uint64_t tile_sz = (uint64_t)blockDim.x * TREE_OUT_ITEMS;
   for (uint64_t tile = (uint64_t)blockIdx.x * tile_sz; tile < n; tile += (uint64_t)gridDim.x * tile_sz) {
@@ -442,18 +449,10 @@ kascade_status rank_tree(kascade_ctx& ctx, const TreeLevels& lv, const typename 
   return tree_propagate<L, N>(ctx, lv, 0, rec, rootel, nout[1], sink, last, s);
 }
 
-}  // namespace
-
-kascade_status root_forest_impl(kascade_ctx& ctx, const uint64_t* parent, uint32_t n, uint64_t* root_out,
-                                uint64_t* depth_out, int keep_roots, const Params& p, cudaStream_t s) {
-  if (n == 0) return KASCADE_OK;
-  const SinkPlain sink{root_out, depth_out, keep_roots};
-  uint32_t* count = alloc<uint32_t>(ctx, 1);
-  if (!count) return KASCADE_ERR_OOM;
-  const TreeLevels lv = plan_tree(n, count, p);
-  if (lv.last == 0) return rank_arrays_one_cta(ctx, parent, WKind::Unit, nullptr, n, sink, CTA_ROOTING, s);
-  ctx.last_levels.assign(1, n);
-  for (int k = 1; k <= lv.last; ++k) ctx.last_levels.push_back(lv.ext[k].cap);
+// Depths and roots of a forest of more than TREE_BASE vertices.
+template <class P, class Sink>
+kascade_status root_levels(kascade_ctx& ctx, const P* parent, uint32_t n, const TreeLevels& lv, uint32_t* count,
+                           const Sink& sink, bool report, bool last, cudaStream_t s) {
   const uint32_t words = (uint32_t)(((uint64_t)n + 31) / 32);
   const uint32_t tiles = (words + WORDS_TILE - 1) / WORDS_TILE;
   unsigned char* inner = alloc<unsigned char>(ctx, 32ull * words);
@@ -475,15 +474,41 @@ kascade_status root_forest_impl(kascade_ctx& ctx, const uint64_t* parent, uint32
     }
     k_tree_number<<<tiles, TREE_THREADS, 0, s>>>(inner, words, sums, iw, count);
     KS_CHECK_LAUNCH();
-    k_tree_records<<<grid, TREE_THREADS, 0, s>>>(parent, n, iw, lv.rulers[0], rec, vert, ctx.d_status);
+    k_tree_records<<<grid, TREE_THREADS, 0, s>>>(parent, n, iw, lv.rulers[0], rec, vert, report, ctx.d_status);
     KS_CHECK_LAUNCH();
   }
   KS_TRY((rank_tree<TreeUnit, Tree8, SinkOut8>(ctx, lv, rec, vert, SinkOut8{out}, false, s)));
   ProfScope ps(ctx, "leaves", s);
   const unsigned grid = grid_for(ctx, ((uint64_t)n + TREE_OUT_ITEMS - 1) / TREE_OUT_ITEMS, TREE_THREADS, 8);
-  k_tree_leaves<<<grid, TREE_THREADS, 0, s>>>(parent, n, iw, out, sink, ctx.d_status, status_host(ctx));
+  k_tree_leaves<<<grid, TREE_THREADS, 0, s>>>(parent, n, iw, out, sink, ctx.d_status,
+                                              last ? status_host(ctx) : nullptr);
   KS_CHECK_LAUNCH();
   return KASCADE_OK;
+}
+
+}  // namespace
+
+kascade_status root_forest_impl(kascade_ctx& ctx, const uint64_t* parent, uint32_t n, uint64_t* root_out,
+                                uint64_t* depth_out, int keep_roots, const Params& p, cudaStream_t s) {
+  if (n == 0) return KASCADE_OK;
+  const SinkPlain sink{root_out, depth_out, keep_roots};
+  uint32_t* count = alloc<uint32_t>(ctx, 1);
+  if (!count) return KASCADE_ERR_OOM;
+  const TreeLevels lv = plan_tree(n, count, p);
+  if (lv.last == 0) return rank_arrays_one_cta(ctx, parent, WKind::Unit, nullptr, n, sink, CTA_ROOTING, s);
+  ctx.last_levels.assign(1, n);
+  for (int k = 1; k <= lv.last; ++k) ctx.last_levels.push_back(lv.ext[k].cap);
+  return root_levels(ctx, parent, n, lv, count, sink, true, true, s);
+}
+
+kascade_status root_forests(kascade_ctx& ctx, const uint32_t* parent, uint32_t n, const SinkBatch& sink, bool last,
+                            const Params& p, cudaStream_t s) {
+  if (n == 0) return KASCADE_OK;
+  uint32_t* count = alloc<uint32_t>(ctx, 1);
+  if (!count) return KASCADE_ERR_OOM;
+  const TreeLevels lv = plan_tree(n, count, p);
+  if (lv.last == 0) return rank_parents_one_cta(ctx, parent, n, sink, last, s);
+  return root_levels(ctx, parent, n, lv, count, sink, false, last, s);
 }
 
 kascade_status rank_forest_weighted(kascade_ctx& ctx, const uint64_t* succ, WKind wk, const void* w, uint32_t n,
