@@ -172,6 +172,9 @@ KASCADE_API kascade_status kascade_ctx_destroy(kascade_ctx* c) {
   }
   for (auto e : c->event_pool) cudaEventDestroy(e);
   if (c->done_event) cudaEventDestroy(c->done_event);
+  if (c->side) cudaStreamDestroy(c->side);
+  if (c->fork) cudaEventDestroy(c->fork);
+  if (c->join) cudaEventDestroy(c->join);
   if (c->d_status) cudaFree(c->d_status);
   if (c->h_pinned) cudaFreeHost(c->h_pinned);
   cudaGetLastError();

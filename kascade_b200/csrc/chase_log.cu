@@ -644,7 +644,7 @@ kascade_status rank_level0_log_as(kascade_ctx& ctx, const Level0& l0, uint32_t n
   {
     ProfScope ps(ctx, "heads", s);
     k_walk_unreached<F><<<ctx.usable_sms() * 4, 256, 0, s>>>(l0.records<F>(), ulist, ucount, n, t.root, t.rank, t.seg,
-                                                             t.keep_roots, ctx.d_status, status_host(ctx));
+                                                             t.keep_roots, ctx.d_status, status_host(ctx, p.last));
     KS_CHECK_LAUNCH();
   }
   return KASCADE_OK;

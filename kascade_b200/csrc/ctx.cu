@@ -85,7 +85,8 @@ kascade_status status_reset(kascade_ctx& ctx, cudaStream_t s) {
   return KASCADE_OK;
 }
 
-unsigned long long* status_host(kascade_ctx& ctx) {
+unsigned long long* status_host(kascade_ctx& ctx, bool last) {
+  if (!last) return nullptr;
   ctx.published = true;
   ctx.status_dirty = false;
   return ctx.h_pinned;
@@ -141,6 +142,21 @@ kascade_status read_u32(kascade_ctx& ctx, const uint32_t* dptr, uint32_t* out, c
   KS_CUDA(cudaMemcpyAsync(hp, dptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   KS_CUDA(cudaStreamSynchronize(s));
   *out = *hp;
+  return KASCADE_OK;
+}
+
+kascade_status side_fork(kascade_ctx& ctx, cudaStream_t s) {
+  if (!ctx.side) KS_CUDA(cudaStreamCreateWithFlags(&ctx.side, cudaStreamNonBlocking));
+  if (!ctx.fork) KS_CUDA(cudaEventCreateWithFlags(&ctx.fork, cudaEventDisableTiming));
+  if (!ctx.join) KS_CUDA(cudaEventCreateWithFlags(&ctx.join, cudaEventDisableTiming));
+  KS_CUDA(cudaEventRecord(ctx.fork, s));
+  KS_CUDA(cudaStreamWaitEvent(ctx.side, ctx.fork, 0));
+  return KASCADE_OK;
+}
+
+kascade_status side_join(kascade_ctx& ctx, cudaStream_t s) {
+  KS_CUDA(cudaEventRecord(ctx.join, ctx.side));
+  KS_CUDA(cudaStreamWaitEvent(s, ctx.join, 0));
   return KASCADE_OK;
 }
 

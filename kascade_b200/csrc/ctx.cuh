@@ -51,6 +51,9 @@ struct kascade_ctx {
   cudaEvent_t done_event = nullptr;
   cudaStream_t last_stream = nullptr;
   bool async_pending = false;
+  // a second stream for device work that is independent within a call
+  cudaStream_t side = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
   // size classes: a batch of at most class_max[i] records uses a ruler spacing
   // of class_spacing[i], a call that ranks one list or tour of that size
   // class_spacing_single[i]; both chase in blocks of class_block[i] threads.
@@ -98,15 +101,20 @@ T* alloc(kascade_ctx& ctx, size_t count) {
 kascade_status cuda_status(cudaError_t e);
 // Start a call: the device status is zero (stream-ordered).
 kascade_status status_reset(kascade_ctx& ctx, cudaStream_t s);
-// For the launch that ends a call's device work: where its publish_status puts
-// the status.
-unsigned long long* status_host(kascade_ctx& ctx);
+// For the launch that ends a call's device work (last): where its
+// publish_status puts the status.
+unsigned long long* status_host(kascade_ctx& ctx, bool last = true);
 // Copy the status to the host by a launch of its own unless a kernel does.
 kascade_status status_publish(kascade_ctx& ctx, cudaStream_t s);
 // Synchronise `s`, read the status, collect kernel timings.
 kascade_status status_finish(kascade_ctx& ctx, cudaStream_t s);
 // Read one device word into the pinned buffer and wait for it.
 kascade_status read_u32(kascade_ctx& ctx, const uint32_t* dptr, uint32_t* out, cudaStream_t s);
+
+// Work on ctx.side that may run beside what is enqueued on `s` from here on,
+// and its end: `s` waits for it.  Every fork is joined, in error paths too.
+kascade_status side_fork(kascade_ctx& ctx, cudaStream_t s);
+kascade_status side_join(kascade_ctx& ctx, cudaStream_t s);
 
 // Profiling ----------------------------------------------------------------
 struct ProfScope {

@@ -874,10 +874,10 @@ kascade_status launch_chase(kascade_ctx& ctx, const Levels& lv, int k, const typ
 // thread instead of eight, so that they fill the chip.
 template <class F, class Sink>
 kascade_status launch_propagate(kascade_ctx& ctx, const Levels& lv, int k, const typename F::R* rec,
-                                const typename F::S* stamp, const Sink& sink, cudaStream_t s) {
+                                const typename F::S* stamp, const Sink& sink, bool last, cudaStream_t s) {
   const uint32_t n = lv.n[k];
   ProfScope ps(ctx, "propagate", s);
-  unsigned long long* status = k == 0 ? status_host(ctx) : nullptr;
+  unsigned long long* status = status_host(ctx, last);
   if (n <= (uint64_t)ctx.usable_sms() * 256 * 8 * 4) {
     const unsigned grid = grid_for(ctx, ((uint64_t)n + 1) / 2, 256, 8);
     k_propagate<F, Sink, 2><<<grid, 256, 0, s>>>(rec, stamp, n, lv.rulers[k], lv.rootel[k],
@@ -905,7 +905,7 @@ kascade_status launch_rank_cta(kascade_ctx& ctx, const Src& src, const Extent& e
   // one ruler per thread; a small input's few barriers are cheaper with fewer warps
   const unsigned threads = ext.cap <= 1024 ? 256 : CTA_THREADS;
   k_rank_cta<Src, Sink><<<1, threads, cta_smem(ext.cap), s>>>(src, ext, sink, mode, ctx.d_status,
-                                                                last ? status_host(ctx) : nullptr);
+                                                                status_host(ctx, last));
   KS_CHECK_LAUNCH();
   return KASCADE_OK;
 }
@@ -1167,7 +1167,7 @@ kascade_status rank_deep(kascade_ctx& ctx, const Levels& lv, cudaStream_t s) {
     KS_TRY(pointer_double_level(ctx, lv.rec[L], ext, lv.rootel[L], lv.out[L], s));
   }
   for (int k = L - 1; k >= 1; --k)
-    KS_TRY(launch_propagate<F16x16>(ctx, lv, k, lv.rec[k], lv.stamp[k], SinkOut{lv.out[k]}, s));
+    KS_TRY(launch_propagate<F16x16>(ctx, lv, k, lv.rec[k], lv.stamp[k], SinkOut{lv.out[k]}, false, s));
   return KASCADE_OK;
 }
 
@@ -1181,13 +1181,13 @@ kascade_status rank_records_as(kascade_ctx& ctx, const Level0& l0, uint32_t n, c
     ctx.last_levels.assign(1, n);
     Extent ext;
     ext.cap = n;
-    return launch_rank_cta(ctx, CtaRecords<F, false>{rec, nullptr}, ext, sink, mode, true, s);
+    return launch_rank_cta(ctx, CtaRecords<F, false>{rec, nullptr}, ext, sink, mode, p.last, s);
   }
   Levels lv;
   KS_TRY(plan_levels(ctx, n, p, &lv));
   KS_TRY(launch_chase<F>(ctx, lv, 0, rec, l0.stamps<F>(), p.block, s));
   KS_TRY(rank_deep(ctx, lv, s));
-  return launch_propagate<F>(ctx, lv, 0, rec, l0.stamps<F>(), sink, s);
+  return launch_propagate<F>(ctx, lv, 0, rec, l0.stamps<F>(), sink, p.last, s);
 }
 
 }  // namespace

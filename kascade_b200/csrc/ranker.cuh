@@ -37,6 +37,7 @@ struct Params {
   uint32_t seed = 0x6b617363u;
   uint32_t algorithm = KASCADE_ALGO_SPARSE_RULING_SET;
   uint32_t level0_mode = 0;  // 0: by size, 1: stamps, 2: write-free
+  bool last = true;          // the ranking is the call's last device work
 };
 
 Params make_params(const kascade_ctx& ctx, const kascade_opts* opts, uint64_t n);

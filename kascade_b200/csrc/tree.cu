@@ -421,7 +421,7 @@ kascade_status tree_propagate(kascade_ctx& ctx, const TreeLevels& lv, int k, con
                               cudaStream_t s) {
   ProfScope ps(ctx, "propagate", s);
   k_tree_propagate<L, N, Sink><<<grid_for(ctx, lv.ext[k].cap, TREE_THREADS, 8), TREE_THREADS, 0, s>>>(
-      rec, lv.ext[k], lv.rulers[k], rootel, out, sink, ctx.d_status, last ? status_host(ctx) : nullptr);
+      rec, lv.ext[k], lv.rulers[k], rootel, out, sink, ctx.d_status, status_host(ctx, last));
   KS_CHECK_LAUNCH();
   return KASCADE_OK;
 }
@@ -481,7 +481,7 @@ kascade_status root_levels(kascade_ctx& ctx, const P* parent, uint32_t n, const 
   ProfScope ps(ctx, "leaves", s);
   const unsigned grid = grid_for(ctx, ((uint64_t)n + TREE_OUT_ITEMS - 1) / TREE_OUT_ITEMS, TREE_THREADS, 8);
   k_tree_leaves<<<grid, TREE_THREADS, 0, s>>>(parent, n, iw, out, sink, ctx.d_status,
-                                              last ? status_host(ctx) : nullptr);
+                                              status_host(ctx, last));
   KS_CHECK_LAUNCH();
   return KASCADE_OK;
 }
