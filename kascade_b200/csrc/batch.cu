@@ -262,8 +262,10 @@ kascade_status batch_enqueue(kascade_ctx& ctx, const BatchTables& t, const uint6
     Params q = p;
     q.last = false;
     KS_TRY(side_fork(ctx, s));
+    ctx.early = false;
     kascade_status st = rank_records(ctx, l0, t.L, lists, mode, q, s);
     const kascade_status sf = root_forests(ctx, fpar, t.F, forests, false, q, ctx.side);
+    ctx.early = true;
     const kascade_status sj = side_join(ctx, s);
     if (st == KASCADE_OK) st = sf == KASCADE_OK ? sj : sf;
     KS_TRY(st);

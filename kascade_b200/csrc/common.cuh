@@ -72,6 +72,14 @@ __device__ __forceinline__ void set_error(DevStatus* st, unsigned int code, unsi
   if (atomicCAS(&st->code, 0u, code) == 0u) st->info = info;
 }
 
+// The beginning of a kernel that `launch` starts: its blocks may be in place
+// while the kernel ahead in the stream still runs, and wait here until that
+// has ended and its stores are visible.  Then the next kernel's may come.
+__device__ __forceinline__ void kernel_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // The words of a status that the host reads.
 constexpr uint32_t STATUS_WORDS = 8;
 static_assert(offsetof(DevStatus, work) == STATUS_WORDS * 8 && sizeof(DevStatus) % 8 == 0, "status words");

@@ -34,6 +34,7 @@ __global__ void __launch_bounds__(256) k_gen_forest(uint64_t n, ks_perm perm, ui
 __global__ void __launch_bounds__(256) k_initial_state(const uint64_t* __restrict__ succ, uint64_t n,
                                                        uint64_t* __restrict__ root, int64_t* __restrict__ rank,
                                                        DevStatus* st, unsigned long long* status) {
+  kernel_begin();
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t s = succ[i];
     root[i] = s;
@@ -123,8 +124,8 @@ kascade_status gen_forest(uint64_t n, uint64_t seed, uint32_t kind, uint64_t blo
 kascade_status initial_state(kascade_ctx& ctx, const uint64_t* succ, uint64_t n, uint64_t* root, int64_t* rank,
                              cudaStream_t s) {
   if (n == 0) return KASCADE_OK;
-  k_initial_state<<<grid_for(ctx, n, 256, 8), 256, 0, s>>>(succ, n, root, rank, ctx.d_status, status_host(ctx));
-  KS_CHECK_LAUNCH();
+  KS_TRY(launch(ctx, k_initial_state, grid_for(ctx, n, 256, 8), 256, 0, s, succ, n, root, rank, ctx.d_status,
+                status_host(ctx)));
   return KASCADE_OK;
 }
 

@@ -58,6 +58,7 @@ template <class F, class W>
 __global__ void __launch_bounds__(256, 4) k_prepare_arrays(const uint64_t* __restrict__ succ, W w, uint32_t n,
                                                         uint64_t start, Rulers rl, typename F::R* __restrict__ rec,
                                                         typename F::S* __restrict__ stamp, DevStatus* st) {
+  kernel_begin();
   const uint64_t tile_sz = (uint64_t)blockDim.x * PREP_ITEMS;
   for (uint64_t tile = start + (uint64_t)blockIdx.x * tile_sz; tile < n; tile += (uint64_t)gridDim.x * tile_sz) {
     unsigned long long sv[PREP_ITEMS];
@@ -101,6 +102,7 @@ __global__ void __launch_bounds__(256) k_prepare_tma(const uint64_t* __restrict_
                                                      uint32_t n, uint32_t ntiles, Rulers rl,
                                                      typename F::R* __restrict__ rec,
                                                      typename F::S* __restrict__ stamp, DevStatus* st) {
+  kernel_begin();
   constexpr uint32_t SB = PT_TILE * 8, WB = W32 ? PT_TILE * 4 : 0, STAGE = SB + WB;
   extern __shared__ __align__(128) unsigned char dyn[];
   __shared__ __align__(8) uint64_t bar[PT_STAGES];
@@ -193,6 +195,7 @@ __global__ void __launch_bounds__(512) k_chase(const typename F::R* rec, typenam
                                                uint32_t r, const uint32_t* __restrict__ rootel, NextLevel nx,
                                                uint32_t* __restrict__ work, uint32_t lanes, uint32_t hop_cap,
                                                DevStatus* st) {
+  kernel_begin();
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
   const uint32_t warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -328,6 +331,7 @@ __global__ void __launch_bounds__(256) k_propagate(const typename F::R* __restri
                                                    const uint32_t* __restrict__ rootel,
                                                    const Out* __restrict__ out_next, Sink sink, DevStatus* st,
                                                    unsigned long long* status) {
+  kernel_begin();
   __shared__ uint32_t walks[PROP_WALKS];
   __shared__ uint32_t nwalks, nfound;
   if (threadIdx.x == 0) nwalks = nfound = 0;
@@ -734,6 +738,7 @@ __device__ __forceinline__ void rank_cta(const Src& src, const Extent& ext, cons
 template <class Src, class Sink>
 __global__ void __launch_bounds__(CTA_THREADS, 1) k_rank_cta(Src src, Extent ext, Sink sink, CtaMode mode,
                                                              DevStatus* st, unsigned long long* status) {
+  kernel_begin();
   rank_cta(src, ext, sink, mode, st);
   publish_status(st, status);
 }
@@ -864,9 +869,8 @@ kascade_status launch_chase(kascade_ctx& ctx, const Levels& lv, int k, const typ
   const uint64_t need = ((uint64_t)r + lanes - 1) / lanes;  // warps worth of work
   const unsigned grid = (unsigned)std::min<uint64_t>(max_grid, (need + wpb - 1) / wpb);
   ProfScope ps(ctx, "chase", s);
-  k_chase<F><<<grid, block, 0, s>>>(rec, stamp, lv.n[k], lv.rulers[k], r, lv.rootel[k], next_level(lv, k + 1),
-                                    &ctx.d_status->work[k], lanes, hop_cap(lv.rulers[k]), ctx.d_status);
-  KS_CHECK_LAUNCH();
+  KS_TRY(launch(ctx, k_chase<F>, grid, block, 0, s, rec, stamp, lv.n[k], lv.rulers[k], r, lv.rootel[k], next_level(lv,
+                k + 1), &ctx.d_status->work[k], lanes, hop_cap(lv.rulers[k]), ctx.d_status));
   return KASCADE_OK;
 }
 
@@ -880,12 +884,12 @@ kascade_status launch_propagate(kascade_ctx& ctx, const Levels& lv, int k, const
   unsigned long long* status = status_host(ctx, last);
   if (n <= (uint64_t)ctx.usable_sms() * 256 * 8 * 4) {
     const unsigned grid = grid_for(ctx, ((uint64_t)n + 1) / 2, 256, 8);
-    k_propagate<F, Sink, 2><<<grid, 256, 0, s>>>(rec, stamp, n, lv.rulers[k], lv.rootel[k],
-                                                 lv.out[k + 1], sink, ctx.d_status, status);
+    KS_TRY(launch(ctx, k_propagate<F, Sink, 2>, grid, 256, 0, s, rec, stamp, n, lv.rulers[k], lv.rootel[k],
+                  lv.out[k + 1], sink, ctx.d_status, status));
   } else {
     const unsigned grid = grid_for(ctx, ((uint64_t)n + 7) / 8, 256, 8);
-    k_propagate<F, Sink, 8><<<grid, 256, 0, s>>>(rec, stamp, n, lv.rulers[k], lv.rootel[k],
-                                                 lv.out[k + 1], sink, ctx.d_status, status);
+    KS_TRY(launch(ctx, k_propagate<F, Sink, 8>, grid, 256, 0, s, rec, stamp, n, lv.rulers[k], lv.rootel[k],
+                  lv.out[k + 1], sink, ctx.d_status, status));
   }
   KS_CHECK_LAUNCH();
   return KASCADE_OK;
@@ -904,9 +908,8 @@ kascade_status launch_rank_cta(kascade_ctx& ctx, const Src& src, const Extent& e
   ProfScope ps(ctx, "base_case", s);
   // one ruler per thread; a small input's few barriers are cheaper with fewer warps
   const unsigned threads = ext.cap <= 1024 ? 256 : CTA_THREADS;
-  k_rank_cta<Src, Sink><<<1, threads, cta_smem(ext.cap), s>>>(src, ext, sink, mode, ctx.d_status,
-                                                                status_host(ctx, last));
-  KS_CHECK_LAUNCH();
+  KS_TRY(launch(ctx, k_rank_cta<Src, Sink>, 1, threads, cta_smem(ext.cap), s, src, ext, sink, mode, ctx.d_status,
+                status_host(ctx, last)));
   return KASCADE_OK;
 }
 
@@ -1009,8 +1012,8 @@ kascade_status prepare_plain(kascade_ctx& ctx, const uint64_t* succ, const W& w,
   if (start >= n) return KASCADE_OK;
   const uint64_t rest = n - start;
   const unsigned grid = grid_for(ctx, (rest + 256 * PREP_ITEMS - 1) / (256 * PREP_ITEMS) * 256, 256, 8);
-  k_prepare_arrays<F, W><<<grid, 256, 0, s>>>(succ, w, n, start, rl, l0.records<F>(), l0.stamps<F>(), ctx.d_status);
-  KS_CHECK_LAUNCH();
+  KS_TRY(launch(ctx, k_prepare_arrays<F, W>, grid, 256, 0, s, succ, w, n, start, rl, l0.records<F>(), l0.stamps<F>(),
+                ctx.d_status));
   return KASCADE_OK;
 }
 
@@ -1032,9 +1035,8 @@ kascade_status prepare_tiles(kascade_ctx& ctx, const uint64_t* succ, const uint3
       KS_CUDA(cudaFuncSetAttribute(k_prepare_tma<F, W32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
       raised.fetch_or(bit);
     }
-    k_prepare_tma<F, W32><<<g, 256, smem, s>>>(succ, w32, n, ntiles, rl, l0.records<F>(), l0.stamps<F>(),
-                                                ctx.d_status);
-    KS_CHECK_LAUNCH();
+    KS_TRY(launch(ctx, k_prepare_tma<F, W32>, g, 256, smem, s, succ, w32, n, ntiles, rl, l0.records<F>(),
+                  l0.stamps<F>(), ctx.d_status));
     start = (uint64_t)ntiles * PT_TILE;
   }
   return prepare_plain<F>(ctx, succ, w, n, start, l0, rl, s);

@@ -103,6 +103,7 @@ __device__ __forceinline__ uint64_t parent_of(const P* parent, uint64_t v, uint3
 template <class P>
 __global__ void __launch_bounds__(TREE_THREADS) k_tree_inner(const P* __restrict__ parent, uint32_t n,
                                                              unsigned char* __restrict__ inner, DevStatus* st) {
+  kernel_begin();
   const uint64_t tile_sz = (uint64_t)blockDim.x * TREE_PREP_ITEMS;
   for (uint64_t tile = (uint64_t)blockIdx.x * tile_sz; tile < n; tile += (uint64_t)gridDim.x * tile_sz) {
     uint64_t p[TREE_PREP_ITEMS];
@@ -143,6 +144,7 @@ __device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t* sm) {  // al
 // Vertices with children per tile of words.
 __global__ void __launch_bounds__(TREE_THREADS) k_tree_count(const unsigned char* __restrict__ inner, uint32_t words,
                                                              uint32_t* __restrict__ sums) {
+  kernel_begin();
   __shared__ uint32_t sm[TREE_THREADS / 32];
   const uint32_t base = blockIdx.x * WORDS_TILE;
   uint32_t c = 0;
@@ -160,6 +162,7 @@ __global__ void __launch_bounds__(TREE_THREADS) k_tree_count(const unsigned char
 __global__ void __launch_bounds__(TREE_THREADS) k_tree_number(const unsigned char* __restrict__ inner, uint32_t words,
                                                               const uint32_t* __restrict__ sums,
                                                               uint2* __restrict__ iw, uint32_t* __restrict__ count) {
+  kernel_begin();
   __shared__ uint32_t sm[TREE_THREADS / 32];
   __shared__ uint32_t tile[WORDS_TILE];
   uint32_t before = 0;
@@ -210,6 +213,7 @@ __global__ void __launch_bounds__(TREE_THREADS) k_tree_records(const P* __restri
                                                                uint32_t* __restrict__ rec,
                                                                uint32_t* __restrict__ vert, bool report,
                                                                DevStatus* st) {
+  kernel_begin();
   const uint64_t tile_sz = (uint64_t)blockDim.x * TREE_PREP_ITEMS;
   uint32_t downs = 0;
   for (uint64_t tile = (uint64_t)blockIdx.x * tile_sz; tile < n; tile += (uint64_t)gridDim.x * tile_sz) {
@@ -253,6 +257,7 @@ __global__ void __launch_bounds__(TREE_THREADS) k_tree_leaves(const P* parent, u
                                                               const uint2* __restrict__ iw,
                                                               const uint2* __restrict__ out, Sink sink,
                                                               DevStatus* st, unsigned long long* status) {
+  kernel_begin();
   const uint64_t tile_sz = (uint64_t)blockDim.x * TREE_OUT_ITEMS;
   for (uint64_t tile = (uint64_t)blockIdx.x * tile_sz; tile < n; tile += (uint64_t)gridDim.x * tile_sz) {
     uint64_t p[TREE_OUT_ITEMS];
@@ -298,6 +303,7 @@ __global__ void __launch_bounds__(TREE_THREADS) k_tree_chase(const typename L::R
                                                              typename N::R* __restrict__ nrec,
                                                              uint32_t* __restrict__ nroot, Rulers nrl,
                                                              uint32_t hop_cap, DevStatus* st) {
+  kernel_begin();
   const uint32_t n = ext.get(), rulers = next_ext.get();
   if (nrl.s == 0) nrl = cta_rulers(rulers);
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rulers; i += (uint64_t)gridDim.x * blockDim.x) {
@@ -340,6 +346,7 @@ __global__ void __launch_bounds__(TREE_THREADS) k_tree_propagate(const typename 
                                                                  Rulers rl, const uint32_t* __restrict__ rootel,
                                                                  const typename N::O* __restrict__ out, Sink sink,
                                                                  DevStatus* st, unsigned long long* status) {
+  kernel_begin();
   const uint32_t n = ext.get();
   for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t x = (uint32_t)v;
@@ -408,10 +415,9 @@ template <class L, class N>
 kascade_status tree_chase(kascade_ctx& ctx, const TreeLevels& lv, int k, const typename L::R* rec,
                           const uint32_t* rootel, typename N::R* nrec, uint32_t* nroot, cudaStream_t s) {
   ProfScope ps(ctx, "chase", s);
-  k_tree_chase<L, N><<<grid_for(ctx, lv.ext[k + 1].cap, TREE_THREADS, 8), TREE_THREADS, 0, s>>>(
-      rec, lv.ext[k], lv.rulers[k], lv.ext[k + 1], rootel, nrec, nroot, lv.rulers[k + 1], hop_cap(lv.rulers[k]),
-      ctx.d_status);
-  KS_CHECK_LAUNCH();
+  KS_TRY(launch(ctx, k_tree_chase<L, N>, grid_for(ctx, lv.ext[k + 1].cap, TREE_THREADS, 8), TREE_THREADS, 0, s, rec,
+                lv.ext[k], lv.rulers[k], lv.ext[k + 1], rootel, nrec, nroot, lv.rulers[k + 1], hop_cap(lv.rulers[k]),
+                ctx.d_status));
   return KASCADE_OK;
 }
 
@@ -420,9 +426,8 @@ kascade_status tree_propagate(kascade_ctx& ctx, const TreeLevels& lv, int k, con
                               const uint32_t* rootel, const typename N::O* out, const Sink& sink, bool last,
                               cudaStream_t s) {
   ProfScope ps(ctx, "propagate", s);
-  k_tree_propagate<L, N, Sink><<<grid_for(ctx, lv.ext[k].cap, TREE_THREADS, 8), TREE_THREADS, 0, s>>>(
-      rec, lv.ext[k], lv.rulers[k], rootel, out, sink, ctx.d_status, status_host(ctx, last));
-  KS_CHECK_LAUNCH();
+  KS_TRY(launch(ctx, k_tree_propagate<L, N, Sink>, grid_for(ctx, lv.ext[k].cap, TREE_THREADS, 8), TREE_THREADS, 0, s,
+                rec, lv.ext[k], lv.rulers[k], rootel, out, sink, ctx.d_status, status_host(ctx, last)));
   return KASCADE_OK;
 }
 
@@ -466,23 +471,19 @@ kascade_status root_levels(kascade_ctx& ctx, const P* parent, uint32_t n, const 
     ProfScope ps(ctx, "prepare", s);
     KS_CUDA(cudaMemsetAsync(inner, 0, 32ull * words, s));
     const unsigned grid = grid_for(ctx, ((uint64_t)n + TREE_PREP_ITEMS - 1) / TREE_PREP_ITEMS, TREE_THREADS, 8);
-    k_tree_inner<<<grid, TREE_THREADS, 0, s>>>(parent, n, inner, ctx.d_status);
-    KS_CHECK_LAUNCH();
+    KS_TRY(launch(ctx, k_tree_inner<P>, grid, TREE_THREADS, 0, s, parent, n, inner, ctx.d_status));
     if (tiles > 1) {
-      k_tree_count<<<tiles, TREE_THREADS, 0, s>>>(inner, words, sums);
-      KS_CHECK_LAUNCH();
+      KS_TRY(launch(ctx, k_tree_count, tiles, TREE_THREADS, 0, s, inner, words, sums));
     }
-    k_tree_number<<<tiles, TREE_THREADS, 0, s>>>(inner, words, sums, iw, count);
-    KS_CHECK_LAUNCH();
-    k_tree_records<<<grid, TREE_THREADS, 0, s>>>(parent, n, iw, lv.rulers[0], rec, vert, report, ctx.d_status);
-    KS_CHECK_LAUNCH();
+    KS_TRY(launch(ctx, k_tree_number, tiles, TREE_THREADS, 0, s, inner, words, sums, iw, count));
+    KS_TRY(launch(ctx, k_tree_records<P>, grid, TREE_THREADS, 0, s, parent, n, iw, lv.rulers[0], rec, vert, report,
+                  ctx.d_status));
   }
   KS_TRY((rank_tree<TreeUnit, Tree8, SinkOut8>(ctx, lv, rec, vert, SinkOut8{out}, false, s)));
   ProfScope ps(ctx, "leaves", s);
   const unsigned grid = grid_for(ctx, ((uint64_t)n + TREE_OUT_ITEMS - 1) / TREE_OUT_ITEMS, TREE_THREADS, 8);
-  k_tree_leaves<<<grid, TREE_THREADS, 0, s>>>(parent, n, iw, out, sink, ctx.d_status,
-                                              status_host(ctx, last));
-  KS_CHECK_LAUNCH();
+  KS_TRY(launch(ctx, k_tree_leaves<P, Sink>, grid, TREE_THREADS, 0, s, parent, n, iw, out, sink, ctx.d_status,
+                status_host(ctx, last)));
   return KASCADE_OK;
 }
 
