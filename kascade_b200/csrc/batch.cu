@@ -32,21 +32,33 @@ struct BatchIn {
 };
 
 // The segment hints of an element range: hint[k] is the segment of element
-// 4096 k, the last entry that of the last element.
-__global__ void __launch_bounds__(BP_THREADS) k_batch_hints(const uint32_t* __restrict__ base, uint32_t n,
-                                                            uint32_t elems, uint32_t entries,
-                                                            uint32_t* __restrict__ hint) {
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < entries; k += gridDim.x * blockDim.x) {
-    const uint32_t x = (uint32_t)min((uint64_t)k * TILE, (uint64_t)elems - 1);
-    uint32_t lo = 0, hi = n;  // the last j with base[j] <= x
-    while (hi - lo > 1) {
-      const uint32_t mid = (lo + hi) >> 1;
-      if (base[mid] <= x)
-        lo = mid;
-      else
-        hi = mid;
+// 4096 k, the last entry that of the last element.  One launch for a batch's
+// three ranges.
+struct HintJob {
+  const uint32_t* base;
+  uint32_t* hint;
+  uint32_t n, elems, entries;
+};
+struct HintJobs {
+  HintJob job[3];
+};
+__global__ void __launch_bounds__(BP_THREADS) k_batch_hints(HintJobs jobs) {
+  kernel_begin();
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const HintJob& j = jobs.job[q];
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < j.entries; k += gridDim.x * blockDim.x) {
+      const uint32_t x = (uint32_t)min((uint64_t)k * TILE, (uint64_t)j.elems - 1);
+      uint32_t lo = 0, hi = j.n;  // the last segment with base <= x
+      while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (j.base[mid] <= x)
+          lo = mid;
+        else
+          hi = mid;
+      }
+      j.hint[k] = lo;
     }
-    hint[k] = lo;
   }
 }
 
@@ -66,6 +78,7 @@ __global__ void __launch_bounds__(BP_THREADS) k_batch_prepare(BatchIn b, uint32_
                                                               typename F::R* __restrict__ rec,
                                                               typename F::S* __restrict__ stamp,
                                                               uint32_t* __restrict__ fpar, DevStatus* st) {
+  kernel_begin();
   constexpr uint32_t STEP = BP_THREADS * BP_PER;
   const uint32_t steps = (uint32_t)(((uint64_t)total + STEP - 1) / STEP);
   for (uint32_t t = blockIdx.x; t < steps; t += gridDim.x) {
@@ -190,22 +203,24 @@ kascade_status batch_upload_tables(kascade_ctx& ctx, BatchTables& t, cudaStream_
   const uint32_t* pos = d + 2ull * t.nseg;
   const uint32_t* lists = pos + t.nseg + 1;
   const uint32_t* forests = lists + 2ull * t.nl + 1;
-  auto map = [&](SegMap* m, const uint32_t* base, uint32_t n, uint64_t elems) {
+  HintJobs jobs{};
+  uint32_t most = 1;
+  auto map = [&](SegMap* m, HintJob* j, const uint32_t* base, uint32_t n, uint64_t elems) {
     m->base = base;
     m->delta = base + n + 1;
     m->n = n;
     if (elems == 0) return KASCADE_OK;
-    const uint32_t entries = (uint32_t)((elems + TILE - 1) / TILE) + 1;
-    uint32_t* hint = alloc<uint32_t>(ctx, entries);
-    if (!hint) return KASCADE_ERR_OOM;
-    m->hint = hint;
-    k_batch_hints<<<grid_for(ctx, entries, BP_THREADS, 8), BP_THREADS, 0, s>>>(base, n, (uint32_t)elems, entries, hint);
-    KS_CHECK_LAUNCH();
+    *j = HintJob{base, nullptr, n, (uint32_t)elems, (uint32_t)((elems + TILE - 1) / TILE) + 1};
+    j->hint = alloc<uint32_t>(ctx, j->entries);
+    if (!j->hint) return KASCADE_ERR_OOM;
+    m->hint = j->hint;
+    most = std::max(most, j->entries);
     return KASCADE_OK;
   };
-  KS_TRY(map(&t.pos, pos, t.nseg, t.total));
-  KS_TRY(map(&t.lists, lists, t.nl, t.L));
-  return map(&t.forests, forests, t.nf, t.F);
+  KS_TRY(map(&t.pos, &jobs.job[0], pos, t.nseg, t.total));
+  KS_TRY(map(&t.lists, &jobs.job[1], lists, t.nl, t.L));
+  KS_TRY(map(&t.forests, &jobs.job[2], forests, t.nf, t.F));
+  return launch(ctx, k_batch_hints, grid_for(ctx, most, BP_THREADS, 8), BP_THREADS, 0, s, jobs);
 }
 
 // A batch's parameters: ruler spacing and block size from the class of its
@@ -233,22 +248,21 @@ kascade_status batch_enqueue(kascade_ctx& ctx, const BatchTables& t, const uint6
     const unsigned grid = grid_for(ctx, (t.total + BP_PER - 1) / BP_PER, BP_THREADS, 8);
     auto prepare = [&](auto f, auto w) {
       using F = decltype(f);
-      k_batch_prepare<F><<<grid, BP_THREADS, 0, s>>>(BatchIn{in, t.pos, t.kinds}, (uint32_t)t.total, w, rl,
-                                                     l0.records<F>(), l0.stamps<F>(), fpar, ctx.d_status);
+      return launch(ctx, k_batch_prepare<F, decltype(w)>, grid, BP_THREADS, 0, s, BatchIn{in, t.pos, t.kinds},
+                    (uint32_t)t.total, w, rl, l0.records<F>(), l0.stamps<F>(), fpar, ctx.d_status);
     };
     if (l0.fmt == Format::F8x16)
-      prepare(F8x16{}, BWU32{weights});
+      KS_TRY(prepare(F8x16{}, BWU32{weights}));
     else if (l0.fmt == Format::F8x8)
-      prepare(F8x8{}, BWUnit{});
+      KS_TRY(prepare(F8x8{}, BWUnit{}));
     else if (l0.fmt == Format::F16i && weights)
-      prepare(F16i{}, BWU32{weights});
+      KS_TRY(prepare(F16i{}, BWU32{weights}));
     else if (l0.fmt == Format::F16i)
-      prepare(F16i{}, BWUnit{});
+      KS_TRY(prepare(F16i{}, BWUnit{}));
     else if (weights)
-      prepare(F16x16{}, BWU32{weights});
+      KS_TRY(prepare(F16x16{}, BWU32{weights}));
     else
-      prepare(F16x16{}, BWUnit{});
-    KS_CHECK_LAUNCH();
+      KS_TRY(prepare(F16x16{}, BWUnit{}));
   }
   // The forests' levels run beside the lists': neither fills the chip for long
   // (128 instances of 3e6 elements 380 -> 270 us, 4096 of 2^28 11.2 -> 10.5 ms).  A
@@ -262,10 +276,8 @@ kascade_status batch_enqueue(kascade_ctx& ctx, const BatchTables& t, const uint6
     Params q = p;
     q.last = false;
     KS_TRY(side_fork(ctx, s));
-    ctx.early = false;
     kascade_status st = rank_records(ctx, l0, t.L, lists, mode, q, s);
     const kascade_status sf = root_forests(ctx, fpar, t.F, forests, false, q, ctx.side);
-    ctx.early = true;
     const kascade_status sj = side_join(ctx, s);
     if (st == KASCADE_OK) st = sf == KASCADE_OK ? sj : sf;
     KS_TRY(st);

@@ -54,7 +54,6 @@ struct kascade_ctx {
   // a second stream for device work that is independent within a call
   cudaStream_t side = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
-  bool early = true;  // see launch()
   // size classes: a batch of at most class_max[i] records uses a ruler spacing
   // of class_spacing[i], a call that ranks one list or tour of that size
   // class_spacing_single[i]; both chase in blocks of class_block[i] threads.
@@ -130,8 +129,8 @@ struct ProfScope {
 // Launch of a kernel that begins with kernel_begin: its blocks are put in place
 // before the kernel ahead has ended, ~1 us less per launch of a call that is a
 // chain of small ones (50K forest 96 -> 84 us, pointer doubling of 1M 190 ->
-// 174, a list of 100K 88 -> 82).  Not while other work of the same call runs
-// beside it or a context has a budget of SMs: waiting blocks take slots.
+// 174, a list of 100K 88 -> 82, 32 instances of 3e4 94 -> 80).  Not while a
+// context has a budget of SMs: waiting blocks take slots.
 template <class... P, class... A>
 kascade_status launch(const kascade_ctx& ctx, void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
                       cudaStream_t s, A&&... args) {
@@ -144,7 +143,7 @@ kascade_status launch(const kascade_ctx& ctx, void (*kernel)(P...), unsigned gri
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cfg.attrs = &attr;
-  cfg.numAttrs = ctx.early && ctx.usable_sms() == ctx.sm_count ? 1 : 0;
+  cfg.numAttrs = ctx.usable_sms() == ctx.sm_count ? 1 : 0;
   return cuda_status(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
 }
 
