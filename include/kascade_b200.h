@@ -230,8 +230,9 @@ KASCADE_API kascade_status kascade_compute_stats(kascade_ctx* ctx, const uint64_
 /* ----------------------------------------------------------------------------
  * Tree rooting (device pointers).
  *   parent[v] (parent[v] == v marks a root) -> root_out[v], depth_out[v]
- *   (edge count to the root; 0 at roots), via an Euler tour of the forest
- *   ranked by the ruling-set ranker.
+ *   (edge count to the root; 0 at roots): the paths to the roots are
+ *   contracted level by level (no Euler tour is built).  Of kascade_opts,
+ *   ruler_spacing(_deep), base_case_size and seed apply.
  * Replaces: rank_via_euler_tour (eulertour.hpp:22-27, eulertour.cpp:337-377).
  * ------------------------------------------------------------------------- */
 KASCADE_API kascade_status kascade_root_forest(kascade_ctx* ctx, const uint64_t* parent,
@@ -290,15 +291,15 @@ KASCADE_API kascade_status kascade_gen_forest(uint64_t n, uint64_t seed, uint32_
                                               void* stream);
 
 /* ----------------------------------------------------------------------------
- * Batched ranking: many independent lists and forests in one call, ranked by
- * one shared ruler chase (one persistent launch, one device work queue).
+ * Batched ranking: many independent lists and forests in one call: the lists
+ * ranked by one shared ruler chase (one persistent launch, one device work
+ * queue), the forests by one contraction of their paths beside it.
  * Instances are concatenated in `input` (instance-local successor or parent
  * indices); segs[i] gives instance i's offset (= sum of the earlier sizes),
  * size and kind.  Outputs are written at the same positions: for lists root
  * and rank, for forests root and depth, roots relative to their instance.
- * weights (optional) apply to list instances.  Each instance's ruler spacing
- * comes from the context's size-class table unless opts->ruler_spacing is
- * set.  No counterpart in the reference (it ranks one distributed instance
+ * weights (optional) apply to list instances.  The lists' ruler spacing comes
+ * from the context's size-class table unless opts->ruler_spacing is set.  No counterpart in the reference (it ranks one distributed instance
  * per call).
  * ------------------------------------------------------------------------- */
 #define KASCADE_SEG_LIST 0u
@@ -316,18 +317,18 @@ KASCADE_API kascade_status kascade_rank_batch(kascade_ctx* ctx, const kascade_se
                                               uint64_t* root_out, uint64_t* rank_out,
                                               const kascade_opts* opts, void* stream);
 
-/* Size classes: an instance of at most max_size[i] elements (tour elements
- * for forests: twice the vertex count) uses mean ruler spacing spacing[i];
- * classes in increasing max_size, the last one covering everything. */
+/* Size classes: a batch of at most max_size[i] list elements uses mean ruler
+ * spacing spacing[i]; classes in increasing max_size, the last one covering
+ * everything.  (Forests have a spacing of their own.) */
 KASCADE_API kascade_status kascade_ctx_set_size_classes(kascade_ctx* ctx, const uint64_t* max_size,
                                                         const uint32_t* spacing, uint32_t count);
 KASCADE_API int kascade_ctx_get_size_classes(kascade_ctx* ctx, uint64_t* max_size, uint32_t* spacing,
                                              int cap);
-/* Per size class (same count and order as the size-class table): chains in
- * flight per chase thread (1, 2 or 4), chase block size (128, 256 or 512) and
- * the ruler spacing for calls that rank one instance on their own (NULL:
- * unchanged; the table's spacing applies inside batches).  A call uses the
- * class of its size; a batch the class that holds most of its elements.
+/* Per size class (same count and order as the size-class table): chains
+ * (accepted, no effect: a chase thread keeps one), chase block size (128, 256
+ * or 512) and the ruler spacing for calls that rank one list on their own
+ * (NULL: unchanged; the table's spacing applies inside batches).  A call uses
+ * the class of its size, a batch that of its list elements.
  * kascade_ctx_set_size_classes resets these to 2, 256 and its own spacing. */
 KASCADE_API kascade_status kascade_ctx_set_class_launch(kascade_ctx* ctx, const uint32_t* chains,
                                                         const uint32_t* block, const uint32_t* single_spacing,
@@ -349,7 +350,7 @@ KASCADE_API kascade_status kascade_ctx_set_sm_budget(kascade_ctx* ctx, int sms);
  * ------------------------------------------------------------------------- */
 typedef struct kascade_server kascade_server;
 /* Batch plans: one batch captured once as a CUDA graph (the whole pipeline:
- * record build, forest tours, every ruling-set level, propagation) and
+ * record build, every level of the lists and of the forests, outputs) and
  * replayed by one graph launch per call.  The segment table
  * and the input / weight / output pointers are fixed at creation; their
  * contents may change between launches.  Creation runs the batch once and

@@ -203,18 +203,17 @@ KASCADE_API kascade_status kascade_ctx_reserve(kascade_ctx* c, uint64_t bytes) {
 }
 
 KASCADE_API uint64_t kascade_scratch_bytes_rank_list(uint64_t n) {
-  // level-0 records (16n) + ruler list (4n) + write-free path: log (16n,
-  // reused by the second partition pass), window partition (16n rounded up
-  // to whole 2^20-element windows), a margin of n, level-1 records/results
-  // and deeper levels + per-warp log chunks, cursors and window rounding
+  // level-0 records (8n or 16n) and write-free path: log (16n, reused by the
+  // second partition pass), window partition (16n rounded up to whole
+  // 2^20-element windows), level-1 records/results and deeper levels + per-warp
+  // log chunks, cursors and window rounding, with a margin of 5n
   return 16 * n + 4 * n + 16 * n + 16 * n + n + (40 * n) / 16 + (192ull << 20);
 }
 
 KASCADE_API uint64_t kascade_scratch_bytes_root_forest(uint64_t n) {
-  // tour records on 2n slots (32n) + ruler list (8n) + child lists, packed
-  // parents and bit tables (~13n) + write-free level 0 over the <= 2n tour
-  // elements: log (32n), first-pass windows (16n) + deeper levels, with
-  // headroom
+  // an upper bound that also holds for a batch of n elements: rooting needs
+  // ~18n for level 0 (child flags, numbers, records, results) and at most 20n
+  // for the levels above, a batch's lists what rank_list needs
   return 16 * n + 8 * n + 32 * n + 8 * n + 32 * n + 16 * n + (80 * n) / 16 + (192ull << 20);
 }
 

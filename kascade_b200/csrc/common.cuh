@@ -64,8 +64,7 @@ struct DevStatus {
   // [1]: level 0's size, when only the device knows it; [2], [3]: elements
   // stamped by chains / found stamped (more of the former: two chains met)
   unsigned long long counter[6];
-  unsigned int work[31];          // per level: rulers handed out beyond the warps' first shares
-  unsigned int heads;             // tour heads found
+  unsigned int work[32];          // per level: rulers handed out beyond the warps' first shares
 };
 
 __device__ __forceinline__ void set_error(DevStatus* st, unsigned int code, unsigned long long info) {
@@ -161,8 +160,7 @@ __device__ __forceinline__ void st_rec_cs(Rec* p, Rec r) {
 // index arithmetic (it was a third of the chase's instructions) and a chain
 // knows that it ends before it asks for another record.  8 B records keep that
 // bit in the successor word: at most 2^31 elements.
-//   F8x8   32-bit weights whose distances are wanted modulo 2^32 only (unit
-//          weights: a chain is shorter; tours: depths), 8 B stamps
+//   F8x8   unit weights (a chain is shorter than 2^32), 8 B stamps
 //   F8x16  32-bit weights, 64-bit distances
 //   F16x16 64-bit weights (in-place calls, every deeper level)
 //   F16i   any weights, the stamp stored into the record: half the memory of

@@ -128,7 +128,7 @@ kascade_status status_finish(kascade_ctx& ctx, cudaStream_t s) {
   }
   collect_times(ctx);
   const DevStatus* st = reinterpret_cast<const DevStatus*>(ctx.h_pinned);
-  // level 0's size when only the device knew it (a tour sized for a bound)
+  // level 0's size when only the device knew it (a forest's)
   if (st->counter[1] && !ctx.last_levels.empty()) ctx.last_levels[0] = st->counter[1];
   ctx.error_info = st->info;
   ctx.last_status = (kascade_status)st->code;

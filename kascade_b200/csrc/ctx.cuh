@@ -55,7 +55,7 @@ struct kascade_ctx {
   cudaStream_t side = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
   // size classes: a batch of at most class_max[i] records uses a ruler spacing
-  // of class_spacing[i], a call that ranks one list or tour of that size
+  // of class_spacing[i], a call that ranks one list of that size
   // class_spacing_single[i]; both chase in blocks of class_block[i] threads.
   // (class_chains: kept for its callers, no effect.)  Defaults: the tuned table.
   std::vector<unsigned long long> class_max = KS_TUNED_MAX;

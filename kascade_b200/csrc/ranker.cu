@@ -1,4 +1,4 @@
-// Ruling-set list ranker and pointer doubling for one B200.
+// Ruling-set list ranker for one B200.
 //
 // Reference counterparts (niklas-uhl/kascade):
 //   ruler sampling      lib/kascade/sparse_ruling_set_detail/ruler_selection.hpp:18-115,
@@ -14,7 +14,8 @@
 //                       dense ruler-id space
 //   propagation (pull)  ruler_propagation.hpp:148-256 -> one coalesced pass
 //   pointer doubling    pointer_doubling_generic.hpp:43-60, 171-212, 418-438,
-//                       609-700 -> double-buffered jump kernel
+//                       609-700 -> the jump kernel of a last level that the caller's
+//                       depth limit leaves larger than one CTA; the calls: tree.cu
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -516,7 +517,7 @@ __device__ __forceinline__ void rank_cta(const Src& src, const Extent& ext, cons
     ends = __reduce_add_sync(FULL, ends);
     if ((tid & 31u) == 0 && ends) atomicAdd(&nends, ends);
     __syncthreads();
-    if (mode == CTA_ROOTING) {  // report the tour's length: the vertices, and those between a root and a leaf again
+    if (mode == CTA_ROOTING) {  // the call's size: the vertices, and again those between a root and a leaf
       for (uint32_t w = tid; w < (n + 3) / 4; w += nthreads) predw[w] = 0;
       __syncthreads();
       for (uint32_t x = tid; x < n; x += nthreads) {
@@ -766,32 +767,23 @@ __global__ void __launch_bounds__(256) k_pd_init(const Rec* __restrict__ rec, Ex
 }
 
 // One round of pointer jumping over the previous round's records `a`: an
-// element not yet at its root follows its pointer JUMPS times there (a chain
+// element not yet at its root follows its pointer three times there (a chain
 // of dependent reads of `a` only, never of `b`), so a round multiplies every
-// pointer's reach by JUMPS + 1.  JUMPS = 1 is classic doubling; the last level
-// of the device-driven recursion (at most 2^17 elements, L2-resident, a fixed
-// number of launches) takes JUMPS = 3: half the launches for three reads each.
-template <int JUMPS>
-__global__ void __launch_bounds__(256) k_pd_round(const PdRec* __restrict__ a, PdRec* __restrict__ b, Extent ext,
-                                                  uint32_t* __restrict__ active) {
+// pointer's reach by four: half the launches of single jumps.
+__global__ void __launch_bounds__(256) k_pd_round(const PdRec* __restrict__ a, PdRec* __restrict__ b, Extent ext) {
   const uint32_t n = ext.get();
-  uint32_t cnt = 0;
   for (uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (uint64_t)gridDim.x * blockDim.x) {
     PdRec e = a[x];
 #pragma unroll
-    for (int j = 0; j < JUMPS; ++j) {
+    for (int j = 0; j < 3; ++j) {
       if (e.done & 1u) break;
       const PdRec t = a[e.succ];
       e.rank += t.rank;
       e.succ = t.succ;
       e.done = t.done & 1u;
     }
-    cnt += (e.done & 1u) ? 0u : 1u;
     b[x] = e;
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(FULL, cnt, o);
-  if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(active, cnt);
 }
 
 template <class Sink>
@@ -1106,8 +1098,7 @@ static kascade_status pointer_double_level(kascade_ctx& ctx, const Rec* rec, con
   const uint32_t m = ext.cap;
   PdRec* a = alloc<PdRec>(ctx, m);
   PdRec* b = alloc<PdRec>(ctx, m);
-  uint32_t* active = alloc<uint32_t>(ctx, 1);
-  if (!a || !b || !active) return KASCADE_ERR_OOM;
+  if (!a || !b) return KASCADE_ERR_OOM;
   const unsigned grid = grid_for(ctx, m, 256, 8);
   ProfScope ps(ctx, "pd_final_level", s);
   k_pd_init<<<grid, 256, 0, s>>>(rec, ext, a, ctx.d_status);
@@ -1117,7 +1108,7 @@ static kascade_status pointer_double_level(kascade_ctx& ctx, const Rec* rec, con
   while ((1ull << lg) < m) ++lg;
   const int rounds = (lg + 1) / 2 + 1;
   for (int i = 0; i < rounds; ++i) {
-    k_pd_round<3><<<grid, 256, 0, s>>>(a, b, ext, active);
+    k_pd_round<<<grid, 256, 0, s>>>(a, b, ext);
     KS_CHECK_LAUNCH();
     std::swap(a, b);
   }

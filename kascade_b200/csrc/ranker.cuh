@@ -85,17 +85,16 @@ __host__ __device__ inline Rulers cta_rulers(uint32_t n) {
 inline uint32_t salt_for(uint32_t seed, int level) { return mix32(seed + 0x9E3779B9u * (uint32_t)(level + 1)); }
 inline uint32_t ruler_count(uint32_t n, const Rulers& r) { return (uint32_t)(((uint64_t)n + r.s - 1) / r.s); }
 
-// A level's element count when only the device knows it: (base + *add) / div,
-// rounded up, at most the capacity the launch was sized for (add == nullptr:
-// the capacity).
+// A level's element count when only the device knows it: *count / div, rounded
+// up, at most the capacity the launch was sized for (count == nullptr: the
+// capacity).
 struct Extent {
   uint32_t cap = 0;
-  uint32_t base = 0;
-  const uint32_t* add = nullptr;
+  const uint32_t* count = nullptr;
   uint32_t div = 1;
   __device__ __forceinline__ uint32_t get() const {
-    if (!add) return cap;
-    uint32_t v = (uint32_t)min((uint64_t)0xFFFFFFFFu, (uint64_t)base + __ldg(add));
+    if (!count) return cap;
+    uint32_t v = __ldg(count);
     if (div != 1) v = v / div + (v % div != 0u ? 1u : 0u);
     return min(cap, v);
   }
@@ -201,7 +200,7 @@ struct Level0 {
   template <class F>
   typename F::S* stamps() const { return static_cast<typename F::S*>(stamp); }
 };
-// How level 0 of n elements of that weight kind (tours: Unit) runs: the
+// How level 0 of n elements of that weight kind runs: the
 // records' format, and whether it takes the write-free path.
 struct Level0Plan {
   Format fmt;
@@ -223,7 +222,7 @@ uint32_t hop_cap(const Rulers& rl);
 constexpr uint32_t ONE_CTA_MAX = 14336;
 constexpr uint32_t ONE_CTA_TREES = 8192;
 // What the one-CTA ranker takes: lists only; lists, and trees up to
-// ONE_CTA_TREES elements; trees; trees whose tour's length is to be reported.
+// ONE_CTA_TREES elements; trees; trees, reporting their size as an Euler tour.
 enum CtaMode : uint32_t { CTA_LISTS, CTA_SMALL_TREES, CTA_TREES, CTA_ROOTING };
 kascade_status rank_arrays_one_cta(kascade_ctx& ctx, const uint64_t* succ, WKind wk, const void* w, uint32_t n,
                                    const SinkPlain& sink, CtaMode mode, cudaStream_t s);

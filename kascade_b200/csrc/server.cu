@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(256) k_gather(const Piece* __restrict__ pieces
 
 uint64_t footprint_of(uint32_t kind, uint64_t n, bool w) {
   // input + weights + result (in its batch) + the batch's concatenated input
-  // + ranking scratch (forests: sort, tour records and log on 2n tour slots)
+  // + ranking scratch
   const uint64_t io = n * (8 + (w ? 4 : 0)) * 2 + 16 * n;
   const uint64_t scratch =
       kind == KASCADE_SEG_FOREST ? kascade_scratch_bytes_root_forest(n) : kascade_scratch_bytes_rank_list(n);
@@ -552,11 +552,8 @@ void kascade_server::lane_loop(int lane) {
       kascade_opts_init(&o);
       o.profile = tracing ? 1 : 0;
       // Both lanes enqueue their whole recursion at once (one host wait per
-      // batch).  The throughput lane took the host-driven recursion before,
-      // so that each level's launches took the SM budget in force when made;
-      // with its batches in the SM partition while the latency lane has work,
-      // the device-driven form serves 3% more (1.16 -> 1.19e10 elements/s on
-      // the 20k req/s mix) for 0.4 ms more on the <=2^20 p99 (3.9 -> 4.3 ms).
+      // batch); the throughput lane's batches run in the SM partition while
+      // the latency lane has work.
       st = kascade_rank_batch(C, segs.data(), (uint32_t)segs.size(), d_in, any_w ? d_w : nullptr, elems, b->d_root,
                               b->d_rank, &o, S);
     }

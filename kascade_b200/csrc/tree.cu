@@ -205,8 +205,9 @@ __device__ __forceinline__ uint32_t number_of(uint2 w, uint32_t v) {
 }
 
 // The records of the numbered vertices; vert: their vertices (the roots').
-// report: the tour's length, the vertices and once more those with children
-// that are not roots, goes to the status.
+// report: the elements of the forest's Euler tour with a leaf's two edges as
+// one (the vertices, and once more those with children that are not roots), the
+// size a call reports for level 0, go to the status.
 template <class P>
 __global__ void __launch_bounds__(TREE_THREADS) k_tree_records(const P* __restrict__ parent, uint32_t n,
                                                                const uint2* __restrict__ iw, Rulers rl,
@@ -396,13 +397,13 @@ TreeLevels plan_tree(uint32_t n, const uint32_t* count, const Params& p) {
   const uint32_t base = std::max(1u, std::min(p.base_max, TREE_BASE));
   int k = 0;
   lv.ext[0].cap = n;
-  lv.ext[0].add = count;
+  lv.ext[0].count = count;
   while (lv.ext[k].cap > base && k < MAX_LEVELS) {
     const uint32_t given = k == 0 ? p.spacing_given : p.spacing_deep;
     const uint32_t s = given ? std::max(2u, given) : lv.ext[k].cap > TREE_LARGE ? TREE_SPACING_LARGE : TREE_SPACING;
     lv.rulers[k] = make_rulers(s, salt_for(p.seed, k));
     lv.ext[k + 1].cap = ruler_count(lv.ext[k].cap, lv.rulers[k]);
-    lv.ext[k + 1].add = count;
+    lv.ext[k + 1].count = count;
     lv.ext[k + 1].div = (uint32_t)std::min<uint64_t>((uint64_t)lv.ext[k].div * lv.rulers[k].s, 0xFFFFFFFFu);
     ++k;
   }
