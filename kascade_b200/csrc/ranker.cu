@@ -866,8 +866,10 @@ kascade_status launch_chase(kascade_ctx& ctx, const Levels& lv, int k, const typ
   return KASCADE_OK;
 }
 
-// Level k's results from level k + 1's.  Small levels take two elements per
-// thread instead of eight, so that they fill the chip.
+// Level k's results from level k + 1's.  Four elements a thread (eight took 86
+// registers, a quarter of the SM's warps: 6e6 elements in place 403 -> 394 us,
+// a list of 2e6 176 -> 170; two: 401 and 171), two on small levels, so that
+// they fill the chip.
 template <class F, class Sink>
 kascade_status launch_propagate(kascade_ctx& ctx, const Levels& lv, int k, const typename F::R* rec,
                                 const typename F::S* stamp, const Sink& sink, bool last, cudaStream_t s) {
@@ -879,8 +881,8 @@ kascade_status launch_propagate(kascade_ctx& ctx, const Levels& lv, int k, const
     KS_TRY(launch(ctx, k_propagate<F, Sink, 2>, grid, 256, 0, s, rec, stamp, n, lv.rulers[k], lv.rootel[k],
                   lv.out[k + 1], sink, ctx.d_status, status));
   } else {
-    const unsigned grid = grid_for(ctx, ((uint64_t)n + 7) / 8, 256, 8);
-    KS_TRY(launch(ctx, k_propagate<F, Sink, 8>, grid, 256, 0, s, rec, stamp, n, lv.rulers[k], lv.rootel[k],
+    const unsigned grid = grid_for(ctx, ((uint64_t)n + 3) / 4, 256, 8);
+    KS_TRY(launch(ctx, k_propagate<F, Sink, 4>, grid, 256, 0, s, rec, stamp, n, lv.rulers[k], lv.rootel[k],
                   lv.out[k + 1], sink, ctx.d_status, status));
   }
   KS_CHECK_LAUNCH();

@@ -28,6 +28,7 @@ namespace {
 
 constexpr int TREE_THREADS = 256;
 constexpr int TREE_PREP_ITEMS = 8;
+constexpr int TREE_REC_ITEMS = 4;  // (8: 95 registers; 2^26 vertices 3.89 -> 3.83 ms, 4.2e6 228 -> 221 us)
 constexpr int TREE_OUT_ITEMS = 4;  // (2: 1.07 ms, 4 and 8: 0.95 for 2^26 vertices)
 // Mean elements per ruler.  Large levels are bound by what they read at
 // random, (s + 1) s / (s - 1) reads an element over all levels; small ones by
@@ -215,26 +216,26 @@ __global__ void __launch_bounds__(TREE_THREADS) k_tree_records(const P* __restri
                                                                uint32_t* __restrict__ vert, bool report,
                                                                DevStatus* st) {
   kernel_begin();
-  const uint64_t tile_sz = (uint64_t)blockDim.x * TREE_PREP_ITEMS;
+  const uint64_t tile_sz = (uint64_t)blockDim.x * TREE_REC_ITEMS;
   uint32_t downs = 0;
   for (uint64_t tile = (uint64_t)blockIdx.x * tile_sz; tile < n; tile += (uint64_t)gridDim.x * tile_sz) {
-    uint64_t p[TREE_PREP_ITEMS];
-    uint2 own[TREE_PREP_ITEMS], up[TREE_PREP_ITEMS];
+    uint64_t p[TREE_REC_ITEMS];
+    uint2 own[TREE_REC_ITEMS], up[TREE_REC_ITEMS];
 #pragma unroll
-    for (int i = 0; i < TREE_PREP_ITEMS; ++i) {
+    for (int i = 0; i < TREE_REC_ITEMS; ++i) {
       const uint64_t v = tile + (uint64_t)i * blockDim.x + threadIdx.x;
       p[i] = parent_of(parent, v, n);
       own[i] = v < n ? __ldg(iw + (v >> 5)) : make_uint2(0, 0);
     }
 #pragma unroll
-    for (int i = 0; i < TREE_PREP_ITEMS; ++i) {
+    for (int i = 0; i < TREE_REC_ITEMS; ++i) {
       const uint64_t v = tile + (uint64_t)i * blockDim.x + threadIdx.x;
       if (p[i] >= n) p[i] = v;
       if (!((own[i].x >> (v & 31)) & 1u)) p[i] = ~0ull;  // a leaf
       up[i] = p[i] < n ? __ldg(iw + (p[i] >> 5)) : make_uint2(0, 0);
     }
 #pragma unroll
-    for (int i = 0; i < TREE_PREP_ITEMS; ++i) {
+    for (int i = 0; i < TREE_REC_ITEMS; ++i) {
       const uint64_t v = tile + (uint64_t)i * blockDim.x + threadIdx.x;
       if (p[i] >= n) continue;
       const uint32_t c = number_of(own[i], (uint32_t)v);
@@ -477,7 +478,8 @@ kascade_status root_levels(kascade_ctx& ctx, const P* parent, uint32_t n, const 
       KS_TRY(launch(ctx, k_tree_count, tiles, TREE_THREADS, 0, s, inner, words, sums));
     }
     KS_TRY(launch(ctx, k_tree_number, tiles, TREE_THREADS, 0, s, inner, words, sums, iw, count));
-    KS_TRY(launch(ctx, k_tree_records<P>, grid, TREE_THREADS, 0, s, parent, n, iw, lv.rulers[0], rec, vert, report,
+    const unsigned rec_grid = grid_for(ctx, ((uint64_t)n + TREE_REC_ITEMS - 1) / TREE_REC_ITEMS, TREE_THREADS, 8);
+    KS_TRY(launch(ctx, k_tree_records<P>, rec_grid, TREE_THREADS, 0, s, parent, n, iw, lv.rulers[0], rec, vert, report,
                   ctx.d_status));
   }
   KS_TRY((rank_tree<TreeUnit, Tree8, SinkOut8>(ctx, lv, rec, vert, SinkOut8{out}, false, s)));
