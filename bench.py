@@ -49,45 +49,46 @@ WORKLOADS = {
 # Algorithmic bytes per unit (HBM roofline, integer work): stream-read succ
 # (8 B) + weights (4 B) + stream-write root and rank (16 B) + one random 32 B
 # sector for the dependent successor load.  Forest: 8 B parent + 16 B outputs
-# + 2 tour elements x (32 B random sector + 16 B streamed tour state).
-B_ALG = {"list": lambda w: 8 + (4 if w else 0) + 16 + 32, "forest": lambda w: 8 + 16 + 2 * (32 + 16)}
+# + one random 32 B sector for the parent's result.
+B_ALG = {"list": lambda w: 8 + (4 if w else 0) + 16 + 32, "forest": lambda w: 8 + 16 + 32}
 # The chase kernel's algorithmic bytes per element it visits: the one random
-# 32 B sector its dependent 16 B record read lands in.  The implementation
+# 32 B sector its dependent record read lands in.  The implementation
 # also writes 16 B per visit (the log entry of the write-free chase, or the
 # stamp of the stamping chase); that figure is reported beside it.
 B_CHASE = 32
 B_CHASE_IMPL = 32 + 16
 # Random-access roofline, stated as 32 B sectors touched x 32 B / peak: the
 # sectors the ranking pipeline touches per level-0 list element.  prepare:
-# succ 8 B (1/4 sector) + weight 4 B (1/8) + record write 16 B (1/2); chase:
-# the record's random sector read + its stamp written back (1 + 1);
-# propagate: record read (1/2) + the ruler result's random sector (1) + root
-# and rank writes (1/2).  Deeper levels add ~2% and are left out.
-SECTORS_LIST = {True: 0.25 + 0.125 + 0.5 + 2 + 2, False: 0.25 + 0.5 + 2 + 2}
-# The same count for the write-free level 0 (the default from 2^25 elements):
-# prepare as above; chase: the record's random sector read + the 16 B log
-# entry (1 + 1/2); resolve: log read + resolved entry written (1/2 + 1/2; its
-# ruler lookups hit L1 for the most part and are left out); partition: read +
-# write (1/2 + 1/2); place: read (1/2) + root and rank writes (1/2).
-SECTORS_LIST_LOG = {True: 0.25 + 0.125 + 0.5 + 1.5 + 1 + 1 + 1, False: 0.25 + 0.5 + 1.5 + 1 + 1 + 1}
+# succ 8 B (1/4 sector) + weight 4 B (1/8) + record write 8 B (1/4); chase:
+# the record's random sector read + a stamp's random sector written (1 + 1);
+# propagate: stamp read (8 B 1/4, 16 B for weights 1/2) + the ruler result's
+# random sector (1) + root and rank writes (1/2).  Deeper levels add ~2% and
+# are left out.
+SECTORS_LIST = {True: 0.25 + 0.125 + 0.25 + 2 + 2, False: 0.25 + 0.25 + 2 + 1.75}
+# The same count for the write-free level 0 (the default from 8 million
+# elements): prepare as above; chase: the record's random sector read + the
+# 16 B log entry (1 + 1/2); resolve: log read + resolved entry written (1/2 +
+# 1/2; its ruler lookups hit L1 for the most part and are left out); partition
+# (from 2^25 elements): read + write (1/2 + 1/2); place: read (1/2) + root and
+# rank writes (1/2).
+SECTORS_LIST_LOG = {True: 0.25 + 0.125 + 0.25 + 1.5 + 1 + 1 + 1, False: 0.25 + 0.25 + 1.5 + 1 + 1 + 1}
 # DRAM bytes the write-free pipeline's kernels move, measured by ncu
 # (dram__bytes_read.sum + dram__bytes_write.sum) on a weighted 2^25-element
 # list: per element for the streaming kernels, per record read for the chase.
 # Scaled to a run, they give the traffic the pipeline really moves (the
 # measured form of "sectors touched").
 NCU_LIST_N = 1 << 25
-DRAM_PER_ELEM_LOG = {"prepare": (402.7e6 + 480.9e6) / NCU_LIST_N, "resolve": (554.3e6 + 480.4e6) / NCU_LIST_N,
-                     "partition": (537.1e6 + 480.8e6) / NCU_LIST_N, "place": (537.0e6 + 480.8e6) / NCU_LIST_N}
+DRAM_PER_ELEM_LOG = {"prepare": (402.7e6 + 223.3e6) / NCU_LIST_N, "resolve": (571.2e6 + 479.4e6) / NCU_LIST_N,
+                     "partition": (537.1e6 + 476.5e6) / NCU_LIST_N, "place": (537.1e6 + 479.4e6) / NCU_LIST_N}
 # DRAM bytes the level-0 stamping chase moves per record it reads (ncu on a
-# 2^25-element list: 3.924 GB read + 1.036 GB written over 2^25 + 2 797 812
-# record reads, every element once plus each chain's closing ruler record).
-CHASE_NCU_VISITS = NCU_LIST_N + 2_797_812
-CHASE_DRAM_BYTES_PER_VISIT = (3.924e9 + 1.036e9) / CHASE_NCU_VISITS
-# The same for the write-free chase (k_chase_log), which reads each record
-# and appends a 16 B log entry: 3.901 GB read + 0.560 GB written over 2^25 +
-# 1 048 211 record reads.
-CHASE_LOG_NCU_VISITS = NCU_LIST_N + 1_048_211
-CHASE_LOG_DRAM_BYTES_PER_VISIT = (3.900669e9 + 0.560097e9) / CHASE_LOG_NCU_VISITS
+# 2^25-element list, stamps in 16 B records: 3.807 GB read + 1.097 GB written
+# over 2^25 record reads; a chain ends in front of the next ruler).
+CHASE_NCU_VISITS = NCU_LIST_N
+CHASE_DRAM_BYTES_PER_VISIT = (3.8067e9 + 1.0973e9) / CHASE_NCU_VISITS
+# The same for the write-free chase (k_chase_log), which reads each 8 B record
+# and appends a 16 B log entry: 3.274 GB read + 0.630 GB written.
+CHASE_LOG_NCU_VISITS = NCU_LIST_N
+CHASE_LOG_DRAM_BYTES_PER_VISIT = (3.2744e9 + 0.6298e9) / CHASE_LOG_NCU_VISITS
 
 
 def log(*a):
@@ -382,7 +383,7 @@ def measure_batched(kb, ctx, dev, steps: int = 3) -> dict:
                  "speedup_vs_plain": round(tp / tg, 2),
                  "results_equal": bool(torch.equal(root, root2) and torch.equal(rk, rk2))}
         plan.close()
-    except kb.KascadeError as e:  # a batch the device-driven recursion cannot hold
+    except kb.KascadeError as e:  # a batch a plan cannot hold
         graph = {"unavailable": str(e)}
     return {"workload": "4096 instances, sizes log-uniform in [2^6,2^22] rescaled to sum 2^28, 70% weighted lists / "
                         "30% random recursive forests, one kascade_rank_batch call",
@@ -712,7 +713,7 @@ def random_access_roofline(r: dict, hbm: float) -> dict | None:
     the pipeline that ran touches per list element."""
     if r["kind"] != "list":
         return None
-    n, weighted, write_free, levels = r["n"], r["weighted"], r["write_free"], r["levels"]
+    n, weighted, write_free = r["n"], r["weighted"], r["write_free"]
     ms = r["ms_per_step"]
     sectors = (SECTORS_LIST_LOG if write_free else SECTORS_LIST)[bool(weighted)]
     floor_ms = n * 32 * sectors / (hbm * 1e9) * 1000.0
@@ -722,8 +723,8 @@ def random_access_roofline(r: dict, hbm: float) -> dict | None:
            "bytes_per_element": 32 * sectors, "floor_ms": round(floor_ms, 3), "frac": round(floor_ms / ms, 4),
            "sectors_min_design": sectors_min, "frac_min_design": round(floor_min_ms / ms, 4), "peak_gbs": hbm}
     if write_free and weighted:
-        visits = sum(levels[:2]) if len(levels) > 1 else n
-        dram = n * sum(DRAM_PER_ELEM_LOG.values()) + visits * CHASE_LOG_DRAM_BYTES_PER_VISIT
+        passes = sum(v for k, v in DRAM_PER_ELEM_LOG.items() if k != "partition" or k in r["ktimes"])
+        dram = n * (passes + CHASE_LOG_DRAM_BYTES_PER_VISIT)
         out["measured"] = {"bytes_per_element": round(dram / n, 1), "sectors_per_element": round(dram / n / 32, 2),
                            "achieved_gbs": round(dram / (ms / 1000.0) / 1e9, 1),
                            "frac": round(dram / (ms / 1000.0) / 1e9 / hbm, 4),
