@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(256) k_propagate(const typename F::R* __restri
 // thread at 8192: 51 us) each element is touched once.  Each element's word
 // also says whether its successor is a ruler, so a hop is one read and one
 // write of the word and of the distance.  Bound by one SM's shared-memory
-// pipe and instructions: 1000 elements 8.7 us, 4000 14.7, 8000 18.2, 14.3
+// pipe and instructions: 1000 elements 9.9 us, 4000 14.7, 8000 18.2, 14.3
 // thousand 27 (46 with a pass of its own for the ruler bits, three barriers a
 // jumping round and a predecessor byte per element in every case).
 // With several lists, their heads (no predecessor) start chains as well, so
@@ -483,7 +483,7 @@ __device__ __forceinline__ void rank_cta(const Src& src, const Extent& ext, cons
     return all || rl.is(x, &j);
   };
   auto elem = [&](uint32_t j) { return all ? j : (uint32_t)rl.elem(j); };
-  bool stamp = mode <= CTA_SMALL_TREES;
+  bool stamp = mode <= CTA_SMALL_TREES && !all;  // (chains of one element pass none)
   uint32_t heads = 0;
   while (true) {
     if (tid == 0) nends = nheads = nstamps = 0;
@@ -900,8 +900,10 @@ kascade_status launch_rank_cta(kascade_ctx& ctx, const Src& src, const Extent& e
     raised.fetch_or(bit);
   }
   ProfScope ps(ctx, "base_case", s);
-  // one ruler per thread; a small input's few barriers are cheaper with fewer warps
-  const unsigned threads = ext.cap <= 1024 ? 256 : CTA_THREADS;
+  // one ruler per thread; a small input's few barriers are cheaper with fewer
+  // warps (a list of 1000: 128 / 256 / 512 / 1024 threads 14.9 / 11.0 / 9.9 / 10.2
+  // us, of 64: 6.2 / 6.2 / 6.3 / 6.9)
+  const unsigned threads = ext.cap <= 256 ? 256 : ext.cap <= 1024 ? 512 : CTA_THREADS;
   KS_TRY(launch(ctx, k_rank_cta<Src, Sink>, 1, threads, cta_smem(ext.cap), s, src, ext, sink, mode, ctx.d_status,
                 status_host(ctx, last)));
   return KASCADE_OK;
