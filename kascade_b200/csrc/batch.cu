@@ -285,7 +285,7 @@ kascade_status batch_enqueue(kascade_ctx& ctx, const BatchTables& t, const uint6
     KS_TRY(root_forests(ctx, fpar, t.F, forests, t.L == 0, p, s));
     KS_TRY(rank_records(ctx, l0, t.L, lists, mode, p, s));
   }
-  ctx.last_levels[0] = t.total;
+  ctx.last_levels[0] = t.total + t.F;  // as a batch's size is reported: a forest's vertex counts twice
   return KASCADE_OK;
 }
 
