@@ -52,6 +52,9 @@ kascade_status begin_call(kascade_ctx* ctx, cudaStream_t s, const kascade_opts* 
 }
 
 kascade_status end_call(kascade_ctx* ctx, cudaStream_t s, kascade_status st, const kascade_opts* o) {
+  // before the event that a call on another stream waits for: that call's
+  // status is not cleared by this one's
+  if (st == KASCADE_OK) st = status_publish(*ctx, s);
   cudaEventRecord(ctx->done_event, s);
   ctx->last_stream = s;
   if (st != KASCADE_OK) {
@@ -64,7 +67,7 @@ kascade_status end_call(kascade_ctx* ctx, cudaStream_t s, kascade_status st, con
   }
   if (o && o->async) {
     ctx->async_pending = true;
-    return status_publish(*ctx, s);
+    return KASCADE_OK;
   }
   return status_finish(*ctx, s);
 }

@@ -85,3 +85,33 @@ def test_plan_replays_both_spaces(kb, oracle_mod):
     x.copy_(dev64(succ))
     root, rank = plan.launch()
     np.testing.assert_array_equal(host_u64(rank), rank_o)
+
+
+def test_status_of_calls_on_two_streams(kb, oracle_mod):
+    """An async call's status is published before a call on another stream
+    starts: that call's error is its own, and neither leaks into the next."""
+    import ctypes
+
+    rng = np.random.default_rng(5)
+    sizes, kinds = [400_000, 300_000], [kb.SEG_LIST, kb.SEG_FOREST]
+    succ, _, root_o, rank_o = _batch(kb, oracle_mod, sizes, kinds, rng, False)
+    x, segs = dev64(succ), kb.make_segments(np.array(sizes, np.int64), np.array(kinds, np.int64))
+    bad = dev64(np.array([1, 7, 2], np.uint64))
+    good = dev64(np.array([1, 1, 1], np.uint64))
+    ctx = kb.Context()
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for _ in range(20):
+        with torch.cuda.stream(a):
+            root, rank = kb.rank_batch(x, segs, tuning=kb.GpuTuning(async_=True), ctx=ctx)
+        with torch.cuda.stream(b):
+            with pytest.raises(kb.KascadeError) as e:
+                kb.rank_list(bad, ctx=ctx)
+            assert e.value.name == "OUT_OF_RANGE"
+            assert kb.rank_list(good, ctx=ctx)[1].tolist() == [1, 0, 1]
+        with torch.cuda.stream(a):
+            root, rank = kb.rank_batch(x, segs, tuning=kb.GpuTuning(async_=True), ctx=ctx)
+            kb._lib.check(kb.lib.kascade_ctx_sync(ctx.handle, ctypes.c_void_p(a.cuda_stream)), "kascade_ctx_sync", ctx.handle)
+        np.testing.assert_array_equal(host_u64(root), root_o)
+        np.testing.assert_array_equal(host_u64(rank), rank_o)
+    ctx.close()
