@@ -18,6 +18,7 @@
 // of n walks is s ln n.  Walks only read: elements near the roots, which many
 // walks pass, stay in L1.
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "ranker.cuh"
@@ -28,6 +29,10 @@ namespace {
 
 constexpr int TREE_THREADS = 256;
 constexpr int TREE_PREP_ITEMS = 8;
+// Child flags in bytes up to here, see k_tree_inner; beside a batch's lists to
+// twice that (8e7 vertices of a 2^28-element batch: 10.0 ms, 10.7 in bits, whose
+// atomics wait behind the chase's traffic).
+constexpr uint32_t TREE_BYTES_MAX = 1u << 26, TREE_BYTES_MAX_BATCH = 1u << 27;
 constexpr int TREE_REC_ITEMS = 4;  // (8: 95 registers; 2^26 vertices 3.89 -> 3.83 ms, 4.2e6 228 -> 221 us)
 constexpr int TREE_OUT_ITEMS = 4;  // (2: 1.07 ms, 4 and 8: 0.95 for 2^26 vertices)
 // Mean elements per ruler.  Large levels are bound by what they read at
@@ -95,15 +100,17 @@ __device__ __forceinline__ uint64_t parent_of(const P* parent, uint64_t v, uint3
   return v < n ? __ldcs(parent + v) : v;
 }
 
-// A byte set for every vertex with a child (zeroed by the caller).  A parent
+// A flag set for every vertex with a child (zeroed by the caller).  A parent
 // out of range is reported; its vertex counts as a root everywhere.
-// Bytes and not bits, although bound by the L2 either way: 2^26 caterpillars
-// 0.56 ms against 0.40 with an atomic OR per vertex, but a hundred hubs with all
-// the leaves 0.3 ms against 15 (atomics on a few words come one at a time), and
-// asking for the word before the atomic costs 0.63.
-template <class P>
+// Bytes, stored plainly, while they stay in L2; above 2^26 vertices bits, asked
+// for before the atomic (an atomic for every vertex comes one at a time where
+// a few hubs have all the leaves: 15 ms instead of 1 at 2^26).  Flags and
+// numbering of random recursive trees, bytes / bits: 2^25 vertices 0.45 / 0.45
+// ms, 2^26 0.87 / 0.92, 2^27 3.61 / 2.01, 2^28 10.7 / 4.3; ten thousand hubs at
+// 2^26 6.0 / 4.5.
+template <class P, class I>
 __global__ void __launch_bounds__(TREE_THREADS) k_tree_inner(const P* __restrict__ parent, uint32_t n,
-                                                             unsigned char* __restrict__ inner, DevStatus* st) {
+                                                             I* __restrict__ inner, DevStatus* st) {
   kernel_begin();
   const uint64_t tile_sz = (uint64_t)blockDim.x * TREE_PREP_ITEMS;
   for (uint64_t tile = (uint64_t)blockIdx.x * tile_sz; tile < n; tile += (uint64_t)gridDim.x * tile_sz) {
@@ -117,11 +124,18 @@ __global__ void __launch_bounds__(TREE_THREADS) k_tree_inner(const P* __restrict
         if (v < n) set_error(st, KASCADE_ERR_OUT_OF_RANGE, v);
         p[i] = v;
       }
-      if (p[i] != v) __stcg(inner + p[i], (unsigned char)1);
+      if (p[i] == v) continue;
+      if constexpr (sizeof(I) == 1) {
+        __stcg(inner + p[i], (unsigned char)1);
+      } else {
+        const uint32_t b = (uint32_t)p[i], bit = 1u << (b & 31);
+        if (!(__ldcg(inner + (b >> 5)) & bit)) atomicOr(inner + (b >> 5), bit);
+      }
     }
   }
 }
 
+__device__ __forceinline__ uint32_t inner_word(const uint32_t* inner, uint32_t w) { return __ldcg(inner + w); }
 // The bits of 32 vertices' bytes (each 0 or 1).
 __device__ __forceinline__ uint32_t inner_word(const unsigned char* inner, uint32_t w) {
   const uint4 a = __ldcg(reinterpret_cast<const uint4*>(inner) + 2ull * w);
@@ -143,7 +157,8 @@ __device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t* sm) {  // al
 }
 
 // Vertices with children per tile of words.
-__global__ void __launch_bounds__(TREE_THREADS) k_tree_count(const unsigned char* __restrict__ inner, uint32_t words,
+template <class I>
+__global__ void __launch_bounds__(TREE_THREADS) k_tree_count(const I* __restrict__ inner, uint32_t words,
                                                              uint32_t* __restrict__ sums) {
   kernel_begin();
   __shared__ uint32_t sm[TREE_THREADS / 32];
@@ -160,7 +175,8 @@ __global__ void __launch_bounds__(TREE_THREADS) k_tree_count(const unsigned char
 
 // iw[w] = (bits, bits set before word w), and their number.  A block adds up
 // the tiles before its own.
-__global__ void __launch_bounds__(TREE_THREADS) k_tree_number(const unsigned char* __restrict__ inner, uint32_t words,
+template <class I>
+__global__ void __launch_bounds__(TREE_THREADS) k_tree_number(const I* __restrict__ inner, uint32_t words,
                                                               const uint32_t* __restrict__ sums,
                                                               uint2* __restrict__ iw, uint32_t* __restrict__ count) {
   kernel_begin();
@@ -462,7 +478,9 @@ kascade_status root_levels(kascade_ctx& ctx, const P* parent, uint32_t n, const 
                            const Sink& sink, bool report, bool last, cudaStream_t s) {
   const uint32_t words = (uint32_t)(((uint64_t)n + 31) / 32);
   const uint32_t tiles = (words + WORDS_TILE - 1) / WORDS_TILE;
-  unsigned char* inner = alloc<unsigned char>(ctx, 32ull * words);
+  const bool bits = n > (sizeof(P) == 4 ? TREE_BYTES_MAX_BATCH : TREE_BYTES_MAX);
+  const uint64_t inner_bytes = (bits ? 4ull : 32ull) * words;
+  char* inner = alloc<char>(ctx, inner_bytes);
   uint32_t* sums = alloc<uint32_t>(ctx, tiles);
   uint2* iw = alloc<uint2>(ctx, words);
   uint32_t* rec = alloc<uint32_t>(ctx, n);
@@ -471,13 +489,15 @@ kascade_status root_levels(kascade_ctx& ctx, const P* parent, uint32_t n, const 
   if (!inner || !sums || !iw || !rec || !vert || !out) return KASCADE_ERR_OOM;
   {
     ProfScope ps(ctx, "prepare", s);
-    KS_CUDA(cudaMemsetAsync(inner, 0, 32ull * words, s));
+    KS_CUDA(cudaMemsetAsync(inner, 0, inner_bytes, s));
     const unsigned grid = grid_for(ctx, ((uint64_t)n + TREE_PREP_ITEMS - 1) / TREE_PREP_ITEMS, TREE_THREADS, 8);
-    KS_TRY(launch(ctx, k_tree_inner<P>, grid, TREE_THREADS, 0, s, parent, n, inner, ctx.d_status));
-    if (tiles > 1) {
-      KS_TRY(launch(ctx, k_tree_count, tiles, TREE_THREADS, 0, s, inner, words, sums));
-    }
-    KS_TRY(launch(ctx, k_tree_number, tiles, TREE_THREADS, 0, s, inner, words, sums, iw, count));
+    auto number = [&](auto* flags) {
+      using I = std::remove_reference_t<decltype(*flags)>;
+      KS_TRY(launch(ctx, k_tree_inner<P, I>, grid, TREE_THREADS, 0, s, parent, n, flags, ctx.d_status));
+      if (tiles > 1) KS_TRY(launch(ctx, k_tree_count<I>, tiles, TREE_THREADS, 0, s, flags, words, sums));
+      return launch(ctx, k_tree_number<I>, tiles, TREE_THREADS, 0, s, flags, words, sums, iw, count);
+    };
+    KS_TRY(bits ? number(reinterpret_cast<uint32_t*>(inner)) : number(reinterpret_cast<unsigned char*>(inner)));
     const unsigned rec_grid = grid_for(ctx, ((uint64_t)n + TREE_REC_ITEMS - 1) / TREE_REC_ITEMS, TREE_THREADS, 8);
     KS_TRY(launch(ctx, k_tree_records<P>, rec_grid, TREE_THREADS, 0, s, parent, n, iw, lv.rulers[0], rec, vert, report,
                   ctx.d_status));

@@ -7,6 +7,8 @@ from __future__ import annotations
 import numpy as np
 import pytest
 
+import torch
+
 from gpu_util import dev64, host_i64
 
 pytestmark = pytest.mark.gpu
@@ -86,3 +88,30 @@ def test_cycles_are_reported(kb, n):
             with pytest.raises(kb.KascadeError) as e:
                 run(dev64(succ.astype(np.uint64)))
             assert e.value.name == "CYCLE"
+
+
+@pytest.mark.parametrize("n", [1 << 26, (1 << 26) + 1, (1 << 26) + 70_001])
+@pytest.mark.parametrize("hubs", [0, 50_000])
+def test_both_kinds_of_child_flags(kb, n, hubs):
+    """Child flags in bytes and in bits: depth and root follow the parent's."""
+    if hubs:
+        g = torch.Generator(device="cuda")
+        g.manual_seed(n)
+        par = torch.randint(0, hubs, (n,), device="cuda", generator=g)
+        par[:hubs] = (torch.arange(hubs, device="cuda") - 1).clamp(min=0)  # the hubs: one path
+    else:
+        par = kb.gen_forest(n, n, 0, 3, 0)
+    root, depth = kb.root_forest(par)
+    idx = torch.arange(n, device="cuda")
+    top = par == idx
+    assert bool((depth == torch.where(top, 0, depth[par] + 1)).all())
+    assert bool((root == torch.where(top, idx, root[par])).all())
+
+
+def test_bits_in_a_batch(kb):
+    n = (1 << 27) + 5
+    par = kb.gen_forest(n, 9, 0, 2, 0)
+    segs = kb.make_segments(np.array([n], np.int64), np.array([kb.SEG_FOREST], np.int64))
+    root, depth = kb.rank_batch(par, segs)
+    root_f, depth_f = kb.root_forest(par)
+    assert torch.equal(root, root_f) and torch.equal(depth, depth_f)
