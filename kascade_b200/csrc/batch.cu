@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(BP_THREADS) k_batch_hints(HintJobs jobs) {
       uint32_t lo = 0, hi = j.n;  // the last segment with base <= x
       while (hi - lo > 1) {
         const uint32_t mid = (lo + hi) >> 1;
-        if (j.base[mid] <= x)
+        if (ld_ca(j.base + mid) <= x)
           lo = mid;
         else
           hi = mid;
@@ -67,7 +67,7 @@ struct BWUnit {
 };
 struct BWU32 {
   const uint32_t* p;
-  __device__ __forceinline__ uint32_t operator()(uint64_t g) const { return __ldcs(p + g); }
+  __device__ __forceinline__ uint32_t operator()(uint64_t g) const { return ld_cs(p + g); }
 };
 
 // List elements' records, and forest vertices' parents, from the caller's
@@ -88,17 +88,17 @@ __global__ void __launch_bounds__(BP_THREADS) k_batch_prepare(BatchIn b, uint32_
 #pragma unroll
     for (int i = 0; i < BP_PER; ++i) {
       const uint64_t g = g0 + i * BP_THREADS + threadIdx.x;
-      v[i] = g < total ? __ldcs(b.in + g) : 0;
+      v[i] = g < total ? ld_cs(b.in + g) : 0;
       wv[i] = g < total ? w(g) : 0u;
     }
     // (a step lies within one tile of the hints)
-    const uint32_t j0 = __ldg(b.pos.hint + (uint32_t)(g0 / TILE)), j1 = __ldg(b.pos.hint + (uint32_t)(g0 / TILE) + 1);
+    const uint32_t j0 = ld_ca(b.pos.hint + (uint32_t)(g0 / TILE)), j1 = ld_ca(b.pos.hint + (uint32_t)(g0 / TILE) + 1);
     uint32_t j = j0, off = 0, size = 0;
     uint2 kind = make_uint2(0, 0);
     auto segment = [&]() {
-      off = __ldg(b.pos.base + j);
-      size = __ldg(b.pos.base + j + 1) - off;
-      kind = __ldg(b.kinds + j);
+      off = ld_ca(b.pos.base + j);
+      size = ld_ca(b.pos.base + j + 1) - off;
+      kind = ld_ca(b.kinds + j);
     };
     if (j0 == j1) segment();
 #pragma unroll

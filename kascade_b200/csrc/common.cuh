@@ -79,6 +79,72 @@ __device__ __forceinline__ void kernel_begin() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// ---------------------------------------------------------------------------
+// Counter hash used for ruler sampling (the "lowbias32" integer mixer,
+// a public-domain construction by C. Wellons).
+// ---------------------------------------------------------------------------
+__host__ __device__ __forceinline__ uint32_t mix32(uint32_t x) {
+  x ^= x >> 16;
+  x *= 0x7feb352du;
+  x ^= x >> 15;
+  x *= 0x846ca68bu;
+  x ^= x >> 16;
+  return x;
+}
+
+__device__ __forceinline__ bool sampled(uint32_t x, uint32_t salt, uint32_t thresh) {
+  return mix32(x ^ salt) < thresh;
+}
+
+// ---------------------------------------------------------------------------
+// Loads of what the kernel ahead may still be storing.  A kernel that `launch`
+// starts is in place while that one runs.  Its loads may not be of the
+// non-coherent kind (__ldg, or what the compiler makes of a const __restrict__
+// pointer): that takes the data as unchanging for as long as the kernel is
+// resident.  Nor may they move above kernel_begin's wait: ld_cg and ld_cs are
+// volatile, as the wait is, and ld_ca is a plain read, which the wait's memory
+// clobber holds back (as a volatile load it cost the forests' walks 1 to 4%:
+// 4.2e6 vertices 232 us, plain 222).
+//   ld_ca  through L1 (what neighbours or later loads read again)
+//   ld_cg  from L2 (random hops, which never hit L1; what other SMs write)
+//   ld_cs  streaming, evict-first
+// ---------------------------------------------------------------------------
+template <class T>
+__device__ __forceinline__ T ld_ca(const T* p) {
+  return *p;
+}
+#define KS_LOADS(name, op)                                                                                  \
+  __device__ __forceinline__ uint32_t name(const uint32_t* p) {                                             \
+    uint32_t v;                                                                                             \
+    asm volatile("ld.global." op ".u32 %0, [%1];" : "=r"(v) : "l"(p));                                      \
+    return v;                                                                                               \
+  }                                                                                                         \
+  __device__ __forceinline__ uint64_t name(const uint64_t* p) {                                             \
+    uint64_t v;                                                                                             \
+    asm volatile("ld.global." op ".u64 %0, [%1];" : "=l"(v) : "l"(p));                                      \
+    return v;                                                                                               \
+  }                                                                                                         \
+  __device__ __forceinline__ unsigned long long name(const unsigned long long* p) {                         \
+    unsigned long long v;                                                                                   \
+    asm volatile("ld.global." op ".u64 %0, [%1];" : "=l"(v) : "l"(p));                                      \
+    return v;                                                                                               \
+  }                                                                                                         \
+  __device__ __forceinline__ uint2 name(const uint2* p) {                                                   \
+    uint2 v;                                                                                                \
+    asm volatile("ld.global." op ".v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));                \
+    return v;                                                                                               \
+  }                                                                                                         \
+  __device__ __forceinline__ uint4 name(const uint4* p) {                                                   \
+    uint4 v;                                                                                                \
+    asm volatile("ld.global." op ".v4.u32 {%0, %1, %2, %3}, [%4];"                                          \
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)                                               \
+                 : "l"(p));                                                                                 \
+    return v;                                                                                               \
+  }
+KS_LOADS(ld_cg, "cg")
+KS_LOADS(ld_cs, "cs")
+#undef KS_LOADS
+
 // The words of a status that the host reads.
 constexpr uint32_t STATUS_WORDS = 8;
 static_assert(offsetof(DevStatus, work) == STATUS_WORDS * 8 && sizeof(DevStatus) % 8 == 0, "status words");
@@ -100,33 +166,12 @@ __device__ __forceinline__ void publish_status(DevStatus* st, unsigned long long
   }
   if (!__shfl_sync(0xffffffffu, last, 0)) return;
   unsigned long long* w = reinterpret_cast<unsigned long long*>(st);
-  if (threadIdx.x < STATUS_WORDS) *(volatile unsigned long long*)(host + threadIdx.x) = __ldcg(w + threadIdx.x);
+  if (threadIdx.x < STATUS_WORDS) *(volatile unsigned long long*)(host + threadIdx.x) = ld_cg(w + threadIdx.x);
   if (threadIdx.x < sizeof(DevStatus) / 8) __stcg(w + threadIdx.x, 0ull);
 }
 
-// ---------------------------------------------------------------------------
-// Counter hash used for ruler sampling (the "lowbias32" integer mixer,
-// a public-domain construction by C. Wellons).
-// ---------------------------------------------------------------------------
-__host__ __device__ __forceinline__ uint32_t mix32(uint32_t x) {
-  x ^= x >> 16;
-  x *= 0x7feb352du;
-  x ^= x >> 15;
-  x *= 0x846ca68bu;
-  x ^= x >> 16;
-  return x;
-}
-
-__device__ __forceinline__ bool sampled(uint32_t x, uint32_t salt, uint32_t thresh) {
-  return mix32(x ^ salt) < thresh;
-}
-
-// ---------------------------------------------------------------------------
-// Cache-hinted 16 B accesses.  .cg bypasses L1 (random hops never hit it and
-// the chase rewrites what it reads); .cs marks streaming data evict-first.
-// ---------------------------------------------------------------------------
 __device__ __forceinline__ Rec ld_rec_cg(const Rec* p) {
-  uint4 v = __ldcg(reinterpret_cast<const uint4*>(p));
+  uint4 v = ld_cg(reinterpret_cast<const uint4*>(p));
   Rec r;
   r.a = (uint64_t)v.x | ((uint64_t)v.y << 32);
   r.b = v.z;
@@ -134,7 +179,7 @@ __device__ __forceinline__ Rec ld_rec_cg(const Rec* p) {
   return r;
 }
 __device__ __forceinline__ Rec ld_rec_cs(const Rec* p) {
-  uint4 v = __ldcs(reinterpret_cast<const uint4*>(p));
+  uint4 v = ld_cs(reinterpret_cast<const uint4*>(p));
   Rec r;
   r.a = (uint64_t)v.x | ((uint64_t)v.y << 32);
   r.b = v.z;
@@ -188,11 +233,11 @@ struct Stamp8 {
   }
   static __device__ __forceinline__ void clear(S* p) { __stcg(p, make_uint2(TAG_UNREACHED, 0u)); }
   static __device__ __forceinline__ Stamp get_stream(const S* p) {
-    const uint2 v = __ldcs(p);
+    const uint2 v = ld_cs(p);
     return Stamp{v.x, v.y};
   }
   static __device__ __forceinline__ Stamp get(const S* p) {
-    const uint2 v = __ldcg(p);
+    const uint2 v = ld_cg(p);
     return Stamp{v.x, v.y};
   }
 };
@@ -203,11 +248,11 @@ struct Stamp16 {
   }
   static __device__ __forceinline__ void clear(S* p) { __stcg(p, make_uint4(0u, 0u, TAG_UNREACHED, 0u)); }
   static __device__ __forceinline__ Stamp get_stream(const S* p) {
-    const uint4 v = __ldcs(p);
+    const uint4 v = ld_cs(p);
     return Stamp{v.z, (uint64_t)v.x | ((uint64_t)v.y << 32)};
   }
   static __device__ __forceinline__ Stamp get(const S* p) {
-    const uint4 v = __ldcg(p);
+    const uint4 v = ld_cg(p);
     return Stamp{v.z, (uint64_t)v.x | ((uint64_t)v.y << 32)};
   }
 };
@@ -217,7 +262,7 @@ struct Record8 {
   static __device__ __forceinline__ Hop unpack(uint2 v) {
     return Hop{v.y, v.x & ~REC8_RULER, (v.x & REC8_RULER) != 0u};
   }
-  static __device__ __forceinline__ Hop hop(const R* p) { return unpack(__ldcg(reinterpret_cast<const uint2*>(p))); }
+  static __device__ __forceinline__ Hop hop(const R* p) { return unpack(ld_cg(reinterpret_cast<const uint2*>(p))); }
   static __device__ __forceinline__ void put(R* p, uint64_t w, uint32_t b, bool ruler) {
     __stcg(reinterpret_cast<uint2*>(p), make_uint2(b | (ruler ? REC8_RULER : 0u), (uint32_t)w));
   }
@@ -281,7 +326,7 @@ struct F16i {
 enum class Format { F8x8, F8x16, F16x16, F16i };
 
 __device__ __forceinline__ Out ld_out(const Out* p) {
-  uint4 v = __ldcg(reinterpret_cast<const uint4*>(p));
+  uint4 v = ld_cg(reinterpret_cast<const uint4*>(p));
   Out o;
   o.rank = (uint64_t)v.x | ((uint64_t)v.y << 32);
   o.root = v.z;
@@ -297,6 +342,7 @@ __device__ __forceinline__ uint64_t l2_keep_policy() {
 }
 // Through the read-only (L1) path with the same L2 hint: for lookups whose
 // neighbours in a warp's stream tend to repeat (log entries of one chain).
+// Non-coherent: for kernels that start after the kernel ahead has ended.
 __device__ __forceinline__ Out ld_out_nc_keep(const Out* p, uint64_t pol) {
   uint32_t a, b, c, d;
   asm volatile("ld.global.nc.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"

@@ -129,8 +129,9 @@ struct ProfScope {
 // Launch of a kernel that begins with kernel_begin: its blocks are put in place
 // before the kernel ahead has ended, ~1 us less per launch of a call that is a
 // chain of small ones (50K forest 96 -> 84 us, pointer doubling of 1M 190 ->
-// 174, a list of 100K 88 -> 82, 32 instances of 3e4 94 -> 80).  Not while a
-// context has a budget of SMs: waiting blocks take slots.
+// 174, a list of 100K 88 -> 82, 32 instances of 3e4 94 -> 80).  Such a kernel
+// reads global memory by ld_ca, ld_cg and ld_cs.  Not while a context has a
+// budget of SMs: waiting blocks take slots.
 template <class... P, class... A>
 kascade_status launch(const kascade_ctx& ctx, void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
                       cudaStream_t s, A&&... args) {

@@ -31,12 +31,12 @@ __global__ void __launch_bounds__(256) k_gen_forest(uint64_t n, ks_perm perm, ui
 }
 
 // list_ranking.cpp:60-80
-__global__ void __launch_bounds__(256) k_initial_state(const uint64_t* __restrict__ succ, uint64_t n,
+__global__ void __launch_bounds__(256) k_initial_state(const uint64_t* succ, uint64_t n,
                                                        uint64_t* __restrict__ root, int64_t* __restrict__ rank,
                                                        DevStatus* st, unsigned long long* status) {
   kernel_begin();
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t s = succ[i];
+    const uint64_t s = ld_cs(succ + i);
     root[i] = s;
     rank[i] = (s == i) ? 0 : 1;
   }

@@ -40,13 +40,13 @@ struct WUnit {
 struct WU32 {
   using T = uint32_t;
   const uint32_t* p;
-  __device__ __forceinline__ T operator()(uint64_t x) const { return __ldcs(p + x); }
+  __device__ __forceinline__ T operator()(uint64_t x) const { return ld_cs(p + x); }
 };
 struct WI64 {
   using T = uint64_t;
   const int64_t* p;
   __device__ __forceinline__ T operator()(uint64_t x) const {
-    return (uint64_t)__ldcs(reinterpret_cast<const long long*>(p) + x);
+    return ld_cs(reinterpret_cast<const uint64_t*>(p) + x);
   }
 };
 
@@ -56,7 +56,7 @@ struct WI64 {
 // 0, so that a chain ending at it adds the record's word like any.
 // ---------------------------------------------------------------------------
 template <class F, class W>
-__global__ void __launch_bounds__(256, 4) k_prepare_arrays(const uint64_t* __restrict__ succ, W w, uint32_t n,
+__global__ void __launch_bounds__(256, 4) k_prepare_arrays(const uint64_t* succ, W w, uint32_t n,
                                                         uint64_t start, Rulers rl, typename F::R* __restrict__ rec,
                                                         typename F::S* __restrict__ stamp, DevStatus* st) {
   kernel_begin();
@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(256, 4) k_prepare_arrays(const uint64_t* __res
       sv[i] = 0;
       wv[i] = 0;
       if (x < n) {
-        sv[i] = __ldcs(reinterpret_cast<const unsigned long long*>(succ) + x);
+        sv[i] = ld_cs(reinterpret_cast<const unsigned long long*>(succ) + x);
         wv[i] = w(x);
       }
     }
@@ -99,7 +99,7 @@ constexpr int PT_STAGES = 4;
 constexpr int PT_ITEMS = PT_TILE / 256;
 
 template <class F, bool W32>
-__global__ void __launch_bounds__(256) k_prepare_tma(const uint64_t* __restrict__ succ, const uint32_t* __restrict__ w,
+__global__ void __launch_bounds__(256) k_prepare_tma(const uint64_t* succ, const uint32_t* w,
                                                      uint32_t n, uint32_t ntiles, Rulers rl,
                                                      typename F::R* __restrict__ rec,
                                                      typename F::S* __restrict__ stamp, DevStatus* st) {
@@ -193,7 +193,7 @@ constexpr int CHASE_REFILL = 8;  // idle lanes worth a refill
 
 template <class F>
 __global__ void __launch_bounds__(512) k_chase(const typename F::R* rec, typename F::S* stamp, uint32_t n, Rulers rl,
-                                               uint32_t r, const uint32_t* __restrict__ rootel, NextLevel nx,
+                                               uint32_t r, const uint32_t* rootel, NextLevel nx,
                                                uint32_t* __restrict__ work, uint32_t lanes, uint32_t hop_cap,
                                                DevStatus* st) {
   kernel_begin();
@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(512) k_chase(const typename F::R* rec, typenam
     if (stop) {  // (a list's end is not stamped: any number of chains may end there)
       uint32_t next = id;
       if (end) {
-        nx.rootel[id] = rootel ? __ldg(rootel + x) : x;
+        nx.rootel[id] = rootel ? ld_ca(rootel + x) : x;
       } else {
         next = rl.block_of(y);
         // back at its own ruler: a cycle without a root that holds one ruler
@@ -289,9 +289,8 @@ __global__ void __launch_bounds__(512) k_chase(const typename F::R* rec, typenam
 constexpr uint32_t PROP_WALKS = 512;  // elements a block collects
 
 template <class F, class Sink>
-__device__ __forceinline__ void walk_to_result(const typename F::R* __restrict__ rec,
-                                               const typename F::S* __restrict__ stamp, uint32_t x, const Rulers& rl,
-                                               const uint32_t* __restrict__ rootel, const Out* __restrict__ out_next,
+__device__ __forceinline__ void walk_to_result(const typename F::R* rec, const typename F::S* stamp, uint32_t x,
+                                               const Rulers& rl, const uint32_t* rootel, const Out* out_next,
                                                const Sink& sink, DevStatus* st) {
   Hop h = F::hop(rec + x);
   uint64_t acc = h.w;
@@ -311,7 +310,7 @@ __device__ __forceinline__ void walk_to_result(const typename F::R* __restrict__
     }
     acc += h.w;
     if (h.b == y) {
-      sink.put(x, acc, rootel ? __ldg(rootel + y) : y, false);
+      sink.put(x, acc, rootel ? ld_ca(rootel + y) : y, false);
       return;
     }
     // an invalid (rootless, ruler-free) cycle comes back to a marked element
@@ -327,11 +326,9 @@ __device__ __forceinline__ void walk_to_result(const typename F::R* __restrict__
 }
 
 template <class F, class Sink, int ITEMS>
-__global__ void __launch_bounds__(256) k_propagate(const typename F::R* __restrict__ rec,
-                                                   const typename F::S* __restrict__ stamp, uint32_t n, Rulers rl,
-                                                   const uint32_t* __restrict__ rootel,
-                                                   const Out* __restrict__ out_next, Sink sink, DevStatus* st,
-                                                   unsigned long long* status) {
+__global__ void __launch_bounds__(256) k_propagate(const typename F::R* rec, const typename F::S* stamp,
+                                                   uint32_t n, Rulers rl, const uint32_t* rootel, const Out* out_next,
+                                                   Sink sink, DevStatus* st, unsigned long long* status) {
   kernel_begin();
   __shared__ uint32_t walks[PROP_WALKS];
   __shared__ uint32_t nwalks, nfound;
@@ -379,7 +376,7 @@ __global__ void __launch_bounds__(256) k_propagate(const typename F::R* __restri
       }
       const Hop h = F::hop(rec + x);
       if (h.b == (uint32_t)x) {
-        sink.put((uint32_t)x, h.w, rootel ? __ldg(rootel + x) : (uint32_t)x, true);
+        sink.put((uint32_t)x, h.w, rootel ? ld_ca(rootel + x) : (uint32_t)x, true);
       } else {
         const uint32_t w = atomicAdd(&nwalks, 1u);
         if (w < PROP_WALKS)
@@ -443,7 +440,7 @@ struct CtaRecords {
     *b = h.b;
     *ruler = h.ruler;
   }
-  __device__ __forceinline__ uint32_t root_of(uint32_t x) const { return rootel ? __ldg(rootel + x) : x; }
+  __device__ __forceinline__ uint32_t root_of(uint32_t x) const { return rootel ? ld_ca(rootel + x) : x; }
 };
 template <class W, class I = uint64_t>
 struct CtaArrays {
@@ -452,7 +449,7 @@ struct CtaArrays {
   W w;
   __device__ __forceinline__ void load(uint32_t x, uint64_t* a, uint32_t* b, bool* ruler) const {
     *ruler = false;
-    const uint64_t s = __ldcg(succ + x);
+    const uint64_t s = ld_cg(succ + x);
     *a = w(x);
     *b = s > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)s;  // beyond any element: found out of range
   }

@@ -94,7 +94,7 @@ struct Extent {
   uint32_t div = 1;
   __device__ __forceinline__ uint32_t get() const {
     if (!count) return cap;
-    uint32_t v = __ldg(count);
+    uint32_t v = ld_ca(count);
     if (div != 1) v = v / div + (v % div != 0u ? 1u : 0u);
     return min(cap, v);
   }
@@ -114,10 +114,10 @@ struct SegMap {
   const uint32_t* hint = nullptr;   // [k]: the segment of element 4096 k, and one more for the end
   uint32_t n = 0;                   // 0: one instance, in place
   __device__ __forceinline__ uint32_t find(uint32_t x) const {  // the last j with base[j] <= x
-    uint32_t lo = __ldg(hint + (x >> 12)), hi = min(__ldg(hint + (x >> 12) + 1) + 1, n);
+    uint32_t lo = ld_ca(hint + (x >> 12)), hi = min(ld_ca(hint + (x >> 12) + 1) + 1, n);
     while (hi - lo > 1) {
       const uint32_t mid = (lo + hi) >> 1;
-      if (__ldg(base + mid) <= x)
+      if (ld_ca(base + mid) <= x)
         lo = mid;
       else
         hi = mid;
@@ -162,7 +162,7 @@ struct SinkBatch {
   LogTarget log_target() const { return LogTarget{root, rank, 0, seg}; }
   __device__ __forceinline__ void put(uint32_t x, uint64_t rk, uint32_t rt, bool is_root) const {
     const uint32_t j = seg.find(x);
-    const uint32_t b = __ldg(seg.base + j), g = x + __ldg(seg.delta + j);
+    const uint32_t b = ld_ca(seg.base + j), g = x + ld_ca(seg.delta + j);
     __stcs(root + g, (unsigned long long)((is_root ? x : rt) - b));
     __stcs(rank + g, is_root ? 0ull : (unsigned long long)rk);
   }

@@ -51,7 +51,7 @@ struct TreeUnit {
   using R = uint32_t;
   static constexpr bool kEndWeight = false;
   static __device__ __forceinline__ Hop hop(const R* p) {
-    const uint32_t v = __ldg(p);
+    const uint32_t v = ld_ca(p);
     return Hop{1, v & ~REC8_RULER, (v & REC8_RULER) != 0u};
   }
 };
@@ -61,10 +61,10 @@ struct Tree8 {
   using O = uint2;  // rank, root
   static constexpr bool kEndWeight = true;
   static __device__ __forceinline__ Hop hop(const R* p) {
-    return Record8::unpack(__ldg(reinterpret_cast<const uint2*>(p)));
+    return Record8::unpack(ld_ca(reinterpret_cast<const uint2*>(p)));
   }
   static __device__ __forceinline__ Out out(const O* p) {
-    const uint2 v = __ldg(p);
+    const uint2 v = ld_ca(p);
     return Out{v.x, v.y, 0};
   }
   static __device__ __forceinline__ void put(R* p, uint64_t w, uint32_t b, bool ruler) { Record8::put(p, w, b, ruler); }
@@ -75,7 +75,7 @@ struct Tree16 {
   using O = Out;
   static constexpr bool kEndWeight = true;  // (level 0: prepared as 0)
   static __device__ __forceinline__ Hop hop(const R* p) {
-    const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
+    const uint4 v = ld_ca(reinterpret_cast<const uint4*>(p));
     return Hop{(uint64_t)v.x | ((uint64_t)v.y << 32), v.z, v.w != 0u};
   }
   static __device__ __forceinline__ Out out(const O* p) { return ld_out(p); }
@@ -97,7 +97,7 @@ constexpr uint32_t WORDS_TILE = TREE_THREADS * WORDS_PER;
 // Parents are the caller's 64-bit indices, or a batch's in one vertex space.
 template <class P>
 __device__ __forceinline__ uint64_t parent_of(const P* parent, uint64_t v, uint32_t n) {
-  return v < n ? __ldcs(parent + v) : v;
+  return v < n ? ld_cs(parent + v) : v;
 }
 
 // A flag set for every vertex with a child (zeroed by the caller).  A parent
@@ -109,7 +109,7 @@ __device__ __forceinline__ uint64_t parent_of(const P* parent, uint64_t v, uint3
 // ms, 2^26 0.87 / 0.92, 2^27 3.61 / 2.01, 2^28 10.7 / 4.3; ten thousand hubs at
 // 2^26 6.0 / 4.5.
 template <class P, class I>
-__global__ void __launch_bounds__(TREE_THREADS) k_tree_inner(const P* __restrict__ parent, uint32_t n,
+__global__ void __launch_bounds__(TREE_THREADS) k_tree_inner(const P* parent, uint32_t n,
                                                              I* __restrict__ inner, DevStatus* st) {
   kernel_begin();
   const uint64_t tile_sz = (uint64_t)blockDim.x * TREE_PREP_ITEMS;
@@ -129,17 +129,17 @@ __global__ void __launch_bounds__(TREE_THREADS) k_tree_inner(const P* __restrict
         __stcg(inner + p[i], (unsigned char)1);
       } else {
         const uint32_t b = (uint32_t)p[i], bit = 1u << (b & 31);
-        if (!(__ldcg(inner + (b >> 5)) & bit)) atomicOr(inner + (b >> 5), bit);
+        if (!(ld_cg(inner + (b >> 5)) & bit)) atomicOr(inner + (b >> 5), bit);
       }
     }
   }
 }
 
-__device__ __forceinline__ uint32_t inner_word(const uint32_t* inner, uint32_t w) { return __ldcg(inner + w); }
+__device__ __forceinline__ uint32_t inner_word(const uint32_t* inner, uint32_t w) { return ld_cg(inner + w); }
 // The bits of 32 vertices' bytes (each 0 or 1).
 __device__ __forceinline__ uint32_t inner_word(const unsigned char* inner, uint32_t w) {
-  const uint4 a = __ldcg(reinterpret_cast<const uint4*>(inner) + 2ull * w);
-  const uint4 b = __ldcg(reinterpret_cast<const uint4*>(inner) + 2ull * w + 1);
+  const uint4 a = ld_cg(reinterpret_cast<const uint4*>(inner) + 2ull * w);
+  const uint4 b = ld_cg(reinterpret_cast<const uint4*>(inner) + 2ull * w + 1);
   auto four = [](uint32_t v) { return (v * 0x01020408u) >> 24; };  // byte i's bit to bit i
   return four(a.x) | four(a.y) << 4 | four(a.z) << 8 | four(a.w) << 12 | four(b.x) << 16 | four(b.y) << 20 |
          four(b.z) << 24 | four(b.w) << 28;
@@ -158,7 +158,7 @@ __device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t* sm) {  // al
 
 // Vertices with children per tile of words.
 template <class I>
-__global__ void __launch_bounds__(TREE_THREADS) k_tree_count(const I* __restrict__ inner, uint32_t words,
+__global__ void __launch_bounds__(TREE_THREADS) k_tree_count(const I* inner, uint32_t words,
                                                              uint32_t* __restrict__ sums) {
   kernel_begin();
   __shared__ uint32_t sm[TREE_THREADS / 32];
@@ -176,14 +176,14 @@ __global__ void __launch_bounds__(TREE_THREADS) k_tree_count(const I* __restrict
 // iw[w] = (bits, bits set before word w), and their number.  A block adds up
 // the tiles before its own.
 template <class I>
-__global__ void __launch_bounds__(TREE_THREADS) k_tree_number(const I* __restrict__ inner, uint32_t words,
-                                                              const uint32_t* __restrict__ sums,
+__global__ void __launch_bounds__(TREE_THREADS) k_tree_number(const I* inner, uint32_t words,
+                                                              const uint32_t* sums,
                                                               uint2* __restrict__ iw, uint32_t* __restrict__ count) {
   kernel_begin();
   __shared__ uint32_t sm[TREE_THREADS / 32];
   __shared__ uint32_t tile[WORDS_TILE];
   uint32_t before = 0;
-  for (uint32_t b = threadIdx.x; b < blockIdx.x; b += TREE_THREADS) before += sums[b];
+  for (uint32_t b = threadIdx.x; b < blockIdx.x; b += TREE_THREADS) before += ld_ca(sums + b);
   before = block_sum(before, sm);
   const uint32_t base = blockIdx.x * WORDS_TILE;
 #pragma unroll
@@ -226,8 +226,8 @@ __device__ __forceinline__ uint32_t number_of(uint2 w, uint32_t v) {
 // one (the vertices, and once more those with children that are not roots), the
 // size a call reports for level 0, go to the status.
 template <class P>
-__global__ void __launch_bounds__(TREE_THREADS) k_tree_records(const P* __restrict__ parent, uint32_t n,
-                                                               const uint2* __restrict__ iw, Rulers rl,
+__global__ void __launch_bounds__(TREE_THREADS) k_tree_records(const P* parent, uint32_t n,
+                                                               const uint2* iw, Rulers rl,
                                                                uint32_t* __restrict__ rec,
                                                                uint32_t* __restrict__ vert, bool report,
                                                                DevStatus* st) {
@@ -241,14 +241,14 @@ __global__ void __launch_bounds__(TREE_THREADS) k_tree_records(const P* __restri
     for (int i = 0; i < TREE_REC_ITEMS; ++i) {
       const uint64_t v = tile + (uint64_t)i * blockDim.x + threadIdx.x;
       p[i] = parent_of(parent, v, n);
-      own[i] = v < n ? __ldg(iw + (v >> 5)) : make_uint2(0, 0);
+      own[i] = v < n ? ld_ca(iw + (v >> 5)) : make_uint2(0, 0);
     }
 #pragma unroll
     for (int i = 0; i < TREE_REC_ITEMS; ++i) {
       const uint64_t v = tile + (uint64_t)i * blockDim.x + threadIdx.x;
       if (p[i] >= n) p[i] = v;
       if (!((own[i].x >> (v & 31)) & 1u)) p[i] = ~0ull;  // a leaf
-      up[i] = p[i] < n ? __ldg(iw + (p[i] >> 5)) : make_uint2(0, 0);
+      up[i] = p[i] < n ? ld_ca(iw + (p[i] >> 5)) : make_uint2(0, 0);
     }
 #pragma unroll
     for (int i = 0; i < TREE_REC_ITEMS; ++i) {
@@ -272,8 +272,8 @@ __global__ void __launch_bounds__(TREE_THREADS) k_tree_records(const P* __restri
 // Every vertex's result from the numbered ones' (depth, root).
 template <class P, class Sink>
 __global__ void __launch_bounds__(TREE_THREADS) k_tree_leaves(const P* parent, uint32_t n,
-                                                              const uint2* __restrict__ iw,
-                                                              const uint2* __restrict__ out, Sink sink,
+                                                              const uint2* iw,
+                                                              const uint2* out, Sink sink,
                                                               DevStatus* st, unsigned long long* status) {
   kernel_begin();
   const uint64_t tile_sz = (uint64_t)blockDim.x * TREE_OUT_ITEMS;
@@ -285,20 +285,20 @@ __global__ void __launch_bounds__(TREE_THREADS) k_tree_leaves(const P* parent, u
     for (int i = 0; i < TREE_OUT_ITEMS; ++i) {
       const uint64_t v = tile + (uint64_t)i * blockDim.x + threadIdx.x;
       p[i] = parent_of(parent, v, n);
-      w[i] = v < n ? __ldg(iw + (v >> 5)) : make_uint2(0, 0);
+      w[i] = v < n ? ld_ca(iw + (v >> 5)) : make_uint2(0, 0);
     }
 #pragma unroll
     for (int i = 0; i < TREE_OUT_ITEMS; ++i) {
       const uint64_t v = tile + (uint64_t)i * blockDim.x + threadIdx.x;
       if (p[i] >= n) p[i] = v;
       leaf[i] = !((w[i].x >> (v & 31)) & 1u);
-      if (leaf[i] && p[i] != v) w[i] = __ldg(iw + (p[i] >> 5));
+      if (leaf[i] && p[i] != v) w[i] = ld_ca(iw + (p[i] >> 5));
     }
 #pragma unroll
     for (int i = 0; i < TREE_OUT_ITEMS; ++i) {
       const uint64_t v = tile + (uint64_t)i * blockDim.x + threadIdx.x;
       o[i] = make_uint2(0, 0);
-      if (p[i] != v) o[i] = __ldg(out + number_of(w[i], leaf[i] ? (uint32_t)p[i] : (uint32_t)v));
+      if (p[i] != v) o[i] = ld_ca(out + number_of(w[i], leaf[i] ? (uint32_t)p[i] : (uint32_t)v));
     }
 #pragma unroll
     for (int i = 0; i < TREE_OUT_ITEMS; ++i) {
@@ -315,9 +315,9 @@ __global__ void __launch_bounds__(TREE_THREADS) k_tree_leaves(const P* parent, u
 // Every ruler's walk to the next ruler or its root.  next.s == 0: the last
 // level's rulers are the one-CTA ranker's.
 template <class L, class N>
-__global__ void __launch_bounds__(TREE_THREADS) k_tree_chase(const typename L::R* __restrict__ rec, Extent ext,
+__global__ void __launch_bounds__(TREE_THREADS) k_tree_chase(const typename L::R* rec, Extent ext,
                                                              Rulers rl, Extent next_ext,
-                                                             const uint32_t* __restrict__ rootel,
+                                                             const uint32_t* rootel,
                                                              typename N::R* __restrict__ nrec,
                                                              uint32_t* __restrict__ nroot, Rulers nrl,
                                                              uint32_t hop_cap, DevStatus* st) {
@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(TREE_THREADS) k_tree_chase(const typename L::R
         const Hop h = L::hop(rec + x);
         if (h.b == x) {
           if (L::kEndWeight) acc += h.w;
-          nroot[id] = rootel ? __ldg(rootel + x) : x;
+          nroot[id] = rootel ? ld_ca(rootel + x) : x;
           break;
         }
         acc += h.w;
@@ -360,9 +360,9 @@ __global__ void __launch_bounds__(TREE_THREADS) k_tree_chase(const typename L::R
 
 // Every element's result: its ruler's, or the first ruler's on its path.
 template <class L, class N, class Sink>
-__global__ void __launch_bounds__(TREE_THREADS) k_tree_propagate(const typename L::R* __restrict__ rec, Extent ext,
-                                                                 Rulers rl, const uint32_t* __restrict__ rootel,
-                                                                 const typename N::O* __restrict__ out, Sink sink,
+__global__ void __launch_bounds__(TREE_THREADS) k_tree_propagate(const typename L::R* rec, Extent ext,
+                                                                 Rulers rl, const uint32_t* rootel,
+                                                                 const typename N::O* out, Sink sink,
                                                                  DevStatus* st, unsigned long long* status) {
   kernel_begin();
   const uint32_t n = ext.get();
@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(TREE_THREADS) k_tree_propagate(const typename 
     const uint32_t x = (uint32_t)v;
     Hop h = L::hop(rec + x);
     if (h.b == x) {
-      sink.put(x, L::kEndWeight ? h.w : 0ull, rootel ? __ldg(rootel + x) : x, true);
+      sink.put(x, L::kEndWeight ? h.w : 0ull, rootel ? ld_ca(rootel + x) : x, true);
       continue;
     }
     uint32_t j;
@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(TREE_THREADS) k_tree_propagate(const typename 
       const Out o = N::out(out + rl.block_of(y));
       sink.put(x, acc + o.rank, o.root, false);
     } else if (h.b == y) {
-      sink.put(x, L::kEndWeight ? acc + h.w : acc, rootel ? __ldg(rootel + y) : y, false);
+      sink.put(x, L::kEndWeight ? acc + h.w : acc, rootel ? ld_ca(rootel + y) : y, false);
     } else {
       set_error(st, KASCADE_ERR_CYCLE, x);
     }
