@@ -69,7 +69,7 @@ SECTORS_LIST = {True: 0.25 + 0.125 + 0.25 + 2 + 2, False: 0.25 + 0.25 + 2 + 1.75
 # elements): prepare as above; chase: the record's random sector read + the
 # 16 B log entry (1 + 1/2); resolve: log read + resolved entry written (1/2 +
 # 1/2; its ruler lookups hit L1 for the most part and are left out); partition
-# (from 2^25 elements): read + write (1/2 + 1/2); place: read (1/2) + root and
+# (above 24.6 million elements): read + write (1/2 + 1/2); place: read (1/2) + root and
 # rank writes (1/2).
 SECTORS_LIST_LOG = {True: 0.25 + 0.125 + 0.25 + 1.5 + 1 + 1 + 1, False: 0.25 + 0.25 + 1.5 + 1 + 1 + 1}
 # DRAM bytes the write-free pipeline's kernels move, measured by ncu

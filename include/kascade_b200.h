@@ -88,8 +88,10 @@ typedef struct kascade_opts {
   uint32_t seed;              /* ruler-sampling seed                                */
   uint32_t level0_mode;       /* first level: 0 by size, 1 stamping chase, 2
                                  write-free chase (read-only chase, log, radix
-                                 partition by element, dense placement; what 0
-                                 takes from 8 to 12 million elements on)           */
+                                 partition by element, dense placement), which 0
+                                 takes from 8 million elements on (12 million with
+                                 64-bit weights).  Above 2^22 elements 2 partitions
+                                 in two passes, 0 only above 24.6 million          */
   uint32_t max_chain;         /* accepted, no effect (chains have no hop cap)      */
 } kascade_opts;
 

@@ -47,20 +47,28 @@ constexpr uint32_t SUB_SHIFT = 13;  // 2^13 elements per sub-window (second pass
 constexpr uint32_t SUB = 1u << SUB_SHIFT;
 constexpr uint32_t SUBS = WIN / SUB;    // sub-windows per window
 constexpr uint32_t MAX_BUCKETS = 4096;  // windows for 2^32 elements
-// One partition pass up to this size: 2e7 elements in runs of 64 890 -> 810 us,
-// a batch of 2e7 records 1554 -> 1471, lists of random order 985 -> 1019 at
-// 1.6e7 and equal at 3.3e7 (a tile's entries then fall into as many
-// sub-windows, and neither way of writing them coalesces).  A call that asks
-// for this path takes two passes from 2^22 elements on.
-constexpr uint32_t DIRECT_MAX = 1u << 25, DIRECT_MAX_FORCED = 1u << 22;
-static_assert(DIRECT_MAX / SUB <= MAX_BUCKETS, "sub-windows per pass");
-constexpr uint32_t CURSOR_STRIDE = 8;   // one 32 B sector per cursor (spreads the atomics)
 constexpr uint32_t PT_THREADS = 256;    // partition: threads per block
 // entries per thread (a tile is PT_THREADS x ITEMS entries) and resident
 // blocks per SM of the two partition passes: 2048-entry tiles, 4 blocks per
 // SM (more tiles in flight per SM than 4096-entry tiles at 2 blocks)
 constexpr uint32_t P1_ITEMS = 8, P1_BLOCKS = 4;
 constexpr uint32_t P2_ITEMS = 8, P2_BLOCKS = 4;
+// One partition pass, straight to the sub-windows, up to as many of these as
+// leave room for four blocks' counters on an SM (24.6 million elements); with
+// three the pass loses to two of them whatever the order.  One / two passes, us:
+//   runs of 64    1.6e7 645 / 706, 2e7 760 / 850, 2.4e7 911 / 993,
+//                 2.8e7 1219 / 1148, 2^25 1922 / 1353
+//   random order  1.4e7 777 / 787, 2e7 1130 / 1088, 2.4e7 1399 / 1297,
+//                 2.8e7 1842 / 1503, 2^25 2806 / 1792
+// (a tile of a random order has as many sub-windows as entries, and neither way
+// of writing them coalesces).  A call that asks for this path takes two passes
+// from 2^22 elements on.
+constexpr uint32_t DIRECT_SUBS = 3000;
+constexpr uint32_t DIRECT_MAX = DIRECT_SUBS * SUB, DIRECT_MAX_FORCED = 1u << 22;
+static_assert(DIRECT_SUBS <= MAX_BUCKETS &&
+                  P1_BLOCKS * (PT_THREADS * P1_ITEMS * 16 + DIRECT_SUBS * 8 + 1088) <= 228 * 1024,
+              "four blocks on an SM");
+constexpr uint32_t CURSOR_STRIDE = 8;   // one 32 B sector per cursor (spreads the atomics)
 constexpr uint32_t FIN_THREADS = 512;  // place: threads per block (one sub-window per iteration; 2 blocks per SM)
 constexpr uint32_t FIN_GROUP = 8;      // place: entries a thread has in flight
 constexpr uint32_t NO_ROOT = 0xFFFFFFFFu;          // shared-memory root slot not written
