@@ -234,7 +234,8 @@ KASCADE_API kascade_status kascade_compute_stats(kascade_ctx* ctx, const uint64_
  *   parent[v] (parent[v] == v marks a root) -> root_out[v], depth_out[v]
  *   (edge count to the root; 0 at roots): the paths to the roots are
  *   contracted level by level (no Euler tour is built).  Of kascade_opts,
- *   ruler_spacing(_deep), base_case_size and seed apply.
+ *   ruler_spacing(_deep), base_case_size and seed apply; a spacing above 4
+ *   counts as 4.
  * Replaces: rank_via_euler_tour (eulertour.hpp:22-27, eulertour.cpp:337-377).
  * ------------------------------------------------------------------------- */
 KASCADE_API kascade_status kascade_root_forest(kascade_ctx* ctx, const uint64_t* parent,
@@ -301,8 +302,9 @@ KASCADE_API kascade_status kascade_gen_forest(uint64_t n, uint64_t seed, uint32_
  * size and kind.  Outputs are written at the same positions: for lists root
  * and rank, for forests root and depth, roots relative to their instance.
  * weights (optional) apply to list instances.  The lists' ruler spacing comes
- * from the context's size-class table unless opts->ruler_spacing is set.  No counterpart in the reference (it ranks one distributed instance
- * per call).
+ * from the context's size-class table unless opts->ruler_spacing is set; the
+ * forests have a spacing of their own.  No counterpart in the reference (it
+ * ranks one distributed instance per call).
  * ------------------------------------------------------------------------- */
 #define KASCADE_SEG_LIST 0u
 #define KASCADE_SEG_FOREST 1u

@@ -38,7 +38,10 @@ constexpr int TREE_OUT_ITEMS = 4;  // (2: 1.07 ms, 4 and 8: 0.95 for 2^26 vertic
 // Mean elements per ruler.  Large levels are bound by what they read at
 // random, (s + 1) s / (s - 1) reads an element over all levels; small ones by
 // their longest walks and by launches.  2^26 caterpillars, s = 2 / 3 / 4:
-// 4.0 / 4.2 / 4.4 ms; 4.2M random recursive trees 314 / 275 / 250 us.
+// 4.0 / 4.2 / 4.4 ms; 4.2M random recursive trees 314 / 275 / 250 us.  A
+// caller's spacing counts up to TREE_SPACING: without stamps a walk reads all of
+// its gap, so that the spacings lists are fast with are slow here (a path of
+// 2^25 vertices, s = 2 / 8 / 24 / 48: 2.9 / 5.3 / 10.1 / 17.3 ms).
 constexpr uint32_t TREE_SPACING = 4, TREE_SPACING_LARGE = 2, TREE_LARGE = 1u << 23;
 // Largest last level: without stamps the one-CTA ranker's walks grow with its
 // spacing (3100 elements 15 us, 6200 24, 8300 44, 12500 75; a level above it
@@ -417,7 +420,9 @@ TreeLevels plan_tree(uint32_t n, const uint32_t* count, const Params& p) {
   lv.ext[0].count = count;
   while (lv.ext[k].cap > base && k < MAX_LEVELS) {
     const uint32_t given = k == 0 ? p.spacing_given : p.spacing_deep;
-    const uint32_t s = given ? std::max(2u, given) : lv.ext[k].cap > TREE_LARGE ? TREE_SPACING_LARGE : TREE_SPACING;
+    const uint32_t s = given                        ? std::clamp(given, 2u, TREE_SPACING)
+                       : lv.ext[k].cap > TREE_LARGE ? TREE_SPACING_LARGE
+                                                    : TREE_SPACING;
     lv.rulers[k] = make_rulers(s, salt_for(p.seed, k));
     lv.ext[k + 1].cap = ruler_count(lv.ext[k].cap, lv.rulers[k]);
     lv.ext[k + 1].count = count;
@@ -427,6 +432,12 @@ TreeLevels plan_tree(uint32_t n, const uint32_t* count, const Params& p) {
   lv.last = k;
   lv.rulers[k].s = 0;
   return lv;
+}
+
+// Parameters without the caller's spacing, where that is not the trees'.
+Params own_spacing(Params p) {
+  p.spacing_given = p.spacing_deep = 0;
+  return p;
 }
 
 template <class L, class N>
@@ -530,14 +541,14 @@ kascade_status root_forests(kascade_ctx& ctx, const uint32_t* parent, uint32_t n
   if (n == 0) return KASCADE_OK;
   uint32_t* count = alloc<uint32_t>(ctx, 1);
   if (!count) return KASCADE_ERR_OOM;
-  const TreeLevels lv = plan_tree(n, count, p);
+  const TreeLevels lv = plan_tree(n, count, own_spacing(p));  // (a batch's is its lists')
   if (lv.last == 0) return rank_parents_one_cta(ctx, parent, n, sink, last, s);
   return root_levels(ctx, parent, n, lv, count, sink, false, last, s);
 }
 
 kascade_status rank_forest_weighted(kascade_ctx& ctx, const uint64_t* succ, WKind wk, const void* w, uint32_t n,
                                     const SinkPlain& sink, const Params& p, cudaStream_t s) {
-  const TreeLevels lv = plan_tree(n, nullptr, p);
+  const TreeLevels lv = plan_tree(n, nullptr, own_spacing(p));
   if (lv.last == 0) return rank_arrays_one_cta(ctx, succ, wk, w, n, sink, CTA_TREES, s);
   ctx.last_levels.assign(1, n);
   Level0 l0;  // F16x16, no stamps
