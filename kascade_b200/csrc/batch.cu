@@ -266,11 +266,12 @@ kascade_status batch_enqueue(kascade_ctx& ctx, const BatchTables& t, const uint6
   }
   // The forests' levels run beside the lists': neither fills the chip for long
   // (128 instances of 3e6 elements 380 -> 270 us, 4096 of 2^28 11.2 -> 10.5 ms).  A
-  // context with a budget of SMs, and profiled calls, keep one stream.
+  // context with a budget of SMs, a stream in a partition of them, and profiled
+  // calls keep one stream.
   const SinkBatch lists{root_out, rank_out, t.lists}, forests{root_out, rank_out, t.forests};
   // (trees among the lists of a small batch are ranked, as in a small call)
   const CtaMode mode = t.total + t.F > ONE_CTA_TREES ? CTA_LISTS : CTA_SMALL_TREES;
-  const bool beside = t.L && t.F && !ctx.profile && ctx.usable_sms() == ctx.sm_count;
+  const bool beside = t.L && t.F && !ctx.profile && ctx.usable_sms() == ctx.sm_count && !in_partition(s);
   ctx.last_levels.assign(1, 0);
   if (beside) {
     Params q = p;

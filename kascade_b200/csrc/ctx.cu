@@ -145,8 +145,27 @@ kascade_status read_u32(kascade_ctx& ctx, const uint32_t* dptr, uint32_t* out, c
   return KASCADE_OK;
 }
 
+bool in_partition(cudaStream_t s) {
+  using Fn = CUresult(CUstream, CUgreenCtx*);
+  static Fn* const green = [] {
+    Fn* fn = nullptr;
+    return driver_fn("cuStreamGetGreenCtx", fn) ? fn : nullptr;
+  }();
+  CUgreenCtx g = nullptr;
+  return green && green(s, &g) == CUDA_SUCCESS && g;
+}
+
 kascade_status side_fork(kascade_ctx& ctx, cudaStream_t s) {
-  if (!ctx.side) KS_CUDA(cudaStreamCreateWithFlags(&ctx.side, cudaStreamNonBlocking));
+  int priority = 0;
+  KS_CUDA(cudaStreamGetPriority(s, &priority));
+  if (ctx.side && priority != ctx.side_priority) {
+    cudaStreamDestroy(ctx.side);  // (every fork was joined)
+    ctx.side = nullptr;
+  }
+  if (!ctx.side) {
+    KS_CUDA(cudaStreamCreateWithPriority(&ctx.side, cudaStreamNonBlocking, priority));
+    ctx.side_priority = priority;
+  }
   if (!ctx.fork) KS_CUDA(cudaEventCreateWithFlags(&ctx.fork, cudaEventDisableTiming));
   if (!ctx.join) KS_CUDA(cudaEventCreateWithFlags(&ctx.join, cudaEventDisableTiming));
   KS_CUDA(cudaEventRecord(ctx.fork, s));

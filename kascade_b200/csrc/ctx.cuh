@@ -2,6 +2,7 @@
 // status word, a pinned read-back buffer and optional per-kernel timing.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -53,6 +54,7 @@ struct kascade_ctx {
   bool async_pending = false;
   // a second stream for device work that is independent within a call
   cudaStream_t side = nullptr;
+  int side_priority = 0;
   cudaEvent_t fork = nullptr, join = nullptr;
   // size classes: a batch of at most class_max[i] records uses a ruler spacing
   // of class_spacing[i], a call that ranks one list of that size
@@ -111,8 +113,26 @@ kascade_status status_finish(kascade_ctx& ctx, cudaStream_t s);
 // Read one device word into the pinned buffer and wait for it.
 kascade_status read_u32(kascade_ctx& ctx, const uint32_t* dptr, uint32_t* out, cudaStream_t s);
 
-// Work on ctx.side that may run beside what is enqueued on `s` from here on,
-// and its end: `s` waits for it.  Every fork is joined, in error paths too.
+// A driver function by name; false where the driver has none.
+template <class F>
+bool driver_fn(const char* name, F*& fn) {
+  void* p = nullptr;
+  cudaDriverEntryPointQueryResult q{};
+  if (cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess ||
+      !p) {
+    cudaGetLastError();
+    return false;
+  }
+  fn = reinterpret_cast<F*>(p);
+  return true;
+}
+
+// Whether `s` belongs to an SM partition (a green context), which another
+// stream would leave.
+bool in_partition(cudaStream_t s);
+// Work on ctx.side, of the priority of `s`, that may run beside what is
+// enqueued on `s` from here on, and its end: `s` waits for it.  Every fork is
+// joined, in error paths too.
 kascade_status side_fork(kascade_ctx& ctx, cudaStream_t s);
 kascade_status side_join(kascade_ctx& ctx, cudaStream_t s);
 

@@ -260,19 +260,6 @@ struct kascade_server {
   void drop_partition();
 };
 
-template <class F>
-static bool driver_fn(const char* name, F*& fn) {
-  void* p = nullptr;
-  cudaDriverEntryPointQueryResult q{};
-  if (cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess ||
-      !p) {
-    cudaGetLastError();
-    return false;
-  }
-  fn = reinterpret_cast<F*>(p);
-  return true;
-}
-
 // Carve an SM partition of (all SMs - latency_sms, rounded down to the
 // partition granularity of 8) as a green context, and give lane 1 a second
 // library context and stream inside it.  Work in the partition cannot use
@@ -281,6 +268,7 @@ static bool driver_fn(const char* name, F*& fn) {
 // budgets only) where the driver offers no green contexts.
 bool kascade_server::setup_partition() {
   if (cfg.latency_sms == 0) return false;
+  using ks::driver_fn;
   Driver& d = drv;
   if (!driver_fn("cuDeviceGet", d.DeviceGet) || !driver_fn("cuDeviceGetDevResource", d.DeviceGetDevResource) ||
       !driver_fn("cuDevSmResourceSplitByCount", d.DevSmResourceSplitByCount) ||
