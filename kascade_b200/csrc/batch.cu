@@ -238,11 +238,15 @@ Params batch_params(const kascade_ctx& ctx, uint64_t records, const kascade_opts
 kascade_status batch_enqueue(kascade_ctx& ctx, const BatchTables& t, const uint64_t* in, const uint32_t* weights,
                              uint64_t* root_out, uint64_t* rank_out, const kascade_opts* opts, cudaStream_t s) {
   const Params p = batch_params(ctx, t.L, opts);
-  Level0 l0;
-  KS_TRY(alloc_level0(ctx, plan_level0(p, t.L, weights ? WKind::U32 : WKind::Unit), t.L, &l0));
-  const Rulers rl = level0_rulers(p);
+  ctx.last_levels.assign(1, 0);
   uint32_t* fpar = alloc<uint32_t>(ctx, t.F);
   if (!fpar) return KASCADE_ERR_OOM;
+  Forest f;
+  KS_TRY(alloc_forests(ctx, t.F, p, &f));
+  Lists l;  // last: they can do with less
+  KS_TRY(alloc_lists(ctx, p, t.L, weights ? WKind::U32 : WKind::Unit, &l));
+  const Level0& l0 = l.l0;
+  const Rulers rl = level0_rulers(p);
   {
     ProfScope ps(ctx, "batch_prepare", s);
     const unsigned grid = grid_for(ctx, (t.total + BP_PER - 1) / BP_PER, BP_THREADS, 8);
@@ -272,19 +276,18 @@ kascade_status batch_enqueue(kascade_ctx& ctx, const BatchTables& t, const uint6
   // (trees among the lists of a small batch are ranked, as in a small call)
   const CtaMode mode = t.total + t.F > ONE_CTA_TREES ? CTA_LISTS : CTA_SMALL_TREES;
   const bool beside = t.L && t.F && !ctx.profile && ctx.usable_sms() == ctx.sm_count && !in_partition(s);
-  ctx.last_levels.assign(1, 0);
   if (beside) {
     Params q = p;
     q.last = false;
     KS_TRY(side_fork(ctx, s));
-    kascade_status st = rank_records(ctx, l0, t.L, lists, mode, q, s);
-    const kascade_status sf = root_forests(ctx, fpar, t.F, forests, false, q, ctx.side);
+    kascade_status st = rank_records(ctx, l, lists, mode, q, s);
+    const kascade_status sf = root_forests(ctx, fpar, f, forests, false, ctx.side);
     const kascade_status sj = side_join(ctx, s);
     if (st == KASCADE_OK) st = sf == KASCADE_OK ? sj : sf;
     KS_TRY(st);
   } else {
-    KS_TRY(root_forests(ctx, fpar, t.F, forests, t.L == 0, p, s));
-    KS_TRY(rank_records(ctx, l0, t.L, lists, mode, p, s));
+    KS_TRY(root_forests(ctx, fpar, f, forests, t.L == 0, s));
+    KS_TRY(rank_records(ctx, l, lists, mode, p, s));
   }
   ctx.last_levels[0] = t.total + t.F;  // as a batch's size is reported: a forest's vertex counts twice
   return KASCADE_OK;
@@ -372,7 +375,7 @@ kascade_status batch_plan_create(int device, const kascade_segment* segs, uint32
   if (st == KASCADE_OK) st = plan_admits(ctx, t, in, &opts, s);
   if (st == KASCADE_OK && cudaStreamSynchronize(s) != cudaSuccess) st = KASCADE_ERR_CUDA;
   if (st != KASCADE_OK) return fail(st);
-  const size_t blocks_before = ctx.blocks.size();
+  ctx.arena_fixed = true;  // (the eager run sized it)
   if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
     cudaGetLastError();
     return fail(KASCADE_ERR_CUDA);
@@ -382,10 +385,9 @@ kascade_status batch_plan_create(int device, const kascade_segment* segs, uint32
   if (st == KASCADE_OK) st = status_publish(ctx, s);
   cudaGraph_t g = nullptr;
   const cudaError_t ce = cudaStreamEndCapture(s, &g);
+  ctx.arena_fixed = false;
   plan->graph = g;
   if (st == KASCADE_OK && (ce != cudaSuccess || !g)) st = KASCADE_ERR_CUDA;
-  // the capture must not have grown the arena (the eager run sized it)
-  if (st == KASCADE_OK && ctx.blocks.size() != blocks_before) st = KASCADE_ERR_UNSUPPORTED;
   if (st == KASCADE_OK && cudaGraphInstantiate(&plan->exec, g, 0) != cudaSuccess) st = KASCADE_ERR_CUDA;
   cudaGetLastError();
   if (st != KASCADE_OK) return fail(st);

@@ -78,12 +78,12 @@ kascade_status rank_list_generic(kascade_ctx& ctx, const uint64_t* succ, WKind w
   if (n == 0) return KASCADE_OK;
   if (n > MAX_LIST) return KASCADE_ERR_TOO_LARGE;
   const SinkPlain sink{root_out, rank_out, keep_roots};
-  Level0 l0;
   if (p.algorithm == KASCADE_ALGO_SPARSE_RULING_SET) {
     if (n <= p.base_max) return rank_arrays_one_cta(ctx, succ, wk, w, (uint32_t)n, sink, CTA_SMALL_TREES, s);
-    KS_TRY(alloc_level0(ctx, plan_level0(p, n, wk), n, &l0));
-    KS_TRY(prepare_arrays(ctx, succ, wk, w, (uint32_t)n, l0, level0_rulers(p), s));
-    return rank_records(ctx, l0, (uint32_t)n, sink, CTA_SMALL_TREES, p, s);
+    Lists l;
+    KS_TRY(alloc_lists(ctx, p, n, wk, &l));
+    KS_TRY(prepare_arrays(ctx, succ, wk, w, (uint32_t)n, l.l0, level0_rulers(p), s));
+    return rank_records(ctx, l, sink, CTA_SMALL_TREES, p, s);
   }
   return rank_forest_weighted(ctx, succ, wk, w, (uint32_t)n, sink, p, s);
 }

@@ -35,6 +35,13 @@
 #include "ranker.cuh"
 
 namespace ks {
+
+struct __align__(16) LogEnt {
+  uint32_t x;
+  uint32_t id;
+  uint64_t off;
+};
+
 namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
@@ -74,11 +81,6 @@ constexpr uint32_t FIN_GROUP = 8;      // place: entries a thread has in flight
 constexpr uint32_t NO_ROOT = 0xFFFFFFFFu;          // shared-memory root slot not written
 constexpr unsigned long long NOT_REACHED = ~0ull;  // root output of an element no chain reached
 
-struct __align__(16) LogEnt {
-  uint32_t x;
-  uint32_t id;
-  uint64_t off;
-};
 __device__ __forceinline__ void st_log(LogEnt* p, uint32_t x, uint32_t id, uint64_t off) {
   __stcs(reinterpret_cast<uint4*>(p), make_uint4(x, id, (uint32_t)off, (uint32_t)(off >> 32)));
 }
@@ -553,48 +555,16 @@ kascade_status raise_smem_limits() {
 }
 
 template <class F>
-unsigned chase_grid(const kascade_ctx& ctx, uint32_t r, uint32_t block) {
-  const uint64_t grid = (uint64_t)ctx.usable_sms() * std::max(1u, LOG_CHAINS_PER_SM / block);
-  return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(grid, ((uint64_t)r + block - 1) / block));
-}
-
-// The chase's log and its size.
-struct Log {
-  LogEnt* ent = nullptr;
-  uint32_t* fill = nullptr;  // per chunk
-  uint32_t* cursor = nullptr;
-  uint32_t nchunks = 0;
-};
-
-template <class F>
-kascade_status rank_level0_log_as(kascade_ctx& ctx, const Level0& l0, uint32_t n, const LogTarget& t, const Params& p,
+kascade_status rank_level0_log_as(kascade_ctx& ctx, const Lists& l, const LogTarget& t, const Params& p,
                                   cudaStream_t s) {
-  Levels lv;
-  KS_TRY(plan_levels(ctx, n, p, &lv));
-  const uint32_t r = lv.n[1];
-  const uint32_t block = p.block;
-  const unsigned grid = chase_grid<F>(ctx, r, block);
-  const uint64_t warps = (uint64_t)grid * (block / 32);
-  Log log;
-  log.nchunks = (uint32_t)(((uint64_t)n + LOG_CHUNK - 1) / LOG_CHUNK + warps + 1);
+  const Levels& lv = l.lv;
+  const Log& log = l.log;
+  const uint32_t n = l.n, r = lv.n[1];
   const uint32_t nb = (uint32_t)(((uint64_t)n + WIN - 1) / WIN);
-  const uint32_t nb1 = nb ? nb : 1;
-  const uint64_t cursor_words = (uint64_t)nb1 * (SUBS + 1) * CURSOR_STRIDE;
-  log.ent = alloc<LogEnt>(ctx, (uint64_t)log.nchunks * LOG_CHUNK);
-  // zeroed by one memset: chunk cursor, unreached count; the partition
-  // cursors; the chunks' fill counts
-  const uint64_t zero_words = 8 + cursor_words + log.nchunks;
-  uint32_t* zero = alloc<uint32_t>(ctx, zero_words);
-  if (!log.ent || !zero) return KASCADE_ERR_OOM;
-  KS_CUDA(cudaMemsetAsync(zero, 0, sizeof(uint32_t) * zero_words, s));
-  log.cursor = zero + 0;
-  uint32_t* ucount = zero + 1;
-  uint32_t* cursor1 = zero + 8;
-  uint32_t* cursor2 = cursor1 + (uint64_t)nb1 * CURSOR_STRIDE;
-  log.fill = cursor1 + cursor_words;
+  KS_CUDA(cudaMemsetAsync(log.zero, 0, sizeof(uint32_t) * log.zero_words, s));
   {
     ProfScope ps(ctx, "chase", s);
-    k_chase_log<F><<<grid, block, 0, s>>>(l0.records<F>(), n, lv.rulers[0], r, next_level(lv, 1),
+    k_chase_log<F><<<log.grid, p.block, 0, s>>>(l.l0.records<F>(), n, lv.rulers[0], r, next_level(lv, 1),
                                           &ctx.d_status->work[0], log.ent,
                                           log.fill, log.cursor, log.nchunks, hop_cap(lv.rulers[0]), ctx.d_status);
     KS_CHECK_LAUNCH();
@@ -602,56 +572,49 @@ kascade_status rank_level0_log_as(kascade_ctx& ctx, const Level0& l0, uint32_t n
   KS_TRY(rank_deep(ctx, lv, s));
 
   // Up to DIRECT_MAX elements the log goes straight to the sub-windows;
-  // larger ones in two passes, windows (part), then sub-windows into the log's
-  // memory when it is large enough (the log is dead by then).
-  const bool direct = n <= (p.level0_mode == 2 ? DIRECT_MAX_FORCED : DIRECT_MAX);
+  // larger ones in two passes, windows (part), then sub-windows (part2).
+  const bool direct = log.direct;
   const uint32_t nsub = (uint32_t)(((uint64_t)n + SUB - 1) / SUB);
-  const uint64_t part2_need = (uint64_t)nsub * SUB;
-  LogEnt* part = alloc<LogEnt>(ctx, direct ? std::max<uint64_t>(part2_need, 1) : (uint64_t)nb1 * WIN);
-  LogEnt* part2 = direct                                                ? part
-                  : (uint64_t)log.nchunks * LOG_CHUNK >= part2_need ? log.ent
-                                                                    : alloc<LogEnt>(ctx, part2_need ? part2_need : 1);
-  if (!part || !part2) return KASCADE_ERR_OOM;
   KS_TRY(raise_smem_limits());
   if (direct) {
     ProfScope ps(ctx, "resolve", s);
     const uint32_t tiles = (log.nchunks + TILE1 / LOG_CHUNK - 1) / (TILE1 / LOG_CHUNK);
     const size_t smem = TILE1 * sizeof(LogEnt) + 2 * sizeof(uint32_t) * std::max(nsub, 1u);
     k_part1<<<(unsigned)std::min<uint64_t>(tiles, (uint64_t)ctx.usable_sms() * P1_BLOCKS), PT_THREADS, smem, s>>>(
-        log.ent, log.fill, log.nchunks, lv.out[1], n, SUB_SHIFT, nsub, part, cursor2, log.cursor, ctx.d_status);
+        log.ent, log.fill, log.nchunks, lv.out[1], n, SUB_SHIFT, nsub, log.part, log.cursor2, log.cursor, ctx.d_status);
     KS_CHECK_LAUNCH();
   } else {
-    const size_t smem1 = TILE1 * sizeof(LogEnt) + 2 * sizeof(uint32_t) * nb1;
+    const size_t smem1 = TILE1 * sizeof(LogEnt) + 2 * sizeof(uint32_t) * nb;
     const size_t smem2 = TILE2 * sizeof(LogEnt) + 2 * sizeof(uint32_t) * SUBS;
     {
       ProfScope ps(ctx, "resolve", s);
       const uint32_t tiles1 = (log.nchunks + TILE1 / LOG_CHUNK - 1) / (TILE1 / LOG_CHUNK);
       k_part1<<<(unsigned)std::min<uint64_t>(tiles1, (uint64_t)ctx.usable_sms() * P1_BLOCKS), PT_THREADS, smem1, s>>>(
-          log.ent, log.fill, log.nchunks, lv.out[1], n, WIN_SHIFT, nb, part, cursor1, log.cursor, ctx.d_status);
+          log.ent, log.fill, log.nchunks, lv.out[1], n, WIN_SHIFT, nb, log.part, log.cursor1, log.cursor, ctx.d_status);
       KS_CHECK_LAUNCH();
     }
     const uint32_t tiles2 = nb * (WIN / TILE2);
     if (tiles2) {
       ProfScope ps(ctx, "partition", s);
       k_part2<<<(unsigned)std::min<uint64_t>(tiles2, (uint64_t)ctx.usable_sms() * P2_BLOCKS), PT_THREADS, smem2, s>>>(
-          part, cursor1, 0, nullptr, n, 0, nb, part2, cursor2, nullptr, ctx.d_status);
+          log.part, log.cursor1, 0, nullptr, n, 0, nb, log.part2, log.cursor2, nullptr, ctx.d_status);
       KS_CHECK_LAUNCH();
     }
   }
   // the first pass's source or output is dead by now: it holds the unreached list
-  uint32_t* ulist = reinterpret_cast<uint32_t*>(direct ? log.ent : part);
+  uint32_t* ulist = reinterpret_cast<uint32_t*>(direct ? log.ent : log.part);
   {
     ProfScope ps(ctx, "place", s);
     const uint32_t items = nb * SUBS;
     const size_t smem = SUB * (sizeof(unsigned long long) + sizeof(uint32_t));
     k_place<<<(unsigned)std::max<uint64_t>(1, std::min<uint64_t>(items, (uint64_t)ctx.usable_sms() * 2)),
-                FIN_THREADS, smem, s>>>(part2, cursor2, nb, n, t.root, t.rank, ulist, ucount, n, t.seg, t.keep_roots,
+                FIN_THREADS, smem, s>>>(log.part2, log.cursor2, nb, n, t.root, t.rank, ulist, log.ucount, n, t.seg, t.keep_roots,
                                         ctx.d_status);
     KS_CHECK_LAUNCH();
   }
   {
     ProfScope ps(ctx, "heads", s);
-    k_walk_unreached<F><<<ctx.usable_sms() * 4, 256, 0, s>>>(l0.records<F>(), ulist, ucount, n, t.root, t.rank, t.seg,
+    k_walk_unreached<F><<<ctx.usable_sms() * 4, 256, 0, s>>>(l.l0.records<F>(), ulist, log.ucount, n, t.root, t.rank, t.seg,
                                                              t.keep_roots, ctx.d_status, status_host(ctx, p.last));
     KS_CHECK_LAUNCH();
   }
@@ -660,11 +623,36 @@ kascade_status rank_level0_log_as(kascade_ctx& ctx, const Level0& l0, uint32_t n
 
 }  // namespace
 
-kascade_status rank_level0_log(kascade_ctx& ctx, const Level0& l0, uint32_t n, const LogTarget& t, const Params& p,
-                               cudaStream_t s) {
+kascade_status alloc_log(kascade_ctx& ctx, uint32_t n, uint32_t rulers, const Params& p, Log* log) {
+  const uint64_t blocks = (uint64_t)ctx.usable_sms() * std::max(1u, LOG_CHAINS_PER_SM / p.block);
+  log->grid = (unsigned)std::max<uint64_t>(1, std::min(blocks, ((uint64_t)rulers + p.block - 1) / p.block));
+  const uint64_t warps = (uint64_t)log->grid * (p.block / 32);
+  log->nchunks = (uint32_t)(((uint64_t)n + LOG_CHUNK - 1) / LOG_CHUNK + warps + 1);
+  log->direct = n <= (p.level0_mode == 2 ? DIRECT_MAX_FORCED : DIRECT_MAX);
+  const uint64_t nb = ((uint64_t)n + WIN - 1) / WIN, nsub = ((uint64_t)n + SUB - 1) / SUB;
+  const uint64_t cursors = nb * (SUBS + 1) * CURSOR_STRIDE;
+  log->ent = alloc<LogEnt>(ctx, (uint64_t)log->nchunks * LOG_CHUNK);
+  log->zero_words = 8 + cursors + log->nchunks;
+  log->zero = alloc<uint32_t>(ctx, log->zero_words);
+  log->part = alloc<LogEnt>(ctx, log->direct ? nsub * SUB : nb * WIN);
+  // the second pass's output takes the log's memory where that is large enough
+  // (the log is dead by then)
+  log->part2 = log->direct                                          ? log->part
+               : (uint64_t)log->nchunks * LOG_CHUNK >= nsub * SUB ? log->ent
+                                                                    : alloc<LogEnt>(ctx, nsub * SUB);
+  if (!log->ent || !log->zero || !log->part || !log->part2) return KASCADE_ERR_OOM;
+  log->cursor = log->zero;
+  log->ucount = log->zero + 1;
+  log->cursor1 = log->zero + 8;
+  log->cursor2 = log->cursor1 + nb * CURSOR_STRIDE;
+  log->fill = log->cursor1 + cursors;
+  return KASCADE_OK;
+}
+
+kascade_status rank_level0_log(kascade_ctx& ctx, const Lists& l, const LogTarget& t, const Params& p, cudaStream_t s) {
   // records of 32-bit weights are alike with and without 64-bit stamps
-  if (l0.fmt == Format::F16x16) return rank_level0_log_as<F16x16>(ctx, l0, n, t, p, s);
-  return rank_level0_log_as<F8x16>(ctx, l0, n, t, p, s);
+  if (l.l0.fmt == Format::F16x16) return rank_level0_log_as<F16x16>(ctx, l, t, p, s);
+  return rank_level0_log_as<F8x16>(ctx, l, t, p, s);
 }
 
 }  // namespace ks

@@ -45,11 +45,14 @@ void* arena_alloc(kascade_ctx& ctx, size_t bytes) {
       return p;
     }
   }
+  if (ctx.arena_fixed) return nullptr;
   size_t prev = ctx.blocks.empty() ? 0 : ctx.blocks.back().cap;
   size_t cap = bytes;
-  if (cap < prev) cap = prev;
-  if (cap < ctx.reserve_bytes) cap = ctx.reserve_bytes;
-  if (cap < (size_t(64) << 20)) cap = size_t(64) << 20;
+  if (!ctx.arena_exact) {
+    if (cap < prev) cap = prev;
+    if (cap < ctx.reserve_bytes) cap = ctx.reserve_bytes;
+    if (cap < (size_t(64) << 20)) cap = size_t(64) << 20;
+  }
   char* p = nullptr;
   if (cudaMalloc(&p, cap) != cudaSuccess) {
     cudaGetLastError();
@@ -62,6 +65,16 @@ void* arena_alloc(kascade_ctx& ctx, size_t bytes) {
   }
   ctx.blocks.push_back({p, cap, bytes, true});
   return p;
+}
+
+ArenaMark arena_mark(const kascade_ctx& ctx) {
+  return ArenaMark{ctx.blocks.size(), ctx.blocks.empty() ? 0 : ctx.blocks.back().used};
+}
+
+void arena_rewind(kascade_ctx& ctx, const ArenaMark& m) {
+  for (; ctx.blocks.size() > m.blocks; ctx.blocks.pop_back())
+    if (ctx.blocks.back().owned) cudaFree(ctx.blocks.back().ptr);
+  if (m.blocks) ctx.blocks.back().used = m.used;
 }
 
 void arena_adopt(kascade_ctx& ctx, char* p, size_t bytes) {

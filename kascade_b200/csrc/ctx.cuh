@@ -33,6 +33,8 @@ struct kascade_ctx {
   };
   std::vector<Block> blocks;
   size_t reserve_bytes = 0;
+  bool arena_fixed = false;  // the arena may not grow (a stream capture)
+  bool arena_exact = false;  // it grows by no more than it is asked for
   // profiling
   bool profile = false;
   struct Pending {
@@ -94,6 +96,28 @@ void arena_adopt(kascade_ctx& ctx, char* p, size_t bytes);
 // (which keeps a context the caller made current, e.g. an SM partition).
 cudaError_t ensure_device(int device);
 void* arena_alloc(kascade_ctx& ctx, size_t bytes);  // nullptr on OOM
+// A point to go back to: what was allocated since, and not yet used by any
+// enqueued work, is given back.
+struct ArenaMark {
+  size_t blocks, used;
+};
+ArenaMark arena_mark(const kascade_ctx& ctx);
+void arena_rewind(kascade_ctx& ctx, const ArenaMark& m);
+// Run `f`, which allocates and enqueues nothing.  Blocks are at least as large
+// as the last one; where that does not fit, it runs again with blocks of the
+// size asked for.  Out of memory all the same: nothing stays allocated.
+template <class F>
+kascade_status arena_try(kascade_ctx& ctx, F f) {
+  const ArenaMark m = arena_mark(ctx);
+  kascade_status st = f();
+  if (st != KASCADE_ERR_OOM) return st;
+  arena_rewind(ctx, m);
+  ctx.arena_exact = true;
+  st = f();
+  ctx.arena_exact = false;
+  if (st == KASCADE_ERR_OOM) arena_rewind(ctx, m);
+  return st;
+}
 template <class T>
 T* alloc(kascade_ctx& ctx, size_t count) {
   return reinterpret_cast<T*>(arena_alloc(ctx, count * sizeof(T) + 16));

@@ -963,6 +963,17 @@ Params make_params(const kascade_ctx& ctx, const kascade_opts* o, uint64_t n) {
   return p;
 }
 
+Rulers level0_rulers(const Params& p) { return make_rulers(p.spacing0, salt_for(p.seed, 0)); }
+
+namespace {
+
+// How level 0 of n elements of that weight kind runs: the records' format, and
+// whether it takes the write-free path.
+struct Level0Plan {
+  Format fmt;
+  bool write_free;
+};
+
 // The three ways to run level 0, by what stays in L2 (lists of random order,
 // unit / 32-bit / 64-bit weights, us):
 //   split records and stamps while both fit: 4e6 elements 247 / 310 / 417
@@ -970,13 +981,14 @@ Params make_params(const kascade_ctx& ctx, const kascade_opts* o, uint64_t n) {
 //     against 242 / 249, 6e6 396 / 500 / 617 against 384 / 389 / 444
 //   stamps in 16 B records while those fit, 8e6: 531 / 536 / 605
 //   write-free above: 8e6 522 / 528 / 653, 1.2e7 711 / 719 against 815 / 823
+// F16i has 31 bits for ruler ids, Record8 for successors.
 Level0Plan plan_level0(const Params& p, uint64_t n, WKind wk) {
   constexpr uint64_t SPLIT_BYTES = 88ull << 20;
   const uint64_t split = n * (wk == WKind::Unit ? 16 : wk == WKind::U32 ? 24 : 32);
   const uint64_t log_min = wk == WKind::I64 ? 12000000 : 8000000;
   Level0Plan plan;
   plan.write_free = p.level0_mode == 2 || (p.level0_mode != 1 && n >= log_min);
-  if (!plan.write_free && split > SPLIT_BYTES && n < F16i::NONE)
+  if (!plan.write_free && split > SPLIT_BYTES && n / p.spacing0 + 1 < F16i::NONE)
     plan.fmt = Format::F16i;
   else if (n > REC8_MAX || wk == WKind::I64)
     plan.fmt = Format::F16x16;
@@ -985,16 +997,68 @@ Level0Plan plan_level0(const Params& p, uint64_t n, WKind wk) {
   return plan;
 }
 
-Rulers level0_rulers(const Params& p) { return make_rulers(p.spacing0, salt_for(p.seed, 0)); }
-
 kascade_status alloc_level0(kascade_ctx& ctx, const Level0Plan& plan, uint64_t cap, Level0* l0) {
   const bool wide = plan.fmt == Format::F16x16 || plan.fmt == Format::F16i;
   l0->fmt = plan.fmt;
+  l0->stamp = nullptr;
   l0->rec = alloc<char>(ctx, cap * (wide ? 16 : 8));
   if (!l0->rec) return KASCADE_ERR_OOM;
   if (plan.write_free) return KASCADE_OK;
   l0->stamp = plan.fmt == Format::F16i ? l0->rec : alloc<char>(ctx, cap * (plan.fmt == Format::F8x8 ? 8 : 16));
   return l0->stamp ? KASCADE_OK : KASCADE_ERR_OOM;
+}
+
+// The levels of n elements, and their arrays.
+kascade_status alloc_levels(kascade_ctx& ctx, uint32_t n, const Params& p, Levels* lv) {
+  *lv = Levels{};
+  const int max_levels = (int)std::min<uint32_t>(p.max_levels, MAX_LEVELS);
+  const uint32_t base = std::max(1u, p.base_max);
+  int k = 0;
+  lv->n[0] = n;
+  while (lv->n[k] > base && k < max_levels) {
+    const uint32_t sp = p.spacing_deep ? p.spacing_deep : deep_spacing(lv->n[k], ONE_CTA_MAX * 3 / 4);
+    lv->rulers[k] = k == 0 ? level0_rulers(p) : make_rulers(sp, salt_for(p.seed, k));
+    lv->n[k + 1] = ruler_count(lv->n[k], lv->rulers[k]);
+    ++k;
+  }
+  lv->last = k;
+  lv->rulers[k] = cta_rulers(lv->n[k]);
+  ctx.last_levels.assign(lv->n, lv->n + k + 1);
+  for (int i = 1; i <= k; ++i) {
+    lv->rec[i] = alloc<Rec>(ctx, lv->n[i]);
+    lv->stamp[i] = i < k ? alloc<uint4>(ctx, lv->n[i]) : nullptr;
+    lv->rootel[i] = alloc<uint32_t>(ctx, lv->n[i]);
+    lv->out[i] = alloc<Out>(ctx, lv->n[i]);
+    if (!lv->rec[i] || (i < k && !lv->stamp[i]) || !lv->rootel[i] || !lv->out[i]) return KASCADE_ERR_OOM;
+  }
+  if (lv->n[k] > ONE_CTA_MAX) {
+    for (PdRec*& j : lv->jump) {
+      j = alloc<PdRec>(ctx, lv->n[k]);
+      if (!j) return KASCADE_ERR_OOM;
+    }
+  }
+  return KASCADE_OK;
+}
+
+kascade_status alloc_lists_as(kascade_ctx& ctx, const Params& p, const Level0Plan& plan, uint64_t n, Lists* l) {
+  *l = Lists{};
+  l->n = (uint32_t)n;
+  l->write_free = plan.write_free;
+  KS_TRY(alloc_level0(ctx, plan, n, &l->l0));
+  if (n <= p.base_max) return KASCADE_OK;
+  KS_TRY(alloc_levels(ctx, l->n, p, &l->lv));
+  return plan.write_free ? alloc_log(ctx, l->n, l->lv.n[1], p, &l->log) : KASCADE_OK;
+}
+
+}  // namespace
+
+kascade_status alloc_lists(kascade_ctx& ctx, const Params& p, uint64_t n, WKind wk, Lists* l) {
+  const Level0Plan plan = plan_level0(p, n, wk);
+  const kascade_status st = arena_try(ctx, [&] { return alloc_lists_as(ctx, p, plan, n, l); });
+  if (st != KASCADE_ERR_OOM || !plan.write_free) return st;
+  Params q = p;
+  q.level0_mode = 1;
+  return arena_try(ctx, [&] { return alloc_lists_as(ctx, q, plan_level0(q, n, wk), n, l); });
 }
 
 namespace {
@@ -1094,12 +1158,10 @@ kascade_status rank_trees_one_cta(kascade_ctx& ctx, const Rec* rec, const uint32
 // Doubling for a fixed number of rounds, enough for any list the level can
 // hold: no host wait.  Only a recursion depth limited by the caller ends on a
 // level larger than one CTA ranks.
-static kascade_status pointer_double_level(kascade_ctx& ctx, const Rec* rec, const Extent& ext,
-                                           const uint32_t* rootel, Out* out, cudaStream_t s) {
+static kascade_status pointer_double_level(kascade_ctx& ctx, const Levels& lv, const Extent& ext, cudaStream_t s) {
   const uint32_t m = ext.cap;
-  PdRec* a = alloc<PdRec>(ctx, m);
-  PdRec* b = alloc<PdRec>(ctx, m);
-  if (!a || !b) return KASCADE_ERR_OOM;
+  const Rec* rec = lv.rec[lv.last];
+  PdRec *a = lv.jump[0], *b = lv.jump[1];
   const unsigned grid = grid_for(ctx, m, 256, 8);
   ProfScope ps(ctx, "pd_final_level", s);
   k_pd_init<<<grid, 256, 0, s>>>(rec, ext, a, ctx.d_status);
@@ -1115,38 +1177,13 @@ static kascade_status pointer_double_level(kascade_ctx& ctx, const Rec* rec, con
   }
   k_pd_check<<<grid, 256, 0, s>>>(a, ext, ctx.d_status);
   KS_CHECK_LAUNCH();
-  k_pd_final<SinkOut><<<grid, 256, 0, s>>>(a, ext, rootel, SinkOut{out});
+  k_pd_final<SinkOut><<<grid, 256, 0, s>>>(a, ext, lv.rootel[lv.last], SinkOut{lv.out[lv.last]});
   KS_CHECK_LAUNCH();
   return KASCADE_OK;
 }
 
 // Ruler gaps are geometric: longer than this has probability ~e^-64.
 uint32_t hop_cap(const Rulers& rl) { return (uint32_t)std::min<uint64_t>(64ull * rl.s + 1024, 0xFFFFFFFFull); }
-
-kascade_status plan_levels(kascade_ctx& ctx, uint32_t n, const Params& p, Levels* lv) {
-  *lv = Levels{};
-  const int max_levels = (int)std::min<uint32_t>(p.max_levels, MAX_LEVELS);
-  const uint32_t base = std::max(1u, p.base_max);
-  int k = 0;
-  lv->n[0] = n;
-  while (lv->n[k] > base && k < max_levels) {
-    const uint32_t sp = p.spacing_deep ? p.spacing_deep : deep_spacing(lv->n[k], ONE_CTA_MAX * 3 / 4);
-    lv->rulers[k] = k == 0 ? level0_rulers(p) : make_rulers(sp, salt_for(p.seed, k));
-    lv->n[k + 1] = ruler_count(lv->n[k], lv->rulers[k]);
-    ++k;
-  }
-  lv->last = k;
-  lv->rulers[k] = cta_rulers(lv->n[k]);
-  ctx.last_levels.assign(lv->n, lv->n + k + 1);
-  for (int i = 1; i <= k; ++i) {
-    lv->rec[i] = alloc<Rec>(ctx, lv->n[i]);
-    lv->stamp[i] = i < k ? alloc<uint4>(ctx, lv->n[i]) : nullptr;
-    lv->rootel[i] = alloc<uint32_t>(ctx, lv->n[i]);
-    lv->out[i] = alloc<Out>(ctx, lv->n[i]);
-    if (!lv->rec[i] || (i < k && !lv->stamp[i]) || !lv->rootel[i] || !lv->out[i]) return KASCADE_ERR_OOM;
-  }
-  return KASCADE_OK;
-}
 
 kascade_status rank_deep(kascade_ctx& ctx, const Levels& lv, cudaStream_t s) {
   for (int k = 1; k < lv.last; ++k)
@@ -1158,7 +1195,7 @@ kascade_status rank_deep(kascade_ctx& ctx, const Levels& lv, cudaStream_t s) {
     KS_TRY(launch_rank_cta(ctx, CtaRecords<F16x16, true>{lv.rec[L], lv.rootel[L]}, ext, SinkOut{lv.out[L]}, CTA_LISTS,
                            false, s));
   } else {
-    KS_TRY(pointer_double_level(ctx, lv.rec[L], ext, lv.rootel[L], lv.out[L], s));
+    KS_TRY(pointer_double_level(ctx, lv, ext, s));
   }
   for (int k = L - 1; k >= 1; --k)
     KS_TRY(launch_propagate<F16x16>(ctx, lv, k, lv.rec[k], lv.stamp[k], SinkOut{lv.out[k]}, false, s));
@@ -1168,38 +1205,36 @@ kascade_status rank_deep(kascade_ctx& ctx, const Levels& lv, cudaStream_t s) {
 namespace {
 
 template <class F, class Sink>
-kascade_status rank_records_as(kascade_ctx& ctx, const Level0& l0, uint32_t n, const Sink& sink, CtaMode mode,
-                               const Params& p, cudaStream_t s) {
-  const typename F::R* rec = l0.records<F>();
-  if (n <= p.base_max) {
-    ctx.last_levels.assign(1, n);
+kascade_status rank_records_as(kascade_ctx& ctx, const Lists& l, const Sink& sink, CtaMode mode, const Params& p,
+                               cudaStream_t s) {
+  const typename F::R* rec = l.l0.records<F>();
+  if (l.n <= p.base_max) {
+    ctx.last_levels.assign(1, l.n);
     Extent ext;
-    ext.cap = n;
+    ext.cap = l.n;
     return launch_rank_cta(ctx, CtaRecords<F, false>{rec, nullptr}, ext, sink, mode, p.last, s);
   }
-  Levels lv;
-  KS_TRY(plan_levels(ctx, n, p, &lv));
-  KS_TRY(launch_chase<F>(ctx, lv, 0, rec, l0.stamps<F>(), p.block, s));
-  KS_TRY(rank_deep(ctx, lv, s));
-  return launch_propagate<F>(ctx, lv, 0, rec, l0.stamps<F>(), sink, p.last, s);
+  KS_TRY(launch_chase<F>(ctx, l.lv, 0, rec, l.l0.stamps<F>(), p.block, s));
+  KS_TRY(rank_deep(ctx, l.lv, s));
+  return launch_propagate<F>(ctx, l.lv, 0, rec, l.l0.stamps<F>(), sink, p.last, s);
 }
 
 }  // namespace
 
 template <class Sink>
-kascade_status rank_records(kascade_ctx& ctx, const Level0& l0, uint32_t n, const Sink& sink, CtaMode mode,
-                            const Params& p, cudaStream_t s) {
-  if (n == 0) return KASCADE_OK;
-  if (n > p.base_max && !l0.stamp) return rank_level0_log(ctx, l0, n, sink.log_target(), p, s);
-  switch (l0.fmt) {
+kascade_status rank_records(kascade_ctx& ctx, const Lists& l, const Sink& sink, CtaMode mode, const Params& p,
+                            cudaStream_t s) {
+  if (l.n == 0) return KASCADE_OK;
+  if (l.n > p.base_max && l.write_free) return rank_level0_log(ctx, l, sink.log_target(), p, s);
+  switch (l.l0.fmt) {
     case Format::F8x8:
-      return rank_records_as<F8x8>(ctx, l0, n, sink, mode, p, s);
+      return rank_records_as<F8x8>(ctx, l, sink, mode, p, s);
     case Format::F8x16:
-      return rank_records_as<F8x16>(ctx, l0, n, sink, mode, p, s);
+      return rank_records_as<F8x16>(ctx, l, sink, mode, p, s);
     case Format::F16i:
-      return rank_records_as<F16i>(ctx, l0, n, sink, mode, p, s);
+      return rank_records_as<F16i>(ctx, l, sink, mode, p, s);
     default:
-      return rank_records_as<F16x16>(ctx, l0, n, sink, mode, p, s);
+      return rank_records_as<F16x16>(ctx, l, sink, mode, p, s);
   }
 }
 
@@ -1223,9 +1258,9 @@ kascade_status check_is_list(kascade_ctx& ctx, const uint64_t* succ, uint64_t n,
 }
 
 // explicit instantiations for the level-0 sinks
-template kascade_status rank_records<SinkPlain>(kascade_ctx&, const Level0&, uint32_t, const SinkPlain&, CtaMode,
-                                                const Params&, cudaStream_t);
-template kascade_status rank_records<SinkBatch>(kascade_ctx&, const Level0&, uint32_t, const SinkBatch&, CtaMode,
-                                                const Params&, cudaStream_t);
+template kascade_status rank_records<SinkPlain>(kascade_ctx&, const Lists&, const SinkPlain&, CtaMode, const Params&,
+                                                cudaStream_t);
+template kascade_status rank_records<SinkBatch>(kascade_ctx&, const Lists&, const SinkBatch&, CtaMode, const Params&,
+                                                cudaStream_t);
 
 }  // namespace ks

@@ -200,15 +200,50 @@ struct Level0 {
   template <class F>
   typename F::S* stamps() const { return static_cast<typename F::S*>(stamp); }
 };
-// How level 0 of n elements of that weight kind runs: the
-// records' format, and whether it takes the write-free path.
-struct Level0Plan {
-  Format fmt;
-  bool write_free;
+
+// The levels of one call.  Level k >= 1 holds level k - 1's rulers: records
+// {distance, next ruler}, the root of a list end and results.
+constexpr int MAX_LEVELS = 24;
+struct Levels {
+  int last = 0;                  // the level ranked by one CTA (or by doubling)
+  uint32_t n[MAX_LEVELS + 1];    // elements per level
+  Rulers rulers[MAX_LEVELS + 1];  // each level's rulers; the last one's: the one-CTA ranker's
+  Rec* rec[MAX_LEVELS + 1];      // from level 1 on
+  uint4* stamp[MAX_LEVELS + 1];  // from level 1 on, but not of the last level
+  uint32_t* rootel[MAX_LEVELS + 1];  // level k >= 1: a list end's root as a level-0 element
+  Out* out[MAX_LEVELS + 1];
+  PdRec* jump[2];                // a last level that doubling ranks
 };
-Level0Plan plan_level0(const Params& p, uint64_t n, WKind wk);
-// Its arrays, for a capacity of `cap` elements.
-kascade_status alloc_level0(kascade_ctx& ctx, const Level0Plan& plan, uint64_t cap, Level0* l0);
+
+// The write-free chase's log and what its entries are partitioned with
+// (chase_log.cu).
+struct LogEnt;
+struct Log {
+  LogEnt* ent = nullptr;
+  uint32_t nchunks = 0;
+  unsigned grid = 1;                 // blocks of the chase
+  bool direct = false;               // one partition pass
+  uint32_t* zero = nullptr;          // zeroed by one memset:
+  uint64_t zero_words = 0;
+  uint32_t *cursor = nullptr, *ucount = nullptr;   // the log's next chunk, unreached elements
+  uint32_t *cursor1 = nullptr, *cursor2 = nullptr;  // windows, sub-windows
+  uint32_t* fill = nullptr;                        // per chunk
+  LogEnt *part = nullptr, *part2 = nullptr;
+};
+
+// What ranking a call's n list elements takes, allocated before anything that
+// uses it is enqueued.
+struct Lists {
+  uint32_t n = 0;
+  bool write_free = false;
+  Level0 l0;
+  Levels lv;  // above base_max elements
+  Log log;    // write-free
+};
+// Write-free takes up to 2.8 times the stamping path's memory (2^26 elements in
+// place 51 B an element against 18.1): a call whose memory does not suffice for
+// it stamps.
+kascade_status alloc_lists(kascade_ctx& ctx, const Params& p, uint64_t n, WKind wk, Lists* l);
 
 // Level-0 records of a list from (succ, weights), stamps cleared; a root's
 // record carries weight 0.
@@ -233,34 +268,44 @@ kascade_status rank_trees_one_cta(kascade_ctx& ctx, const Rec* rec, const uint32
                                   Out* out, cudaStream_t s);
 kascade_status rank_parents_one_cta(kascade_ctx& ctx, const uint32_t* parent, uint32_t n, const SinkBatch& sink,
                                     bool last, cudaStream_t s);
-// A batch's forests, parents in one compact vertex space (tree.cu).  last: the
-// call's last device work.
-kascade_status root_forests(kascade_ctx& ctx, const uint32_t* parent, uint32_t n, const SinkBatch& sink, bool last,
-                            const Params& p, cudaStream_t s);
+// A forest's levels: level k + 1 holds level k's rulers.
+struct TreeLevels {
+  int last = 0;
+  Extent ext[MAX_LEVELS + 1];
+  Rulers rulers[MAX_LEVELS + 1];
+};
+// Records, roots and results of the levels from 1 on.
+template <class R, class O>
+struct TreeRulers {
+  R* rec[MAX_LEVELS + 1] = {};
+  uint32_t* root[MAX_LEVELS + 1] = {};
+  O* out[MAX_LEVELS + 1] = {};
+};
+// What rooting a forest takes, allocated before anything is enqueued (tree.cu).
+struct Forest {
+  uint32_t n = 0;
+  TreeLevels lv;
+  bool bits = false;  // child flags in bits
+  char* inner = nullptr;
+  uint32_t *sums = nullptr, *count = nullptr, *rec = nullptr, *vert = nullptr;
+  uint2 *iw = nullptr, *out = nullptr;
+  TreeRulers<Rec8, uint2> up;
+};
+// A batch's forests, parents in one compact vertex space.  last: the call's
+// last device work.
+kascade_status alloc_forests(kascade_ctx& ctx, uint32_t n, const Params& p, Forest* f);
+kascade_status root_forests(kascade_ctx& ctx, const uint32_t* parent, const Forest& f, const SinkBatch& sink, bool last,
+                            cudaStream_t s);
 // Any forest: results of every element (tree.cu).
 kascade_status rank_forest_weighted(kascade_ctx& ctx, const uint64_t* succ, WKind wk, const void* w, uint32_t n,
                                     const SinkPlain& sink, const Params& p, cudaStream_t s);
 
 // Rank level-0 records and deliver the results to the sink.  Every level's
-// size is known on the host: no host wait between the launches.  `ext`: the
-// record count when only the device knows it (ext.cap == n).
+// size is known on the host: no host wait between the launches.
 template <class Sink>
-kascade_status rank_records(kascade_ctx& ctx, const Level0& l0, uint32_t n, const Sink& sink, CtaMode mode,
-                            const Params& p, cudaStream_t s);
+kascade_status rank_records(kascade_ctx& ctx, const Lists& l, const Sink& sink, CtaMode mode, const Params& p,
+                            cudaStream_t s);
 
-// The levels of one call.  Level k >= 1 holds level k - 1's rulers: records
-// {distance, next ruler}, the root of a list end and results.
-constexpr int MAX_LEVELS = 24;
-struct Levels {
-  int last = 0;                  // the level ranked by one CTA (or by doubling)
-  uint32_t n[MAX_LEVELS + 1];    // elements per level
-  Rulers rulers[MAX_LEVELS + 1];  // each level's rulers; the last one's: the one-CTA ranker's
-  Rec* rec[MAX_LEVELS + 1];      // from level 1 on
-  uint4* stamp[MAX_LEVELS + 1];  // from level 1 on, but not of the last level
-  uint32_t* rootel[MAX_LEVELS + 1];  // level k >= 1: a list end's root as a level-0 element
-  Out* out[MAX_LEVELS + 1];
-};
-kascade_status plan_levels(kascade_ctx& ctx, uint32_t n, const Params& p, Levels* lv);
 // Levels 1..last once the level-0 chase has written level 1: fills lv.out[1].
 kascade_status rank_deep(kascade_ctx& ctx, const Levels& lv, cudaStream_t s);
 
@@ -308,8 +353,8 @@ kascade_status compute_stats(kascade_ctx& ctx, const uint64_t* root, const int64
 // Write-free level 0: read-only chase that logs (element, ruler, distance),
 // recursion on the ruler list, then two radix passes over the log by element
 // and a dense placement into the outputs.
-kascade_status rank_level0_log(kascade_ctx& ctx, const Level0& l0, uint32_t n, const LogTarget& t, const Params& p,
-                               cudaStream_t s);
+kascade_status alloc_log(kascade_ctx& ctx, uint32_t n, uint32_t rulers, const Params& p, Log* log);
+kascade_status rank_level0_log(kascade_ctx& ctx, const Lists& l, const LogTarget& t, const Params& p, cudaStream_t s);
 
 // Validation: *ok = 1 if no element has two predecessors.
 kascade_status check_is_list(kascade_ctx& ctx, const uint64_t* succ, uint64_t n, int* ok,

@@ -405,12 +405,6 @@ __global__ void __launch_bounds__(TREE_THREADS) k_tree_propagate(const typename 
   publish_status(st, status);
 }
 
-struct TreeLevels {
-  int last = 0;
-  Extent ext[MAX_LEVELS + 1];
-  Rulers rulers[MAX_LEVELS + 1];
-};
-
 // Levels of n elements, or of as many of them as *count says.
 TreeLevels plan_tree(uint32_t n, const uint32_t* count, const Params& p) {
   TreeLevels lv;
@@ -460,63 +454,83 @@ kascade_status tree_propagate(kascade_ctx& ctx, const TreeLevels& lv, int k, con
   return KASCADE_OK;
 }
 
+template <class R, class O>
+kascade_status alloc_rulers(kascade_ctx& ctx, const TreeLevels& lv, TreeRulers<R, O>* up) {
+  for (int k = 1; k <= lv.last; ++k) {
+    const uint64_t cap = lv.ext[k].cap;
+    up->rec[k] = alloc<R>(ctx, cap);
+    up->root[k] = alloc<uint32_t>(ctx, cap);
+    up->out[k] = alloc<O>(ctx, cap);
+    if (!up->rec[k] || !up->root[k] || !up->out[k]) return KASCADE_ERR_OOM;
+  }
+  return KASCADE_OK;
+}
+
 // Levels 0..last from level 0's records; there is at least one ruler level.
 template <class L, class N, class SinkN, class Sink>
 kascade_status rank_tree(kascade_ctx& ctx, const TreeLevels& lv, const typename L::R* rec, const uint32_t* rootel,
-                         const Sink& sink, bool last, cudaStream_t s) {
-  typename N::R* nrec[MAX_LEVELS + 1] = {};
-  uint32_t* nroot[MAX_LEVELS + 1] = {};
-  typename N::O* nout[MAX_LEVELS + 1] = {};
-  for (int k = 1; k <= lv.last; ++k) {
-    const uint64_t cap = lv.ext[k].cap;
-    nrec[k] = alloc<typename N::R>(ctx, cap);
-    nroot[k] = alloc<uint32_t>(ctx, cap);
-    nout[k] = alloc<typename N::O>(ctx, cap);
-    if (!nrec[k] || !nroot[k] || !nout[k]) return KASCADE_ERR_OOM;
-  }
-  KS_TRY((tree_chase<L, N>(ctx, lv, 0, rec, rootel, nrec[1], nroot[1], s)));
+                         const TreeRulers<typename N::R, typename N::O>& up, const Sink& sink, bool last,
+                         cudaStream_t s) {
+  KS_TRY((tree_chase<L, N>(ctx, lv, 0, rec, rootel, up.rec[1], up.root[1], s)));
   for (int k = 1; k < lv.last; ++k)
-    KS_TRY((tree_chase<N, N>(ctx, lv, k, nrec[k], nroot[k], nrec[k + 1], nroot[k + 1], s)));
-  KS_TRY(rank_trees_one_cta(ctx, nrec[lv.last], nroot[lv.last], lv.ext[lv.last], nout[lv.last], s));
+    KS_TRY((tree_chase<N, N>(ctx, lv, k, up.rec[k], up.root[k], up.rec[k + 1], up.root[k + 1], s)));
+  KS_TRY(rank_trees_one_cta(ctx, up.rec[lv.last], up.root[lv.last], lv.ext[lv.last], up.out[lv.last], s));
   for (int k = lv.last - 1; k >= 1; --k)
-    KS_TRY((tree_propagate<N, N>(ctx, lv, k, nrec[k], nroot[k], nout[k + 1], SinkN{nout[k]}, false, s)));
-  return tree_propagate<L, N>(ctx, lv, 0, rec, rootel, nout[1], sink, last, s);
+    KS_TRY((tree_propagate<N, N>(ctx, lv, k, up.rec[k], up.root[k], up.out[k + 1], SinkN{up.out[k]}, false, s)));
+  return tree_propagate<L, N>(ctx, lv, 0, rec, rootel, up.out[1], sink, last, s);
+}
+
+uint32_t words_of(uint32_t n) { return (uint32_t)(((uint64_t)n + 31) / 32); }
+uint32_t tiles_of(uint32_t n) { return (words_of(n) + WORDS_TILE - 1) / WORDS_TILE; }
+uint64_t inner_bytes(const Forest& f) { return (f.bits ? 4ull : 32ull) * words_of(f.n); }
+
+kascade_status alloc_forest_once(kascade_ctx& ctx, uint32_t n, bool bits, const Params& p, Forest* f) {
+  *f = Forest{};
+  f->n = n;
+  f->bits = bits;
+  if (n == 0) return KASCADE_OK;
+  f->count = alloc<uint32_t>(ctx, 1);
+  if (!f->count) return KASCADE_ERR_OOM;
+  f->lv = plan_tree(n, f->count, p);
+  if (f->lv.last == 0) return KASCADE_OK;
+  f->inner = alloc<char>(ctx, inner_bytes(*f));
+  f->sums = alloc<uint32_t>(ctx, tiles_of(n));
+  f->iw = alloc<uint2>(ctx, words_of(n));
+  f->rec = alloc<uint32_t>(ctx, n);
+  f->vert = alloc<uint32_t>(ctx, n);
+  f->out = alloc<uint2>(ctx, n);
+  if (!f->inner || !f->sums || !f->iw || !f->rec || !f->vert || !f->out) return KASCADE_ERR_OOM;
+  return alloc_rulers(ctx, f->lv, &f->up);
+}
+
+kascade_status alloc_forest(kascade_ctx& ctx, uint32_t n, bool bits, const Params& p, Forest* f) {
+  return arena_try(ctx, [&] { return alloc_forest_once(ctx, n, bits, p, f); });
 }
 
 // Depths and roots of a forest of more than TREE_BASE vertices.
 template <class P, class Sink>
-kascade_status root_levels(kascade_ctx& ctx, const P* parent, uint32_t n, const TreeLevels& lv, uint32_t* count,
-                           const Sink& sink, bool report, bool last, cudaStream_t s) {
-  const uint32_t words = (uint32_t)(((uint64_t)n + 31) / 32);
-  const uint32_t tiles = (words + WORDS_TILE - 1) / WORDS_TILE;
-  const bool bits = n > (sizeof(P) == 4 ? TREE_BYTES_MAX_BATCH : TREE_BYTES_MAX);
-  const uint64_t inner_bytes = (bits ? 4ull : 32ull) * words;
-  char* inner = alloc<char>(ctx, inner_bytes);
-  uint32_t* sums = alloc<uint32_t>(ctx, tiles);
-  uint2* iw = alloc<uint2>(ctx, words);
-  uint32_t* rec = alloc<uint32_t>(ctx, n);
-  uint32_t* vert = alloc<uint32_t>(ctx, n);
-  uint2* out = alloc<uint2>(ctx, n);
-  if (!inner || !sums || !iw || !rec || !vert || !out) return KASCADE_ERR_OOM;
+kascade_status root_levels(kascade_ctx& ctx, const P* parent, const Forest& f, const Sink& sink, bool report, bool last,
+                           cudaStream_t s) {
+  const uint32_t n = f.n, words = words_of(n), tiles = tiles_of(n);
   {
     ProfScope ps(ctx, "prepare", s);
-    KS_CUDA(cudaMemsetAsync(inner, 0, inner_bytes, s));
+    KS_CUDA(cudaMemsetAsync(f.inner, 0, inner_bytes(f), s));
     const unsigned grid = grid_for(ctx, ((uint64_t)n + TREE_PREP_ITEMS - 1) / TREE_PREP_ITEMS, TREE_THREADS, 8);
     auto number = [&](auto* flags) {
       using I = std::remove_reference_t<decltype(*flags)>;
       KS_TRY(launch(ctx, k_tree_inner<P, I>, grid, TREE_THREADS, 0, s, parent, n, flags, ctx.d_status));
-      if (tiles > 1) KS_TRY(launch(ctx, k_tree_count<I>, tiles, TREE_THREADS, 0, s, flags, words, sums));
-      return launch(ctx, k_tree_number<I>, tiles, TREE_THREADS, 0, s, flags, words, sums, iw, count);
+      if (tiles > 1) KS_TRY(launch(ctx, k_tree_count<I>, tiles, TREE_THREADS, 0, s, flags, words, f.sums));
+      return launch(ctx, k_tree_number<I>, tiles, TREE_THREADS, 0, s, flags, words, f.sums, f.iw, f.count);
     };
-    KS_TRY(bits ? number(reinterpret_cast<uint32_t*>(inner)) : number(reinterpret_cast<unsigned char*>(inner)));
+    KS_TRY(f.bits ? number(reinterpret_cast<uint32_t*>(f.inner)) : number(reinterpret_cast<unsigned char*>(f.inner)));
     const unsigned rec_grid = grid_for(ctx, ((uint64_t)n + TREE_REC_ITEMS - 1) / TREE_REC_ITEMS, TREE_THREADS, 8);
-    KS_TRY(launch(ctx, k_tree_records<P>, rec_grid, TREE_THREADS, 0, s, parent, n, iw, lv.rulers[0], rec, vert, report,
+    KS_TRY(launch(ctx, k_tree_records<P>, rec_grid, TREE_THREADS, 0, s, parent, n, f.iw, f.lv.rulers[0], f.rec, f.vert, report,
                   ctx.d_status));
   }
-  KS_TRY((rank_tree<TreeUnit, Tree8, SinkOut8>(ctx, lv, rec, vert, SinkOut8{out}, false, s)));
+  KS_TRY((rank_tree<TreeUnit, Tree8, SinkOut8>(ctx, f.lv, f.rec, f.vert, f.up, SinkOut8{f.out}, false, s)));
   ProfScope ps(ctx, "leaves", s);
   const unsigned grid = grid_for(ctx, ((uint64_t)n + TREE_OUT_ITEMS - 1) / TREE_OUT_ITEMS, TREE_THREADS, 8);
-  KS_TRY(launch(ctx, k_tree_leaves<P, Sink>, grid, TREE_THREADS, 0, s, parent, n, iw, out, sink, ctx.d_status,
+  KS_TRY(launch(ctx, k_tree_leaves<P, Sink>, grid, TREE_THREADS, 0, s, parent, n, f.iw, f.out, sink, ctx.d_status,
                 status_host(ctx, last)));
   return KASCADE_OK;
 }
@@ -527,23 +541,23 @@ kascade_status root_forest_impl(kascade_ctx& ctx, const uint64_t* parent, uint32
                                 uint64_t* depth_out, int keep_roots, const Params& p, cudaStream_t s) {
   if (n == 0) return KASCADE_OK;
   const SinkPlain sink{root_out, depth_out, keep_roots};
-  uint32_t* count = alloc<uint32_t>(ctx, 1);
-  if (!count) return KASCADE_ERR_OOM;
-  const TreeLevels lv = plan_tree(n, count, p);
-  if (lv.last == 0) return rank_arrays_one_cta(ctx, parent, WKind::Unit, nullptr, n, sink, CTA_ROOTING, s);
+  Forest f;
+  KS_TRY(alloc_forest(ctx, n, n > TREE_BYTES_MAX, p, &f));
+  if (f.lv.last == 0) return rank_arrays_one_cta(ctx, parent, WKind::Unit, nullptr, n, sink, CTA_ROOTING, s);
   ctx.last_levels.assign(1, n);
-  for (int k = 1; k <= lv.last; ++k) ctx.last_levels.push_back(lv.ext[k].cap);
-  return root_levels(ctx, parent, n, lv, count, sink, true, true, s);
+  for (int k = 1; k <= f.lv.last; ++k) ctx.last_levels.push_back(f.lv.ext[k].cap);
+  return root_levels(ctx, parent, f, sink, true, true, s);
 }
 
-kascade_status root_forests(kascade_ctx& ctx, const uint32_t* parent, uint32_t n, const SinkBatch& sink, bool last,
-                            const Params& p, cudaStream_t s) {
-  if (n == 0) return KASCADE_OK;
-  uint32_t* count = alloc<uint32_t>(ctx, 1);
-  if (!count) return KASCADE_ERR_OOM;
-  const TreeLevels lv = plan_tree(n, count, own_spacing(p));  // (a batch's is its lists')
-  if (lv.last == 0) return rank_parents_one_cta(ctx, parent, n, sink, last, s);
-  return root_levels(ctx, parent, n, lv, count, sink, false, last, s);
+kascade_status alloc_forests(kascade_ctx& ctx, uint32_t n, const Params& p, Forest* f) {
+  return alloc_forest(ctx, n, n > TREE_BYTES_MAX_BATCH, own_spacing(p), f);  // (a batch's spacing is its lists')
+}
+
+kascade_status root_forests(kascade_ctx& ctx, const uint32_t* parent, const Forest& f, const SinkBatch& sink, bool last,
+                            cudaStream_t s) {
+  if (f.n == 0) return KASCADE_OK;
+  if (f.lv.last == 0) return rank_parents_one_cta(ctx, parent, f.n, sink, last, s);
+  return root_levels(ctx, parent, f, sink, false, last, s);
 }
 
 kascade_status rank_forest_weighted(kascade_ctx& ctx, const uint64_t* succ, WKind wk, const void* w, uint32_t n,
@@ -552,11 +566,15 @@ kascade_status rank_forest_weighted(kascade_ctx& ctx, const uint64_t* succ, WKin
   if (lv.last == 0) return rank_arrays_one_cta(ctx, succ, wk, w, n, sink, CTA_TREES, s);
   ctx.last_levels.assign(1, n);
   Level0 l0;  // F16x16, no stamps
-  Rec* rec = alloc<Rec>(ctx, n);
-  if (!rec) return KASCADE_ERR_OOM;
+  Rec* rec = nullptr;
+  TreeRulers<Rec, Out> up;
+  KS_TRY(arena_try(ctx, [&] {
+    rec = alloc<Rec>(ctx, n);
+    return rec ? alloc_rulers(ctx, lv, &up) : KASCADE_ERR_OOM;
+  }));
   l0.rec = rec;
   KS_TRY(prepare_arrays(ctx, succ, wk, w, n, l0, lv.rulers[0], s));
-  return rank_tree<Tree16, Tree16, SinkOut>(ctx, lv, rec, nullptr, sink, true, s);
+  return rank_tree<Tree16, Tree16, SinkOut>(ctx, lv, rec, nullptr, up, sink, true, s);
 }
 
 }  // namespace ks
