@@ -113,7 +113,8 @@ KASCADE_API uint64_t kascade_scratch_bytes_rank_list(uint64_t n);
 KASCADE_API uint64_t kascade_scratch_bytes_root_forest(uint64_t n);
 /* Wait for the context's last call on `stream` and return its status. */
 KASCADE_API kascade_status kascade_ctx_sync(kascade_ctx* ctx, void* stream);
-/* Detail of the last device-side error (e.g. the offending index). */
+/* Detail of the last device-side error: the offending index.  (NOT_A_LIST: the
+ * first element with two predecessors, by its place in the caller's arrays.) */
 KASCADE_API uint64_t kascade_ctx_error_info(kascade_ctx* ctx);
 /* Kernel timings of the last profiled call(s): fills up to `cap` entries of
  * names/milliseconds/launch counts, returns the number of kernels. */

@@ -193,6 +193,7 @@ KASCADE_API kascade_status kascade_ctx_reserve(kascade_ctx* c, uint64_t bytes) {
   for (auto& b : c->blocks) have += b.cap;
   c->reserve_bytes = bytes;
   if (have >= bytes && c->blocks.size() == 1) return KASCADE_OK;
+  c->listed = Listed{};
   for (auto& b : c->blocks)
     if (b.owned) cudaFree(b.ptr);
   c->blocks.clear();

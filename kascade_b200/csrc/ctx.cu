@@ -13,6 +13,7 @@ kascade_status cuda_status(cudaError_t e) {
 
 kascade_status arena_begin_call(kascade_ctx& ctx, cudaStream_t s) {
   (void)s;
+  ctx.listed = Listed{};  // (in the arena)
   if (ctx.blocks.size() > 1) {
     // The previous call grew the arena: fold the blocks into one so that the
     // next call of the same size needs no allocation.  Growth is rare, so a
@@ -78,6 +79,7 @@ void arena_rewind(kascade_ctx& ctx, const ArenaMark& m) {
 }
 
 void arena_adopt(kascade_ctx& ctx, char* p, size_t bytes) {
+  ctx.listed = Listed{};
   for (auto& b : ctx.blocks)
     if (b.owned) cudaFree(b.ptr);
   ctx.blocks.clear();
@@ -114,6 +116,34 @@ kascade_status status_publish(kascade_ctx& ctx, cudaStream_t s) {
   return KASCADE_OK;
 }
 
+// Which element has two predecessors, once a call has found that one has.
+static __global__ void __launch_bounds__(256) k_two_predecessors(Listed l, uint32_t* bits, uint32_t* place) {
+  auto succ = [&](uint32_t x) {
+    return l.wide ? static_cast<const Rec*>(l.rec)[x].b : static_cast<const Rec8*>(l.rec)[x].b & ~REC8_RULER;
+  };
+  for (uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; x < l.n; x += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t y = succ((uint32_t)x), bit = 1u << (y & 31);
+    if (y == x || !(atomicOr(bits + (y >> 5), bit) & bit) || succ(y) == y) continue;
+    atomicMin(place, l.seg.n ? y + l.seg.delta[l.seg.find(y)] : y);
+  }
+}
+
+kascade_status find_two_predecessors(kascade_ctx& ctx, uint32_t* place, cudaStream_t s) {
+  const uint64_t words = ((uint64_t)ctx.listed.n + 31) / 32;
+  const ArenaMark m = arena_mark(ctx);
+  uint32_t* bits = alloc<uint32_t>(ctx, words + 1);
+  if (!bits) return KASCADE_ERR_OOM;
+  kascade_status st = cuda_status(cudaMemsetAsync(bits, 0, words * 4, s));
+  if (st == KASCADE_OK) st = cuda_status(cudaMemsetAsync(bits + words, 0xFF, 4, s));
+  if (st == KASCADE_OK) {
+    k_two_predecessors<<<grid_for(ctx, ctx.listed.n, 256, 8), 256, 0, s>>>(ctx.listed, bits, bits + words);
+    st = cuda_status(cudaGetLastError());
+  }
+  if (st == KASCADE_OK) st = read_u32(ctx, bits + words, place, s);
+  arena_rewind(ctx, m);
+  return st;
+}
+
 static void collect_times(kascade_ctx& ctx) {
   for (auto& p : ctx.pending) {
     float ms = 0.f;
@@ -147,6 +177,10 @@ kascade_status status_finish(kascade_ctx& ctx, cudaStream_t s) {
   ctx.last_status = (kascade_status)st->code;
   // two chains stamped one element: it has two predecessors
   if (ctx.last_status == KASCADE_OK && st->counter[2] != st->counter[3]) ctx.last_status = KASCADE_ERR_NOT_A_LIST;
+  if (ctx.last_status == KASCADE_ERR_NOT_A_LIST && ctx.listed.rec) {
+    uint32_t place = ~0u;
+    if (find_two_predecessors(ctx, &place, s) == KASCADE_OK && place != ~0u) ctx.error_info = place;
+  }
   return ctx.last_status;
 }
 

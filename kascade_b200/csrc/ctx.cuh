@@ -13,6 +13,17 @@
 #include "common.cuh"
 #include "tuned_classes.h"
 
+namespace ks {
+// A call's list elements: level-0 records, which keep their successors, and
+// where the elements are in the caller's arrays.
+struct Listed {
+  const void* rec = nullptr;  // nullptr: none
+  bool wide = false;          // 16 B records
+  uint32_t n = 0;
+  SegMap seg;
+};
+}  // namespace ks
+
 struct kascade_ctx {
   int device = 0;
   int sm_count = 148;
@@ -23,6 +34,7 @@ struct kascade_ctx {
   // the device status: whether a call since its last clearing may have left it
   // non-zero, and whether the call's last kernel copies it to h_pinned
   bool status_dirty = false, published = false;
+  ks::Listed listed;  // the last call's, if it ranked lists by their records
   // scratch arena: blocks are never freed inside a call, so pointers handed
   // out by alloc() stay valid until the next begin_call()
   struct Block {
@@ -134,6 +146,9 @@ unsigned long long* status_host(kascade_ctx& ctx, bool last = true);
 kascade_status status_publish(kascade_ctx& ctx, cudaStream_t s);
 // Synchronise `s`, read the status, collect kernel timings.
 kascade_status status_finish(kascade_ctx& ctx, cudaStream_t s);
+// The smallest place in the caller's arrays of an element with two
+// predecessors, a list's end aside (ctx.listed; waits for it); ~0: none.
+kascade_status find_two_predecessors(kascade_ctx& ctx, uint32_t* place, cudaStream_t s);
 // Read one device word into the pinned buffer and wait for it.
 kascade_status read_u32(kascade_ctx& ctx, const uint32_t* dptr, uint32_t* out, cudaStream_t s);
 

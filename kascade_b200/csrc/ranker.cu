@@ -456,6 +456,27 @@ struct CtaArrays {
   __device__ __forceinline__ uint32_t root_of(uint32_t x) const { return x; }
 };
 
+// The first element that has two predecessors, a list's end aside (~0: none).
+// predw: a byte for each element, found: one word, both in shared memory.
+template <class Src>
+__device__ __noinline__ uint32_t two_predecessors(const Src& src, uint32_t n, uint32_t* predw, uint32_t* found) {
+  uint64_t a;
+  uint32_t y, z;
+  bool f;
+  if (threadIdx.x == 0) *found = ~0u;
+  for (uint32_t w = threadIdx.x; w < (n + 3) / 4; w += blockDim.x) predw[w] = 0;
+  __syncthreads();
+  for (uint32_t x = threadIdx.x; x < n; x += blockDim.x) {
+    src.load(x, &a, &y, &f);
+    const uint32_t bit = 1u << (8 * (y & 3));
+    if (y >= n || y == x || !(atomicOr(predw + (y >> 2), bit) & bit)) continue;
+    src.load(y, &a, &z, &f);
+    if (z != y) atomicMin(found, y);
+  }
+  __syncthreads();
+  return *found;
+}
+
 template <class Src, class Sink>
 __device__ __forceinline__ void rank_cta(const Src& src, const Extent& ext, const Sink& sink, CtaMode mode,
                                          DevStatus* st) {
@@ -612,7 +633,8 @@ __device__ __forceinline__ void rank_cta(const Src& src, const Extent& ext, cons
     __syncthreads();
     if (!clash && nstamps == 0) break;
     if (mode == CTA_LISTS || n > ONE_CTA_TREES) {
-      if (tid == 0) set_error(st, KASCADE_ERR_NOT_A_LIST, n);
+      const uint32_t x = two_predecessors(src, n, predw, &nheads);
+      if (tid == 0) set_error(st, KASCADE_ERR_NOT_A_LIST, x);
       return;
     }
     __syncthreads();
@@ -1225,6 +1247,8 @@ template <class Sink>
 kascade_status rank_records(kascade_ctx& ctx, const Lists& l, const Sink& sink, CtaMode mode, const Params& p,
                             cudaStream_t s) {
   if (l.n == 0) return KASCADE_OK;
+  const bool wide = l.l0.fmt == Format::F16x16 || l.l0.fmt == Format::F16i;
+  ctx.listed = Listed{l.l0.rec, wide, l.n, sink.log_target().seg};
   if (l.n > p.base_max && l.write_free) return rank_level0_log(ctx, l, sink.log_target(), p, s);
   switch (l.l0.fmt) {
     case Format::F8x8:

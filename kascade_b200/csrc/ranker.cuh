@@ -104,28 +104,6 @@ struct Extent {
 // A sink receives, for element x, its rank, its root (level-0 index) and
 // whether x itself is a root.
 
-// Segments of an element range and where their outputs go: a batch's list or
-// forest elements, instance after instance, are numbered densely; outputs are
-// at the instances' places in the caller's arrays, roots relative to their
-// instance.  At most 2^32 elements: offsets wrap.
-struct SegMap {
-  const uint32_t* base = nullptr;   // n + 1: the segments' first elements, non-decreasing; then the end
-  const uint32_t* delta = nullptr;  // element + delta: its place in the outputs
-  const uint32_t* hint = nullptr;   // [k]: the segment of element 4096 k, and one more for the end
-  uint32_t n = 0;                   // 0: one instance, in place
-  __device__ __forceinline__ uint32_t find(uint32_t x) const {  // the last j with base[j] <= x
-    uint32_t lo = ld_ca(hint + (x >> 12)), hi = min(ld_ca(hint + (x >> 12) + 1) + 1, n);
-    while (hi - lo > 1) {
-      const uint32_t mid = (lo + hi) >> 1;
-      if (ld_ca(base + mid) <= x)
-        lo = mid;
-      else
-        hi = mid;
-    }
-    return lo;
-  }
-};
-
 // Level-0 output description for the write-free (log) pipeline.
 struct LogTarget {
   uint64_t* root;
