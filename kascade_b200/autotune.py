@@ -9,8 +9,10 @@ batched workload's mix) and picks
   3. the ruler spacing for calls that rank one list on their own (up to 32
      lists of the class's sizes, one call each),
 
-by measured elements/s.  Forests have a spacing of their own.  The table it returns is what `load_tuning` installs
-in a context; `write_header` turns it into the library's built-in defaults
+by measured elements/s.  A class that one CTA ranks, without these, keeps what
+the context has.  Forests have a spacing of their own, which a batch's does not
+reach.  The table it returns is what `load_tuning` installs in a context;
+`write_header` turns it into the library's built-in defaults
 (kascade_b200/csrc/tuned_classes.h), so every context starts tuned.
 
     python -m kascade_b200.autotune --json tuning.json --header kascade_b200/csrc/tuned_classes.h
@@ -29,10 +31,16 @@ import numpy as np
 CLASS_MAX = (1 << 10, 1 << 13, 1 << 16, 1 << 19, 1 << 22, 1 << 25, 1 << 27, (1 << 64) - 1)
 SPACINGS = (4, 6, 8, 12, 16, 24, 32, 48, 64, 96, 128)
 BLOCKS = (128, 256, 512)
+ONE_CTA_MAX = 14336  # elements that one CTA ranks, whatever the spacing
 
 
 def class_bounds(k: int):
     return (64 if k == 0 else CLASS_MAX[k - 1] + 1, CLASS_MAX[k] if k + 1 < len(CLASS_MAX) else 1 << 28)
+
+
+def uses_rulers(k: int) -> bool:
+    """Whether the spacing and block size of class k matter to a call of its sizes."""
+    return CLASS_MAX[k] > ONE_CTA_MAX
 
 
 def batch_of_class(k: int, seed: int):
@@ -107,14 +115,16 @@ def tune(device: int = 0, total: int = 1 << 24, reps: int = 3, log=print) -> dic
         def run(t):
             kb.rank_batch(inp, segs, w, tuning=t, root_out=root, rank_out=rank, ctx=ctx)
 
+        had = {"spacing": kb.get_size_classes(ctx)[1][k], "block": kb.get_class_launch(ctx)[1][k],
+               "single": kb.get_class_launch(ctx)[2][k]}
         best = None
-        for sp in SPACINGS:
+        for sp in SPACINGS if uses_rulers(k) else [had["spacing"]]:
             ms = _time_ms(lambda: run(kb.GpuTuning(ruler_spacing=sp)), reps)
             if best is None or ms < best[0]:
                 best = (ms, sp)
         spacing = best[1]
         best = None
-        for b in BLOCKS:
+        for b in BLOCKS if uses_rulers(k) else [had["block"]]:
             t = kb.GpuTuning(ruler_spacing=spacing, block_size=b)
             ms = _time_ms(lambda: run(t), reps)
             if best is None or ms < best[0]:
@@ -140,7 +150,7 @@ def tune(device: int = 0, total: int = 1 << 24, reps: int = 3, log=print) -> dic
                 kb.rank_list(inp[a:b_], w[a:b_], tuning=t, root_out=root[a:b_], rank_out=rank[a:b_], ctx=ctx)
 
         best_single = None
-        for sp in SPACINGS:
+        for sp in SPACINGS if uses_rulers(k) else [had["single"]]:
             t = kb.GpuTuning(ruler_spacing=sp, block_size=block)
             ms1 = _time_ms(lambda: run_single(t), reps)
             if best_single is None or ms1 < best_single[0]:
