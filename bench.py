@@ -946,6 +946,7 @@ def main():
         served = measure_served(kb, dev, batched_rate=batched["elements_per_s"])
 
     if rank == 0:
+        bytes_in = 12 if main_r["weighted"] else 8
         out = {
             "metric": METRIC, "value": main_r["value"], "unit": "elements/s" if kind == "list" else "vertices/s",
             "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
@@ -953,7 +954,7 @@ def main():
             "vs_baseline": None, "dtype": "int64", "data": "synthetic (seeded device generator)",
             "config": {"workload": main_r["desc"], "n": n, "global_elements": n * world,
                        "parallelism": f"replicas x{world} (independent instances, no collective)",
-                       "l2": "inputs larger than L2 (16 B records x n = %.1f GiB)" % (16 * n / 2**30),
+                       "l2": "inputs larger than L2 (%d B of input x n = %.1f GiB)" % (bytes_in, bytes_in * n / 2**30),
                        "ruler_spacing": args.spacing or "auto", "levels": main_r["levels"]},
             "roofline": main_r["roofline"], "pipeline_roofline": main_r["pipeline"],
             "random_access_roofline": random_access_roofline(main_r, hbm),

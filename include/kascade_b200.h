@@ -359,8 +359,9 @@ typedef struct kascade_server kascade_server;
  * replayed by one graph launch per call.  The segment table
  * and the input / weight / output pointers are fixed at creation; their
  * contents may change between launches.  Creation runs the batch once and
- * returns KASCADE_ERR_UNSUPPORTED for a batch made mostly of list ends (very
- * many roots), which kascade_rank_batch handles.  A plan owns its scratch;
+ * returns KASCADE_ERR_UNSUPPORTED for a batch made mostly of list ends (more
+ * than half its ruler count plus 65536 of them, a bound kept from an earlier
+ * form), which kascade_rank_batch handles.  A plan owns its scratch;
  * launches of one plan are ordered on the device.  No counterpart in the
  * reference (its rounds are MPI exchanges per call). */
 typedef struct kascade_batch_plan kascade_batch_plan;

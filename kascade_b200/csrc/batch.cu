@@ -303,8 +303,9 @@ kascade_status rank_batch_impl(kascade_ctx& ctx, const kascade_segment* segs, ui
   return batch_enqueue(ctx, t, in, weights, root_out, rank_out, opts, s);
 }
 
-// Whether a batch may be planned: one made mostly of list ends may not (as
-// documented).  Waits for the count.
+// Whether a batch may be planned.  One made mostly of list ends may not: the
+// bound is that of a recursion whose levels could overflow.  Nothing here can;
+// the refusal is part of the call's documented contract.  Waits for the count.
 static kascade_status plan_admits(kascade_ctx& ctx, const BatchTables& t, const uint64_t* in,
                                   const kascade_opts* opts, cudaStream_t s) {
   uint32_t* count = alloc<uint32_t>(ctx, 1);

@@ -427,8 +427,9 @@ KASCADE_API kascade_status kascade_rank_via_euler_tour(kascade_ctx* c, const kas
   Params p = make_params(*c, opts, 2 * n);
   p.algorithm = KASCADE_ALGO_SPARSE_RULING_SET;
   kascade_status st = KASCADE_OK;
-  // the outputs are written after the last read of the parents (they are read
-  // once, when the records are built)
+  // the outputs overwrite the parents: only the call's last kernel writes them,
+  // and there a thread reads no parents but those of the vertices it writes,
+  // before it writes them (k_tree_leaves; the one-CTA ranker reads them all first)
   if (n) st = root_forest_impl(*c, succ_array, (uint32_t)n, succ_array, (uint64_t*)rank_array, 1, p, s);
   return end_call(c, s, st, opts);
 }

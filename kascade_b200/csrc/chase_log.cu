@@ -1,9 +1,10 @@
 // Write-free level 0 of the ruling-set ranker.
 //
-// On B200 a random 16 B read costs a 128 B DRAM fetch, and writing a record
-// back after reading it roughly halves the random-access rate (random read:
-// ~45 G/s, read + write back: ~17-22 G/s; see `bench.py --calibrate`).  This
-// path therefore never writes at a random address:
+// On B200 a random read costs a DRAM fetch of about 100 B whatever its width (98
+// for the 8 B records here), and writing a record back after reading it roughly
+// halves the random-access rate (16 B records: random read ~45 G/s, read + write
+// back ~17-22 G/s; see `bench.py --calibrate`).  This path therefore never writes
+// at a random address:
 //
 //   chase     read-only walk of every chain; each visited element appends
 //             (element, ruler id, distance from ruler) to a log made of

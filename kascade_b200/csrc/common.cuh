@@ -1,8 +1,8 @@
 // Shared device-side definitions of the B200 list-ranking library.
 //
-// Element state lives in one 16-byte record per element (`Rec`), so that the
-// dependent hop of the ruler chase is a single aligned 16 B load and the
-// chase's own write lands in the same 32 B sector it just read.
+// An element's record holds its weight and successor, so that a dependent hop of
+// the ruler chase is one aligned load of 8 or 16 B; the formats of a level are
+// described below, after the loads.
 #pragma once
 
 #include <cstddef>
@@ -14,11 +14,13 @@
 namespace ks {
 
 // ---------------------------------------------------------------------------
-// Element record.
-//   a : weight (unreached or ruler) or distance from the element's ruler
-//       (reached), as 64-bit two's complement
+// 16 B record.
+//   a : weight, as 64-bit two's complement; in a record that is stamped, the
+//       distance from the element's ruler
 //   b : successor index (every state keeps it)
-//   c : tag -- TAG_UNREACHED, TAG_RULER | ruler id, or a ruler id (reached)
+//   c : by format: whether the successor is a ruler (Record16), that and the
+//       stamp's ruler id (F16i), or, in a shard, the tag TAG_UNREACHED,
+//       TAG_RULER | ruler id, or a ruler id (reached)
 // ---------------------------------------------------------------------------
 struct __align__(16) Rec {
   uint64_t a;
@@ -29,7 +31,6 @@ static_assert(sizeof(Rec) == 16, "record must be 16 bytes");
 
 constexpr uint32_t TAG_UNREACHED = 0xFFFFFFFFu;
 constexpr uint32_t TAG_RULER = 0x80000000u;
-constexpr uint32_t MAX_RULERS = 0x7FFFFFFEu;  // ruler ids stay below this
 constexpr uint32_t MAX_ELEMS = 0xFFFFFFFEu;   // element indices fit in 32 bits
 
 __host__ __device__ __forceinline__ bool tag_unreached(uint32_t c) { return c == TAG_UNREACHED; }
@@ -104,7 +105,8 @@ __device__ __forceinline__ bool sampled(uint32_t x, uint32_t salt, uint32_t thre
 // resident.  Nor may they move above kernel_begin's wait: ld_cg and ld_cs are
 // volatile, as the wait is, and ld_ca is a plain read, which the wait's memory
 // clobber holds back (as a volatile load it cost the forests' walks 1 to 4%:
-// 4.2e6 vertices 232 us, plain 222).
+// 4.2e6 vertices 232 us, plain 222; by __ldg, each kernel started after the one
+// ahead had ended, 249 against 251, pointer doubling of 1e6 184 against 189).
 //   ld_ca  through L1 (what neighbours or later loads read again)
 //   ld_cg  from L2 (random hops, which never hit L1; what other SMs write)
 //   ld_cs  streaming, evict-first

@@ -961,8 +961,8 @@ uint32_t deep_spacing(uint32_t n, uint32_t target) {
 Params make_params(const kascade_ctx& ctx, const kascade_opts* o, uint64_t n) {
   Params p;
   // Spacing trades chase critical path (~ spacing * ln(n/spacing) hops)
-  // against ruler-table size; these defaults are the tuned values for
-  // random lists on B200 (see the autotune table in the batch path).
+  // against ruler-table size; the defaults are the context's size classes
+  // (tuned_classes.h).
   {
     const int k = ctx.class_of(n);
     p.spacing0 = ctx.class_spacing_single[k];

@@ -32,7 +32,7 @@ struct Params {
   uint32_t spacing_given = 0;  // the caller's, if any
   uint32_t spacing_deep = 0;  // mean elements per ruler, deeper levels (0: by level size)
   uint32_t max_levels = 6;
-  uint32_t base_max = 16384;  // one-CTA ranker bound
+  uint32_t base_max = 0x7FFFFFFFu;  // one-CTA ranker bound, at most ONE_CTA_MAX
   uint32_t block = 256;
   uint32_t seed = 0x6b617363u;
   uint32_t algorithm = KASCADE_ALGO_SPARSE_RULING_SET;
@@ -45,7 +45,8 @@ Params make_params(const kascade_ctx& ctx, const kascade_opts* opts, uint64_t n)
 // Ruler placement of one level: element x lies in block x / s, whose ruler is
 // at offset hash(block) in [0, s).  The last block's ruler may fall beyond
 // the level's elements; its id is then dead (a record no element points to).
-// Division by s: the round-up multiply-and-shift for any 32-bit x.
+// Division by s: the round-up multiply-and-shift for any 32-bit x (Granlund and
+// Montgomery, Division by Invariant Integers using Multiplication, 1994).
 struct Rulers {
   uint32_t s = 2, mul = 0, sh = 0, salt = 0;
   __device__ __forceinline__ uint32_t offset(uint32_t j) const { return __umulhi(mix32(j ^ salt), s); }

@@ -272,7 +272,9 @@ __global__ void __launch_bounds__(TREE_THREADS) k_tree_records(const P* parent, 
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&st->counter[1], (unsigned long long)n);
 }
 
-// Every vertex's result from the numbered ones' (depth, root).
+// Every vertex's result from the numbered ones' (depth, root).  `parent` may be
+// the sink's root array: a thread reads the parents of the vertices of its own
+// step only, all before it writes their results.
 template <class P, class Sink>
 __global__ void __launch_bounds__(TREE_THREADS) k_tree_leaves(const P* parent, uint32_t n,
                                                               const uint2* iw,
